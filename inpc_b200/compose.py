@@ -9,7 +9,7 @@ import torch
 from torch.autograd.function import once_differentiable
 
 from . import _cabi
-from .rasterization import _cuda_f32, _ptr, _stream
+from .rasterization import _cuda_f32, _on, _ptr, _stream
 
 
 def _planes(image, alpha, name="image"):
@@ -28,7 +28,7 @@ class _ComposeBackground(torch.autograd.Function):
         if background.shape != image.shape:
             raise ValueError(f"background must have the image's shape {tuple(image.shape)}, got {tuple(background.shape)}")
         out = torch.empty_like(image)
-        with torch.cuda.device(image.device):
+        with _on(image.device):
             _cabi.check(_cabi.lib().inpc_compose_background(_ptr(image), _ptr(alpha), _ptr(background), image.shape[0],
                                                             image.shape[1] * image.shape[2], _ptr(out), _stream()))
         ctx.save_for_backward(alpha, background)
@@ -43,7 +43,7 @@ class _ComposeBackground(torch.autograd.Function):
         grad_alpha = torch.empty_like(alpha) if need_alpha else None
         grad_bg = torch.empty_like(background) if need_bg else None
         if need_alpha or need_bg:
-            with torch.cuda.device(grad_out.device):
+            with _on(grad_out.device):
                 _cabi.check(_cabi.lib().inpc_compose_background_backward(
                     _ptr(grad_out), _ptr(alpha), _ptr(background), grad_out.shape[0], grad_out.shape[1] * grad_out.shape[2],
                     _ptr(grad_alpha), _ptr(grad_bg), _stream()))
@@ -82,7 +82,7 @@ class MultisampleAccumulator:
             self.image, self.depth, self.alpha = torch.empty_like(image), torch.empty_like(depth), torch.empty_like(alpha)
         elif image.shape != self.image.shape:
             raise ValueError("all multisamples must have the same shape")
-        with torch.cuda.device(image.device):
+        with _on(image.device):
             _cabi.check(_cabi.lib().inpc_multisample_accumulate(
                 _ptr(self.image), _ptr(self.depth), _ptr(self.alpha), _ptr(image), _ptr(depth), _ptr(alpha), image.shape[0],
                 alpha.numel(), int(first), int(self.unpremultiply), _stream()))
@@ -98,7 +98,7 @@ class MultisampleAccumulator:
             if background.shape != self.image.shape:
                 raise ValueError("background must have the image's shape")
         alpha_sum = torch.empty_like(self.alpha)
-        with torch.cuda.device(self.image.device):
+        with _on(self.image.device):
             _cabi.check(_cabi.lib().inpc_multisample_resolve(
                 _ptr(self.image), _ptr(self.depth), _ptr(self.alpha), _ptr(alpha_sum), _ptr(background), self.image.shape[0],
                 self.alpha.numel(), self.n, int(self.unpremultiply), _stream()))

@@ -10,7 +10,7 @@ import ctypes as C
 import torch
 
 from . import _cabi
-from .rasterization import _cuda_f32, _ptr, _stream
+from .rasterization import _cuda_f32, _on, _ptr, _stream
 
 DECAY = 0.9968
 
@@ -45,7 +45,7 @@ class LeafStatistics:
         return decode_statistics(self.stats)[1]
 
     def reset(self) -> None:
-        with torch.cuda.device(self.stats.device):
+        with _on(self.stats.device):
             _cabi.check(_cabi.lib().inpc_leaf_stats_reset(_ptr(self.stats), self.stats.shape[0], _stream()))
 
     def accumulate(self, indices: torch.Tensor, weights: torch.Tensor) -> None:
@@ -55,7 +55,7 @@ class LeafStatistics:
         indices = indices.contiguous()
         if indices.numel() != weights.numel():
             raise ValueError("indices and weights must have the same number of elements")
-        with torch.cuda.device(self.stats.device):
+        with _on(self.stats.device):
             _cabi.check(_cabi.lib().inpc_leaf_stats_accumulate(_ptr(indices), _ptr(weights), indices.numel(), _ptr(self.stats),
                                                                self.stats.shape[0], _stream()))
 
@@ -72,7 +72,7 @@ def update(leaf_weights: torch.Tensor, leaf_subdivision_scores: torch.Tensor, st
     for t, name in ((leaf_weights, "leaf_weights"), (leaf_subdivision_scores, "leaf_subdivision_scores")):
         if not t.is_cuda or t.dtype != torch.float32 or not t.is_contiguous():
             raise TypeError(f"{name} must be a contiguous CUDA float32 tensor")
-    with torch.cuda.device(leaf_weights.device):
+    with _on(leaf_weights.device):
         _cabi.check(_cabi.lib().inpc_leaf_update(_ptr(leaf_weights), _ptr(leaf_subdivision_scores), _ptr(stats.stats),
                                                  leaf_weights.numel(), float(decay), _stream()))
 
@@ -116,14 +116,13 @@ def prune(leaf_centers, leaf_levels, leaf_weights, leaf_subdivision_scores, thre
     in their old order, as four new tensors (centers, levels, weights, scores)."""
     centers, levels, weights, scores, n = _leaf_arrays(leaf_centers, leaf_levels, leaf_weights, leaf_subdivision_scores)
     dev = weights.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws, kept = _select(0, weights, levels, n, threshold, 0, dev)
         out = (torch.empty((kept, 3), dtype=torch.float32, device=dev), torch.empty(kept, dtype=torch.int32, device=dev),
                torch.empty(kept, dtype=torch.float32, device=dev), torch.empty(kept, dtype=torch.float32, device=dev))
         if kept:
             _cabi.check(_cabi.lib().inpc_leaf_prune_fill(_ptr(centers), _ptr(levels), _ptr(weights), _ptr(scores), n,
                                                          float(threshold), _ptr(ws), *[_ptr(o) for o in out], _stream()))
-            ws.record_stream(torch.cuda.current_stream())
     return out
 
 
@@ -135,7 +134,7 @@ def subdivide(leaf_centers, leaf_levels, leaf_weights, leaf_subdivision_scores, 
     then leaves the octree as it is)."""
     centers, levels, weights, scores, n = _leaf_arrays(leaf_centers, leaf_levels, leaf_weights, leaf_subdivision_scores)
     dev = weights.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws, split = _select(1, scores, levels, n, threshold, max_level, dev)
         total = n + 7 * split
         if total > max_leaves:
@@ -146,5 +145,4 @@ def subdivide(leaf_centers, leaf_levels, leaf_weights, leaf_subdivision_scores, 
             _cabi.check(_cabi.lib().inpc_leaf_subdivide_fill(_ptr(centers), _ptr(levels), _ptr(weights), _ptr(scores), n,
                                                              float(threshold), int(max_level), float(initial_size), split,
                                                              _ptr(ws), *[_ptr(o) for o in out], _stream()))
-            ws.record_stream(torch.cuda.current_stream())
     return out

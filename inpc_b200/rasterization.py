@@ -7,6 +7,7 @@ is a kernel of the shared library.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import warnings
 from enum import Enum
@@ -62,12 +63,23 @@ def _cuda_f16(t: torch.Tensor, name: str) -> torch.Tensor:
     return t.contiguous()
 
 
-def _ptr(t: torch.Tensor | None) -> C.c_void_p:
-    return C.c_void_p(0 if t is None or t.numel() == 0 else t.data_ptr())
+def _ptr(t: torch.Tensor | None) -> int:
+    """Device address for a `void*` argument; an empty tensor has none."""
+    return 0 if t is None or t.numel() == 0 else t.data_ptr()
 
 
-def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """Handle of torch's current stream on the current device.  (torch.cuda.current_stream() builds a Stream object around
+    the same handle: 3.2 us against 0.2 us, ten times per training step.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """Makes `device` current; nothing to do where it already is (1.4 us less per call)."""
+    return _SAME_DEVICE if device.index == torch._C._cuda_getDevice() else torch.cuda.device(device)
 
 
 class _ViewArg:
@@ -148,7 +160,7 @@ def forward_with_state(positions: torch.Tensor, features: torch.Tensor, opacitie
         raise ValueError(f"opacities must hold N={n} values, got {tuple(opacities.shape)}")
     dev = positions.device
     s = rasterizer_settings
-    with torch.cuda.device(dev):
+    with _on(dev):
         view = _ViewArg(s, dev)
         image = torch.empty((4, s.height, s.width), dtype=torch.float32, device=dev)
         alpha = torch.empty((1, s.height, s.width), dtype=torch.float32, device=dev)
@@ -188,7 +200,7 @@ class _Rasterize(torch.autograd.Function):
         # set_materialize_grads(False): an unused output arrives as None
         grad_image = torch.zeros_like(image) if grad_image is None else _cuda_f32(grad_image, "grad_image")
         grad_alpha = torch.zeros_like(alpha) if grad_alpha is None else _cuda_f32(grad_alpha, "grad_alpha")
-        with torch.cuda.device(dev):
+        with _on(dev):
             view = _ViewArg(s, dev)
             grad_features_view = torch.empty((n, 33), dtype=torch.float32, device=dev)   # per-point gradient slots
             grad_features = torch.empty((n, 36), dtype=torch.float16, device=dev)
@@ -224,7 +236,7 @@ class _RasterizeRows(torch.autograd.Function):
         n, channels = features.shape
         dev = positions.device
         s = rasterizer_settings
-        with torch.cuda.device(dev):
+        with _on(dev):
             view = _ViewArg(s, dev)
             image = torch.empty((channels, s.height, s.width), dtype=torch.float32, device=dev)
             alpha = torch.empty((1, s.height, s.width), dtype=torch.float32, device=dev)
@@ -250,7 +262,7 @@ class _RasterizeRows(torch.autograd.Function):
         dev = features.device
         grad_image = torch.zeros_like(image) if grad_image is None else _cuda_f32(grad_image, "grad_image")
         grad_alpha = torch.zeros_like(alpha) if grad_alpha is None else _cuda_f32(grad_alpha, "grad_alpha")
-        with torch.cuda.device(dev):
+        with _on(dev):
             view = _ViewArg(s, dev)
             grad_features = torch.empty_like(features)
             grad_opacities = torch.empty((features.shape[0], 1), dtype=torch.float32, device=dev)
@@ -310,7 +322,7 @@ class INPCRasterizer(torch.nn.Module):
         if features_raw.shape != (n, 37):
             raise ValueError(f"features_raw must be (N,37), got {tuple(features_raw.shape)}")
         dev = positions.device
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(s, dev)
             image = torch.empty((4, s.height, s.width), dtype=torch.float32, device=dev)
             depth = torch.empty((1, s.height, s.width), dtype=torch.float32, device=dev)
@@ -320,10 +332,6 @@ class INPCRasterizer(torch.nn.Module):
                 s.mode.value, self.tile_size, C.byref(varg.c), n, _ptr(positions), _ptr(features_raw),
                 float(sigma_world_scale * self.extract_base_sigma_world(view.camera)), float(sigma_cutoff),
                 _ptr(image), _ptr(depth), _ptr(alpha), blobs.cb_point, blobs.cb_instance, None, _stream()), blobs)
-            # the blobs must outlive the kernels already enqueued on this stream
-            for b in (blobs.point, blobs.instance):
-                if b is not None:
-                    b.record_stream(torch.cuda.current_stream())
         return image, depth, alpha
 
     @torch.no_grad()
@@ -342,7 +350,7 @@ class INPCRasterizer(torch.nn.Module):
             if f.shape != (p.shape[0], 37):
                 raise ValueError(f"features_raw must be (N,37), got {tuple(f.shape)}")
         dev = sets[0][0].device
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(s, dev)
             images = torch.empty((k, 4, s.height, s.width), dtype=torch.float32, device=dev)
             depths = torch.empty((k, 1, s.height, s.width), dtype=torch.float32, device=dev)
@@ -353,9 +361,6 @@ class INPCRasterizer(torch.nn.Module):
             blobs = _Blobs(dev)
             _check(_cabi.lib().inpc_render_multi(self.tile_size, C.byref(varg.c), k, n_points, pos_ptrs, feat_ptrs, _ptr(images),
                                                  _ptr(depths), _ptr(alphas), blobs.cb_point, blobs.cb_instance, None, _stream()), blobs)
-            for b in (blobs.point, blobs.instance):
-                if b is not None:
-                    b.record_stream(torch.cuda.current_stream())
         return images, depths, alphas
 
     @torch.no_grad()
@@ -378,7 +383,7 @@ class INPCRasterizer(torch.nn.Module):
             if scales.numel() != n:
                 raise ValueError(f"scales must hold N={n} values")
         dev = positions.device
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(s, dev)
             image = torch.empty((4, s.height, s.width), dtype=torch.float32, device=dev)
             depth = torch.empty((1, s.height, s.width), dtype=torch.float32, device=dev)
@@ -389,9 +394,6 @@ class INPCRasterizer(torch.nn.Module):
                 _ptr(scales), float(sigma_world_scale * self.extract_base_sigma_world(view.camera)),
                 float(sigma_cutoff), _ptr(image), _ptr(depth), _ptr(alpha), blobs.cb_point, blobs.cb_instance, None,
                 _stream()), blobs)
-            for b in (blobs.point, blobs.instance):
-                if b is not None:
-                    b.record_stream(torch.cuda.current_stream())
         return image, depth, alpha
 
 
@@ -408,7 +410,7 @@ class INPCRasterizer(torch.nn.Module):
         positions, features, opacities = _check_rows(positions, features, opacities)
         n, channels = features.shape
         dev = positions.device
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(s, dev)
             image = torch.empty((channels, s.height, s.width), dtype=torch.float32, device=dev)
             depth = torch.empty((1, s.height, s.width), dtype=torch.float32, device=dev)
@@ -417,9 +419,6 @@ class INPCRasterizer(torch.nn.Module):
             _check(_cabi.lib().inpc_render_rows(
                 self.tile_size, C.byref(varg.c), n, _ptr(positions), _ptr(features), int(channels), _ptr(opacities),
                 _ptr(image), _ptr(depth), _ptr(alpha), blobs.cb_point, blobs.cb_instance, None, _stream()), blobs)
-            for b in (blobs.point, blobs.instance):
-                if b is not None:
-                    b.record_stream(torch.cuda.current_stream())
         return image, depth, alpha
 
 
@@ -445,7 +444,7 @@ def debug_arrays(ctx_or_state, view_settings: RasterizerSettings, point_blob: to
     }
     order = ["sorted_points", "sorted_depth_keys", "inst_point", "ranges", "n_touched", "screen", "depth",
              "feat_view", "bounds"]
-    with torch.cuda.device(dev):
+    with _on(dev):
         varg = _ViewArg(s, dev)
         for which, name in enumerate(order):
             if out[name].numel() == 0:

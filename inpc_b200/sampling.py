@@ -14,7 +14,7 @@ import warnings
 import torch
 
 from . import _cabi
-from .rasterization import _cuda_f32, _ptr, _stream
+from .rasterization import _cuda_f32, _on, _ptr, _stream
 
 
 def _check_view(view) -> None:
@@ -56,7 +56,7 @@ def compute_viewpoint_weights(centers: torch.Tensor, levels: torch.Tensor, weigh
     _check_view(view)
     centers, levels, weights, n = _leaf_args(centers, levels, weights)
     dev = centers.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         varg = _ViewArg(view, dev)
         out = torch.empty((n,), dtype=torch.float32, device=dev)
         _cabi.check(_cabi.lib().inpc_compute_viewpoint_weights(C.byref(varg.c), n, _ptr(centers), _ptr(levels),
@@ -114,12 +114,11 @@ class ProbabilityFieldSampler(torch.nn.Module):
             raise TypeError("weights must be a CUDA float32 tensor")
         weights = weights.contiguous()
         n, dev = weights.numel(), weights.device
-        with torch.cuda.device(dev):
+        with _on(dev):
             counts = torch.empty(n, dtype=torch.int32, device=dev)
             ws = self._workspace(n, dev)
             _cabi.check(_cabi.lib().inpc_draw_leaf_counts(self._handle, n, _ptr(weights), int(n_samples), _ptr(counts), _ptr(ws),
                                                           _stream()))
-            ws.record_stream(torch.cuda.current_stream())
         return counts
 
     def generate_training_samples(self, centers: torch.Tensor, levels: torch.Tensor, weights: torch.Tensor, view,
@@ -131,7 +130,7 @@ class ProbabilityFieldSampler(torch.nn.Module):
             # the previous call's flag, read without waiting for anything: by now it is normally final
             warnings.warn("the previous generate_training_samples call left sample slots unfilled (rejection attempts "
                           "exhausted): they hold positions outside the view frustum")
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(view, dev)
             positions = torch.empty((n_samples, 3), dtype=torch.float32, device=dev)
             indices = torch.empty((n_samples,), dtype=torch.int64, device=dev)
@@ -139,7 +138,6 @@ class ProbabilityFieldSampler(torch.nn.Module):
             _cabi.check(_cabi.lib().inpc_generate_training_samples(
                 self._handle, C.byref(varg.c), n, _ptr(centers), _ptr(levels), _ptr(weights), float(initial_size),
                 int(n_samples), _ptr(positions), _ptr(indices), _ptr(ws), _stream()))
-            ws.record_stream(torch.cuda.current_stream())
         return positions, indices
 
     def generate_samples(self, centers: torch.Tensor, levels: torch.Tensor, weights: torch.Tensor, view,
@@ -147,7 +145,7 @@ class ProbabilityFieldSampler(torch.nn.Module):
         _check_view(view)
         centers, levels, weights, n = _leaf_args(centers, levels, weights)
         dev = centers.device
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(view, dev)
             positions = torch.empty((n_samples, 3), dtype=torch.float32, device=dev)
             ws = self._workspace(n, dev)
@@ -155,7 +153,6 @@ class ProbabilityFieldSampler(torch.nn.Module):
             _cabi.check(_cabi.lib().inpc_generate_samples(
                 self._handle, C.byref(varg.c), n, _ptr(centers), _ptr(levels), _ptr(weights), float(initial_size),
                 int(n_samples), _ptr(positions), C.byref(written), _ptr(ws), _stream()))
-            ws.record_stream(torch.cuda.current_stream())
         if written.value == 0 and n_samples > 0:
             return torch.empty((0, 3), dtype=torch.float32, device=dev)
         return positions
@@ -165,7 +162,7 @@ class ProbabilityFieldSampler(torch.nn.Module):
         _check_view(view)
         centers, levels, weights, n = _leaf_args(centers, levels, weights)
         dev = centers.device
-        with torch.cuda.device(dev):
+        with _on(dev):
             varg = _ViewArg(view, dev)
             ws = self._workspace(n, dev)
             created = C.c_int64(0)
@@ -178,7 +175,6 @@ class ProbabilityFieldSampler(torch.nn.Module):
             _cabi.check(_cabi.lib().inpc_generate_expected_samples_fill(
                 self._handle, n, _ptr(centers), _ptr(levels), float(initial_size), created.value, int(n_multi),
                 _ptr(positions), _ptr(ws), _stream()))
-            ws.record_stream(torch.cuda.current_stream())
         return positions
 
 
@@ -193,12 +189,11 @@ def halton_samples(counts: torch.Tensor, centers: torch.Tensor, levels: torch.Te
     counts = counts.contiguous()
     total = int(counts.sum().item())
     dev = centers.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         positions = torch.empty((total, 3), dtype=torch.float32, device=dev)
         ws = torch.empty(int(_cabi.lib().inpc_sampler_workspace_bytes(n)), dtype=torch.uint8, device=dev)
         _cabi.check(_cabi.lib().inpc_halton_samples(_ptr(counts), n, _ptr(centers), _ptr(levels), float(initial_size), total,
                                                     _ptr(positions), _ptr(ws), _stream()))
-        ws.record_stream(torch.cuda.current_stream())
     return positions
 
 
@@ -216,11 +211,10 @@ def morton_order(positions: torch.Tensor) -> torch.Tensor:
     extent = extent * (1.0 + 1e-6) if extent > 0 else 1.0
     box_lo = (C.c_float * 3)(*[float(v) for v in lo.tolist()])
     dev = positions.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty_like(positions)
         ws = torch.empty(int(_cabi.lib().inpc_morton_workspace_bytes(n)), dtype=torch.uint8, device=dev)
         _cabi.check(_cabi.lib().inpc_morton_order(_ptr(positions), n, box_lo, extent, _ptr(out), _ptr(ws), _stream()))
-        ws.record_stream(torch.cuda.current_stream())
     return out
 
 
@@ -246,12 +240,11 @@ def build_cdf(weights: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     weights = _cuda_f32(weights, "weights")
     n = weights.numel()
     dev = weights.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         cdf = torch.empty_like(weights)
         total = torch.empty((1,), dtype=torch.float32, device=dev)
         ws = torch.empty(int(_cabi.lib().inpc_sampler_workspace_bytes(n)), dtype=torch.uint8, device=dev)
         _cabi.check(_cabi.lib().inpc_build_cdf(_ptr(weights), n, _ptr(cdf), _ptr(total), _ptr(ws), _stream()))
-        ws.record_stream(torch.cuda.current_stream())
     return cdf, total
 
 
@@ -259,7 +252,7 @@ def draw_leaves(cdf: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
     """out[i] = min(lower_bound(cdf, u[i]), L-1) as int64."""
     cdf, u = _cuda_f32(cdf, "cdf"), _cuda_f32(u, "u")
     dev = cdf.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         out = torch.empty((u.numel(),), dtype=torch.int64, device=dev)
         _cabi.check(_cabi.lib().inpc_draw_leaves(_ptr(cdf), cdf.numel(), _ptr(u), u.numel(), _ptr(out), _stream()))
     return out
