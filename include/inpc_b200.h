@@ -263,6 +263,11 @@ int inpc_compute_viewpoint_weights(const inpc_view* view, int64_t n_cells, const
                                    const int32_t* levels, const float* weights, float initial_size,
                                    float* out, void* stream);
 
+/* out[l] = largest of the n_views (>= 1) viewpoint weights of leaf l: the loop over the training views of
+ * Modules/ProbabilityField.py:121-128 in one launch per 32 views.  `views` is an array on the host. */
+int inpc_max_viewpoint_weights(const inpc_view* views, int n_views, int64_t n_cells, const float* centers, const int32_t* levels,
+                               const float* weights, float initial_size, float* out, void* stream);
+
 /* Opaque sampler: a counter-based Philox4x32-10 stream keyed by `seed`; each generate_* call consumes
  * one value of a 64-bit call counter, which is all the state there is.  Replaces
  * struct ProbabilityFieldSampler and its host-side pcg32 (sampling/include/sampling_api.h:26-82). */
@@ -300,7 +305,7 @@ int inpc_generate_samples(inpc_sampler* s, const inpc_view* view, int64_t n_cell
 
 /* Expected-count samples in two steps so the caller can size the output.  _count reads one integer
  * back: *n_created = sum over visible leaves of max(1, round(w/sum*n_samples)), 0 if sum <= 0.
- * _fill writes n_created*n_multi positions.  Replaces compute_sample_distribution +
+ * _fill writes n_created*n_multi positions of the leaves given to _count (it reads them from the workspace).  Replaces compute_sample_distribution +
  * create_expected_samples (sampling/include/sampling.h:68-83). */
 int inpc_generate_expected_samples_count(inpc_sampler* s, const inpc_view* view, int64_t n_cells,
                                          const float* centers, const int32_t* levels,
@@ -419,7 +424,9 @@ int inpc_multisample_resolve(float* acc_image, float* acc_depth, float* acc_alph
  *                          ProbabilityField.py:131-140 (the Halton elements are formed in double
  *                          precision and stored as float32 as there).
  *   inpc_morton_order      out = positions sorted by a 30-bit Morton code (10 bits per axis) inside
- *                          the cube [box_lo, box_lo + box_extent]^3 (box_lo: 3 HOST floats); stable.
+ *                          the cube [box_lo, box_lo + box_extent]^3 (box_lo: 3 HOST floats), or
+ *                          inside the cloud's own bounding cube (box_lo NULL, found on the device:
+ *                          no synchronisation); stable.
  *                          Stands in for NeRFICG's CudaUtils.MortonEncoding.morton_encode + argsort
  *                          (ProbabilityField.py:141-143), which is not part of the reference tree:
  *                          the code width and the box are this library's choice.

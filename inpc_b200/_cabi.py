@@ -64,6 +64,7 @@ PROTOTYPES = {
     "inpc_call_status": (_I, [C.c_longlong, C.POINTER(C.c_uint)]),
     "inpc_sampler_exhausted": (_I, [_P]),
     "inpc_compute_viewpoint_weights": (_I, [_VP, _L, _P, _P, _P, _F, _P, _P]),
+    "inpc_max_viewpoint_weights": (_I, [_VP, _I, _L, _P, _P, _P, _F, _P, _P]),
     "inpc_sampler_create": (_P, [_L]),
     "inpc_sampler_destroy": (None, [_P]),
     "inpc_sampler_get_counter": (C.c_uint64, [_P]),

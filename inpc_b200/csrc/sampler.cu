@@ -44,17 +44,9 @@ __device__ __forceinline__ bool in_frustum(const Rows& m, const ViewParams& v, f
     return (z >= v.near_plane) & (z <= v.far_plane) & (x >= 0.0f) & (x < (float)v.width) & (y >= 0.0f) & (y < (float)v.height);
 }
 
-__global__ void __launch_bounds__(kThreads) viewpoint_weights_kernel(ViewParams v, int64_t n_cells,
-                                                                     const float* __restrict__ centers,
-                                                                     const int* __restrict__ levels,
-                                                                     const float* __restrict__ weights,
-                                                                     float initial_size, float* __restrict__ out,
-                                                                     float4* __restrict__ leaf_pack) {
-    const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (l >= n_cells) return;
+// weight of a leaf in a view: 0 outside the frustum
+__device__ __forceinline__ float viewpoint_weight(const ViewParams& v, float cx, float cy, float cz, int level, float weight, float initial_size) {
     const Rows m = load_rows(v.w2c);
-    const float cx = __ldg(centers + 3 * l), cy = __ldg(centers + 3 * l + 1), cz = __ldg(centers + 3 * l + 2);
-    const int level = __ldg(levels + l);
     float z;
     bool valid = in_frustum(m, v, cx, cy, cz, &z);
     if (!valid) {
@@ -65,16 +57,46 @@ __global__ void __launch_bounds__(kThreads) viewpoint_weights_kernel(ViewParams 
             valid |= in_frustum(m, v, fmaf(half_size, ox, cx), fmaf(half_size, oy, cy), fmaf(half_size, oz, cz), nullptr);
         }
     }
-    float w = 0.0f;
-    if (valid) {
-        const float depth_scale = fmaxf(fabsf(z - v.near_plane) / v.far_plane, kEps);
-        // 2^(level/2), exact: the reference's exp2f(level * 0.5f) agrees to within the 2 ulp of exp2f
-        const float size_scale = scalbnf((level & 1) ? 1.41421356237309504880f : 1.0f, level >> 1);
-        w = 1.0f / (depth_scale * size_scale) * __ldg(weights + l);
-    }
-    out[l] = w;
+    if (!valid) return 0.0f;
+    const float depth_scale = fmaxf(fabsf(z - v.near_plane) / v.far_plane, kEps);
+    // 2^(level/2), exact: the reference's exp2f(level * 0.5f) agrees to within the 2 ulp of exp2f
+    const float size_scale = scalbnf((level & 1) ? 1.41421356237309504880f : 1.0f, level >> 1);
+    return 1.0f / (depth_scale * size_scale) * weight;
+}
+
+__global__ void __launch_bounds__(kThreads) viewpoint_weights_kernel(ViewParams v, int64_t n_cells,
+                                                                     const float* __restrict__ centers,
+                                                                     const int* __restrict__ levels,
+                                                                     const float* __restrict__ weights,
+                                                                     float initial_size, float* __restrict__ out,
+                                                                     float4* __restrict__ leaf_pack) {
+    const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (l >= n_cells) return;
+    const float cx = __ldg(centers + 3 * l), cy = __ldg(centers + 3 * l + 1), cz = __ldg(centers + 3 * l + 2);
+    const int level = __ldg(levels + l);
+    out[l] = viewpoint_weight(v, cx, cy, cz, level, __ldg(weights + l), initial_size);
     // centre and edge length in one 16-byte record: a draw then needs one load per leaf instead of four
     if (leaf_pack) leaf_pack[l] = make_float4(cx, cy, cz, 1.0f / scalbnf(1.0f, level) * initial_size);
+}
+
+// Largest weight of every leaf over up to kViewsPerPass views (and over *out, when earlier passes left something there).
+// The leaf is read once for all views; one launch per view and a maximum after it were 32 launches for 16 views.
+constexpr int kViewsPerPass = 32;
+struct ViewSet {
+    int count;
+    ViewParams v[kViewsPerPass];
+};
+__global__ void __launch_bounds__(kThreads) max_viewpoint_weights_kernel(const __grid_constant__ ViewSet views, int64_t n_cells, const float* __restrict__ centers,
+                                                                         const int* __restrict__ levels, const float* __restrict__ weights,
+                                                                         float initial_size, bool first, float* __restrict__ out) {
+    const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (l >= n_cells) return;
+    const float cx = __ldg(centers + 3 * l), cy = __ldg(centers + 3 * l + 1), cz = __ldg(centers + 3 * l + 2);
+    const int level = __ldg(levels + l);
+    const float weight = __ldg(weights + l);
+    float best = first ? 0.0f : out[l];
+    for (int j = 0; j < views.count; ++j) best = fmaxf(best, viewpoint_weight(views.v[j], cx, cy, cz, level, weight, initial_size));
+    out[l] = best;
 }
 
 // ---- CDF: src/sampling.cu:97-125 (Sum, multiply by 1/sum, InclusiveSum) -------------------------
@@ -240,95 +262,116 @@ __device__ __forceinline__ unsigned lower_bound_clamped(const float* __restrict_
     return min(first, n - 1);
 }
 
-// Guide table: guide[b] = lower_bound(cdf, b / 2^k) for b = 0 .. 2^k.  The CDF is monotone (integer
-// prefix sums), so the look-up for a uniform in bucket b only has to search [guide[b], guide[b+1]):
-// about L / 2^k entries instead of log2(L) dependent loads, with bit-identical results.
-__global__ void __launch_bounds__(kThreads) guide_table_kernel(const float* __restrict__ cdf, unsigned n_cells, int k,
-                                                               unsigned* __restrict__ guide) {
-    const unsigned b = blockIdx.x * kThreads + threadIdx.x;
-    if (b > (1u << k)) return;
+// Guide table: one 16-byte record per bucket b of [0, 1), b = 0 .. 2^k - 1: {lower_bound(cdf, b / 2^k), the two CDF values from
+// there on, lower_bound(cdf, (b + 1) / 2^k)}.  The CDF is monotone (integer prefix sums), so the look-up for a uniform in
+// bucket b only has to search between the two bounds, with bit-identical results.  A draw is bound by the number of 32-byte
+// sectors it gathers from L2 (all tables are larger than L1): the record settles the draws whose bucket holds at most two
+// CDF steps, nine in ten with as many buckets as leaves, in one sector where separate guide and CDF arrays took three.
+constexpr int kGuidePerBlock = kThreads - 1;   // the last thread of a block only finds the end of the last bucket
+__global__ void __launch_bounds__(kThreads) guide_table_kernel(const float* __restrict__ cdf, unsigned n_cells, int k, uint4* __restrict__ guide) {
+    __shared__ unsigned s_first[kThreads];
+    const unsigned b = blockIdx.x * kGuidePerBlock + threadIdx.x, n_buckets = 1u << k;
+    unsigned first = 0, count = b <= n_buckets ? n_cells : 0u;
     // bucket edge as a float: (b << (23 - k)) * 2^-23, exact
     const float edge = (float)(b << (23 - k)) * 1.1920928955078125e-07f;
-    unsigned first = 0, count = n_cells;
     while (count > 0) {
         const unsigned step = count >> 1;
         if (__ldg(cdf + first + step) < edge) { first += step + 1; count -= step + 1; }
         else count = step;
     }
-    guide[b] = first;
+    s_first[threadIdx.x] = first;
+    __syncthreads();
+    if (threadIdx.x == kGuidePerBlock || b >= n_buckets) return;
+    const float c0 = first < n_cells ? __ldg(cdf + first) : 2.0f, c1 = first + 1u < n_cells ? __ldg(cdf + first + 1u) : 2.0f;
+    guide[b] = make_uint4(first, __float_as_uint(c0), __float_as_uint(c1), s_first[threadIdx.x + 1]);
 }
 
 // r: the raw 32 random bits the uniform is made of (u = (r >> 9) * 2^-23)
-__device__ __forceinline__ unsigned guided_lower_bound(const float* __restrict__ cdf, const unsigned* __restrict__ guide, int k,
+__device__ __forceinline__ unsigned guided_lower_bound(const float* __restrict__ cdf, const uint4* __restrict__ guide, int k,
                                                        unsigned r, float u, unsigned n) {
-    const unsigned b = (r >> 9) >> (23 - k);
-    const uint2 g = make_uint2(__ldg(guide + b), __ldg(guide + b + 1));
-    unsigned first = g.x, count = g.y - g.x;
-    while (count > 0) {
-        const unsigned step = count >> 1;
-        if (__ldg(cdf + first + step) < u) { first += step + 1; count -= step + 1; }
-        else count = step;
+    const uint4 g = __ldg(guide + ((r >> 9) >> (23 - k)));
+    unsigned first = g.x;
+    if (__uint_as_float(g.y) < u) {
+        first += 1u;
+        if (__uint_as_float(g.z) < u) {
+            first += 1u;
+            unsigned count = g.w > first ? g.w - first : 0u;
+            while (count > 0) {
+                const unsigned step = count >> 1;
+                if (__ldg(cdf + first + step) < u) { first += step + 1; count -= step + 1; }
+                else count = step;
+            }
+        }
     }
     return min(first, n - 1);
 }
 
-__device__ __forceinline__ float leaf_scale(int level, float initial_size) {
-    return 1.0f / scalbnf(1.0f, level) * initial_size;
+// Positions of the kThreads consecutive samples of a block, first sample `first`, leave as 16-byte vectors through shared
+// memory (three 4-byte stores with a stride of 12 bytes write every sector three times into L2).
+__device__ __forceinline__ void store_positions(float* s_pos, float x, float y, float z, int64_t first, int64_t n, float* __restrict__ positions) {
+    s_pos[3 * threadIdx.x] = x; s_pos[3 * threadIdx.x + 1] = y; s_pos[3 * threadIdx.x + 2] = z;
+    __syncthreads();
+    const int floats = 3 * (int)min((int64_t)kThreads, n - first);
+    float* dst = positions + 3 * first;
+    if (floats == 3 * kThreads && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        if (threadIdx.x < 3 * kThreads / 4) reinterpret_cast<float4*>(dst)[threadIdx.x] = reinterpret_cast<const float4*>(s_pos)[threadIdx.x];
+    } else {
+        for (int k = threadIdx.x; k < floats; k += kThreads) dst[k] = s_pos[k];
+    }
 }
 
 // ---- training samples: same acceptance test as src/sampling_kernels.cu:98-113 -------------------
 __global__ void __launch_bounds__(kThreads) training_samples_kernel(
     ViewParams v, unsigned long long seed, unsigned long long call, const float* __restrict__ cdf,
-    const unsigned* __restrict__ guide, int guide_bits, const float* __restrict__ sum_ptr, unsigned n_cells,
+    const uint4* __restrict__ guide, int guide_bits, const float* __restrict__ sum_ptr, unsigned n_cells,
     const float4* __restrict__ leaf_pack, int64_t n_samples, float* __restrict__ positions, long long* __restrict__ indices,
     volatile unsigned* status) {
-    const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (s >= n_samples) return;
+    __shared__ __align__(16) float s_pos[3 * kThreads];
+    const int64_t block_first = (int64_t)blockIdx.x * kThreads;
+    const int64_t s = block_first + threadIdx.x;
+    const bool mine = s < n_samples;
+    float x = 0.0f, y = 0.0f, z = 0.0f;
     if (!(__ldg(sum_ptr) > 0.0f)) {
         // src/sampling.cu:107-111: zero positions, indices of -1
-        positions[3 * s] = 0.0f; positions[3 * s + 1] = 0.0f; positions[3 * s + 2] = 0.0f;
-        indices[s] = -1;
-        return;
+        if (mine) indices[s] = -1;
+    } else if (mine) {
+        const Rows m = load_rows(v.w2c);
+        unsigned leaf = 0;
+        bool ok = false;
+        for (unsigned a = 0; a < (unsigned)kMaxAttempts && !ok; ++a) {
+            const Draw d = philox_draw(seed, call, (unsigned)s, a);
+            leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
+            const float4 lp = __ldg(leaf_pack + leaf);
+            x = fmaf(d.jx - 0.5f, lp.w, lp.x);
+            y = fmaf(d.jy - 0.5f, lp.w, lp.y);
+            z = fmaf(d.jz - 0.5f, lp.w, lp.z);
+            const float vz = affine(m.r2, x, y, z);
+            if (vz < v.near_plane || vz > v.far_plane) continue;
+            const float inv_z = 1.0f / (vz + kEps);
+            const float sx = fmaf(affine(m.r0, x, y, z) * inv_z, v.fx, v.cx);
+            if (sx < 0.0f || sx >= (float)v.width) continue;
+            const float sy = fmaf(affine(m.r1, x, y, z) * inv_z, v.fy, v.cy);
+            if (sy < 0.0f || sy >= (float)v.height) continue;
+            ok = true;
+        }
+        if (!ok) status[STATUS_SAMPLER_EXHAUSTED] = 1u;
+        indices[s] = (long long)leaf;
     }
-    const Rows m = load_rows(v.w2c);
-    unsigned leaf = 0;
-    float x = 0.0f, y = 0.0f, z = 0.0f;
-    bool ok = false;
-    for (unsigned a = 0; a < (unsigned)kMaxAttempts && !ok; ++a) {
-        const Draw d = philox_draw(seed, call, (unsigned)s, a);
-        leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
-        const float4 lp = __ldg(leaf_pack + leaf);
-        x = fmaf(d.jx - 0.5f, lp.w, lp.x);
-        y = fmaf(d.jy - 0.5f, lp.w, lp.y);
-        z = fmaf(d.jz - 0.5f, lp.w, lp.z);
-        const float vz = affine(m.r2, x, y, z);
-        if (vz < v.near_plane || vz > v.far_plane) continue;
-        const float inv_z = 1.0f / (vz + kEps);
-        const float sx = fmaf(affine(m.r0, x, y, z) * inv_z, v.fx, v.cx);
-        if (sx < 0.0f || sx >= (float)v.width) continue;
-        const float sy = fmaf(affine(m.r1, x, y, z) * inv_z, v.fy, v.cy);
-        if (sy < 0.0f || sy >= (float)v.height) continue;
-        ok = true;
-    }
-    if (!ok) status[STATUS_SAMPLER_EXHAUSTED] = 1u;
-    positions[3 * s] = x; positions[3 * s + 1] = y; positions[3 * s + 2] = z;
-    indices[s] = (long long)leaf;
+    store_positions(s_pos, x, y, z, block_first, n_samples, positions);
 }
 
 // ---- unconditional samples: src/sampling_kernels.cu:128-150 with the Philox stream ----------------
 __global__ void __launch_bounds__(kThreads) samples_kernel(unsigned long long seed, unsigned long long call,
-                                                           const float* __restrict__ cdf, const unsigned* __restrict__ guide,
+                                                           const float* __restrict__ cdf, const uint4* __restrict__ guide,
                                                            int guide_bits, unsigned n_cells,
                                                            const float4* __restrict__ leaf_pack, int64_t n_samples,
                                                            float* __restrict__ positions) {
-    const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (s >= n_samples) return;
-    const Draw d = philox_draw(seed, call, (unsigned)s, 0u);
+    __shared__ __align__(16) float s_pos[3 * kThreads];
+    const int64_t block_first = (int64_t)blockIdx.x * kThreads;
+    const Draw d = philox_draw(seed, call, (unsigned)(block_first + threadIdx.x), 0u);
     const unsigned leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
     const float4 lp = __ldg(leaf_pack + leaf);
-    positions[3 * s] = fmaf(d.jx - 0.5f, lp.w, lp.x);
-    positions[3 * s + 1] = fmaf(d.jy - 0.5f, lp.w, lp.y);
-    positions[3 * s + 2] = fmaf(d.jz - 0.5f, lp.w, lp.z);
+    store_positions(s_pos, fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), block_first, n_samples, positions);
 }
 
 __global__ void __launch_bounds__(kThreads) draw_leaves_kernel(const float* __restrict__ cdf, unsigned n_cells,
@@ -400,36 +443,97 @@ __global__ void __launch_bounds__(kThreads) count_offsets_kernel(const unsigned*
     if (i < n) offsets[i] = chunk_base[blockIdx.x] + ex + c;
 }
 
-// slot i jitters inside leaf upper_bound(offsets, i % n_created): the load-balanced form of the
-// reference's per-leaf fill loop + gather
+// Slots whose leaves are given by inclusive offsets: slot r lies in leaf upper_bound(offsets, r).  A block takes
+// kRunSlots consecutive slots, so its leaves are consecutive too: one warp finds the first and last of them (a 32-way
+// search, four dependent trips to L2 for 2^20 leaves), their offsets are copied to shared memory and every slot searches
+// those few.  (A search of all leaves per slot was 18 dependent gathers: 561 us for 2^25 slots over 2^18 leaves.)
+constexpr int kRunPerThread = 8;
+constexpr int kRunSlots = kThreads * kRunPerThread;
+constexpr unsigned kRunLeaves = 2048;   // offsets kept in shared memory; a run over more leaves (empty ones between) reads L2
+
+struct LeafRun {
+    unsigned offsets[kRunLeaves];
+    unsigned first, count;   // leaves first .. first + count - 1 hold the block's slots
+};
+
+// first index with offsets[idx] > r, by all lanes of one warp; n if there is none
+__device__ __forceinline__ unsigned warp_upper_bound(const unsigned* __restrict__ offsets, unsigned n, unsigned r) {
+    unsigned lo = 0, hi = n;   // the answer lies in [lo, hi]
+    while (hi - lo > 0) {
+        const unsigned step = (hi - lo + 31u) / 32u;
+        const unsigned probe = lo + lane_id() * step + step - 1u;   // last element of this lane's piece
+        const bool above = probe >= hi || __ldg(offsets + probe) > r;
+        const unsigned b = __ballot_sync(0xffffffffu, above);
+        if (b == 0u) return hi;
+        lo += (unsigned)(__ffs(b) - 1) * step;
+        hi = min(hi, lo + step - 1u);
+    }
+    return lo;
+}
+
+// Finds the run of leaves that holds slots [r0, r1]; ends with a block barrier.
+__device__ __forceinline__ void find_leaf_run(LeafRun& run, const unsigned* __restrict__ offsets, unsigned n_cells, unsigned r0, unsigned r1) {
+    const unsigned warp = threadIdx.x >> 5;
+    if (warp < 2) {
+        const unsigned l = min(warp_upper_bound(offsets, n_cells, warp == 0 ? r0 : r1), n_cells - 1u);
+        if (lane_id() == 0) { if (warp == 0) run.first = l; else run.count = l; }
+    }
+    __syncthreads();
+    const unsigned first = run.first, count = run.count - first + 1u;
+    __syncthreads();
+    if (threadIdx.x == 0) run.count = count;
+    for (unsigned k = threadIdx.x; k < min(count, kRunLeaves); k += kThreads) run.offsets[k] = __ldg(offsets + first + k);
+    __syncthreads();
+}
+
+__device__ __forceinline__ unsigned leaf_of_slot(const LeafRun& run, const unsigned* __restrict__ offsets, unsigned r) {
+    const unsigned m = run.count;
+    unsigned first = 0, count = m;
+    if (m <= kRunLeaves) {
+        while (count > 0) {
+            const unsigned step = count >> 1;
+            if (run.offsets[first + step] <= r) { first += step + 1; count -= step + 1; }
+            else count = step;
+        }
+    } else {
+        while (count > 0) {
+            const unsigned step = count >> 1;
+            if (__ldg(offsets + run.first + first + step) <= r) { first += step + 1; count -= step + 1; }
+            else count = step;
+        }
+    }
+    return run.first + min(first, m - 1u);
+}
+
+// slot i jitters inside leaf upper_bound(offsets, i % n_created): the load-balanced form of the reference's per-leaf fill
+// loop + gather.  blockIdx.y counts the copies i / n_created, whose slots a run never leaves.
 __global__ void __launch_bounds__(kThreads) expected_samples_kernel(unsigned long long seed, unsigned long long call,
                                                                     const unsigned* __restrict__ offsets, unsigned n_cells,
-                                                                    const float* __restrict__ centers, const int* __restrict__ levels,
-                                                                    float initial_size, int64_t n_total, unsigned n_created,
-                                                                    float* __restrict__ positions) {
-    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n_total) return;
-    const unsigned r = (unsigned)(i % n_created);
-    // first leaf whose inclusive offset exceeds r
-    unsigned first = 0, count = n_cells;
-    while (count > 0) {
-        const unsigned step = count >> 1;
-        if (__ldg(offsets + first + step) <= r) { first += step + 1; count -= step + 1; }
-        else count = step;
+                                                                    const float4* __restrict__ leaf_pack, unsigned n_created,
+                                                                    unsigned n_copies, float* __restrict__ positions) {
+    __shared__ LeafRun run;
+    __shared__ __align__(16) float s_pos[3 * kThreads];
+    const unsigned r0 = blockIdx.x * (unsigned)kRunSlots;
+    const unsigned in_block = min((unsigned)kRunSlots, n_created - r0);
+    find_leaf_run(run, offsets, n_cells, r0, r0 + in_block - 1u);
+    for (unsigned copy = blockIdx.y; copy < n_copies; copy += gridDim.y) {
+        const int64_t copy_first = (int64_t)copy * n_created, copy_end = copy_first + n_created;
+        for (unsigned k0 = 0; k0 < in_block; k0 += kThreads) {
+            const unsigned r = min(r0 + k0 + threadIdx.x, n_created - 1u);
+            const float4 lp = __ldg(leaf_pack + leaf_of_slot(run, offsets, r));
+            const Draw d = philox_draw(seed, call, (unsigned)(copy_first + r), 0u);
+            store_positions(s_pos, fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), copy_first + r0 + k0,
+                            copy_end, positions);
+            __syncthreads();
+        }
     }
-    const unsigned leaf = min(first, n_cells - 1);
-    const Draw d = philox_draw(seed, call, (unsigned)i, 0u);
-    const float scale = leaf_scale(__ldg(levels + leaf), initial_size);
-    positions[3 * i] = fmaf(d.jx - 0.5f, scale, __ldg(centers + 3 * (int64_t)leaf));
-    positions[3 * i + 1] = fmaf(d.jy - 0.5f, scale, __ldg(centers + 3 * (int64_t)leaf + 1));
-    positions[3 * i + 2] = fmaf(d.jz - 0.5f, scale, __ldg(centers + 3 * (int64_t)leaf + 2));
 }
 
 // ---- global point cloud: Modules/ProbabilityField.py:121-144 + utils.py:36-64 -----------------------
 // counts[leaf] = number of the n multinomial draws that fell into the leaf (torch.multinomial +
 // bincount in the reference; here the library's own Philox stream, one draw per slot)
 __global__ void __launch_bounds__(kThreads) leaf_histogram_kernel(unsigned long long seed, unsigned long long call,
-                                                                  const float* __restrict__ cdf, const unsigned* __restrict__ guide,
+                                                                  const float* __restrict__ cdf, const uint4* __restrict__ guide,
                                                                   int guide_bits, unsigned n_cells, int64_t n_samples,
                                                                   unsigned* __restrict__ counts) {
     const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -438,17 +542,30 @@ __global__ void __launch_bounds__(kThreads) leaf_histogram_kernel(unsigned long 
     atomicAdd(counts + guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells), 1u);
 }
 
-// Element `index` (1-based) of the Halton sequence in `base`, with the reference's arithmetic
-// (utils.py:36-46): double precision, one rounding per product, sum and division; the value is then
-// stored as float32 (utils.py:52-55).
-__device__ __forceinline__ float halton_element(unsigned index, unsigned base) {
+// Element `index` (1-based) of the Halton sequence in base B, with the reference's arithmetic (utils.py:36-46): double
+// precision, one rounding per product, sum and division f = f / B; the value is then stored as float32 (utils.py:52-55).
+// The scale factors f do not depend on the index: they are divided out at compile time, with the same roundings.
+template <unsigned B>
+struct HaltonScale {
+    static constexpr int kDigits = B == 3u ? 21 : 14;   // digits of 2^32 - 1
+    double f[kDigits];
+    constexpr HaltonScale() : f() {
+        double v = 1.0;
+        for (int k = 0; k < kDigits; ++k) { v = v / (double)B; f[k] = v; }
+    }
+};
+template <unsigned B>
+__device__ __forceinline__ float halton_element(unsigned index) {
+    // in base 2 every term is a power of two and every sum exact: the value is the reversed index, rounded once
+    if (B == 2u) return __uint2float_rn(__brev(index)) * 2.3283064365386962890625e-10f;
+    constexpr HaltonScale<B> scale;
     double result = 0.0;
-    double f = __ddiv_rn(1.0, (double)base);
     unsigned i = index;
-    while (i > 0u) {
-        result = __dadd_rn(result, __dmul_rn(f, (double)(i % base)));
-        i /= base;
-        f = __ddiv_rn(f, (double)base);
+#pragma unroll
+    for (int k = 0; k < HaltonScale<B>::kDigits; ++k) {
+        if (i == 0u) break;
+        result = __dadd_rn(result, __dmul_rn(scale.f[k], (double)(i % B)));
+        i /= B;
     }
     return __double2float_rn(result);
 }
@@ -458,31 +575,31 @@ __device__ __forceinline__ float halton_element(unsigned index, unsigned base) {
 // puts it at its centre (ProbabilityField.py:131-140).
 __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned* __restrict__ counts, const unsigned* __restrict__ offsets,
                                                                   unsigned n_cells, const float* __restrict__ centers,
-                                                                  const int* __restrict__ levels, float initial_size, int64_t n_total,
+                                                                  const int* __restrict__ levels, float initial_size, unsigned n_total,
                                                                   float* __restrict__ positions) {
-    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n_total) return;
-    unsigned first = 0, count = n_cells;
-    while (count > 0) {
-        const unsigned step = count >> 1;
-        if (__ldg(offsets + first + step) <= (unsigned)i) { first += step + 1; count -= step + 1; }
-        else count = step;
+    __shared__ LeafRun run;
+    __shared__ __align__(16) float s_pos[3 * kThreads];
+    const unsigned r0 = blockIdx.x * (unsigned)kRunSlots;
+    const unsigned in_block = min((unsigned)kRunSlots, n_total - r0);
+    find_leaf_run(run, offsets, n_cells, r0, r0 + in_block - 1u);
+    for (unsigned k0 = 0; k0 < in_block; k0 += kThreads) {
+        const unsigned i = min(r0 + k0 + threadIdx.x, n_total - 1u);
+        const unsigned leaf = leaf_of_slot(run, offsets, i);
+        const unsigned c = __ldg(counts + leaf);
+        const unsigned h = i - (__ldg(offsets + leaf) - c);
+        float x = __ldg(centers + 3 * (int64_t)leaf), y = __ldg(centers + 3 * (int64_t)leaf + 1), z = __ldg(centers + 3 * (int64_t)leaf + 2);
+        if (c != 1u) {
+            // cell edge = initial_size / 2^level, exact in fp32 for the levels an octree has; every further
+            // operation rounds on its own like the torch expression  centre - cell/2 + halton * cell
+            const float cell = __fdiv_rn(initial_size, (float)(1u << __ldg(levels + leaf)));
+            const float half = __fmul_rn(cell, 0.5f);
+            x = __fadd_rn(__fsub_rn(x, half), __fmul_rn(halton_element<2>(h + 1u), cell));
+            y = __fadd_rn(__fsub_rn(y, half), __fmul_rn(halton_element<3>(h + 1u), cell));
+            z = __fadd_rn(__fsub_rn(z, half), __fmul_rn(halton_element<5>(h + 1u), cell));
+        }
+        store_positions(s_pos, x, y, z, (int64_t)r0 + k0, n_total, positions);
+        __syncthreads();
     }
-    const unsigned leaf = min(first, n_cells - 1);
-    const unsigned c = __ldg(counts + leaf);
-    const unsigned h = (unsigned)i - (__ldg(offsets + leaf) - c);
-    const float cx = __ldg(centers + 3 * (int64_t)leaf), cy = __ldg(centers + 3 * (int64_t)leaf + 1), cz = __ldg(centers + 3 * (int64_t)leaf + 2);
-    if (c == 1u) {
-        positions[3 * i] = cx; positions[3 * i + 1] = cy; positions[3 * i + 2] = cz;
-        return;
-    }
-    // cell edge = initial_size / 2^level, exact in fp32 for the levels an octree has; every further
-    // operation rounds on its own like the torch expression  centre - cell/2 + halton * cell
-    const float cell = __fdiv_rn(initial_size, (float)(1u << __ldg(levels + leaf)));
-    const float half = __fmul_rn(cell, 0.5f);
-    positions[3 * i] = __fadd_rn(__fsub_rn(cx, half), __fmul_rn(halton_element(h + 1u, 2u), cell));
-    positions[3 * i + 1] = __fadd_rn(__fsub_rn(cy, half), __fmul_rn(halton_element(h + 1u, 3u), cell));
-    positions[3 * i + 2] = __fadd_rn(__fsub_rn(cz, half), __fmul_rn(halton_element(h + 1u, 5u), cell));
 }
 
 // 30-bit Morton code (10 bits per axis, x lowest) of a position inside the box [lo, lo + extent]^3
@@ -495,18 +612,84 @@ __device__ __forceinline__ unsigned spread_bits_10(unsigned v) {
     return v;
 }
 
-__global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __restrict__ positions, int64_t n, float lo_x, float lo_y,
-                                                                float lo_z, float inv_extent, unsigned* __restrict__ codes,
-                                                                unsigned* __restrict__ order) {
-    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (i >= n) return;
-    const float qx = (__ldg(positions + 3 * i) - lo_x) * inv_extent * 1024.0f;
-    const float qy = (__ldg(positions + 3 * i + 1) - lo_y) * inv_extent * 1024.0f;
-    const float qz = (__ldg(positions + 3 * i + 2) - lo_z) * inv_extent * 1024.0f;
-    const unsigned x = (unsigned)fminf(fmaxf(qx, 0.0f), 1023.0f), y = (unsigned)fminf(fmaxf(qy, 0.0f), 1023.0f),
-                   z = (unsigned)fminf(fmaxf(qz, 0.0f), 1023.0f);
-    codes[i] = spread_bits_10(x) | (spread_bits_10(y) << 1) | (spread_bits_10(z) << 2);
-    order[i] = (unsigned)i;
+// Corners of the cloud's bounding box, one partial result {min x, y, z, max x, y, z} per block: one pass over the positions,
+// four of them per thread and round in three 16-byte loads where the array allows.
+constexpr int kBoxBlocks = 592;   // 148 multiprocessors x 4
+__device__ __forceinline__ void block_box(float* box, float (*s_box)[6]) {
+    // box[0..2] minima, box[3..5] maxima of a thread -> of the block, in every thread of warp 0
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float t = __shfl_xor_sync(0xffffffffu, box[c], o);
+            box[c] = c < 3 ? fminf(box[c], t) : fmaxf(box[c], t);
+        }
+    if (lane_id() == 0) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) s_box[threadIdx.x >> 5][c] = box[c];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        box[c] = s_box[0][c];
+#pragma unroll
+        for (int w = 1; w < kThreads / 32; ++w) box[c] = c < 3 ? fminf(box[c], s_box[w][c]) : fmaxf(box[c], s_box[w][c]);
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, float* __restrict__ partial) {
+    __shared__ float s_box[kThreads / 32][6];
+    float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    auto add = [&](float x, float y, float z) {
+        box[0] = fminf(box[0], x); box[1] = fminf(box[1], y); box[2] = fminf(box[2], z);
+        box[3] = fmaxf(box[3], x); box[4] = fmaxf(box[4], y); box[5] = fmaxf(box[5], z);
+    };
+    const int64_t stride = (int64_t)gridDim.x * kThreads, tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const int64_t n4 = vec_ok ? n / 4 : 0;
+    const float4* src = reinterpret_cast<const float4*>(positions);
+    for (int64_t v = tid; v < n4; v += stride) {
+        const float4 a = __ldg(src + 3 * v), b = __ldg(src + 3 * v + 1), c = __ldg(src + 3 * v + 2);
+        add(a.x, a.y, a.z); add(a.w, b.x, b.y); add(b.z, b.w, c.x); add(c.y, c.z, c.w);
+    }
+    for (int64_t i = 4 * n4 + tid; i < n; i += stride) add(__ldg(positions + 3 * i), __ldg(positions + 3 * i + 1), __ldg(positions + 3 * i + 2));
+    block_box(box, s_box);
+    if (threadIdx.x < 6) partial[6 * blockIdx.x + threadIdx.x] = threadIdx.x == 0 ? box[0] : threadIdx.x == 1 ? box[1] : threadIdx.x == 2 ? box[2] : threadIdx.x == 3 ? box[3] : threadIdx.x == 4 ? box[4] : box[5];
+}
+
+// The cube the codes refer to: the caller's, or (box_parts > 0) the cloud's own from the partial boxes, its edge widened by
+// a millionth so that the largest coordinate stays inside.  Same roundings as float32 corners and a double product.
+struct MortonBox {
+    float lo[3];
+    float inv_extent;
+    const float* parts;
+    int box_parts;
+};
+__global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __restrict__ positions, int64_t n, MortonBox mb,
+                                                                unsigned* __restrict__ codes, unsigned* __restrict__ order) {
+    if (mb.box_parts > 0) {
+        __shared__ float s_box[kThreads / 32][6];
+        float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        for (int k = threadIdx.x; k < mb.box_parts; k += kThreads)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                const float t = __ldg(mb.parts + 6 * k + c);
+                box[c] = c < 3 ? fminf(box[c], t) : fmaxf(box[c], t);
+            }
+        block_box(box, s_box);
+        const float extent = fmaxf(fmaxf(__fsub_rn(box[3], box[0]), __fsub_rn(box[4], box[1])), __fsub_rn(box[5], box[2]));
+        mb.inv_extent = extent > 0.0f ? __fdiv_rn(1.0f, __double2float_rn(__dmul_rn((double)extent, 1.0 + 1e-6))) : 1.0f;
+        mb.lo[0] = box[0]; mb.lo[1] = box[1]; mb.lo[2] = box[2];
+    }
+    const int64_t stride = (int64_t)gridDim.x * kThreads;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
+        const float qx = (__ldg(positions + 3 * i) - mb.lo[0]) * mb.inv_extent * 1024.0f;
+        const float qy = (__ldg(positions + 3 * i + 1) - mb.lo[1]) * mb.inv_extent * 1024.0f;
+        const float qz = (__ldg(positions + 3 * i + 2) - mb.lo[2]) * mb.inv_extent * 1024.0f;
+        const unsigned x = (unsigned)fminf(fmaxf(qx, 0.0f), 1023.0f), y = (unsigned)fminf(fmaxf(qy, 0.0f), 1023.0f),
+                       z = (unsigned)fminf(fmaxf(qz, 0.0f), 1023.0f);
+        codes[i] = spread_bits_10(x) | (spread_bits_10(y) << 1) | (spread_bits_10(z) << 2);
+        order[i] = (unsigned)i;
+    }
 }
 
 __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float* __restrict__ positions, const unsigned* __restrict__ order,
@@ -530,7 +713,7 @@ struct SamplerWs {
     unsigned* offsets;  // inclusive offsets (n_cells)
     unsigned* chunk_sums;
     unsigned long long* total;
-    unsigned* guide;    // 2^guide_bits + 1 entries
+    uint4* guide;       // 2^guide_bits bucket records
     int guide_bits;
     float4* leaf_pack;  // (n_cells) centre + edge length
     size_t bytes;
@@ -557,7 +740,7 @@ SamplerWs carve_sampler_ws(void* p, int64_t n_cells) {
     w.chunk_sums = c.take<unsigned>(ceil_div<int64_t>(n, kThreads));
     w.total = c.take<unsigned long long>(2);
     w.guide_bits = guide_bits_for(n);
-    w.guide = c.take<unsigned>(((size_t)1 << w.guide_bits) + 2);
+    w.guide = c.take<uint4>((size_t)1 << w.guide_bits);
     w.leaf_pack = c.take<float4>(n);
     w.bytes = c.used();
     return w;
@@ -577,7 +760,7 @@ int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out,
         cdf_finalize_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits, w.chunk_sums64, w.total64, cdf);
         INPC_LAUNCH_CHECK("cdf_finalize_kernel");
         if (cdf == w.cdf) {
-            guide_table_kernel<<<(unsigned)ceil_div<int64_t>(((int64_t)1 << w.guide_bits) + 1, kThreads), kThreads, 0, stream>>>(
+            guide_table_kernel<<<(unsigned)ceil_div<int64_t>((int64_t)1 << w.guide_bits, kGuidePerBlock), kThreads, 0, stream>>>(
                 cdf, (unsigned)n_cells, w.guide_bits, w.guide);
             INPC_LAUNCH_CHECK("guide_table_kernel");
         }
@@ -645,6 +828,26 @@ extern "C" int inpc_compute_viewpoint_weights(const inpc_view* view, int64_t n_c
     viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(
         to_params(view), n_cells, centers, levels, weights, initial_size, out, nullptr);
     INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
+    return INPC_OK;
+}
+
+extern "C" int inpc_max_viewpoint_weights(const inpc_view* views, int n_views, int64_t n_cells, const float* centers, const int32_t* levels,
+                                          const float* weights, float initial_size, float* out, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (n_cells == 0) return INPC_OK;
+    if (n_views < 1 || !out) { set_error("inpc_max_viewpoint_weights: bad argument"); return INPC_E_INVALID; }
+    for (int j = 0; j < n_views; ++j) {
+        const int rc = check_cells(views ? views + j : nullptr, n_cells, centers, levels, weights);
+        if (rc != INPC_OK) return rc;
+    }
+    for (int j = 0; j < n_views; j += kViewsPerPass) {
+        ViewSet set;
+        set.count = n_views - j < kViewsPerPass ? n_views - j : kViewsPerPass;
+        for (int k = 0; k < set.count; ++k) set.v[k] = to_params(views + j + k);
+        max_viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(set, n_cells, centers, levels, weights,
+                                                                                                           initial_size, j == 0, out);
+        INPC_LAUNCH_CHECK("max_viewpoint_weights_kernel");
+    }
     return INPC_OK;
 }
 
@@ -734,7 +937,7 @@ extern "C" int inpc_generate_expected_samples_count(inpc_sampler* s, const inpc_
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     const ViewParams v = to_params(view);
     const unsigned blocks = (unsigned)ceil_div<int64_t>(n_cells, kThreads);
-    viewpoint_weights_kernel<<<blocks, kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw, nullptr);
+    viewpoint_weights_kernel<<<blocks, kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw, w.leaf_pack);
     INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
     rc = build_cdf(w.vw, n_cells, nullptr, w.sum, w, stream);
     if (rc != INPC_OK) return rc;
@@ -766,8 +969,9 @@ extern "C" int inpc_generate_expected_samples_fill(inpc_sampler* s, int64_t n_ce
         return INPC_E_INVALID;
     }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
-    expected_samples_kernel<<<(unsigned)ceil_div<int64_t>(total, kThreads), kThreads, 0, stream>>>(
-        s->seed, s->counter, w.offsets, (unsigned)n_cells, centers, levels, initial_size, total, (unsigned)n_created, positions);
+    const dim3 grid((unsigned)ceil_div<int64_t>(n_created, kRunSlots), (unsigned)(n_multi < 65535 ? n_multi : 65535));
+    expected_samples_kernel<<<grid, kThreads, 0, stream>>>(s->seed, s->counter, w.offsets, (unsigned)n_cells, w.leaf_pack, (unsigned)n_created,
+                                                           (unsigned)n_multi, positions);
     INPC_LAUNCH_CHECK("expected_samples_kernel");
     s->counter += 1;
     return INPC_OK;
@@ -824,32 +1028,42 @@ extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, cons
     INPC_CUDA_TRY(cudaMemcpyAsync(w.counts, counts, sizeof(uint32_t) * (size_t)n_cells, cudaMemcpyDeviceToDevice, stream));
     const int rc = scan_counts(w, n_cells, stream);
     if (rc != INPC_OK) return rc;
-    halton_samples_kernel<<<(unsigned)ceil_div<int64_t>(n_total, kThreads), kThreads, 0, stream>>>(w.counts, w.offsets, (unsigned)n_cells, centers, levels,
-                                                                                                 initial_size, n_total, positions);
+    halton_samples_kernel<<<(unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream>>>(w.counts, w.offsets, (unsigned)n_cells, centers, levels,
+                                                                                                 initial_size, (unsigned)n_total, positions);
     INPC_LAUNCH_CHECK("halton_samples_kernel");
     return INPC_OK;
 }
 
 extern "C" size_t inpc_morton_workspace_bytes(int64_t n) {
     const size_t arr = align_up(sizeof(uint32_t) * (size_t)(n > 0 ? n : 1));
-    return 4 * arr + sort_workspace_bytes(n) + 256;
+    return 4 * arr + align_up(6 * sizeof(float) * kBoxBlocks) + sort_workspace_bytes(n) + 256;
 }
 
 extern "C" int inpc_morton_order(const float* positions, int64_t n, const float* box_lo, float box_extent, float* out, void* workspace,
                                  void* stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (n == 0) return INPC_OK;
-    if (n < 0 || n >= ((int64_t)1 << 30) || !positions || !box_lo || !(box_extent > 0.0f) || !out || !workspace || out == positions) {
+    if (n < 0 || n >= ((int64_t)1 << 30) || !positions || (box_lo && !(box_extent > 0.0f)) || !out || !workspace || out == positions) {
         set_error("inpc_morton_order: bad argument");
         return INPC_E_INVALID;
     }
     Carver c(workspace);
     uint32_t* codes[2] = {c.take<uint32_t>(n), c.take<uint32_t>(n)};
     uint32_t* order[2] = {c.take<uint32_t>(n), c.take<uint32_t>(n)};
+    float* parts = c.take<float>(6 * kBoxBlocks);
     c.off = align_up(c.off);
     void* sort_ws = c.base + c.off;
-    morton_codes_kernel<<<(unsigned)ceil_div<int64_t>(n, kThreads), kThreads, 0, stream>>>(positions, n, box_lo[0], box_lo[1], box_lo[2],
-                                                                                       1.0f / box_extent, codes[0], order[0]);
+    MortonBox mb{{0.0f, 0.0f, 0.0f}, 1.0f, parts, 0};
+    if (box_lo) {
+        for (int k = 0; k < 3; ++k) mb.lo[k] = box_lo[k];
+        mb.inv_extent = 1.0f / box_extent;
+    } else {
+        mb.box_parts = (int)(ceil_div<int64_t>(n, 4 * kThreads) < kBoxBlocks ? ceil_div<int64_t>(n, 4 * kThreads) : kBoxBlocks);
+        bounding_box_kernel<<<mb.box_parts, kThreads, 0, stream>>>(positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, parts);
+        INPC_LAUNCH_CHECK("bounding_box_kernel");
+    }
+    const int64_t code_blocks = ceil_div<int64_t>(n, kThreads), code_cap = (int64_t)sm_count() * 8;
+    morton_codes_kernel<<<(unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kThreads, 0, stream>>>(positions, n, mb, codes[0], order[0]);
     INPC_LAUNCH_CHECK("morton_codes_kernel");
     int in_alt = 0;
     {

@@ -65,6 +65,19 @@ def compute_viewpoint_weights(centers: torch.Tensor, levels: torch.Tensor, weigh
     return out
 
 
+def _max_viewpoint_weights(centers: torch.Tensor, levels: torch.Tensor, weights: torch.Tensor, views, initial_size: float) -> torch.Tensor:
+    """Maximum over `views` of `compute_viewpoint_weights`."""
+    for view in views:
+        _check_view(view)
+    dev = centers.device
+    with _on(dev):
+        args = [_ViewArg(view, dev) for view in views]
+        out = torch.empty_like(weights)
+        _cabi.check(_cabi.lib().inpc_max_viewpoint_weights((_cabi.View * len(args))(*[a.c for a in args]), len(args), weights.numel(), _ptr(centers),
+                                                           _ptr(levels), _ptr(weights), float(initial_size), _ptr(out), _stream()))
+    return out
+
+
 class ProbabilityFieldSampler(torch.nn.Module):
     def __init__(self, seed: int) -> None:
         super().__init__()
@@ -186,9 +199,11 @@ def halton_samples(counts: torch.Tensor, centers: torch.Tensor, levels: torch.Te
     centers, levels, _, n = _leaf_args(centers, levels, torch.empty(centers.shape[0], dtype=torch.float32, device=centers.device))
     if counts.numel() != n:
         raise ValueError(f"counts must hold one entry per leaf ({n}), got {counts.numel()}")
-    counts = counts.contiguous()
-    total = int(counts.sum().item())
-    dev = centers.device
+    return _halton_samples(counts.contiguous(), centers, levels, initial_size, int(counts.sum().item()))
+
+
+def _halton_samples(counts: torch.Tensor, centers: torch.Tensor, levels: torch.Tensor, initial_size: float, total: int) -> torch.Tensor:
+    n, dev = counts.numel(), centers.device
     with _on(dev):
         positions = torch.empty((total, 3), dtype=torch.float32, device=dev)
         ws = torch.empty(int(_cabi.lib().inpc_sampler_workspace_bytes(n)), dtype=torch.uint8, device=dev)
@@ -206,15 +221,11 @@ def morton_order(positions: torch.Tensor) -> torch.Tensor:
     n = positions.shape[0]
     if n == 0:
         return positions.clone()
-    lo = positions.amin(dim=0)
-    extent = float((positions.amax(dim=0) - lo).max().item())
-    extent = extent * (1.0 + 1e-6) if extent > 0 else 1.0
-    box_lo = (C.c_float * 3)(*[float(v) for v in lo.tolist()])
     dev = positions.device
     with _on(dev):
         out = torch.empty_like(positions)
         ws = torch.empty(int(_cabi.lib().inpc_morton_workspace_bytes(n)), dtype=torch.uint8, device=dev)
-        _cabi.check(_cabi.lib().inpc_morton_order(_ptr(positions), n, box_lo, extent, _ptr(out), _ptr(ws), _stream()))
+        _cabi.check(_cabi.lib().inpc_morton_order(_ptr(positions), n, None, 0.0, _ptr(out), _ptr(ws), _stream()))
     return out
 
 
@@ -225,13 +236,11 @@ def extract_global(sampler: "ProbabilityFieldSampler", centers: torch.Tensor, le
     sample counts per leaf, Halton placement inside every leaf, optional Morton order."""
     centers, levels, weights, n = _leaf_args(centers, levels, weights)
     if views:
-        global_weights = torch.zeros_like(weights)
-        for view in views:
-            torch.maximum(compute_viewpoint_weights(centers, levels, weights, view, initial_size), global_weights, out=global_weights)
+        global_weights = _max_viewpoint_weights(centers, levels, weights, views, initial_size)
     else:
         global_weights = weights * torch.exp2(-levels * 0.5)             # ProbabilityField.get_current_weights(None)
     counts = sampler.draw_leaf_counts(global_weights, n_samples)
-    positions = halton_samples(counts, centers, levels, initial_size)
+    positions = _halton_samples(counts, centers, levels, initial_size, int(n_samples))   # every draw lands in a leaf
     return morton_order(positions) if use_morton_order else positions
 
 
