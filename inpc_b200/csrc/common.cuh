@@ -115,14 +115,16 @@ inline ViewParams to_params(const inpc_view* v) {
 }
 
 // ---- radix sort (radix_sort.cu) ------------------------------------------------------------
-size_t sort_workspace_bytes(int64_t n);
+// The workspace for n pairs (an upper bound) of which n_likely are expected: the expectation picks the tile size, no more.
+size_t sort_workspace_bytes(int64_t n, int64_t n_likely);
 int sort_pass_count(int end_bit);   // passes sort_pairs makes; the result is in the alternate buffers iff odd (and n > 1)
 // `status`: device address of the STATUS_WORDS words a tile that gives up its look-back reports to.
-int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n,
+// `n_likely`: the one the workspace was sized with (for at least n pairs).
+int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
                int end_bit, void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream);
-// The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for n_max.  The result is in the
+// The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for (n_max, n_likely).  The result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
-int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max,
+int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
                             const unsigned long long* n_dev, int end_bit, void* workspace, unsigned* status, int* result_in_alt,
                             cudaStream_t stream);
 

@@ -20,10 +20,10 @@ constexpr int kRadixBits = 9;            // widest digit of a pass: 27 key bits 
 constexpr int kRadix = 1 << kRadixBits;  // capacity of every per-digit array
 constexpr int kMaxPasses = 4;
 constexpr int kThreads = 512;
-constexpr int kItems = 16;
-constexpr int kTile = kThreads * kItems;   // 8192 pairs per tile
 constexpr int kWarps = kThreads / 32;
-constexpr int kDigitsPerThread = (kRadix + kThreads - 1) / kThreads;   // digits a thread owns in the scan / look-back phase
+constexpr int kLargeItems = 16;          // pairs per thread and tile, see tile_items
+constexpr int kLargeTile = kThreads * kLargeItems;
+static_assert(kRadix <= kThreads, "a thread owns at most one digit");
 
 constexpr unsigned kFlagAggregate = 1u << 30;
 constexpr unsigned kFlagPrefix = 2u << 30;
@@ -46,265 +46,289 @@ constexpr int kHistItemsPerBlock = kHistThreads * 4 * 8;   // 8 uint4 loads per 
 // brought them in with bulk asynchronous copies (cp.async.bulk into two 16 KB slabs per block, an mbarrier per slab)
 // measured the same on B200 -- whole sort of 2^23 pairs, 32 / 27 / 24 key bits: 316 / 271 / 241 us against
 // 314 / 267 / 239 us with the plain 16-byte loads below; 2^25 pairs, 25 bits: 794 against 799 us.
+// The block that finishes last turns the counts of every pass into digit bases (exclusive scans): no launch of its own.
 __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
-    const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, PassTable pt, unsigned* __restrict__ hist) {
+    const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, PassTable pt, unsigned* hist, unsigned* blocks_done,
+    unsigned* __restrict__ base) {
     const int64_t n = n_dev ? (int64_t)*n_dev : n_arg;
     if ((int64_t)blockIdx.x * kHistItemsPerBlock >= n) return;
     __shared__ unsigned s_hist[kMaxPasses][kRadix];
+    __shared__ unsigned s_scan[kHistThreads / 32 + 1];
+    __shared__ bool s_last;
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads) (&s_hist[0][0])[i] = 0;
     __syncthreads();
 
-    const int64_t block_base = (int64_t)blockIdx.x * kHistItemsPerBlock;
-    const int64_t block_end = min(n, block_base + (int64_t)kHistItemsPerBlock);
     auto count = [&](uint32_t k) {
 #pragma unroll
         for (int p = 0; p < kMaxPasses; ++p)
             if (p < pt.n_passes) atomicAdd(&s_hist[p][(k >> pt.shift[p]) & ((1u << pt.bits[p]) - 1u)], 1u);
     };
-    // keys is 16-byte aligned (carved at 256 bytes) and block_base is a multiple of 4
-    const uint4* keys4 = reinterpret_cast<const uint4*>(keys + block_base);
-    const int64_t n_vec = (block_end - block_base) / 4;
-    for (int64_t v = threadIdx.x; v < n_vec; v += kHistThreads) {
-        const uint4 k = __ldg(keys4 + v);
-        count(k.x); count(k.y); count(k.z); count(k.w);
+    for (int64_t block_base = (int64_t)blockIdx.x * kHistItemsPerBlock; block_base < n; block_base += (int64_t)gridDim.x * kHistItemsPerBlock) {
+        const int64_t block_end = min(n, block_base + (int64_t)kHistItemsPerBlock);
+        // keys is 16-byte aligned (carved at 256 bytes) and block_base is a multiple of 4
+        const uint4* keys4 = reinterpret_cast<const uint4*>(keys + block_base);
+        const int n_vec = (int)((block_end - block_base) / 4);
+        for (int v = threadIdx.x; v < n_vec; v += kHistThreads) {
+            const uint4 k = __ldg(keys4 + v);
+            count(k.x); count(k.y); count(k.z); count(k.w);
+        }
+        for (int64_t i = block_base + (int64_t)n_vec * 4 + threadIdx.x; i < block_end; i += kHistThreads) count(keys[i]);
     }
-    for (int64_t i = block_base + n_vec * 4 + threadIdx.x; i < block_end; i += kHistThreads) count(keys[i]);
     __syncthreads();
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads) {
         const unsigned c = (&s_hist[0][0])[i];
         if (c) atomicAdd(hist + i, c);
     }
-}
-
-// exclusive scan of each pass's 256 counters -> global digit bases
-__global__ void __launch_bounds__(kRadix) radix_scan_histogram_kernel(const unsigned* __restrict__ hist,
-                                                                      unsigned* __restrict__ base) {
-    __shared__ unsigned s_scan[kRadix / 32 + 1];
-    const int p = blockIdx.x;
-    const unsigned c = hist[p * kRadix + threadIdx.x];
-    unsigned total;
-    const unsigned ex = block_exclusive_scan(c, s_scan, &total);
-    base[p * kRadix + threadIdx.x] = ex;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int64_t all = ceil_div<int64_t>(n, kHistItemsPerBlock);
+        const unsigned working = (unsigned)min(all, (int64_t)gridDim.x);
+        s_last = atomicAdd(blocks_done, 1u) == working - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int p = 0; p < pt.n_passes; ++p) {
+        unsigned total;
+        const unsigned ex = block_exclusive_scan(__ldcg(hist + p * kRadix + threadIdx.x), s_scan, &total);
+        base[p * kRadix + threadIdx.x] = ex;
+    }
 }
 
 // ---- one pass ---------------------------------------------------------------------------------
+// Bound by shared-memory wavefronts (63 % of the LSU data pipe over the whole pass, 40 wavefronts per 32 pairs) and by
+// the phases of a tile waiting on one another, not by DRAM (16 bytes per pair, 16 % of its peak).  Persistent blocks take
+// tiles from a ticket counter: the grid fits the chip whatever the bound on n is (a grid sized for an upper bound of a
+// device-side count was mostly empty blocks).  Per tile:
+//   1. rank: every lane ORs its bit into its warp's match word of its digit; the word then names the lanes that hold the
+//      digit, and the last of them advances the warp's counter and clears the word.  (One ballot per digit bit instead
+//      keeps the integer pipe busy for 9.5 thousand cycles per tile of 9-bit digits, this takes 8.)
+//   2. thread d adds up digit d over the warps and publishes the tile's count; directly behind it -- so that few tiles are
+//      ever between their count and their prefix -- the decoupled look-back;
+//   3. the pairs go to their tile-local slots in shared memory as 8-byte words;
+//   4. coalesced write-out: consecutive slots of one digit go to consecutive addresses.
+// Measured against the pass before it (ballots, one block per possible tile): 2^23 pairs of 27 bits 265 -> 228 us, 10.6 M of 14
+// bits 190 -> 167, 2^25 of 30 bits 976 -> 860.  Without any look-back the same passes take 214, 167 and 860: the waiting is
+// hidden.  Tried and not kept: the next tile's ticket and keys asked for before the write-out (tiles then publish later
+// and less evenly: 2^25 pairs 978 us), look-back windows of 16 and 32 (234 and 269), 256 x 24 / 256 x 32 / 384 x 20 threads x
+// items (243, 230, 243).
+template <int BITS, int ITEMS>
 struct PassSmem {
+    static constexpr int kBins = BITS > 0 ? 1 << BITS : kRadix;
     union {
-        unsigned warp_hist[kWarps][kRadix];   // ranking phase
-        uint32_t keys[kTile];                 // reorder phase (keys); the two never live at the same time
+        struct {                        // steps 1 and 2
+            unsigned count[kWarps][kBins];
+            unsigned match[kWarps][kBins];
+        };
+        uint2 pairs[kThreads * ITEMS];  // steps 3 and 4; the two never live at the same time
     };
-    uint32_t values[kTile];
-    unsigned bin_start[kRadix];    // tile-local exclusive start of each digit
-    unsigned global_off[kRadix];   // global position of a digit's first key minus bin_start
+    unsigned global_off[kBins];         // global position of a digit's first pair minus its tile-local one
     unsigned scan[kWarps + 1];
     unsigned tile_id;
 };
 
-// BITS > 0 fixes the digit width at compile time (the ballot loop of the ranking unrolls); BITS == 0
-// takes it from `bits_arg`.
-template <int BITS>
-__global__ void __launch_bounds__(kThreads) radix_onesweep_pass_kernel(
+// BITS > 0 fixes the digit width at compile time; BITS == 0 takes it from `bits_arg`.
+template <int BITS, int ITEMS>
+__global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n_arg, const unsigned long long* __restrict__ n_dev,
     int shift, int bits_arg, const unsigned* __restrict__ digit_base, volatile unsigned* tile_state, unsigned* ticket,
     volatile unsigned* status, int spin_limit, unsigned mute_tile) {
+    using Smem = PassSmem<BITS, ITEMS>;
+    constexpr int kBins = Smem::kBins;
+    constexpr unsigned kTile = kThreads * ITEMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PassSmem& s = *reinterpret_cast<PassSmem*>(smem_raw);
+    Smem& s = *reinterpret_cast<Smem*>(smem_raw);
 
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const int bits = BITS > 0 ? BITS : bits_arg;
-    const unsigned digit_mask = (1u << bits) - 1u;
+    const unsigned digit_mask = (1u << (BITS > 0 ? BITS : bits_arg)) - 1u;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned n = n_dev ? (unsigned)*n_dev : (unsigned)n_arg;   // < 2^30
+    const unsigned n_tiles = (n + kTile - 1u) / kTile;
+    unsigned *const my_count = s.count[warp], *const my_match = s.match[warp];
+    // warp-striped layout: warp w owns [w*32*ITEMS, (w+1)*32*ITEMS) of the tile, item i of lane l
+    // is element i*32+l of that segment, so (warp, item, lane) order is the input order.
+    const unsigned local = warp * (32u * ITEMS) + lane;
+
+    uint32_t key[ITEMS];
+    auto load_keys = [&](unsigned tile) {
+        if (tile >= n_tiles) return;
+        const unsigned first = tile * kTile + local;
+        const uint32_t* kp = keys_in + first;
+        if (tile * kTile + kTile <= n) {
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) key[i] = __ldg(kp + i * 32);
+        } else {
+            // padding ranks behind every real key of its digit: it is last in the tile, and its digit is the largest
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) key[i] = first + i * 32u < n ? __ldg(kp + i * 32) : 0xFFFFFFFFu;
+        }
+    };
 
     if (tid == 0) s.tile_id = atomicAdd(ticket, 1u);
-    for (int i = tid; i < kWarps * kRadix; i += kThreads) (&s.warp_hist[0][0])[i] = 0;
     __syncthreads();
-    const unsigned tile = s.tile_id;
-    // `mute_tile` (no tile in normal operation) leaves without publishing anything: the tiles behind it then
+    unsigned tile = s.tile_id;
+    // `mute_tile` (no tile in normal operation) is dropped without publishing anything: the tiles behind it then
     // run into the limit of their look-back wait, which is how the tests exercise that path
     if (tile == mute_tile) return;
-    const int64_t n = n_dev ? (int64_t)*n_dev : n_arg;
-    const int64_t tile_base = (int64_t)tile * kTile;
-    if (tile_base >= n) return;   // grid sized for an upper bound of n: nothing here, and no tile waits for this one
-    const int valid = (int)min((int64_t)kTile, n - tile_base);
-
-    // warp-striped load: warp w owns [w*32*kItems, (w+1)*32*kItems) of the tile, item i of lane l
-    // is element i*32+l of that segment, so (warp, item, lane) order is the input order.
-    uint32_t key[kItems];
-    unsigned rank[kItems];
-    const int seg = warp * 32 * kItems;
+    load_keys(tile);
+    while (tile < n_tiles) {
+        const unsigned valid = min(kTile, n - tile * kTile);
+        const bool full = valid == kTile;
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const int local = seg + i * 32 + lane;
-        key[i] = local < valid ? __ldg(keys_in + tile_base + local) : 0xFFFFFFFFu;
-    }
-
-    // stable rank within the warp's segment, per digit.  The lanes holding the same digit are found
-    // with one ballot per digit bit (independent across items, so they pipeline); only the update of
-    // the warp's digit counter is a serial chain.
-    unsigned peers[kItems];
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const unsigned d = (key[i] >> shift) & digit_mask;
-        unsigned p = 0xffffffffu;
-        if (BITS > 0) {
-#pragma unroll
-            for (int b = 0; b < BITS; ++b) {
-                const bool one = (d >> b) & 1u;
-                const unsigned m = __ballot_sync(0xffffffffu, one);
-                p &= one ? m : ~m;
-            }
-        } else {
-            for (int b = 0; b < bits; ++b) {
-                const bool one = (d >> b) & 1u;
-                const unsigned m = __ballot_sync(0xffffffffu, one);
-                p &= one ? m : ~m;
-            }
-        }
-        peers[i] = p;
-    }
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const unsigned d = (key[i] >> shift) & digit_mask;
-        const int leader = __ffs(peers[i]) - 1;
-        unsigned base = 0;
-        if ((int)lane == leader) {
-            base = s.warp_hist[warp][d];
-            s.warp_hist[warp][d] = base + __popc(peers[i]);
-        }
-        base = __shfl_sync(0xffffffffu, base, leader);
-        rank[i] = base + __popc(peers[i] & ((1u << lane) - 1u));
+        for (int i = 0; i < kBins / 32; ++i) my_count[i * 32 + lane] = my_match[i * 32 + lane] = 0u;
         __syncwarp();
-    }
-    __syncthreads();
 
-    // per digit: exclusive scan over warps, tile total.  Thread t owns digits t*kDigitsPerThread ...
-    const unsigned radix = 1u << bits;
-    unsigned total[kDigitsPerThread];
-    unsigned thread_sum = 0;
+        // 1. stable rank within the warp's segment, per digit
+        unsigned pos[ITEMS];
 #pragma unroll
-    for (int q = 0; q < kDigitsPerThread; ++q) {
-        const unsigned d = tid * kDigitsPerThread + q;
-        total[q] = 0;
-        if (d < radix) {
+        for (int i = 0; i < ITEMS; ++i) {
+            const unsigned d = (key[i] >> shift) & digit_mask;
+            atomicOr(my_match + d, 1u << lane);
+            const unsigned before = my_count[d];
+            __syncwarp();
+            const unsigned peers = my_match[d];
+            pos[i] = before + __popc(peers & lt_mask);
+            __syncwarp();
+            if ((peers >> lane) == 1u) { my_count[d] = pos[i] + 1u; my_match[d] = 0u; }   // the last lane with this digit
+            __syncwarp();
+        }
+        uint32_t val[ITEMS];
+        {
+            const unsigned first = tile * kTile + local;
+            const uint32_t* vp = vals_in + first;
+            if (full) {
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) val[i] = __ldg(vp + i * 32);
+            } else {
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) val[i] = first + i * 32u < n ? __ldg(vp + i * 32) : 0u;
+            }
+        }
+        __syncthreads();
+
+        // 2. digit `tid` over the warps
+        unsigned total = 0;
+        if (tid < (unsigned)kBins) {
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) total += s.count[w][tid];
+            // publish this tile's digit count before any waiting
+            tile_state[tile * kBins + tid] = total | (tile == 0 ? kFlagPrefix : kFlagAggregate);
+        }
+        unsigned block_total;
+        const unsigned start = block_exclusive_scan(total, s.scan, &block_total);
+        if (tid < (unsigned)kBins) {
+            unsigned run = start;
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) {
-                const unsigned c = s.warp_hist[w][d];
-                s.warp_hist[w][d] = total[q];
-                total[q] += c;
+                const unsigned c = s.count[w][tid];
+                s.count[w][tid] = run;
+                run += c;
             }
-            // publish this tile's digit count before any waiting
-            tile_state[(size_t)tile * kRadix + d] = total[q] | (tile == 0 ? kFlagPrefix : kFlagAggregate);
-        }
-        thread_sum += total[q];
-    }
-    unsigned block_total;
-    unsigned start = block_exclusive_scan(thread_sum, s.scan, &block_total);
+            // decoupled look-back, a window of predecessors per round trip: the loads of a window are
+            // independent, so their latencies overlap; entries are then consumed nearest-first
+            unsigned exclusive = 0;
+            if (tile > 0) {
+                constexpr int kWindow = 8;
+                int j = (int)tile - 1;
+                bool gave_up = false, finished = false;
+                while (j >= 0 && !finished && !gave_up) {
+                    unsigned v[kWindow];
+                    volatile unsigned* sp = tile_state + j * kBins + tid;
 #pragma unroll
-    for (int q = 0; q < kDigitsPerThread; ++q) {
-        const unsigned d = tid * kDigitsPerThread + q;
-        if (d >= radix) break;
-        s.bin_start[d] = start;
-        // decoupled look-back, a window of predecessors per round trip: the loads of a window are
-        // independent, so their latencies overlap; entries are then consumed nearest-first
-        unsigned exclusive = 0;
-        if (tile > 0) {
-            constexpr int kWindow = 8;
-            int64_t j = (int64_t)tile - 1;
-            bool gave_up = false, finished = false;
-            while (j >= 0 && !finished && !gave_up) {
-                unsigned v[kWindow];
-#pragma unroll
-                for (int k = 0; k < kWindow; ++k) {
-                    v[k] = 2u << 30;   // beyond tile 0: an empty inclusive prefix
-                    if (j - k >= 0) v[k] = tile_state[(size_t)(j - k) * kRadix + d];
-                }
-#pragma unroll
-                for (int k = 0; k < kWindow; ++k) {
-                    if (finished || gave_up) break;
-                    unsigned x = v[k];
-                    int spins = 0;
-                    while ((x & kFlagMask) == 0u && spins < spin_limit) {   // not published yet: poll this one
-                        __nanosleep(20);
-                        x = tile_state[(size_t)(j - k) * kRadix + d];
-                        ++spins;
+                    for (int k = 0; k < kWindow; ++k) {
+                        v[k] = kFlagPrefix;   // beyond tile 0: an empty inclusive prefix
+                        if (j - k >= 0) v[k] = sp[-k * kBins];
                     }
-                    if ((x & kFlagMask) == 0u) { gave_up = true; break; }
-                    exclusive += x & kValueMask;
-                    if (x & kFlagPrefix) finished = true;
+#pragma unroll
+                    for (int k = 0; k < kWindow; ++k) {
+                        if (finished || gave_up) break;
+                        unsigned x = v[k];
+                        int spins = 0;
+                        while ((x & kFlagMask) == 0u && spins < spin_limit) {   // not published yet: poll this one
+                            __nanosleep(20);
+                            x = sp[-k * kBins];
+                            ++spins;
+                        }
+                        if ((x & kFlagMask) == 0u) { gave_up = true; break; }
+                        exclusive += x & kValueMask;
+                        if (x & kFlagPrefix) finished = true;
+                    }
+                    j -= kWindow;
                 }
-                j -= kWindow;
+                if (gave_up) status[STATUS_LOOKBACK_TIMEOUT] = 1u;
+                tile_state[tile * kBins + tid] = ((exclusive + total) & kValueMask) | kFlagPrefix;
             }
-            if (gave_up) status[STATUS_LOOKBACK_TIMEOUT] = 1u;
-            tile_state[(size_t)tile * kRadix + d] = ((exclusive + total[q]) & kValueMask) | kFlagPrefix;
+            s.global_off[tid] = __ldg(digit_base + tid) + exclusive - start;
         }
-        s.global_off[d] = digit_base[d] + exclusive - start;
-        start += total[q];
-    }
-    __syncthreads();
+        __syncthreads();
 
-    // tile-local position of every key; values follow the same permutation
-    unsigned pos[kItems];
+        // 3. tile-local slots
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const unsigned d = (key[i] >> shift) & digit_mask;
-        pos[i] = s.bin_start[d] + s.warp_hist[warp][d] + rank[i];
-    }
-    uint32_t val[kItems];
+        for (int i = 0; i < ITEMS; ++i) pos[i] += my_count[(key[i] >> shift) & digit_mask];
+        __syncthreads();   // the counters are dead from here on: their storage holds the staged pairs
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const int local = seg + i * 32 + lane;
-        val[i] = local < valid ? __ldg(vals_in + tile_base + local) : 0u;
-    }
-    __syncthreads();   // warp_hist is dead from here on: its storage becomes the key staging area
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        s.keys[pos[i]] = key[i];
-        s.values[pos[i]] = val[i];
-    }
-    __syncthreads();
+        for (int i = 0; i < ITEMS; ++i) s.pairs[pos[i]] = make_uint2(key[i], val[i]);
+        __syncthreads();
 
-    // coalesced write-out: consecutive staged slots of one digit go to consecutive addresses.
-    // Padding keys (0xFFFFFFFF) rank behind every real key of the last tile, i.e. at slots >= valid.
-    for (int q = tid; q < valid; q += kThreads) {
-        const uint32_t k = s.keys[q];
-        const unsigned d = (k >> shift) & digit_mask;
-        const unsigned dst = s.global_off[d] + (unsigned)q;
-        // always true in a healthy sort.  After a look-back that gave up, a later pass meets keys whose digits no
-        // longer match the histogram taken up front, and its positions can then run past the end: drop those.
-        if (dst < (unsigned)n) {
-            keys_out[dst] = k;
-            vals_out[dst] = s.values[q];
+        // 4. write-out.  Padding ranks behind every real pair of the last tile, i.e. at slots >= valid.  dst < n always holds
+        // in a healthy sort; after a look-back that gave up, a later pass meets keys whose digits no longer match the
+        // histogram taken up front, and its positions can then run past the end: those are dropped.
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const unsigned q = tid + i * kThreads;
+            if (full || q < valid) {
+                const uint2 kv = s.pairs[q];
+                const unsigned dst = s.global_off[(kv.x >> shift) & digit_mask] + q;
+                if (dst < n) {
+                    keys_out[dst] = kv.x;
+                    vals_out[dst] = kv.y;
+                }
+            }
         }
+        __syncthreads();   // everybody has read the staged pairs
+        if (tid == 0) s.tile_id = atomicAdd(ticket, 1u);
+        __syncthreads();
+        tile = s.tile_id;
+        load_keys(tile);
     }
 }
 
+// Pairs per thread of a tile, from the number of pairs a call most likely sorts.  Large tiles have longer output runs, less
+// bookkeeping per pair and a shorter chain of look-backs; small ones have less to do one after the other.  Measured, tiles of
+// 8192 / 2048 pairs, 27 key bits: 2^14 pairs 50 / 40 us, 2^17 56 / 48, 2^18 58 / 50, 2^19 62 / 64, 2^20 62 / 87.
+constexpr int kSmallItems = 4;
+constexpr int64_t kSmallMax = 1 << 18;
+int tile_items(int64_t n_likely) { return n_likely > kSmallMax ? kLargeItems : kSmallItems; }
+
+// Digit bins a pass keeps per tile: digits of 7, 8 and 9 bits (depth keys 9 or 8, tile keys 7 to 9) have unrolled kernels.
+int pass_bins(int bits) { return bits >= 7 && bits <= 9 ? 1 << bits : kRadix; }
+
 struct SortWorkspace {
     unsigned* hist;     // [kMaxPasses][kRadix]
-    unsigned* ticket;   // [kMaxPasses]
+    unsigned* ticket;   // [kMaxPasses] tickets, then the histogram's count of finished blocks
     unsigned* base;     // [kMaxPasses][kRadix]
-    unsigned* state;    // [kMaxPasses][tiles][kRadix]
-    size_t zero_bytes;  // leading bytes that must be cleared per sort (hist + ticket)
-    size_t state_bytes;
+    unsigned* state;    // [passes][tiles][bins]
+    size_t zero_bytes;  // leading bytes that must be cleared per sort (hist + ticket), the state follows them
     size_t total;
 };
 
-SortWorkspace carve_sort_workspace(void* ws, int64_t n) {
+SortWorkspace carve_sort_workspace(void* ws, int64_t n, int items) {
     SortWorkspace w;
-    const int64_t tiles = n > 0 ? ceil_div<int64_t>(n, kTile) : 1;
+    const int64_t tiles = n > 0 ? ceil_div<int64_t>(n, (int64_t)kThreads * items) : 1;
     Carver c(ws);
     w.hist = c.take<unsigned>(kMaxPasses * kRadix);
     w.ticket = c.take<unsigned>(64);
     w.zero_bytes = c.used();
     w.state = c.take<unsigned>((size_t)kMaxPasses * tiles * kRadix);
-    w.state_bytes = c.used() - w.zero_bytes;
     w.base = c.take<unsigned>(kMaxPasses * kRadix);
     w.total = c.used();
     return w;
 }
 
-
 struct PassArgs {
-    int64_t tiles;
+    int64_t tiles;         // upper bound
     const uint32_t *kin, *vin;
     uint32_t *kout, *vout;
     int64_t n;
@@ -316,35 +340,32 @@ struct PassArgs {
     unsigned mute_tile;    // tile that never publishes (tests only); 0xFFFFFFFF = none
 };
 
-template <int BITS>
+template <int BITS, int ITEMS>
 int launch_onesweep_instance(const PassArgs& a, cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
-    static std::mutex attr_mutex;
-    constexpr size_t kSmemBytes = sizeof(PassSmem);
-    {
-        std::lock_guard<std::mutex> lock(attr_mutex);
-        const int rc = opt_in_dynamic_smem(radix_onesweep_pass_kernel<BITS>, kSmemBytes, attr_set);
-        if (rc != INPC_OK) return rc;
-    }
-    radix_onesweep_pass_kernel<BITS><<<(unsigned)a.tiles, kThreads, kSmemBytes, stream>>>(a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base,
-                                                                                         a.state, a.ticket, a.status, a.spin_limit, a.mute_tile);
+    constexpr size_t kSmemBytes = sizeof(PassSmem<BITS, ITEMS>);
+    const int rc = opt_in_dynamic_smem(radix_onesweep_pass_kernel<BITS, ITEMS>, kSmemBytes, attr_set);
+    if (rc != INPC_OK) return rc;
+    const int64_t resident = (int64_t)sm_count() * 2;
+    radix_onesweep_pass_kernel<BITS, ITEMS><<<(unsigned)(a.tiles < resident ? a.tiles : resident), kThreads, kSmemBytes, stream>>>(
+        a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base, a.state, a.ticket, a.status, a.spin_limit, a.mute_tile);
     INPC_LAUNCH_CHECK("radix_onesweep_pass_kernel");
     return INPC_OK;
 }
 
-// the digit widths the rasterizer's sorts use (depth keys 9/8, tile keys 7) get unrolled kernels
+template <int ITEMS>
 int launch_onesweep_pass(const PassArgs& a, cudaStream_t stream) {
     switch (a.bits) {
-        case 7: return launch_onesweep_instance<7>(a, stream);
-        case 8: return launch_onesweep_instance<8>(a, stream);
-        case 9: return launch_onesweep_instance<9>(a, stream);
-        default: return launch_onesweep_instance<0>(a, stream);
+        case 7: return launch_onesweep_instance<7, ITEMS>(a, stream);
+        case 8: return launch_onesweep_instance<8, ITEMS>(a, stream);
+        case 9: return launch_onesweep_instance<9, ITEMS>(a, stream);
+        default: return launch_onesweep_instance<0, ITEMS>(a, stream);
     }
 }
 
 }  // namespace
 
-size_t sort_workspace_bytes(int64_t n) { return carve_sort_workspace(nullptr, n).total; }
+size_t sort_workspace_bytes(int64_t n, int64_t n_likely) { return carve_sort_workspace(nullptr, n, tile_items(n_likely)).total; }
 
 int sort_pass_count(int end_bit) { return end_bit > 0 ? ceil_div(end_bit, kRadixBits) : 0; }
 
@@ -365,8 +386,9 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 
 // The sort proper: `workspace` holds sort_workspace_bytes(n) bytes, `status` is the device address of the
 // status words a tile that gives up its look-back writes to.  Every entry point ends up here.
+// `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
-                           void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
+                           int items, void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
                            unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
@@ -384,29 +406,30 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
         bit += b;
     }
 
-    SortWorkspace w = carve_sort_workspace(workspace, n);
-    const int64_t tiles = ceil_div<int64_t>(n, kTile);
+    SortWorkspace w = carve_sort_workspace(workspace, n, items);
+    const int64_t tiles = ceil_div<int64_t>(n, (int64_t)kThreads * items);
+    size_t state_words = 0;
+    for (int p = 0; p < pt.n_passes; ++p) state_words += (size_t)tiles * pass_bins(pt.bits[p]);
     // hist, tickets and the look-back state are contiguous at the front of the workspace; a workspace that
     // is reused keeps the previous call's contents, so everything this call reads is cleared first
-    INPC_CUDA_TRY(cudaMemsetAsync(workspace, 0, w.zero_bytes + (size_t)pt.n_passes * tiles * kRadix * sizeof(unsigned), stream));
+    INPC_CUDA_TRY(cudaMemsetAsync(workspace, 0, w.zero_bytes + state_words * sizeof(unsigned), stream));
 
-    const int hist_blocks = (int)ceil_div<int64_t>(n, kHistItemsPerBlock);
-    radix_histogram_kernel<<<hist_blocks, kHistThreads, 0, stream>>>(keys, n, n_dev, pt, w.hist);
+    const int64_t hist_blocks = ceil_div<int64_t>(n, kHistItemsPerBlock), hist_cap = (int64_t)sm_count() * 4;
+    radix_histogram_kernel<<<(unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap), kHistThreads, 0, stream>>>(keys, n, n_dev, pt, w.hist, w.ticket + kMaxPasses, w.base);
     INPC_LAUNCH_CHECK("radix_histogram_kernel");
-    radix_scan_histogram_kernel<<<pt.n_passes, kRadix, 0, stream>>>(w.hist, w.base);
-    INPC_LAUNCH_CHECK("radix_scan_histogram_kernel");
 
     PassArgs a;
     a.tiles = tiles; a.n = n; a.n_dev = n_dev; a.status = status;
     a.spin_limit = spin_limit; a.mute_tile = mute_tile;
     a.kin = keys; a.kout = keys_alt; a.vin = values; a.vout = values_alt;
+    a.state = w.state;
     for (int p = 0; p < pt.n_passes; ++p) {
         a.shift = pt.shift[p]; a.bits = pt.bits[p];
         a.base = w.base + p * kRadix;
-        a.state = w.state + (size_t)p * tiles * kRadix;
         a.ticket = w.ticket + p;
-        const int rc = launch_onesweep_pass(a, stream);
+        const int rc = items == kLargeItems ? launch_onesweep_pass<kLargeItems>(a, stream) : launch_onesweep_pass<kSmallItems>(a, stream);
         if (rc != INPC_OK) return rc;
+        a.state += (size_t)tiles * pass_bins(a.bits);
         const uint32_t* t = a.kin; a.kin = a.kout; a.kout = const_cast<uint32_t*>(t);
         t = a.vin; a.vin = a.vout; a.vout = const_cast<uint32_t*>(t);
     }
@@ -414,20 +437,20 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
     return INPC_OK;
 }
 
-int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n,
+int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
                int end_bit, void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream) {
     if (result_in_alt) *result_in_alt = 0;
     bool nothing = false;
     const int rc = check_sort_args("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, &nothing);
     if (rc != INPC_OK || nothing) return rc;
     if (!workspace) { set_error("sort_pairs: null workspace"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, workspace, status, result_in_alt, stream);
+    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n_likely), workspace, status, result_in_alt, stream);
 }
 
 // The same sort with the number of pairs in device memory (*n_dev <= n_max): grids and the look-back state are
 // sized for n_max, the kernels read the count themselves, and the result is always in the alternate buffers iff
 // the number of passes is odd.  No host synchronisation anywhere.
-int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max,
+int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
                             const unsigned long long* n_dev, int end_bit, void* workspace, unsigned* status, int* result_in_alt,
                             cudaStream_t stream) {
     if (result_in_alt) *result_in_alt = 0;
@@ -436,7 +459,7 @@ int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values
     const int rc = check_sort_args("sort_pairs", keys, keys_alt, values, values_alt, n_max < 2 ? 2 : n_max, end_bit, &nothing);
     if (rc != INPC_OK) return rc;
     if (!workspace || !n_dev) { set_error("sort_pairs: null workspace or count"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n_max, end_bit, workspace, status, result_in_alt, stream, kSpinLimit,
+    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n_max, end_bit, tile_items(n_likely), workspace, status, result_in_alt, stream, kSpinLimit,
                            0xFFFFFFFFu, n_dev);
 }
 
@@ -449,7 +472,7 @@ int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values
 namespace inpc {
 namespace {
 constexpr int64_t kStaticMaxPairs = 1 << 20;
-constexpr size_t kStaticTiles = (kStaticMaxPairs + kTile - 1) / kTile;
+constexpr size_t kStaticTiles = (kStaticMaxPairs + kLargeTile - 1) / kLargeTile;   // the static sort always takes large tiles: its scratch stays small
 constexpr size_t kStaticWorkspaceBytes = (kMaxPasses * kRadix * 4 + 256)            // histograms + tickets
                                          + kMaxPasses * kStaticTiles * kRadix * 4   // look-back state
                                          + kMaxPasses * kRadix * 4;                 // digit bases
@@ -490,9 +513,10 @@ extern "C" int inpc_sort_pairs_static(uint32_t* keys, uint32_t* keys_alt, uint32
         return INPC_E_CAPACITY;
     }
     // the hand-written size of the fixed array must be what the ordinary workspace layout needs at capacity
-    if (sort_workspace_bytes(kStaticMaxPairs) != kStaticWorkspaceBytes) {
+    const size_t needed = carve_sort_workspace(nullptr, kStaticMaxPairs, kLargeItems).total;
+    if (needed != kStaticWorkspaceBytes) {
         set_error("inpc_sort_pairs_static: fixed scratch of %zu bytes does not match the workspace layout (%zu bytes)",
-                  kStaticWorkspaceBytes, sort_workspace_bytes(kStaticMaxPairs));
+                  kStaticWorkspaceBytes, needed);
         return INPC_E_INVALID;
     }
     bool nothing = false;
@@ -504,10 +528,10 @@ extern "C" int inpc_sort_pairs_static(uint32_t* keys, uint32_t* keys_alt, uint32
     // the status words of this entry point live behind the workspace, inside the same fixed array
     unsigned* status = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(scratch) + kStaticWorkspaceBytes);
     INPC_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned) * STATUS_WORDS, stream));
-    return sort_pairs_with("inpc_sort_pairs_static", keys, keys_alt, values, values_alt, n, end_bit, scratch, status, result_in_alt, stream);
+    return sort_pairs_with("inpc_sort_pairs_static", keys, keys_alt, values, values_alt, n, end_bit, kLargeItems, scratch, status, result_in_alt, stream);
 }
 
-extern "C" size_t inpc_sort_workspace_bytes(int64_t n) { return inpc::sort_workspace_bytes(n < 0 ? 0 : n); }
+extern "C" size_t inpc_sort_workspace_bytes(int64_t n) { return inpc::sort_workspace_bytes(n < 0 ? 0 : n, n); }
 
 extern "C" int inpc_sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt,
                                int64_t n, int end_bit, void* workspace, int* result_in_alt, void* stream) {
@@ -521,7 +545,7 @@ extern "C" int inpc_sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* val
     if (rc != INPC_OK) return rc;
     unsigned* status = acquire_status("inpc_sort_pairs");
     if (!status) return INPC_E_CUDA;
-    return sort_pairs(keys, keys_alt, values, values_alt, n, end_bit, workspace, status, result_in_alt, static_cast<cudaStream_t>(stream));
+    return sort_pairs(keys, keys_alt, values, values_alt, n, n, end_bit, workspace, status, result_in_alt, static_cast<cudaStream_t>(stream));
 }
 
 // Test hook: inpc_sort_pairs with tile 0 of every pass leaving before it publishes its digit counts and a
@@ -537,7 +561,7 @@ extern "C" int inpc_debug_sort_lookback_timeout(uint32_t* keys, uint32_t* keys_a
     if (nothing || !workspace || !ticket) { set_error("inpc_debug_sort_lookback_timeout: needs n > 1, end_bit > 0, a workspace and a ticket pointer"); return INPC_E_INVALID; }
     unsigned* status = acquire_status("inpc_debug_sort_lookback_timeout", ticket);
     if (!status) return INPC_E_CUDA;
-    return sort_pairs_with("inpc_debug_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, workspace, status, nullptr,
+    return sort_pairs_with("inpc_debug_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, status, nullptr,
                            static_cast<cudaStream_t>(stream), 1 << 10, 0u);
 }
 

@@ -1036,7 +1036,7 @@ extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, cons
 
 extern "C" size_t inpc_morton_workspace_bytes(int64_t n) {
     const size_t arr = align_up(sizeof(uint32_t) * (size_t)(n > 0 ? n : 1));
-    return 4 * arr + align_up(6 * sizeof(float) * kBoxBlocks) + sort_workspace_bytes(n) + 256;
+    return 4 * arr + align_up(6 * sizeof(float) * kBoxBlocks) + sort_workspace_bytes(n, n) + 256;
 }
 
 extern "C" int inpc_morton_order(const float* positions, int64_t n, const float* box_lo, float box_extent, float* out, void* workspace,
@@ -1072,7 +1072,7 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
     }
     unsigned* status = acquire_status("inpc_morton_order");
     if (!status) return INPC_E_CUDA;
-    const int rc = sort_pairs(codes[0], codes[1], order[0], order[1], n, 30, sort_ws, status, &in_alt, stream);
+    const int rc = sort_pairs(codes[0], codes[1], order[0], order[1], n, n, 30, sort_ws, status, &in_alt, stream);
     if (rc != INPC_OK) return rc;
     gather_positions_kernel<<<(unsigned)ceil_div<int64_t>(n, kThreads), kThreads, 0, stream>>>(positions, order[in_alt], n, out);
     INPC_LAUNCH_CHECK("gather_positions_kernel");
