@@ -425,6 +425,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
             // feature rows are gathered by the blend itself: the record carries the geometry only
             *reinterpret_cast<float4*>(rec + iv) = make_float4(pr.sx, pr.sy, __ldg(opacities + i), pr.depth);
             bounds[iv] = make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16));
+            if (quad) quad[iv] = pack_quad(pr, set * rp.gh);
         } else if (pr.visible) {
             const __half* h = reinterpret_cast<const __half*>(s_feat) + threadIdx.x * kHalves;
             float b[9];
@@ -1428,11 +1429,28 @@ constexpr int kGatherDepthRest = 2;       // later segments,
 constexpr int kGatherDepthBackward = 2;   // backward pass
 constexpr int kIdsAhead = 3;      // later segments: batches whose point ids are loaded ahead of their gather
 
+// Where the features of a splat come from: the second half of its record (four view-space channels), or, for feature rows,
+// the caller's (n, 4 C4) array.  A staged row of more than four channels is padded by one float4, so that the lanes of a
+// warp, which read the same channels of different rows, meet different shared-memory banks.
+__host__ __device__ constexpr int feature_stride(int c4) { return c4 == 1 ? 1 : c4 + 1; }
+
+// Starts the copies of the feature rows of a batch (`id` of lane j: the point of staged instance j) into `ring`:
+// C4 neighbouring lanes copy the C4 16-byte pieces of one row.
+template <int C4>
+__device__ __forceinline__ void gather_rows(float4* ring, const float4* __restrict__ features, uint32_t id, unsigned lane) {
+#pragma unroll
+    for (int k = 0; k < C4; ++k) {
+        const int piece = k * 32 + (int)lane, row = piece / C4, c = piece % C4;
+        const uint32_t rid = __shfl_sync(0xffffffffu, id, row);
+        if (rid != 0xffffffffu) async_copy_16(ring + row * feature_stride(C4) + c, features + (size_t)rid * C4 + c);
+    }
+}
+
 // Shared memory of one warp of the forward passes.
-template <bool BLEND, bool WEIGHTS, int DEPTH>
+template <bool BLEND, bool WEIGHTS, int DEPTH, int C4>
 struct __align__(16) WarpForwardSmem {
     float4 ring_a[DEPTH][32];                        // records of the batches in flight: position, alpha, depth ...
-    float4 ring_f[BLEND ? DEPTH : 1][32];            // ... and features
+    float4 ring_f[BLEND ? DEPTH : 1][BLEND ? 32 * feature_stride(C4) : 1];   // ... and features
     float2 frag[kBatchFragments];                    // fragments in per-pixel order: alpha, lane of the staged instance
     float frag_seen[WEIGHTS ? kBatchFragments : 1];  // transmittance the fragment met (0: it was dropped)
     uint32_t ring_id[DEPTH][32];                     // point ids of the batches in flight (0xFFFFFFFF: no instance)
@@ -1441,17 +1459,18 @@ struct __align__(16) WarpForwardSmem {
     uint32_t queue[kQueueCap];
 };
 
-template <int PASS, int KIND>
+template <int PASS, int KIND, int C4>
 constexpr size_t warp_forward_smem_bytes() {
     return 256 * sizeof(unsigned long long) +
            kWarpBlendWarps * sizeof(WarpForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN,
-                                                    PASS == PASS_REST ? kGatherDepthRest : kGatherDepthFilter>);
+                                                    PASS == PASS_REST ? kGatherDepthRest : kGatherDepthFilter, C4>);
 }
 
-template <int PASS, int KIND>
-__global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4 : 3) blend_bilinear_warp_forward_kernel(
+// ROWS: features are rows of 4 C4 channels in `rows` (a (4 C4, H, W) image); otherwise C4 is 1 and they are in the record.
+template <int PASS, int KIND, int C4, bool ROWS>
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4 : C4 == 8 ? 2 : 3) blend_bilinear_warp_forward_kernel(
     const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, const uint32_t* __restrict__ inst_keys,
-    const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, float* __restrict__ seg_T, float4* __restrict__ seg_C,
+    const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ rows, float* __restrict__ seg_T, float4* __restrict__ seg_C,
     float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1,
     uint32_t* __restrict__ n_kept, int width, int height, int gw, int gh) {
@@ -1461,7 +1480,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
     constexpr bool kWeights = kBlend && KIND == BLEND_TRAIN;
     constexpr bool kDepth = kBlend && KIND == BLEND_INFER;
     constexpr int kGatherDepth = PASS == PASS_REST ? kGatherDepthRest : kGatherDepthFilter;
-    using Smem = WarpForwardSmem<kBlend, kWeights, kGatherDepth>;
+    constexpr int kStride = feature_stride(C4);
+    static_assert(ROWS || C4 == 1, "a record holds four channels");
+    using Smem = WarpForwardSmem<kBlend, kWeights, kGatherDepth, C4>;
     extern __shared__ __align__(16) unsigned char blend_smem[];
     unsigned long long* s_reach = reinterpret_cast<unsigned long long*>(blend_smem);     // key code -> pixels reached
     Smem& sm = reinterpret_cast<Smem*>(blend_smem + 256 * sizeof(unsigned long long))[threadIdx.x >> 5];
@@ -1503,7 +1524,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
         const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
         const bool inside = px < width && py < height;
 
-        float Tr = 1.0f, Z = 0.0f, C0 = 0.0f, C1 = 0.0f, C2 = 0.0f, C3 = 0.0f;
+        float Tr = 1.0f, Z = 0.0f;
+        float4 C[C4];
+#pragma unroll
+        for (int c = 0; c < C4; ++c) C[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         double log_sum = 0.0, log_stop = 0.0;   // PRODUCT: -log2 of the product so far, and where the pixel counts as stopped
         bool done = !inside;
         if (PASS == PASS_PRODUCT) {
@@ -1576,8 +1600,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                     id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(q_head + lane) & (kQueueCap - 1)]);
                     const float4* p = reinterpret_cast<const float4*>(rec + id);
                     async_copy_16(&sm.ring_a[stage][lane], p);
-                    if (kBlend) async_copy_16(&sm.ring_f[stage][lane], p + 1);
+                    if (kBlend && !ROWS) async_copy_16(&sm.ring_f[stage][lane], p + 1);
                 }
+                if (kBlend && ROWS) gather_rows<C4>(sm.ring_f[stage], rows, id, lane);
                 sm.ring_id[stage][lane] = id;
                 async_copy_commit();   // one group per batch, empty or not: the waits below count groups
                 if (PASS == PASS_REST) {
@@ -1597,6 +1622,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
             for (unsigned batch = 0;; ++batch) {
                 gather((batch + kGatherDepth - 1) & (kGatherDepth - 1));
                 async_copy_wait<kGatherDepth - 1>();   // all but the newest kGatherDepth - 1 groups: this batch has arrived
+                if (ROWS) __syncwarp();                // a row was copied by several lanes
                 const unsigned stage = batch & (kGatherDepth - 1);
                 const uint32_t id_cur = sm.ring_id[stage][lane];
                 const bool staged = id_cur != kNoInstance;
@@ -1684,13 +1710,15 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                     float a[kChunk];
                     float4 f[kChunk];
                     float zd[kChunk];
+                    unsigned from[kChunk];
 #pragma unroll
                     for (int u = 0; u < kChunk; ++u) {
                         const unsigned k = min(k0 + u, off + cnt - 1u);   // the tail repeats the last slot: masked out below
                         const float2 e = sm.frag[k];
                         a[u] = e.x;
-                        if (kBlend) f[u] = sm.ring_f[stage][__float_as_uint(e.y)];
-                        if (kDepth) zd[u] = sm.ring_a[stage][__float_as_uint(e.y)].w;
+                        from[u] = __float_as_uint(e.y);
+                        if (kBlend && C4 == 1) f[u] = sm.ring_f[stage][from[u]];
+                        if (kDepth) zd[u] = sm.ring_a[stage][from[u]].w;
                     }
 #pragma unroll
                     for (int u = 0; u < kChunk; ++u) {
@@ -1698,10 +1726,20 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                         if (kBlend) {
                             const float bw = Tr * a[u];
                             if (kWeights && k0 + u < off + cnt) sm.frag_seen[k0 + u] = live ? Tr : 0.0f;
-                            C0 = live ? C0 + bw * f[u].x : C0;
-                            C1 = live ? C1 + bw * f[u].y : C1;
-                            C2 = live ? C2 + bw * f[u].z : C2;
-                            C3 = live ? C3 + bw * f[u].w : C3;
+                            if (C4 == 1) {
+                                C[0].x = live ? C[0].x + bw * f[u].x : C[0].x;
+                                C[0].y = live ? C[0].y + bw * f[u].y : C[0].y;
+                                C[0].z = live ? C[0].z + bw * f[u].z : C[0].z;
+                                C[0].w = live ? C[0].w + bw * f[u].w : C[0].w;
+                            } else if (live) {
+                                // wide rows are read where they are used: a chunk of them would not fit the registers
+                                const float4* row = sm.ring_f[stage] + from[u] * kStride;
+#pragma unroll
+                                for (int c = 0; c < C4; ++c) {
+                                    const float4 v = row[c];
+                                    C[c].x += bw * v.x; C[c].y += bw * v.y; C[c].z += bw * v.z; C[c].w += bw * v.w;
+                                }
+                            }
                             if (kDepth) Z = live ? Z + bw * zd[u] : Z;
                             Tr = live ? Tr * (1.0f - a[u]) : Tr;
                             done = done || Tr < kTransmittanceEps;
@@ -1741,10 +1779,14 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
         float* alpha_s = alpha_image + (int64_t)set * n_px;
         if (n_seg == 1u) {
             if (inside) {
-                image_s[pi] = C0;
-                image_s[n_px + pi] = C1;
-                image_s[2 * n_px + pi] = C2;
-                image_s[3 * n_px + pi] = C3;
+#pragma unroll
+                for (int c = 0; c < C4; ++c) {
+                    float* plane = image_s + (int64_t)(4 * c) * n_px + pi;
+                    plane[0] = C[c].x;
+                    plane[n_px] = C[c].y;
+                    plane[2 * n_px] = C[c].z;
+                    plane[3 * n_px] = C[c].w;
+                }
                 if (KIND == BLEND_INFER) {
                     const float A = 1.0f - Tr;
                     depth_image[(int64_t)set * n_px + pi] = A > 0.0f ? Z / A : 0.0f;
@@ -1756,7 +1798,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
         } else {
             // partial colour of this segment; the per-tile combine adds the segments up in order
             const size_t si = sidx * 32 + lane;
-            seg_C[si] = make_float4(C0, C1, C2, C3);
+#pragma unroll
+            for (int c = 0; c < C4; ++c) seg_C[(sidx * C4 + c) * 32 + lane] = C[c];
             if (PASS == PASS_FIRST) seg_T[si] = Tr;   // the exact state behind segment 0
             if (KIND == BLEND_INFER) {
                 seg_Z[si] = Z;
@@ -1799,7 +1842,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel
 // For training the running sum before each segment replaces the segment's own colour (the backward pass
 // starts from it).  Inference: expected depth, and the transmittance where the pixel stopped = the end value
 // of the first segment that fell below the threshold.
-template <int KIND>
+template <int KIND, int C4>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kernel(
     const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts, float4* __restrict__ seg_C, const float* __restrict__ seg_Z,
     const float* __restrict__ seg_E,
@@ -1816,38 +1859,49 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
         const int px = tx * 8 + (int)(lane & 7u);
         const int py = ty * 8 + 4 * (int)half + (int)(lane >> 3);
         const size_t base = ((size_t)first * 2u + half) * 32 + lane;   // segment g of this half: base + g * 64
-        float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
-        float z = 0.0f, t_final = 1.0f;
-        bool stopped = false;
-        for (unsigned g0 = 0; g0 < n_seg; g0 += 4) {
-            float4 c[4];
-            float zz[4], ee[4];
+        const bool inside = px < width && py < height;
+        const int64_t n_px = (int64_t)width * height;
+        const int64_t pi = (int64_t)py * width + px;
+        float* image_s = image + (int64_t)set * 4 * n_px;
+        for (int ch = 0; ch < C4; ++ch) {
+            float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4* part = seg_C + (((size_t)first * 2u + half) * C4 + ch) * 32 + lane;   // segment g: part + g * 64 C4
+            for (unsigned g0 = 0; g0 < n_seg; g0 += 4) {
+                float4 c[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const bool ok = g0 + k < n_seg;
-                const size_t si = base + (size_t)(g0 + k) * 64;
-                c[k] = ok ? seg_C[si] : make_float4(0.f, 0.f, 0.f, 0.f);
-                zz[k] = (KIND == BLEND_INFER && ok) ? seg_Z[si] : 0.0f;
-                ee[k] = (KIND == BLEND_INFER && ok) ? seg_E[si] : 1.0f;
+                for (int k = 0; k < 4; ++k) c[k] = g0 + k < n_seg ? part[(size_t)(g0 + k) * (64 * C4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (KIND == BLEND_TRAIN && g0 + k < n_seg) part[(size_t)(g0 + k) * (64 * C4)] = run;
+                    run.x += c[k].x; run.y += c[k].y; run.z += c[k].z; run.w += c[k].w;
+                }
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const bool ok = g0 + k < n_seg;
-                if (KIND == BLEND_TRAIN && ok) seg_C[base + (size_t)(g0 + k) * 64] = run;
-                run.x += c[k].x; run.y += c[k].y; run.z += c[k].z; run.w += c[k].w;
-                z += zz[k];
-                if (KIND == BLEND_INFER && ok && !stopped) { t_final = ee[k]; stopped = t_final < kTransmittanceEps; }
+            if (inside) {
+                float* plane = image_s + (int64_t)(4 * ch) * n_px + pi;
+                plane[0] = run.x;
+                plane[n_px] = run.y;
+                plane[2 * n_px] = run.z;
+                plane[3 * n_px] = run.w;
             }
         }
-        if (px < width && py < height) {
-            const int64_t n_px = (int64_t)width * height;
-            const int64_t pi = (int64_t)py * width + px;
-            float* image_s = image + (int64_t)set * 4 * n_px;
-            image_s[pi] = run.x;
-            image_s[n_px + pi] = run.y;
-            image_s[2 * n_px + pi] = run.z;
-            image_s[3 * n_px + pi] = run.w;
-            if (KIND == BLEND_INFER) {
+        if (KIND == BLEND_INFER) {
+            float z = 0.0f, t_final = 1.0f;
+            bool stopped = false;
+            for (unsigned g0 = 0; g0 < n_seg; g0 += 4) {
+                float zz[4], ee[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const bool ok = g0 + k < n_seg;
+                    zz[k] = ok ? seg_Z[base + (size_t)(g0 + k) * 64] : 0.0f;
+                    ee[k] = ok ? seg_E[base + (size_t)(g0 + k) * 64] : 1.0f;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    z += zz[k];
+                    if (g0 + k < n_seg && !stopped) { t_final = ee[k]; stopped = t_final < kTransmittanceEps; }
+                }
+            }
+            if (inside) {
                 const float A = 1.0f - t_final;
                 depth_image[(int64_t)set * n_px + pi] = A > 0.0f ? z / A : 0.0f;
                 alpha_image[(int64_t)set * n_px + pi] = t_final < kTransmittanceEps ? 1.0f : A;
@@ -2072,6 +2126,234 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
                     e[0] = sf;
                     e[1] = make_float4(so, 0.0f, 0.0f, 0.0f);
                     atomicOr(slot_mask + id_cur, 1u << slot_of_point);
+                }
+            }
+            done_w = __ballot_sync(kFull, done);
+            __syncwarp();
+            if (done_w == kFull) break;
+        }
+        async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
+        __syncwarp();
+    }
+}
+
+// Backward pass over feature rows, the walk and the lists of the kernel above.  Per fragment only scalars are kept: with
+// G = <g, .> over the channels, dL/dalpha = Tr * G(f) + (G(C_run) - G(C_final)) / (1 - alpha) + K / (1 - alpha), and
+// G(C_run) is a running scalar.  The pixel lanes leave a fragment's blending weight and dL/dalpha in shared memory; the
+// gradient of a point's row, sum over its pixels of weight * g, is then formed per instance with every staged lane busy.
+// A splat whose 2x2 pixels all lie in this 8x4 half has no other writer in the launch and stores its row; the others
+// (about a third) add theirs with one vector atomic per four channels.
+template <int C4>
+struct __align__(16) RowsBackwardSmem {
+    float4 ring_a[kGatherDepthBackward][32];
+    float4 ring_f[kGatherDepthBackward][32 * feature_stride(C4)];
+    float4 pixel_grad[32 * feature_stride(C4)];   // image gradient of the half's pixels
+    float2 frag[kBatchFragments];                 // fragments in per-pixel order: alpha, lane of the staged instance
+    float2 frag_out[kBatchFragments];             // ... and what the pixel lane made of them: blending weight, dL/dalpha
+    uint32_t ring_id[kGatherDepthBackward][32];
+    unsigned mask[32];
+    unsigned off[32];
+};
+template <int C4>
+constexpr size_t rows_warp_backward_smem_bytes() { return kWarpBlendWarps * sizeof(RowsBackwardSmem<C4>); }
+
+template <int C4>
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_rows_warp_backward_kernel(
+    const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
+    unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0,
+    const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept, const PointRec* __restrict__ rec, const float4* __restrict__ rows,
+    const float* __restrict__ seg_T, const float4* __restrict__ seg_C, const float* __restrict__ grad_image,
+    const float* __restrict__ grad_alpha, const float* __restrict__ image, const float* __restrict__ alpha_image,
+    float4* __restrict__ grad_rows, float* __restrict__ grad_opacity, int width, int height, int gw) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr unsigned kNoInstance = 0xffffffffu;
+    constexpr int kGatherDepth = kGatherDepthBackward;
+    constexpr int kStride = feature_stride(C4);
+    extern __shared__ __align__(16) unsigned char blend_smem[];
+    const unsigned lane = lane_id();
+    const unsigned lt_mask = (1u << lane) - 1u;
+    RowsBackwardSmem<C4>& sm = reinterpret_cast<RowsBackwardSmem<C4>*>(blend_smem)[threadIdx.x >> 5];
+    sm.mask[lane] = 0u;
+    __syncwarp();
+    const unsigned n_first = __ldg(counts) * 2u;
+    const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
+    const unsigned n_rest = n_items - n_first;
+    const int64_t n_px = (int64_t)width * height;
+
+    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));
+    unsigned next_item = 0, visit_end = 0;
+    for (;;) {
+        if (next_item == visit_end) {
+            unsigned first_item = 0;
+            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
+            first_item = __shfl_sync(kFull, first_item, 0);
+            if (first_item >= n_items) break;
+            next_item = first_item;
+            visit_end = min(first_item + per_visit, n_items);
+        }
+        const unsigned item = next_item++;
+        const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
+        const int half = (int)((item < n_rest ? item : item - n_rest) & 1u);
+        const unsigned n_list = __ldg(n_kept + (size_t)(it.first + it.seg) * 2u + half);
+        const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg;
+        const size_t sidx = (size_t)(it.first + seg) * 2u + half;
+        if (n_list == 0u) continue;
+        const uint32_t* list = (half ? kept1 : kept0) + it.begin;
+        const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
+        const int px0 = tx * 8, py0 = ty * 8 + 4 * half;
+        const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+
+        float4 g[C4];
+        float G_final = 0.0f, G_run = 0.0f, K = 0.0f, Tr = 1.0f;
+        bool done = !(px < width && py < height);
+#pragma unroll
+        for (int c = 0; c < C4; ++c) g[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!done) {
+            const int64_t pi = (int64_t)py * width + px;
+#pragma unroll
+            for (int c = 0; c < C4; ++c) {
+                const float* gp = grad_image + (int64_t)(4 * c) * n_px + pi;
+                const float* ip = image + (int64_t)(4 * c) * n_px + pi;
+                g[c] = make_float4(__ldg(gp), __ldg(gp + n_px), __ldg(gp + 2 * n_px), __ldg(gp + 3 * n_px));
+                G_final += __ldg(ip) * g[c].x + __ldg(ip + n_px) * g[c].y + __ldg(ip + 2 * n_px) * g[c].z + __ldg(ip + 3 * n_px) * g[c].w;
+            }
+            K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
+            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
+            if (n_seg > 1u) {
+#pragma unroll
+                for (int c = 0; c < C4; ++c) {
+                    const float4 v = seg_C[(sidx * C4 + c) * 32 + lane];
+                    G_run += v.x * g[c].x + v.y * g[c].y + v.z * g[c].z + v.w * g[c].w;
+                }
+            }
+            done = Tr < kTransmittanceEps;
+        }
+        __syncwarp();   // the previous item's readers of pixel_grad are through
+#pragma unroll
+        for (int c = 0; c < C4; ++c) sm.pixel_grad[lane * kStride + c] = g[c];
+        unsigned done_w = __ballot_sync(kFull, done);
+
+        uint32_t idf[kIdsAhead];
+#pragma unroll
+        for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < n_list ? __ldg(list + 32u * k + lane) : 0u;
+        unsigned issued = 0;
+        auto gather = [&](unsigned stage) {
+            const unsigned n = min(32u, n_list - issued);
+            uint32_t id = kNoInstance;
+            if (lane < n) {
+                id = checked_point(idf[0]);
+                async_copy_16(&sm.ring_a[stage][lane], reinterpret_cast<const float4*>(rec + id));
+            }
+            gather_rows<C4>(sm.ring_f[stage], rows, id, lane);
+            sm.ring_id[stage][lane] = id;
+            async_copy_commit();   // one group per batch, empty or not
+#pragma unroll
+            for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
+            const unsigned nxt = issued + 32u * kIdsAhead + lane;
+            idf[kIdsAhead - 1] = nxt < n_list ? __ldg(list + nxt) : 0u;
+            issued += n;
+        };
+#pragma unroll
+        for (int st = 0; st + 1 < kGatherDepth; ++st) gather((unsigned)st);
+        for (unsigned batch = 0;; ++batch) {
+            gather((batch + kGatherDepth - 1) & (kGatherDepth - 1));
+            async_copy_wait<kGatherDepth - 1>();
+            __syncwarp();   // a row was copied by several lanes
+            const unsigned stage = batch & (kGatherDepth - 1);
+            const uint32_t id_cur = sm.ring_id[stage][lane];
+            const bool staged = id_cur != kNoInstance;
+            if (__ballot_sync(kFull, staged) == 0u) break;
+            const float4 a_cur = sm.ring_a[stage][lane];
+            // ---- lane j: the fragments of staged instance j
+            const int qx = __float2int_rd(a_cur.x - 0.5f) - px0;
+            const int qy = __float2int_rd(a_cur.y - 0.5f) - py0;
+            float al[4], wg[4];
+            int pix[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int cx = qx + (c & 1), cy = qy + (c >> 1);
+                const float pcx = (float)(px0 + cx) + 0.5f, pcy = (float)(py0 + cy) + 0.5f;
+                const float dx = fabsf(a_cur.x - pcx), dy = fabsf(a_cur.y - pcy);
+                wg[c] = __saturatef(1.0f - dx) * __saturatef(1.0f - dy);
+                al[c] = a_cur.z * wg[c];
+                const int p = cy * 8 + cx;
+                const bool ok = staged && cx >= 0 && cx < 8 && cy >= 0 && cy < 4 && dx < 1.0f && dy < 1.0f &&
+                                !((done_w >> (p & 31)) & 1u);
+                pix[c] = ok ? p : -1;
+                if (ok) atomicOr(sm.mask + p, 1u << lane);
+            }
+            __syncwarp();
+            const unsigned my_mask = sm.mask[lane];
+            const unsigned cnt = __popc(my_mask);
+            const unsigned off = warp_inclusive_scan(cnt) - cnt;
+            sm.off[lane] = off;
+            __syncwarp();
+            int slot[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                slot[c] = 0;
+                if (pix[c] >= 0) {
+                    slot[c] = (int)(sm.off[pix[c]] + __popc(sm.mask[pix[c]] & lt_mask));
+                    sm.frag[slot[c]] = make_float2(al[c], __uint_as_float(lane));
+                }
+            }
+            __syncwarp();
+            if (my_mask) sm.mask[lane] = 0u;
+            for (unsigned k = off; k < off + cnt; ++k) {
+                const float2 e = sm.frag[k];
+                float2 out = make_float2(0.0f, 0.0f);
+                if (!done) {
+                    const float4* row = sm.ring_f[stage] + __float_as_uint(e.y) * kStride;
+                    float fg = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < C4; ++c) {
+                        const float4 f = row[c];
+                        fg += f.x * g[c].x + f.y * g[c].y + f.z * g[c].z + f.w * g[c].w;
+                    }
+                    const float bw = Tr * e.x;
+                    G_run += bw * fg;
+                    const float oma = 1.0f - e.x;
+                    const float rcp = 1.0f / fmaxf(oma, kOneMinusAlphaEps);
+                    out = make_float2(bw, Tr * fg + (G_run - G_final) * rcp + K * rcp);
+                    Tr *= oma;
+                    done = Tr < kTransmittanceEps;
+                }
+                sm.frag_out[k] = out;
+            }
+            __syncwarp();
+            if (staged) {
+                float bw[4], so = 0.0f;
+                bool any = false;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    bw[c] = 0.0f;
+                    if (pix[c] >= 0) {
+                        const float2 o = sm.frag_out[slot[c]];
+                        bw[c] = o.x;
+                        so += o.y * wg[c];
+                        any = any || o.x != 0.0f;
+                    }
+                }
+                const bool alone = qx >= 0 && qx < 7 && qy >= 0 && qy < 3;   // all four pixels in this half
+                if (any) {
+                    float4* dst = grad_rows + (size_t)id_cur * C4;
+#pragma unroll
+                    for (int c = 0; c < C4; ++c) {
+                        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            if (bw[q] != 0.0f) {
+                                const float4 v = sm.pixel_grad[pix[q] * kStride + c];
+                                sum.x += bw[q] * v.x; sum.y += bw[q] * v.y; sum.z += bw[q] * v.z; sum.w += bw[q] * v.w;
+                            }
+                        }
+                        if (alone) dst[c] = sum;
+                        else if (sum.x != 0.0f || sum.y != 0.0f || sum.z != 0.0f || sum.w != 0.0f) atomicAdd(dst + c, sum);
+                    }
+                }
+                if (so != 0.0f) {
+                    if (alone) grad_opacity[id_cur] = so;
+                    else atomicAdd(grad_opacity + id_cur, so);
                 }
             }
             done_w = __ballot_sync(kFull, done);
@@ -2886,18 +3168,18 @@ int64_t max_segments(int64_t n_instances, int n_tiles, int tile) {
 }
 
 // Which of the two blend organisations a call uses: one warp per tile part with the dead-instance filter
-// (bilinear splats, 8x8 tiles, four view-space channels) or one block per (tile, segment).
+// (bilinear splats, 8x8 tiles) or one block per (tile, segment).
 constexpr int kWarpBlendParts = 2;   // work items per (tile, segment): the two 8x4 halves
-bool uses_warp_blend(int mode, int tile, bool rows) { return mode == INPC_MODE_BILINEAR && tile == 8 && !rows; }
+bool uses_warp_blend(int mode, int tile) { return mode == INPC_MODE_BILINEAR && tile == 8; }
 
 // The warp-blend path sizes its arrays for 4 instances per point; most splats touch one tile of four or none twice, about 1.3
 // on average (2^23 samples at 1237x822: 1.26; at 3840x2160 less).  Only picks tile sizes.
 int64_t likely_instances(int64_t capacity, bool deferred) { return deferred ? capacity / 3 : capacity; }
 
-InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int tile, int mode, bool with_depth, int c4 = 1, bool rows = false) {
+InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int tile, int mode, bool with_depth, int c4 = 1) {
     InstanceBlob b;
     Carver c(p);
-    const bool warp_blend = uses_warp_blend(mode, tile, rows);
+    const bool warp_blend = uses_warp_blend(mode, tile);
     b.ranges = c.take<uint2>(n_tiles);
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n_instances);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n_instances);
@@ -3032,8 +3314,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     }
     unsigned* status = acquire_status(entry);
     if (!status) return INPC_E_CUDA;
-    constexpr bool kRows = VARIANT == VAR_ROWS;
-    const bool warp_blend = uses_warp_blend(MODE, rp.tile, kRows);
+    const bool warp_blend = uses_warp_blend(MODE, rp.tile);
     const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
     const PointBlob sizing = carve_point_blob(nullptr, n, MODE);
     void* pblob = alloc_point(user, sizing.total);
@@ -3121,10 +3402,10 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         return INPC_E_CAPACITY;
     }
 
-    const InstanceBlob isz = carve_instance_blob(nullptr, n_instances, n_tiles, rp.tile, MODE, with_depth, c4, kRows);
+    const InstanceBlob isz = carve_instance_blob(nullptr, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
     void* iblob = alloc_instance(user, isz.total);
     if (!iblob) { set_error("instance allocator returned NULL for %zu bytes", isz.total); return INPC_E_ALLOC; }
-    InstanceBlob ib = carve_instance_blob(iblob, n_instances, n_tiles, rp.tile, MODE, with_depth, c4, kRows);
+    InstanceBlob ib = carve_instance_blob(iblob, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
     INPC_CUDA_TRY(cudaMemsetAsync(ib.ranges, 0, sizeof(uint2) * (size_t)n_tiles, stream));
 
     int in_alt = 0;
@@ -3229,6 +3510,7 @@ int warp_blend_grid(unsigned* grid) {
 struct ForwardPassArgs {
     const uint32_t *keys, *ids;
     const PointRec* rec;
+    const float4* rows;   // feature rows, or nullptr
     float* seg_T;
     float4* seg_C;
     float *seg_Z, *seg_E, *image, *depth, *alpha, *blending_weights;
@@ -3237,22 +3519,23 @@ struct ForwardPassArgs {
 };
 
 // One pass of the warp blend's forward: its shared memory (the per-warp rings) is above the 48 KB a kernel gets unasked.
-template <int PASS, int KIND>
+template <int PASS, int KIND, int C4, bool ROWS>
 int launch_warp_forward_pass(unsigned grid, const WarpItem* items, const uint32_t* counts, unsigned* ticket, const ForwardPassArgs& a,
                              cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
-    constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND>();
-    const int rc = opt_in_dynamic_smem(blend_bilinear_warp_forward_kernel<PASS, KIND>, smem, attr_set);
+    constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
+    const int rc = opt_in_dynamic_smem(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    blend_bilinear_warp_forward_kernel<PASS, KIND><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
-        items, counts, ticket, a.keys, a.ids, a.rec, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
+    blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
+        items, counts, ticket, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, a.gh);
     INPC_LAUNCH_CHECK("blend_bilinear_warp_forward_kernel");
     return INPC_OK;
 }
 
-template <int KIND>
-int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image,
+// C4, `rows`: feature rows of 4 C4 channels (ROWS), or one group of four channels in the records.
+template <int KIND, int C4 = 1, bool ROWS = false>
+int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float4* rows, float* image,
                                  float* depth, float* alpha, float* blending_weights, cudaStream_t stream) {
     unsigned grid = 1;
     const int rc = warp_blend_grid(&grid);
@@ -3260,7 +3543,7 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const int W = rp.v.width, H = rp.v.height;
     // tiles without instances are not work items: their pixels are cleared here
     const size_t n_px = (size_t)W * H * rp.n_sets;
-    INPC_CUDA_TRY(cudaMemsetAsync(image, 0, sizeof(float) * 4 * n_px, stream));
+    INPC_CUDA_TRY(cudaMemsetAsync(image, 0, sizeof(float) * 4 * C4 * n_px, stream));
     INPC_CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(float) * n_px, stream));
     if (KIND == BLEND_INFER) INPC_CUDA_TRY(cudaMemsetAsync(depth, 0, sizeof(float) * n_px, stream));
     // the ping-pong buffers the tile sort left unused receive the compacted lists (part 0: ids, part 1: keys)
@@ -3269,17 +3552,17 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     uint32_t* kept0 = ib.ids[1 - t_alt];
     uint32_t* kept1 = ib.keys[1 - t_alt];
     const unsigned threads = kWarpBlendWarps * 32;
-    const ForwardPassArgs a{keys, ids, pb.rec, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
+    const ForwardPassArgs a{keys, ids, pb.rec, rows, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             kept0, kept1, ib.n_kept, W, H, rp.gw, rp.gh};
-    int rc_pass = launch_warp_forward_pass<PASS_FIRST, KIND>(grid, ib.items0, ib.n_segments, ib.n_segments + 2, a, stream);
+    int rc_pass = launch_warp_forward_pass<PASS_FIRST, KIND, C4, ROWS>(grid, ib.items0, ib.n_segments, ib.n_segments + 2, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
+    rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, false>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     warp_blend_prefix_kernel<<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
-    rc_pass = launch_warp_forward_pass<PASS_REST, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
+    rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    warp_blend_combine_kernel<KIND><<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E,
+    warp_blend_combine_kernel<KIND, C4><<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E,
                                                                       image, depth, alpha, W, H, rp.gw, rp.gh);
     INPC_LAUNCH_CHECK("warp_blend_combine_kernel");
     return INPC_OK;
@@ -3369,7 +3652,7 @@ int launch_blend_forward(int mode, const RasterParams& rp, const PointBlob& pb, 
     const uint32_t* ids = ib.ids[t_alt];
     StageScope scope(STAGE_BLEND_FWD, stream);
     if (mode == INPC_MODE_BILINEAR) {
-        if (rp.tile == 8) return launch_bilinear_warp_forward<KIND>(rp, pb, ib, t_alt, image, depth, alpha, blending_weights, stream);
+        if (rp.tile == 8) return launch_bilinear_warp_forward<KIND>(rp, pb, ib, t_alt, nullptr, image, depth, alpha, blending_weights, stream);
         return launch_bilinear_forward<16, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, stream);
     }
     if (rp.tile == 8) return launch_gaussian_forward<8, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, threshold, stream);
@@ -3379,6 +3662,7 @@ int launch_blend_forward(int mode, const RasterParams& rp, const PointBlob& pb, 
 template <int T, int C4, int KIND>
 int launch_rows_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, const uint32_t* ids, const float* features,
                         float* image, float* depth, float* alpha, float* blending_weights, cudaStream_t stream) {
+    static_assert(T == 16, "8x8 tiles take the warp blend");
     constexpr size_t smem = rows_forward_smem_bytes<T, C4>();
     static bool attr_set[kMaxDevices] = {false};
     {
@@ -3401,6 +3685,26 @@ int launch_rows_forward(const RasterParams& rp, const PointBlob& pb, const Insta
     return INPC_OK;
 }
 
+template <int C4>
+int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* features,
+                              const float* grad_image, const float* grad_alpha, const float* image, const float* alpha,
+                              float* grad_features, float* grad_opacities, cudaStream_t stream) {
+    unsigned grid = 1;
+    const int rc = warp_blend_grid(&grid);
+    if (rc != INPC_OK) return rc;
+    INPC_CUDA_TRY(cudaMemsetAsync(ib.n_segments + 5, 0, sizeof(uint32_t), stream));   // the work ticket
+    static bool attr_set[kMaxDevices] = {false};
+    constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
+    const int rc_attr = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
+    if (rc_attr != INPC_OK) return rc_attr;
+    blend_rows_warp_backward_kernel<C4><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
+        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
+        reinterpret_cast<const float4*>(features), ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha,
+        reinterpret_cast<float4*>(grad_features), grad_opacities, rp.v.width, rp.v.height, rp.gw);
+    INPC_LAUNCH_CHECK("blend_rows_warp_backward_kernel");
+    return INPC_OK;
+}
+
 template <int T, int C4>
 int launch_rows_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, const uint32_t* ids, const float* features,
                          const float* grad_image, const float* grad_alpha, const float* image, const float* alpha,
@@ -3418,21 +3722,14 @@ int launch_rows_backward(const RasterParams& rp, const PointBlob& pb, const Inst
     return INPC_OK;
 }
 
-// Tile edge and channel count are template parameters of the kernels: one switch for all of them.
+// The channel count is a template parameter of the kernels: one switch for all of them.
 template <typename F>
-int dispatch_rows(int tile, int channels, F&& f) {
-    if (tile == 8) {
-        if (channels == 4) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 1>());
-        if (channels == 8) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 2>());
-        if (channels == 16) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 4>());
-        if (channels == 32) return f(std::integral_constant<int, 8>(), std::integral_constant<int, 8>());
-    } else if (tile == 16) {
-        if (channels == 4) return f(std::integral_constant<int, 16>(), std::integral_constant<int, 1>());
-        if (channels == 8) return f(std::integral_constant<int, 16>(), std::integral_constant<int, 2>());
-        if (channels == 16) return f(std::integral_constant<int, 16>(), std::integral_constant<int, 4>());
-        if (channels == 32) return f(std::integral_constant<int, 16>(), std::integral_constant<int, 8>());
-    }
-    set_error("feature rows: channels must be 4, 8, 16 or 32 (got %d) and tile_size 8 or 16 (got %d)", channels, tile);
+int dispatch_rows(int channels, F&& f) {
+    if (channels == 4) return f(std::integral_constant<int, 1>());
+    if (channels == 8) return f(std::integral_constant<int, 2>());
+    if (channels == 16) return f(std::integral_constant<int, 4>());
+    if (channels == 32) return f(std::integral_constant<int, 8>());
+    set_error("feature rows: channels must be 4, 8, 16 or 32 (got %d)", channels);
     return INPC_E_INVALID;
 }
 
@@ -3446,11 +3743,14 @@ int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* p
     int rc = run_front<INPC_MODE_BILINEAR, VAR_ROWS>(rp, n, positions, nullptr, opacities, alloc_point, alloc_instance, alloc_user, state,
                                                      KIND == BLEND_INFER, &pb, &ib, stream, KIND == BLEND_INFER ? "inpc_render_rows" : "inpc_rasterize_rows_forward", channels / 4);
     if (rc != INPC_OK) return rc;
-    const uint32_t* ids = ib.ids[tile_buffer_of(state, rp.gw * rp.gh)];
+    const int t_alt = tile_buffer_of(state, rp.gw * rp.gh);
     {
         StageScope scope(STAGE_BLEND_FWD, stream);
-        rc = dispatch_rows(tile_size, channels, [&](auto t, auto c4) {
-            return launch_rows_forward<decltype(t)::value, decltype(c4)::value, KIND>(rp, pb, ib, ids, features, image, depth, alpha, blending_weights, stream);
+        rc = dispatch_rows(channels, [&](auto c4) {
+            constexpr int kC4 = decltype(c4)::value;
+            if (tile_size == 8)
+                return launch_bilinear_warp_forward<KIND, kC4, true>(rp, pb, ib, t_alt, reinterpret_cast<const float4*>(features), image, depth, alpha, blending_weights, stream);
+            return launch_rows_forward<16, kC4, KIND>(rp, pb, ib, ib.ids[t_alt], features, image, depth, alpha, blending_weights, stream);
         });
     }
     return rc != INPC_OK ? rc : end_index_checks(stream);
@@ -3512,7 +3812,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     const int W = rp.v.width, H = rp.v.height;
     // the caller's scratch holds 33 floats per point: four 32-byte slot records and one mask word for the warp blend
     // or, for the other paths, the (n,4) accumulation buffer of their atomics
-    const bool slots = uses_warp_blend(state->mode, state->tile_size, false);
+    const bool slots = uses_warp_blend(state->mode, state->tile_size);
     if (slots && (reinterpret_cast<uintptr_t>(grad_features_view) & 31u)) {
         set_error("inpc_rasterize_backward: grad_features_view must be 32-byte aligned");
         return INPC_E_INVALID;
@@ -3712,17 +4012,19 @@ extern "C" int inpc_rasterize_rows_backward(const inpc_raster_state* state, cons
     const RasterParams rp = make_params(view, state->tile_size, 0.0f, 3.0f, nullptr);
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode);
-    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), n_tiles, state->tile_size, state->mode, false, channels / 4, true);
-    const uint32_t* ids = ib.ids[tile_buffer_of(state, n_tiles)];
+    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), n_tiles, state->tile_size, state->mode, false, channels / 4);
+    const int t_alt = tile_buffer_of(state, n_tiles);
     INPC_CUDA_TRY(cudaMemsetAsync(grad_features, 0, sizeof(float) * (size_t)n * channels, stream));
     INPC_CUDA_TRY(cudaMemsetAsync(grad_opacities, 0, sizeof(float) * (size_t)n, stream));
     rc = begin_index_checks(n, stream);
     if (rc != INPC_OK) return rc;
     {
         StageScope scope(STAGE_BLEND_BWD, stream);
-        rc = dispatch_rows(state->tile_size, channels, [&](auto t, auto c4) {
-            return launch_rows_backward<decltype(t)::value, decltype(c4)::value>(rp, pb, ib, ids, features, grad_image, grad_alpha, image, alpha,
-                                                                                grad_features, grad_opacities, stream);
+        rc = dispatch_rows(channels, [&](auto c4) {
+            constexpr int kC4 = decltype(c4)::value;
+            if (state->tile_size == 8)
+                return launch_rows_warp_backward<kC4>(rp, pb, ib, t_alt, features, grad_image, grad_alpha, image, alpha, grad_features, grad_opacities, stream);
+            return launch_rows_backward<16, kC4>(rp, pb, ib, ib.ids[t_alt], features, grad_image, grad_alpha, image, alpha, grad_features, grad_opacities, stream);
         });
     }
     return rc != INPC_OK ? rc : end_index_checks(stream);
