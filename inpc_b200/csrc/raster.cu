@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     const unsigned* __restrict__ depth_min,
     const unsigned* __restrict__ depth_max, PointRec* __restrict__ rec, uint2* __restrict__ bounds, uint32_t* __restrict__ quad,
     float4* __restrict__ conic, uint32_t* __restrict__ depth_keys,
-    uint32_t* __restrict__ point_ids, int pack_count, volatile unsigned* status) {
+    uint32_t* __restrict__ point_ids, int pack_count, int rec_stride, volatile unsigned* status) {
     constexpr int kHalves = VARIANT == VAR_RAW37 ? 37 : 36;
     constexpr int kSlabBytes = VARIANT == VAR_ROWS ? 16 : kPreThreads * kHalves * 2;   // multiple of 16 for both layouts
     __shared__ __align__(16) unsigned char s_feat[kSlabBytes];
@@ -422,8 +422,9 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     if (i >= n && iv < ps.start[ps.count]) bounds[iv] = make_uint2(0u, 0u);   // padding behind a set
     if (i < n && slab_ready) {
         if (pr.visible && VARIANT == VAR_ROWS) {
-            // feature rows are gathered by the blend itself: the record carries the geometry only
-            *reinterpret_cast<float4*>(rec + iv) = make_float4(pr.sx, pr.sy, __ldg(opacities + i), pr.depth);
+            // feature rows are gathered by the blend itself: the record carries the geometry only.  The warp blend reads such
+            // records 16 bytes apart (rec_stride 1): half-written 32-byte sectors cost as much DRAM traffic as whole ones
+            reinterpret_cast<float4*>(rec)[(size_t)iv * rec_stride] = make_float4(pr.sx, pr.sy, __ldg(opacities + i), pr.depth);
             bounds[iv] = make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16));
             if (quad) quad[iv] = pack_quad(pr, set * rp.gh);
         } else if (pr.visible) {
@@ -1251,7 +1252,7 @@ constexpr size_t backward_smem_bytes() {
 // and its order are those of a plain front-to-back loop per pixel.
 //
 // (3) Segments.  Front-to-back compositing is associative: (C, T) o (C', T') = (C + T C', T T').  A
-// tile's list is cut into a first segment of kFirstSegment instances and later ones of kLaterSegment, and every (tile half, segment) is one
+// tile's list is cut into a first segment and later ones (see segment_lengths), and every (tile half, segment) is one
 // item, so a tile with 100x the average load does not set the critical path.  Pass FIRST blends
 // segment 0 of every tile exactly; the pixels that dense clusters hit stop there.  Pass PRODUCT
 // computes, for the later segments, the per-pixel product of (1 - alpha) over the segment, starting
@@ -1272,14 +1273,31 @@ constexpr size_t backward_smem_bytes() {
 constexpr int kWarpBlendWarps = 8;        // warps per block; every warp works on items of its own
 constexpr int kQueueCap = 256;            // ring of candidate point ids per warp: >= 31 left over + 128 of one filter step
 constexpr int kFilterKeys = 4;            // keys per lane and filter step
-// Measured on B200 (2^23 clustered samples, 1237x822; forward / backward stage in microseconds), first + later segment:
-// 1024 + 4096: 422 / 276, 1024 + 2048: 439 / 268, 512 + 4096: 437 / 297, 512 + 2048: 458 / 274, 1024 + 1024: 488 / 291,
-// 512 + 1024: 518 / 283, 256 + 2048: 469 / 283.  Per-item timestamps of the same run: every pass is full (about 3000 of
-// the 3552 resident warps busy) for its first half and then drains for as long again while the longest items finish at
-// 1.0 - 1.4 us per batch; shorter segments shorten that tail but add more work (more lists to filter, more states to
-// carry) than they save.
-constexpr unsigned kFirstSegment = 1024;    // instances in a tile's first segment
-constexpr unsigned kLaterSegment = 4096;    // ... and in every later one
+// Segment lengths.  Measured on B200 (2^23 clustered samples, 1237x822; forward / backward stage in microseconds), first + later
+// segment: 1024 + 4096: 422 / 276, 1024 + 2048: 439 / 268, 512 + 4096: 437 / 297, 512 + 2048: 458 / 274, 1024 + 1024: 488 / 291,
+// 512 + 1024: 518 / 283, 256 + 2048: 469 / 283: with this many instances every pass is full (about 3000 of the 3552 resident
+// warps busy) for its first half, and shorter segments add more work (more lists to filter, more states to carry) than they
+// save.  With fewer instances the passes are as long as their longest items, at 1.0 - 1.4 us per batch of 32, while most
+// warps have none: the segments then get shorter, so that the later ones of all tiles number about kSegmentTarget (two items
+// each, one and a half times the resident warps).  10^6 samples, 801x533: forward / backward 283 / 153 us with 1024 + 4096,
+// 120 / 56 with the lengths below (149 / 70 with half the target); 2 * 10^5 samples, 600x400: 190 / 86 -> 85 / 35; first segments
+// of a quarter or of all of a later one measured the same or worse.
+constexpr unsigned kSegmentMin = 256;
+constexpr unsigned kFirstSegmentMax = 1024;
+constexpr unsigned kLaterSegmentMax = 4096;
+constexpr unsigned kSegmentTarget = 2560;
+constexpr int kManyTiles = 1 << 15;   // from here on the first segments alone keep the chip busy: half as many later ones are aimed at
+struct SegmentLengths {
+    unsigned first, later;   // instances in a tile's first segment, and in every later one
+};
+__device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_instances, int n_tiles) {
+    const unsigned target = n_tiles > kManyTiles ? kSegmentTarget / 2u : kSegmentTarget;
+    SegmentLengths s;
+    s.later = kSegmentMin;
+    while (s.later < kLaterSegmentMax && (unsigned long long)s.later * target < n_instances) s.later *= 2u;
+    s.first = max(kSegmentMin, min(kFirstSegmentMax, s.later / 2u));
+    return s;
+}
 constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
 
@@ -1292,8 +1310,8 @@ __device__ __forceinline__ unsigned long long key_pixels(unsigned code) {
     return cy == 0u ? two >> 8 : two << (8u * (cy - 1u));                // rows cy - 1 and cy, clipped likewise
 }
 
-__device__ __forceinline__ unsigned warp_segments(unsigned len) {
-    return len <= kFirstSegment ? 1u : 1u + ceil_div(len - kFirstSegment, kLaterSegment);
+__device__ __forceinline__ unsigned warp_segments(unsigned len, const SegmentLengths& sl) {
+    return len <= sl.first ? 1u : 1u + ceil_div(len - sl.first, sl.later);
 }
 
 // Work lists of the warp blend.  Step 1 (one block per 1024 tiles): segments and non-empty tiles of the block's tiles.
@@ -1304,7 +1322,7 @@ constexpr int kItemThreads = 256;
 constexpr int kItemTilesPerThread = 4;
 constexpr int kItemTilesPerBlock = kItemThreads * kItemTilesPerThread;
 
-__device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ranges, int n_tiles, int t0, unsigned (&ns)[kItemTilesPerThread],
+__device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ranges, int n_tiles, int t0, const SegmentLengths& sl, unsigned (&ns)[kItemTilesPerThread],
                                                    uint2 (&rg)[kItemTilesPerThread]) {
 #pragma unroll
     for (int k = 0; k < kItemTilesPerThread; k += 2) {
@@ -1314,16 +1332,18 @@ __device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ran
         else if (t0 + k < n_tiles) { const uint2 r0 = __ldg(ranges + t0 + k); r.x = r0.x; r.y = r0.y; }
         rg[k] = make_uint2(r.x, r.y);
         rg[k + 1] = make_uint2(r.z, r.w);
-        ns[k] = r.y > r.x ? warp_segments(r.y - r.x) : 0u;
-        ns[k + 1] = r.w > r.z ? warp_segments(r.w - r.z) : 0u;
+        ns[k] = r.y > r.x ? warp_segments(r.y - r.x, sl) : 0u;
+        ns[k + 1] = r.w > r.z ? warp_segments(r.w - r.z, sl) : 0u;
     }
 }
 
-__global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, uint2* __restrict__ block_sums) {
+__global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, unsigned long long n_instances_arg,
+                                                                        const unsigned long long* __restrict__ n_instances_dev, uint2* __restrict__ block_sums) {
     __shared__ unsigned s_seg[kItemThreads / 32], s_tiles[kItemThreads / 32];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
-    load_tile_segments(ranges, n_tiles, blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread, ns, rg);
+    const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles);
+    load_tile_segments(ranges, n_tiles, blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread, sl, ns, rg);
     unsigned seg = 0, tiles = 0;
 #pragma unroll
     for (int k = 0; k < kItemTilesPerThread; ++k) { seg += ns[k]; tiles += ns[k] ? 1u : 0u; }
@@ -1375,14 +1395,16 @@ __device__ __forceinline__ WarpItem load_item(const WarpItem* p) {
 }
 
 // Step 3: items0 = segment 0 of the non-empty tiles, items1 = every later segment, tile by tile.
-__global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles,
+__global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, unsigned long long n_instances_arg,
+                                                                      const unsigned long long* __restrict__ n_instances_dev,
                                                                       const uint2* __restrict__ block_base, WarpItem* __restrict__ items0,
                                                                       WarpItem* __restrict__ items1) {
     __shared__ unsigned s_scan[kItemThreads / 32 + 1];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
     const int t0 = blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread;
-    load_tile_segments(ranges, n_tiles, t0, ns, rg);
+    const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles);
+    load_tile_segments(ranges, n_tiles, t0, sl, ns, rg);
     unsigned seg = 0, tiles = 0;
 #pragma unroll
     for (int k = 0; k < kItemTilesPerThread; ++k) { seg += ns[k]; tiles += ns[k] ? 1u : 0u; }
@@ -1395,8 +1417,8 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
         if (ns[k] == 0u) continue;
         const uint2 r = rg[k];
         for (unsigned sg = 0; sg < ns[k]; ++sg) {
-            const unsigned begin = sg == 0 ? r.x : r.x + kFirstSegment + (sg - 1u) * kLaterSegment;
-            const unsigned end = min(r.y, begin + (sg == 0 ? kFirstSegment : kLaterSegment));
+            const unsigned begin = sg == 0 ? r.x : r.x + sl.first + (sg - 1u) * sl.later;
+            const unsigned end = min(r.y, begin + (sg == 0 ? sl.first : sl.later));
             // later segments: position = segments before this tile minus tiles before it
             WarpItem* dst = sg == 0 ? items0 + rank : items1 + (first - rank + sg - 1u);
             reinterpret_cast<uint4*>(dst)[0] = make_uint4((uint32_t)(t0 + k), sg, begin, end);
@@ -1598,7 +1620,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                 uint32_t id = kNoInstance;
                 if (lane < n) {
                     id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(q_head + lane) & (kQueueCap - 1)]);
-                    const float4* p = reinterpret_cast<const float4*>(rec + id);
+                    const float4* p = reinterpret_cast<const float4*>(rec) + (size_t)id * (ROWS ? 1 : 2);
                     async_copy_16(&sm.ring_a[stage][lane], p);
                     if (kBlend && !ROWS) async_copy_16(&sm.ring_f[stage][lane], p + 1);
                 }
@@ -1849,7 +1871,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
     float* __restrict__ image, float* __restrict__ depth_image, float* __restrict__ alpha_image, int width, int height, int gw, int gh) {
     const unsigned lane = lane_id();
     const unsigned n_parts = __ldg(counts) * 2u;
-    for (unsigned w = blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5); w < n_parts; w += gridDim.x * kWarpBlendWarps) {
+    // a warp takes one group of four channels of a tile half
+    for (unsigned wc = blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5); wc < n_parts * C4; wc += gridDim.x * kWarpBlendWarps) {
+        const unsigned w = wc / C4, ch = wc % C4;
         const WarpItem it = load_item(items0 + (w >> 1));
         const unsigned half = w & 1u;
         const unsigned tile = it.tile, n_seg = it.n_seg, first = it.first;
@@ -1863,7 +1887,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
         const int64_t n_px = (int64_t)width * height;
         const int64_t pi = (int64_t)py * width + px;
         float* image_s = image + (int64_t)set * 4 * n_px;
-        for (int ch = 0; ch < C4; ++ch) {
+        {
             float4 run = make_float4(0.f, 0.f, 0.f, 0.f);
             float4* part = seg_C + (((size_t)first * 2u + half) * C4 + ch) * 32 + lane;   // segment g: part + g * 64 C4
             for (unsigned g0 = 0; g0 < n_seg; g0 += 4) {
@@ -1884,7 +1908,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
                 plane[3 * n_px] = run.w;
             }
         }
-        if (KIND == BLEND_INFER) {
+        if (KIND == BLEND_INFER && ch == 0) {
             float z = 0.0f, t_final = 1.0f;
             bool stopped = false;
             for (unsigned g0 = 0; g0 < n_seg; g0 += 4) {
@@ -2242,7 +2266,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
             uint32_t id = kNoInstance;
             if (lane < n) {
                 id = checked_point(idf[0]);
-                async_copy_16(&sm.ring_a[stage][lane], reinterpret_cast<const float4*>(rec + id));
+                async_copy_16(&sm.ring_a[stage][lane], reinterpret_cast<const float4*>(rec) + id);
             }
             gather_rows<C4>(sm.ring_f[stage], rows, id, lane);
             sm.ring_id[stage][lane] = id;
@@ -3161,6 +3185,15 @@ struct InstanceBlob {
     size_t total;
 };
 
+// Upper bound on the segments of the warp blend for up to n_instances instances (see segment_lengths): one per tile, one more
+// for every tile that is longer than a first segment, and the later segments that are full.
+int64_t max_warp_segments(int64_t n_instances, int n_tiles) {
+    const int64_t target = kSegmentTarget;
+    const int64_t by_first = ceil_div<int64_t>(n_instances, kFirstSegmentMax), by_later = ceil_div<int64_t>(n_instances, kLaterSegmentMax);
+    const int64_t longer = by_first > 2 * target ? by_first : 2 * target;
+    return n_tiles + (longer < n_tiles ? longer : n_tiles) + (by_later > target ? by_later : target) + 1;
+}
+
 // Upper bound on the number of (tile, segment) work items, known from the instance count alone.
 int blend_batch(int tile);
 int64_t max_segments(int64_t n_instances, int n_tiles, int tile) {
@@ -3184,7 +3217,7 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int 
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n_instances);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n_instances);
     // upper bound on the number of (tile, segment) pairs, known from the instance count alone
-    b.max_segments = warp_blend ? (int64_t)n_tiles + ceil_div<int64_t>(n_instances, (int64_t)kLaterSegment) : max_segments(n_instances, n_tiles, tile);
+    b.max_segments = warp_blend ? max_warp_segments(n_instances, n_tiles) : max_segments(n_instances, n_tiles, tile);
     const size_t px = (size_t)b.max_segments * tile * tile;
     b.segs = c.take<Segment>(warp_blend ? 0 : b.max_segments);
     b.tile_first = c.take<uint32_t>(n_tiles);
@@ -3216,13 +3249,13 @@ int tile_result_buffer(int64_t n_instances, int n_tiles) {
 
 // One event per host thread and device: an event belongs to the device that was current when it was made.
 // Instance capacity the blobs of `st` were carved for, and which ping-pong buffer holds the tile-sorted lists.
-int64_t instance_capacity(const inpc_raster_state* st) { return st->deferred_counts ? 4 * st->n_points : st->n_instances; }
+int64_t instance_capacity(const inpc_raster_state* st) { return (st->deferred_counts & 1) ? 4 * st->n_points : st->n_instances; }
 int tile_buffer_of(const inpc_raster_state* st, int n_tiles) {
-    if (st->deferred_counts) return sort_pass_count(bit_length((uint32_t)(n_tiles - 1))) & 1;
+    if (st->deferred_counts & 1) return sort_pass_count(bit_length((uint32_t)(n_tiles - 1))) & 1;
     return tile_result_buffer(st->n_instances, n_tiles);
 }
 int depth_buffer_of(const inpc_raster_state* st) {
-    if (st->deferred_counts) return sort_pass_count(st->depth_key_bits) & 1;
+    if (st->deferred_counts & 1) return sort_pass_count(st->depth_key_bits) & 1;
     return depth_result_buffer(st->n_visible, st->depth_key_bits);
 }
 
@@ -3377,7 +3410,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             preprocess_kernel<MODE, VARIANT><<<(unsigned)nb, kPreThreads, 0, stream>>>(
                 ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max,
                 pb.rec, pb.bounds, warp_blend ? pb.quad : nullptr,
-                pb.conic, pb.keys[0], pb.ids[0], pack_count, status);
+                pb.conic, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
             INPC_LAUNCH_CHECK("preprocess_kernel");
         }
         if (!deferred) {
@@ -3449,11 +3482,11 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         INPC_CUDA_TRY(cudaMemsetAsync(ib.n_segments, 0, 8 * sizeof(uint32_t), stream));
         const int item_blocks = ceil_div(n_tiles, kItemTilesPerBlock);
         uint2* item_sums = reinterpret_cast<uint2*>(ib.tile_rank);
-        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, item_sums);
+        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums);
         INPC_LAUNCH_CHECK("warp_items_count_kernel");
         warp_items_scan_kernel<<<1, kScanThreads, 0, stream>>>(item_sums, item_blocks, ib.n_segments);
         INPC_LAUNCH_CHECK("warp_items_scan_kernel");
-        warp_items_fill_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, item_sums, ib.items0, ib.items1);
+        warp_items_fill_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
         INPC_LAUNCH_CHECK("warp_items_fill_kernel");
     } else {
         StageScope scope(STAGE_SORT_TILE, stream);
@@ -3472,7 +3505,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     st->depth_key_base = key_base;
     st->depth_key_bits = key_bits;
     st->channels = VARIANT == VAR_ROWS ? 4 * c4 : 4;
-    st->deferred_counts = deferred ? 1 : 0;
+    st->deferred_counts = (deferred ? 1 : 0) | (VARIANT == VAR_ROWS && warp_blend ? 2 : 0);   // bit 1: records 16 bytes apart, without features
     *pb_out = pb;
     *ib_out = ib;
     return INPC_OK;
@@ -3556,7 +3589,7 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
                             kept0, kept1, ib.n_kept, W, H, rp.gw, rp.gh};
     int rc_pass = launch_warp_forward_pass<PASS_FIRST, KIND, C4, ROWS>(grid, ib.items0, ib.n_segments, ib.n_segments + 2, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, false>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
+    rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     warp_blend_prefix_kernel<<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
@@ -4033,7 +4066,7 @@ extern "C" int inpc_rasterize_rows_backward(const inpc_raster_state* state, cons
 extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (!state) { set_error("inpc_raster_resolve: null state"); return INPC_E_INVALID; }
-    if (!state->deferred_counts || state->n_points == 0) return INPC_OK;
+    if (!(state->deferred_counts & 1) || state->n_points == 0) return INPC_OK;
     if (!state->point_blob) { set_error("inpc_raster_resolve: state without a point blob"); return INPC_E_INVALID; }
     const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode);
     unsigned long long host[4];
@@ -4056,17 +4089,17 @@ __global__ void add_base_kernel(const uint32_t* __restrict__ src, int64_t n, uin
     if (i < n) dst[i] = (src[i] & mask) + base;
 }
 
-__global__ void unpack_points_kernel(const PointRec* __restrict__ rec, const uint2* __restrict__ bounds, int64_t n, int which,
+__global__ void unpack_points_kernel(const PointRec* __restrict__ rec, int rec_stride, const uint2* __restrict__ bounds, int64_t n, int which,
                                      void* __restrict__ dst) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint2 b = bounds[i];
     const bool vis = tiles_of(b) != 0u;
-    const float4* r = reinterpret_cast<const float4*>(rec + i);
+    const float4* r = reinterpret_cast<const float4*>(rec) + i * rec_stride;
     if (which == 4) static_cast<unsigned*>(dst)[i] = tiles_of(b);
     else if (which == 5) { const float4 a = vis ? r[0] : make_float4(0, 0, 0, 0); static_cast<float2*>(dst)[i] = make_float2(a.x, a.y); }
     else if (which == 6) static_cast<float*>(dst)[i] = vis ? r[0].w : 0.0f;
-    else if (which == 7) static_cast<float4*>(dst)[i] = vis ? r[1] : make_float4(0, 0, 0, 0);
+    else if (which == 7) static_cast<float4*>(dst)[i] = vis && rec_stride == 2 ? r[1] : make_float4(0, 0, 0, 0);
     else if (which == 8) {
         unsigned short* o = static_cast<unsigned short*>(dst) + 4 * i;
         o[0] = (unsigned short)(b.x & 0xffffu); o[1] = (unsigned short)(b.x >> 16);
@@ -4100,7 +4133,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
         case 3: INPC_CUDA_TRY(cudaMemcpyAsync(dst, ib.ranges, 8 * (size_t)n_tiles, cudaMemcpyDeviceToDevice, stream)); break;
         case 4: case 5: case 6: case 7: case 8:
             if (state->n_points > 0) {
-                inpc_debug::unpack_points_kernel<<<(unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream>>>(pb.rec, pb.bounds, state->n_points, which, dst);
+                inpc_debug::unpack_points_kernel<<<(unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream>>>(pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, state->n_points, which, dst);
                 INPC_LAUNCH_CHECK("unpack_points_kernel");
             }
             break;

@@ -47,3 +47,59 @@ def test_halton_samples_over_runs_of_empty_leaves(total, gap):
     levels = torch.randint(0, 11, (n,), generator=g, dtype=torch.int32)
     out = halton_samples(counts.to(DEV), centers.to(DEV), levels.to(DEV), 2.0)
     np.testing.assert_array_equal(out.cpu().numpy(), O.halton_samples(counts.numpy(), centers.numpy(), levels.numpy(), 2.0))
+
+
+def _one_tile_scene(n, seed):
+    """n faint points in front of a 24x16 image, three quarters of them over one 8x8 tile."""
+    from inpc_b200.views import look_at_view
+    g = torch.Generator().manual_seed(seed)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 24, 16, 24.0, 24.0)
+    z = torch.rand(n, generator=g) * 2 - 1
+    px = torch.where(torch.rand(n, generator=g) < 0.75, 8 + torch.rand(n, generator=g) * 8, torch.rand(n, generator=g) * 24)
+    py = torch.rand(n, generator=g) * 8
+    depth = 3.0 - z
+    # looking down -z: image x runs along +x, image y along -y
+    pos = torch.stack([(px - 12) / 24 * depth, -(py - 8) / 24 * depth, z], dim=1).contiguous()
+    opac = (torch.rand((n, 1), generator=g) * 0.9 + 0.1) * min(0.5, 40.0 / n)
+    return view, pos, opac
+
+
+# a tile's list is cut into segments of at least 256 instances; their length doubles from 655,360 instances on
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 511, 513, 769, 4097, 655_000, 700_001])
+@pytest.mark.parametrize("rows", [0, 4, 16, 32])
+def test_blend_at_the_edges_of_its_segments(n, rows):
+    import inpc_b200
+    from helpers import assert_close, oracle_camera
+    if n > 100_000 and rows not in (0, 16):
+        pytest.skip("the long lists are walked in one layout of each kind")
+    view, pos, opac = _one_tile_scene(n, n)
+    g = torch.Generator().manual_seed(n + 1)
+    gi, ga = torch.randn((rows or 4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
+    cam, v, rast = oracle_camera(view), view.to(DEV), inpc_b200.INPCRasterizer()
+    o = opac.to(DEV).requires_grad_(True)
+    if rows:
+        feats = torch.randn((n, rows), generator=g) * 0.5
+        f = feats.to(DEV).requires_grad_(True)
+        image, alpha, bw = rast.forward_rows(v, pos.to(DEV), f, o)
+        st = O.rasterize_rows_forward(cam, pos.numpy(), feats.numpy(), opac.numpy())
+        gf, go = O.rasterize_rows_backward(st, gi.numpy(), ga.numpy())
+        tol_f = dict(rtol=2e-4, atol=1e-9)
+    else:
+        feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+        f = feats.to(DEV).requires_grad_(True)
+        image, alpha, bw = rast(v, 0, pos.to(DEV), f, o)
+        st = O.rasterize_forward(O.BILINEAR, cam, pos.numpy(), feats.numpy(), opac.numpy())
+        gf, go, _ = O.rasterize_backward(st, gi.numpy(), ga.numpy())
+        tol_f = dict(rtol=2e-3, atol=1.2e-7)      # two steps of the smallest halves
+    # A pixel meets up to N = n / 16 fragments (four per point, three quarters of the points on 64 pixels).  Its transmittance is
+    # a product of N factors; every product rounds by at most 2^-25, and while it is close to 1 mostly in the same direction, so
+    # two orders of multiplication differ by up to N 2^-25 (measured against double precision: the oracle is off by 2.5e-5 for
+    # n = 655,000, a tenth of the bound).  Everything else is proportional to it; sums of N terms add sqrt(N) 2^-24.
+    eps = n / 16 * 2.0 ** -25
+    assert_close(image.detach().cpu().numpy(), st.image, rtol=1e-4, atol=3e-6 + 0.2 * eps, what="image")
+    assert_close(alpha.detach().cpu().numpy(), st.alpha, rtol=1e-5, atol=1e-6 + eps, what="alpha")
+    assert_close(bw.cpu().numpy(), st.blending_weights, rtol=2e-4 + eps, atol=1e-9, what="blending weights")
+    torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
+    assert_close(f.grad.float().cpu().numpy(), np.asarray(gf, np.float32), rtol=tol_f["rtol"] + eps, atol=tol_f["atol"], what="grad_features")
+    # opacity gradients are differences of sums of the order of 1e-3
+    assert_close(o.grad.cpu().numpy(), go, rtol=1e-3 + eps, atol=2e-8 + 1e-3 * eps, what="grad_opacities")
