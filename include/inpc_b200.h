@@ -364,6 +364,10 @@ int inpc_leaf_stats_accumulate(const int64_t* indices, const float* weights, int
  * Replaces Modules/ProbabilityField.py:148-149 and :156-157. */
 int inpc_leaf_update(float* leaf_weights, float* leaf_subdivision_scores, const uint32_t* stats,
                      int64_t n_leaves, float decay, void* stream);
+/* The three steps above for one set of samples (ProbabilityField.update, Modules/ProbabilityField.py:146-157);
+ * `stats` (n_leaves, 2) is scratch. */
+int inpc_leaf_update_from_samples(const int64_t* indices, const float* weights, int64_t n, uint32_t* stats, float* leaf_weights,
+                                  float* leaf_subdivision_scores, int64_t n_leaves, float decay, void* stream);
 
 /* Structural updates of the octree probability field (the reference does them in torch:
  * Modules/ProbabilityField.py:159-165 prune, :217-257 subdivide).  Both are two calls: *_count

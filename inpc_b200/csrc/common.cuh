@@ -119,13 +119,15 @@ inline ViewParams to_params(const inpc_view* v) {
 size_t sort_workspace_bytes(int64_t n, int64_t n_likely);
 int sort_pass_count(int end_bit);   // passes sort_pairs makes; the result is in the alternate buffers iff odd (and n > 1)
 // `status`: device address of the STATUS_WORDS words a tile that gives up its look-back reports to.
-// `n_likely`: the one the workspace was sized with (for at least n pairs).
+// `n_likely`: the one the workspace was sized with (for at least n pairs).  `zeroed`: the caller has cleared the first
+// sort_zero_bytes(n, n_likely, end_bit) bytes of the workspace.
+size_t sort_zero_bytes(int64_t n, int64_t n_likely, int end_bit);
 int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
-               int end_bit, void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream);
+               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for (n_max, n_likely).  The result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
-                            const unsigned long long* n_dev, int end_bit, void* workspace, unsigned* status, int* result_in_alt,
+                            const unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
                             cudaStream_t stream);
 
 // More than 48 KB of dynamic shared memory is an opt-in per kernel AND per device: `done` is the
@@ -205,6 +207,18 @@ __device__ __forceinline__ void bulk_store_from_shared(void* dst_global, const v
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_global), "r"(shared_address(src_shared)), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
+// ---- the block of a launch that finishes last goes on with what would be a one-block launch of its own ---------
+// Every block calls this behind its last write; true in all threads of the last one.  `done` starts at zero.
+__device__ __forceinline__ bool last_block(unsigned* done, unsigned n_blocks) {
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == n_blocks - 1u;
+    __syncthreads();
+    if (s_last) __threadfence();
+    return s_last;
 }
 
 // Block-wide exclusive scan of one unsigned per thread; `smem` needs (blockDim.x/32 + 1) words.

@@ -143,6 +143,14 @@ constexpr int kCauchyMaxBlocks = 148 * 8;
 // update reads as max = min = 0 (scatter_reduce with include_self=False on a zero tensor).
 constexpr unsigned kMinFlip = 0x7FFFFFFFu;
 
+// A read through L1, where the pair may be older than what other multiprocessors have written since: good enough for a value
+// that only grows and is only compared against.  The few leaves most samples fall into are then L1 hits.
+__device__ __forceinline__ uint2 cached_pair(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.global.ca.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
 __global__ void __launch_bounds__(kThreads) leaf_stats_kernel(const long long* __restrict__ indices, const float* __restrict__ weights,
                                                               int64_t n, int64_t n_leaves, uint2* __restrict__ stats) {
     // four samples per thread and round, their loads issued together: the kernel is bound by the latency of the
@@ -162,7 +170,7 @@ __global__ void __launch_bounds__(kThreads) leaf_stats_kernel(const long long* _
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             if (leaf[k] < 0 || leaf[k] >= n_leaves) leaf[k] = -1;
-            cur[k] = leaf[k] >= 0 ? __ldcg(stats + leaf[k]) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+            cur[k] = leaf[k] >= 0 ? cached_pair(stats + leaf[k]) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
         }
         // Both halves only grow, so a value that does not beat what a plain (possibly stale) read
         // returns cannot beat the current one either: most samples of a leaf that has already seen a
@@ -337,6 +345,14 @@ extern "C" int inpc_leaf_stats_accumulate(const int64_t* indices, const float* w
                                                                                      reinterpret_cast<uint2*>(stats));
     INPC_LAUNCH_CHECK("leaf_stats_kernel");
     return INPC_OK;
+}
+
+extern "C" int inpc_leaf_update_from_samples(const int64_t* indices, const float* weights, int64_t n, uint32_t* stats, float* leaf_weights,
+                                             float* leaf_subdivision_scores, int64_t n_leaves, float decay, void* stream) {
+    int rc = inpc_leaf_stats_reset(stats, n_leaves, stream);
+    if (rc == INPC_OK) rc = inpc_leaf_stats_accumulate(indices, weights, n, stats, n_leaves, stream);
+    if (rc == INPC_OK) rc = inpc_leaf_update(leaf_weights, leaf_subdivision_scores, stats, n_leaves, decay, stream);
+    return rc;
 }
 
 extern "C" int inpc_leaf_update(float* leaf_weights, float* leaf_subdivision_scores, const uint32_t* stats, int64_t n_leaves, float decay,

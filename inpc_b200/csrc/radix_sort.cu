@@ -365,6 +365,24 @@ int launch_onesweep_pass(const PassArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
+static size_t state_words(int64_t tiles, int end_bit) {
+    const int n_passes = ceil_div(end_bit, kRadixBits);
+    size_t words = 0;
+    for (int p = 0, bit = 0; p < n_passes; ++p) {
+        const int b = (end_bit - bit + (n_passes - p) - 1) / (n_passes - p);
+        words += (size_t)tiles * pass_bins(b);
+        bit += b;
+    }
+    return words;
+}
+
+// Histograms, tickets and the look-back state lie at the front of the workspace.
+size_t sort_zero_bytes(int64_t n, int64_t n_likely, int end_bit) {
+    if (n <= 0 || end_bit <= 0) return 0;
+    const int items = tile_items(n_likely);
+    return carve_sort_workspace(nullptr, n, items).zero_bytes + state_words(ceil_div<int64_t>(n, (int64_t)kThreads * items), end_bit) * sizeof(unsigned);
+}
+
 size_t sort_workspace_bytes(int64_t n, int64_t n_likely) { return carve_sort_workspace(nullptr, n, tile_items(n_likely)).total; }
 
 int sort_pass_count(int end_bit) { return end_bit > 0 ? ceil_div(end_bit, kRadixBits) : 0; }
@@ -388,7 +406,7 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 // status words a tile that gives up its look-back writes to.  Every entry point ends up here.
 // `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
-                           int items, void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
+                           int items, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
                            unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
@@ -408,11 +426,8 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
 
     SortWorkspace w = carve_sort_workspace(workspace, n, items);
     const int64_t tiles = ceil_div<int64_t>(n, (int64_t)kThreads * items);
-    size_t state_words = 0;
-    for (int p = 0; p < pt.n_passes; ++p) state_words += (size_t)tiles * pass_bins(pt.bits[p]);
-    // hist, tickets and the look-back state are contiguous at the front of the workspace; a workspace that
-    // is reused keeps the previous call's contents, so everything this call reads is cleared first
-    INPC_CUDA_TRY(cudaMemsetAsync(workspace, 0, w.zero_bytes + state_words * sizeof(unsigned), stream));
+    // a workspace that is reused keeps the previous call's contents, so everything this call reads is cleared first
+    if (!zeroed) INPC_CUDA_TRY(cudaMemsetAsync(workspace, 0, w.zero_bytes + state_words(tiles, end_bit) * sizeof(unsigned), stream));
 
     const int64_t hist_blocks = ceil_div<int64_t>(n, kHistItemsPerBlock), hist_cap = (int64_t)sm_count() * 4;
     radix_histogram_kernel<<<(unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap), kHistThreads, 0, stream>>>(keys, n, n_dev, pt, w.hist, w.ticket + kMaxPasses, w.base);
@@ -438,20 +453,20 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
 }
 
 int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
-               int end_bit, void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream) {
+               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream) {
     if (result_in_alt) *result_in_alt = 0;
     bool nothing = false;
     const int rc = check_sort_args("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, &nothing);
     if (rc != INPC_OK || nothing) return rc;
     if (!workspace) { set_error("sort_pairs: null workspace"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n_likely), workspace, status, result_in_alt, stream);
+    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n_likely), workspace, zeroed, status, result_in_alt, stream);
 }
 
 // The same sort with the number of pairs in device memory (*n_dev <= n_max): grids and the look-back state are
 // sized for n_max, the kernels read the count themselves, and the result is always in the alternate buffers iff
 // the number of passes is odd.  No host synchronisation anywhere.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
-                            const unsigned long long* n_dev, int end_bit, void* workspace, unsigned* status, int* result_in_alt,
+                            const unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
                             cudaStream_t stream) {
     if (result_in_alt) *result_in_alt = 0;
     if (n_max <= 0 || end_bit == 0) return INPC_OK;
@@ -459,7 +474,7 @@ int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values
     const int rc = check_sort_args("sort_pairs", keys, keys_alt, values, values_alt, n_max < 2 ? 2 : n_max, end_bit, &nothing);
     if (rc != INPC_OK) return rc;
     if (!workspace || !n_dev) { set_error("sort_pairs: null workspace or count"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n_max, end_bit, tile_items(n_likely), workspace, status, result_in_alt, stream, kSpinLimit,
+    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n_max, end_bit, tile_items(n_likely), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
                            0xFFFFFFFFu, n_dev);
 }
 
@@ -528,7 +543,7 @@ extern "C" int inpc_sort_pairs_static(uint32_t* keys, uint32_t* keys_alt, uint32
     // the status words of this entry point live behind the workspace, inside the same fixed array
     unsigned* status = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(scratch) + kStaticWorkspaceBytes);
     INPC_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned) * STATUS_WORDS, stream));
-    return sort_pairs_with("inpc_sort_pairs_static", keys, keys_alt, values, values_alt, n, end_bit, kLargeItems, scratch, status, result_in_alt, stream);
+    return sort_pairs_with("inpc_sort_pairs_static", keys, keys_alt, values, values_alt, n, end_bit, kLargeItems, scratch, false, status, result_in_alt, stream);
 }
 
 extern "C" size_t inpc_sort_workspace_bytes(int64_t n) { return inpc::sort_workspace_bytes(n < 0 ? 0 : n, n); }
@@ -545,7 +560,7 @@ extern "C" int inpc_sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* val
     if (rc != INPC_OK) return rc;
     unsigned* status = acquire_status("inpc_sort_pairs");
     if (!status) return INPC_E_CUDA;
-    return sort_pairs(keys, keys_alt, values, values_alt, n, n, end_bit, workspace, status, result_in_alt, static_cast<cudaStream_t>(stream));
+    return sort_pairs(keys, keys_alt, values, values_alt, n, n, end_bit, workspace, false, status, result_in_alt, static_cast<cudaStream_t>(stream));
 }
 
 // Test hook: inpc_sort_pairs with tile 0 of every pass leaving before it publishes its digit counts and a
@@ -561,7 +576,7 @@ extern "C" int inpc_debug_sort_lookback_timeout(uint32_t* keys, uint32_t* keys_a
     if (nothing || !workspace || !ticket) { set_error("inpc_debug_sort_lookback_timeout: needs n > 1, end_bit > 0, a workspace and a ticket pointer"); return INPC_E_INVALID; }
     unsigned* status = acquire_status("inpc_debug_sort_lookback_timeout", ticket);
     if (!status) return INPC_E_CUDA;
-    return sort_pairs_with("inpc_debug_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, status, nullptr,
+    return sort_pairs_with("inpc_debug_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, false, status, nullptr,
                            static_cast<cudaStream_t>(stream), 1 << 10, 0u);
 }
 

@@ -178,16 +178,85 @@ __device__ __forceinline__ Projection project_point(const float px, const float 
     return o;
 }
 
+// ---- one launch for everything a call needs zeroed (images, weights, sort state, counters) ---------
+// Nine separate memsets were a fifth of the launches of a small training step.
+constexpr int kMaxClear = 8;
+struct ClearList {
+    int count = 0;
+    void* ptr[kMaxClear];
+    size_t bytes[kMaxClear];   // multiples of 4
+    void add(void* p, size_t n) {
+        if (p && n) { ptr[count] = p; bytes[count] = n; ++count; }
+    }
+};
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearList list) {
+    const size_t tid = (size_t)blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
+    for (int r = 0; r < list.count; ++r) {
+        char* p = static_cast<char*>(list.ptr[r]);
+        const size_t lead = min(list.bytes[r], (size_t)((16u - (unsigned)(reinterpret_cast<uintptr_t>(p) & 15u)) & 15u));
+        const size_t n16 = (list.bytes[r] - lead) / 16, tail = lead + n16 * 16;
+        for (size_t k = tid; k < n16; k += stride) reinterpret_cast<uint4*>(p + lead)[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (4 * tid < lead) *reinterpret_cast<unsigned*>(p + 4 * tid) = 0u;
+        if (tail + 4 * tid < list.bytes[r]) *reinterpret_cast<unsigned*>(p + tail + 4 * tid) = 0u;
+    }
+}
+
+// Exclusive scan of n words in place by one block of THREADS threads (16 words per thread and round, read past L1: other
+// blocks have just written them).  Returns the total; smem: THREADS / 32 + 1 words.
+template <int THREADS>
+__device__ __forceinline__ unsigned scan_words(unsigned* data, int64_t n, unsigned* smem) {
+    constexpr int kPer = 16;
+    unsigned running = 0;
+    for (int64_t base = 0; base < n; base += THREADS * kPer) {
+        const int64_t j0 = base + (int64_t)threadIdx.x * kPer;
+        unsigned v[kPer], sum = 0;
+        if (j0 + kPer <= n) {
+#pragma unroll
+            for (int k = 0; k < kPer; k += 4) {
+                const uint4 q = __ldcg(reinterpret_cast<const uint4*>(data + j0 + k));
+                v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) v[k] = j0 + k < n ? __ldcg(data + j0 + k) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) sum += v[k];
+        unsigned total;
+        unsigned ex = running + block_exclusive_scan(sum, smem, &total);
+        if (j0 + kPer <= n) {
+#pragma unroll
+            for (int k = 0; k < kPer; k += 4) {
+                uint4 q;
+                q.x = ex; q.y = q.x + v[k]; q.z = q.y + v[k + 1]; q.w = q.z + v[k + 2];
+                ex = q.w + v[k + 3];
+                *reinterpret_cast<uint4*>(data + j0 + k) = q;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kPer; ++k) {
+                if (j0 + k < n) data[j0 + k] = ex;
+                ex += v[k];
+            }
+        }
+        running += total;
+    }
+    return running;
+}
+
 constexpr int kPreThreads = 256;
 constexpr unsigned kCountShift = 30;   // bilinear: (tiles touched - 1) in key bits 30..31 when the depth offsets fit below
 
 // Pass 1 of the deterministic compaction: per block, how many points survive culling and how many
-// (point, tile) instances they create.
+// (point, tile) instances they create.  The last block scans the groups' counts (groups of 4 chunks of kPreThreads points)
+// and leaves the totals in counters[0] (visible) and counters[1] (instances), the range of depth bit patterns the
+// keys are offsets into in counters[2..3] and *depth_min, *depth_max: measured (`range` given: the words start at zero
+// and collect the largest pattern and the largest complement), or fixed_lo .. fixed_hi.
 template <int MODE, int VARIANT>
 __global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
     PointSets ps, RasterParams rp, unsigned* __restrict__ block_visible,
-    unsigned* __restrict__ group_visible, unsigned long long* __restrict__ group_instances, unsigned* __restrict__ depth_min,
-    unsigned* __restrict__ depth_max) {
+    unsigned* group_visible, unsigned long long* group_instances, unsigned* range, unsigned* done, unsigned fixed_lo, unsigned fixed_hi,
+    unsigned* __restrict__ depth_min, unsigned* __restrict__ depth_max, unsigned long long* __restrict__ counters) {
     // this block's set; indices below are local to it
     const int set = set_of_block(ps, (int64_t)blockIdx.x * kPreThreads * 4);
     const float* __restrict__ positions = ps.positions[set];
@@ -260,60 +329,31 @@ __global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
         // totals of this group of 4 chunks: the one-block scan runs over groups, four times fewer entries
         group_visible[blockIdx.x] = tv;
         group_instances[blockIdx.x] = ti;
-        // (callers that know a bound on the depths beforehand pass no pointers; measured: no difference in time)
-        if (depth_min && tlo <= thi) { atomicMin(depth_min, tlo); atomicMax(depth_max, thi); }
+        // (callers that know a bound on the depths beforehand pass no pointer; measured: no difference in time)
+        if (range && tlo <= thi) { atomicMax(range, ~tlo); atomicMax(range + 1, thi); }
     }
-}
-
-// Exclusive scan of the per-group counts (groups of 4 chunks) by one block; totals land in counters[0]
-// (visible) and counters[1] (instances), the depth range in counters[2..3].
-constexpr int kScanThreads = 1024;
-__global__ void __launch_bounds__(kScanThreads) scan_block_counts_kernel(unsigned* __restrict__ block_visible,
-                                                                         const unsigned long long* __restrict__ block_instances,
-                                                                         int64_t n_blocks,
-                                                                         unsigned* __restrict__ depth_min,
-                                                                         unsigned* __restrict__ depth_max,
-                                                                         unsigned long long* __restrict__ counters, int fixed_range,
-                                                                         unsigned fixed_lo, unsigned fixed_hi) {
-    constexpr int kItems = 8;
-    __shared__ unsigned s_scan[kScanThreads / 32 + 1];
-    __shared__ unsigned long long s_inst[kScanThreads / 32];
-    unsigned running = 0;
+    if (!last_block(done, gridDim.x)) return;
+    __shared__ unsigned s_scan[kPreThreads / 32 + 1];
+    const unsigned visible = scan_words<kPreThreads>(group_visible, gridDim.x, s_scan);
     unsigned long long inst = 0;
-    for (int64_t base = 0; base < n_blocks; base += (int64_t)kScanThreads * kItems) {
-        const int64_t j0 = base + (int64_t)threadIdx.x * kItems;
-        unsigned v[kItems];
-        unsigned sum = 0;
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            v[k] = j0 + k < n_blocks ? block_visible[j0 + k] : 0u;
-            sum += v[k];
-            if (j0 + k < n_blocks) inst += block_instances[j0 + k];
-        }
-        unsigned total;
-        unsigned ex = running + block_exclusive_scan(sum, s_scan, &total);
-#pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            if (j0 + k < n_blocks) block_visible[j0 + k] = ex;
-            ex += v[k];
-        }
-        running += total;
-    }
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += kPreThreads) inst += __ldcg(group_instances + k);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
-    if (lane_id() == 0) s_inst[threadIdx.x >> 5] = inst;
+    if (lane_id() == 0) s_i[threadIdx.x >> 5] = inst;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
-        for (int w = 0; w < kScanThreads / 32; ++w) t += s_inst[w];
-        counters[0] = running;
+#pragma unroll
+        for (int w = 0; w < kPreThreads / 32; ++w) t += s_i[w];
+        const unsigned lo = range ? ~__ldcg(range) : fixed_lo, hi = range ? __ldcg(range + 1) : fixed_hi;
+        counters[0] = visible;
         counters[1] = t;
-        // the range of depth bit patterns the keys are offsets into: measured by the count pass, or given by the caller
-        if (fixed_range) { *depth_min = fixed_lo; *depth_max = fixed_hi; }
-        counters[2] = *depth_min;
-        counters[3] = *depth_max;
+        counters[2] = *depth_min = lo;
+        counters[3] = *depth_max = hi;
     }
 }
+
+constexpr int kScanThreads = 1024;
 
 // SH degree 2 along the view ray -> 4 channels: include/sh_utils.cuh:6-23.  `h` points at 36 halves
 // (coefficient-major, channel-minor) in shared memory.
@@ -485,7 +525,7 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
                                                                           const uint32_t* __restrict__ sorted_ids,
                                                                           const uint2* __restrict__ bounds, int64_t n_visible_arg,
                                                                           const unsigned long long* __restrict__ n_visible_dev,
-                                                                          unsigned* __restrict__ block_sums) {
+                                                                          unsigned* block_sums, unsigned* done) {
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     // a block of kInstThreads / 4 threads covers kInstThreads points, four consecutive ones per thread
     // (one 16-byte load when the keys carry the count)
@@ -512,30 +552,8 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
         for (int w = 0; w < kInstThreads / 4 / 32; ++w) t += s_w[w];
         block_sums[blockIdx.x] = t;
     }
-}
-
-constexpr int kScanItems = 8;
-__global__ void __launch_bounds__(kScanThreads) scan_u32_kernel(unsigned* __restrict__ data, int64_t n) {
-    __shared__ unsigned s_scan[kScanThreads / 32 + 1];
-    unsigned running = 0;
-    for (int64_t base = 0; base < n; base += (int64_t)kScanThreads * kScanItems) {
-        const int64_t j0 = base + (int64_t)threadIdx.x * kScanItems;
-        unsigned v[kScanItems];
-        unsigned sum = 0;
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            v[k] = j0 + k < n ? data[j0 + k] : 0u;
-            sum += v[k];
-        }
-        unsigned total;
-        unsigned ex = running + block_exclusive_scan(sum, s_scan, &total);
-#pragma unroll
-        for (int k = 0; k < kScanItems; ++k) {
-            if (j0 + k < n) data[j0 + k] = ex;
-            ex += v[k];
-        }
-        running += total;
-    }
+    __shared__ unsigned s_scan[kInstThreads / 4 / 32 + 1];
+    if (last_block(done, gridDim.x)) scan_words<kInstThreads / 4>(block_sums, gridDim.x, s_scan);   // sums -> first instance of every block
 }
 
 // Instance key: the tile index in the low 24 bits, the only bits the tile sort looks at (it carries the
@@ -604,8 +622,8 @@ __global__ void __launch_bounds__(256) tile_ranges_kernel(const uint32_t* __rest
                                                           uint2* __restrict__ ranges) {
     constexpr int kPer = 8;   // two 16-byte loads per thread (the key array is 256-byte aligned)
     const int64_t n_instances = n_instances_dev ? (int64_t)*n_instances_dev : n_instances_arg;
-    const int64_t first = ((int64_t)blockIdx.x * 256 + threadIdx.x) * kPer;
-    if (first >= n_instances) return;
+    // the grid fits the chip: sized for the bound on the instance count it was three quarters empty blocks
+    for (int64_t first = ((int64_t)blockIdx.x * 256 + threadIdx.x) * kPer; first < n_instances; first += (int64_t)gridDim.x * 256 * kPer) {
     uint32_t prev = first > 0 ? __ldg(keys + first - 1) & kTileKeyMask : 0u;
     uint32_t k8[kPer];
     if (first + kPer <= n_instances) {
@@ -624,6 +642,7 @@ __global__ void __launch_bounds__(256) tile_ranges_kernel(const uint32_t* __rest
         else if (key != prev) { ranges[prev].y = (unsigned)i; ranges[key].x = (unsigned)i; }
         if (i == n_instances - 1) ranges[key].y = (unsigned)n_instances;
         prev = key;
+    }
     }
 }
 
@@ -1315,8 +1334,7 @@ __device__ __forceinline__ unsigned warp_segments(unsigned len, const SegmentLen
 }
 
 // Work lists of the warp blend.  Step 1 (one block per 1024 tiles): segments and non-empty tiles of the block's tiles.
-// Step 2 (one block): exclusive scan of those block sums; counts[0] = non-empty tiles, counts[1] = segments behind a
-// tile's first.  Step 3 (same blocks as step 1): every tile's position from its block's base and a scan inside the
+// Its last block scans those block sums; counts[0] = non-empty tiles, counts[1] = segments behind a tile's first.  Step 2 (same blocks as step 1): every tile's position from its block's base and a scan inside the
 // block, and its items.  (One block scanning all tiles took 177 us for the 129,600 tiles of a 3840x2160 image.)
 constexpr int kItemThreads = 256;
 constexpr int kItemTilesPerThread = 4;
@@ -1338,7 +1356,8 @@ __device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ran
 }
 
 __global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, unsigned long long n_instances_arg,
-                                                                        const unsigned long long* __restrict__ n_instances_dev, uint2* __restrict__ block_sums) {
+                                                                        const unsigned long long* __restrict__ n_instances_dev, uint2* block_sums, unsigned* done,
+                                                                        uint32_t* __restrict__ counts) {
     __shared__ unsigned s_seg[kItemThreads / 32], s_tiles[kItemThreads / 32];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
@@ -1360,18 +1379,16 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const ui
         for (int w = 0; w < kItemThreads / 32; ++w) { a += s_seg[w]; c += s_tiles[w]; }
         block_sums[blockIdx.x] = make_uint2(a, c);
     }
-}
-
-__global__ void __launch_bounds__(kScanThreads) warp_items_scan_kernel(uint2* __restrict__ block_sums, int n_blocks, uint32_t* __restrict__ counts) {
-    __shared__ unsigned s_scan[kScanThreads / 32 + 1];
+    if (!last_block(done, gridDim.x)) return;
+    __shared__ unsigned s_scan[kItemThreads / 32 + 1];
     unsigned run_seg = 0, run_tiles = 0;
-    for (int base = 0; base < n_blocks; base += kScanThreads) {
-        const int j = base + threadIdx.x;
-        const uint2 v = j < n_blocks ? block_sums[j] : make_uint2(0u, 0u);
+    for (unsigned base = 0; base < gridDim.x; base += kItemThreads) {
+        const unsigned j = base + threadIdx.x;
+        const uint2 v = j < gridDim.x ? __ldcg(block_sums + j) : make_uint2(0u, 0u);
         unsigned total_seg, total_tiles;
         const unsigned ex_seg = run_seg + block_exclusive_scan(v.x, s_scan, &total_seg);
         const unsigned ex_tiles = run_tiles + block_exclusive_scan(v.y, s_scan, &total_tiles);
-        if (j < n_blocks) block_sums[j] = make_uint2(ex_seg, ex_tiles);
+        if (j < gridDim.x) block_sums[j] = make_uint2(ex_seg, ex_tiles);
         run_seg += total_seg;
         run_tiles += total_tiles;
     }
@@ -1394,7 +1411,7 @@ __device__ __forceinline__ WarpItem load_item(const WarpItem* p) {
     return w;
 }
 
-// Step 3: items0 = segment 0 of the non-empty tiles, items1 = every later segment, tile by tile.
+// Step 2: items0 = segment 0 of the non-empty tiles, items1 = every later segment, tile by tile.
 __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, unsigned long long n_instances_arg,
                                                                       const unsigned long long* __restrict__ n_instances_dev,
                                                                       const uint2* __restrict__ block_base, WarpItem* __restrict__ items0,
@@ -3065,8 +3082,14 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_backward_kernel(
     const int in_block = (int)min((int64_t)kPreThreads, n - block_first);
     const int64_t i = block_first + threadIdx.x;
     __half* o = s_out + threadIdx.x * 36;
+    // With slots the mask alone says whether a point received anything: most points of a dense scene lie behind stopped pixels,
+    // and neither their bounds nor their positions are read (2^23 samples: 184 -> 165 us).
     bool touched = false;
-    if (i < n) touched = tiles_of(__ldg(bounds + i)) != 0u;
+    unsigned m = 0;
+    if (i < n) {
+        if (SLOTS) touched = (m = __ldg(slots.mask + i)) != 0u;
+        else touched = tiles_of(__ldg(bounds + i)) != 0u;
+    }
     if (touched) {
         float b[9];
         sh_basis(__ldg(positions + 3 * i), __ldg(positions + 3 * i + 1), __ldg(positions + 3 * i + 2), cam, b);
@@ -3074,7 +3097,6 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_backward_kernel(
         float4 gv = make_float4(0.f, 0.f, 0.f, 0.f);
         if (SLOTS) {
             float go = 0.0f;
-            const unsigned m = __ldg(slots.mask + i);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 if ((m >> q) & 1u) {
@@ -3135,7 +3157,8 @@ struct PointBlob {
     uint32_t* keys[2];
     uint32_t* ids[2];
     unsigned* inst_block_sums;
-    void* sort_ws;
+    unsigned* state;                      // words that start at zero: [0..1] depth range, [2..4] finished blocks of the counting passes
+    void* sort_ws;                        // directly behind `state`: cleared together
     size_t total;
 };
 
@@ -3158,6 +3181,7 @@ PointBlob carve_point_blob(void* p, int64_t n, int mode) {
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n);
     b.inst_block_sums = c.take<unsigned>(ceil_div<int64_t>(n > 0 ? n : 1, kInstThreads));
+    b.state = c.take<unsigned>(64);
     c.off = align_up(c.off);
     b.sort_ws = c.base + c.off;
     c.off += sort_workspace_bytes(n, n);
@@ -3213,7 +3237,14 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int 
     InstanceBlob b;
     Carver c(p);
     const bool warp_blend = uses_warp_blend(mode, tile);
+    // [0] segments (block blend) or non-empty tiles (warp blend), [1] later segments (warp blend), [2..5] work tickets of
+    // the warp blend passes FIRST, PRODUCT, REST and of its backward pass.  Counters, tile ranges and the sort's state lie side
+    // by side: they are cleared together.
+    b.n_segments = c.take<uint32_t>(64);
     b.ranges = c.take<uint2>(n_tiles);
+    c.off = align_up(c.off);
+    b.sort_ws = c.base + c.off;
+    c.off += sort_workspace_bytes(n_instances, likely_instances(n_instances, warp_blend));
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n_instances);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n_instances);
     // upper bound on the number of (tile, segment) pairs, known from the instance count alone
@@ -3221,9 +3252,6 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int 
     const size_t px = (size_t)b.max_segments * tile * tile;
     b.segs = c.take<Segment>(warp_blend ? 0 : b.max_segments);
     b.tile_first = c.take<uint32_t>(n_tiles);
-    // [0] segments (block blend) or non-empty tiles (warp blend), [1] later segments (warp blend), [2..5] work tickets of
-    // the warp blend passes FIRST, PRODUCT, REST and of its backward pass
-    b.n_segments = c.take<uint32_t>(8);
     b.seg_T = c.take<float>(px);
     b.seg_C = c.take<float4>(px * (size_t)c4);
     b.seg_Z = c.take<float>(with_depth ? px : 0);
@@ -3232,9 +3260,6 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int 
     b.items0 = c.take<WarpItem>(warp_blend ? (size_t)n_tiles : 0);
     b.items1 = c.take<WarpItem>(warp_blend ? (size_t)b.max_segments : 0);
     b.n_kept = c.take<uint32_t>(warp_blend ? (size_t)b.max_segments * kWarpBlendParts : 0);
-    c.off = align_up(c.off);
-    b.sort_ws = c.base + c.off;
-    c.off += sort_workspace_bytes(n_instances, likely_instances(n_instances, warp_blend));
     b.total = c.used();
     return b;
 }
@@ -3324,11 +3349,22 @@ int end_index_checks(cudaStream_t stream) {
     return INPC_OK;
 }
 
+int launch_clear(const ClearList& list, cudaStream_t stream) {
+    if (list.count == 0) return INPC_OK;
+    size_t total = 0;
+    for (int k = 0; k < list.count; ++k) total += list.bytes[k];
+    const size_t blocks = ceil_div<size_t>(total, 256 * 16 * 4), cap = (size_t)sm_count() * 8;
+    clear_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks < cap ? blocks : cap), 256, 0, stream>>>(list);
+    INPC_LAUNCH_CHECK("clear_kernel");
+    return INPC_OK;
+}
+
 template <int MODE, int VARIANT>
 int run_front(const RasterParams& rp, int64_t n, const float* positions, const void* features, const float* opacities,
               inpc_alloc_fn alloc_point, inpc_alloc_fn alloc_instance, void* user, inpc_raster_state* st,
-              bool with_depth, PointBlob* pb_out, InstanceBlob* ib_out, cudaStream_t stream, const char* entry, int c4 = 1,
+              bool with_depth, PointBlob* pb_out, InstanceBlob* ib_out, cudaStream_t stream, const char* entry, ClearList clear, int c4 = 1,
               const PointSets* sets = nullptr) {
+    // `clear`: outputs of the call that have to start at zero
     // `sets`: the input of a batched multi-set call (then n is the virtual total and the three pointers are unused)
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     PointSets ps;
@@ -3366,6 +3402,21 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     int64_t n_visible = 0, n_instances = 0;
     uint32_t key_base = 0;
     int key_bits = 0;
+    const int tile_bits = bit_length((uint32_t)(n_tiles - 1));
+    void* iblob = nullptr;
+    InstanceBlob ib;
+    auto make_instance_blob = [&]() -> int {
+        const InstanceBlob isz = carve_instance_blob(nullptr, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
+        iblob = alloc_instance(user, isz.total);
+        if (!iblob) { set_error("instance allocator returned NULL for %zu bytes", isz.total); return INPC_E_ALLOC; }
+        ib = carve_instance_blob(iblob, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
+        return INPC_OK;
+    };
+    auto clear_instance_blob = [&](ClearList& list) {
+        list.add(ib.n_segments, (size_t)(static_cast<char*>(ib.sort_ws) - reinterpret_cast<char*>(ib.n_segments)) +
+                                    sort_zero_bytes(n_instances, likely_instances(n_instances, warp_blend), tile_bits));
+    };
+    int rc;
     const unsigned long long* n_visible_dev = deferred ? pb.counters : nullptr;
     const unsigned long long* n_instances_dev = deferred ? pb.counters + 1 : nullptr;
     if (n > 0) {
@@ -3385,6 +3436,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             pack_count = key_bits <= (int)kCountShift ? 1 : 0;
             n_visible = n;                // capacities from here on
             n_instances = 4 * n;
+            rc = make_instance_blob();
+            if (rc != INPC_OK) return rc;
+            clear_instance_blob(clear);
         } else {
             host = pinned_counters();
             ready = counters_event();
@@ -3392,16 +3446,15 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         }
         {
             StageScope scope(STAGE_PREPROCESS, stream);
-            INPC_CUDA_TRY(cudaMemsetAsync(pb.depth_min, 0xFF, sizeof(unsigned), stream));
-            INPC_CUDA_TRY(cudaMemsetAsync(pb.depth_max, 0, sizeof(unsigned), stream));
+            // (non-deferred: the number of key bits is not known yet, the sort clears its own state)
+            clear.add(pb.state, (size_t)(static_cast<char*>(pb.sort_ws) - reinterpret_cast<char*>(pb.state)) + (deferred ? sort_zero_bytes(n, n, key_bits) : 0));
+            rc = launch_clear(clear, stream);
+            if (rc != INPC_OK) return rc;
             const int64_t groups = ceil_div<int64_t>(nb, 4);
-            visibility_count_kernel<MODE, VARIANT><<<(unsigned)groups, kPreThreads, 0, stream>>>(ps, rp, pb.block_visible, pb.group_visible,
-                                                                                             pb.group_instances, deferred ? nullptr : pb.depth_min,
-                                                                                             deferred ? nullptr : pb.depth_max);
+            visibility_count_kernel<MODE, VARIANT><<<(unsigned)groups, kPreThreads, 0, stream>>>(
+                ps, rp, pb.block_visible, pb.group_visible, pb.group_instances, deferred ? nullptr : pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min,
+                pb.depth_max, pb.counters);
             INPC_LAUNCH_CHECK("visibility_count_kernel");
-            scan_block_counts_kernel<<<1, kScanThreads, 0, stream>>>(pb.group_visible, pb.group_instances, groups, pb.depth_min, pb.depth_max, pb.counters,
-                                                                     deferred ? 1 : 0, lo_bits, hi_bits);
-            INPC_LAUNCH_CHECK("scan_block_counts_kernel");
             if (!deferred) {
                 INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
                 INPC_CUDA_TRY(cudaEventRecord(ready, stream));
@@ -3435,18 +3488,22 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         return INPC_E_CAPACITY;
     }
 
-    const InstanceBlob isz = carve_instance_blob(nullptr, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
-    void* iblob = alloc_instance(user, isz.total);
-    if (!iblob) { set_error("instance allocator returned NULL for %zu bytes", isz.total); return INPC_E_ALLOC; }
-    InstanceBlob ib = carve_instance_blob(iblob, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
-    INPC_CUDA_TRY(cudaMemsetAsync(ib.ranges, 0, sizeof(uint2) * (size_t)n_tiles, stream));
+    if (!deferred) {
+        // (n == 0: the outputs are cleared here, nothing has launched yet)
+        rc = make_instance_blob();
+        if (rc != INPC_OK) return rc;
+        ClearList rest;
+        if (n == 0) rest = clear;
+        clear_instance_blob(rest);
+        rc = launch_clear(rest, stream);
+        if (rc != INPC_OK) return rc;
+    }
 
     int in_alt = 0;
-    int rc;
     {
         StageScope scope(STAGE_SORT_DEPTH, stream);
-        rc = deferred ? sort_pairs_device_count(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n_visible, n_visible_dev, key_bits, pb.sort_ws, status, &in_alt, stream)
-                      : sort_pairs(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n, key_bits, pb.sort_ws, status, &in_alt, stream);
+        rc = deferred ? sort_pairs_device_count(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n_visible, n_visible_dev, key_bits, pb.sort_ws, true, status, &in_alt, stream)
+                      : sort_pairs(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n, key_bits, pb.sort_ws, false, status, &in_alt, stream);
     }
     if (rc != INPC_OK) return rc;
     const uint32_t* sorted_ids = pb.ids[in_alt];
@@ -3456,12 +3513,10 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles rides in the top key bits when the depth offsets left them free
             if (MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift)
-                instance_count_kernel<true><<<(unsigned)ibk, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums);
+                instance_count_kernel<true><<<(unsigned)ibk, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, pb.state + 3);
             else
-                instance_count_kernel<false><<<(unsigned)ibk, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums);
+                instance_count_kernel<false><<<(unsigned)ibk, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
-            scan_u32_kernel<<<1, kScanThreads, 0, stream>>>(pb.inst_block_sums, ibk);
-            INPC_LAUNCH_CHECK("scan_u32_kernel");
             if (warp_blend)
                 emit_instances_kernel<true><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             else
@@ -3470,22 +3525,19 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
-        const int tile_bits = bit_length((uint32_t)(n_tiles - 1));
-        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, warp_blend), n_instances_dev, tile_bits, ib.sort_ws, status, &t_alt, stream)
-                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, n_instances, tile_bits, ib.sort_ws, status, &t_alt, stream);
+        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, warp_blend), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream)
+                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, warp_blend), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
         if (rc != INPC_OK) return rc;
-        tile_ranges_kernel<<<(unsigned)ceil_div<int64_t>(n_instances, 256 * 8), 256, 0, stream>>>(ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
+        const int64_t range_blocks = ceil_div<int64_t>(n_instances, 256 * 8), range_cap = (int64_t)sm_count() * 8;
+        tile_ranges_kernel<<<(unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream>>>(ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
         INPC_LAUNCH_CHECK("tile_ranges_kernel");
     }
     if (warp_blend) {
         StageScope scope(STAGE_SORT_TILE, stream);
-        INPC_CUDA_TRY(cudaMemsetAsync(ib.n_segments, 0, 8 * sizeof(uint32_t), stream));
         const int item_blocks = ceil_div(n_tiles, kItemTilesPerBlock);
         uint2* item_sums = reinterpret_cast<uint2*>(ib.tile_rank);
-        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums);
+        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
         INPC_LAUNCH_CHECK("warp_items_count_kernel");
-        warp_items_scan_kernel<<<1, kScanThreads, 0, stream>>>(item_sums, item_blocks, ib.n_segments);
-        INPC_LAUNCH_CHECK("warp_items_scan_kernel");
         warp_items_fill_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
         INPC_LAUNCH_CHECK("warp_items_fill_kernel");
     } else {
@@ -3574,11 +3626,6 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const int rc = warp_blend_grid(&grid);
     if (rc != INPC_OK) return rc;
     const int W = rp.v.width, H = rp.v.height;
-    // tiles without instances are not work items: their pixels are cleared here
-    const size_t n_px = (size_t)W * H * rp.n_sets;
-    INPC_CUDA_TRY(cudaMemsetAsync(image, 0, sizeof(float) * 4 * C4 * n_px, stream));
-    INPC_CUDA_TRY(cudaMemsetAsync(alpha, 0, sizeof(float) * n_px, stream));
-    if (KIND == BLEND_INFER) INPC_CUDA_TRY(cudaMemsetAsync(depth, 0, sizeof(float) * n_px, stream));
     // the ping-pong buffers the tile sort left unused receive the compacted lists (part 0: ids, part 1: keys)
     const uint32_t* keys = ib.keys[t_alt];
     const uint32_t* ids = ib.ids[t_alt];
@@ -3607,7 +3654,6 @@ int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, c
     unsigned grid = 1;
     const int rc = warp_blend_grid(&grid);
     if (rc != INPC_OK) return rc;
-    INPC_CUDA_TRY(cudaMemsetAsync(ib.n_segments + 5, 0, sizeof(uint32_t), stream));   // the work ticket
     static bool attr_set[kMaxDevices] = {false};
     const int rc_attr = opt_in_dynamic_smem(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, attr_set);
     if (rc_attr != INPC_OK) return rc_attr;
@@ -3725,7 +3771,6 @@ int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const
     unsigned grid = 1;
     const int rc = warp_blend_grid(&grid);
     if (rc != INPC_OK) return rc;
-    INPC_CUDA_TRY(cudaMemsetAsync(ib.n_segments + 5, 0, sizeof(uint32_t), stream));   // the work ticket
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
     const int rc_attr = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
@@ -3766,6 +3811,20 @@ int dispatch_rows(int channels, F&& f) {
     return INPC_E_INVALID;
 }
 
+// The outputs of a call that start at zero.  The warp blend has no work items for tiles without instances, so their pixels
+// are cleared; the block blend writes every tile.  `depth` and `weights` may be null.
+ClearList outputs_to_clear(const RasterParams& rp, int mode, int channels, float* image, float* depth, float* alpha, float* weights, int64_t n) {
+    ClearList list;
+    if (uses_warp_blend(mode, rp.tile)) {
+        const size_t n_px = (size_t)rp.v.width * rp.v.height * rp.n_sets;
+        list.add(image, sizeof(float) * channels * n_px);
+        list.add(depth, sizeof(float) * n_px);
+        list.add(alpha, sizeof(float) * n_px);
+    }
+    list.add(weights, sizeof(float) * (size_t)n);
+    return list;
+}
+
 template <int KIND>
 int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* positions, const float* features, int channels,
                  const float* opacities, float* image, float* depth, float* alpha, float* blending_weights,
@@ -3774,7 +3833,8 @@ int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* p
     PointBlob pb;
     InstanceBlob ib;
     int rc = run_front<INPC_MODE_BILINEAR, VAR_ROWS>(rp, n, positions, nullptr, opacities, alloc_point, alloc_instance, alloc_user, state,
-                                                     KIND == BLEND_INFER, &pb, &ib, stream, KIND == BLEND_INFER ? "inpc_render_rows" : "inpc_rasterize_rows_forward", channels / 4);
+                                                     KIND == BLEND_INFER, &pb, &ib, stream, KIND == BLEND_INFER ? "inpc_render_rows" : "inpc_rasterize_rows_forward",
+                                                     outputs_to_clear(rp, INPC_MODE_BILINEAR, channels, image, depth, alpha, blending_weights, n), channels / 4);
     if (rc != INPC_OK) return rc;
     const int t_alt = tile_buffer_of(state, rp.gw * rp.gh);
     {
@@ -3807,13 +3867,13 @@ extern "C" int inpc_rasterize_forward(int mode, int tile_size, const inpc_view* 
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, 0.0f, 3.0f, nullptr);
-    if (n > 0) INPC_CUDA_TRY(cudaMemsetAsync(blending_weights, 0, sizeof(float) * (size_t)n, stream));
+    const ClearList clear = outputs_to_clear(rp, mode, 4, image, nullptr, alpha, blending_weights, n);
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
-        rc = run_front<INPC_MODE_BILINEAR, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward");
+        rc = run_front<INPC_MODE_BILINEAR, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward", clear);
     else
-        rc = run_front<INPC_MODE_GAUSSIAN, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward");
+        rc = run_front<INPC_MODE_GAUSSIAN, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward", clear);
     if (rc != INPC_OK) return rc;
     rc = launch_blend_forward<BLEND_TRAIN>(mode, rp, pb, ib, state, image, nullptr, alpha, blending_weights, kTrainGaussThreshold, stream);
     return rc != INPC_OK ? rc : end_index_checks(stream);
@@ -3852,12 +3912,16 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     }
     float4* slot_grad = gfv;
     unsigned* slot_mask = reinterpret_cast<unsigned*>(grad_features_view + 32 * (size_t)n);
+    ClearList clear;
     if (slots) {
-        INPC_CUDA_TRY(cudaMemsetAsync(slot_mask, 0, sizeof(unsigned) * (size_t)n, stream));
+        clear.add(slot_mask, sizeof(unsigned) * (size_t)n);
+        clear.add(ib.n_segments + 5, sizeof(uint32_t));   // the work ticket
     } else {
-        INPC_CUDA_TRY(cudaMemsetAsync(grad_features_view, 0, sizeof(float4) * (size_t)n, stream));
-        INPC_CUDA_TRY(cudaMemsetAsync(grad_opacities, 0, sizeof(float) * (size_t)n, stream));
+        clear.add(grad_features_view, sizeof(float4) * (size_t)n);
+        clear.add(grad_opacities, sizeof(float) * (size_t)n);
     }
+    rc = launch_clear(clear, stream);
+    if (rc != INPC_OK) return rc;
     {
         StageScope scope(STAGE_BLEND_BWD, stream);
         if (state->mode == INPC_MODE_BILINEAR) {
@@ -3898,13 +3962,14 @@ extern "C" int inpc_render(int mode, int tile_size, const inpc_view* view, int64
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, sigma_world, sigma_cutoff, nullptr);
+    const ClearList clear = outputs_to_clear(rp, mode, 4, image, depth, alpha, nullptr, n);
     inpc_raster_state st;
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
-        rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render");
+        rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render", clear);
     else
-        rc = run_front<INPC_MODE_GAUSSIAN, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render");
+        rc = run_front<INPC_MODE_GAUSSIAN, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render", clear);
     if (rc != INPC_OK) return rc;
     // runtime cut-off exp(-cutoff^2/2): src/gaussian/inference.cu:171
     const float threshold = expf(-0.5f * sigma_cutoff * sigma_cutoff);
@@ -3925,13 +3990,14 @@ extern "C" int inpc_render_preextracted(int mode, int tile_size, const inpc_view
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, sigma_world, sigma_cutoff, scales);
+    const ClearList clear = outputs_to_clear(rp, mode, 4, image, depth, alpha, nullptr, n);
     inpc_raster_state st;
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
-        rc = run_front<INPC_MODE_BILINEAR, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted");
+        rc = run_front<INPC_MODE_BILINEAR, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted", clear);
     else
-        rc = run_front<INPC_MODE_GAUSSIAN, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted");
+        rc = run_front<INPC_MODE_GAUSSIAN, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted", clear);
     if (rc != INPC_OK) return rc;
     const float threshold = expf(-0.5f * sigma_cutoff * sigma_cutoff);
     rc = launch_blend_forward<BLEND_INFER>(mode, rp, pb, ib, &st, image, depth, alpha, nullptr, threshold, stream);
@@ -3975,7 +4041,7 @@ extern "C" int inpc_render_multi(int tile_size, const inpc_view* view, int n_set
     PointBlob pb;
     InstanceBlob ib;
     rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n_virtual, nullptr, nullptr, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib,
-                                                  stream, "inpc_render_multi", 1, &ps);
+                                                  stream, "inpc_render_multi", outputs_to_clear(rp, INPC_MODE_BILINEAR, 4, images, depths, alphas, nullptr, n_virtual), 1, &ps);
     if (rc != INPC_OK) return rc;
     rc = launch_blend_forward<BLEND_INFER>(INPC_MODE_BILINEAR, rp, pb, ib, &st, images, depths, alphas, nullptr, 0.0f, stream);
     return rc != INPC_OK ? rc : end_index_checks(stream);
@@ -4002,7 +4068,6 @@ extern "C" int inpc_rasterize_rows_forward(int tile_size, const inpc_view* view,
         return INPC_E_INVALID;
     }
     if (reinterpret_cast<uintptr_t>(features) & 15u) { set_error("inpc_rasterize_rows_forward: features must be 16-byte aligned"); return INPC_E_INVALID; }
-    if (n > 0) INPC_CUDA_TRY(cudaMemsetAsync(blending_weights, 0, sizeof(float) * (size_t)n, stream));
     return rows_forward<BLEND_TRAIN>(tile_size, view, n, positions, features, channels, opacities, image, nullptr, alpha, blending_weights,
                                      alloc_point, alloc_instance, alloc_user, state, stream);
 }
@@ -4047,8 +4112,12 @@ extern "C" int inpc_rasterize_rows_backward(const inpc_raster_state* state, cons
     const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode);
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), n_tiles, state->tile_size, state->mode, false, channels / 4);
     const int t_alt = tile_buffer_of(state, n_tiles);
-    INPC_CUDA_TRY(cudaMemsetAsync(grad_features, 0, sizeof(float) * (size_t)n * channels, stream));
-    INPC_CUDA_TRY(cudaMemsetAsync(grad_opacities, 0, sizeof(float) * (size_t)n, stream));
+    ClearList clear;
+    clear.add(grad_features, sizeof(float) * (size_t)n * channels);
+    clear.add(grad_opacities, sizeof(float) * (size_t)n);
+    if (state->tile_size == 8) clear.add(ib.n_segments + 5, sizeof(uint32_t));   // the work ticket
+    rc = launch_clear(clear, stream);
+    if (rc != INPC_OK) return rc;
     rc = begin_index_checks(n, stream);
     if (rc != INPC_OK) return rc;
     {

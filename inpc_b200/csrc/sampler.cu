@@ -64,17 +64,25 @@ __device__ __forceinline__ float viewpoint_weight(const ViewParams& v, float cx,
     return 1.0f / (depth_scale * size_scale) * weight;
 }
 
+// `max_bits` (optional, zero before): bit pattern of the largest weight, for the CDF behind it.
 __global__ void __launch_bounds__(kThreads) viewpoint_weights_kernel(ViewParams v, int64_t n_cells,
                                                                      const float* __restrict__ centers,
                                                                      const int* __restrict__ levels,
                                                                      const float* __restrict__ weights,
                                                                      float initial_size, float* __restrict__ out,
-                                                                     float4* __restrict__ leaf_pack) {
+                                                                     float4* __restrict__ leaf_pack, unsigned* max_bits) {
     const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const unsigned active = __ballot_sync(0xffffffffu, l < n_cells);
     if (l >= n_cells) return;
     const float cx = __ldg(centers + 3 * l), cy = __ldg(centers + 3 * l + 1), cz = __ldg(centers + 3 * l + 2);
     const int level = __ldg(levels + l);
-    out[l] = viewpoint_weight(v, cx, cy, cz, level, __ldg(weights + l), initial_size);
+    const float w = viewpoint_weight(v, cx, cy, cz, level, __ldg(weights + l), initial_size);
+    out[l] = w;
+    if (max_bits) {
+        // NaN, infinite and non-positive weights do not take part (see to_fixed); the others order like their bit patterns
+        const unsigned m = __reduce_max_sync(active, w > 0.0f && w <= 3.402823466e38f ? __float_as_uint(w) : 0u);
+        if (lane_id() == 0 && m > 0u) atomicMax(max_bits, m);
+    }
     // centre and edge length in one 16-byte record: a draw then needs one load per leaf instead of four
     if (leaf_pack) leaf_pack[l] = make_float4(cx, cy, cz, 1.0f / scalbnf(1.0f, level) * initial_size);
 }
@@ -163,8 +171,9 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan_u64(unsigned 
 }
 
 __global__ void __launch_bounds__(kCdfThreads) cdf_chunk_sums_kernel(const float* __restrict__ w, int64_t n,
-                                                                     const unsigned* __restrict__ max_bits,
-                                                                     unsigned long long* __restrict__ chunk_sums) {
+                                                                     const unsigned* __restrict__ max_bits, unsigned* done,
+                                                                     unsigned long long* chunk_sums, unsigned long long* __restrict__ total_out,
+                                                                     float* __restrict__ sum_out) {
     __shared__ unsigned long long s[kCdfThreads / 32 + 1];
     const float w_max = __uint_as_float(__ldg(max_bits));
     const int64_t base = (int64_t)blockIdx.x * kCdfChunk + (int64_t)threadIdx.x * kCdfItems;
@@ -175,26 +184,19 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_chunk_sums_kernel(const float
     unsigned long long total;
     block_exclusive_scan_u64(acc, s, &total);
     if (threadIdx.x == 0) chunk_sums[blockIdx.x] = total;
-}
-
-// one block: exclusive scan of the chunk sums in place; total -> *total_out, fp32 sum -> *sum_out
-__global__ void __launch_bounds__(1024) cdf_scan_chunks_kernel(unsigned long long* __restrict__ chunk_sums, int64_t n_chunks,
-                                                               const unsigned* __restrict__ max_bits,
-                                                               unsigned long long* __restrict__ total_out,
-                                                               float* __restrict__ sum_out) {
-    __shared__ unsigned long long s[1024 / 32 + 1];
+    // the last block: exclusive scan of the chunk sums in place; total -> *total_out, fp32 sum -> *sum_out
+    if (!last_block(done, gridDim.x)) return;
     unsigned long long running = 0;
-    for (int64_t base = 0; base < n_chunks; base += 1024) {
-        const int64_t j = base + threadIdx.x;
-        const unsigned long long c = j < n_chunks ? chunk_sums[j] : 0ull;
-        unsigned long long total;
+    for (unsigned first = 0; first < gridDim.x; first += kCdfThreads) {
+        const unsigned j = first + threadIdx.x;
+        const unsigned long long c = j < gridDim.x ? __ldcg(chunk_sums + j) : 0ull;
         const unsigned long long ex = block_exclusive_scan_u64(c, s, &total);
-        if (j < n_chunks) chunk_sums[j] = running + ex;
+        if (j < gridDim.x) chunk_sums[j] = running + ex;
         running += total;
     }
     if (threadIdx.x == 0) {
         *total_out = running;
-        *sum_out = (float)((double)running * kFixedInv * (double)__uint_as_float(*max_bits));
+        *sum_out = (float)((double)running * kFixedInv * (double)w_max);
     }
 }
 
@@ -321,7 +323,9 @@ __device__ __forceinline__ void store_positions(float* s_pos, float x, float y, 
 }
 
 // ---- training samples: same acceptance test as src/sampling_kernels.cu:98-113 -------------------
-__global__ void __launch_bounds__(kThreads) training_samples_kernel(
+// Bound by the latency of its two dependent gathers and the integer work of Philox: six blocks per multiprocessor (40 registers)
+// hide more of it than the four that 60 registers allow.
+__global__ void __launch_bounds__(kThreads, 6) training_samples_kernel(
     ViewParams v, unsigned long long seed, unsigned long long call, const float* __restrict__ cdf,
     const uint4* __restrict__ guide, int guide_bits, const float* __restrict__ sum_ptr, unsigned n_cells,
     const float4* __restrict__ leaf_pack, int64_t n_samples, float* __restrict__ positions, long long* __restrict__ indices,
@@ -383,49 +387,43 @@ __global__ void __launch_bounds__(kThreads) draw_leaves_kernel(const float* __re
 }
 
 // ---- expected samples: src/sampling_kernels.cu:152-205 ----------------------------------------
-__global__ void __launch_bounds__(kThreads) sample_counts_kernel(const float* __restrict__ vw, const float* __restrict__ sum_ptr,
-                                                                 unsigned n_samples, int64_t n_cells, unsigned* __restrict__ counts) {
-    const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (l >= n_cells) return;
-    const float w = __ldg(vw + l);
-    const float sum = __ldg(sum_ptr);
-    int c = 0;
-    if (w > 0.0f && sum > 0.0f) {
-        const float norm = 1.0f / sum;
-        c = max(__float2int_rn(w * norm * static_cast<float>(n_samples)), 1);
-    }
-    counts[l] = (unsigned)c;
-}
-
-constexpr int kIScanThreads = 1024;
-// in-place inclusive scan of per-chunk sums is not needed: the counts array is small enough for a
-// two-level scheme (chunk sums by one kernel, one block scans them, one kernel finalises).
-__global__ void __launch_bounds__(kThreads) count_chunk_sums_kernel(const unsigned* __restrict__ counts, int64_t n,
-                                                                    unsigned* __restrict__ chunk_sums) {
-    __shared__ unsigned s[kThreads / 32];
+// Sums of the counts of kThreads leaves, exclusively scanned in place by the block that finishes last; the total -> *total_out.
+// `weights` (optional): the counts are made here, max(1, round(w / sum * n_samples)) for every leaf with a positive weight.
+__global__ void __launch_bounds__(kThreads) count_chunk_sums_kernel(const float* __restrict__ weights, const float* __restrict__ sum_ptr, unsigned n_samples,
+                                                                    unsigned* __restrict__ counts, int64_t n, unsigned* done, unsigned* chunk_sums,
+                                                                    unsigned long long* __restrict__ total_out) {
+    __shared__ unsigned s_scan[kThreads / 32 + 1];
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    unsigned c = i < n ? counts[i] : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if (lane_id() == 0) s[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned t = 0;
-        for (int w = 0; w < kThreads / 32; ++w) t += s[w];
-        chunk_sums[blockIdx.x] = t;
+    unsigned c = 0;
+    if (i < n) {
+        if (weights) {
+            const float w = __ldg(weights + i);
+            const float sum = __ldg(sum_ptr);
+            if (w > 0.0f && sum > 0.0f) {
+                const float norm = 1.0f / sum;
+                c = (unsigned)max(__float2int_rn(w * norm * static_cast<float>(n_samples)), 1);
+            }
+            counts[i] = c;
+        } else {
+            c = counts[i];
+        }
     }
-}
-
-__global__ void __launch_bounds__(kIScanThreads) scan_chunk_sums_kernel(unsigned* __restrict__ chunk_sums, int64_t n_chunks,
-                                                                        unsigned long long* __restrict__ total_out) {
-    __shared__ unsigned s_scan[kIScanThreads / 32 + 1];
+    unsigned total;
+    block_exclusive_scan(c, s_scan, &total);
+    if (threadIdx.x == 0) chunk_sums[blockIdx.x] = total;
+    if (!last_block(done, gridDim.x)) return;
     unsigned long long running = 0;
-    for (int64_t base = 0; base < n_chunks; base += kIScanThreads) {
-        const int64_t j = base + threadIdx.x;
-        const unsigned c = j < n_chunks ? chunk_sums[j] : 0u;
-        unsigned total;
-        const unsigned ex = block_exclusive_scan(c, s_scan, &total);
-        if (j < n_chunks) chunk_sums[j] = (unsigned)running + ex;
+    for (unsigned first = 0; first < gridDim.x; first += kThreads * 8) {
+        const unsigned j0 = first + threadIdx.x * 8;
+        unsigned v[8], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { v[k] = j0 + k < gridDim.x ? __ldcg(chunk_sums + j0 + k) : 0u; sum += v[k]; }
+        unsigned ex = (unsigned)running + block_exclusive_scan(sum, s_scan, &total);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (j0 + k < gridDim.x) chunk_sums[j0 + k] = ex;
+            ex += v[k];
+        }
         running += total;
     }
     if (threadIdx.x == 0) *total_out = running;
@@ -707,7 +705,7 @@ struct SamplerWs {
     float* cdf;         // (n_cells)
     unsigned long long* chunk_sums64;   // fixed-point chunk sums / bases
     unsigned long long* total64;        // fixed-point total
-    unsigned* max_bits;                 // bit pattern of the largest weight
+    unsigned* max_bits;                 // [0] bit pattern of the largest weight, [1] finished blocks of the CDF's sums, [2] of the counts': zero before
     float* sum;         // 1 float (+ padding)
     unsigned* counts;   // expected-sample counts (n_cells)
     unsigned* offsets;  // inclusive offsets (n_cells)
@@ -746,16 +744,16 @@ SamplerWs carve_sampler_ws(void* p, int64_t n_cells) {
     return w;
 }
 
-// weight sum only (expected-sample mode) or sum + CDF
-int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out, const SamplerWs& w, cudaStream_t stream) {
+// weight sum only (expected-sample mode) or sum + CDF.  `max_known`: the largest weight is in w.max_bits already.
+int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out, const SamplerWs& w, bool max_known, cudaStream_t stream) {
     const int64_t chunks = ceil_div<int64_t>(n_cells, kCdfChunk);
-    INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, sizeof(unsigned), stream));
-    cdf_max_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits);
-    INPC_LAUNCH_CHECK("cdf_max_kernel");
-    cdf_chunk_sums_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits, w.chunk_sums64);
+    if (!max_known) {
+        INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
+        cdf_max_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits);
+        INPC_LAUNCH_CHECK("cdf_max_kernel");
+    }
+    cdf_chunk_sums_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits, w.max_bits + 1, w.chunk_sums64, w.total64, sum_out);
     INPC_LAUNCH_CHECK("cdf_chunk_sums_kernel");
-    cdf_scan_chunks_kernel<<<1, 1024, 0, stream>>>(w.chunk_sums64, chunks, w.max_bits, w.total64, sum_out);
-    INPC_LAUNCH_CHECK("cdf_scan_chunks_kernel");
     if (cdf) {
         cdf_finalize_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits, w.chunk_sums64, w.total64, cdf);
         INPC_LAUNCH_CHECK("cdf_finalize_kernel");
@@ -765,6 +763,16 @@ int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out,
             INPC_LAUNCH_CHECK("guide_table_kernel");
         }
     }
+    return INPC_OK;
+}
+
+// viewpoint weights into w.vw, leaf records, the largest weight
+int view_weights(const ViewParams& v, int64_t n_cells, const float* centers, const int32_t* levels, const float* weights, float initial_size,
+                 const SamplerWs& w, cudaStream_t stream) {
+    INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
+    viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw,
+                                                                                                   w.leaf_pack, w.max_bits);
+    INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
     return INPC_OK;
 }
 
@@ -826,7 +834,7 @@ extern "C" int inpc_compute_viewpoint_weights(const inpc_view* view, int64_t n_c
     if (rc != INPC_OK) return rc;
     if (!out) { set_error("inpc_compute_viewpoint_weights: null output"); return INPC_E_INVALID; }
     viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(
-        to_params(view), n_cells, centers, levels, weights, initial_size, out, nullptr);
+        to_params(view), n_cells, centers, levels, weights, initial_size, out, nullptr, nullptr);
     INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
     return INPC_OK;
 }
@@ -855,7 +863,7 @@ extern "C" int inpc_build_cdf(const float* weights, int64_t n_cells, float* cdf,
                               void* stream_) {
     if (n_cells <= 0 || !weights || !cdf || !sum_out || !workspace) { set_error("inpc_build_cdf: bad argument"); return INPC_E_INVALID; }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
-    return build_cdf(weights, n_cells, cdf, sum_out, w, static_cast<cudaStream_t>(stream_));
+    return build_cdf(weights, n_cells, cdf, sum_out, w, false, static_cast<cudaStream_t>(stream_));
 }
 
 extern "C" int inpc_draw_leaves(const float* cdf, int64_t n_cells, const float* u, int64_t n, int64_t* out, void* stream_) {
@@ -880,9 +888,9 @@ extern "C" int inpc_generate_training_samples(inpc_sampler* s, const inpc_view* 
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     const ViewParams v = to_params(view);
     StageScope scope(STAGE_SAMPLE, stream);
-    viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw, w.leaf_pack);
-    INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
-    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, stream);
+    rc = view_weights(v, n_cells, centers, levels, weights, initial_size, w, stream);
+    if (rc != INPC_OK) return rc;
+    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, true, stream);
     if (rc != INPC_OK) return rc;
     unsigned* status = acquire_status("inpc_generate_training_samples", &s->training_ticket);
     if (!status) return INPC_E_CUDA;
@@ -905,9 +913,9 @@ extern "C" int inpc_generate_samples(inpc_sampler* s, const inpc_view* view, int
     if (n_samples < 0 || n_samples >= ((int64_t)1 << 32) || !workspace || (n_samples > 0 && !positions)) { set_error("inpc_generate_samples: bad argument"); return INPC_E_INVALID; }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     const ViewParams v = to_params(view);
-    viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw, w.leaf_pack);
-    INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
-    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, stream);
+    rc = view_weights(v, n_cells, centers, levels, weights, initial_size, w, stream);
+    if (rc != INPC_OK) return rc;
+    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, true, stream);
     if (rc != INPC_OK) return rc;
     float* host = pinned_float();
     if (!host) return cuda_fail(cudaGetLastError(), "cudaHostAlloc");
@@ -937,16 +945,12 @@ extern "C" int inpc_generate_expected_samples_count(inpc_sampler* s, const inpc_
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     const ViewParams v = to_params(view);
     const unsigned blocks = (unsigned)ceil_div<int64_t>(n_cells, kThreads);
-    viewpoint_weights_kernel<<<blocks, kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw, w.leaf_pack);
-    INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
-    rc = build_cdf(w.vw, n_cells, nullptr, w.sum, w, stream);
+    rc = view_weights(v, n_cells, centers, levels, weights, initial_size, w, stream);
     if (rc != INPC_OK) return rc;
-    sample_counts_kernel<<<blocks, kThreads, 0, stream>>>(w.vw, w.sum, (unsigned)n_samples, n_cells, w.counts);
-    INPC_LAUNCH_CHECK("sample_counts_kernel");
-    count_chunk_sums_kernel<<<blocks, kThreads, 0, stream>>>(w.counts, n_cells, w.chunk_sums);
+    rc = build_cdf(w.vw, n_cells, nullptr, w.sum, w, true, stream);
+    if (rc != INPC_OK) return rc;
+    count_chunk_sums_kernel<<<blocks, kThreads, 0, stream>>>(w.vw, w.sum, (unsigned)n_samples, w.counts, n_cells, w.max_bits + 2, w.chunk_sums, w.total);
     INPC_LAUNCH_CHECK("count_chunk_sums_kernel");
-    scan_chunk_sums_kernel<<<1, kIScanThreads, 0, stream>>>(w.chunk_sums, blocks, w.total);
-    INPC_LAUNCH_CHECK("scan_chunk_sums_kernel");
     count_offsets_kernel<<<blocks, kThreads, 0, stream>>>(w.counts, n_cells, w.chunk_sums, w.offsets);
     INPC_LAUNCH_CHECK("count_offsets_kernel");
     unsigned long long* host = reinterpret_cast<unsigned long long*>(pinned_float());
@@ -981,10 +985,9 @@ namespace {
 // inclusive offsets of w.counts into w.offsets
 int scan_counts(const SamplerWs& w, int64_t n_cells, cudaStream_t stream) {
     const unsigned blocks = (unsigned)ceil_div<int64_t>(n_cells, kThreads);
-    count_chunk_sums_kernel<<<blocks, kThreads, 0, stream>>>(w.counts, n_cells, w.chunk_sums);
+    INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
+    count_chunk_sums_kernel<<<blocks, kThreads, 0, stream>>>(nullptr, nullptr, 0u, w.counts, n_cells, w.max_bits + 2, w.chunk_sums, w.total);
     INPC_LAUNCH_CHECK("count_chunk_sums_kernel");
-    scan_chunk_sums_kernel<<<1, kIScanThreads, 0, stream>>>(w.chunk_sums, blocks, w.total);
-    INPC_LAUNCH_CHECK("scan_chunk_sums_kernel");
     count_offsets_kernel<<<blocks, kThreads, 0, stream>>>(w.counts, n_cells, w.chunk_sums, w.offsets);
     INPC_LAUNCH_CHECK("count_offsets_kernel");
     return INPC_OK;
@@ -999,7 +1002,7 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
         return INPC_E_INVALID;
     }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
-    int rc = build_cdf(weights, n_cells, w.cdf, w.sum, w, stream);
+    int rc = build_cdf(weights, n_cells, w.cdf, w.sum, w, false, stream);
     if (rc != INPC_OK) return rc;
     INPC_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * (size_t)n_cells, stream));
     float* host = pinned_float();
@@ -1072,7 +1075,7 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
     }
     unsigned* status = acquire_status("inpc_morton_order");
     if (!status) return INPC_E_CUDA;
-    const int rc = sort_pairs(codes[0], codes[1], order[0], order[1], n, n, 30, sort_ws, status, &in_alt, stream);
+    const int rc = sort_pairs(codes[0], codes[1], order[0], order[1], n, n, 30, sort_ws, false, status, &in_alt, stream);
     if (rc != INPC_OK) return rc;
     gather_positions_kernel<<<(unsigned)ceil_div<int64_t>(n, kThreads), kThreads, 0, stream>>>(positions, order[in_alt], n, out);
     INPC_LAUNCH_CHECK("gather_positions_kernel");

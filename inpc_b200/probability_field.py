@@ -49,12 +49,7 @@ class LeafStatistics:
             _cabi.check(_cabi.lib().inpc_leaf_stats_reset(_ptr(self.stats), self.stats.shape[0], _stream()))
 
     def accumulate(self, indices: torch.Tensor, weights: torch.Tensor) -> None:
-        if not indices.is_cuda or indices.dtype != torch.int64:
-            raise TypeError("indices must be a CUDA int64 tensor")
-        weights = _cuda_f32(weights.reshape(-1), "weights")
-        indices = indices.contiguous()
-        if indices.numel() != weights.numel():
-            raise ValueError("indices and weights must have the same number of elements")
+        indices, weights = _sample_args(indices, weights)
         with _on(self.stats.device):
             _cabi.check(_cabi.lib().inpc_leaf_stats_accumulate(_ptr(indices), _ptr(weights), indices.numel(), _ptr(self.stats),
                                                                self.stats.shape[0], _stream()))
@@ -66,12 +61,26 @@ class LeafStatistics:
         dist.all_reduce(self.stats, op=dist.ReduceOp.MAX, group=group)
 
 
-def update(leaf_weights: torch.Tensor, leaf_subdivision_scores: torch.Tensor, stats: LeafStatistics,
-           decay: float = DECAY) -> None:
-    """In-place `ProbabilityField.update` from accumulated statistics."""
+def _check_occupancy(leaf_weights: torch.Tensor, leaf_subdivision_scores: torch.Tensor) -> None:
     for t, name in ((leaf_weights, "leaf_weights"), (leaf_subdivision_scores, "leaf_subdivision_scores")):
         if not t.is_cuda or t.dtype != torch.float32 or not t.is_contiguous():
             raise TypeError(f"{name} must be a contiguous CUDA float32 tensor")
+
+
+def _sample_args(indices: torch.Tensor, weights: torch.Tensor):
+    if not indices.is_cuda or indices.dtype != torch.int64:
+        raise TypeError("indices must be a CUDA int64 tensor")
+    weights = _cuda_f32(weights.reshape(-1), "weights")
+    indices = indices.contiguous()
+    if indices.numel() != weights.numel():
+        raise ValueError("indices and weights must have the same number of elements")
+    return indices, weights
+
+
+def update(leaf_weights: torch.Tensor, leaf_subdivision_scores: torch.Tensor, stats: LeafStatistics,
+           decay: float = DECAY) -> None:
+    """In-place `ProbabilityField.update` from accumulated statistics."""
+    _check_occupancy(leaf_weights, leaf_subdivision_scores)
     with _on(leaf_weights.device):
         _cabi.check(_cabi.lib().inpc_leaf_update(_ptr(leaf_weights), _ptr(leaf_subdivision_scores), _ptr(stats.stats),
                                                  leaf_weights.numel(), float(decay), _stream()))
@@ -80,9 +89,12 @@ def update(leaf_weights: torch.Tensor, leaf_subdivision_scores: torch.Tensor, st
 def update_from_samples(leaf_weights: torch.Tensor, leaf_subdivision_scores: torch.Tensor, indices: torch.Tensor,
                         weights: torch.Tensor, decay: float = DECAY) -> None:
     """Drop-in for `ProbabilityField.update(indices, weights)` on the module's two leaf buffers."""
-    stats = LeafStatistics(leaf_weights.numel(), leaf_weights.device)
-    stats.accumulate(indices, weights)
-    update(leaf_weights, leaf_subdivision_scores, stats, decay)
+    _check_occupancy(leaf_weights, leaf_subdivision_scores)
+    indices, weights = _sample_args(indices, weights)
+    with _on(leaf_weights.device):
+        stats = torch.empty((leaf_weights.numel(), 2), dtype=torch.int32, device=leaf_weights.device)
+        _cabi.check(_cabi.lib().inpc_leaf_update_from_samples(_ptr(indices), _ptr(weights), indices.numel(), _ptr(stats), _ptr(leaf_weights),
+                                                              _ptr(leaf_subdivision_scores), leaf_weights.numel(), float(decay), _stream()))
 
 
 MAX_LEVEL = 6                 # ProbabilityField.py:220
