@@ -213,11 +213,13 @@ __device__ __forceinline__ void bulk_store_from_shared(void* dst_global, const v
 // Every block calls this behind its last write; true in all threads of the last one.  `done` starts at zero.
 __device__ __forceinline__ bool last_block(unsigned* done, unsigned n_blocks) {
     __shared__ bool s_last;
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == n_blocks - 1u;
+    if (threadIdx.x == 0) {
+        __threadfence();   // covers the whole block's writes: they are ordered before it by the barrier
+        s_last = atomicAdd(done, 1u) == n_blocks - 1u;
+        __threadfence();
+    }
     __syncthreads();
-    if (s_last) __threadfence();
     return s_last;
 }
 

@@ -54,7 +54,6 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
     if ((int64_t)blockIdx.x * kHistItemsPerBlock >= n) return;
     __shared__ unsigned s_hist[kMaxPasses][kRadix];
     __shared__ unsigned s_scan[kHistThreads / 32 + 1];
-    __shared__ bool s_last;
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads) (&s_hist[0][0])[i] = 0;
     __syncthreads();
 
@@ -79,16 +78,8 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
         const unsigned c = (&s_hist[0][0])[i];
         if (c) atomicAdd(hist + i, c);
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int64_t all = ceil_div<int64_t>(n, kHistItemsPerBlock);
-        const unsigned working = (unsigned)min(all, (int64_t)gridDim.x);
-        s_last = atomicAdd(blocks_done, 1u) == working - 1u;
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
+    const int64_t all = ceil_div<int64_t>(n, kHistItemsPerBlock);
+    if (!last_block(blocks_done, (unsigned)min(all, (int64_t)gridDim.x))) return;
     for (int p = 0; p < pt.n_passes; ++p) {
         unsigned total;
         const unsigned ex = block_exclusive_scan(__ldcg(hist + p * kRadix + threadIdx.x), s_scan, &total);
@@ -138,6 +129,7 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
     using Smem = PassSmem<BITS, ITEMS>;
     constexpr int kBins = Smem::kBins;
     constexpr unsigned kTile = kThreads * ITEMS;
+    constexpr unsigned kFull = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
 
@@ -185,13 +177,20 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
             const unsigned d = (key[i] >> shift) & digit_mask;
-            atomicOr(my_match + d, 1u << lane);
             const unsigned before = my_count[d];
-            __syncwarp();
-            const unsigned peers = my_match[d];
-            pos[i] = before + __popc(peers & lt_mask);
-            __syncwarp();
-            if ((peers >> lane) == 1u) { my_count[d] = pos[i] + 1u; my_match[d] = 0u; }   // the last lane with this digit
+            if (__all_sync(kFull, d == __shfl_sync(kFull, d, 0))) {
+                // one digit in the whole row, as in keys that are nearly in order: 32 atomics on one word would go one by one
+                pos[i] = before + lane;
+                __syncwarp();
+                if (lane == 31u) my_count[d] = before + 32u;
+            } else {
+                atomicOr(my_match + d, 1u << lane);
+                __syncwarp();
+                const unsigned peers = my_match[d];
+                pos[i] = before + __popc(peers & lt_mask);
+                __syncwarp();
+                if ((peers >> lane) == 1u) { my_count[d] = pos[i] + 1u; my_match[d] = 0u; }   // the last lane with this digit
+            }
             __syncwarp();
         }
         uint32_t val[ITEMS];

@@ -336,6 +336,7 @@ __global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
     __shared__ unsigned s_scan[kPreThreads / 32 + 1];
     const unsigned visible = scan_words<kPreThreads>(group_visible, gridDim.x, s_scan);
     unsigned long long inst = 0;
+#pragma unroll 8
     for (unsigned k = threadIdx.x; k < gridDim.x; k += kPreThreads) inst += __ldcg(group_instances + k);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
@@ -525,35 +526,37 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
                                                                           const uint32_t* __restrict__ sorted_ids,
                                                                           const uint2* __restrict__ bounds, int64_t n_visible_arg,
                                                                           const unsigned long long* __restrict__ n_visible_dev,
-                                                                          unsigned* block_sums, unsigned* done) {
+                                                                          unsigned* block_sums, unsigned n_groups, unsigned* done) {
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     // a block of kInstThreads / 4 threads covers kInstThreads points, four consecutive ones per thread
-    // (one 16-byte load when the keys carry the count)
-    __shared__ unsigned s_w[kInstThreads / 4 / 32];
-    const int64_t first = (int64_t)blockIdx.x * kInstThreads + 4 * (int64_t)threadIdx.x;
-    unsigned c = 0;
-    if (PACKED && first + 4 <= n_visible) {
-        const uint4 k = __ldg(reinterpret_cast<const uint4*>(sorted_keys + first));   // the key buffers are 16-byte aligned
-        c = (k.x >> kCountShift) + (k.y >> kCountShift) + (k.z >> kCountShift) + (k.w >> kCountShift) + 4u;
-    } else {
+    // (one 16-byte load when the keys carry the count), and takes several such groups one after the other
+    __shared__ unsigned s_w[2][kInstThreads / 4 / 32];
+    int flip = 0;
+    for (unsigned group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1) {
+        const int64_t first = (int64_t)group * kInstThreads + 4 * (int64_t)threadIdx.x;
+        unsigned c = 0;
+        if (PACKED && first + 4 <= n_visible) {
+            const uint4 k = __ldg(reinterpret_cast<const uint4*>(sorted_keys + first));   // the key buffers are 16-byte aligned
+            c = (k.x >> kCountShift) + (k.y >> kCountShift) + (k.z >> kCountShift) + (k.w >> kCountShift) + 4u;
+        } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int64_t s = first + q;
-            if (s < n_visible) c += PACKED ? (__ldg(sorted_keys + s) >> kCountShift) + 1u : tiles_of(__ldg(bounds + checked_point(__ldg(sorted_ids + s))));
+            for (int q = 0; q < 4; ++q) {
+                const int64_t s = first + q;
+                if (s < n_visible) c += PACKED ? (__ldg(sorted_keys + s) >> kCountShift) + 1u : tiles_of(__ldg(bounds + checked_point(__ldg(sorted_ids + s))));
+            }
+        }
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane_id() == 0) s_w[flip][threadIdx.x >> 5] = c;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned t = 0;
+#pragma unroll
+            for (int w = 0; w < kInstThreads / 4 / 32; ++w) t += s_w[flip][w];
+            block_sums[group] = t;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if (lane_id() == 0) s_w[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned t = 0;
-#pragma unroll
-        for (int w = 0; w < kInstThreads / 4 / 32; ++w) t += s_w[w];
-        block_sums[blockIdx.x] = t;
-    }
     __shared__ unsigned s_scan[kInstThreads / 4 / 32 + 1];
-    if (last_block(done, gridDim.x)) scan_words<kInstThreads / 4>(block_sums, gridDim.x, s_scan);   // sums -> first instance of every block
+    if (last_block(done, gridDim.x)) scan_words<kInstThreads / 4>(block_sums, n_groups, s_scan);   // sums -> first instance of every block
 }
 
 // Instance key: the tile index in the low 24 bits, the only bits the tile sort looks at (it carries the
@@ -3508,14 +3511,15 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     if (rc != INPC_OK) return rc;
     const uint32_t* sorted_ids = pb.ids[in_alt];
     if (n_visible > 0 && n_instances > 0) {
-        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads);
+        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_cap = (int64_t)sm_count() * 8;
+        const unsigned count_blocks = (unsigned)(ibk < count_cap ? ibk : count_cap);
         {
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles rides in the top key bits when the depth offsets left them free
             if (MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift)
-                instance_count_kernel<true><<<(unsigned)ibk, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, pb.state + 3);
+                instance_count_kernel<true><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             else
-                instance_count_kernel<false><<<(unsigned)ibk, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, pb.state + 3);
+                instance_count_kernel<false><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (warp_blend)
                 emit_instances_kernel<true><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);

@@ -224,14 +224,25 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_finalize_kernel(const float* 
 }
 
 // ---- Philox4x32-10 ----------------------------------------------------------------------------
-__device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint2 k) {
+// The ten round keys are the same for all threads of a launch: the host makes them, the kernels read them from the
+// constant bank as operands of the xors.
+struct PhiloxKeys {
+    uint2 k[10];
+    unsigned call_lo, call_hi;
+};
+PhiloxKeys philox_keys(unsigned long long seed, unsigned long long call) {
+    PhiloxKeys p;
+    unsigned x = (unsigned)seed, y = (unsigned)(seed >> 32);
+    for (int r = 0; r < 10; ++r, x += 0x9E3779B9u, y += 0xBB67AE85u) p.k[r] = make_uint2(x, y);
+    p.call_lo = (unsigned)call;
+    p.call_hi = (unsigned)(call >> 32);
+    return p;
+}
+__device__ __forceinline__ uint4 philox4x32_10(uint4 c, const PhiloxKeys& keys) {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        const unsigned hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-        const unsigned hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-        c = make_uint4(hi1 ^ c.y ^ k.x, lo1, hi0 ^ c.w ^ k.y, lo0);
-        k.x += 0x9E3779B9u;
-        k.y += 0xBB67AE85u;
+        const unsigned long long p0 = (unsigned long long)0xD2511F53u * c.x, p1 = (unsigned long long)0xCD9E8D57u * c.z;
+        c = make_uint4((unsigned)(p1 >> 32) ^ c.y ^ keys.k[r].x, (unsigned)p1, (unsigned)(p0 >> 32) ^ c.w ^ keys.k[r].y, (unsigned)p0);
     }
     return c;
 }
@@ -244,9 +255,8 @@ struct Draw {
     unsigned raw_u;   // the 32 bits u was made of
 };
 // stream layout: counter = (slot, attempt, call lo, call hi), key = seed (lo, hi)
-__device__ __forceinline__ Draw philox_draw(unsigned long long seed, unsigned long long call, unsigned slot, unsigned attempt) {
-    const uint4 o = philox4x32_10(make_uint4(slot, attempt, (unsigned)call, (unsigned)(call >> 32)),
-                                  make_uint2((unsigned)seed, (unsigned)(seed >> 32)));
+__device__ __forceinline__ Draw philox_draw(const PhiloxKeys& keys, unsigned slot, unsigned attempt) {
+    const uint4 o = philox4x32_10(make_uint4(slot, attempt, keys.call_lo, keys.call_hi), keys);
     Draw d;
     d.u = unit_float(o.x); d.jx = unit_float(o.y); d.jy = unit_float(o.z); d.jz = unit_float(o.w);
     d.raw_u = o.x;
@@ -326,7 +336,7 @@ __device__ __forceinline__ void store_positions(float* s_pos, float x, float y, 
 // Bound by the latency of its two dependent gathers and the integer work of Philox: six blocks per multiprocessor (40 registers)
 // hide more of it than the four that 60 registers allow.
 __global__ void __launch_bounds__(kThreads, 6) training_samples_kernel(
-    ViewParams v, unsigned long long seed, unsigned long long call, const float* __restrict__ cdf,
+    ViewParams v, const __grid_constant__ PhiloxKeys keys, const float* __restrict__ cdf,
     const uint4* __restrict__ guide, int guide_bits, const float* __restrict__ sum_ptr, unsigned n_cells,
     const float4* __restrict__ leaf_pack, int64_t n_samples, float* __restrict__ positions, long long* __restrict__ indices,
     volatile unsigned* status) {
@@ -343,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 6) training_samples_kernel(
         unsigned leaf = 0;
         bool ok = false;
         for (unsigned a = 0; a < (unsigned)kMaxAttempts && !ok; ++a) {
-            const Draw d = philox_draw(seed, call, (unsigned)s, a);
+            const Draw d = philox_draw(keys, (unsigned)s, a);
             leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
             const float4 lp = __ldg(leaf_pack + leaf);
             x = fmaf(d.jx - 0.5f, lp.w, lp.x);
@@ -365,14 +375,14 @@ __global__ void __launch_bounds__(kThreads, 6) training_samples_kernel(
 }
 
 // ---- unconditional samples: src/sampling_kernels.cu:128-150 with the Philox stream ----------------
-__global__ void __launch_bounds__(kThreads) samples_kernel(unsigned long long seed, unsigned long long call,
+__global__ void __launch_bounds__(kThreads) samples_kernel(const __grid_constant__ PhiloxKeys keys,
                                                            const float* __restrict__ cdf, const uint4* __restrict__ guide,
                                                            int guide_bits, unsigned n_cells,
                                                            const float4* __restrict__ leaf_pack, int64_t n_samples,
                                                            float* __restrict__ positions) {
     __shared__ __align__(16) float s_pos[3 * kThreads];
     const int64_t block_first = (int64_t)blockIdx.x * kThreads;
-    const Draw d = philox_draw(seed, call, (unsigned)(block_first + threadIdx.x), 0u);
+    const Draw d = philox_draw(keys, (unsigned)(block_first + threadIdx.x), 0u);
     const unsigned leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
     const float4 lp = __ldg(leaf_pack + leaf);
     store_positions(s_pos, fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), block_first, n_samples, positions);
@@ -505,7 +515,7 @@ __device__ __forceinline__ unsigned leaf_of_slot(const LeafRun& run, const unsig
 
 // slot i jitters inside leaf upper_bound(offsets, i % n_created): the load-balanced form of the reference's per-leaf fill
 // loop + gather.  blockIdx.y counts the copies i / n_created, whose slots a run never leaves.
-__global__ void __launch_bounds__(kThreads) expected_samples_kernel(unsigned long long seed, unsigned long long call,
+__global__ void __launch_bounds__(kThreads) expected_samples_kernel(const __grid_constant__ PhiloxKeys keys,
                                                                     const unsigned* __restrict__ offsets, unsigned n_cells,
                                                                     const float4* __restrict__ leaf_pack, unsigned n_created,
                                                                     unsigned n_copies, float* __restrict__ positions) {
@@ -519,7 +529,7 @@ __global__ void __launch_bounds__(kThreads) expected_samples_kernel(unsigned lon
         for (unsigned k0 = 0; k0 < in_block; k0 += kThreads) {
             const unsigned r = min(r0 + k0 + threadIdx.x, n_created - 1u);
             const float4 lp = __ldg(leaf_pack + leaf_of_slot(run, offsets, r));
-            const Draw d = philox_draw(seed, call, (unsigned)(copy_first + r), 0u);
+            const Draw d = philox_draw(keys, (unsigned)(copy_first + r), 0u);
             store_positions(s_pos, fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), copy_first + r0 + k0,
                             copy_end, positions);
             __syncthreads();
@@ -530,40 +540,69 @@ __global__ void __launch_bounds__(kThreads) expected_samples_kernel(unsigned lon
 // ---- global point cloud: Modules/ProbabilityField.py:121-144 + utils.py:36-64 -----------------------
 // counts[leaf] = number of the n multinomial draws that fell into the leaf (torch.multinomial +
 // bincount in the reference; here the library's own Philox stream, one draw per slot)
-__global__ void __launch_bounds__(kThreads) leaf_histogram_kernel(unsigned long long seed, unsigned long long call,
+constexpr int kDrawsPerThread = 4;
+__global__ void __launch_bounds__(kThreads) leaf_histogram_kernel(const __grid_constant__ PhiloxKeys keys,
                                                                   const float* __restrict__ cdf, const uint4* __restrict__ guide,
                                                                   int guide_bits, unsigned n_cells, int64_t n_samples,
                                                                   unsigned* __restrict__ counts) {
-    const int64_t s = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (s >= n_samples) return;
-    const Draw d = philox_draw(seed, call, (unsigned)s, 0u);
-    atomicAdd(counts + guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells), 1u);
+    // the table gathers of a thread's draws are in flight together
+    const int64_t first = (int64_t)blockIdx.x * (kThreads * kDrawsPerThread) + threadIdx.x;
+    unsigned leaf[kDrawsPerThread];
+#pragma unroll
+    for (int k = 0; k < kDrawsPerThread; ++k) {
+        const Draw d = philox_draw(keys, (unsigned)(first + k * kThreads), 0u);
+        leaf[k] = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
+    }
+#pragma unroll
+    for (int k = 0; k < kDrawsPerThread; ++k)
+        if (first + k * kThreads < n_samples) atomicAdd(counts + leaf[k], 1u);
 }
 
 // Element `index` (1-based) of the Halton sequence in base B, with the reference's arithmetic (utils.py:36-46): double
 // precision, one rounding per product, sum and division f = f / B; the value is then stored as float32 (utils.py:52-55).
 // The scale factors f do not depend on the index: they are divided out at compile time, with the same roundings.
-template <unsigned B>
-struct HaltonScale {
-    static constexpr int kDigits = B == 3u ? 21 : 14;   // digits of 2^32 - 1
-    double f[kDigits];
-    constexpr HaltonScale() : f() {
+// They, and the sums over every value of the first kHead digits (in the same order), are tables: most indices are settled by
+// one look-up, the others add one table entry per further digit.
+// DIGITS: digits of 2^32 - 1.
+template <unsigned B, int HEAD, int DIGITS>
+struct HaltonTable {
+    static constexpr unsigned kBase = B;
+    static constexpr int kHead = HEAD;         // digits summed up in advance
+    static constexpr unsigned kHeads = B == 3u ? 81u : 125u;   // B^HEAD
+    double head[kHeads];
+    double term[DIGITS][B];                    // digit value * f
+    constexpr HaltonTable() : head(), term() {
         double v = 1.0;
-        for (int k = 0; k < kDigits; ++k) { v = v / (double)B; f[k] = v; }
+        for (int k = 0; k < DIGITS; ++k) {
+            v = v / (double)B;
+            for (unsigned d = 0; d < B; ++d) term[k][d] = v * (double)d;
+        }
+        for (unsigned h = 0; h < kHeads; ++h) {
+            double r = 0.0;
+            unsigned i = h;
+            for (int k = 0; k < HEAD; ++k) { r = r + term[k][i % B]; i /= B; }
+            head[h] = r;
+        }
     }
 };
-template <unsigned B>
-__device__ __forceinline__ float halton_element(unsigned index) {
+struct HaltonTables {
+    HaltonTable<3u, 4, 21> b3;
+    HaltonTable<5u, 3, 14> b5;
+};
+static_assert(sizeof(HaltonTables) % 8 == 0, "copied as doubles");
+__device__ const HaltonTables g_halton{};
+
+__device__ __forceinline__ float halton_base2(unsigned index) {
     // in base 2 every term is a power of two and every sum exact: the value is the reversed index, rounded once
-    if (B == 2u) return __uint2float_rn(__brev(index)) * 2.3283064365386962890625e-10f;
-    constexpr HaltonScale<B> scale;
-    double result = 0.0;
-    unsigned i = index;
-#pragma unroll
-    for (int k = 0; k < HaltonScale<B>::kDigits; ++k) {
-        if (i == 0u) break;
-        result = __dadd_rn(result, __dmul_rn(scale.f[k], (double)(i % B)));
-        i /= B;
+    return __uint2float_rn(__brev(index)) * 2.3283064365386962890625e-10f;
+}
+template <typename Table>
+__device__ __forceinline__ float halton_element(const Table& t, unsigned index) {
+    double result = t.head[index % Table::kHeads];
+    unsigned i = index / Table::kHeads;
+    for (int k = Table::kHead; i > 0u; ++k) {
+        result = __dadd_rn(result, t.term[k][i % Table::kBase]);
+        i /= Table::kBase;
     }
     return __double2float_rn(result);
 }
@@ -577,6 +616,9 @@ __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned
                                                                   float* __restrict__ positions) {
     __shared__ LeafRun run;
     __shared__ __align__(16) float s_pos[3 * kThreads];
+    __shared__ double s_tables[sizeof(HaltonTables) / 8];
+    const HaltonTables& tables = *reinterpret_cast<const HaltonTables*>(s_tables);
+    for (unsigned k = threadIdx.x; k < sizeof(HaltonTables) / 8; k += kThreads) s_tables[k] = reinterpret_cast<const double*>(&g_halton)[k];
     const unsigned r0 = blockIdx.x * (unsigned)kRunSlots;
     const unsigned in_block = min((unsigned)kRunSlots, n_total - r0);
     find_leaf_run(run, offsets, n_cells, r0, r0 + in_block - 1u);
@@ -591,9 +633,9 @@ __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned
             // operation rounds on its own like the torch expression  centre - cell/2 + halton * cell
             const float cell = __fdiv_rn(initial_size, (float)(1u << __ldg(levels + leaf)));
             const float half = __fmul_rn(cell, 0.5f);
-            x = __fadd_rn(__fsub_rn(x, half), __fmul_rn(halton_element<2>(h + 1u), cell));
-            y = __fadd_rn(__fsub_rn(y, half), __fmul_rn(halton_element<3>(h + 1u), cell));
-            z = __fadd_rn(__fsub_rn(z, half), __fmul_rn(halton_element<5>(h + 1u), cell));
+            x = __fadd_rn(__fsub_rn(x, half), __fmul_rn(halton_base2(h + 1u), cell));
+            y = __fadd_rn(__fsub_rn(y, half), __fmul_rn(halton_element(tables.b3, h + 1u), cell));
+            z = __fadd_rn(__fsub_rn(z, half), __fmul_rn(halton_element(tables.b5, h + 1u), cell));
         }
         store_positions(s_pos, x, y, z, (int64_t)r0 + k0, n_total, positions);
         __syncthreads();
@@ -895,7 +937,7 @@ extern "C" int inpc_generate_training_samples(inpc_sampler* s, const inpc_view* 
     unsigned* status = acquire_status("inpc_generate_training_samples", &s->training_ticket);
     if (!status) return INPC_E_CUDA;
     training_samples_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream>>>(
-        v, s->seed, s->counter, w.cdf, w.guide, w.guide_bits, w.sum, (unsigned)n_cells, w.leaf_pack, n_samples, positions,
+        v, philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, w.sum, (unsigned)n_cells, w.leaf_pack, n_samples, positions,
         reinterpret_cast<long long*>(indices), status);
     INPC_LAUNCH_CHECK("training_samples_kernel");
     s->counter += 1;
@@ -924,7 +966,7 @@ extern "C" int inpc_generate_samples(inpc_sampler* s, const inpc_view* view, int
     if (!(host[0] > 0.0f)) return INPC_OK;   // src/sampling_api.cu:154: empty result
     if (n_samples > 0) {
         samples_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream>>>(
-            s->seed, s->counter, w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, w.leaf_pack, n_samples, positions);
+            philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, w.leaf_pack, n_samples, positions);
         INPC_LAUNCH_CHECK("samples_kernel");
     }
     s->counter += 1;
@@ -974,7 +1016,7 @@ extern "C" int inpc_generate_expected_samples_fill(inpc_sampler* s, int64_t n_ce
     }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     const dim3 grid((unsigned)ceil_div<int64_t>(n_created, kRunSlots), (unsigned)(n_multi < 65535 ? n_multi : 65535));
-    expected_samples_kernel<<<grid, kThreads, 0, stream>>>(s->seed, s->counter, w.offsets, (unsigned)n_cells, w.leaf_pack, (unsigned)n_created,
+    expected_samples_kernel<<<grid, kThreads, 0, stream>>>(philox_keys(s->seed, s->counter), w.offsets, (unsigned)n_cells, w.leaf_pack, (unsigned)n_created,
                                                            (unsigned)n_multi, positions);
     INPC_LAUNCH_CHECK("expected_samples_kernel");
     s->counter += 1;
@@ -1011,8 +1053,8 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
     if (!(host[0] > 0.0f)) { set_error("inpc_draw_leaf_counts: the weights sum to zero"); return INPC_E_INVALID; }
     if (n_samples > 0) {
-        leaf_histogram_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream>>>(
-            s->seed, s->counter, w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, n_samples, counts);
+        leaf_histogram_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads * kDrawsPerThread), kThreads, 0, stream>>>(
+            philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, n_samples, counts);
         INPC_LAUNCH_CHECK("leaf_histogram_kernel");
     }
     s->counter += 1;
