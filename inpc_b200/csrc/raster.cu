@@ -254,98 +254,104 @@ constexpr unsigned kCountShift = 30;   // bilinear: (tiles touched - 1) in key b
 // and collect the largest pattern and the largest complement), or fixed_lo .. fixed_hi.
 template <int MODE, int VARIANT>
 __global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
-    PointSets ps, RasterParams rp, unsigned* __restrict__ block_visible,
+    const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_groups, unsigned* __restrict__ block_visible,
     unsigned* group_visible, unsigned long long* group_instances, unsigned* range, unsigned* done, unsigned fixed_lo, unsigned fixed_hi,
     unsigned* __restrict__ depth_min, unsigned* __restrict__ depth_max, unsigned long long* __restrict__ counters) {
-    // this block's set; indices below are local to it
-    const int set = set_of_block(ps, (int64_t)blockIdx.x * kPreThreads * 4);
-    const float* __restrict__ positions = ps.positions[set];
-    const int64_t n = ps.size[set];
-    const int64_t n_virtual = ps.start[ps.count];
     // Every thread takes 4 consecutive points (three 16-byte loads when the array is aligned), so a
-    // block covers 4 chunks of kPreThreads points; counts are kept per chunk because the projection
-    // pass works on chunks of kPreThreads points.
+    // group of a block covers 4 chunks of kPreThreads points; counts are kept per chunk because the projection
+    // pass works on chunks of kPreThreads points.  A block takes several groups one after the other (one block per group, each
+    // with its fence and atomic for the last-block test: 61 us for 2^23 points, 36 us without the test).
     constexpr int kPerThread = 4;
     constexpr int kWarpsPerChunk = kPreThreads / kPerThread / 32;   // 2
-    __shared__ unsigned s_v[kPreThreads / 32];
-    __shared__ unsigned long long s_i[kPreThreads / 32];
-    __shared__ unsigned s_lo[kPreThreads / 32], s_hi[kPreThreads / 32];
+    __shared__ unsigned s_v[2][kPreThreads / 32];
+    __shared__ unsigned long long s_i[2][kPreThreads / 32];
+    const int64_t n_virtual = ps.start[ps.count];
+    const int warp = threadIdx.x >> 5;
     const W2C m = load_w2c(rp.v.w2c);
-    const int64_t first = ((int64_t)blockIdx.x * kPreThreads + threadIdx.x) * kPerThread - ps.start[set];   // local to the set
-    float p[3 * kPerThread];
-    if (first + kPerThread <= n && (reinterpret_cast<uintptr_t>(positions) & 15u) == 0) {
-        const float4* src = reinterpret_cast<const float4*>(positions + 3 * first);
+    unsigned lo = 0xFFFFFFFFu, hi = 0u;
+    int flip = 0;
+    for (unsigned group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1) {
+        // this group's set; indices below are local to it
+        const int set = set_of_block(ps, (int64_t)group * kPreThreads * 4);
+        const float* __restrict__ positions = ps.positions[set];
+        const int64_t n = ps.size[set];
+        const int64_t first = ((int64_t)group * kPreThreads + threadIdx.x) * kPerThread - ps.start[set];
+        float p[3 * kPerThread];
+        if (first + kPerThread <= n && (reinterpret_cast<uintptr_t>(positions) & 15u) == 0) {
+            const float4* src = reinterpret_cast<const float4*>(positions + 3 * first);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float4 v = __ldg(src + k);
-            p[4 * k] = v.x; p[4 * k + 1] = v.y; p[4 * k + 2] = v.z; p[4 * k + 3] = v.w;
+            for (int k = 0; k < 3; ++k) {
+                const float4 v = __ldg(src + k);
+                p[4 * k] = v.x; p[4 * k + 1] = v.y; p[4 * k + 2] = v.z; p[4 * k + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3 * kPerThread; ++k) p[k] = first * 3 + k < 3 * n ? __ldg(positions + 3 * first + k) : 0.0f;
         }
-    } else {
+        unsigned v = 0;
+        unsigned long long c = 0;
 #pragma unroll
-        for (int k = 0; k < 3 * kPerThread; ++k) p[k] = first * 3 + k < 3 * n ? __ldg(positions + 3 * first + k) : 0.0f;
-    }
-    unsigned v = 0, lo = 0xFFFFFFFFu, hi = 0u;
-    unsigned long long c = 0;
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        if (first + k < n) {
-            const Projection pr = project_point<MODE, VARIANT>(p[3 * k], p[3 * k + 1], p[3 * k + 2], m, rp, first + k, set);
-            if (pr.visible) {
-                v += 1u;
-                c += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
-                const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
-                lo = min(lo, bits);
-                hi = max(hi, bits);
+        for (int k = 0; k < kPerThread; ++k) {
+            if (first + k < n) {
+                const Projection pr = project_point<MODE, VARIANT>(p[3 * k], p[3 * k + 1], p[3 * k + 2], m, rp, first + k, set);
+                if (pr.visible) {
+                    v += 1u;
+                    c += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
+                    const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
+                    lo = min(lo, bits);
+                    hi = max(hi, bits);
+                }
             }
         }
-    }
+        v = __reduce_add_sync(0xffffffffu, v);
+        if (MODE == INPC_MODE_BILINEAR) {
+            c = __reduce_add_sync(0xffffffffu, (unsigned)c);   // at most 4 per point
+        } else {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        v += __shfl_down_sync(0xffffffffu, v, o);
-        c += __shfl_down_sync(0xffffffffu, c, o);
-        lo = min(lo, __shfl_down_sync(0xffffffffu, lo, o));
-        hi = max(hi, __shfl_down_sync(0xffffffffu, hi, o));
-    }
-    const int warp = threadIdx.x >> 5;
-    if (lane_id() == 0) { s_v[warp] = v; s_i[warp] = c; s_lo[warp] = lo; s_hi[warp] = hi; }
-    __syncthreads();
-    if (threadIdx.x < kPerThread) {
-        // chunk `threadIdx.x` of this block
-        const int64_t chunk = (int64_t)blockIdx.x * kPerThread + threadIdx.x;
-        if (chunk * kPreThreads < n_virtual) {   // chunks of the padding behind a set count zero survivors
+            for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+        }
+        if (lane_id() == 0) { s_v[flip][warp] = v; s_i[flip][warp] = c; }
+        __syncthreads();
+        if (threadIdx.x < kPerThread) {
+            // chunk `threadIdx.x` of this group
+            const int64_t chunk = (int64_t)group * kPerThread + threadIdx.x;
+            if (chunk * kPreThreads < n_virtual) {   // chunks of the padding behind a set count zero survivors
+                unsigned tv = 0;
+#pragma unroll
+                for (int w = 0; w < kWarpsPerChunk; ++w) tv += s_v[flip][threadIdx.x * kWarpsPerChunk + w];
+                block_visible[chunk] = tv;
+            }
+        }
+        if (threadIdx.x == 0) {
             unsigned tv = 0;
             unsigned long long ti = 0;
 #pragma unroll
-            for (int w = 0; w < kWarpsPerChunk; ++w) { tv += s_v[threadIdx.x * kWarpsPerChunk + w]; ti += s_i[threadIdx.x * kWarpsPerChunk + w]; }
-            block_visible[chunk] = tv;
-            (void)ti;
+            for (int w = 0; w < kPreThreads / 32; ++w) { tv += s_v[flip][w]; ti += s_i[flip][w]; }
+            // totals of this group of 4 chunks: the scan runs over groups, four times fewer entries
+            group_visible[group] = tv;
+            group_instances[group] = ti;
         }
     }
-    if (threadIdx.x == 0) {
-        unsigned tlo = 0xFFFFFFFFu, thi = 0u, tv = 0;
-        unsigned long long ti = 0;
-#pragma unroll
-        for (int w = 0; w < kPreThreads / 32; ++w) { tlo = min(tlo, s_lo[w]); thi = max(thi, s_hi[w]); tv += s_v[w]; ti += s_i[w]; }
-        // totals of this group of 4 chunks: the one-block scan runs over groups, four times fewer entries
-        group_visible[blockIdx.x] = tv;
-        group_instances[blockIdx.x] = ti;
-        // (callers that know a bound on the depths beforehand pass no pointer; measured: no difference in time)
-        if (range && tlo <= thi) { atomicMax(range, ~tlo); atomicMax(range + 1, thi); }
+    // (callers that know a bound on the depths beforehand pass no pointer)
+    if (range) {
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if (lane_id() == 0 && lo <= hi) { atomicMax(range, ~lo); atomicMax(range + 1, hi); }
     }
     if (!last_block(done, gridDim.x)) return;
     __shared__ unsigned s_scan[kPreThreads / 32 + 1];
-    const unsigned visible = scan_words<kPreThreads>(group_visible, gridDim.x, s_scan);
+    const unsigned visible = scan_words<kPreThreads>(group_visible, n_groups, s_scan);
     unsigned long long inst = 0;
 #pragma unroll 8
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += kPreThreads) inst += __ldcg(group_instances + k);
+    for (unsigned k = threadIdx.x; k < n_groups; k += kPreThreads) inst += __ldcg(group_instances + k);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
-    if (lane_id() == 0) s_i[threadIdx.x >> 5] = inst;
+    if (lane_id() == 0) s_i[0][threadIdx.x >> 5] = inst;
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long t = 0;
 #pragma unroll
-        for (int w = 0; w < kPreThreads / 32; ++w) t += s_i[w];
+        for (int w = 0; w < kPreThreads / 32; ++w) t += s_i[0][w];
         const unsigned lo = range ? ~__ldcg(range) : fixed_lo, hi = range ? __ldcg(range + 1) : fixed_hi;
         counters[0] = visible;
         counters[1] = t;
@@ -568,13 +574,9 @@ constexpr unsigned kTileKeyBits = 24;
 constexpr uint32_t kTileKeyMask = (1u << kTileKeyBits) - 1u;
 
 // One (tile key, point id) pair per touched tile, row-major over the point's bounds, points in depth
-// order (src/bilinear/kernels.cu:198-220).  CODED (bilinear, 8x8 tiles): bounds and footprint origin come
-// from the packed word the projection pass left per point (see pack_quad), a 4-byte gather.
-// (Four consecutive points per thread, with the four gathers in flight together, measured the same 0.12 ms for 2^23
-// points: the kernel is bound by the throughput of the random 4-byte gathers, one 32-byte sector each, not by latency.)
-template <bool CODED>
+// order (src/bilinear/kernels.cu:198-220).
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
-                                                                      const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad,
+                                                                      const uint2* __restrict__ bounds,
                                                                       int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
                                                                       const unsigned* __restrict__ block_base, int gw,
                                                                       uint32_t* __restrict__ inst_keys,
@@ -585,38 +587,81 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
     const int64_t s = (int64_t)blockIdx.x * kInstThreads + threadIdx.x;
     uint32_t id = 0;
     unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0;
-    int qx = 0, qy = 0;
     if (s < n_visible) {
         id = checked_point(__ldg(sorted_ids + s));
-        if (CODED) {
-            // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0
-            const uint32_t q = __ldg(quad + id);
-            qx = (int)(q & 0x7FFFu) - 1;
-            x0 = qx < 0 ? 0u : (unsigned)qx >> 3;
-            y0 = (q >> 16) & 0x7FFu;
-            qy = (int)y0 * 8 + (int)((q >> 27) & 0xFu) - 1;   // row of the upper pixel in the stacked grid (or one above its image)
-            x1 = x0 + 1u + ((q >> 15) & 1u);
-            y1 = y0 + 1u + (q >> 31);
-        } else {
-            const uint2 b = __ldg(bounds + id);
-            x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
-        }
+        const uint2 b = __ldg(bounds + id);
+        x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
     }
     const unsigned c = (x1 - x0) * (y1 - y0);
     unsigned total;
     unsigned off = block_base[blockIdx.x] + block_exclusive_scan(c, s_scan, &total);
     for (unsigned ty = y0; ty < y1; ++ty)
         for (unsigned tx = x0; tx < x1; ++tx) {
-            uint32_t key = ty * (unsigned)gw + tx;
-            if (CODED) {
-                const unsigned cx = (unsigned)min(max(qx - (int)tx * 8 + 1, 0), 8);
-                const unsigned cy = (unsigned)min(max(qy - (int)ty * 8 + 1, 0), 8);
-                key |= (cx << kTileKeyBits) | (cy << (kTileKeyBits + 4));
-            }
-            inst_keys[off] = key;
+            inst_keys[off] = ty * (unsigned)gw + tx;
             inst_ids[off] = id;
             ++off;
         }
+}
+
+// The same for bilinear splats on 8x8 tiles, with the footprint codes.  Everything comes from the packed word the projection
+// pass left per point (see pack_quad), a 4-byte gather.  A splat touches one tile, or the next column's or row's too, and then
+// its footprint starts in the last column (row) of the first and in column (row) -1 of the second.  A thread takes four
+// consecutive points with their gathers in flight together; the instances of a block are staged in shared memory and leave in
+// whole sectors.  (One point per thread of a 1024-thread block, a loop over its tiles and direct stores: 104 us for 2^23 points.)
+constexpr int kEmitThreads = kInstThreads / 4;
+__global__ void __launch_bounds__(kEmitThreads, 6) emit_coded_instances_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ quad,
+                                                                            int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
+                                                                            const unsigned* __restrict__ block_base, unsigned gw,
+                                                                            uint32_t* __restrict__ inst_keys, uint32_t* __restrict__ inst_ids) {
+    __shared__ unsigned s_scan[kEmitThreads / 32 + 1];
+    __shared__ uint2 s_inst[kInstThreads * 4];   // as many as there can be
+    const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
+    if ((int64_t)blockIdx.x * kInstThreads >= n_visible) return;
+    const int64_t first = (int64_t)blockIdx.x * kInstThreads + 4 * threadIdx.x;
+    uint32_t id[4], q[4];
+    if (first + 4 <= n_visible) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(sorted_ids + first));   // the id buffers are 16-byte aligned
+        id[0] = v.x; id[1] = v.y; id[2] = v.z; id[3] = v.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) id[k] = first + k < n_visible ? __ldg(sorted_ids + first + k) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        id[k] = checked_point(id[k]);
+        q[k] = __ldg(quad + id[k]);
+    }
+    unsigned count = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (first + k < n_visible) count += (1u + ((q[k] >> 15) & 1u)) << (q[k] >> 31);
+    unsigned total;
+    unsigned off = block_exclusive_scan(count, s_scan, &total);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (first + k < n_visible) {
+            const unsigned qx1 = q[k] & 0x7FFFu;                              // column of the footprint's left pixel + 1
+            const unsigned tx = qx1 == 0u ? 0u : (qx1 - 1u) >> 3;
+            const unsigned cx = qx1 - 8u * tx;                                // relative to the tile, + 1
+            const unsigned cy = (q[k] >> 27) & 0xFu;
+            const uint32_t tile = ((q[k] >> 16) & 0x7FFu) * gw + tx;
+            const bool two_x = (q[k] >> 15) & 1u, two_y = q[k] >> 31;
+            const uint32_t col = cx << kTileKeyBits, row = cy << (kTileKeyBits + 4);
+            s_inst[off++] = make_uint2(tile | col | row, id[k]);
+            if (two_x) s_inst[off++] = make_uint2((tile + 1u) | row, id[k]);
+            if (two_y) {
+                s_inst[off++] = make_uint2((tile + gw) | col, id[k]);
+                if (two_x) s_inst[off++] = make_uint2(tile + gw + 1u, id[k]);
+            }
+        }
+    }
+    __syncthreads();
+    const unsigned base = __ldg(block_base + blockIdx.x);
+    for (unsigned k = threadIdx.x; k < total; k += kEmitThreads) {
+        const uint2 v = s_inst[k];
+        inst_keys[base + k] = v.x;
+        inst_ids[base + k] = v.y;
+    }
 }
 
 // Run boundaries of the sorted tile keys -> [first, last+1) per tile (src/bilinear/kernels.cu:222-239).
@@ -3076,7 +3121,7 @@ struct GradientSlots {
     const unsigned* mask;    // [n] bit s: slot s was written
 };
 template <bool SLOTS>
-__global__ void __launch_bounds__(kPreThreads) preprocess_backward_kernel(
+__global__ void __launch_bounds__(kPreThreads, 8) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ cam, const uint2* __restrict__ bounds,
     const float4* __restrict__ grad_feat_view, GradientSlots slots, float* __restrict__ grad_opacities,
     __half* __restrict__ grad_features, int64_t n, bool bulk_ok) {
@@ -3453,9 +3498,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             clear.add(pb.state, (size_t)(static_cast<char*>(pb.sort_ws) - reinterpret_cast<char*>(pb.state)) + (deferred ? sort_zero_bytes(n, n, key_bits) : 0));
             rc = launch_clear(clear, stream);
             if (rc != INPC_OK) return rc;
-            const int64_t groups = ceil_div<int64_t>(nb, 4);
-            visibility_count_kernel<MODE, VARIANT><<<(unsigned)groups, kPreThreads, 0, stream>>>(
-                ps, rp, pb.block_visible, pb.group_visible, pb.group_instances, deferred ? nullptr : pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min,
+            const int64_t groups = ceil_div<int64_t>(nb, 4), group_cap = (int64_t)sm_count() * 4;
+            visibility_count_kernel<MODE, VARIANT><<<(unsigned)(groups < group_cap ? groups : group_cap), kPreThreads, 0, stream>>>(
+                ps, rp, (unsigned)groups, pb.block_visible, pb.group_visible, pb.group_instances, deferred ? nullptr : pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min,
                 pb.depth_max, pb.counters);
             INPC_LAUNCH_CHECK("visibility_count_kernel");
             if (!deferred) {
@@ -3522,9 +3567,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                 instance_count_kernel<false><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (warp_blend)
-                emit_instances_kernel<true><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                emit_coded_instances_kernel<<<(unsigned)ibk, kEmitThreads, 0, stream>>>(sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)rp.gw, ib.keys[0], ib.ids[0]);
             else
-                emit_instances_kernel<false><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                emit_instances_kernel<<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             INPC_LAUNCH_CHECK("emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
