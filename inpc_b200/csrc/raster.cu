@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
     // Every thread takes 4 consecutive points (three 16-byte loads when the array is aligned), so a
     // group of a block covers 4 chunks of kPreThreads points; counts are kept per chunk because the projection
     // pass works on chunks of kPreThreads points.  A block takes several groups one after the other (one block per group, each
-    // with its fence and atomic for the last-block test: 61 us for 2^23 points, 36 us without the test).
+    // with its fence and atomic for the last-block test: 62 / 226 us for 2^23 / 2^25 points, 44 / 154 like this).
     constexpr int kPerThread = 4;
     constexpr int kWarpsPerChunk = kPreThreads / kPerThread / 32;   // 2
     __shared__ unsigned s_v[2][kPreThreads / 32];
@@ -574,9 +574,15 @@ constexpr unsigned kTileKeyBits = 24;
 constexpr uint32_t kTileKeyMask = (1u << kTileKeyBits) - 1u;
 
 // One (tile key, point id) pair per touched tile, row-major over the point's bounds, points in depth
-// order (src/bilinear/kernels.cu:198-220).
+// order (src/bilinear/kernels.cu:198-220).  CODED (bilinear, 8x8 tiles): bounds and footprint origin come
+// from the packed word the projection pass left per point (see pack_quad), a 4-byte gather.
+// Bound by the throughput of the random 4-byte gathers, one 32-byte sector each, not by their latency.  What is read or written
+// once bypasses the caches' replacement, so that more of the gathered array stays in L2: 2^23 / 2^24 / 2^25 points
+// 104 / 221 / 488 -> 97 / 205 / 469 us.  (Four consecutive points per thread with their gathers in flight together and the
+// instances staged in shared memory: 116 / 396 / 952 us, the gathers of fewer, busier warps miss L2 more often.)
+template <bool CODED>
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
-                                                                      const uint2* __restrict__ bounds,
+                                                                      const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad,
                                                                       int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
                                                                       const unsigned* __restrict__ block_base, int gw,
                                                                       uint32_t* __restrict__ inst_keys,
@@ -587,81 +593,38 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
     const int64_t s = (int64_t)blockIdx.x * kInstThreads + threadIdx.x;
     uint32_t id = 0;
     unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0;
+    int qx = 0, qy = 0;
     if (s < n_visible) {
-        id = checked_point(__ldg(sorted_ids + s));
-        const uint2 b = __ldg(bounds + id);
-        x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
+        id = checked_point(__ldcs(sorted_ids + s));
+        if (CODED) {
+            // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0
+            const uint32_t q = __ldg(quad + id);
+            qx = (int)(q & 0x7FFFu) - 1;
+            x0 = qx < 0 ? 0u : (unsigned)qx >> 3;
+            y0 = (q >> 16) & 0x7FFu;
+            qy = (int)y0 * 8 + (int)((q >> 27) & 0xFu) - 1;   // row of the upper pixel in the stacked grid (or one above its image)
+            x1 = x0 + 1u + ((q >> 15) & 1u);
+            y1 = y0 + 1u + (q >> 31);
+        } else {
+            const uint2 b = __ldg(bounds + id);
+            x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
+        }
     }
     const unsigned c = (x1 - x0) * (y1 - y0);
     unsigned total;
     unsigned off = block_base[blockIdx.x] + block_exclusive_scan(c, s_scan, &total);
     for (unsigned ty = y0; ty < y1; ++ty)
         for (unsigned tx = x0; tx < x1; ++tx) {
-            inst_keys[off] = ty * (unsigned)gw + tx;
-            inst_ids[off] = id;
+            uint32_t key = ty * (unsigned)gw + tx;
+            if (CODED) {
+                const unsigned cx = (unsigned)min(max(qx - (int)tx * 8 + 1, 0), 8);
+                const unsigned cy = (unsigned)min(max(qy - (int)ty * 8 + 1, 0), 8);
+                key |= (cx << kTileKeyBits) | (cy << (kTileKeyBits + 4));
+            }
+            __stcs(inst_keys + off, key);
+            __stcs(inst_ids + off, id);
             ++off;
         }
-}
-
-// The same for bilinear splats on 8x8 tiles, with the footprint codes.  Everything comes from the packed word the projection
-// pass left per point (see pack_quad), a 4-byte gather.  A splat touches one tile, or the next column's or row's too, and then
-// its footprint starts in the last column (row) of the first and in column (row) -1 of the second.  A thread takes four
-// consecutive points with their gathers in flight together; the instances of a block are staged in shared memory and leave in
-// whole sectors.  (One point per thread of a 1024-thread block, a loop over its tiles and direct stores: 104 us for 2^23 points.)
-constexpr int kEmitThreads = kInstThreads / 4;
-__global__ void __launch_bounds__(kEmitThreads, 6) emit_coded_instances_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ quad,
-                                                                            int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
-                                                                            const unsigned* __restrict__ block_base, unsigned gw,
-                                                                            uint32_t* __restrict__ inst_keys, uint32_t* __restrict__ inst_ids) {
-    __shared__ unsigned s_scan[kEmitThreads / 32 + 1];
-    __shared__ uint2 s_inst[kInstThreads * 4];   // as many as there can be
-    const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
-    if ((int64_t)blockIdx.x * kInstThreads >= n_visible) return;
-    const int64_t first = (int64_t)blockIdx.x * kInstThreads + 4 * threadIdx.x;
-    uint32_t id[4], q[4];
-    if (first + 4 <= n_visible) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(sorted_ids + first));   // the id buffers are 16-byte aligned
-        id[0] = v.x; id[1] = v.y; id[2] = v.z; id[3] = v.w;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) id[k] = first + k < n_visible ? __ldg(sorted_ids + first + k) : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        id[k] = checked_point(id[k]);
-        q[k] = __ldg(quad + id[k]);
-    }
-    unsigned count = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (first + k < n_visible) count += (1u + ((q[k] >> 15) & 1u)) << (q[k] >> 31);
-    unsigned total;
-    unsigned off = block_exclusive_scan(count, s_scan, &total);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (first + k < n_visible) {
-            const unsigned qx1 = q[k] & 0x7FFFu;                              // column of the footprint's left pixel + 1
-            const unsigned tx = qx1 == 0u ? 0u : (qx1 - 1u) >> 3;
-            const unsigned cx = qx1 - 8u * tx;                                // relative to the tile, + 1
-            const unsigned cy = (q[k] >> 27) & 0xFu;
-            const uint32_t tile = ((q[k] >> 16) & 0x7FFu) * gw + tx;
-            const bool two_x = (q[k] >> 15) & 1u, two_y = q[k] >> 31;
-            const uint32_t col = cx << kTileKeyBits, row = cy << (kTileKeyBits + 4);
-            s_inst[off++] = make_uint2(tile | col | row, id[k]);
-            if (two_x) s_inst[off++] = make_uint2((tile + 1u) | row, id[k]);
-            if (two_y) {
-                s_inst[off++] = make_uint2((tile + gw) | col, id[k]);
-                if (two_x) s_inst[off++] = make_uint2(tile + gw + 1u, id[k]);
-            }
-        }
-    }
-    __syncthreads();
-    const unsigned base = __ldg(block_base + blockIdx.x);
-    for (unsigned k = threadIdx.x; k < total; k += kEmitThreads) {
-        const uint2 v = s_inst[k];
-        inst_keys[base + k] = v.x;
-        inst_ids[base + k] = v.y;
-    }
 }
 
 // Run boundaries of the sorted tile keys -> [first, last+1) per tile (src/bilinear/kernels.cu:222-239).
@@ -3120,6 +3083,9 @@ struct GradientSlots {
     const float4* grad;      // [4 n][2]: {feature gradient}, {opacity gradient, -, -, -}
     const unsigned* mask;    // [n] bit s: slot s was written
 };
+// Bound by the 76 bytes a point's gradients take (97 us of 162 for 2^23 samples) and by waiting for the slots of the touched
+// ones: eight blocks per multiprocessor (32 registers) keep more of them in flight (without the bound 180 us; 2^24
+// points 318 -> 285).
 template <bool SLOTS>
 __global__ void __launch_bounds__(kPreThreads, 8) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ cam, const uint2* __restrict__ bounds,
@@ -3567,9 +3533,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                 instance_count_kernel<false><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (warp_blend)
-                emit_coded_instances_kernel<<<(unsigned)ibk, kEmitThreads, 0, stream>>>(sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)rp.gw, ib.keys[0], ib.ids[0]);
+                emit_instances_kernel<true><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             else
-                emit_instances_kernel<<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                emit_instances_kernel<false><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             INPC_LAUNCH_CHECK("emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
