@@ -60,6 +60,7 @@ struct RasterParams {
     int n_sets;     // images drawn by the call (1 except for batched multi-set inference): the grid has n_sets * gh rows
     float sigma_world, sigma_cutoff;
     const float* scales;   // optional per-point sigma (gaussian, pre-extracted)
+    float reach;           // gaussian: -2 log(threshold), the squared Mahalanobis distance at which a splat is cut off
 };
 
 // Input points of a call: one array triple, or (batched multi-set inference) up to kMaxSets of them laid end to end in
@@ -403,6 +404,23 @@ __device__ __forceinline__ uint32_t pack_quad(const Projection& pr, int tile_row
     return (qx1 & 0x7FFFu) | ((pr.x1 - pr.x0 - 1u) << 15) | ((pr.y0 & 0x7FFu) << 16) | ((ry1 & 0xFu) << 27) | ((pr.y1 - pr.y0 - 1u) << 31);
 }
 
+// What the instance emission needs of a gaussian splat on 8x8 tiles: its tile bounds, and how far its ellipse stays away from
+// their sides in cells of 2x2 pixels, four bits each (left, right, top, bottom; rounded down, so the cells between are a superset).
+__device__ __forceinline__ uint4 pack_footprint(const Projection& pr, float reach) {
+    const float det = pr.cx * pr.cz - pr.cy * pr.cy;
+    unsigned inset = 0u;
+    if (det > 0.0f) {
+        const float s = reach / det;
+        const float rx = sqrtf(fmaxf(s * pr.cz, 0.0f)) * 1.001f + 0.01f;
+        const float ry = sqrtf(fmaxf(s * pr.cx, 0.0f)) * 1.001f + 0.01f;
+        const int left = (__float2int_ru(pr.sx - rx - 0.5f) >> 1) - 4 * (int)pr.x0, right = 4 * (int)pr.x1 - 1 - (__float2int_rd(pr.sx + rx - 0.5f) >> 1);
+        const int top = (__float2int_ru(pr.sy - ry - 0.5f) >> 1) - 4 * (int)pr.y0, bottom = 4 * (int)pr.y1 - 1 - (__float2int_rd(pr.sy + ry - 0.5f) >> 1);
+        inset = (unsigned)min(max(left, 0), 15) | ((unsigned)min(max(right, 0), 15) << 4) | ((unsigned)min(max(top, 0), 15) << 8) |
+                ((unsigned)min(max(bottom, 0), 15) << 12);
+    }
+    return make_uint4(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16), inset, 0u);
+}
+
 // Pass 2: project again (same arithmetic, same outcome), evaluate SH, write the point record and
 // bounds, and append (depth key, point id) at the slot given by the block offset plus the rank of
 // the point among the block's survivors — index order, hence reproducible.
@@ -412,7 +430,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     PointSets ps, RasterParams rp, const unsigned* __restrict__ block_visible, const unsigned* __restrict__ group_offset,
     const unsigned* __restrict__ depth_min,
     const unsigned* __restrict__ depth_max, PointRec* __restrict__ rec, uint2* __restrict__ bounds, uint32_t* __restrict__ quad,
-    float4* __restrict__ conic, uint32_t* __restrict__ depth_keys,
+    float4* __restrict__ conic, uint4* __restrict__ foot, uint32_t* __restrict__ depth_keys,
     uint32_t* __restrict__ point_ids, int pack_count, int rec_stride, volatile unsigned* status) {
     constexpr int kHalves = VARIANT == VAR_RAW37 ? 37 : 36;
     constexpr int kSlabBytes = VARIANT == VAR_ROWS ? 16 : kPreThreads * kHalves * 2;   // multiple of 16 for both layouts
@@ -494,7 +512,10 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
             dst[1] = make_float4(r.f[0], r.f[1], r.f[2], r.f[3]);
             bounds[iv] = make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16));
             if (quad) quad[iv] = pack_quad(pr, set * rp.gh);
-            if (MODE == INPC_MODE_GAUSSIAN) conic[iv] = make_float4(pr.cx, pr.cy, pr.cz, 0.0f);
+            if (MODE == INPC_MODE_GAUSSIAN) {
+                conic[iv] = make_float4(pr.cx, pr.cy, pr.cz, 0.0f);
+                if (foot) foot[iv] = pack_footprint(pr, rp.reach);
+            }
         } else {
             bounds[iv] = make_uint2(0u, 0u);
         }
@@ -573,17 +594,36 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
 constexpr unsigned kTileKeyBits = 24;
 constexpr uint32_t kTileKeyMask = (1u << kTileKeyBits) - 1u;
 
+// For gaussian splats on 8x8 tiles the 8 bits above the tile index name the 2x2-pixel cells of the tile that the ellipse can
+// reach: columns [left, right] and rows [top, bottom] of the 4x4 cells, clipped to the tile, ten times ten ranges.
+constexpr unsigned kNoCells = 255u;
+__device__ __forceinline__ unsigned cell_range_index(unsigned lo, unsigned hi) { return lo * 4u - lo * (lo - 1u) / 2u + (hi - lo); }
+__device__ __forceinline__ void cell_range(unsigned index, unsigned* lo, unsigned* hi) {
+    unsigned l = 0;
+    while (l < 3u && index >= 4u - l) { index -= 4u - l; ++l; }
+    *lo = l;
+    *hi = l + index;
+}
+__device__ __forceinline__ unsigned cell_code(int left, int right, int top, int bottom) {
+    left = max(left, 0); top = max(top, 0);
+    right = min(right, 3); bottom = min(bottom, 3);
+    if (left > right || top > bottom) return kNoCells;
+    return cell_range_index((unsigned)left, (unsigned)right) + 10u * cell_range_index((unsigned)top, (unsigned)bottom);
+}
+
 // One (tile key, point id) pair per touched tile, row-major over the point's bounds, points in depth
-// order (src/bilinear/kernels.cu:198-220).  CODED (bilinear, 8x8 tiles): bounds and footprint origin come
-// from the packed word the projection pass left per point (see pack_quad), a 4-byte gather.
+// order (src/bilinear/kernels.cu:198-220).  EMIT_QUAD (bilinear, 8x8 tiles): bounds and footprint origin come
+// from the packed word the projection pass left per point (see pack_quad), a 4-byte gather.  EMIT_CELLS (gaussian, 8x8 tiles):
+// the key also says which cells of the tile the ellipse can reach (see cell_code).
 // Bound by the throughput of the random 4-byte gathers, one 32-byte sector each, not by their latency.  What is read or written
 // once bypasses the caches' replacement, so that more of the gathered array stays in L2: 2^23 / 2^24 / 2^25 points
 // 104 / 221 / 488 -> 97 / 205 / 469 us.  (Four consecutive points per thread with their gathers in flight together and the
 // instances staged in shared memory: 116 / 396 / 952 us, the gathers of fewer, busier warps miss L2 more often.)
-template <bool CODED>
+enum { EMIT_BOUNDS = 0, EMIT_QUAD = 1, EMIT_CELLS = 2 };
+template <int KEYS>
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
                                                                       const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad,
-                                                                      int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
+                                                                      const uint4* __restrict__ foot, int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
                                                                       const unsigned* __restrict__ block_base, int gw,
                                                                       uint32_t* __restrict__ inst_keys,
                                                                       uint32_t* __restrict__ inst_ids) {
@@ -592,11 +632,11 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
     if ((int64_t)blockIdx.x * kInstThreads >= n_visible) return;
     const int64_t s = (int64_t)blockIdx.x * kInstThreads + threadIdx.x;
     uint32_t id = 0;
-    unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0;
+    unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0, inset = 0;
     int qx = 0, qy = 0;
     if (s < n_visible) {
         id = checked_point(__ldcs(sorted_ids + s));
-        if (CODED) {
+        if (KEYS == EMIT_QUAD) {
             // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0
             const uint32_t q = __ldg(quad + id);
             qx = (int)(q & 0x7FFFu) - 1;
@@ -606,7 +646,14 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
             x1 = x0 + 1u + ((q >> 15) & 1u);
             y1 = y0 + 1u + (q >> 31);
         } else {
-            const uint2 b = __ldg(bounds + id);
+            uint2 b;
+            if (KEYS == EMIT_CELLS) {
+                const uint4 f = __ldg(foot + id);
+                b = make_uint2(f.x, f.y);
+                inset = f.z;
+            } else {
+                b = __ldg(bounds + id);
+            }
             x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
         }
     }
@@ -616,10 +663,15 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
     for (unsigned ty = y0; ty < y1; ++ty)
         for (unsigned tx = x0; tx < x1; ++tx) {
             uint32_t key = ty * (unsigned)gw + tx;
-            if (CODED) {
+            if (KEYS == EMIT_QUAD) {
                 const unsigned cx = (unsigned)min(max(qx - (int)tx * 8 + 1, 0), 8);
                 const unsigned cy = (unsigned)min(max(qy - (int)ty * 8 + 1, 0), 8);
                 key |= (cx << kTileKeyBits) | (cy << (kTileKeyBits + 4));
+            }
+            if (KEYS == EMIT_CELLS) {
+                const int left = (int)(inset & 15u) - 4 * (int)(tx - x0), right = 4 * (int)(x1 - tx) - 1 - (int)((inset >> 4) & 15u);
+                const int top = (int)((inset >> 8) & 15u) - 4 * (int)(ty - y0), bottom = 4 * (int)(y1 - ty) - 1 - (int)(inset >> 12);
+                key |= cell_code(left, right, top, bottom) << kTileKeyBits;
             }
             __stcs(inst_keys + off, key);
             __stcs(inst_ids + off, id);
@@ -1320,12 +1372,23 @@ constexpr int kManyTiles = 1 << 15;   // from here on the first segments alone k
 struct SegmentLengths {
     unsigned first, later;   // instances in a tile's first segment, and in every later one
 };
-__device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_instances, int n_tiles) {
-    const unsigned target = n_tiles > kManyTiles ? kSegmentTarget / 2u : kSegmentTarget;
+// The largest lengths, and how many later segments are aimed at.  A batch of gaussian splats takes a training pass two to three
+// times as long (more fragments, their sums), so its long items weigh more than the states of more segments; inference has little of
+// that work.  Blend passes of a training step at 1237x822, forward and backward, first + later segment 1024 + 4096 / 512 + 2048 /
+// 512 + 1024 / 256 + 512: 2^22 samples 1086 / 999 / 991 / 1035 us, 2^20 (which twice the number of segments gives 256 + 512)
+// - / 472 / 462 / 350; inference, 2 * 10^6 splats at 1297x840: 200 / 216 / - / 251 (256 + 1024).
+struct SegmentLimits {
+    unsigned first_max, later_max, target;
+};
+constexpr SegmentLimits segment_limits(int mode, bool training) {
+    return mode == INPC_MODE_GAUSSIAN && training ? SegmentLimits{512u, 1024u, 2u * kSegmentTarget} : SegmentLimits{kFirstSegmentMax, kLaterSegmentMax, kSegmentTarget};
+}
+__device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_instances, int n_tiles, const SegmentLimits limits) {
+    const unsigned target = n_tiles > kManyTiles ? limits.target / 2u : limits.target;
     SegmentLengths s;
     s.later = kSegmentMin;
-    while (s.later < kLaterSegmentMax && (unsigned long long)s.later * target < n_instances) s.later *= 2u;
-    s.first = max(kSegmentMin, min(kFirstSegmentMax, s.later / 2u));
+    while (s.later < limits.later_max && (unsigned long long)s.later * target < n_instances) s.later *= 2u;
+    s.first = max(kSegmentMin, min(limits.first_max, s.later / 2u));
     return s;
 }
 constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
@@ -1366,13 +1429,13 @@ __device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ran
     }
 }
 
-__global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, unsigned long long n_instances_arg,
+__global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, unsigned long long n_instances_arg,
                                                                         const unsigned long long* __restrict__ n_instances_dev, uint2* block_sums, unsigned* done,
                                                                         uint32_t* __restrict__ counts) {
     __shared__ unsigned s_seg[kItemThreads / 32], s_tiles[kItemThreads / 32];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
-    const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles);
+    const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles, limits);
     load_tile_segments(ranges, n_tiles, blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread, sl, ns, rg);
     unsigned seg = 0, tiles = 0;
 #pragma unroll
@@ -1423,7 +1486,7 @@ __device__ __forceinline__ WarpItem load_item(const WarpItem* p) {
 }
 
 // Step 2: items0 = segment 0 of the non-empty tiles, items1 = every later segment, tile by tile.
-__global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, unsigned long long n_instances_arg,
+__global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, unsigned long long n_instances_arg,
                                                                       const unsigned long long* __restrict__ n_instances_dev,
                                                                       const uint2* __restrict__ block_base, WarpItem* __restrict__ items0,
                                                                       WarpItem* __restrict__ items1) {
@@ -1431,7 +1494,7 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
     const int t0 = blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread;
-    const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles);
+    const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles, limits);
     load_tile_segments(ranges, n_tiles, t0, sl, ns, rg);
     unsigned seg = 0, tiles = 0;
 #pragma unroll
@@ -2757,7 +2820,7 @@ __global__ void __launch_bounds__(T * T) blend_rows_backward_kernel(
 }
 
 // ------------------------------------------------------------------------------------------------
-// Gaussian blend (src/gaussian/kernels.cu:401-474 forward, :476-579 backward, :581-660 inference).
+// Gaussian blend on 16x16 tiles (src/gaussian/kernels.cu:401-474 forward, :476-579 backward, :581-660 inference).
 // A footprint is an ellipse of a few pixels, not a fixed 2x2: the staging thread sets its instance's bit
 // for the pixels of the ellipse's bounding box inside the tile (slightly widened, so a superset of the
 // pixels that pass the reference's tests), and every pixel thread walks only its set bits and applies
@@ -3073,6 +3136,471 @@ __global__ void __launch_bounds__(T * T) blend_gaussian_backward_kernel(
     flush_gradients();
 }
 
+// ------------------------------------------------------------------------------------------------
+// Gaussian blend on 8x8 tiles, one warp per work item: the passes, lists and segments of the bilinear warp blend above.
+// (Arithmetic per fragment: src/gaussian/kernels.cu:401-474 forward, :476-579 backward, :581-660 inference.)
+//
+// A footprint is an ellipse instead of 2x2 pixels.  The key says which 2x2-pixel cells of the tile it can reach (a column range
+// and a row range, see cell_code), so that dead instances are dropped unread like bilinear ones.  Of a batch of 32 staged
+// instances, lane j first finds the pixels of the half inside the ellipse of instance j, row by row and slightly widened (a
+// superset of what passes the reference's tests); a 32x32 bit transposition over the warp turns these masks into one word per
+// pixel with the instances that reach it, and every lane walks down the set bits of its own pixel.  What a fragment adds to its
+// point is left in shared memory, the words of accepted fragments are transposed back, and lane j adds up the sums of
+// instance j: no shared-memory floating-point atomics (compare-and-swap loops, five per fragment of the backward pass), one
+// global atomic per instance and half.
+//
+// Bound by the chain of instructions of a batch (masks, transposition, the pixels' lists, the sums) and by the passes draining while
+// their longest items finish (6 to 10 of 64 warps of a multiprocessor active on average).  Against one block of 64 threads per
+// (tile, segment) that staged every instance: 2^22 samples at 1237x822, forward and backward 1680 -> 990 us; 2 * 10^6 splats
+// with sizes at 1297x840, inference 511 -> 200 us.
+// ------------------------------------------------------------------------------------------------
+// Pixels of the tile (bit = row * 8 + column) in the cells of a code.
+__device__ __forceinline__ unsigned long long cell_pixels(unsigned code) {
+    if (code >= 100u) return 0ull;
+    unsigned c0, c1, r0, r1;
+    cell_range(code % 10u, &c0, &c1);
+    cell_range(code / 10u, &r0, &r1);
+    const unsigned row = ((1u << (2u * c1 + 2u)) - 1u) & ~((1u << (2u * c0)) - 1u);
+    unsigned long long m = 0ull;
+    for (unsigned y = 2u * r0; y < 2u * r1 + 2u; ++y) m |= (unsigned long long)row << (8u * y);
+    return m;
+}
+
+// Bit l of lane k's word becomes bit k of lane l's word.
+__device__ __forceinline__ unsigned warp_transpose_bits(unsigned x, unsigned lane) {
+    unsigned m = 0x0000FFFFu;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
+        x = (lane & (unsigned)s) ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y & m) << s);
+        m ^= m << (s >> 1);
+    }
+    return x;
+}
+
+// Pixels of the 8x4 half at (px0, py0) (bit = row * 8 + column) that a splat at `a` with conic `c` can reach: a superset of
+// those with  c.x dx^2 + 2 c.y dx dy + c.z dy^2 <= reach  (reach = -2 log threshold).
+__device__ __forceinline__ unsigned ellipse_pixels(const float4& a, const float4& c, float reach, int px0, int py0) {
+    const float det = c.x * c.z - c.y * c.y;
+    if (!(det > 0.0f)) return 0xffffffffu;   // degenerate (or not a number): the per-pixel tests decide
+    const float inv = 1.0f / c.x, peak = reach * c.x;
+    const float ry = sqrtf(peak / det) * 1.001f + 0.01f;
+    const float x0 = a.x - 0.5f - (float)px0, y0 = a.y - 0.5f - (float)py0;
+    unsigned m = 0u;
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+        const float dy = y0 - (float)y;
+        // the rounding of det of a long ellipse (a thousandth at most) is covered by the widening, as is that of the root
+        const float r = sqrtf(fmaxf(peak * 1.002f - det * dy * dy, 0.0f)) * inv * 1.001f + 0.01f;
+        const float mid = x0 + c.y * dy * inv;
+        const int lo = __float2int_ru(fminf(fmaxf(mid - r, 0.0f), 8.0f)), hi = __float2int_rd(fminf(fmaxf(mid + r, -1.0f), 7.0f));
+        if (fabsf(dy) <= ry && lo <= hi) m |= ((2u << hi) - (1u << lo)) << (8 * y);
+    }
+    return m;
+}
+
+template <bool BLEND, bool WEIGHTS>
+struct __align__(16) GaussForwardSmem {
+    float4 ring_a[2][32], ring_c[2][32];              // records and conics of the batches in flight
+    float4 ring_f[BLEND ? 2 : 1][BLEND ? 32 : 1];     // ... and features
+    float out[WEIGHTS ? 32 : 1][33];                  // [staged instance][pixel]: what the fragment adds to the blending weight
+    uint32_t ring_id[2][32];
+    uint32_t queue[kQueueCap];
+};
+template <int PASS, int KIND>
+constexpr size_t gauss_forward_smem_bytes() {
+    return 256 * sizeof(unsigned long long) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN>);
+}
+
+template <int PASS, int KIND>
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_forward_kernel(
+    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, const uint32_t* __restrict__ inst_keys,
+    const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T,
+    float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
+    float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
+    int width, int height, int gw, float threshold, float reach) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr unsigned kNoInstance = 0xffffffffu;
+    constexpr bool kBlend = PASS != PASS_PRODUCT;
+    constexpr bool kWeights = kBlend && KIND == BLEND_TRAIN;
+    constexpr bool kDepth = kBlend && KIND == BLEND_INFER;
+    using Smem = GaussForwardSmem<kBlend, kWeights>;
+    extern __shared__ __align__(16) unsigned char blend_smem[];
+    unsigned long long* s_reach = reinterpret_cast<unsigned long long*>(blend_smem);     // key code -> pixels reached
+    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 256 * sizeof(unsigned long long))[threadIdx.x >> 5];
+    const unsigned lane = lane_id();
+    const unsigned lt_mask = (1u << lane) - 1u;
+    s_reach[threadIdx.x] = cell_pixels(threadIdx.x);
+    __syncthreads();
+    const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
+    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));   // see the bilinear kernel
+    unsigned next_item = 0, visit_end = 0;
+    for (;;) {
+        if (next_item == visit_end) {
+            unsigned first_item = 0;
+            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
+            first_item = __shfl_sync(kFull, first_item, 0);
+            if (first_item >= n_items) break;
+            next_item = first_item;
+            visit_end = min(first_item + per_visit, n_items);
+        }
+        const unsigned item = next_item++;
+        const WarpItem it = load_item(items + (item >> 1));
+        const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg, first = it.first;
+        const int half = (int)(item & 1u);
+        const size_t sidx = (size_t)(first + seg) * 2u + half;      // this item's slot in the per-segment arrays
+        const size_t sidx0 = (size_t)first * 2u + half;             // segment 0 of the same tile half
+        const uint2 rg = make_uint2(it.begin, it.end);
+        const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
+        const int px0 = tx * 8, py0 = ty * 8 + 4 * half;            // first pixel of this half
+        const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+        const bool inside = px < width && py < height;
+        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
+
+        float Tr = 1.0f, Z = 0.0f, stop = kTransmittanceEps;
+        float4 C = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool done = !inside;
+        if (PASS == PASS_PRODUCT) {
+            // product of (1 - alpha) over the segment, until it would carry the state segment 0 left below the threshold; the
+            // margin keeps a pixel open when rounding could be what carries it over the line
+            const float T0 = seg_T[sidx0 * 32 + lane];
+            done = done || T0 < kTransmittanceEps;
+            if (!done) stop = kTransmittanceEps / T0 * (1.0f - 1e-4f);
+        } else if (PASS == PASS_REST) {
+            Tr = seg_T[sidx * 32 + lane];
+            done = done || Tr < kTransmittanceEps;
+        }
+        unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
+
+        uint32_t* kept = half ? kept1 : kept0;
+        unsigned n_out = 0;
+        if (done_w != kFull) {
+            unsigned pos = rg.x;           // next key to load
+            bool loaded = false;
+            uint32_t kq[kFilterKeys], iq[kFilterKeys];
+            auto load_step = [&]() {
+#pragma unroll
+                for (int k = 0; k < kFilterKeys; ++k) {
+                    const unsigned idx = pos + 32u * k + lane;
+                    const bool ok = idx < rg.y;
+                    kq[k] = ok ? __ldg(inst_keys + idx) : 0xFFFFFFFFu;   // code 0xFF reaches nothing
+                    iq[k] = ok ? __ldg(inst_ids + idx) : 0u;
+                }
+                pos = min(pos + 32u * kFilterKeys, rg.y);
+                loaded = true;
+            };
+            unsigned q_head = 0, q_tail = 0;   // candidates [q_head, q_tail) wait for their gather
+            auto fill = [&]() {
+                while (PASS != PASS_REST && q_tail - q_head < 32u && loaded) {
+                    uint32_t ck[kFilterKeys], ci[kFilterKeys];
+#pragma unroll
+                    for (int k = 0; k < kFilterKeys; ++k) { ck[k] = kq[k]; ci[k] = iq[k]; }
+                    loaded = false;
+                    if (pos < rg.y) load_step();
+#pragma unroll
+                    for (int k = 0; k < kFilterKeys; ++k) {
+                        const unsigned long long cells = s_reach[ck[k] >> kTileKeyBits];
+                        const bool keep = ((unsigned)(cells >> (32 * half)) & ~done_w) != 0u;
+                        const unsigned b = __ballot_sync(kFull, keep);
+                        if (keep) sm.queue[(q_tail + __popc(b & lt_mask)) & (kQueueCap - 1)] = ci[k];
+                        q_tail += __popc(b);
+                    }
+                }
+                __syncwarp();
+            };
+            uint32_t idf[kIdsAhead];
+            if (PASS == PASS_REST) {
+                q_tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
+#pragma unroll
+                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < q_tail ? kept[rg.x + 32u * k + lane] : 0u;
+            } else if (pos < rg.y) {
+                load_step();
+            }
+            auto gather = [&](unsigned stage) {
+                const unsigned n = min(32u, q_tail - q_head);
+                uint32_t id = kNoInstance;
+                if (lane < n) {
+                    id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(q_head + lane) & (kQueueCap - 1)]);
+                    const float4* p = reinterpret_cast<const float4*>(rec + id);
+                    async_copy_16(&sm.ring_a[stage][lane], p);
+                    async_copy_16(&sm.ring_c[stage][lane], conic + id);
+                    if (kBlend) async_copy_16(&sm.ring_f[stage][lane], p + 1);
+                }
+                sm.ring_id[stage][lane] = id;
+                async_copy_commit();   // one group per batch, empty or not: the waits below count groups
+                if (PASS == PASS_REST) {
+#pragma unroll
+                    for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
+                    const unsigned nxt = q_head + 32u * kIdsAhead + lane;
+                    idf[kIdsAhead - 1] = nxt < q_tail ? kept[rg.x + nxt] : 0u;
+                }
+                q_head += n;
+            };
+            fill();
+            gather(0u);
+            fill();
+            for (unsigned batch = 0;; ++batch) {
+                gather((batch + 1u) & 1u);
+                async_copy_wait<1>();   // all but the newest group: this batch has arrived
+                const unsigned stage = batch & 1u;
+                const uint32_t id_cur = sm.ring_id[stage][lane];
+                const bool staged = id_cur != kNoInstance;
+                if (__ballot_sync(kFull, staged) == 0u) break;   // batches are filled in order: nothing is left
+                // ---- lane j: the pixels instance j can reach that have not stopped
+                unsigned pixels = 0u;
+                if (staged) pixels = ellipse_pixels(sm.ring_a[stage][lane], sm.ring_c[stage][lane], reach, px0, py0) & ~done_w;
+                fill();   // (its __syncwarp also shows every lane the records the others have copied)
+                if (PASS == PASS_PRODUCT || kWeights) {
+                    // the list of this item: see the bilinear kernel
+                    const unsigned b = __ballot_sync(kFull, pixels != 0u);
+                    if (pixels) kept[rg.x + n_out + __popc(b & lt_mask)] = id_cur;
+                    n_out += __popc(b);
+                }
+                // ---- every lane runs down the instances of its own pixel, front to back
+                unsigned todo = warp_transpose_bits(pixels, lane);
+                unsigned taken = 0u;   // instances whose blending weight this pixel adds to
+                while (todo) {
+                    // two at a time: their exponentials do not wait for one another
+                    constexpr int kPair = 2;
+                    int j[kPair];
+                    float al[kPair], G[kPair];
+                    bool ok[kPair];
+#pragma unroll
+                    for (int u = 0; u < kPair; ++u) {
+                        ok[u] = todo != 0u;
+                        j[u] = ok[u] ? __ffs(todo) - 1 : j[0];
+                        todo &= todo - 1u;
+                        const float4 a = sm.ring_a[stage][j[u]], c = sm.ring_c[stage][j[u]];
+                        const float dx = a.x - pcx, dy = a.y - pcy;
+                        const float e = -0.5f * (c.x * dx * dx + c.z * dy * dy) - c.y * dx * dy;
+                        G[u] = KIND == BLEND_INFER ? __expf(e) : expf(e);
+                        ok[u] = ok[u] && !(e > 0.0f) && !(G[u] < threshold);
+                        al[u] = a.z * G[u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < kPair; ++u) {
+                        if (!ok[u] || done) continue;
+                        if (kBlend) {
+                            const float bw = Tr * al[u];
+                            if (kWeights && bw > 0.0f) {
+                                sm.out[j[u]][lane] = G[u] * bw;
+                                taken |= 1u << j[u];
+                            }
+                            const float4 f = sm.ring_f[stage][j[u]];
+                            C.x += bw * f.x; C.y += bw * f.y; C.z += bw * f.z; C.w += bw * f.w;
+                            if (kDepth) Z += bw * sm.ring_a[stage][j[u]].w;
+                        }
+                        Tr *= 1.0f - al[u];
+                        if (Tr < stop) done = true;
+                    }
+                    if (done) todo = 0u;
+                }
+                __syncwarp();
+                if (kWeights) {
+                    unsigned from = warp_transpose_bits(taken, lane);
+                    float sum = 0.0f;
+                    while (from) {
+                        sum += sm.out[lane][__ffs(from) - 1];
+                        from &= from - 1u;
+                    }
+                    if (sum > 0.0f) atomicAdd(blending_weights + id_cur, sum);
+                }
+                done_w = __ballot_sync(kFull, done);
+                __syncwarp();
+                if (done_w == kFull) break;   // every pixel has stopped: the rest of the list has no effect
+            }
+            async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
+            __syncwarp();
+        }
+        if ((PASS == PASS_PRODUCT || kWeights) && lane == 0) n_kept[sidx] = n_out;
+
+        if (PASS == PASS_PRODUCT) {
+            seg_T[sidx * 32 + lane] = Tr;   // this segment's product
+            continue;
+        }
+        const int64_t n_px = (int64_t)width * height;
+        const int64_t pi = (int64_t)py * width + px;
+        if (n_seg == 1u) {
+            if (inside) {
+                image[pi] = C.x;
+                image[n_px + pi] = C.y;
+                image[2 * n_px + pi] = C.z;
+                image[3 * n_px + pi] = C.w;
+                if (KIND == BLEND_INFER) {
+                    const float A = 1.0f - Tr;
+                    depth_image[pi] = A > 0.0f ? Z / A : 0.0f;
+                    alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : A;
+                } else {
+                    alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
+                }
+            }
+        } else {
+            // partial colour of this segment; the per-tile combine adds the segments up in order
+            const size_t si = sidx * 32 + lane;
+            seg_C[si] = C;
+            if (PASS == PASS_FIRST) seg_T[si] = Tr;   // the exact state behind segment 0
+            if (KIND == BLEND_INFER) {
+                seg_Z[si] = Z;
+                seg_E[si] = Tr;
+            } else if (seg + 1u == n_seg && inside) {
+                alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
+            }
+        }
+    }
+}
+
+struct __align__(16) GaussBackwardSmem {
+    float4 ring_a[2][32], ring_c[2][32], ring_f[2][32];
+    float4 pixel_grad[32];      // image gradient of the half's pixels
+    float out_bw[32][33];       // [staged instance][pixel]: blending weight of the fragment ...
+    float out_go[32][33];       // ... and what it adds to the opacity gradient
+    uint32_t ring_id[2][32];
+};
+constexpr size_t kGaussBackwardSmemBytes = kWarpBlendWarps * sizeof(GaussBackwardSmem);
+
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_backward_kernel(
+    const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
+    unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0, const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept,
+    const PointRec* __restrict__ rec, const float4* __restrict__ conic, const float* __restrict__ seg_T, const float4* __restrict__ seg_C,
+    const float* __restrict__ grad_image, const float* __restrict__ grad_alpha, const float* __restrict__ image,
+    const float* __restrict__ alpha_image, float4* __restrict__ grad_feat_view, float* __restrict__ grad_opacity, int width, int height, int gw,
+    float reach) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr unsigned kNoInstance = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char blend_smem[];
+    const unsigned lane = lane_id();
+    GaussBackwardSmem& sm = reinterpret_cast<GaussBackwardSmem*>(blend_smem)[threadIdx.x >> 5];
+    const unsigned n_first = __ldg(counts) * 2u;
+    const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
+    const unsigned n_rest = n_items - n_first;
+    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));
+    unsigned next_item = 0, visit_end = 0;
+    for (;;) {
+        if (next_item == visit_end) {
+            unsigned first_item = 0;
+            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
+            first_item = __shfl_sync(kFull, first_item, 0);
+            if (first_item >= n_items) break;
+            next_item = first_item;
+            visit_end = min(first_item + per_visit, n_items);
+        }
+        const unsigned item = next_item++;
+        const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
+        const int half = (int)((item < n_rest ? item : item - n_rest) & 1u);
+        const unsigned n_list = __ldg(n_kept + (size_t)(it.first + it.seg) * 2u + half);
+        const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg;
+        const size_t sidx = (size_t)(it.first + seg) * 2u + half;
+        if (n_list == 0u) continue;
+        const uint32_t* list = (half ? kept1 : kept0) + it.begin;
+        const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
+        const int px0 = tx * 8, py0 = ty * 8 + 4 * half;
+        const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
+
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f), Cfin = g, Crun = g;
+        float K = 0.0f, Tr = 1.0f;
+        bool done = !(px < width && py < height);
+        if (!done) {
+            const int64_t n_px = (int64_t)width * height;
+            const int64_t pi = (int64_t)py * width + px;
+            g = make_float4(__ldg(grad_image + pi), __ldg(grad_image + n_px + pi), __ldg(grad_image + 2 * n_px + pi),
+                            __ldg(grad_image + 3 * n_px + pi));
+            Cfin = make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi),
+                               __ldg(image + 3 * n_px + pi));
+            K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
+            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
+            if (n_seg > 1u) Crun = seg_C[sidx * 32 + lane];
+            done = Tr < kTransmittanceEps;
+        }
+        __syncwarp();   // the previous item's readers of pixel_grad are through
+        sm.pixel_grad[lane] = g;
+        unsigned done_w = __ballot_sync(kFull, done);
+
+        uint32_t idf[kIdsAhead];
+#pragma unroll
+        for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < n_list ? __ldg(list + 32u * k + lane) : 0u;
+        unsigned issued = 0;   // instances whose gather has started
+        auto gather = [&](unsigned stage) {
+            const unsigned n = min(32u, n_list - issued);
+            uint32_t id = kNoInstance;
+            if (lane < n) {
+                id = checked_point(idf[0]);
+                const float4* p = reinterpret_cast<const float4*>(rec + id);
+                async_copy_16(&sm.ring_a[stage][lane], p);
+                async_copy_16(&sm.ring_c[stage][lane], conic + id);
+                async_copy_16(&sm.ring_f[stage][lane], p + 1);
+            }
+            sm.ring_id[stage][lane] = id;
+            async_copy_commit();   // one group per batch, empty or not
+#pragma unroll
+            for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
+            const unsigned nxt = issued + 32u * kIdsAhead + lane;
+            idf[kIdsAhead - 1] = nxt < n_list ? __ldg(list + nxt) : 0u;
+            issued += n;
+        };
+        gather(0u);
+        for (unsigned batch = 0;; ++batch) {
+            gather((batch + 1u) & 1u);
+            async_copy_wait<1>();
+            const unsigned stage = batch & 1u;
+            const uint32_t id_cur = sm.ring_id[stage][lane];
+            const bool staged = id_cur != kNoInstance;
+            if (__ballot_sync(kFull, staged) == 0u) break;
+            unsigned pixels = 0u;
+            if (staged) pixels = ellipse_pixels(sm.ring_a[stage][lane], sm.ring_c[stage][lane], reach, px0, py0) & ~done_w;
+            __syncwarp();   // every lane sees the records the others have copied
+            unsigned todo = warp_transpose_bits(pixels, lane);
+            unsigned taken = 0u;   // instances this pixel hands a gradient to
+            while (todo) {
+                const int j = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const float4 a = sm.ring_a[stage][j], c = sm.ring_c[stage][j];
+                const float dx = a.x - pcx, dy = a.y - pcy;
+                const float e = -0.5f * (c.x * dx * dx + c.z * dy * dy) - c.y * dx * dy;
+                const float G = expf(e);
+                if (e > 0.0f || G < kTrainGaussThreshold) continue;
+                const float al = a.z * G;
+                const float bw = Tr * al;
+                const float4 f = sm.ring_f[stage][j];
+                Crun.x += bw * f.x; Crun.y += bw * f.y; Crun.z += bw * f.z; Crun.w += bw * f.w;
+                const float oma = 1.0f - al;
+                const float rcp = 1.0f / fmaxf(oma, kOneMinusAlphaEps);
+                const float from_features = (Tr * f.x + (Crun.x - Cfin.x) * rcp) * g.x +
+                                            (Tr * f.y + (Crun.y - Cfin.y) * rcp) * g.y +
+                                            (Tr * f.z + (Crun.z - Cfin.z) * rcp) * g.z +
+                                            (Tr * f.w + (Crun.w - Cfin.w) * rcp) * g.w;
+                sm.out_bw[j][lane] = bw > 0.0f ? bw : 0.0f;
+                sm.out_go[j][lane] = (from_features + K * rcp) * G;
+                taken |= 1u << j;
+                Tr *= oma;
+                if (Tr < kTransmittanceEps) { done = true; break; }
+            }
+            __syncwarp();
+            // ---- lane j: the sums of instance j over its pixels
+            unsigned from = warp_transpose_bits(taken, lane);
+            if (from) {
+                float4 sf = make_float4(0.f, 0.f, 0.f, 0.f);
+                float so = 0.0f;
+                do {
+                    const int p = __ffs(from) - 1;
+                    from &= from - 1u;
+                    const float bw = sm.out_bw[lane][p];
+                    const float4 pg = sm.pixel_grad[p];
+                    sf.x += bw * pg.x; sf.y += bw * pg.y; sf.z += bw * pg.z; sf.w += bw * pg.w;
+                    so += sm.out_go[lane][p];
+                } while (from);
+                if (sf.x != 0.0f || sf.y != 0.0f || sf.z != 0.0f || sf.w != 0.0f) atomicAdd(grad_feat_view + id_cur, sf);
+                if (so != 0.0f) atomicAdd(grad_opacity + id_cur, so);
+            }
+            done_w = __ballot_sync(kFull, done);
+            __syncwarp();
+            if (done_w == kFull) break;
+        }
+        async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
+        __syncwarp();
+    }
+}
+
 // SH chain rule for every point, zero rows for culled ones, written as 72 contiguous bytes per point
 // through a shared-memory slab so the stores are coalesced 16-byte vectors.
 // src/bilinear/kernels.cu:86-104 + include/sh_utils.cuh:44-62; the zero rows replace the
@@ -3162,6 +3690,7 @@ struct PointBlob {
     uint2* bounds;
     uint32_t* quad;                       // warp blend: packed footprint origin per point (see pack_quad)
     float4* conic;
+    uint4* foot;                          // gaussian: tile bounds and ellipse per point (see pack_footprint)
     unsigned* block_visible;              // survivors per chunk of kPreThreads points
     unsigned* group_visible;              // per group of 4 chunks; scanned in place
     unsigned long long* group_instances;
@@ -3184,8 +3713,9 @@ PointBlob carve_point_blob(void* p, int64_t n, int mode) {
     const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
     b.rec = c.take<PointRec>(n);
     b.bounds = c.take<uint2>(n);
-    b.quad = c.take<uint32_t>(mode == INPC_MODE_BILINEAR ? n : 0);
+    b.quad = mode == INPC_MODE_BILINEAR ? c.take<uint32_t>(n) : nullptr;
     b.conic = mode == INPC_MODE_GAUSSIAN ? c.take<float4>(n) : nullptr;
+    b.foot = mode == INPC_MODE_GAUSSIAN ? c.take<uint4>(n) : nullptr;
     b.block_visible = c.take<unsigned>(nb);
     b.group_visible = c.take<unsigned>(ceil_div<int64_t>(nb, 4));
     b.group_instances = c.take<unsigned long long>(ceil_div<int64_t>(nb, 4));
@@ -3225,9 +3755,9 @@ struct InstanceBlob {
 
 // Upper bound on the segments of the warp blend for up to n_instances instances (see segment_lengths): one per tile, one more
 // for every tile that is longer than a first segment, and the later segments that are full.
-int64_t max_warp_segments(int64_t n_instances, int n_tiles) {
-    const int64_t target = kSegmentTarget;
-    const int64_t by_first = ceil_div<int64_t>(n_instances, kFirstSegmentMax), by_later = ceil_div<int64_t>(n_instances, kLaterSegmentMax);
+int64_t max_warp_segments(int64_t n_instances, int n_tiles, const SegmentLimits limits) {
+    const int64_t target = limits.target;
+    const int64_t by_first = ceil_div<int64_t>(n_instances, limits.first_max), by_later = ceil_div<int64_t>(n_instances, limits.later_max);
     const int64_t longer = by_first > 2 * target ? by_first : 2 * target;
     return n_tiles + (longer < n_tiles ? longer : n_tiles) + (by_later > target ? by_later : target) + 1;
 }
@@ -3239,18 +3769,20 @@ int64_t max_segments(int64_t n_instances, int n_tiles, int tile) {
 }
 
 // Which of the two blend organisations a call uses: one warp per tile part with the dead-instance filter
-// (bilinear splats, 8x8 tiles) or one block per (tile, segment).
+// (8x8 tiles) or one block per (tile, segment).
 constexpr int kWarpBlendParts = 2;   // work items per (tile, segment): the two 8x4 halves
-bool uses_warp_blend(int mode, int tile) { return mode == INPC_MODE_BILINEAR && tile == 8; }
+bool uses_warp_blend(int tile) { return tile == 8; }
+// Bilinear splats touch at most 2x2 tiles: with the warp blend nothing waits for their counts.
+bool has_instance_bound(int mode, int tile) { return mode == INPC_MODE_BILINEAR && uses_warp_blend(tile); }
 
-// The warp-blend path sizes its arrays for 4 instances per point; most splats touch one tile of four or none twice, about 1.3
+// The bounded path sizes its arrays for 4 instances per point; most splats touch one tile of four or none twice, about 1.3
 // on average (2^23 samples at 1237x822: 1.26; at 3840x2160 less).  Only picks tile sizes.
-int64_t likely_instances(int64_t capacity, bool deferred) { return deferred ? capacity / 3 : capacity; }
+int64_t likely_instances(int64_t capacity, int mode, int tile) { return has_instance_bound(mode, tile) ? capacity / 3 : capacity; }
 
 InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int tile, int mode, bool with_depth, int c4 = 1) {
     InstanceBlob b;
     Carver c(p);
-    const bool warp_blend = uses_warp_blend(mode, tile);
+    const bool warp_blend = uses_warp_blend(tile);
     // [0] segments (block blend) or non-empty tiles (warp blend), [1] later segments (warp blend), [2..5] work tickets of
     // the warp blend passes FIRST, PRODUCT, REST and of its backward pass.  Counters, tile ranges and the sort's state lie side
     // by side: they are cleared together.
@@ -3258,11 +3790,11 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int 
     b.ranges = c.take<uint2>(n_tiles);
     c.off = align_up(c.off);
     b.sort_ws = c.base + c.off;
-    c.off += sort_workspace_bytes(n_instances, likely_instances(n_instances, warp_blend));
+    c.off += sort_workspace_bytes(n_instances, likely_instances(n_instances, mode, tile));
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n_instances);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n_instances);
     // upper bound on the number of (tile, segment) pairs, known from the instance count alone
-    b.max_segments = warp_blend ? max_warp_segments(n_instances, n_tiles) : max_segments(n_instances, n_tiles, tile);
+    b.max_segments = warp_blend ? max_warp_segments(n_instances, n_tiles, segment_limits(mode, !with_depth)) : max_segments(n_instances, n_tiles, tile);
     const size_t px = (size_t)b.max_segments * tile * tile;
     b.segs = c.take<Segment>(warp_blend ? 0 : b.max_segments);
     b.tile_first = c.take<uint32_t>(n_tiles);
@@ -3397,7 +3929,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     }
     unsigned* status = acquire_status(entry);
     if (!status) return INPC_E_CUDA;
-    const bool warp_blend = uses_warp_blend(MODE, rp.tile);
+    const bool warp_blend = uses_warp_blend(rp.tile);
     const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
     const PointBlob sizing = carve_point_blob(nullptr, n, MODE);
     void* pblob = alloc_point(user, sizing.total);
@@ -3412,7 +3944,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     // for 4 n instances and lets the kernels read the two counts from device memory: no host synchronisation at
     // all (the reference reads both counts back with blocking copies, src/bilinear/forward.cu:86-89).  The other
     // paths (gaussian splats have no such bound) read the counts back once.
-    const bool deferred = warp_blend && n > 0 && n < ((int64_t)1 << 28);
+    const bool deferred = has_instance_bound(MODE, rp.tile) && n > 0 && n < ((int64_t)1 << 28);
     int64_t n_visible = 0, n_instances = 0;
     uint32_t key_base = 0;
     int key_bits = 0;
@@ -3428,7 +3960,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     };
     auto clear_instance_blob = [&](ClearList& list) {
         list.add(ib.n_segments, (size_t)(static_cast<char*>(ib.sort_ws) - reinterpret_cast<char*>(ib.n_segments)) +
-                                    sort_zero_bytes(n_instances, likely_instances(n_instances, warp_blend), tile_bits));
+                                    sort_zero_bytes(n_instances, likely_instances(n_instances, MODE, rp.tile), tile_bits));
     };
     int rc;
     const unsigned long long* n_visible_dev = deferred ? pb.counters : nullptr;
@@ -3476,8 +4008,8 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             // the projection pass needs nothing from the host: it runs while the host waits for the counters
             preprocess_kernel<MODE, VARIANT><<<(unsigned)nb, kPreThreads, 0, stream>>>(
                 ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max,
-                pb.rec, pb.bounds, warp_blend ? pb.quad : nullptr,
-                pb.conic, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
+                pb.rec, pb.bounds, MODE == INPC_MODE_BILINEAR && warp_blend ? pb.quad : nullptr,
+                pb.conic, warp_blend ? pb.foot : nullptr, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
             INPC_LAUNCH_CHECK("preprocess_kernel");
         }
         if (!deferred) {
@@ -3532,16 +4064,18 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             else
                 instance_count_kernel<false><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
-            if (warp_blend)
-                emit_instances_kernel<true><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+            if (warp_blend && MODE == INPC_MODE_GAUSSIAN)
+                emit_instances_kernel<EMIT_CELLS><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, pb.foot, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+            else if (warp_blend)
+                emit_instances_kernel<EMIT_QUAD><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             else
-                emit_instances_kernel<false><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                emit_instances_kernel<EMIT_BOUNDS><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             INPC_LAUNCH_CHECK("emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
-        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, warp_blend), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream)
-                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, warp_blend), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
+        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, MODE, rp.tile), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream)
+                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, MODE, rp.tile), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
         if (rc != INPC_OK) return rc;
         const int64_t range_blocks = ceil_div<int64_t>(n_instances, 256 * 8), range_cap = (int64_t)sm_count() * 8;
         tile_ranges_kernel<<<(unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream>>>(ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
@@ -3551,9 +4085,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         StageScope scope(STAGE_SORT_TILE, stream);
         const int item_blocks = ceil_div(n_tiles, kItemTilesPerBlock);
         uint2* item_sums = reinterpret_cast<uint2*>(ib.tile_rank);
-        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
+        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
         INPC_LAUNCH_CHECK("warp_items_count_kernel");
-        warp_items_fill_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
+        warp_items_fill_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
         INPC_LAUNCH_CHECK("warp_items_fill_kernel");
     } else {
         StageScope scope(STAGE_SORT_TILE, stream);
@@ -3589,6 +4123,7 @@ RasterParams make_params(const inpc_view* view, int tile_size, float sigma_world
     rp.sigma_world = sigma_world;
     rp.sigma_cutoff = sigma_cutoff;
     rp.scales = scales;
+    rp.reach = -2.0f * logf(expf(-0.5f * sigma_cutoff * sigma_cutoff));
     return rp;
 }
 
@@ -3596,10 +4131,9 @@ RasterParams make_params(const inpc_view* view, int tile_size, float sigma_world
 // scenes): one per thread is fastest for both tile sizes; deeper batches lose more to mask traffic
 // and same-word atomicOr contention than they gain from fewer barriers.
 template <int T> struct BlendConfig;
-template <> struct BlendConfig<8> { static constexpr int kIpt = 1; };
 template <> struct BlendConfig<16> { static constexpr int kIpt = 1; };
 
-int blend_batch(int tile) { return tile == 8 ? 64 * BlendConfig<8>::kIpt : 256 * BlendConfig<16>::kIpt; }
+int blend_batch(int tile) { return tile * tile * BlendConfig<16>::kIpt; }
 
 // Persistent grid of the warp blend: enough blocks to fill the GPU (the item counts live on the device).
 int warp_blend_grid(unsigned* grid) {
@@ -3717,6 +4251,60 @@ int launch_bilinear_backward(const RasterParams& rp, const PointBlob& pb, const 
     return INPC_OK;
 }
 
+template <int PASS, int KIND>
+int launch_gaussian_warp_forward_pass(unsigned grid, const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic,
+                                      const ForwardPassArgs& a, float threshold, float reach, cudaStream_t stream) {
+    static bool attr_set[kMaxDevices] = {false};
+    constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
+    const int rc = opt_in_dynamic_smem(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, attr_set);
+    if (rc != INPC_OK) return rc;
+    blend_gaussian_warp_forward_kernel<PASS, KIND><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
+        items, counts, ticket, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
+        a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, threshold, reach);
+    INPC_LAUNCH_CHECK("blend_gaussian_warp_forward_kernel");
+    return INPC_OK;
+}
+
+template <int KIND>
+int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image, float* depth,
+                                 float* alpha, float* blending_weights, float threshold, cudaStream_t stream) {
+    unsigned grid = 1;
+    int rc = warp_blend_grid(&grid);
+    if (rc != INPC_OK) return rc;
+    const int W = rp.v.width, H = rp.v.height;
+    const unsigned threads = kWarpBlendWarps * 32;
+    const ForwardPassArgs a{ib.keys[t_alt], ib.ids[t_alt], pb.rec, nullptr, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
+                            ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, W, H, rp.gw, rp.gh};
+    rc = launch_gaussian_warp_forward_pass<PASS_FIRST, KIND>(grid, ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, threshold, rp.reach, stream);
+    if (rc != INPC_OK) return rc;
+    rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
+    if (rc != INPC_OK) return rc;
+    warp_blend_prefix_kernel<<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_T);
+    INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
+    rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
+    if (rc != INPC_OK) return rc;
+    warp_blend_combine_kernel<KIND, 1><<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
+                                                                     rp.gw, rp.gh);
+    INPC_LAUNCH_CHECK("warp_blend_combine_kernel");
+    return INPC_OK;
+}
+
+int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
+                                  const float* grad_alpha, const float* image, const float* alpha, float4* gfv, float* grad_opacities,
+                                  cudaStream_t stream) {
+    unsigned grid = 1;
+    const int rc = warp_blend_grid(&grid);
+    if (rc != INPC_OK) return rc;
+    static bool attr_set[kMaxDevices] = {false};
+    const int rc_attr = opt_in_dynamic_smem(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, attr_set);
+    if (rc_attr != INPC_OK) return rc_attr;
+    blend_gaussian_warp_backward_kernel<<<grid, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream>>>(
+        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
+        grad_image, grad_alpha, image, alpha, gfv, grad_opacities, rp.v.width, rp.v.height, rp.gw, rp.reach);
+    INPC_LAUNCH_CHECK("blend_gaussian_warp_backward_kernel");
+    return INPC_OK;
+}
+
 template <int T, int KIND>
 int launch_gaussian_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, const uint32_t* ids, float* image,
                             float* depth, float* alpha, float* blending_weights, float threshold, cudaStream_t stream) {
@@ -3749,7 +4337,7 @@ int launch_blend_forward(int mode, const RasterParams& rp, const PointBlob& pb, 
         if (rp.tile == 8) return launch_bilinear_warp_forward<KIND>(rp, pb, ib, t_alt, nullptr, image, depth, alpha, blending_weights, stream);
         return launch_bilinear_forward<16, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, stream);
     }
-    if (rp.tile == 8) return launch_gaussian_forward<8, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, threshold, stream);
+    if (rp.tile == 8) return launch_gaussian_warp_forward<KIND>(rp, pb, ib, t_alt, image, depth, alpha, blending_weights, threshold, stream);
     return launch_gaussian_forward<16, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, threshold, stream);
 }
 
@@ -3828,9 +4416,9 @@ int dispatch_rows(int channels, F&& f) {
 
 // The outputs of a call that start at zero.  The warp blend has no work items for tiles without instances, so their pixels
 // are cleared; the block blend writes every tile.  `depth` and `weights` may be null.
-ClearList outputs_to_clear(const RasterParams& rp, int mode, int channels, float* image, float* depth, float* alpha, float* weights, int64_t n) {
+ClearList outputs_to_clear(const RasterParams& rp, int channels, float* image, float* depth, float* alpha, float* weights, int64_t n) {
     ClearList list;
-    if (uses_warp_blend(mode, rp.tile)) {
+    if (uses_warp_blend(rp.tile)) {
         const size_t n_px = (size_t)rp.v.width * rp.v.height * rp.n_sets;
         list.add(image, sizeof(float) * channels * n_px);
         list.add(depth, sizeof(float) * n_px);
@@ -3849,7 +4437,7 @@ int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* p
     InstanceBlob ib;
     int rc = run_front<INPC_MODE_BILINEAR, VAR_ROWS>(rp, n, positions, nullptr, opacities, alloc_point, alloc_instance, alloc_user, state,
                                                      KIND == BLEND_INFER, &pb, &ib, stream, KIND == BLEND_INFER ? "inpc_render_rows" : "inpc_rasterize_rows_forward",
-                                                     outputs_to_clear(rp, INPC_MODE_BILINEAR, channels, image, depth, alpha, blending_weights, n), channels / 4);
+                                                     outputs_to_clear(rp, channels, image, depth, alpha, blending_weights, n), channels / 4);
     if (rc != INPC_OK) return rc;
     const int t_alt = tile_buffer_of(state, rp.gw * rp.gh);
     {
@@ -3882,7 +4470,7 @@ extern "C" int inpc_rasterize_forward(int mode, int tile_size, const inpc_view* 
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, 0.0f, 3.0f, nullptr);
-    const ClearList clear = outputs_to_clear(rp, mode, 4, image, nullptr, alpha, blending_weights, n);
+    const ClearList clear = outputs_to_clear(rp, 4, image, nullptr, alpha, blending_weights, n);
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
@@ -3920,7 +4508,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     const int W = rp.v.width, H = rp.v.height;
     // the caller's scratch holds 33 floats per point: four 32-byte slot records and one mask word for the warp blend
     // or, for the other paths, the (n,4) accumulation buffer of their atomics
-    const bool slots = uses_warp_blend(state->mode, state->tile_size);
+    const bool slots = has_instance_bound(state->mode, state->tile_size);
     if (slots && (reinterpret_cast<uintptr_t>(grad_features_view) & 31u)) {
         set_error("inpc_rasterize_backward: grad_features_view must be 32-byte aligned");
         return INPC_E_INVALID;
@@ -3930,11 +4518,11 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     ClearList clear;
     if (slots) {
         clear.add(slot_mask, sizeof(unsigned) * (size_t)n);
-        clear.add(ib.n_segments + 5, sizeof(uint32_t));   // the work ticket
     } else {
         clear.add(grad_features_view, sizeof(float4) * (size_t)n);
         clear.add(grad_opacities, sizeof(float) * (size_t)n);
     }
+    if (uses_warp_blend(state->tile_size)) clear.add(ib.n_segments + 5, sizeof(uint32_t));   // the work ticket
     rc = launch_clear(clear, stream);
     if (rc != INPC_OK) return rc;
     {
@@ -3944,12 +4532,13 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
                               : launch_bilinear_backward<16>(rp, pb, ib, ids, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
             if (rc != INPC_OK) return rc;
         } else {
-            const unsigned grid = (unsigned)ib.max_segments;
-            if (rp.tile == 8)
-                blend_gaussian_backward_kernel<8><<<grid, 64, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, W, H, rp.gw);
-            else
-                blend_gaussian_backward_kernel<16><<<grid, 256, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, W, H, rp.gw);
-            INPC_LAUNCH_CHECK("blend_gaussian_backward_kernel");
+            if (rp.tile == 8) {
+                rc = launch_gaussian_warp_backward(rp, pb, ib, tile_buffer_of(state, n_tiles), grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
+                if (rc != INPC_OK) return rc;
+            } else {
+                blend_gaussian_backward_kernel<16><<<(unsigned)ib.max_segments, 256, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, W, H, rp.gw);
+                INPC_LAUNCH_CHECK("blend_gaussian_backward_kernel");
+            }
         }
     }
     StageScope scope(STAGE_PREPROCESS_BWD, stream);
@@ -3977,7 +4566,7 @@ extern "C" int inpc_render(int mode, int tile_size, const inpc_view* view, int64
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, sigma_world, sigma_cutoff, nullptr);
-    const ClearList clear = outputs_to_clear(rp, mode, 4, image, depth, alpha, nullptr, n);
+    const ClearList clear = outputs_to_clear(rp, 4, image, depth, alpha, nullptr, n);
     inpc_raster_state st;
     PointBlob pb;
     InstanceBlob ib;
@@ -4005,7 +4594,7 @@ extern "C" int inpc_render_preextracted(int mode, int tile_size, const inpc_view
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, sigma_world, sigma_cutoff, scales);
-    const ClearList clear = outputs_to_clear(rp, mode, 4, image, depth, alpha, nullptr, n);
+    const ClearList clear = outputs_to_clear(rp, 4, image, depth, alpha, nullptr, n);
     inpc_raster_state st;
     PointBlob pb;
     InstanceBlob ib;
@@ -4056,7 +4645,7 @@ extern "C" int inpc_render_multi(int tile_size, const inpc_view* view, int n_set
     PointBlob pb;
     InstanceBlob ib;
     rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n_virtual, nullptr, nullptr, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib,
-                                                  stream, "inpc_render_multi", outputs_to_clear(rp, INPC_MODE_BILINEAR, 4, images, depths, alphas, nullptr, n_virtual), 1, &ps);
+                                                  stream, "inpc_render_multi", outputs_to_clear(rp, 4, images, depths, alphas, nullptr, n_virtual), 1, &ps);
     if (rc != INPC_OK) return rc;
     rc = launch_blend_forward<BLEND_INFER>(INPC_MODE_BILINEAR, rp, pb, ib, &st, images, depths, alphas, nullptr, 0.0f, stream);
     return rc != INPC_OK ? rc : end_index_checks(stream);

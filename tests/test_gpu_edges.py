@@ -103,3 +103,51 @@ def test_blend_at_the_edges_of_its_segments(n, rows):
     assert_close(f.grad.float().cpu().numpy(), np.asarray(gf, np.float32), rtol=tol_f["rtol"] + eps, atol=tol_f["atol"], what="grad_features")
     # opacity gradients are differences of sums of the order of 1e-3
     assert_close(o.grad.cpu().numpy(), go, rtol=1e-3 + eps, atol=2e-8 + 1e-3 * eps, what="grad_opacities")
+
+
+# gaussian splats on 8x8 tiles: footprints from a fraction of a pixel to several tiles, image sides around tile and half borders
+@pytest.mark.parametrize("width,height", [(8, 4), (9, 5), (64, 36), (67, 45)])
+@pytest.mark.parametrize("sigma_px", [0.01, 0.7, 3.0, 40.0])
+def test_gaussian_footprints_at_tile_edges(width, height, sigma_px):
+    import inpc_b200
+    from helpers import assert_close, oracle_camera
+    from inpc_b200.views import look_at_view
+    g = torch.Generator().manual_seed(width * 7 + int(sigma_px * 100))
+    n, focal = 300, 0.5 * width                     # a wide view: splats off the axis are long ellipses
+    view = look_at_view((0.1, 0.2, 2.0), (0.0, 0.0, 0.0), width, height, focal, focal * 1.1)
+    pos = ((torch.rand((n, 3), generator=g) * 2 - 1) * torch.tensor([2.5, 2.0, 1.2])).contiguous()
+    feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+    opac = torch.rand((n, 1), generator=g) * 0.3 + 0.01
+    scales = torch.exp(torch.randn((n, 1), generator=g) * 0.5) * (2.0 * sigma_px / focal)
+    img, dep, alp = inpc_b200.INPCRasterizer().render_preextracted(view.to(DEV), 1, pos.to(DEV), feats.to(DEV), opac.to(DEV), scales.to(DEV))
+    oi, od, oa, _ = O.render_preextracted(O.GAUSSIAN, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy(), scales.numpy(),
+                                          0.05 / view.camera.focal_y, 3.0)
+    # a fragment within rounding of the cut-off (weight 0.011 of at most 0.31) may fall on either side of it
+    for got, want, what in ((img, oi, "image"), (dep, od, "depth"), (alp, oa, "alpha")):
+        assert_close(got.cpu().numpy(), want, rtol=2e-4, atol=2e-5, max_bad=4, what=what)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 513, 20_001, 700_001])
+def test_gaussian_blend_at_the_edges_of_its_segments(n):
+    import inpc_b200
+    from helpers import assert_close, oracle_camera
+    view, pos, opac = _one_tile_scene(n, n)
+    g = torch.Generator().manual_seed(n + 1)
+    gi, ga = torch.randn((4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
+    feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+    f, o = feats.to(DEV).requires_grad_(True), opac.to(DEV).requires_grad_(True)
+    image, alpha, bw = inpc_b200.INPCRasterizer()(view.to(DEV), 1, pos.to(DEV), f, o)
+    st = O.rasterize_forward(O.GAUSSIAN, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy())
+    gf, go, _ = O.rasterize_backward(st, gi.numpy(), ga.numpy())
+    torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
+    # the bounds of the bilinear test with about six fragments per point; the exponentials of device and oracle differ by two
+    # units of the last place, and a fragment within rounding of the cut-off may fall on either side of it, which moves its point
+    # by a hundredth and the pixel by a hundredth of the point's opacity
+    eps = n / 10 * 2.0 ** -25 + 2.0 ** -22
+    cut = 0.012 * float(opac.max())
+    few = 4 + n // 5000
+    assert_close(image.detach().cpu().numpy(), st.image, rtol=1e-4, atol=1e-5 + 0.2 * eps + cut * (n > 1000), what="image")
+    assert_close(alpha.detach().cpu().numpy(), st.alpha, rtol=1e-5, atol=1e-6 + eps + cut * (n > 1000), max_bad=4, what="alpha")
+    assert_close(bw.cpu().numpy(), st.blending_weights, rtol=4e-4 + eps, atol=1e-9, max_bad=few, what="blending weights")
+    assert_close(f.grad.float().cpu().numpy(), np.asarray(gf, np.float32), rtol=4e-3 + eps, atol=2e-7, max_bad=36 * few, what="grad_features")
+    assert_close(o.grad.cpu().numpy(), go, rtol=2e-3 + eps, atol=4e-8 + 1e-3 * eps, max_bad=few, what="grad_opacities")
