@@ -248,36 +248,35 @@ __device__ __forceinline__ unsigned scan_words(unsigned* data, int64_t n, unsign
 constexpr int kPreThreads = 256;
 constexpr unsigned kCountShift = 30;   // bilinear: (tiles touched - 1) in key bits 30..31 when the depth offsets fit below
 
-// Pass 1 of the deterministic compaction: per block, how many points survive culling and how many
-// (point, tile) instances they create.  The last block scans the groups' counts (groups of 4 chunks of kPreThreads points)
-// and leaves the totals in counters[0] (visible) and counters[1] (instances), the range of depth bit patterns the
-// keys are offsets into in counters[2..3] and *depth_min, *depth_max: measured (`range` given: the words start at zero
-// and collect the largest pattern and the largest complement), or fixed_lo .. fixed_hi.
-template <int MODE, int VARIANT>
-__global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
-    const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_groups, unsigned* __restrict__ block_visible,
-    unsigned* group_visible, unsigned long long* group_instances, unsigned* range, unsigned* done, unsigned fixed_lo, unsigned fixed_hi,
+// Pass 1 of the deterministic compaction: per chunk of kPreThreads points, how many points survive culling, and how many
+// (point, tile) instances there are in all.  The last block scans the counts of the groups of 4 chunks (group_visible and
+// *instances start at zero) and leaves the totals in counters[0] (visible) and counters[1] (instances), the range of depth bit
+// patterns the keys are offsets into in counters[2..3] and *depth_min, *depth_max: measured (RANGE: the words of `range` start
+// at zero and collect the largest pattern and the largest complement), or fixed_lo .. fixed_hi.
+//
+// Bound by the instructions of the projection (96 per point; 33 % of DRAM).  Every lane takes 4 consecutive points (three 16-byte
+// loads when the array is aligned), a warp a chunk in two steps, the positions of the next step travelling while this one's are
+// projected; nothing waits for other warps before the last block's scan.  2^23 / 2^25 points 36 / 129 us
+// (one block per group with its fence and atomic 62 / 226; persistent blocks with a barrier per group 44 / 154, with the
+// positions loaded ahead 39 / 144).
+template <int MODE, int VARIANT, bool RANGE>
+__global__ void __launch_bounds__(kPreThreads, 4) visibility_count_kernel(
+    const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_chunks, unsigned* __restrict__ block_visible,
+    unsigned* group_visible, unsigned long long* instances, unsigned* range, unsigned* done, unsigned fixed_lo, unsigned fixed_hi,
     unsigned* __restrict__ depth_min, unsigned* __restrict__ depth_max, unsigned long long* __restrict__ counters) {
-    // Every thread takes 4 consecutive points (three 16-byte loads when the array is aligned), so a
-    // group of a block covers 4 chunks of kPreThreads points; counts are kept per chunk because the projection
-    // pass works on chunks of kPreThreads points.  A block takes several groups one after the other (one block per group, each
-    // with its fence and atomic for the last-block test: 62 / 226 us for 2^23 / 2^25 points, 44 / 154 like this).
     constexpr int kPerThread = 4;
-    constexpr int kWarpsPerChunk = kPreThreads / kPerThread / 32;   // 2
-    __shared__ unsigned s_v[2][kPreThreads / 32];
-    __shared__ unsigned long long s_i[2][kPreThreads / 32];
-    const int64_t n_virtual = ps.start[ps.count];
-    const int warp = threadIdx.x >> 5;
+    constexpr unsigned kStep = 32 * kPerThread;        // points of a warp and step
+    static_assert(kPreThreads == 2 * kStep, "a chunk is two steps");
     const W2C m = load_w2c(rp.v.w2c);
     unsigned lo = 0xFFFFFFFFu, hi = 0u;
-    int flip = 0;
-    for (unsigned group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1) {
-        // this group's set; indices below are local to it
-        const int set = set_of_block(ps, (int64_t)group * kPreThreads * 4);
+    unsigned long long inst = 0;
+    // the positions of this lane's points of a step, zeros behind the end of their set; returns how many points there are
+    auto load_step = [&](unsigned step, float (&p)[3 * kPerThread], int& set, int64_t& first) -> int {
+        // indices are local to the step's set
+        set = set_of_block(ps, (int64_t)step * kStep);
         const float* __restrict__ positions = ps.positions[set];
         const int64_t n = ps.size[set];
-        const int64_t first = ((int64_t)group * kPreThreads + threadIdx.x) * kPerThread - ps.start[set];
-        float p[3 * kPerThread];
+        first = (int64_t)step * kStep + lane_id() * kPerThread - ps.start[set];
         if (first + kPerThread <= n && (reinterpret_cast<uintptr_t>(positions) & 15u) == 0) {
             const float4* src = reinterpret_cast<const float4*>(positions + 3 * first);
 #pragma unroll
@@ -285,79 +284,69 @@ __global__ void __launch_bounds__(kPreThreads) visibility_count_kernel(
                 const float4 v = __ldg(src + k);
                 p[4 * k] = v.x; p[4 * k + 1] = v.y; p[4 * k + 2] = v.z; p[4 * k + 3] = v.w;
             }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 3 * kPerThread; ++k) p[k] = first * 3 + k < 3 * n ? __ldg(positions + 3 * first + k) : 0.0f;
+            return kPerThread;
         }
-        unsigned v = 0;
-        unsigned long long c = 0;
 #pragma unroll
-        for (int k = 0; k < kPerThread; ++k) {
-            if (first + k < n) {
-                const Projection pr = project_point<MODE, VARIANT>(p[3 * k], p[3 * k + 1], p[3 * k + 2], m, rp, first + k, set);
-                if (pr.visible) {
-                    v += 1u;
-                    c += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
-                    const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
-                    lo = min(lo, bits);
-                    hi = max(hi, bits);
+        for (int k = 0; k < 3 * kPerThread; ++k) p[k] = first * 3 + k < 3 * n ? __ldg(positions + 3 * first + k) : 0.0f;
+        return (int)max((int64_t)0, min((int64_t)kPerThread, n - first));
+    };
+    const unsigned n_warps = gridDim.x * (kPreThreads / 32);
+    unsigned chunk = blockIdx.x * (kPreThreads / 32) + (threadIdx.x >> 5);
+    float next[3 * kPerThread];
+    int next_set = 0, next_here = 0;
+    int64_t next_first = 0;
+    if (chunk < n_chunks) next_here = load_step(2u * chunk, next, next_set, next_first);
+    for (; chunk < n_chunks; chunk += n_warps) {
+        unsigned v = 0;
+#pragma unroll 1
+        for (unsigned half = 0; half < 2u; ++half) {
+            float p[3 * kPerThread];
+#pragma unroll
+            for (int k = 0; k < 3 * kPerThread; ++k) p[k] = next[k];
+            const int set = next_set, here = next_here;
+            const int64_t first = next_first;
+            const unsigned following = half == 0u ? chunk : chunk + n_warps;
+            if (following < n_chunks) next_here = load_step(2u * following + (half ^ 1u), next, next_set, next_first);
+#pragma unroll
+            for (int k = 0; k < kPerThread; ++k) {
+                if (k < here) {
+                    const Projection pr = project_point<MODE, VARIANT>(p[3 * k], p[3 * k + 1], p[3 * k + 2], m, rp, first + k, set);
+                    if (pr.visible) {
+                        v += 1u;
+                        inst += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
+                        if (RANGE) {
+                            const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
+                            lo = min(lo, bits);
+                            hi = max(hi, bits);
+                        }
+                    }
                 }
             }
         }
         v = __reduce_add_sync(0xffffffffu, v);
-        if (MODE == INPC_MODE_BILINEAR) {
-            c = __reduce_add_sync(0xffffffffu, (unsigned)c);   // at most 4 per point
-        } else {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-        }
-        if (lane_id() == 0) { s_v[flip][warp] = v; s_i[flip][warp] = c; }
-        __syncthreads();
-        if (threadIdx.x < kPerThread) {
-            // chunk `threadIdx.x` of this group
-            const int64_t chunk = (int64_t)group * kPerThread + threadIdx.x;
-            if (chunk * kPreThreads < n_virtual) {   // chunks of the padding behind a set count zero survivors
-                unsigned tv = 0;
-#pragma unroll
-                for (int w = 0; w < kWarpsPerChunk; ++w) tv += s_v[flip][threadIdx.x * kWarpsPerChunk + w];
-                block_visible[chunk] = tv;
-            }
-        }
-        if (threadIdx.x == 0) {
-            unsigned tv = 0;
-            unsigned long long ti = 0;
-#pragma unroll
-            for (int w = 0; w < kPreThreads / 32; ++w) { tv += s_v[flip][w]; ti += s_i[flip][w]; }
-            // totals of this group of 4 chunks: the scan runs over groups, four times fewer entries
-            group_visible[group] = tv;
-            group_instances[group] = ti;
+        if (lane_id() == 0) {
+            block_visible[chunk] = v;
+            if (v) atomicAdd(group_visible + (chunk >> 2), v);   // the scan runs over groups, four times fewer entries
         }
     }
-    // (callers that know a bound on the depths beforehand pass no pointer)
-    if (range) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
+    if (lane_id() == 0 && inst) atomicAdd(instances, inst);
+    // (callers that know a bound on the depths beforehand do not ask for the range)
+    if (RANGE) {
         lo = __reduce_min_sync(0xffffffffu, lo);
         hi = __reduce_max_sync(0xffffffffu, hi);
         if (lane_id() == 0 && lo <= hi) { atomicMax(range, ~lo); atomicMax(range + 1, hi); }
     }
     if (!last_block(done, gridDim.x)) return;
     __shared__ unsigned s_scan[kPreThreads / 32 + 1];
-    const unsigned visible = scan_words<kPreThreads>(group_visible, n_groups, s_scan);
-    unsigned long long inst = 0;
-#pragma unroll 8
-    for (unsigned k = threadIdx.x; k < n_groups; k += kPreThreads) inst += __ldcg(group_instances + k);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
-    if (lane_id() == 0) s_i[0][threadIdx.x >> 5] = inst;
-    __syncthreads();
+    const unsigned visible = scan_words<kPreThreads>(group_visible, (n_chunks + 3u) / 4u, s_scan);
     if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-#pragma unroll
-        for (int w = 0; w < kPreThreads / 32; ++w) t += s_i[0][w];
-        const unsigned lo = range ? ~__ldcg(range) : fixed_lo, hi = range ? __ldcg(range + 1) : fixed_hi;
+        const unsigned first_key = RANGE ? ~__ldcg(range) : fixed_lo, last_key = RANGE ? __ldcg(range + 1) : fixed_hi;
         counters[0] = visible;
-        counters[1] = t;
-        counters[2] = *depth_min = lo;
-        counters[3] = *depth_max = hi;
+        counters[1] = __ldcg(instances);
+        counters[2] = *depth_min = first_key;
+        counters[3] = *depth_max = last_key;
     }
 }
 
@@ -3693,14 +3682,13 @@ struct PointBlob {
     uint4* foot;                          // gaussian: tile bounds and ellipse per point (see pack_footprint)
     unsigned* block_visible;              // survivors per chunk of kPreThreads points
     unsigned* group_visible;              // per group of 4 chunks; scanned in place
-    unsigned long long* group_instances;
     unsigned long long* counters;   // visible, instances, smallest / largest depth bit pattern
     unsigned* depth_min;
     unsigned* depth_max;
     uint32_t* keys[2];
     uint32_t* ids[2];
     unsigned* inst_block_sums;
-    unsigned* state;                      // words that start at zero: [0..1] depth range, [2..4] finished blocks of the counting passes
+    unsigned* state;                      // words that start at zero: [0..1] depth range, [2..4] finished blocks of the counting passes, [8..9] instances
     void* sort_ws;                        // directly behind `state`: cleared together
     size_t total;
 };
@@ -3718,7 +3706,6 @@ PointBlob carve_point_blob(void* p, int64_t n, int mode) {
     b.foot = mode == INPC_MODE_GAUSSIAN ? c.take<uint4>(n) : nullptr;
     b.block_visible = c.take<unsigned>(nb);
     b.group_visible = c.take<unsigned>(ceil_div<int64_t>(nb, 4));
-    b.group_instances = c.take<unsigned long long>(ceil_div<int64_t>(nb, 4));
     b.counters = c.take<unsigned long long>(4);
     b.depth_min = c.take<unsigned>(1);
     b.depth_max = c.take<unsigned>(1);
@@ -3993,13 +3980,19 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         {
             StageScope scope(STAGE_PREPROCESS, stream);
             // (non-deferred: the number of key bits is not known yet, the sort clears its own state)
+            clear.add(pb.group_visible, sizeof(unsigned) * (size_t)ceil_div<int64_t>(nb, 4));
             clear.add(pb.state, (size_t)(static_cast<char*>(pb.sort_ws) - reinterpret_cast<char*>(pb.state)) + (deferred ? sort_zero_bytes(n, n, key_bits) : 0));
             rc = launch_clear(clear, stream);
             if (rc != INPC_OK) return rc;
-            const int64_t groups = ceil_div<int64_t>(nb, 4), group_cap = (int64_t)sm_count() * 4;
-            visibility_count_kernel<MODE, VARIANT><<<(unsigned)(groups < group_cap ? groups : group_cap), kPreThreads, 0, stream>>>(
-                ps, rp, (unsigned)groups, pb.block_visible, pb.group_visible, pb.group_instances, deferred ? nullptr : pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min,
-                pb.depth_max, pb.counters);
+            const int64_t count_blocks = ceil_div<int64_t>(nb, kPreThreads / 32), count_cap = (int64_t)sm_count() * 4;
+            const unsigned count_grid = (unsigned)(count_blocks < count_cap ? count_blocks : count_cap);
+            unsigned long long* instances = reinterpret_cast<unsigned long long*>(pb.state + 8);
+            if (deferred)
+                visibility_count_kernel<MODE, VARIANT, false><<<count_grid, kPreThreads, 0, stream>>>(
+                    ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, instances, nullptr, pb.state + 2, lo_bits, hi_bits, pb.depth_min, pb.depth_max, pb.counters);
+            else
+                visibility_count_kernel<MODE, VARIANT, true><<<count_grid, kPreThreads, 0, stream>>>(
+                    ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, instances, pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min, pb.depth_max, pb.counters);
             INPC_LAUNCH_CHECK("visibility_count_kernel");
             if (!deferred) {
                 INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
