@@ -197,7 +197,10 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
         {
             const unsigned first = tile * kTile + local;
             const uint32_t* vp = vals_in + first;
-            if (full) {
+            if (!vals_in) {   // the values are the positions
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) val[i] = first + i * 32u;
+            } else if (full) {
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) val[i] = __ldg(vp + i * 32);
             } else {
@@ -328,7 +331,7 @@ SortWorkspace carve_sort_workspace(void* ws, int64_t n, int items) {
 
 struct PassArgs {
     int64_t tiles;         // upper bound
-    const uint32_t *kin, *vin;
+    const uint32_t *kin, *vin;   // vin may be null: the values are the positions 0, 1, ...
     uint32_t *kout, *vout;
     int64_t n;
     const unsigned long long* n_dev;
@@ -406,7 +409,7 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 // `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
                            int items, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
-                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr) {
+                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
 
@@ -435,7 +438,7 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
     PassArgs a;
     a.tiles = tiles; a.n = n; a.n_dev = n_dev; a.status = status;
     a.spin_limit = spin_limit; a.mute_tile = mute_tile;
-    a.kin = keys; a.kout = keys_alt; a.vin = values; a.vout = values_alt;
+    a.kin = keys; a.kout = keys_alt; a.vin = position_values ? nullptr : values; a.vout = values_alt;
     a.state = w.state;
     for (int p = 0; p < pt.n_passes; ++p) {
         a.shift = pt.shift[p]; a.bits = pt.bits[p];
@@ -445,20 +448,23 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
         if (rc != INPC_OK) return rc;
         a.state += (size_t)tiles * pass_bins(a.bits);
         const uint32_t* t = a.kin; a.kin = a.kout; a.kout = const_cast<uint32_t*>(t);
-        t = a.vin; a.vin = a.vout; a.vout = const_cast<uint32_t*>(t);
+        a.vin = a.vout; a.vout = a.vout == values ? values_alt : values;
     }
     if (result_in_alt) *result_in_alt = pt.n_passes & 1;
     return INPC_OK;
 }
 
+// `position_values`: the values to be sorted are 0 .. n - 1 and need not lie in `values` (with fewer than two pairs, where nothing
+// is done, they do).
 int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
-               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream) {
+               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, bool position_values) {
     if (result_in_alt) *result_in_alt = 0;
     bool nothing = false;
     const int rc = check_sort_args("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, &nothing);
     if (rc != INPC_OK || nothing) return rc;
     if (!workspace) { set_error("sort_pairs: null workspace"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n_likely), workspace, zeroed, status, result_in_alt, stream);
+    return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n_likely), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
+                           0xFFFFFFFFu, nullptr, position_values);
 }
 
 // The same sort with the number of pairs in device memory (*n_dev <= n_max): grids and the look-back state are

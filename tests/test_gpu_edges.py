@@ -151,3 +151,21 @@ def test_gaussian_blend_at_the_edges_of_its_segments(n):
     assert_close(bw.cpu().numpy(), st.blending_weights, rtol=4e-4 + eps, atol=1e-9, max_bad=few, what="blending weights")
     assert_close(f.grad.float().cpu().numpy(), np.asarray(gf, np.float32), rtol=4e-3 + eps, atol=2e-7, max_bad=36 * few, what="grad_features")
     assert_close(o.grad.cpu().numpy(), go, rtol=2e-3 + eps, atol=4e-8 + 1e-3 * eps, max_bad=few, what="grad_opacities")
+
+
+# four points per thread and 16-byte loads where the positions are aligned; one block gathers 256 points
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 255, 257, 1023, 1025, 300_001])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_morton_order_at_block_edges_and_offsets(n, offset):
+    from inpc_b200.sampling import morton_order
+    g = torch.Generator().manual_seed(n)
+    pos = (torch.rand((n + offset, 3), generator=g) * torch.tensor([2.0, 1.0, 3.0]) - 1.0)[offset:]     # offset 1: rows start 12 bytes on
+    lo = pos.min(dim=0).values
+    extent = float((pos.max(dim=0).values - lo).max())
+    inv = np.float32(1.0) / np.float32(np.float64(extent) * (1.0 + 1e-6)) if extent > 0 else np.float32(1.0)
+    q = ((pos - lo) * torch.tensor(inv) * 1024.0).clamp(0.0, 1023.0).to(torch.int64)
+    code = sum((((q[:, c] >> b) & 1) << (3 * b + c)) for b in range(10) for c in range(3))
+    store = torch.empty((n + offset, 3), device=DEV)
+    src = store[offset:]
+    src.copy_(pos)
+    assert torch.equal(morton_order(src).cpu(), pos[torch.sort(code, stable=True).indices])
