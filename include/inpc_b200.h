@@ -216,7 +216,8 @@ int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc_view* view
 
 /* Stable least-significant-digit radix sort of (u32 key, u32 value) pairs on bits [0, end_bit),
  * the library's own onesweep.  keys_alt / values_alt are same-sized ping-pong buffers; `workspace`
- * needs inpc_sort_workspace_bytes(n).  *result_in_alt tells which pair holds the result.
+ * needs inpc_sort_workspace_bytes(n), which never falls as n grows: one sized for the largest n serves
+ * every smaller one.  *result_in_alt tells which pair holds the result.
  * Replaces the two cub::DeviceRadixSort::SortPairs calls of
  * rasterization/src/bilinear/forward.cu:91-98 and :132-139. */
 size_t inpc_sort_workspace_bytes(int64_t n);

@@ -385,7 +385,14 @@ size_t sort_zero_bytes(int64_t n, int64_t n_likely, int end_bit) {
     return carve_sort_workspace(nullptr, n, items).zero_bytes + state_words(ceil_div<int64_t>(n, (int64_t)kThreads * items), end_bit) * sizeof(unsigned);
 }
 
-size_t sort_workspace_bytes(int64_t n, int64_t n_likely) { return carve_sort_workspace(nullptr, n, tile_items(n_likely)).total; }
+// A workspace serves every smaller sort as well.  The look-back state of kSmallMax pairs in small tiles is larger than that of
+// up to four times as many in large ones (1.07 MB against 0.29 MB just above), so from there on the size does not fall below it.
+size_t sort_workspace_bytes(int64_t n, int64_t n_likely) {
+    const size_t own = carve_sort_workspace(nullptr, n, tile_items(n_likely)).total;
+    if (tile_items(n_likely) == kSmallItems) return own;
+    const size_t small = carve_sort_workspace(nullptr, kSmallMax, kSmallItems).total;
+    return own > small ? own : small;
+}
 
 int sort_pass_count(int end_bit) { return end_bit > 0 ? ceil_div(end_bit, kRadixBits) : 0; }
 

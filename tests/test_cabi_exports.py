@@ -47,6 +47,22 @@ def test_every_declaration_cites_the_reference():
             "inpc_version", "inpc_launch_count", "inpc_sampler_get_counter", "inpc_sampler_workspace_bytes"), name
 
 
+@pytest.mark.parametrize("name", ["inpc_sort_workspace_bytes", "inpc_morton_workspace_bytes", "inpc_sampler_workspace_bytes"])
+def test_a_workspace_for_more_serves_fewer(name):
+    """A caller sizes one workspace for its largest n: the size must not fall as n grows, in particular not where the sort
+    goes over to larger tiles (2^18 pairs)."""
+    from inpc_b200 import _cabi
+    size = getattr(_cabi.lib(), name)
+    edge = 1 << 18
+    ns = sorted({1, 2, 100, 2047, 2048, 2049, 8192, 100_003, 200_000, edge - 2049, edge - 1, edge, edge + 1, edge + 8192, 300_000, 500_000,
+                 3 * edge, 4 * edge - 1, 4 * edge, 4 * edge + 1, 5 * edge, 1 << 22, 1 << 23} | {edge + 2048 * k for k in range(-8, 40)})
+    if name == "inpc_sampler_workspace_bytes":
+        ns = [n for n in ns if n <= 1 << 22]
+    sizes = [int(size(n)) for n in ns]
+    fell = [(a, b) for (a, x), (b, y) in zip(zip(ns, sizes), zip(ns[1:], sizes[1:])) if y < x]
+    assert not fell, f"{name} falls between {fell}"
+
+
 def test_host_side_validation_without_gpu():
     from inpc_b200 import _cabi
     L = _cabi.lib()

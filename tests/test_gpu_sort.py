@@ -56,6 +56,24 @@ def test_sort_skewed_and_constant_keys():
     _check(depth_like, 32)
 
 
+@pytest.mark.parametrize("n_ws,n", [(300_000, 200_000), ((1 << 18) + 1, 1 << 18), (1 << 20, 1 << 18), (1 << 20, 100_003)])
+def test_sort_in_a_workspace_sized_for_more(n_ws, n):
+    """A workspace sized for a larger n holds a smaller sort: the bytes behind it stay as they are."""
+    from inpc_b200 import _cabi
+    L = _cabi.lib()
+    size, guard = int(L.inpc_sort_workspace_bytes(n_ws)), 2 << 20      # the guard holds whatever a sort of 2^18 pairs can need
+    ws = torch.full((size + guard,), 0xA5, dtype=torch.uint8, device=DEV)
+    g = torch.Generator(device=DEV).manual_seed(n)
+    keys64 = torch.randint(0, 1 << 27, (n,), generator=g, device=DEV, dtype=torch.int64)
+    k, v = keys64.to(torch.int32), torch.arange(n, device=DEV, dtype=torch.int32)
+    ka, va = torch.empty_like(k), torch.empty_like(v)
+    alt = C.c_int(0)
+    _cabi.check(L.inpc_sort_pairs(k.data_ptr(), ka.data_ptr(), v.data_ptr(), va.data_ptr(), n, 27, ws.data_ptr(), C.byref(alt),
+                                  torch.cuda.current_stream().cuda_stream))
+    assert torch.equal((va if alt.value else v).to(torch.int64), torch.sort(keys64, stable=True).indices)
+    assert bool((ws[size:] == 0xA5).all())
+
+
 def test_sort_full_size_depth_keys():
     """The bench's size: 2^23 pairs with 27 significant bits (three passes), keys larger than L2."""
     g = torch.Generator(device=DEV).manual_seed(23)
