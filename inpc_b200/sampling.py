@@ -66,7 +66,8 @@ def compute_viewpoint_weights(centers: torch.Tensor, levels: torch.Tensor, weigh
 
 
 def _max_viewpoint_weights(centers: torch.Tensor, levels: torch.Tensor, weights: torch.Tensor, views, initial_size: float) -> torch.Tensor:
-    """Maximum over `views` of `compute_viewpoint_weights`."""
+    """Maximum over `views` (any iterable) of `compute_viewpoint_weights`."""
+    views = list(views)     # walked twice: a generator would be empty the second time
     for view in views:
         _check_view(view)
     dev = centers.device

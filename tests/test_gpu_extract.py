@@ -102,3 +102,35 @@ def test_extract_global_end_to_end():
                            use_morton_order=False)
     key = lambda p: p[:, 0].double() * 1e6 + p[:, 1].double() * 1e3 + p[:, 2].double()
     assert torch.equal(torch.sort(key(pts)).values, torch.sort(key(plain)).values)
+
+
+def test_extract_global_takes_any_iterable_of_views():
+    import inpc_b200
+    import synthetic_workloads as syn
+    from inpc_b200.sampling import extract_global
+    tree = syn.uniform_octree(4, seed=0).to(DEV)
+    views = [v.to(DEV) for v in syn.orbit_views(3, seed=2, width=160, height=120, focal=140.0)]
+
+    def cloud(v):
+        return extract_global(inpc_b200.ProbabilityFieldSampler(1), tree.centers, tree.levels, tree.weights, v, 20_000, tree.initial_size)
+    want = cloud(views)
+    assert torch.equal(cloud(v for v in views), want)
+    assert torch.equal(cloud(tuple(views)), want)
+    with pytest.raises(Exception):
+        cloud(iter([]))          # an iterable without views leaves no leaf with a weight
+
+
+# a launch takes up to 32 views; the second one starts from what the first has left
+@pytest.mark.parametrize("n_views", [1, 31, 32, 33, 64, 65])
+def test_max_viewpoint_weights_over_several_launches(n_views):
+    import synthetic_workloads as syn
+    from inpc_b200.sampling import _max_viewpoint_weights, compute_viewpoint_weights
+    tree = syn.uniform_octree(4, seed=0).to(DEV)
+    n = 3001                                        # not a multiple of the block
+    centers, levels, weights = tree.centers[:n].contiguous(), tree.levels[:n].contiguous(), tree.weights[:n].contiguous()
+    # narrow views: most leaves are seen by a few of them only, some by none
+    views = [v.to(DEV) for v in syn.orbit_views(n_views, seed=5, width=64, height=48, focal=400.0)]
+    each = torch.stack([compute_viewpoint_weights(centers, levels, weights, v, tree.initial_size) for v in views])
+    assert torch.equal(_max_viewpoint_weights(centers, levels, weights, views, tree.initial_size), each.amax(dim=0))
+    if n_views > 32:
+        assert bool((each[32:].amax(dim=0) > each[:32].amax(dim=0)).any()) and bool((each[:32].amax(dim=0) > each[32:].amax(dim=0)).any())
