@@ -306,8 +306,9 @@ int inpc_generate_samples(inpc_sampler* s, const inpc_view* view, int64_t n_cell
 
 /* Expected-count samples in two steps so the caller can size the output.  _count reads one integer
  * back: *n_created = sum over visible leaves of max(1, round(w/sum*n_samples)), 0 if sum <= 0.
- * _fill writes n_created*n_multi positions of the leaves given to _count (it reads them from the workspace).  Replaces compute_sample_distribution +
- * create_expected_samples (sampling/include/sampling.h:68-83). */
+ * _fill writes n_created*n_multi positions inside the cells it is given, as many per cell as _count left in
+ * the workspace.  Replaces compute_sample_distribution + create_expected_samples
+ * (sampling/include/sampling.h:68-83). */
 int inpc_generate_expected_samples_count(inpc_sampler* s, const inpc_view* view, int64_t n_cells,
                                          const float* centers, const int32_t* levels,
                                          const float* weights, float initial_size, int64_t n_samples,

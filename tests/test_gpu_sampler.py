@@ -108,6 +108,31 @@ def test_zero_weight_sum_behaviour():
         s.generate_samples(t.centers, t.levels, t.weights, v, 10, tree.initial_size)
 
 
+def test_expected_samples_fill_uses_the_cells_it_is_given():
+    """The counts come from the counting call, the cells from the filling one: a caller may fill other cells (moved, resized)."""
+    import ctypes as C
+
+    from inpc_b200 import ProbabilityFieldSampler, _cabi
+    from inpc_b200.sampling import _ViewArg
+    tree, view = _scene()
+    t, v = tree.to(DEV), view.to(DEV)
+    n, L, s = t.weights.numel(), _cabi.lib(), ProbabilityFieldSampler(99)
+    stream = torch.cuda.current_stream().cuda_stream
+    ws = torch.empty(int(L.inpc_sampler_workspace_bytes(n)), dtype=torch.uint8, device=DEV)
+    arg, created = _ViewArg(v, torch.device(DEV)), C.c_int64(0)
+    _cabi.check(L.inpc_generate_expected_samples_count(s._handle, C.byref(arg.c), n, t.centers.data_ptr(), t.levels.data_ptr(), t.weights.data_ptr(),
+                                                       float(tree.initial_size), 40000, C.byref(created), ws.data_ptr(), stream))
+    ovw = O.viewpoint_weights(oracle_camera(view), *_np(tree), tree.initial_size)
+    counts, n_created = O.expected_counts(ovw, O.build_cdf(ovw)[1], 40000)
+    assert created.value == n_created
+    centers, levels, size = (t.centers * 0.75 + 0.125).contiguous(), (t.levels + 1).contiguous(), 1.5 * tree.initial_size
+    out = torch.empty((2 * n_created, 3), device=DEV)
+    counter = int(L.inpc_sampler_get_counter(s._handle))
+    _cabi.check(L.inpc_generate_expected_samples_fill(s._handle, n, centers.data_ptr(), levels.data_ptr(), float(size), n_created, 2, out.data_ptr(),
+                                                      ws.data_ptr(), stream))
+    want = O.expected_samples(99, counter, counts, centers.cpu().numpy(), levels.cpu().numpy(), size, 2)
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
+
 def test_draw_leaves_edge_cases_on_device():
     from inpc_b200 import sampling as S
     cdf = torch.tensor([0.0, 0.0, 0.25, 0.25, 0.25, 0.75, 1.0], device=DEV)
