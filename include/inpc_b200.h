@@ -105,7 +105,7 @@ int inpc_call_status(long long ticket, unsigned* words);
  * tile_size is 8 (the reference's tiling; tile ranges comparable with it) or 16.
  * Bilinear mode with 8x8 tiles makes no host synchronisation at all: a splat touches at most 2x2 tiles, so the
  * instance scratch is sized for 4 n instances, the kernels read the two counts from device memory, and
- * state->n_visible / n_instances stay -1 until inpc_raster_resolve is called.  The other combinations read
+ * state->n_visible / n_instances stay -1 until inpc_raster_resolve is called (n >= 2^28 excepted).  The other combinations read
  * the two counters back once to size the instance scratch (the reference does so twice, with blocking copies:
  * rasterization/src/bilinear/forward.cu:86-89).
  * Replaces inpc::rasterization::{bilinear,gaussian}::forward
@@ -171,7 +171,8 @@ int inpc_render_preextracted(int mode, int tile_size, const inpc_view* view, int
 /* Feature-row layout (bilinear splats): every point carries `channels` fp32 values (4, 8, 16 or 32;
  * features (n, channels), 16-byte aligned) that are blended as they are, without spherical
  * harmonics, into image (channels,H,W).  alpha (H,W), blending_weights (n), the scratch callbacks
- * and `state` are as in inpc_rasterize_forward.
+ * and `state` are as in inpc_rasterize_forward; the two counters are read back once for either tile size, so the
+ * instance scratch has the size the scene needs and state->n_visible / n_instances are final on return.
  * No counterpart in the reference, whose backend only blends the four channels it evaluates from 36
  * SH halves (rasterization/src/rasterization_api.cu:23-107): the ordering is that of
  * rasterization/src/bilinear/forward.cu:59-170 and the per-fragment arithmetic that of

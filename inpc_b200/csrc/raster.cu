@@ -3759,14 +3759,20 @@ int64_t max_segments(int64_t n_instances, int n_tiles, int tile) {
 // (8x8 tiles) or one block per (tile, segment).
 constexpr int kWarpBlendParts = 2;   // work items per (tile, segment): the two 8x4 halves
 bool uses_warp_blend(int tile) { return tile == 8; }
-// Bilinear splats touch at most 2x2 tiles: with the warp blend nothing waits for their counts.
+// Bilinear splats touch at most 2x2 tiles.
 bool has_instance_bound(int mode, int tile) { return mode == INPC_MODE_BILINEAR && uses_warp_blend(tile); }
+
+// Whether a call sizes everything for that bound and leaves its counts on the device.  Feature rows do not: the bound takes three times
+// the instance scratch the counts ask for (64 bytes per point against about 20), and with C / 4 times the segment colours that is
+// memory a scene of wide rows has better use for; the counts are also part of what their forward returns.
+bool defers_counts(int mode, int tile, bool rows, int64_t n) { return has_instance_bound(mode, tile) && !rows && n > 0 && n < ((int64_t)1 << 28); }
 
 // The bounded path sizes its arrays for 4 instances per point; most splats touch one tile of four or none twice, about 1.3
 // on average (2^23 samples at 1237x822: 1.26; at 3840x2160 less).  Only picks tile sizes.
-int64_t likely_instances(int64_t capacity, int mode, int tile) { return has_instance_bound(mode, tile) ? capacity / 3 : capacity; }
+int64_t likely_instances(int64_t capacity, bool deferred) { return deferred ? capacity / 3 : capacity; }
 
-InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int tile, int mode, bool with_depth, int c4 = 1) {
+// `deferred`: n_instances is the bound, not a count.
+InstanceBlob carve_instance_blob(void* p, int64_t n_instances, bool deferred, int n_tiles, int tile, int mode, bool with_depth, int c4 = 1) {
     InstanceBlob b;
     Carver c(p);
     const bool warp_blend = uses_warp_blend(tile);
@@ -3777,7 +3783,7 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, int n_tiles, int 
     b.ranges = c.take<uint2>(n_tiles);
     c.off = align_up(c.off);
     b.sort_ws = c.base + c.off;
-    c.off += sort_workspace_bytes(n_instances, likely_instances(n_instances, mode, tile));
+    c.off += sort_workspace_bytes(n_instances, likely_instances(n_instances, deferred));
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n_instances);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n_instances);
     // upper bound on the number of (tile, segment) pairs, known from the instance count alone
@@ -3930,8 +3936,8 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     // Bilinear splats touch at most 2x2 tiles, so the warp-blend path sizes everything behind the visibility pass
     // for 4 n instances and lets the kernels read the two counts from device memory: no host synchronisation at
     // all (the reference reads both counts back with blocking copies, src/bilinear/forward.cu:86-89).  The other
-    // paths (gaussian splats have no such bound) read the counts back once.
-    const bool deferred = has_instance_bound(MODE, rp.tile) && n > 0 && n < ((int64_t)1 << 28);
+    // paths (gaussian splats have no such bound, feature rows keep their scratch small) read the counts back once.
+    const bool deferred = defers_counts(MODE, rp.tile, VARIANT == VAR_ROWS, n);
     int64_t n_visible = 0, n_instances = 0;
     uint32_t key_base = 0;
     int key_bits = 0;
@@ -3939,15 +3945,15 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     void* iblob = nullptr;
     InstanceBlob ib;
     auto make_instance_blob = [&]() -> int {
-        const InstanceBlob isz = carve_instance_blob(nullptr, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
+        const InstanceBlob isz = carve_instance_blob(nullptr, n_instances, deferred, n_tiles, rp.tile, MODE, with_depth, c4);
         iblob = alloc_instance(user, isz.total);
         if (!iblob) { set_error("instance allocator returned NULL for %zu bytes", isz.total); return INPC_E_ALLOC; }
-        ib = carve_instance_blob(iblob, n_instances, n_tiles, rp.tile, MODE, with_depth, c4);
+        ib = carve_instance_blob(iblob, n_instances, deferred, n_tiles, rp.tile, MODE, with_depth, c4);
         return INPC_OK;
     };
     auto clear_instance_blob = [&](ClearList& list) {
         list.add(ib.n_segments, (size_t)(static_cast<char*>(ib.sort_ws) - reinterpret_cast<char*>(ib.n_segments)) +
-                                    sort_zero_bytes(n_instances, likely_instances(n_instances, MODE, rp.tile), tile_bits));
+                                    sort_zero_bytes(n_instances, likely_instances(n_instances, deferred), tile_bits));
     };
     int rc;
     const unsigned long long* n_visible_dev = deferred ? pb.counters : nullptr;
@@ -4067,8 +4073,8 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
-        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, MODE, rp.tile), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream)
-                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, MODE, rp.tile), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
+        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream)
+                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
         if (rc != INPC_OK) return rc;
         const int64_t range_blocks = ceil_div<int64_t>(n_instances, 256 * 8), range_cap = (int64_t)sm_count() * 8;
         tile_ranges_kernel<<<(unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream>>>(ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
@@ -4495,7 +4501,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     const RasterParams rp = make_params(view, state->tile_size, 0.0f, 3.0f, nullptr);
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode);
-    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), n_tiles, state->tile_size, state->mode, false);
+    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false);
     const uint32_t* ids = ib.ids[tile_buffer_of(state, n_tiles)];
     float4* gfv = reinterpret_cast<float4*>(grad_features_view);
     const int W = rp.v.width, H = rp.v.height;
@@ -4707,7 +4713,7 @@ extern "C" int inpc_rasterize_rows_backward(const inpc_raster_state* state, cons
     const RasterParams rp = make_params(view, state->tile_size, 0.0f, 3.0f, nullptr);
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode);
-    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), n_tiles, state->tile_size, state->mode, false, channels / 4);
+    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false, channels / 4);
     const int t_alt = tile_buffer_of(state, n_tiles);
     ClearList clear;
     clear.add(grad_features, sizeof(float) * (size_t)n * channels);
@@ -4782,7 +4788,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
     const int n_tiles = gw * gh;
     const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode);
     if (state->n_visible < 0 || state->n_instances < 0) { set_error("inpc_raster_debug_copy: the counts of this state are still on the device; call inpc_raster_resolve first"); return INPC_E_INVALID; }
-    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), n_tiles, state->tile_size, state->mode, false);
+    const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false);
     const int d = depth_buffer_of(state);
     const int ti = tile_buffer_of(state, n_tiles);
     switch (which) {

@@ -148,6 +148,33 @@ def test_rows_match_reference_backend_run_per_channel_group():
     assert_close(o.grad.reshape(-1).cpu().numpy(), go_ref.cpu().numpy(), rtol=1e-4, atol=1e-9, max_bad=3, what="rows grad_opacities vs reference")
 
 
+@pytest.mark.parametrize("tile", [8, 16])
+def test_rows_forward_returns_its_counts_and_holds_no_more_than_they_need(tile):
+    """The counts of the state are final when the forward returns, and the instance scratch follows them."""
+    import ctypes as C
+
+    from inpc_b200 import _cabi
+    from inpc_b200 import rasterization as R
+    n, channels = 300_000, 32
+    view, pos, _, opac = small_scene(n=n, width=136, height=104, focal=120.0)
+    settings = R.INPCRasterizer.extract_settings(view.to(DEV), 0)
+    feats, p, o = _rows(n, channels, 47).to(DEV), pos.to(DEV), opac.to(DEV)
+    _, _, _, want, _, _ = R.forward_with_state(p, torch.zeros((n, 36), dtype=torch.float16, device=DEV), o, settings, tile)
+    image, alpha, bw = (torch.empty(k, device=DEV) for k in (channels * 136 * 104, 136 * 104, n))
+    arg, blobs, state = R._ViewArg(settings, torch.device(DEV)), R._Blobs(torch.device(DEV)), _cabi.RasterState()
+    R._check(_cabi.lib().inpc_rasterize_rows_forward(tile, C.byref(arg.c), n, p.data_ptr(), feats.data_ptr(), channels, o.data_ptr(), image.data_ptr(),
+                                                     alpha.data_ptr(), bw.data_ptr(), blobs.cb_point, blobs.cb_instance, None, C.byref(state),
+                                                     torch.cuda.current_stream().cuda_stream), blobs)
+    assert (state.n_visible, state.n_instances) == (want.n_visible, want.n_instances) and state.n_visible > 0
+    assert not state.deferred_counts & 1
+    R.resolve_counts(state)                        # a no-op
+    assert state.n_instances == want.n_instances
+    # 16 bytes per instance, up to 4 of look-back state, and per (tile, segment) 64 or 256 pixels of transmittance and colours
+    tiles, per_px = -(-136 // tile) * -(-104 // tile), 4 + 4 * channels
+    segments = 2 * tiles + 2560 + state.n_instances // 1024 + 1 if tile == 8 else tiles + state.n_instances // 256 + 1
+    assert blobs.instance.numel() <= 20 * state.n_instances + segments * tile * tile * per_px + (4 << 20)
+
+
 def test_rows_empty_culled_and_bad_arguments():
     import inpc_b200
     view, pos, _, opac = small_scene(n=64, width=40, height=24, focal=30.0)
