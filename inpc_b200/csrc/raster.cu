@@ -3677,9 +3677,9 @@ __global__ void __launch_bounds__(kPreThreads, 8) preprocess_backward_kernel(
 struct PointBlob {
     PointRec* rec;
     uint2* bounds;
-    uint32_t* quad;                       // warp blend: packed footprint origin per point (see pack_quad)
+    uint32_t* quad;                       // bilinear, warp blend: packed footprint origin per point (see pack_quad)
     float4* conic;
-    uint4* foot;                          // gaussian: tile bounds and ellipse per point (see pack_footprint)
+    uint4* foot;                          // gaussian, warp blend: tile bounds and ellipse per point (see pack_footprint)
     unsigned* block_visible;              // survivors per chunk of kPreThreads points
     unsigned* group_visible;              // per group of 4 chunks; scanned in place
     unsigned long long* counters;   // visible, instances, smallest / largest depth bit pattern
@@ -3693,17 +3693,21 @@ struct PointBlob {
     size_t total;
 };
 
-// Sized by the number of input points alone (every per-visible array gets room for all of them), so
+// Which of the two blend organisations a call uses: one warp per tile part with the dead-instance filter
+// (8x8 tiles) or one block per (tile, segment).
+bool uses_warp_blend(int tile) { return tile == 8; }
+
+// Sized by the number of input points (every per-visible array gets room for all of them), so
 // that the layout is known before the visible count has been read back.
-PointBlob carve_point_blob(void* p, int64_t n, int mode) {
+PointBlob carve_point_blob(void* p, int64_t n, int mode, int tile) {
     PointBlob b;
     Carver c(p);
     const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
     b.rec = c.take<PointRec>(n);
     b.bounds = c.take<uint2>(n);
-    b.quad = mode == INPC_MODE_BILINEAR ? c.take<uint32_t>(n) : nullptr;
+    b.quad = mode == INPC_MODE_BILINEAR && uses_warp_blend(tile) ? c.take<uint32_t>(n) : nullptr;
     b.conic = mode == INPC_MODE_GAUSSIAN ? c.take<float4>(n) : nullptr;
-    b.foot = mode == INPC_MODE_GAUSSIAN ? c.take<uint4>(n) : nullptr;
+    b.foot = mode == INPC_MODE_GAUSSIAN && uses_warp_blend(tile) ? c.take<uint4>(n) : nullptr;
     b.block_visible = c.take<unsigned>(nb);
     b.group_visible = c.take<unsigned>(ceil_div<int64_t>(nb, 4));
     b.counters = c.take<unsigned long long>(4);
@@ -3755,10 +3759,7 @@ int64_t max_segments(int64_t n_instances, int n_tiles, int tile) {
     return (int64_t)n_tiles + ceil_div<int64_t>(n_instances, (int64_t)blend_batch(tile) * kMinBatchesPerSegment);
 }
 
-// Which of the two blend organisations a call uses: one warp per tile part with the dead-instance filter
-// (8x8 tiles) or one block per (tile, segment).
-constexpr int kWarpBlendParts = 2;   // work items per (tile, segment): the two 8x4 halves
-bool uses_warp_blend(int tile) { return tile == 8; }
+constexpr int kWarpBlendParts = 2;   // work items of the warp blend per (tile, segment): the two 8x4 halves
 // Bilinear splats touch at most 2x2 tiles.
 bool has_instance_bound(int mode, int tile) { return mode == INPC_MODE_BILINEAR && uses_warp_blend(tile); }
 
@@ -3924,10 +3925,10 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     if (!status) return INPC_E_CUDA;
     const bool warp_blend = uses_warp_blend(rp.tile);
     const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
-    const PointBlob sizing = carve_point_blob(nullptr, n, MODE);
+    const PointBlob sizing = carve_point_blob(nullptr, n, MODE, rp.tile);
     void* pblob = alloc_point(user, sizing.total);
     if (!pblob) { set_error("point allocator returned NULL for %zu bytes", sizing.total); return INPC_E_ALLOC; }
-    const PointBlob pb = carve_point_blob(pblob, n, MODE);
+    const PointBlob pb = carve_point_blob(pblob, n, MODE, rp.tile);
     {
         const int rc_check = begin_index_checks(n, stream);
         if (rc_check != INPC_OK) return rc_check;
@@ -4007,8 +4008,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             // the projection pass needs nothing from the host: it runs while the host waits for the counters
             preprocess_kernel<MODE, VARIANT><<<(unsigned)nb, kPreThreads, 0, stream>>>(
                 ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max,
-                pb.rec, pb.bounds, MODE == INPC_MODE_BILINEAR && warp_blend ? pb.quad : nullptr,
-                pb.conic, warp_blend ? pb.foot : nullptr, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
+                pb.rec, pb.bounds, pb.quad, pb.conic, pb.foot, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
             INPC_LAUNCH_CHECK("preprocess_kernel");
         }
         if (!deferred) {
@@ -4500,7 +4500,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     if (rc != INPC_OK) return rc;
     const RasterParams rp = make_params(view, state->tile_size, 0.0f, 3.0f, nullptr);
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
-    const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode);
+    const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode, state->tile_size);
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false);
     const uint32_t* ids = ib.ids[tile_buffer_of(state, n_tiles)];
     float4* gfv = reinterpret_cast<float4*>(grad_features_view);
@@ -4712,7 +4712,7 @@ extern "C" int inpc_rasterize_rows_backward(const inpc_raster_state* state, cons
     if (n == 0) return INPC_OK;
     const RasterParams rp = make_params(view, state->tile_size, 0.0f, 3.0f, nullptr);
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
-    const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode);
+    const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode, state->tile_size);
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false, channels / 4);
     const int t_alt = tile_buffer_of(state, n_tiles);
     ClearList clear;
@@ -4740,7 +4740,7 @@ extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
     if (!state) { set_error("inpc_raster_resolve: null state"); return INPC_E_INVALID; }
     if (!(state->deferred_counts & 1) || state->n_points == 0) return INPC_OK;
     if (!state->point_blob) { set_error("inpc_raster_resolve: state without a point blob"); return INPC_E_INVALID; }
-    const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode);
+    const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode, state->tile_size);
     unsigned long long host[4];
     INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, sizeof(host), cudaMemcpyDeviceToHost, stream));
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
@@ -4786,7 +4786,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
     if (!state || !view || !dst) { set_error("inpc_raster_debug_copy: null argument"); return INPC_E_INVALID; }
     const int gw = ceil_div(view->width, state->tile_size), gh = ceil_div(view->height, state->tile_size);
     const int n_tiles = gw * gh;
-    const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode);
+    const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode, state->tile_size);
     if (state->n_visible < 0 || state->n_instances < 0) { set_error("inpc_raster_debug_copy: the counts of this state are still on the device; call inpc_raster_resolve first"); return INPC_E_INVALID; }
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false);
     const int d = depth_buffer_of(state);

@@ -459,3 +459,14 @@ def test_gaussian_deep_tiles_training_and_inference(tile):
     assert_close(img.cpu().numpy(), oi, rtol=2e-4, atol=2e-5, max_bad=12, what="gaussian deep inference image")
     assert_close(dep.cpu().numpy(), od, rtol=2e-4, atol=2e-5, max_bad=12, what="gaussian deep inference depth")
     assert_close(alp.cpu().numpy(), oa, rtol=2e-4, atol=2e-5, max_bad=12, what="gaussian deep inference alpha")
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_point_scratch_holds_what_its_tile_size_uses(mode):
+    """The records of the 8x8-tile instance emission (4 bytes per bilinear point, 16 per gaussian) take no room with 16x16 tiles."""
+    from inpc_b200 import rasterization as R
+    n = 20000
+    view, pos, feats, opac = small_scene(n=n)
+    settings = R.INPCRasterizer.extract_settings(view.to(DEV), mode)
+    size = {tile: R.forward_with_state(pos.to(DEV), feats.to(DEV), opac.to(DEV), settings, tile)[4].point.numel() for tile in (8, 16)}
+    assert size[8] - size[16] >= (4, 16)[mode] * n
