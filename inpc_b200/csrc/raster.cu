@@ -1380,6 +1380,13 @@ __device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_i
     s.first = max(kSegmentMin, min(limits.first_max, s.later / 2u));
     return s;
 }
+// How far past its stop a pixel must be before pass PRODUCT closes it, relative (or in units of log2, where the same number
+// is wider).  REST multiplies up to `len` factors into a transmittance of its own, each product rounded by at most 2^-24 and, for
+// faint splats, mostly in one direction; PRODUCT's chain of products does the same from another start (gaussian), its sum of
+// logarithms is off by at most 2^-25 a term and 2^-23 of the 13.3 it can reach (bilinear): together less than len 2^-23.  A
+// pixel closed too early loses the fragments behind it, a ten-thousandth of the image's range.
+__device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f, (float)(len + 8u) * 1.1920928955078125e-07f); }
+
 constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
 
@@ -1636,10 +1643,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
             // the state segment 0 left: a pixel that has stopped there stays stopped; for the others the
             // product is taken until T0 * product falls below the threshold (the true transmittance at
             // that point is smaller still, so everything behind is dead whatever the product says).  The margin
-            // keeps a pixel open when the sum's rounding could be what carries it over the line.
+            // keeps a pixel open when rounding, of this sum or of the products REST forms, could be what carries it over.
             const float T0 = seg_T[sidx0 * 32 + lane];
             done = done || T0 < kTransmittanceEps;
-            log_stop = done ? 0.0 : log2((double)T0 / (double)kTransmittanceEps) + 1e-4;
+            log_stop = done ? 0.0 : log2((double)T0 / (double)kTransmittanceEps) + (double)stop_margin(rg.y - rg.x);
         } else if (PASS == PASS_REST) {
             Tr = seg_T[sidx * 32 + lane];
             done = done || Tr < kTransmittanceEps;
@@ -3251,10 +3258,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_f
         bool done = !inside;
         if (PASS == PASS_PRODUCT) {
             // product of (1 - alpha) over the segment, until it would carry the state segment 0 left below the threshold; the
-            // margin keeps a pixel open when rounding could be what carries it over the line
+            // margin keeps a pixel open when rounding, of this product or of REST's, could be what carries it over the line
             const float T0 = seg_T[sidx0 * 32 + lane];
             done = done || T0 < kTransmittanceEps;
-            if (!done) stop = kTransmittanceEps / T0 * (1.0f - 1e-4f);
+            if (!done) stop = kTransmittanceEps / T0 * (1.0f - stop_margin(rg.y - rg.x));
         } else if (PASS == PASS_REST) {
             Tr = seg_T[sidx * 32 + lane];
             done = done || Tr < kTransmittanceEps;

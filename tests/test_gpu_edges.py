@@ -153,6 +153,54 @@ def test_gaussian_blend_at_the_edges_of_its_segments(n):
     assert_close(o.grad.cpu().numpy(), go, rtol=2e-3 + eps, atol=4e-8 + 1e-3 * eps, max_bad=few, what="grad_opacities")
 
 
+# The pass that cuts the lists of later segments (4096 instances from 5,242,881 on) multiplies in another order than the pass
+# that blends them.  Both round up to 4096 times: a pixel may be closed only when no rounding can have carried it over its stop.
+@pytest.mark.parametrize("mode", [0, 1])
+def test_a_long_segment_of_faint_splats_is_not_cut_before_its_end(mode):
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    f32, eps = np.float32, np.float32(1e-4)
+    width, height, focal, n_bulk, n_tail = 257, 129, 256.0, 5_600_000, 11
+    # every splat of the list sits on the centre of pixel (128, 64) and nothing else does: its alpha is its opacity
+    if mode == 1:       # products from 1 down: just above a half, a step of 2^-24 is rounded up to twice its size
+        faint, head, delta = f32(2.0 ** -24), [f32(0.499)], 3.2e-4
+    else:               # near the stop, a step of 2^-22 is rounded down by 8 %, its logarithm up by 4 % (to 6 / 2^24)
+        faint, head, delta = f32(2.0 ** -22), [], 9.1e-4
+    later = head + [faint] * (4096 - n_tail - len(head)) + [f32(0.9)] * n_tail
+    start = float(np.prod([1.0 - float(a) for a in head]))
+    want = float(eps) * (1 + delta) / start              # transmittance behind the first segment: three splats and 1021 that are clear
+    a1 = f32(1) - f32(want ** (1 / 3))
+    t2 = (f32(1) - a1) * (f32(1) - a1)
+    first = [a1, a1, f32(1) - f32(want / float(t2))] + [f32(0)] * 1021
+
+    def chain(t, alphas):
+        for a in alphas:
+            t = f32(t * (f32(1) - a))
+            yield t
+    t0 = list(chain(f32(1), first))[-1]
+    blended = list(chain(t0, later))
+    if mode == 1:
+        product = np.array([float(t0) * float(t) for t in chain(f32(1), later)])
+    else:
+        product = float(t0) * 2.0 ** -np.cumsum([round(-float(np.log2(f32(1) - a)) * 2 ** 24) / 2 ** 24 for a in later])
+    # the blend is still open behind the faint splats and closed by the last ones; the product is past the stop before them
+    assert blended[-n_tail - 1] >= eps > blended[-1]
+    assert product[-n_tail - 50] < (1 - 1e-4) * float(eps) if mode == 1 else product[-n_tail - 50] < 2.0 ** -1e-4 * float(eps)
+
+    g = torch.Generator(device=DEV).manual_seed(mode)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, focal, focal, center_x=128.5, center_y=64.5).to(DEV)
+    stack = torch.zeros((5120, 3), device=DEV)
+    stack[:, 2] = 1.0 - torch.arange(5120, device=DEV) * 2.0 ** -12
+    bulk = torch.rand((n_bulk, 3), generator=g, device=DEV) * torch.tensor([0.6, 1.0, 0.0], device=DEV) + torch.tensor([0.6, -0.5, 0.0], device=DEV)
+    pos = torch.cat([stack, bulk]).contiguous()
+    opac = torch.cat([torch.from_numpy(np.array(first + later, np.float32)).to(DEV), torch.rand(n_bulk, generator=g, device=DEV)]).reshape(-1, 1)
+    feats = torch.zeros((pos.shape[0], 36), dtype=torch.float16, device=DEV)
+    scales = torch.full((pos.shape[0], 1), 1e-6, device=DEV) if mode == 1 else None
+    _, _, alpha = inpc_b200.INPCRasterizer().render_preextracted(view, mode, pos, feats, opac, scales, sigma_cutoff=1.0)
+    assert float(alpha[0, 64, 128]) == 1.0
+    assert int((alpha[0, 56:72, 120:144] != 0).sum()) == 1
+
+
 # four points per thread and 16-byte loads where the positions are aligned; one block gathers 256 points
 @pytest.mark.parametrize("n", [1, 2, 3, 5, 255, 257, 1023, 1025, 300_001])
 @pytest.mark.parametrize("offset", [0, 1])
