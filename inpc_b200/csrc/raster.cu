@@ -2425,7 +2425,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
                     G_run += bw * fg;
                     const float oma = 1.0f - e.x;
                     const float rcp = 1.0f / fmaxf(oma, kOneMinusAlphaEps);
-                    out = make_float2(bw, Tr * fg + (G_run - G_final) * rcp + K * rcp);
+                    // (no feature gradient from a weight that is not positive: a negative opacity, or not a number)
+                    out = make_float2(bw > 0.0f ? bw : 0.0f, Tr * fg + (G_run - G_final) * rcp + K * rcp);
                     Tr *= oma;
                     done = Tr < kTransmittanceEps;
                 }

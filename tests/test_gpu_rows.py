@@ -149,6 +149,27 @@ def test_rows_match_reference_backend_run_per_channel_group():
 
 
 @pytest.mark.parametrize("tile", [8, 16])
+def test_rows_of_points_without_positive_weight_have_no_gradient(tile):
+    """A fragment hands its row a gradient only where its blending weight is positive (bilinear/kernels.cu:361-415)."""
+    import inpc_b200
+    view, pos, _, opac = small_scene(n=6000, width=96, height=72, focal=85.0)
+    opac = opac.clone()
+    opac[::7] *= -0.2
+    opac[::11] = 0.0
+    feats = _rows(pos.shape[0], 16, 48)
+    f, o = feats.to(DEV).requires_grad_(True), opac.to(DEV).requires_grad_(True)
+    image, alpha, _ = inpc_b200.INPCRasterizer(tile_size=tile).forward_rows(view.to(DEV), pos.to(DEV), f, o)
+    g = torch.Generator().manual_seed(49)
+    gi, ga = torch.randn(image.shape, generator=g) * 1e-3, torch.randn(alpha.shape, generator=g) * 1e-3
+    torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
+    st = O.rasterize_rows_forward(oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy(), tile=tile)
+    gf, go = O.rasterize_rows_backward(st, gi.numpy(), ga.numpy())
+    assert_close(f.grad.cpu().numpy(), gf, rtol=1e-5, atol=1e-9, what="rows grad_features")
+    assert_close(o.grad.cpu().numpy(), go, rtol=1e-4, atol=1e-8, what="rows grad_opacities")
+    assert float(f.grad[::7].abs().max()) == 0.0 and float(f.grad[::11].abs().max()) == 0.0 and float(f.grad.abs().max()) > 0.0
+
+
+@pytest.mark.parametrize("tile", [8, 16])
 def test_rows_forward_returns_its_counts_and_holds_no_more_than_they_need(tile):
     """The counts of the state are final when the forward returns, and the instance scratch follows them."""
     import ctypes as C
