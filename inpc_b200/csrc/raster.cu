@@ -3566,7 +3566,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_b
                                             (Tr * f.y + (Crun.y - Cfin.y) * rcp) * g.y +
                                             (Tr * f.z + (Crun.z - Cfin.z) * rcp) * g.z +
                                             (Tr * f.w + (Crun.w - Cfin.w) * rcp) * g.w;
-                sm.out_bw[j][lane] = bw > 0.0f ? bw : 0.0f;
+                sm.out_bw[j][lane] = bw;
                 sm.out_go[j][lane] = (from_features + K * rcp) * G;
                 taken |= 1u << j;
                 Tr *= oma;
@@ -3582,8 +3582,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_b
                     const int p = __ffs(from) - 1;
                     from &= from - 1u;
                     const float bw = sm.out_bw[lane][p];
-                    const float4 pg = sm.pixel_grad[p];
-                    sf.x += bw * pg.x; sf.y += bw * pg.y; sf.z += bw * pg.z; sf.w += bw * pg.w;
+                    if (bw > 0.0f) {   // (zero times an upstream gradient that has overflowed would be no number)
+                        const float4 pg = sm.pixel_grad[p];
+                        sf.x += bw * pg.x; sf.y += bw * pg.y; sf.z += bw * pg.z; sf.w += bw * pg.w;
+                    }
                     so += sm.out_go[lane][p];
                 } while (from);
                 if (sf.x != 0.0f || sf.y != 0.0f || sf.z != 0.0f || sf.w != 0.0f) atomicAdd(grad_feat_view + id_cur, sf);

@@ -470,3 +470,21 @@ def test_point_scratch_holds_what_its_tile_size_uses(mode):
     settings = R.INPCRasterizer.extract_settings(view.to(DEV), mode)
     size = {tile: R.forward_with_state(pos.to(DEV), feats.to(DEV), opac.to(DEV), settings, tile)[4].point.numel() for tile in (8, 16)}
     assert size[8] - size[16] >= (4, 16)[mode] * n
+
+
+@pytest.mark.parametrize("tile", [8, 16])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_clear_points_have_no_feature_gradient_under_an_infinite_upstream(mode, tile):
+    """A fragment without weight adds nothing to its point's features, whatever the upstream gradient of its pixel is (a loss
+    scaled too far overflows to infinity)."""
+    import inpc_b200
+    view, pos, feats, opac = small_scene(n=6000, width=96, height=72, focal=85.0)
+    opac = opac.clone()
+    opac[::3] = 0.0
+    f, o = feats.to(DEV).requires_grad_(True), opac.to(DEV).requires_grad_(True)
+    image, alpha, _ = inpc_b200.INPCRasterizer(tile_size=tile)(view.to(DEV), mode, pos.to(DEV), f, o)
+    gi = torch.full_like(image, 1e-3)
+    gi[:, 20:50, 30:60] = float("inf")
+    torch.autograd.backward([image, alpha], [gi, torch.full_like(alpha, 1e-3)])
+    assert not bool(torch.isfinite(f.grad).all())                   # points with weight do carry it
+    assert bool((f.grad[::3] == 0).all())
