@@ -1383,12 +1383,13 @@ __device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_i
 // How far past its stop a pixel must be before pass PRODUCT closes it, relative (or in units of log2, where the same number
 // is wider).  REST multiplies up to `len` factors into a transmittance of its own, each product rounded by at most 2^-24 and, for
 // faint splats, mostly in one direction; PRODUCT's chain of products does the same from another start (gaussian), its sum of
-// logarithms is off by at most 2^-25 a term and 2^-23 of the 13.3 it can reach (bilinear): together less than len 2^-23.  A
+// logarithms is off by at most 2^-27 a term and 2^-23 of the 13.3 it can reach (bilinear): together less than len 2^-23.  A
 // pixel closed too early loses the fragments behind it, a ten-thousandth of the image's range.
 __device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f, (float)(len + 8u) * 1.1920928955078125e-07f); }
 
 constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
+constexpr float kLogScale = 67108864.0f;   // 2^26, see the product of pass PRODUCT
 
 // Pixels of the tile (bit = row * 8 + column) that the instance with this key reaches.
 __device__ __forceinline__ unsigned long long key_pixels(unsigned code) {
@@ -1758,12 +1759,14 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                         if (ok) atomicOr(sm.mask + p, 1u << lane);
                     } else if (ok) {
                         // A product does not care about order.  Its factors are added up as -log2(1 - alpha) in fixed
-                        // point (integer part and 24 fractional bits in two words per pixel): integer atomics commute, so
-                        // the sum is the same on every run, and none of the per-pixel ordering below is needed.
+                        // point (integer part and 26 fractional bits in two words per pixel, 32 of which fit a word): integer
+                        // atomics commute, so the sum is the same on every run, and none of the per-pixel ordering below is
+                        // needed.  (24 bits round a factor as coarsely as an fp32 product; on top of the rounding of 1 - alpha
+                        // that made the alpha of 200,000 splats of opacity 10^-6 twice as far off as a chain of products.)
                         const float x = 1.0f - al[c];
                         const float t = x > 0.0f ? fminf(-log2f(x), 64.0f) : 64.0f;   // 2^-64: far below the threshold
                         const float ti = floorf(t);
-                        atomicAdd(sm.mask + p, __float2uint_rn((t - ti) * 16777216.0f));
+                        atomicAdd(sm.mask + p, __float2uint_rn((t - ti) * kLogScale));
                         if (ti > 0.0f) atomicAdd(sm.off + p, (unsigned)ti);
                     }
                 }
@@ -1784,7 +1787,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                     if (frac | whole) {
                         sm.mask[lane] = 0u;
                         sm.off[lane] = 0u;
-                        log_sum += (double)whole + (double)frac * (1.0 / 16777216.0);
+                        log_sum += (double)whole + (double)frac * (1.0 / (double)kLogScale);
                     }
                     done = done || log_sum > log_stop;
                     done_w = __ballot_sync(kFull, done);

@@ -105,6 +105,31 @@ def test_blend_at_the_edges_of_its_segments(n, rows):
     assert_close(o.grad.cpu().numpy(), go, rtol=1e-3 + eps, atol=2e-8 + 1e-3 * eps, what="grad_opacities")
 
 
+# Lists of several segments of very faint splats: the segments' transmittances come from sums of logarithms, which may be no
+# further from double precision than the chain of fp32 products the oracle forms.
+@pytest.mark.parametrize("n,opacity", [(40_000, 2e-6), (200_000, 2e-6), (200_000, 2e-5)])
+def test_faint_splats_are_as_exact_as_a_chain_of_products(n, opacity):
+    import inpc_b200
+    from helpers import oracle_camera, small_scene
+    view, pos, feats, opac = small_scene(n=n, width=96, height=64, focal=82.0)
+    opac = (opac * opacity).contiguous()
+    _, alpha, _ = inpc_b200.INPCRasterizer()(view.to(DEV), 0, pos.to(DEV), feats.to(DEV), opac.to(DEV))
+    st = O.rasterize_forward(O.BILINEAR, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy())
+    # double precision: -log of the product over the 2x2 pixels of every visible point
+    seen = np.unique(st.inst_point)
+    xy, op = st.screen.reshape(-1, 2)[seen].astype(np.float64), opac.numpy().reshape(-1)[seen].astype(np.float64)
+    total, base = np.zeros((64, 96)), np.floor(xy - 0.5).astype(np.int64)
+    for dx in (0, 1):
+        for dy in (0, 1):
+            px, py = base[:, 0] + dx, base[:, 1] + dy
+            w = np.clip(1 - np.abs(xy[:, 0] - px - 0.5), 0, 1) * np.clip(1 - np.abs(xy[:, 1] - py - 0.5), 0, 1)
+            ok = (px >= 0) & (px < 96) & (py >= 0) & (py < 64)
+            np.add.at(total, (py[ok], px[ok]), np.log1p(-op[ok] * w[ok]))
+    exact = -np.expm1(total)
+    off = [np.sqrt(((a.reshape(64, 96).astype(np.float64) - exact) ** 2).mean()) for a in (alpha.cpu().numpy(), st.alpha)]
+    assert off[0] <= 1.25 * off[1], off
+
+
 # gaussian splats on 8x8 tiles: footprints from a fraction of a pixel to several tiles, image sides around tile and half borders
 @pytest.mark.parametrize("width,height", [(8, 4), (9, 5), (64, 36), (67, 45)])
 @pytest.mark.parametrize("sigma_px", [0.01, 0.7, 3.0, 40.0])
@@ -164,8 +189,8 @@ def test_a_long_segment_of_faint_splats_is_not_cut_before_its_end(mode):
     # every splat of the list sits on the centre of pixel (128, 64) and nothing else does: its alpha is its opacity
     if mode == 1:       # products from 1 down: just above a half, a step of 2^-24 is rounded up to twice its size
         faint, head, delta = f32(2.0 ** -24), [f32(0.499)], 3.2e-4
-    else:               # near the stop, a step of 2^-22 is rounded down by 8 %, its logarithm up by 4 % (to 6 / 2^24)
-        faint, head, delta = f32(2.0 ** -22), [], 9.1e-4
+    else:               # near the stop, a step of 3 x 2^-24 is rounded down by a fifth, its logarithm by 2 % (to 17 / 2^26)
+        faint, head, delta = f32(3 * 2.0 ** -24), [], 6.1e-4
     later = head + [faint] * (4096 - n_tail - len(head)) + [f32(0.9)] * n_tail
     start = float(np.prod([1.0 - float(a) for a in head]))
     want = float(eps) * (1 + delta) / start              # transmittance behind the first segment: three splats and 1021 that are clear
@@ -182,7 +207,7 @@ def test_a_long_segment_of_faint_splats_is_not_cut_before_its_end(mode):
     if mode == 1:
         product = np.array([float(t0) * float(t) for t in chain(f32(1), later)])
     else:
-        product = float(t0) * 2.0 ** -np.cumsum([round(-float(np.log2(f32(1) - a)) * 2 ** 24) / 2 ** 24 for a in later])
+        product = float(t0) * 2.0 ** -np.cumsum([round(-float(np.log2(f32(1) - a)) * 2 ** 26) / 2 ** 26 for a in later])
     # the blend is still open behind the faint splats and closed by the last ones; the product is past the stop before them
     assert blended[-n_tail - 1] >= eps > blended[-1]
     assert product[-n_tail - 50] < (1 - 1e-4) * float(eps) if mode == 1 else product[-n_tail - 50] < 2.0 ** -1e-4 * float(eps)
