@@ -1390,6 +1390,7 @@ __device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f,
 constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
 constexpr float kLogScale = 67108864.0f;   // 2^26, see the product of pass PRODUCT
+constexpr float kLogNaN = 1048576.0f;      // far above what 32 factors add up to
 
 // Pixels of the tile (bit = row * 8 + column) that the instance with this key reaches.
 __device__ __forceinline__ unsigned long long key_pixels(unsigned code) {
@@ -1763,11 +1764,13 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                         // atomics commute, so the sum is the same on every run, and none of the per-pixel ordering below is
                         // needed.  (24 bits round a factor as coarsely as an fp32 product; on top of the rounding of 1 - alpha
                         // that made the alpha of 200,000 splats of opacity 10^-6 twice as far off as a chain of products.)
+                        // An opacity below zero makes a factor above one: the integer part is signed.  A factor that is not a number
+                        // counts more than 32 others can, by which the pixel's product is known to be none either.
                         const float x = 1.0f - al[c];
-                        const float t = x > 0.0f ? fminf(-log2f(x), 64.0f) : 64.0f;   // 2^-64: far below the threshold
+                        const float t = x > 0.0f ? fminf(-log2f(x), 64.0f) : x <= 0.0f ? 64.0f : kLogNaN;   // 2^-64: far below the threshold
                         const float ti = floorf(t);
                         atomicAdd(sm.mask + p, __float2uint_rn((t - ti) * kLogScale));
-                        if (ti > 0.0f) atomicAdd(sm.off + p, (unsigned)ti);
+                        if (ti != 0.0f) atomicAdd(sm.off + p, (unsigned)(int)ti);
                     }
                 }
                 if (PASS == PASS_PRODUCT || kWeights) {   // inference keeps no lists for a backward pass
@@ -1787,7 +1790,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                     if (frac | whole) {
                         sm.mask[lane] = 0u;
                         sm.off[lane] = 0u;
-                        log_sum += (double)whole + (double)frac * (1.0 / (double)kLogScale);
+                        log_sum += (int)whole < (int)(kLogNaN / 2.0f) ? (double)(int)whole + (double)frac * (1.0 / (double)kLogScale) : (double)NAN;
                     }
                     done = done || log_sum > log_stop;
                     done_w = __ballot_sync(kFull, done);

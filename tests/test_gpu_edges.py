@@ -105,6 +105,43 @@ def test_blend_at_the_edges_of_its_segments(n, rows):
     assert_close(o.grad.cpu().numpy(), go, rtol=1e-3 + eps, atol=2e-8 + 1e-3 * eps, what="grad_opacities")
 
 
+# Opacities that are none: the products of later segments are sums of logarithms, which know no factor above one and no NaN by
+# themselves.  A pixel whose transmittance is no number has no stop, and its alpha is no number.
+@pytest.mark.parametrize("n", [700, 4097])
+@pytest.mark.parametrize("odd", ["negative", "nan"])
+@pytest.mark.parametrize("rows", [0, 8])
+def test_odd_opacities_in_lists_of_several_segments(n, odd, rows):
+    import inpc_b200
+    from helpers import assert_close, oracle_camera
+    view, pos, opac = _one_tile_scene(n, n)
+    opac = opac.clone()
+    if odd == "negative":
+        opac[::9] *= -0.5
+    else:
+        opac[torch.argsort(3.0 - pos[:, 2])[n * 3 // 4]] = float("nan")     # behind the first segment of the tile it is in
+    g = torch.Generator().manual_seed(n + 1)
+    cam, v, rast = oracle_camera(view), view.to(DEV), inpc_b200.INPCRasterizer()
+    if rows:
+        feats = torch.randn((n, rows), generator=g) * 0.5
+        image, alpha, bw = rast.forward_rows(v, pos.to(DEV), feats.to(DEV), opac.to(DEV))
+        st = O.rasterize_rows_forward(cam, pos.numpy(), feats.numpy(), opac.numpy())
+    else:
+        feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+        image, alpha, bw = rast(v, 0, pos.to(DEV), feats.to(DEV), opac.to(DEV))
+        st = O.rasterize_forward(O.BILINEAR, cam, pos.numpy(), feats.numpy(), opac.numpy())
+        _, depth, inferred = rast.render_preextracted(v, 0, pos.to(DEV), feats.to(DEV), opac.to(DEV))
+        _, odepth, oinferred, _ = O.render_preextracted(O.BILINEAR, cam, pos.numpy(), feats.numpy(), opac.numpy(), None, 0.05, 3.0)
+        np.testing.assert_array_equal(np.isnan(inferred.cpu().numpy()), np.isnan(oinferred))
+        np.testing.assert_array_equal(np.isnan(depth.cpu().numpy()), np.isnan(odepth))
+        assert_close(inferred.cpu().numpy(), oinferred, rtol=1e-5, atol=1e-6 + n / 16 * 2.0 ** -25, what="alpha of inference")
+    eps = n / 16 * 2.0 ** -25      # see the test of the segment edges
+    for got, want, what in ((image, st.image, "image"), (alpha, st.alpha, "alpha"), (bw, st.blending_weights, "blending weights")):
+        got = got.detach().cpu().numpy()
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want), err_msg=what)
+        assert_close(got, want, rtol=2e-4 + eps, atol=3e-6 + eps, what=what)
+    assert bool(np.isnan(st.alpha).any()) == (odd == "nan")
+
+
 # Lists of several segments of very faint splats: the segments' transmittances come from sums of logarithms, which may be no
 # further from double precision than the chain of fp32 products the oracle forms.
 @pytest.mark.parametrize("n,opacity", [(40_000, 2e-6), (200_000, 2e-6), (200_000, 2e-5)])
