@@ -1954,8 +1954,11 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel
 }
 
 // Per tile half with several segments, after the REST pass: image = sum of the segment colours in order.
-// For training the running sum before each segment replaces the segment's own colour (the backward pass
-// starts from it).  Inference: expected depth, and the transmittance where the pixel stopped = the end value
+// For training the sum of a segment's colour and those behind it replaces the segment's own: what the backward pass takes the
+// segment's running colour from.  Where a pixel stops in a segment nothing is behind it, and the two agree to the bit at the last
+// fragment, as in an undivided list; the image less the colours before the segment would leave their rounding there, which an
+// opacity close to one multiplies by 1 / (1 - alpha).
+// Inference: expected depth, and the transmittance where the pixel stopped = the end value
 // of the first segment that fell below the threshold.
 template <int KIND, int C4>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kernel(
@@ -1988,9 +1991,19 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
 #pragma unroll
                 for (int k = 0; k < 4; ++k) c[k] = g0 + k < n_seg ? part[(size_t)(g0 + k) * (64 * C4)] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (KIND == BLEND_TRAIN && g0 + k < n_seg) part[(size_t)(g0 + k) * (64 * C4)] = run;
-                    run.x += c[k].x; run.y += c[k].y; run.z += c[k].z; run.w += c[k].w;
+                for (int k = 0; k < 4; ++k) { run.x += c[k].x; run.y += c[k].y; run.z += c[k].z; run.w += c[k].w; }
+            }
+            if (KIND == BLEND_TRAIN) {
+                float4 rest = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int g0 = (int)((n_seg - 1u) & ~3u); g0 >= 0; g0 -= 4) {
+                    float4 c[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) c[k] = g0 + k < (int)n_seg ? part[(size_t)(g0 + k) * (64 * C4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int k = 3; k >= 0; --k) {
+                        rest.x += c[k].x; rest.y += c[k].y; rest.z += c[k].z; rest.w += c[k].w;
+                        if (g0 + k < (int)n_seg) part[(size_t)(g0 + k) * (64 * C4)] = rest;
+                    }
                 }
             }
             if (inside) {
@@ -2095,11 +2108,11 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
             const int64_t pi = (int64_t)py * width + px;
             g = make_float4(__ldg(grad_image + pi), __ldg(grad_image + n_px + pi), __ldg(grad_image + 2 * n_px + pi),
                             __ldg(grad_image + 3 * n_px + pi));
-            Cfin = make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi),
-                               __ldg(image + 3 * n_px + pi));
+            // what this segment and the ones behind it add to the pixel: the running colour starts at zero
+            Cfin = n_seg > 1u ? seg_C[sidx * 32 + lane]
+                              : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
             if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
-            if (n_seg > 1u) Crun = seg_C[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -2330,19 +2343,19 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
 #pragma unroll
             for (int c = 0; c < C4; ++c) {
                 const float* gp = grad_image + (int64_t)(4 * c) * n_px + pi;
-                const float* ip = image + (int64_t)(4 * c) * n_px + pi;
                 g[c] = make_float4(__ldg(gp), __ldg(gp + n_px), __ldg(gp + 2 * n_px), __ldg(gp + 3 * n_px));
-                G_final += __ldg(ip) * g[c].x + __ldg(ip + n_px) * g[c].y + __ldg(ip + 2 * n_px) * g[c].z + __ldg(ip + 3 * n_px) * g[c].w;
+                // what this segment and the ones behind it add to the pixel
+                float4 v;
+                if (n_seg > 1u) {
+                    v = seg_C[(sidx * C4 + c) * 32 + lane];
+                } else {
+                    const float* ip = image + (int64_t)(4 * c) * n_px + pi;
+                    v = make_float4(__ldg(ip), __ldg(ip + n_px), __ldg(ip + 2 * n_px), __ldg(ip + 3 * n_px));
+                }
+                G_final += v.x * g[c].x + v.y * g[c].y + v.z * g[c].z + v.w * g[c].w;
             }
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
             if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
-            if (n_seg > 1u) {
-#pragma unroll
-                for (int c = 0; c < C4; ++c) {
-                    const float4 v = seg_C[(sidx * C4 + c) * 32 + lane];
-                    G_run += v.x * g[c].x + v.y * g[c].y + v.z * g[c].z + v.w * g[c].w;
-                }
-            }
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -3508,11 +3521,11 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_b
             const int64_t pi = (int64_t)py * width + px;
             g = make_float4(__ldg(grad_image + pi), __ldg(grad_image + n_px + pi), __ldg(grad_image + 2 * n_px + pi),
                             __ldg(grad_image + 3 * n_px + pi));
-            Cfin = make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi),
-                               __ldg(image + 3 * n_px + pi));
+            // what this segment and the ones behind it add to the pixel: the running colour starts at zero
+            Cfin = n_seg > 1u ? seg_C[sidx * 32 + lane]
+                              : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
             if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
-            if (n_seg > 1u) Crun = seg_C[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through

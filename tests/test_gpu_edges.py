@@ -142,6 +142,31 @@ def test_odd_opacities_in_lists_of_several_segments(n, odd, rows):
     assert bool(np.isnan(st.alpha).any()) == (odd == "nan")
 
 
+# Where a pixel stops, its colour minus the running colour is zero to the bit, which 1 / (1 - alpha) would else multiply by up to 10^8:
+# also where the opaque splat lies in a later segment.
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n_before", [100, 255, 256, 300, 511, 700, 1500])
+def test_opacity_gradient_of_an_opaque_splat_in_a_later_segment(mode, n_before):
+    import inpc_b200
+    from helpers import assert_close, oracle_camera
+    from inpc_b200.views import look_at_view
+    n, g = n_before + 20, torch.Generator().manual_seed(n_before)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 17, 9, 16.0, 16.0)      # the axis meets the centre of pixel (8, 4)
+    pos = torch.zeros((n, 3))
+    pos[:, 2] = 1.0 - torch.arange(n) * 2.0 ** -11
+    opac = torch.rand((n, 1), generator=g) * min(2e-3, 1.0 / n)
+    opac[n_before] = 1.0
+    feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+    gi, ga = torch.randn((4, 9, 17), generator=g) * 1e-3, torch.randn((1, 9, 17), generator=g) * 1e-3
+    o = opac.to(DEV).requires_grad_(True)
+    image, alpha, _ = inpc_b200.INPCRasterizer()(view.to(DEV), mode, pos.to(DEV), feats.to(DEV), o)
+    torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
+    st = O.rasterize_forward(mode, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy())
+    _, go, _ = O.rasterize_backward(st, gi.numpy(), ga.numpy())
+    assert float(alpha.detach()[0, 4, 8]) == 1.0
+    assert_close(o.grad.cpu().numpy(), go, rtol=1e-3, atol=2e-8, what="grad_opacities")
+
+
 # Lists of several segments of very faint splats: the segments' transmittances come from sums of logarithms, which may be no
 # further from double precision than the chain of fp32 products the oracle forms.
 @pytest.mark.parametrize("n,opacity", [(40_000, 2e-6), (200_000, 2e-6), (200_000, 2e-5)])
