@@ -664,6 +664,18 @@ __device__ __forceinline__ unsigned spread_bits_10(unsigned v) {
     return v;
 }
 
+// Minimum and maximum that are NaN when an operand is, as a tensor's amin and amax are.
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // Corners of the cloud's bounding box, one partial result {min x, y, z, max x, y, z} per block: one pass over the positions,
 // four of them per thread and round in three 16-byte loads where the array allows.
 constexpr int kBoxBlocks = 592;   // 148 multiprocessors x 4
@@ -674,7 +686,7 @@ __device__ __forceinline__ void block_box(float* box, float (*s_box)[6]) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const float t = __shfl_xor_sync(0xffffffffu, box[c], o);
-            box[c] = c < 3 ? fminf(box[c], t) : fmaxf(box[c], t);
+            box[c] = c < 3 ? min_nan(box[c], t) : max_nan(box[c], t);
         }
     if (lane_id() == 0) {
 #pragma unroll
@@ -685,7 +697,7 @@ __device__ __forceinline__ void block_box(float* box, float (*s_box)[6]) {
     for (int c = 0; c < 6; ++c) {
         box[c] = s_box[0][c];
 #pragma unroll
-        for (int w = 1; w < kThreads / 32; ++w) box[c] = c < 3 ? fminf(box[c], s_box[w][c]) : fmaxf(box[c], s_box[w][c]);
+        for (int w = 1; w < kThreads / 32; ++w) box[c] = c < 3 ? min_nan(box[c], s_box[w][c]) : max_nan(box[c], s_box[w][c]);
     }
 }
 
@@ -693,8 +705,8 @@ __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __r
     __shared__ float s_box[kThreads / 32][6];
     float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
     auto add = [&](float x, float y, float z) {
-        box[0] = fminf(box[0], x); box[1] = fminf(box[1], y); box[2] = fminf(box[2], z);
-        box[3] = fmaxf(box[3], x); box[4] = fmaxf(box[4], y); box[5] = fmaxf(box[5], z);
+        box[0] = min_nan(box[0], x); box[1] = min_nan(box[1], y); box[2] = min_nan(box[2], z);
+        box[3] = max_nan(box[3], x); box[4] = max_nan(box[4], y); box[5] = max_nan(box[5], z);
     };
     const int64_t stride = (int64_t)gridDim.x * kThreads, tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t n4 = vec_ok ? n / 4 : 0;
@@ -709,7 +721,8 @@ __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __r
 }
 
 // The cube the codes refer to: the caller's, or (box_parts > 0) the cloud's own from the partial boxes, its edge widened by
-// a millionth so that the largest coordinate stays inside.  Same roundings as float32 corners and a double product.
+// a millionth so that the largest coordinate stays inside.  Same roundings as float32 corners and a double product.  An axis with
+// a NaN in it has no corner and takes no part in the codes, and the edge is then 1.
 struct MortonBox {
     float lo[3];
     float inv_extent;
@@ -725,10 +738,10 @@ __global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __r
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
                 const float t = __ldg(mb.parts + 6 * k + c);
-                box[c] = c < 3 ? fminf(box[c], t) : fmaxf(box[c], t);
+                box[c] = c < 3 ? min_nan(box[c], t) : max_nan(box[c], t);
             }
         block_box(box, s_box);
-        const float extent = fmaxf(fmaxf(__fsub_rn(box[3], box[0]), __fsub_rn(box[4], box[1])), __fsub_rn(box[5], box[2]));
+        const float extent = max_nan(max_nan(__fsub_rn(box[3], box[0]), __fsub_rn(box[4], box[1])), __fsub_rn(box[5], box[2]));
         mb.inv_extent = extent > 0.0f ? __fdiv_rn(1.0f, __double2float_rn(__dmul_rn((double)extent, 1.0 + 1e-6))) : 1.0f;
         mb.lo[0] = box[0]; mb.lo[1] = box[1]; mb.lo[2] = box[2];
     }

@@ -304,3 +304,27 @@ def test_morton_order_at_block_edges_and_offsets(n, offset):
     src = store[offset:]
     src.copy_(pos)
     assert torch.equal(morton_order(src).cpu(), pos[torch.sort(code, stable=True).indices])
+
+
+# a NaN leaves its axis without a corner (its part of the codes is zero) and the cube with an edge of 1; infinities are ordinary values
+@pytest.mark.parametrize("n", [2, 5, 257, 4099, 300_001])
+@pytest.mark.parametrize("odd", ["one_nan", "nan_axis", "nan_rows", "inf", "minus_inf"])
+def test_morton_order_of_clouds_with_odd_coordinates(n, odd):
+    from inpc_b200.sampling import morton_order
+    g = torch.Generator().manual_seed(n)
+    pos = torch.rand((n, 3), generator=g) * torch.tensor([2.0, 1.0, 3.0]) - 1.0
+    if odd == "one_nan":
+        pos[n // 2, 2] = float("nan")
+    elif odd == "nan_axis":
+        pos[::3, 1] = float("nan")
+    elif odd == "nan_rows":
+        pos[::4] = float("nan")
+    else:
+        pos[n - 1, 0] = float("inf") if odd == "inf" else -float("inf")
+    lo = pos.amin(dim=0)
+    extent = float((pos.amax(dim=0) - lo).max())
+    inv = np.float32(1.0) / np.float32(np.float64(extent) * (1.0 + 1e-6)) if extent > 0 else np.float32(1.0)
+    q = ((pos - lo) * torch.tensor(inv) * 1024.0).nan_to_num(nan=0.0).clamp(0.0, 1023.0).to(torch.int64)
+    code = sum((((q[:, c] >> b) & 1) << (3 * b + c)) for b in range(10) for c in range(3))
+    want = pos[torch.sort(code, stable=True).indices]
+    assert torch.equal(morton_order(pos.to(DEV)).cpu().view(torch.int32), want.view(torch.int32))
