@@ -2855,10 +2855,12 @@ __device__ __forceinline__ void gaussian_mask_bits(int j, const float4& a, const
         const float s = 2.0f * neg_log_threshold / det;
         const float rx = sqrtf(fmaxf(s * c.z, 0.0f)) * 1.001f + 0.01f;
         const float ry = sqrtf(fmaxf(s * c.x, 0.0f)) * 1.001f + 0.01f;
-        x0 = max(0, __float2int_ru(a.x - rx - 0.5f) - tile_x * T);
-        x1 = min(T - 1, __float2int_rd(a.x + rx - 0.5f) - tile_x * T);
-        y0 = max(0, __float2int_ru(a.y - ry - 0.5f) - tile_y * T);
-        y1 = min(T - 1, __float2int_rd(a.y + ry - 0.5f) - tile_y * T);
+        // (an ellipse that reaches beyond the integers, as with a cut-off whose threshold underflows to zero, must not wrap round)
+        constexpr float kFar = 1e9f;
+        x0 = max(0, __float2int_ru(fmaxf(a.x - rx - 0.5f, -kFar)) - tile_x * T);
+        x1 = min(T - 1, __float2int_rd(fminf(a.x + rx - 0.5f, kFar)) - tile_x * T);
+        y0 = max(0, __float2int_ru(fmaxf(a.y - ry - 0.5f, -kFar)) - tile_y * T);
+        y1 = min(T - 1, __float2int_rd(fminf(a.y + ry - 0.5f, kFar)) - tile_y * T);
     }
     const unsigned bit = 1u << (j & 31);
     unsigned* mrow = s_mask[j >> 5];

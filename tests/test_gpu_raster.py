@@ -488,3 +488,17 @@ def test_clear_points_have_no_feature_gradient_under_an_infinite_upstream(mode, 
     torch.autograd.backward([image, alpha], [gi, torch.full_like(alpha, 1e-3)])
     assert not bool(torch.isfinite(f.grad).all())                   # points with weight do carry it
     assert bool((f.grad[::3] == 0).all())
+
+
+# exp(-cutoff^2 / 2) is a normal float up to 13.2, none at all from 14.5 on: the ellipse then has no end
+@pytest.mark.parametrize("tile", [8, 16])
+@pytest.mark.parametrize("cutoff", [13.0, 14.0, 15.0, 40.0])
+def test_gaussian_cutoffs_around_the_smallest_threshold(cutoff, tile):
+    import inpc_b200
+    view, pos, feats, opac = small_scene(n=1500, width=96, height=72, focal=85.0)
+    rast = inpc_b200.INPCRasterizer(tile_size=tile)
+    img, dep, alp = rast.render_preextracted(view.to(DEV), 1, pos.to(DEV), feats.to(DEV), opac.to(DEV), sigma_cutoff=cutoff)
+    sigma = rast.extract_base_sigma_world(view.camera)
+    oi, od, oa, _ = O.render_preextracted(O.GAUSSIAN, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy(), None, sigma, cutoff, tile)
+    for got, want, what in ((img, oi, "image"), (dep, od, "depth"), (alp, oa, "alpha")):
+        assert_close(got.cpu().numpy(), want, rtol=2e-4, atol=2e-5, what=what)
