@@ -31,12 +31,16 @@ def test_sort_at_the_edges_of_its_tiles(n, end_bit):
 
 
 # a block places 2048 consecutive samples; it keeps the offsets of at most 2048 leaves in shared memory
-@pytest.mark.parametrize("total,gap", [(1, 0), (2047, 0), (2048, 1), (2049, 3000), (6145, 2049), (20_000, 2047)])
-def test_halton_samples_over_runs_of_empty_leaves(total, gap):
+@pytest.mark.parametrize("total,gap,largest", [(1, 0, 1), (2047, 0, 39), (2048, 0, 39), (2048, 1, 39), (2049, 3000, 39), (6145, 2049, 39),
+                                               (20_000, 2047, 39), (4096, 0, 2048), (300_001, 5, 300_000)])
+def test_halton_samples_over_runs_of_empty_leaves(total, gap, largest):
     from inpc_b200.sampling import halton_samples
     g = torch.Generator().manual_seed(total)
-    filled = torch.randint(1, 40, (max(1, total // 17),), generator=g)
-    filled[-1] += max(0, total - int(filled.sum()))
+    filled = torch.randint(1, largest + 1, (total,), generator=g)
+    filled[0] = largest                                    # up to 300,000 samples in one leaf: many digits behind the tabulated ones
+    filled = filled[:int((filled.cumsum(0) < total).sum()) + 1]
+    filled[-1] -= int(filled.sum()) - total                # the last leaf takes what is left, at least one
+    assert int(filled.sum()) == total and int(filled.min()) >= 1
     counts = torch.zeros(len(filled) * 2 + gap * 3, dtype=torch.int32)
     at = torch.arange(len(filled)) * 2
     at[len(filled) // 2:] += gap
@@ -46,6 +50,7 @@ def test_halton_samples_over_runs_of_empty_leaves(total, gap):
     centers = torch.rand((n, 3), generator=g) * 2 - 1
     levels = torch.randint(0, 11, (n,), generator=g, dtype=torch.int32)
     out = halton_samples(counts.to(DEV), centers.to(DEV), levels.to(DEV), 2.0)
+    assert out.shape == (total, 3)
     np.testing.assert_array_equal(out.cpu().numpy(), O.halton_samples(counts.numpy(), centers.numpy(), levels.numpy(), 2.0))
 
 
@@ -214,78 +219,79 @@ def test_gaussian_footprints_at_tile_edges(width, height, sigma_px):
         assert_close(got.cpu().numpy(), want, rtol=2e-4, atol=2e-5, max_bad=4, what=what)
 
 
+def _clear_of_the_cutoff(st, pos, threshold, reach):
+    """The points, those behind the camera whose weight at some pixel within `reach` lies so close to the threshold that rounding
+    (two units of the last place of the exponential, and of its argument) decides on which side it falls."""
+    xy, c = st.screen.reshape(-1, 2).astype(np.float64), st.conic.reshape(-1, 3).astype(np.float64)
+    near = np.zeros(len(xy), bool)
+    base = np.floor(xy) + 0.5
+    for ox in range(-reach, reach + 1):
+        for oy in range(-reach, reach + 1):
+            dx, dy = xy[:, 0] - base[:, 0] - ox, xy[:, 1] - base[:, 1] - oy
+            q = -0.5 * (c[:, 0] * dx * dx + c[:, 2] * dy * dy) - c[:, 1] * dx * dy
+            near |= np.abs(q - np.log(threshold)) < 1e-4
+    out = pos.clone()
+    out[torch.from_numpy(near)] = torch.tensor([0.0, 0.0, 10.0])
+    return out, int(near.sum())
+
+
 @pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 513, 20_001, 700_001])
 def test_gaussian_blend_at_the_edges_of_its_segments(n):
     import inpc_b200
     from helpers import assert_close, oracle_camera
     view, pos, opac = _one_tile_scene(n, n)
+    cam = oracle_camera(view)
     g = torch.Generator().manual_seed(n + 1)
     gi, ga = torch.randn((4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
     feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+    pos, dropped = _clear_of_the_cutoff(O.preprocess_and_order(O.GAUSSIAN, O.TRAIN, cam, pos.numpy(), feats.numpy(), opac.numpy()), pos,
+                                        0.01110899653, 3)
+    assert dropped <= n // 200
     f, o = feats.to(DEV).requires_grad_(True), opac.to(DEV).requires_grad_(True)
     image, alpha, bw = inpc_b200.INPCRasterizer()(view.to(DEV), 1, pos.to(DEV), f, o)
-    st = O.rasterize_forward(O.GAUSSIAN, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy())
+    st = O.rasterize_forward(O.GAUSSIAN, cam, pos.numpy(), feats.numpy(), opac.numpy())
     gf, go, _ = O.rasterize_backward(st, gi.numpy(), ga.numpy())
     torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
     # the bounds of the bilinear test with about six fragments per point; the exponentials of device and oracle differ by two
-    # units of the last place, and a fragment within rounding of the cut-off may fall on either side of it, which moves its point
-    # by a hundredth and the pixel by a hundredth of the point's opacity
+    # units of the last place
     eps = n / 10 * 2.0 ** -25 + 2.0 ** -22
-    cut = 0.012 * float(opac.max())
-    few = 4 + n // 5000
-    assert_close(image.detach().cpu().numpy(), st.image, rtol=1e-4, atol=1e-5 + 0.2 * eps + cut * (n > 1000), what="image")
-    assert_close(alpha.detach().cpu().numpy(), st.alpha, rtol=1e-5, atol=1e-6 + eps + cut * (n > 1000), max_bad=4, what="alpha")
-    assert_close(bw.cpu().numpy(), st.blending_weights, rtol=4e-4 + eps, atol=1e-9, max_bad=few, what="blending weights")
-    assert_close(f.grad.float().cpu().numpy(), np.asarray(gf, np.float32), rtol=4e-3 + eps, atol=2e-7, max_bad=36 * few, what="grad_features")
-    assert_close(o.grad.cpu().numpy(), go, rtol=2e-3 + eps, atol=4e-8 + 1e-3 * eps, max_bad=few, what="grad_opacities")
+    assert_close(image.detach().cpu().numpy(), st.image, rtol=1e-4, atol=1e-5 + 0.2 * eps, what="image")
+    assert_close(alpha.detach().cpu().numpy(), st.alpha, rtol=1e-5, atol=1e-6 + eps, what="alpha")
+    assert_close(bw.cpu().numpy(), st.blending_weights, rtol=4e-4 + eps, atol=1e-9, what="blending weights")
+    assert_close(f.grad.float().cpu().numpy(), np.asarray(gf, np.float32), rtol=4e-3 + eps, atol=2e-7, what="grad_features")
+    assert_close(o.grad.cpu().numpy(), go, rtol=2e-3 + eps, atol=4e-8 + 1e-3 * eps, what="grad_opacities")
+    assert all(bool(torch.isfinite(t).all()) for t in (image, alpha, bw, f.grad, o.grad))
 
 
-# The pass that cuts the lists of later segments (4096 instances from 5,242,881 on) multiplies in another order than the pass
-# that blends them.  Both round up to 4096 times: a pixel may be closed only when no rounding can have carried it over its stop.
-@pytest.mark.parametrize("mode", [0, 1])
-def test_a_long_segment_of_faint_splats_is_not_cut_before_its_end(mode):
+# inference with a size per splat over lists of several segments: the depth and the transmittance at which a pixel stopped come from
+# the segments' own
+@pytest.mark.parametrize("n", [255, 257, 1023, 4097, 20_001])
+@pytest.mark.parametrize("strength", [0.1, 1.0, 30.0])
+def test_gaussian_inference_over_several_segments(n, strength):
     import inpc_b200
-    from inpc_b200.views import look_at_view
-    f32, eps = np.float32, np.float32(1e-4)
-    width, height, focal, n_bulk, n_tail = 257, 129, 256.0, 5_600_000, 11
-    # every splat of the list sits on the centre of pixel (128, 64) and nothing else does: its alpha is its opacity
-    if mode == 1:       # products from 1 down: just above a half, a step of 2^-24 is rounded up to twice its size
-        faint, head, delta = f32(2.0 ** -24), [f32(0.499)], 3.2e-4
-    else:               # near the stop, a step of 3 x 2^-24 is rounded down by a fifth, its logarithm by 2 % (to 17 / 2^26)
-        faint, head, delta = f32(3 * 2.0 ** -24), [], 6.1e-4
-    later = head + [faint] * (4096 - n_tail - len(head)) + [f32(0.9)] * n_tail
-    start = float(np.prod([1.0 - float(a) for a in head]))
-    want = float(eps) * (1 + delta) / start              # transmittance behind the first segment: three splats and 1021 that are clear
-    a1 = f32(1) - f32(want ** (1 / 3))
-    t2 = (f32(1) - a1) * (f32(1) - a1)
-    first = [a1, a1, f32(1) - f32(want / float(t2))] + [f32(0)] * 1021
+    from helpers import assert_close, oracle_camera
+    view, pos, opac = _one_tile_scene(n, n)
+    opac, cam = (opac * strength).clamp(max=0.9).contiguous(), oracle_camera(view)
+    g = torch.Generator().manual_seed(n + 2)
+    feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+    scales = torch.exp(torch.randn((n, 1), generator=g) * 0.4) * 0.06          # about one and a half pixels
+    sigma = inpc_b200.INPCRasterizer.extract_base_sigma_world(view.camera)
 
-    def chain(t, alphas):
-        for a in alphas:
-            t = f32(t * (f32(1) - a))
-            yield t
-    t0 = list(chain(f32(1), first))[-1]
-    blended = list(chain(t0, later))
-    if mode == 1:
-        product = np.array([float(t0) * float(t) for t in chain(f32(1), later)])
-    else:
-        product = float(t0) * 2.0 ** -np.cumsum([round(-float(np.log2(f32(1) - a)) * 2 ** 26) / 2 ** 26 for a in later])
-    # the blend is still open behind the faint splats and closed by the last ones; the product is past the stop before them
-    assert blended[-n_tail - 1] >= eps > blended[-1]
-    assert product[-n_tail - 50] < (1 - 1e-4) * float(eps) if mode == 1 else product[-n_tail - 50] < 2.0 ** -1e-4 * float(eps)
-
-    g = torch.Generator(device=DEV).manual_seed(mode)
-    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, focal, focal, center_x=128.5, center_y=64.5).to(DEV)
-    stack = torch.zeros((5120, 3), device=DEV)
-    stack[:, 2] = 1.0 - torch.arange(5120, device=DEV) * 2.0 ** -12
-    bulk = torch.rand((n_bulk, 3), generator=g, device=DEV) * torch.tensor([0.6, 1.0, 0.0], device=DEV) + torch.tensor([0.6, -0.5, 0.0], device=DEV)
-    pos = torch.cat([stack, bulk]).contiguous()
-    opac = torch.cat([torch.from_numpy(np.array(first + later, np.float32)).to(DEV), torch.rand(n_bulk, generator=g, device=DEV)]).reshape(-1, 1)
-    feats = torch.zeros((pos.shape[0], 36), dtype=torch.float16, device=DEV)
-    scales = torch.full((pos.shape[0], 1), 1e-6, device=DEV) if mode == 1 else None
-    _, _, alpha = inpc_b200.INPCRasterizer().render_preextracted(view, mode, pos, feats, opac, scales, sigma_cutoff=1.0)
-    assert float(alpha[0, 64, 128]) == 1.0
-    assert int((alpha[0, 56:72, 120:144] != 0).sum()) == 1
+    def oracle(p):
+        return O.render_preextracted(O.GAUSSIAN, cam, p.numpy(), feats.numpy(), opac.numpy(), scales.numpy(), sigma, 3.0)
+    pos, dropped = _clear_of_the_cutoff(oracle(pos)[3], pos, np.exp(-4.5), 12)
+    assert dropped <= n // 10
+    image, depth, alpha = inpc_b200.INPCRasterizer().render_preextracted(view.to(DEV), 1, pos.to(DEV), feats.to(DEV), opac.to(DEV), scales.to(DEV))
+    oi, od, oa, _ = oracle(pos)
+    # inference takes the fast exponential: off by 2 + 1.2 |q| units of the last place, |q| <= 4.5; some 25 fragments per point.  A
+    # pixel within rounding of its stop may take a fragment more or less: up to 10^-4 of its transmittance, where pixels stop at all.
+    stop = 1.1e-4 if float(oa.max()) == 1.0 else 0.0
+    eps = n * 2.0 ** -25 + 2.0 ** -21
+    assert_close(image.cpu().numpy(), oi, rtol=1e-4, atol=1e-5 + 0.2 * eps + stop, what="image")
+    assert_close(alpha.cpu().numpy(), oa, rtol=1e-5, atol=1e-6 + eps + stop, what="alpha")
+    some = oa[0] > 1e-2            # the depth divides by alpha
+    assert_close(depth.cpu().numpy()[0][some], od[0][some], rtol=1e-4 + 100 * eps + stop, what="depth")
+    assert all(bool(torch.isfinite(t).all()) for t in (image, depth, alpha))
 
 
 # four points per thread and 16-byte loads where the positions are aligned; one block gathers 256 points
