@@ -676,25 +676,25 @@ __global__ void __launch_bounds__(256) tile_ranges_kernel(const uint32_t* __rest
     const int64_t n_instances = n_instances_dev ? (int64_t)*n_instances_dev : n_instances_arg;
     // the grid fits the chip: sized for the bound on the instance count it was three quarters empty blocks
     for (int64_t first = ((int64_t)blockIdx.x * 256 + threadIdx.x) * kPer; first < n_instances; first += (int64_t)gridDim.x * 256 * kPer) {
-    uint32_t prev = first > 0 ? __ldg(keys + first - 1) & kTileKeyMask : 0u;
-    uint32_t k8[kPer];
-    if (first + kPer <= n_instances) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(keys + first)), b = __ldg(reinterpret_cast<const uint4*>(keys + first) + 1);
-        k8[0] = a.x; k8[1] = a.y; k8[2] = a.z; k8[3] = a.w; k8[4] = b.x; k8[5] = b.y; k8[6] = b.z; k8[7] = b.w;
-    } else {
+        uint32_t prev = first > 0 ? __ldg(keys + first - 1) & kTileKeyMask : 0u;
+        uint32_t k8[kPer];
+        if (first + kPer <= n_instances) {
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(keys + first)), b = __ldg(reinterpret_cast<const uint4*>(keys + first) + 1);
+            k8[0] = a.x; k8[1] = a.y; k8[2] = a.z; k8[3] = a.w; k8[4] = b.x; k8[5] = b.y; k8[6] = b.z; k8[7] = b.w;
+        } else {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) k8[k] = first + k < n_instances ? __ldg(keys + first + k) : 0u;
-    }
+            for (int k = 0; k < kPer; ++k) k8[k] = first + k < n_instances ? __ldg(keys + first + k) : 0u;
+        }
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-        const int64_t i = first + k;
-        if (i >= n_instances) break;
-        const uint32_t key = k8[k] & kTileKeyMask;
-        if (i == 0) ranges[key].x = 0u;
-        else if (key != prev) { ranges[prev].y = (unsigned)i; ranges[key].x = (unsigned)i; }
-        if (i == n_instances - 1) ranges[key].y = (unsigned)n_instances;
-        prev = key;
-    }
+        for (int k = 0; k < kPer; ++k) {
+            const int64_t i = first + k;
+            if (i >= n_instances) break;
+            const uint32_t key = k8[k] & kTileKeyMask;
+            if (i == 0) ranges[key].x = 0u;
+            else if (key != prev) { ranges[prev].y = (unsigned)i; ranges[key].x = (unsigned)i; }
+            if (i == n_instances - 1) ranges[key].y = (unsigned)n_instances;
+            prev = key;
+        }
     }
 }
 
@@ -891,29 +891,14 @@ __global__ void __launch_bounds__(T * T) blend_bilinear_transmittance_kernel(
     __syncthreads();
     float Tr = 1.0f;
     bool done = !inside;
-    // With 8x8 tiles the next batch's loads are issued before the current batch is walked (measured 3 %
-    // faster); with 16x16 tiles the extra registers cost more than the overlap gains.
-    constexpr bool kPrefetch = T == 8;
+    // (fetching the next batch before the current one is walked costs more registers than the overlap gains)
     Fetched<false> next[IPT];
-    int cnt_next = (int)min((unsigned)B, sg.end - sg.begin);
-    if (kPrefetch) {
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<false>(t + k * P, cnt_next, sg.begin, inst_ids, rec);
-    }
     for (unsigned base = sg.begin; base < sg.end; base += B) {
-        if (!kPrefetch) {
-            cnt_next = (int)min((unsigned)B, sg.end - base);
+        const int cnt = (int)min((unsigned)B, sg.end - base);
 #pragma unroll
-            for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<false>(t + k * P, cnt_next, base, inst_ids, rec);
-        }
-        const int cnt = cnt_next;
+        for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<false>(t + k * P, cnt, base, inst_ids, rec);
 #pragma unroll
         for (int k = 0; k < IPT; ++k) commit_instance<T, false>(t + k * P, cnt, next[k], tx, ty, s_a, nullptr, s_mask);
-        if (kPrefetch) {
-            cnt_next = base + B < sg.end ? (int)min((unsigned)B, sg.end - (base + B)) : 0;
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<false>(t + k * P, cnt_next, base + B, inst_ids, rec);
-        }
         __syncthreads();
 #pragma unroll 1
         for (int w = 0; w < WORDS; ++w) {
@@ -1015,32 +1000,17 @@ __global__ void __launch_bounds__(T * T) blend_bilinear_forward_kernel(
             }
         }
     };
-    // With 8x8 tiles the next batch's loads are issued before the current batch is walked (measured 3 %
-    // faster); with 16x16 tiles the extra registers cost more than the overlap gains.
-    constexpr bool kPrefetch = T == 8;
+    // (fetching the next batch before the current one is walked costs more registers than the overlap gains)
     Fetched<true> next[IPT];
-    int cnt_next = (int)min((unsigned)B, sg.end - sg.begin);
-    if (kPrefetch) {
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt_next, sg.begin, inst_ids, rec);
-    }
     for (unsigned base = sg.begin; base < sg.end; base += B) {
         if (KIND == BLEND_TRAIN) flush_weights();
-        if (!kPrefetch) {
-            cnt_next = (int)min((unsigned)B, sg.end - base);
+        cnt = (int)min((unsigned)B, sg.end - base);
 #pragma unroll
-            for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt_next, base, inst_ids, rec);
-        }
-        cnt = cnt_next;
+        for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt, base, inst_ids, rec);
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
             id[k] = next[k].id;
             commit_instance<T, true>(t + k * P, cnt, next[k], tx, ty, s_a, s_f, s_mask);
-        }
-        if (kPrefetch) {
-            cnt_next = base + B < sg.end ? (int)min((unsigned)B, sg.end - (base + B)) : 0;
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt_next, base + B, inst_ids, rec);
         }
         __syncthreads();
 #pragma unroll 1
@@ -1232,32 +1202,17 @@ __global__ void __launch_bounds__(T * T) blend_bilinear_backward_kernel(
             }
         }
     };
-    // With 8x8 tiles the next batch's loads are issued before the current batch is walked (measured 3 %
-    // faster); with 16x16 tiles the extra registers cost more than the overlap gains.
-    constexpr bool kPrefetch = T == 8;
+    // (fetching the next batch before the current one is walked costs more registers than the overlap gains)
     Fetched<true> next[IPT];
-    int cnt_next = (int)min((unsigned)B, sg.end - sg.begin);
-    if (kPrefetch) {
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt_next, sg.begin, inst_ids, rec);
-    }
     for (unsigned base = sg.begin; base < sg.end; base += B) {
         flush_gradients();
-        if (!kPrefetch) {
-            cnt_next = (int)min((unsigned)B, sg.end - base);
+        cnt = (int)min((unsigned)B, sg.end - base);
 #pragma unroll
-            for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt_next, base, inst_ids, rec);
-        }
-        cnt = cnt_next;
+        for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt, base, inst_ids, rec);
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
             id[k] = next[k].id;
             commit_instance<T, true>(t + k * P, cnt, next[k], tx, ty, s_a, s_f, s_mask);
-        }
-        if (kPrefetch) {
-            cnt_next = base + B < sg.end ? (int)min((unsigned)B, sg.end - (base + B)) : 0;
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) next[k] = fetch_instance<true>(t + k * P, cnt_next, base + B, inst_ids, rec);
         }
         __syncthreads();
 #pragma unroll 1

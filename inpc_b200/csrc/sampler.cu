@@ -678,7 +678,7 @@ __device__ __forceinline__ float max_nan(float a, float b) {
 
 // Corners of the cloud's bounding box, one partial result {min x, y, z, max x, y, z} per block: one pass over the positions,
 // four of them per thread and round in three 16-byte loads where the array allows.
-constexpr int kBoxBlocks = 592;   // 148 multiprocessors x 4
+constexpr int kMaxBoxBlocks = 1024;   // room for the partial boxes; four blocks per multiprocessor are launched
 __device__ __forceinline__ void block_box(float* box, float (*s_box)[6]) {
     // box[0..2] minima, box[3..5] maxima of a thread -> of the block, in every thread of warp 0
 #pragma unroll
@@ -1135,7 +1135,7 @@ extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, cons
 
 extern "C" size_t inpc_morton_workspace_bytes(int64_t n) {
     const size_t arr = align_up(sizeof(uint32_t) * (size_t)(n > 0 ? n : 1));
-    return 4 * arr + align_up(6 * sizeof(float) * kBoxBlocks) + sort_workspace_bytes(n, n) + 256;
+    return 4 * arr + align_up(6 * sizeof(float) * kMaxBoxBlocks) + sort_workspace_bytes(n, n) + 256;
 }
 
 extern "C" int inpc_morton_order(const float* positions, int64_t n, const float* box_lo, float box_extent, float* out, void* workspace,
@@ -1149,7 +1149,7 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
     Carver c(workspace);
     uint32_t* codes[2] = {c.take<uint32_t>(n), c.take<uint32_t>(n)};
     uint32_t* order[2] = {c.take<uint32_t>(n), c.take<uint32_t>(n)};
-    float* parts = c.take<float>(6 * kBoxBlocks);
+    float* parts = c.take<float>(6 * kMaxBoxBlocks);
     c.off = align_up(c.off);
     void* sort_ws = c.base + c.off;
     MortonBox mb{{0.0f, 0.0f, 0.0f}, 1.0f, parts, 0};
@@ -1157,7 +1157,8 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
         for (int k = 0; k < 3; ++k) mb.lo[k] = box_lo[k];
         mb.inv_extent = 1.0f / box_extent;
     } else {
-        mb.box_parts = (int)(ceil_div<int64_t>(n, 4 * kThreads) < kBoxBlocks ? ceil_div<int64_t>(n, 4 * kThreads) : kBoxBlocks);
+        const int64_t blocks = ceil_div<int64_t>(n, 4 * kThreads), cap = 4 * sm_count() < kMaxBoxBlocks ? 4 * sm_count() : kMaxBoxBlocks;
+        mb.box_parts = (int)(blocks < cap ? blocks : cap);
         bounding_box_kernel<<<mb.box_parts, kThreads, 0, stream>>>(positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, parts);
         INPC_LAUNCH_CHECK("bounding_box_kernel");
     }
