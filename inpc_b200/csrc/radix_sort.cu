@@ -88,8 +88,8 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
 }
 
 // ---- one pass ---------------------------------------------------------------------------------
-// Bound by shared-memory wavefronts (63 % of the LSU data pipe over the whole pass, 40 wavefronts per 32 pairs) and by
-// the phases of a tile waiting on one another, not by DRAM (16 bytes per pair, 16 % of its peak).  Persistent blocks take
+// Bound by shared-memory wavefronts (63 % of the LSU data pipe over the whole pass, 39 wavefronts per 32 pairs) and by
+// the phases of a tile waiting on one another, not by DRAM (16 bytes per pair, 15 % of its peak).  Persistent blocks take
 // tiles from a ticket counter: the grid fits the chip whatever the bound on n is (a grid sized for an upper bound of a
 // device-side count was mostly empty blocks).  Per tile:
 //   1. rank: every lane ORs its bit into its warp's match word of its digit; the word then names the lanes that hold the
