@@ -172,7 +172,8 @@ int inpc_render_preextracted(int mode, int tile_size, const inpc_view* view, int
  * features (n, channels), 16-byte aligned) that are blended as they are, without spherical
  * harmonics, into image (channels,H,W).  alpha (H,W), blending_weights (n), the scratch callbacks
  * and `state` are as in inpc_rasterize_forward; the two counters are read back once for either tile size, so the
- * instance scratch has the size the scene needs and state->n_visible / n_instances are final on return.
+ * instance scratch has the size the scene needs and state->n_visible / n_instances are final on return (while
+ * `stream` is being captured nothing can be read back: 8x8 tiles then defer as in inpc_rasterize_forward).
  * No counterpart in the reference, whose backend only blends the four channels it evaluates from 36
  * SH halves (rasterization/src/rasterization_api.cu:23-107): the ordering is that of
  * rasterization/src/bilinear/forward.cu:59-170 and the per-fragment arithmetic that of

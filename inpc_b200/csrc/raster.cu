@@ -3749,10 +3749,20 @@ constexpr int kWarpBlendParts = 2;   // work items of the warp blend per (tile, 
 // Bilinear splats touch at most 2x2 tiles.
 bool has_instance_bound(int mode, int tile) { return mode == INPC_MODE_BILINEAR && uses_warp_blend(tile); }
 
-// Whether a call sizes everything for that bound and leaves its counts on the device.  Feature rows do not: the bound takes three times
-// the instance scratch the counts ask for (64 bytes per point against about 20), and with C / 4 times the segment colours that is
-// memory a scene of wide rows has better use for; the counts are also part of what their forward returns.
-bool defers_counts(int mode, int tile, bool rows, int64_t n) { return has_instance_bound(mode, tile) && !rows && n > 0 && n < ((int64_t)1 << 28); }
+// Whether a call sizes everything for that bound and leaves its counts on the device.  Feature rows do so only where nothing can be read
+// back, while their stream is being captured: the bound takes three times the instance scratch the counts ask for (64 bytes per
+// point against about 20), and with C / 4 times the segment colours that is memory a scene of wide rows has better use for; the
+// counts are also part of what their forward returns.
+bool defers_counts(int mode, int tile, bool rows, int64_t n, cudaStream_t stream) {
+    if (!has_instance_bound(mode, tile) || n <= 0 || n >= ((int64_t)1 << 28)) return false;
+    if (!rows) return true;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return status == cudaStreamCaptureStatusActive;
+}
 
 // The bounded path sizes its arrays for 4 instances per point; most splats touch one tile of four or none twice, about 1.3
 // on average (2^23 samples at 1237x822: 1.26; at 3840x2160 less).  Only picks tile sizes.
@@ -3924,7 +3934,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     // for 4 n instances and lets the kernels read the two counts from device memory: no host synchronisation at
     // all (the reference reads both counts back with blocking copies, src/bilinear/forward.cu:86-89).  The other
     // paths (gaussian splats have no such bound, feature rows keep their scratch small) read the counts back once.
-    const bool deferred = defers_counts(MODE, rp.tile, VARIANT == VAR_ROWS, n);
+    const bool deferred = defers_counts(MODE, rp.tile, VARIANT == VAR_ROWS, n, stream);
     int64_t n_visible = 0, n_instances = 0;
     uint32_t key_base = 0;
     int key_bits = 0;

@@ -196,6 +196,40 @@ def test_rows_forward_returns_its_counts_and_holds_no_more_than_they_need(tile):
     assert blobs.instance.numel() <= 20 * state.n_instances + segments * tile * tile * per_px + (4 << 20)
 
 
+@pytest.mark.parametrize("channels", [4, 16])
+def test_rows_step_can_be_captured(channels):
+    """Nothing can be read back from a stream that is being captured: the step then sizes its scratch by the bound and replays."""
+    import os
+
+    import inpc_b200
+    if "checked" in os.environ.get("INPC_B200_LIB", ""):
+        pytest.skip("the index-checking build reads its failure count back in every call")
+    view, pos, _, opac = small_scene(n=20000, width=136, height=104, focal=120.0)
+    v, p, feats, o = view.to(DEV), pos.to(DEV), _rows(20000, channels, 50).to(DEV), opac.to(DEV)
+
+    def step():
+        f, a = feats.detach().requires_grad_(True), o.detach().requires_grad_(True)
+        image, alpha, bw = inpc_b200.INPCRasterizer().forward_rows(v, p, f, a)
+        (image.sum() + alpha.sum()).backward()
+        return [t.detach() for t in (image, alpha, bw, f.grad, a.grad)]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            want = step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        got = step()
+    for _ in range(2):
+        for t in got:
+            t.fill_(-1.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b, what in zip(got, want, ("image", "alpha", "blending weights", "grad_features", "grad_opacities")):
+            # the order of the atomics that add a point's shares may differ; the list itself does not
+            assert_close(a.cpu().numpy(), b.cpu().numpy(), rtol=1e-5, atol=1e-6, what=what)
+
+
 def test_rows_empty_culled_and_bad_arguments():
     import inpc_b200
     view, pos, _, opac = small_scene(n=64, width=40, height=24, focal=30.0)
