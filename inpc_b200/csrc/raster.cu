@@ -1268,14 +1268,15 @@ constexpr size_t backward_smem_bytes() {
 // in flight while the current one is blended.  The mask used by the filter lags the blend by a batch;
 // that only lets a few extra instances through, whose fragments are then dropped.
 //
-// (2) A batch.  The geometry of a fragment (bilinear weight, alpha) depends on nothing that came
-// before it, the blend itself is a serial chain per pixel.  So lane j first evaluates the (up to) four
-// fragments of staged instance j, then the fragments are brought into per-pixel order in shared
-// memory (bit masks per pixel give every fragment its rank, a scan of the counts gives every pixel
-// its offset), and only then does every lane run down the short list of its own pixel: load alpha
-// and features, accumulate, update the transmittance.  What a fragment saw (its transmittance) goes
-// back to the instance lane, which forms the per-point sums in fixed corner order.  The arithmetic
-// and its order are those of a plain front-to-back loop per pixel.
+// (2) A batch is 32 staged instances.  Lane j finds the pixels of the half that the 2x2 footprint of instance j covers and that
+// have not stopped; a 32x32 bit transposition over the warp turns these masks into one word per pixel, and every lane walks the
+// set bits of its own pixel front to back: it reads the record, forms weight and alpha, accumulates and updates the transmittance.
+// What a fragment adds to its point (blending weight, gradient) goes to a slot per instance and parity of the pixel's column
+// and row -- the four pixels of a footprint have four different parities, so the slot is a constant of the lane -- and lane j adds
+// up the slots of instance j in a fixed order.  Against forming weight and alpha per instance and sorting the fragments by pixel in
+// shared memory (masks by atomics, a scan, a slot per fragment): forward passes of 16-channel rows 614 -> 496 us (2^23
+// samples at 1237x822), first pass of a 2^25-point cloud at 1920x1080 411 -> 343, all passes of the 4-channel
+// training step 342 -> 332.  The backward pass of four channels still sorts its fragments (walking: 243 -> 262 us).
 //
 // (3) Segments.  Front-to-back compositing is associative: (C, T) o (C', T') = (C + T C', T T').  A
 // tile's list is cut into a first segment and later ones (see segment_lengths), and every (tile half, segment) is one
@@ -1298,7 +1299,6 @@ constexpr size_t backward_smem_bytes() {
 // ------------------------------------------------------------------------------------------------
 constexpr int kWarpBlendWarps = 8;        // warps per block; every warp works on items of its own
 constexpr int kQueueCap = 256;            // ring of candidate point ids per warp: >= 31 left over + 128 of one filter step
-constexpr int kFilterKeys = 4;            // keys per lane and filter step
 // Segment lengths.  Measured on B200 (2^23 clustered samples, 1237x822; forward / backward stage in microseconds), first + later
 // segment: 1024 + 4096: 422 / 276, 1024 + 2048: 439 / 268, 512 + 4096: 437 / 297, 512 + 2048: 458 / 274, 1024 + 1024: 488 / 291,
 // 512 + 1024: 518 / 283, 256 + 2048: 469 / 283: with this many instances every pass is full (about 3000 of the 3552 resident
@@ -1342,7 +1342,6 @@ __device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_i
 // pixel closed too early loses the fragments behind it, a ten-thousandth of the image's range.
 __device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f, (float)(len + 8u) * 1.1920928955078125e-07f); }
 
-constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
 constexpr float kLogScale = 67108864.0f;   // 2^26, see the product of pass PRODUCT
 constexpr float kLogNaN = 1048576.0f;      // far above what 32 factors add up to
@@ -1493,6 +1492,7 @@ __device__ __forceinline__ void async_copy_wait() { asm volatile("cp.async.wait_
 constexpr int kGatherDepthFilter = 2;     // stages of the ring, a power of two: first segments and products,
 constexpr int kGatherDepthRest = 2;       // later segments,
 constexpr int kGatherDepthBackward = 2;   // backward pass
+constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 constexpr int kIdsAhead = 3;      // later segments: batches whose point ids are loaded ahead of their gather
 
 // Where the features of a splat come from: the second half of its record (four view-space channels), or, for feature rows,
@@ -1512,22 +1512,98 @@ __device__ __forceinline__ void gather_rows(float4* ring, const float4* __restri
     }
 }
 
+// Bit l of lane k's word becomes bit k of lane l's word.
+__device__ __forceinline__ unsigned warp_transpose_bits(unsigned x, unsigned lane) {
+    unsigned m = 0x0000FFFFu;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
+        x = (lane & (unsigned)s) ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y & m) << s);
+        m ^= m << (s >> 1);
+    }
+    return x;
+}
+
+// Pixels (bit = row * 8 + column) of the 8x4 half at (px0, py0) that the 2x2 footprint of a bilinear splat at (x, y) covers.  A
+// pixel at a distance of exactly one is among them; its weight is zero, by which it is told apart where the weight is formed.
+__device__ __forceinline__ unsigned footprint_pixels(float x, float y, int px0, int py0) {
+    const int qx = __float2int_rd(x - 0.5f) - px0, qy = __float2int_rd(y - 0.5f) - py0;   // left column, upper row
+    if ((unsigned)(qx + 1) > 8u || (unsigned)(qy + 1) > 4u) return 0u;
+    const unsigned two_by_two = qx < 0 ? 0x202u : qx == 7 ? 0x101u : 0x303u;              // clipped to the eight columns
+    return (unsigned)(((unsigned long long)two_by_two << (8 * qy + qx + 9)) >> 9);        // rows outside the half fall off either end
+}
+
+// The instances of a work item that can still have an effect, in list order: streams the item's keys and point ids, keeps those whose
+// pixels (`reach`, by key code, of this half) have not all stopped, and queues their ids.  A step is 128 keys, four consecutive
+// ones per lane in one 16-byte load, asked for a step ahead; the list need not start or end at such a boundary.
+struct CandidateStream {
+    const uint32_t *keys, *ids;
+    unsigned begin, end;    // the item's range
+    unsigned pos;           // next step to load, a multiple of 4 (the arrays are 256-byte aligned)
+    unsigned head, tail;    // candidates [head, tail) wait for their gather
+    bool loaded;
+    uint4 key, id;          // the step that is loaded; behind `end` and before `begin` keys whose code reaches nothing
+
+    __device__ __forceinline__ void load(unsigned lane) {
+        const unsigned first = pos + 4u * lane;
+        key = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        id = make_uint4(0u, 0u, 0u, 0u);
+        if (first < end) {
+            key = __ldg(reinterpret_cast<const uint4*>(keys + first));
+            id = __ldg(reinterpret_cast<const uint4*>(ids + first));
+        }
+        if (pos < begin || pos + 128u > end) {   // the first or the last step of the list
+            const unsigned n = end - begin;
+            if (first - begin >= n) key.x = 0xFFFFFFFFu;
+            if (first + 1u - begin >= n) key.y = 0xFFFFFFFFu;
+            if (first + 2u - begin >= n) key.z = 0xFFFFFFFFu;
+            if (first + 3u - begin >= n) key.w = 0xFFFFFFFFu;
+        }
+        pos += 128u;
+        loaded = true;
+    }
+    __device__ __forceinline__ void start(const uint32_t* keys_, const uint32_t* ids_, unsigned begin_, unsigned end_, unsigned lane) {
+        keys = keys_; ids = ids_;
+        begin = begin_; end = end_;
+        pos = begin_ & ~3u;
+        head = tail = 0u;
+        loaded = false;
+        if (begin < end) load(lane);
+    }
+    // until 32 candidates wait or the list ends
+    __device__ __forceinline__ void fill(const unsigned* reach, unsigned done_w, uint32_t* queue, unsigned lane, unsigned lt_mask) {
+        while (tail - head < 32u && loaded) {
+            const uint4 k4 = key, i4 = id;
+            loaded = false;
+            if (pos < end) load(lane);
+            const bool k0 = (reach[k4.x >> kTileKeyBits] & ~done_w) != 0u, k1 = (reach[k4.y >> kTileKeyBits] & ~done_w) != 0u;
+            const bool k2 = (reach[k4.z >> kTileKeyBits] & ~done_w) != 0u, k3 = (reach[k4.w >> kTileKeyBits] & ~done_w) != 0u;
+            const unsigned b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
+            const unsigned b2 = __ballot_sync(0xffffffffu, k2), b3 = __ballot_sync(0xffffffffu, k3);
+            unsigned at = tail + __popc(b0 & lt_mask) + __popc(b1 & lt_mask) + __popc(b2 & lt_mask) + __popc(b3 & lt_mask);
+            if (k0) queue[at++ & (kQueueCap - 1)] = i4.x;
+            if (k1) queue[at++ & (kQueueCap - 1)] = i4.y;
+            if (k2) queue[at++ & (kQueueCap - 1)] = i4.z;
+            if (k3) queue[at & (kQueueCap - 1)] = i4.w;
+            tail += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3);
+        }
+    }
+};
+
 // Shared memory of one warp of the forward passes.
 template <bool BLEND, bool WEIGHTS, int DEPTH, int C4>
 struct __align__(16) WarpForwardSmem {
     float4 ring_a[DEPTH][32];                        // records of the batches in flight: position, alpha, depth ...
     float4 ring_f[BLEND ? DEPTH : 1][BLEND ? 32 * feature_stride(C4) : 1];   // ... and features
-    float2 frag[kBatchFragments];                    // fragments in per-pixel order: alpha, lane of the staged instance
-    float frag_seen[WEIGHTS ? kBatchFragments : 1];  // transmittance the fragment met (0: it was dropped)
+    float4 weight[WEIGHTS ? 32 : 1];                 // per staged instance: what its pixels add to its blending weight, by parity
     uint32_t ring_id[DEPTH][32];                     // point ids of the batches in flight (0xFFFFFFFF: no instance)
-    unsigned mask[32];                               // per pixel: staged instances with a fragment there
-    unsigned off[32];                                // per pixel: first slot of its fragment list
+    unsigned sum[BLEND ? 1 : 2][BLEND ? 1 : 32];     // PRODUCT: per pixel, the two words of a batch's sum of logarithms
     uint32_t queue[kQueueCap];
 };
 
 template <int PASS, int KIND, int C4>
 constexpr size_t warp_forward_smem_bytes() {
-    return 256 * sizeof(unsigned long long) +
+    return 2 * 256 * sizeof(unsigned) +
            kWarpBlendWarps * sizeof(WarpForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN,
                                                     PASS == PASS_REST ? kGatherDepthRest : kGatherDepthFilter, C4>);
 }
@@ -1550,13 +1626,17 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
     static_assert(ROWS || C4 == 1, "a record holds four channels");
     using Smem = WarpForwardSmem<kBlend, kWeights, kGatherDepth, C4>;
     extern __shared__ __align__(16) unsigned char blend_smem[];
-    unsigned long long* s_reach = reinterpret_cast<unsigned long long*>(blend_smem);     // key code -> pixels reached
-    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 256 * sizeof(unsigned long long))[threadIdx.x >> 5];
+    unsigned* s_reach = reinterpret_cast<unsigned*>(blend_smem);     // [half][key code] -> pixels of the half reached
+    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 2 * 256 * sizeof(unsigned))[threadIdx.x >> 5];
     const unsigned lane = lane_id();
     const unsigned lt_mask = (1u << lane) - 1u;
-    s_reach[threadIdx.x] = key_pixels(threadIdx.x);
-    sm.mask[lane] = 0u;   // the masks start at zero and every batch leaves them at zero again
-    sm.off[lane] = 0u;    // (the product pass uses both arrays as per-pixel accumulators)
+    const unsigned parity = (lane & 1u) | ((lane >> 2) & 2u);        // of this lane's pixel: a footprint has each of the four once
+    {
+        const unsigned long long m = key_pixels(threadIdx.x);
+        s_reach[threadIdx.x] = (unsigned)m;
+        s_reach[256 + threadIdx.x] = (unsigned)(m >> 32);
+    }
+    if (PASS == PASS_PRODUCT) { sm.sum[0][lane] = 0u; sm.sum[1][lane] = 0u; }   // every batch leaves the sums at zero again
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
     // Items are handed out one at a time through a ticket counter: consecutive items cost about the same (neighbouring
@@ -1589,6 +1669,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
         const int px0 = tx * 8, py0 = ty * 8 + 4 * half;            // first pixel of this half
         const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
         const bool inside = px < width && py < height;
+        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
 
         float Tr = 1.0f, Z = 0.0f;
         float4 C[C4];
@@ -1613,57 +1694,30 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
         uint32_t* kept = half ? kept1 : kept0;
         unsigned n_out = 0;
         if (done_w != kFull) {   // else: nothing in this list can have an effect, and it is not even read
-            // ---- where the instances come from.  FIRST and PRODUCT filter the item's keys (loaded one step ahead of
-            // their use); REST blends the list PRODUCT compacted for this item (a superset of what is still alive at
-            // the true transmittance, see above), its ids loaded kIdsAhead batches ahead of their gather.
-            unsigned pos = rg.x;           // next key to load
-            bool loaded = false;
-            uint32_t kq[kFilterKeys], iq[kFilterKeys];
-            auto load_step = [&]() {
-#pragma unroll
-                for (int k = 0; k < kFilterKeys; ++k) {
-                    const unsigned idx = pos + 32u * k + lane;
-                    const bool ok = idx < rg.y;
-                    kq[k] = ok ? __ldg(inst_keys + idx) : 0xFFFFFFFFu;   // code 0xFF reaches nothing
-                    iq[k] = ok ? __ldg(inst_ids + idx) : 0u;
-                }
-                pos = min(pos + 32u * kFilterKeys, rg.y);
-                loaded = true;
-            };
-            unsigned q_head = 0, q_tail = 0;   // candidates [q_head, q_tail) wait for their gather
-            // (measured: a second filter step of keys in flight gains 10 % in the PRODUCT pass and loses as much in FIRST)
+            // ---- where the instances come from.  FIRST and PRODUCT filter the item's keys; REST blends the list PRODUCT
+            // compacted for this item (a superset of what is still alive at the true transmittance, see above), its ids
+            // loaded kIdsAhead batches ahead of their gather.
+            CandidateStream in;
+            const unsigned* reach = s_reach + 256 * half;
             auto fill = [&]() {
-                while (PASS != PASS_REST && q_tail - q_head < 32u && loaded) {
-                    uint32_t ck[kFilterKeys], ci[kFilterKeys];
-#pragma unroll
-                    for (int k = 0; k < kFilterKeys; ++k) { ck[k] = kq[k]; ci[k] = iq[k]; }
-                    loaded = false;
-                    if (pos < rg.y) load_step();
-#pragma unroll
-                    for (int k = 0; k < kFilterKeys; ++k) {
-                        const unsigned long long reach = s_reach[ck[k] >> kTileKeyBits];
-                        const bool keep = ((unsigned)(reach >> (32 * half)) & ~done_w) != 0u;
-                        const unsigned b = __ballot_sync(kFull, keep);
-                        if (keep) sm.queue[(q_tail + __popc(b & lt_mask)) & (kQueueCap - 1)] = ci[k];
-                        q_tail += __popc(b);
-                    }
-                }
+                if (PASS != PASS_REST) in.fill(reach, done_w, sm.queue, lane, lt_mask);
                 __syncwarp();
             };
             uint32_t idf[kIdsAhead];
             if (PASS == PASS_REST) {
-                q_tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
+                in.head = 0u;
+                in.tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
 #pragma unroll
-                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < q_tail ? kept[rg.x + 32u * k + lane] : 0u;
-            } else if (pos < rg.y) {
-                load_step();
+                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < in.tail ? kept[rg.x + 32u * k + lane] : 0u;
+            } else {
+                in.start(inst_keys, inst_ids, rg.x, rg.y, lane);
             }
             // the next (up to) 32 candidates become a batch: their records start to travel into `stage` of the ring
             auto gather = [&](unsigned stage) {
-                const unsigned n = min(32u, q_tail - q_head);
+                const unsigned n = min(32u, in.tail - in.head);
                 uint32_t id = kNoInstance;
                 if (lane < n) {
-                    id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(q_head + lane) & (kQueueCap - 1)]);
+                    id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(in.head + lane) & (kQueueCap - 1)]);
                     const float4* p = reinterpret_cast<const float4*>(rec) + (size_t)id * (ROWS ? 1 : 2);
                     async_copy_16(&sm.ring_a[stage][lane], p);
                     if (kBlend && !ROWS) async_copy_16(&sm.ring_f[stage][lane], p + 1);
@@ -1674,10 +1728,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                 if (PASS == PASS_REST) {
 #pragma unroll
                     for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
-                    const unsigned nxt = q_head + 32u * kIdsAhead + lane;
-                    idf[kIdsAhead - 1] = nxt < q_tail ? kept[rg.x + nxt] : 0u;
+                    const unsigned nxt = in.head + 32u * kIdsAhead + lane;
+                    idf[kIdsAhead - 1] = nxt < in.tail ? kept[rg.x + nxt] : 0u;
                 }
-                q_head += n;
+                in.head += n;
             };
             fill();
 #pragma unroll
@@ -1688,44 +1742,36 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
             for (unsigned batch = 0;; ++batch) {
                 gather((batch + kGatherDepth - 1) & (kGatherDepth - 1));
                 async_copy_wait<kGatherDepth - 1>();   // all but the newest kGatherDepth - 1 groups: this batch has arrived
-                if (ROWS) __syncwarp();                // a row was copied by several lanes
                 const unsigned stage = batch & (kGatherDepth - 1);
                 const uint32_t id_cur = sm.ring_id[stage][lane];
                 const bool staged = id_cur != kNoInstance;
                 if (__ballot_sync(kFull, staged) == 0u) break;   // batches are filled in order: nothing is left
-                const float4 a_cur = sm.ring_a[stage][lane];
-                fill();
-                // ---- lane j: the fragments of staged instance j
-                const int qx = __float2int_rd(a_cur.x - 0.5f) - px0;
-                const int qy = __float2int_rd(a_cur.y - 0.5f) - py0;
-                float al[4], wg[4];
-                int pix[4];
+                // ---- lane j: the pixels of staged instance j that have not stopped
+                const float4 own = sm.ring_a[stage][lane];
+                const unsigned pixels = staged ? footprint_pixels(own.x, own.y, px0, py0) & ~done_w : 0u;
+                if (kWeights) sm.weight[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+                fill();   // (its __syncwarp also shows every lane what the others have copied)
+                if (PASS == PASS_PRODUCT) {
+                    // A product does not care about order.  Its factors are added up as -log2(1 - alpha) in fixed
+                    // point (integer part and 26 fractional bits in two words per pixel, 32 of which fit a word): integer
+                    // atomics commute, so the sum is the same on every run, and none of the per-pixel ordering below is
+                    // needed.  (24 bits round a factor as coarsely as an fp32 product; on top of the rounding of 1 - alpha
+                    // that made the alpha of 200,000 splats of opacity 10^-6 twice as far off as a chain of products.)
+                    // An opacity below zero makes a factor above one: the integer part is signed.  A factor that is not a number
+                    // counts more than 32 others can, by which the pixel's product is known to be none either.
+                    const int qx = __float2int_rd(own.x - 0.5f) - px0, qy = __float2int_rd(own.y - 0.5f) - py0;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int cx = qx + (c & 1), cy = qy + (c >> 1);
-                    const float pcx = (float)(px0 + cx) + 0.5f, pcy = (float)(py0 + cy) + 0.5f;
-                    const float dx = fabsf(a_cur.x - pcx), dy = fabsf(a_cur.y - pcy);
-                    wg[c] = __saturatef(1.0f - dx) * __saturatef(1.0f - dy);
-                    al[c] = a_cur.z * wg[c];
-                    const int p = cy * 8 + cx;
-                    const bool ok = staged && cx >= 0 && cx < 8 && cy >= 0 && cy < 4 && dx < 1.0f && dy < 1.0f &&
-                                    !((done_w >> (p & 31)) & 1u);
-                    pix[c] = ok ? p : -1;
-                    if (PASS != PASS_PRODUCT) {
-                        if (ok) atomicOr(sm.mask + p, 1u << lane);
-                    } else if (ok) {
-                        // A product does not care about order.  Its factors are added up as -log2(1 - alpha) in fixed
-                        // point (integer part and 26 fractional bits in two words per pixel, 32 of which fit a word): integer
-                        // atomics commute, so the sum is the same on every run, and none of the per-pixel ordering below is
-                        // needed.  (24 bits round a factor as coarsely as an fp32 product; on top of the rounding of 1 - alpha
-                        // that made the alpha of 200,000 splats of opacity 10^-6 twice as far off as a chain of products.)
-                        // An opacity below zero makes a factor above one: the integer part is signed.  A factor that is not a number
-                        // counts more than 32 others can, by which the pixel's product is known to be none either.
-                        const float x = 1.0f - al[c];
-                        const float t = x > 0.0f ? fminf(-log2f(x), 64.0f) : x <= 0.0f ? 64.0f : kLogNaN;   // 2^-64: far below the threshold
-                        const float ti = floorf(t);
-                        atomicAdd(sm.mask + p, __float2uint_rn((t - ti) * kLogScale));
-                        if (ti != 0.0f) atomicAdd(sm.off + p, (unsigned)(int)ti);
+                    for (int c = 0; c < 4; ++c) {
+                        const int cx = qx + (c & 1), cy = qy + (c >> 1), p = cy * 8 + cx;
+                        const float dx = fabsf(own.x - ((float)(px0 + cx) + 0.5f)), dy = fabsf(own.y - ((float)(py0 + cy) + 0.5f));
+                        const float wg = __saturatef(1.0f - dx) * __saturatef(1.0f - dy);
+                        if ((unsigned)p < 32u && ((pixels >> (p & 31)) & 1u) && wg > 0.0f) {
+                            const float x = 1.0f - own.z * wg;
+                            const float t = x > 0.0f ? fminf(-log2f(x), 64.0f) : x <= 0.0f ? 64.0f : kLogNaN;   // 2^-64: far below the threshold
+                            const float ti = floorf(t);
+                            atomicAdd(&sm.sum[0][p], __float2uint_rn((t - ti) * kLogScale));
+                            if (ti != 0.0f) atomicAdd(&sm.sum[1][p], (unsigned)(int)ti);
+                        }
                     }
                 }
                 if (PASS == PASS_PRODUCT || kWeights) {   // inference keeps no lists for a backward pass
@@ -1734,17 +1780,16 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                     // transmittance; written in place, behind the part of PRODUCT's list already read) the backward
                     // pass's again.  The filter runs several batches ahead of the blend, so some of what it let
                     // through is dead by now and is dropped here.
-                    const bool live = (pix[0] & pix[1] & pix[2] & pix[3]) >= 0;
-                    const unsigned b = __ballot_sync(kFull, live);
-                    if (live) kept[rg.x + n_out + __popc(b & lt_mask)] = id_cur;
+                    const unsigned b = __ballot_sync(kFull, pixels != 0u);
+                    if (pixels) kept[rg.x + n_out + __popc(b & lt_mask)] = id_cur;
                     n_out += __popc(b);
                 }
-                __syncwarp();
                 if (PASS == PASS_PRODUCT) {
-                    const unsigned frac = sm.mask[lane], whole = sm.off[lane];
+                    __syncwarp();
+                    const unsigned frac = sm.sum[0][lane], whole = sm.sum[1][lane];
                     if (frac | whole) {
-                        sm.mask[lane] = 0u;
-                        sm.off[lane] = 0u;
+                        sm.sum[0][lane] = 0u;
+                        sm.sum[1][lane] = 0u;
                         log_sum += (int)whole < (int)(kLogNaN / 2.0f) ? (double)(int)whole + (double)frac * (1.0 / (double)kLogScale) : (double)NAN;
                     }
                     done = done || log_sum > log_stop;
@@ -1753,82 +1798,60 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                     if (done_w == kFull) break;   // every pixel has stopped: the rest of the list has no effect
                     continue;
                 }
-                // ---- per-pixel order: offset of every pixel's list, slot of every fragment
-                const unsigned my_mask = sm.mask[lane];
-                const unsigned cnt = __popc(my_mask);
-                const unsigned off = warp_inclusive_scan(cnt) - cnt;
-                sm.off[lane] = off;
-                __syncwarp();
-                int slot[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    slot[c] = 0;
-                    if (pix[c] >= 0) {
-                        slot[c] = (int)(sm.off[pix[c]] + __popc(sm.mask[pix[c]] & lt_mask));
-                        sm.frag[slot[c]] = make_float2(al[c], __uint_as_float(lane));
-                    }
-                }
-                __syncwarp();
-                // ---- every lane runs down the list of its own pixel, front to back
-                if (my_mask) sm.mask[lane] = 0u;
-                // The chain from one fragment to the next is one multiply (the transmittance); everything else of a step
-                // hangs off it.  The steps are therefore written without branches -- a stopped pixel selects its old
-                // values -- and in chunks whose loads are issued together, so that consecutive steps overlap in the
-                // pipeline instead of each waiting for its own shared-memory loads.
-                constexpr int kChunk = 4;
-                for (unsigned k0 = off; k0 < off + cnt; k0 += kChunk) {
-                    float a[kChunk];
+                // ---- every lane runs down the instances of its own pixel, front to back
+                unsigned todo = warp_transpose_bits(pixels, lane);
+                while (todo) {
+                    // A few at a time: what they load and the weights they form do not wait for one another, and the chain from one
+                    // fragment to the next is one multiply (the transmittance), everything else of a step hanging off it.  The steps
+                    // are written without branches: a stopped pixel selects its old values.
+                    constexpr int kChunk = C4 == 1 ? 3 : 2;
+                    int j[kChunk];
+                    float wg[kChunk], al[kChunk], zd[kChunk];
                     float4 f[kChunk];
-                    float zd[kChunk];
-                    unsigned from[kChunk];
+                    bool ok[kChunk];
 #pragma unroll
                     for (int u = 0; u < kChunk; ++u) {
-                        const unsigned k = min(k0 + u, off + cnt - 1u);   // the tail repeats the last slot: masked out below
-                        const float2 e = sm.frag[k];
-                        a[u] = e.x;
-                        from[u] = __float_as_uint(e.y);
-                        if (kBlend && C4 == 1) f[u] = sm.ring_f[stage][from[u]];
-                        if (kDepth) zd[u] = sm.ring_a[stage][from[u]].w;
+                        ok[u] = todo != 0u;
+                        j[u] = ok[u] ? __ffs(todo) - 1 : j[0];
+                        todo &= todo - 1u;
+                        const float4 a = sm.ring_a[stage][j[u]];
+                        if (C4 == 1) f[u] = sm.ring_f[stage][j[u]];
+                        wg[u] = __saturatef(1.0f - fabsf(a.x - pcx)) * __saturatef(1.0f - fabsf(a.y - pcy));
+                        al[u] = a.z * wg[u];
+                        zd[u] = a.w;
+                        ok[u] = ok[u] && wg[u] > 0.0f;
                     }
 #pragma unroll
                     for (int u = 0; u < kChunk; ++u) {
-                        const bool live = !done && k0 + u < off + cnt;
-                        if (kBlend) {
-                            const float bw = Tr * a[u];
-                            if (kWeights && k0 + u < off + cnt) sm.frag_seen[k0 + u] = live ? Tr : 0.0f;
-                            if (C4 == 1) {
-                                C[0].x = live ? C[0].x + bw * f[u].x : C[0].x;
-                                C[0].y = live ? C[0].y + bw * f[u].y : C[0].y;
-                                C[0].z = live ? C[0].z + bw * f[u].z : C[0].z;
-                                C[0].w = live ? C[0].w + bw * f[u].w : C[0].w;
-                            } else if (live) {
-                                // wide rows are read where they are used: a chunk of them would not fit the registers
-                                const float4* row = sm.ring_f[stage] + from[u] * kStride;
+                        const bool live = ok[u] && !done;
+                        const float bw = Tr * al[u];
+                        if (kWeights && live && bw > 0.0f) reinterpret_cast<float*>(sm.weight + j[u])[parity] = bw * wg[u];
+                        if (C4 == 1) {
+                            C[0].x = live ? C[0].x + bw * f[u].x : C[0].x;
+                            C[0].y = live ? C[0].y + bw * f[u].y : C[0].y;
+                            C[0].z = live ? C[0].z + bw * f[u].z : C[0].z;
+                            C[0].w = live ? C[0].w + bw * f[u].w : C[0].w;
+                        } else if (live) {
+                            // wide rows are read where they are used: a chunk of them would not fit the registers
+                            const float4* row = sm.ring_f[stage] + j[u] * kStride;
 #pragma unroll
-                                for (int c = 0; c < C4; ++c) {
-                                    const float4 v = row[c];
-                                    C[c].x += bw * v.x; C[c].y += bw * v.y; C[c].z += bw * v.z; C[c].w += bw * v.w;
-                                }
+                            for (int c = 0; c < C4; ++c) {
+                                const float4 v = row[c];
+                                C[c].x += bw * v.x; C[c].y += bw * v.y; C[c].z += bw * v.z; C[c].w += bw * v.w;
                             }
-                            if (kDepth) Z = live ? Z + bw * zd[u] : Z;
-                            Tr = live ? Tr * (1.0f - a[u]) : Tr;
-                            done = done || Tr < kTransmittanceEps;
                         }
+                        if (kDepth) Z = live ? Z + bw * zd[u] : Z;
+                        Tr = live ? Tr * (1.0f - al[u]) : Tr;
+                        done = done || Tr < kTransmittanceEps;
                     }
+                    if (done) todo = 0u;
                 }
                 __syncwarp();
                 if (kWeights) {
-                    // blending weight of every staged instance: its (up to) four fragments in fixed corner order
-                    if (staged) {
-                        float v[4];
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const float bw = pix[c] >= 0 ? sm.frag_seen[slot[c]] * al[c] : 0.0f;
-                            v[c] = bw > 0.0f ? bw * wg[c] : 0.0f;
-                        }
-                        const float sum = ((v[0] + v[1]) + v[2]) + v[3];
-                        if (sum > 0.0f) atomicAdd(blending_weights + id_cur, sum);
-                    }
+                    // blending weight of every staged instance: its (up to) four pixels in a fixed order
+                    const float4 v = sm.weight[lane];
+                    const float sum = ((v.x + v.y) + v.z) + v.w;
+                    if (sum > 0.0f) atomicAdd(blending_weights + id_cur, sum);
                 }
                 done_w = __ballot_sync(kFull, done);
                 __syncwarp();
@@ -2233,11 +2256,8 @@ struct __align__(16) RowsBackwardSmem {
     float4 ring_a[kGatherDepthBackward][32];
     float4 ring_f[kGatherDepthBackward][32 * feature_stride(C4)];
     float4 pixel_grad[32 * feature_stride(C4)];   // image gradient of the half's pixels
-    float2 frag[kBatchFragments];                 // fragments in per-pixel order: alpha, lane of the staged instance
-    float2 frag_out[kBatchFragments];             // ... and what the pixel lane made of them: blending weight, dL/dalpha
+    float4 out[32][2];                            // per staged instance and parity of the pixel: blending weight, opacity gradient
     uint32_t ring_id[kGatherDepthBackward][32];
-    unsigned mask[32];
-    unsigned off[32];
 };
 template <int C4>
 constexpr size_t rows_warp_backward_smem_bytes() { return kWarpBlendWarps * sizeof(RowsBackwardSmem<C4>); }
@@ -2256,10 +2276,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
     constexpr int kStride = feature_stride(C4);
     extern __shared__ __align__(16) unsigned char blend_smem[];
     const unsigned lane = lane_id();
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned parity = (lane & 1u) | ((lane >> 2) & 2u);   // of this lane's pixel: a footprint has each of the four once
     RowsBackwardSmem<C4>& sm = reinterpret_cast<RowsBackwardSmem<C4>*>(blend_smem)[threadIdx.x >> 5];
-    sm.mask[lane] = 0u;
-    __syncwarp();
     const unsigned n_first = __ldg(counts) * 2u;
     const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
     const unsigned n_rest = n_items - n_first;
@@ -2287,6 +2305,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
         const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
         const int px0 = tx * 8, py0 = ty * 8 + 4 * half;
         const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
 
         float4 g[C4];
         float G_final = 0.0f, G_run = 0.0f, K = 0.0f, Tr = 1.0f;
@@ -2343,82 +2362,54 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
         for (unsigned batch = 0;; ++batch) {
             gather((batch + kGatherDepth - 1) & (kGatherDepth - 1));
             async_copy_wait<kGatherDepth - 1>();
-            __syncwarp();   // a row was copied by several lanes
             const unsigned stage = batch & (kGatherDepth - 1);
             const uint32_t id_cur = sm.ring_id[stage][lane];
             const bool staged = id_cur != kNoInstance;
             if (__ballot_sync(kFull, staged) == 0u) break;
-            const float4 a_cur = sm.ring_a[stage][lane];
-            // ---- lane j: the fragments of staged instance j
-            const int qx = __float2int_rd(a_cur.x - 0.5f) - px0;
-            const int qy = __float2int_rd(a_cur.y - 0.5f) - py0;
-            float al[4], wg[4];
-            int pix[4];
+            // ---- lane j: the pixels of staged instance j that have not stopped
+            const float4 own = sm.ring_a[stage][lane];
+            const unsigned pixels = staged ? footprint_pixels(own.x, own.y, px0, py0) & ~done_w : 0u;
+            sm.out[lane][0] = sm.out[lane][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned todo = warp_transpose_bits(pixels, lane);
+            __syncwarp();   // every lane sees what the others have copied
+            // ---- every lane runs down the instances of its own pixel, front to back
+            while (todo) {
+                const int j = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const float4 a = sm.ring_a[stage][j];
+                const float wg = __saturatef(1.0f - fabsf(a.x - pcx)) * __saturatef(1.0f - fabsf(a.y - pcy));
+                if (!(wg > 0.0f)) continue;
+                const float4* row = sm.ring_f[stage] + j * kStride;
+                float fg = 0.0f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int cx = qx + (c & 1), cy = qy + (c >> 1);
-                const float pcx = (float)(px0 + cx) + 0.5f, pcy = (float)(py0 + cy) + 0.5f;
-                const float dx = fabsf(a_cur.x - pcx), dy = fabsf(a_cur.y - pcy);
-                wg[c] = __saturatef(1.0f - dx) * __saturatef(1.0f - dy);
-                al[c] = a_cur.z * wg[c];
-                const int p = cy * 8 + cx;
-                const bool ok = staged && cx >= 0 && cx < 8 && cy >= 0 && cy < 4 && dx < 1.0f && dy < 1.0f &&
-                                !((done_w >> (p & 31)) & 1u);
-                pix[c] = ok ? p : -1;
-                if (ok) atomicOr(sm.mask + p, 1u << lane);
-            }
-            __syncwarp();
-            const unsigned my_mask = sm.mask[lane];
-            const unsigned cnt = __popc(my_mask);
-            const unsigned off = warp_inclusive_scan(cnt) - cnt;
-            sm.off[lane] = off;
-            __syncwarp();
-            int slot[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                slot[c] = 0;
-                if (pix[c] >= 0) {
-                    slot[c] = (int)(sm.off[pix[c]] + __popc(sm.mask[pix[c]] & lt_mask));
-                    sm.frag[slot[c]] = make_float2(al[c], __uint_as_float(lane));
+                for (int c = 0; c < C4; ++c) {
+                    const float4 f = row[c];
+                    fg += f.x * g[c].x + f.y * g[c].y + f.z * g[c].z + f.w * g[c].w;
                 }
+                const float al = a.z * wg;
+                const float bw = Tr * al;
+                G_run += bw * fg;
+                const float oma = 1.0f - al;
+                const float rcp = 1.0f / fmaxf(oma, kOneMinusAlphaEps);
+                // (no feature gradient from a weight that is not positive: a negative opacity, or not a number)
+                reinterpret_cast<float2*>(sm.out[j])[parity] = make_float2(bw > 0.0f ? bw : 0.0f, (Tr * fg + (G_run - G_final) * rcp + K * rcp) * wg);
+                Tr *= oma;
+                done = Tr < kTransmittanceEps;
+                if (done) todo = 0u;
             }
             __syncwarp();
-            if (my_mask) sm.mask[lane] = 0u;
-            for (unsigned k = off; k < off + cnt; ++k) {
-                const float2 e = sm.frag[k];
-                float2 out = make_float2(0.0f, 0.0f);
-                if (!done) {
-                    const float4* row = sm.ring_f[stage] + __float_as_uint(e.y) * kStride;
-                    float fg = 0.0f;
-#pragma unroll
-                    for (int c = 0; c < C4; ++c) {
-                        const float4 f = row[c];
-                        fg += f.x * g[c].x + f.y * g[c].y + f.z * g[c].z + f.w * g[c].w;
-                    }
-                    const float bw = Tr * e.x;
-                    G_run += bw * fg;
-                    const float oma = 1.0f - e.x;
-                    const float rcp = 1.0f / fmaxf(oma, kOneMinusAlphaEps);
-                    // (no feature gradient from a weight that is not positive: a negative opacity, or not a number)
-                    out = make_float2(bw > 0.0f ? bw : 0.0f, Tr * fg + (G_run - G_final) * rcp + K * rcp);
-                    Tr *= oma;
-                    done = Tr < kTransmittanceEps;
-                }
-                sm.frag_out[k] = out;
-            }
-            __syncwarp();
-            if (staged) {
+            // ---- lane j: the sums of instance j over its (up to) four pixels, in fixed corner order
+            if (pixels) {
+                const int qx = __float2int_rd(own.x - 0.5f) - px0, qy = __float2int_rd(own.y - 0.5f) - py0;
+                const unsigned first_parity = ((unsigned)qx & 1u) | (((unsigned)qy & 1u) << 1);
                 float bw[4], so = 0.0f;
                 bool any = false;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    bw[c] = 0.0f;
-                    if (pix[c] >= 0) {
-                        const float2 o = sm.frag_out[slot[c]];
-                        bw[c] = o.x;
-                        so += o.y * wg[c];
-                        any = any || o.x != 0.0f;
-                    }
+                    const float2 o = reinterpret_cast<const float2*>(sm.out[lane])[first_parity ^ (unsigned)c];
+                    bw[c] = o.x;
+                    so += o.y;
+                    any = any || o.x != 0.0f;
                 }
                 const bool alone = qx >= 0 && qx < 7 && qy >= 0 && qy < 3;   // all four pixels in this half
                 if (any) {
@@ -2429,7 +2420,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             if (bw[q] != 0.0f) {
-                                const float4 v = sm.pixel_grad[pix[q] * kStride + c];
+                                const float4 v = sm.pixel_grad[((qy + (q >> 1)) * 8 + qx + (q & 1)) * kStride + c];
                                 sum.x += bw[q] * v.x; sum.y += bw[q] * v.y; sum.z += bw[q] * v.z; sum.w += bw[q] * v.w;
                             }
                         }
@@ -3139,18 +3130,6 @@ __device__ __forceinline__ unsigned long long cell_pixels(unsigned code) {
     return m;
 }
 
-// Bit l of lane k's word becomes bit k of lane l's word.
-__device__ __forceinline__ unsigned warp_transpose_bits(unsigned x, unsigned lane) {
-    unsigned m = 0x0000FFFFu;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        const unsigned y = __shfl_xor_sync(0xffffffffu, x, s);
-        x = (lane & (unsigned)s) ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y & m) << s);
-        m ^= m << (s >> 1);
-    }
-    return x;
-}
-
 // Pixels of the 8x4 half at (px0, py0) (bit = row * 8 + column) that a splat at `a` with conic `c` can reach: a superset of
 // those with  c.x dx^2 + 2 c.y dx dy + c.z dy^2 <= reach  (reach = -2 log threshold).
 __device__ __forceinline__ unsigned ellipse_pixels(const float4& a, const float4& c, float reach, int px0, int py0) {
@@ -3182,7 +3161,7 @@ struct __align__(16) GaussForwardSmem {
 };
 template <int PASS, int KIND>
 constexpr size_t gauss_forward_smem_bytes() {
-    return 256 * sizeof(unsigned long long) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN>);
+    return 2 * 256 * sizeof(unsigned) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN>);
 }
 
 template <int PASS, int KIND>
@@ -3199,11 +3178,15 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_f
     constexpr bool kDepth = kBlend && KIND == BLEND_INFER;
     using Smem = GaussForwardSmem<kBlend, kWeights>;
     extern __shared__ __align__(16) unsigned char blend_smem[];
-    unsigned long long* s_reach = reinterpret_cast<unsigned long long*>(blend_smem);     // key code -> pixels reached
-    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 256 * sizeof(unsigned long long))[threadIdx.x >> 5];
+    unsigned* s_reach = reinterpret_cast<unsigned*>(blend_smem);     // [half][key code] -> pixels of the half reached
+    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 2 * 256 * sizeof(unsigned))[threadIdx.x >> 5];
     const unsigned lane = lane_id();
     const unsigned lt_mask = (1u << lane) - 1u;
-    s_reach[threadIdx.x] = cell_pixels(threadIdx.x);
+    {
+        const unsigned long long m = cell_pixels(threadIdx.x);
+        s_reach[threadIdx.x] = (unsigned)m;
+        s_reach[256 + threadIdx.x] = (unsigned)(m >> 32);
+    }
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
     const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));   // see the bilinear kernel
@@ -3248,52 +3231,26 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_f
         uint32_t* kept = half ? kept1 : kept0;
         unsigned n_out = 0;
         if (done_w != kFull) {
-            unsigned pos = rg.x;           // next key to load
-            bool loaded = false;
-            uint32_t kq[kFilterKeys], iq[kFilterKeys];
-            auto load_step = [&]() {
-#pragma unroll
-                for (int k = 0; k < kFilterKeys; ++k) {
-                    const unsigned idx = pos + 32u * k + lane;
-                    const bool ok = idx < rg.y;
-                    kq[k] = ok ? __ldg(inst_keys + idx) : 0xFFFFFFFFu;   // code 0xFF reaches nothing
-                    iq[k] = ok ? __ldg(inst_ids + idx) : 0u;
-                }
-                pos = min(pos + 32u * kFilterKeys, rg.y);
-                loaded = true;
-            };
-            unsigned q_head = 0, q_tail = 0;   // candidates [q_head, q_tail) wait for their gather
+            CandidateStream in;
+            const unsigned* reach_of_key = s_reach + 256 * half;
             auto fill = [&]() {
-                while (PASS != PASS_REST && q_tail - q_head < 32u && loaded) {
-                    uint32_t ck[kFilterKeys], ci[kFilterKeys];
-#pragma unroll
-                    for (int k = 0; k < kFilterKeys; ++k) { ck[k] = kq[k]; ci[k] = iq[k]; }
-                    loaded = false;
-                    if (pos < rg.y) load_step();
-#pragma unroll
-                    for (int k = 0; k < kFilterKeys; ++k) {
-                        const unsigned long long cells = s_reach[ck[k] >> kTileKeyBits];
-                        const bool keep = ((unsigned)(cells >> (32 * half)) & ~done_w) != 0u;
-                        const unsigned b = __ballot_sync(kFull, keep);
-                        if (keep) sm.queue[(q_tail + __popc(b & lt_mask)) & (kQueueCap - 1)] = ci[k];
-                        q_tail += __popc(b);
-                    }
-                }
+                if (PASS != PASS_REST) in.fill(reach_of_key, done_w, sm.queue, lane, lt_mask);
                 __syncwarp();
             };
             uint32_t idf[kIdsAhead];
             if (PASS == PASS_REST) {
-                q_tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
+                in.head = 0u;
+                in.tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
 #pragma unroll
-                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < q_tail ? kept[rg.x + 32u * k + lane] : 0u;
-            } else if (pos < rg.y) {
-                load_step();
+                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < in.tail ? kept[rg.x + 32u * k + lane] : 0u;
+            } else {
+                in.start(inst_keys, inst_ids, rg.x, rg.y, lane);
             }
             auto gather = [&](unsigned stage) {
-                const unsigned n = min(32u, q_tail - q_head);
+                const unsigned n = min(32u, in.tail - in.head);
                 uint32_t id = kNoInstance;
                 if (lane < n) {
-                    id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(q_head + lane) & (kQueueCap - 1)]);
+                    id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(in.head + lane) & (kQueueCap - 1)]);
                     const float4* p = reinterpret_cast<const float4*>(rec + id);
                     async_copy_16(&sm.ring_a[stage][lane], p);
                     async_copy_16(&sm.ring_c[stage][lane], conic + id);
@@ -3304,10 +3261,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_f
                 if (PASS == PASS_REST) {
 #pragma unroll
                     for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
-                    const unsigned nxt = q_head + 32u * kIdsAhead + lane;
-                    idf[kIdsAhead - 1] = nxt < q_tail ? kept[rg.x + nxt] : 0u;
+                    const unsigned nxt = in.head + 32u * kIdsAhead + lane;
+                    idf[kIdsAhead - 1] = nxt < in.tail ? kept[rg.x + nxt] : 0u;
                 }
-                q_head += n;
+                in.head += n;
             };
             fill();
             gather(0u);
