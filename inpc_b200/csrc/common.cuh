@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdarg>
 #include <mutex>
+#include <utility>
 #include "../../include/inpc_b200.h"
 
 namespace inpc {
@@ -151,6 +152,33 @@ int opt_in_dynamic_smem(Kernel kernel, size_t bytes, bool (&done)[kMaxDevices]) 
 
 // ---- device helpers ------------------------------------------------------------------------
 #ifdef __CUDACC__
+// ---- launches that overlap the end of the kernel before them ------------------------------------------
+// Every kernel of the library is launched by `launch_chained` and starts with `await_previous_kernel()`.  The launch allows the
+// grid to be set up, and its blocks to be placed, as soon as all blocks of the kernel before it in the stream have left, without
+// waiting for that kernel's memory to be flushed and its completion to be reported; the wait returns when both are done.  A
+// kernel that waits has also waited for everything before the one it waits for, so nothing but the gap between two
+// launches changes.  No kernel may read or write global memory before the wait, and none may leave it out: a later one relies on it.
+// Measured against plain launches, 36 kernels one after the other: training step of 10^6 samples at 801x533 485 -> 418 us, of 2^23 at
+// 1237x822 1806 -> 1726, 2 * 10^6 gaussian splats 632 -> 580.  (With griddepcontrol.launch_dependents at the start of every kernel, so
+// that the next one's blocks are placed while it still runs: 454, 1738 and 588, since waiting blocks take room from running
+// ones; eight views on four streams 11318 -> 11464.)
+template <typename... KernelArgs, typename... Args>
+void launch_chained(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(std::forward<Args>(args))...);   // the launch check behind it reads the error
+}
+
+__device__ __forceinline__ void await_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 __device__ __forceinline__ unsigned warp_inclusive_scan(unsigned v) {

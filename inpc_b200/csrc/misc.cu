@@ -47,6 +47,7 @@ __device__ __forceinline__ float decay_factor(unsigned idx) {
 template <bool ADD>
 __global__ void __launch_bounds__(kThreads) weight_decay_kernel(const float* __restrict__ w, float* __restrict__ g, int64_t n,
                                                                 bool vec_ok) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t n4 = vec_ok ? n / 4 : 0;
@@ -71,6 +72,7 @@ __global__ void __launch_bounds__(kThreads) weight_decay_kernel(const float* __r
 
 // src/misc_kernels.cu:49-66
 __global__ void __launch_bounds__(kThreads) contraction_kernel(const float* __restrict__ p, float* __restrict__ out, int64_t n) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
         const float x = __ldg(p + 3 * i), y = __ldg(p + 3 * i + 1), z = __ldg(p + 3 * i + 2);
@@ -86,6 +88,7 @@ __global__ void __launch_bounds__(kThreads) contraction_kernel(const float* __re
 // fixed order, then one block adds the partials in index order.
 __global__ void __launch_bounds__(kThreads) cauchy_partial_kernel(const float* __restrict__ a, const float* __restrict__ b,
                                                                   int64_t n, float* __restrict__ partial) {
+    await_previous_kernel();
     __shared__ float s[kThreads / 32];
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     const float nf = (float)(unsigned)n;
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(kThreads) cauchy_partial_kernel(const float* _
 }
 
 __global__ void __launch_bounds__(1024) cauchy_final_kernel(const float* __restrict__ partial, int n_partial, float* __restrict__ loss) {
+    await_previous_kernel();
     __shared__ float s[32];
     float acc = 0.0f;
     for (int i = threadIdx.x; i < n_partial; i += 1024) acc += partial[i];
@@ -123,6 +127,7 @@ __global__ void __launch_bounds__(1024) cauchy_final_kernel(const float* __restr
 // src/misc_kernels.cu:81-94
 __global__ void __launch_bounds__(kThreads) cauchy_backward_kernel(const float* __restrict__ grad, const float* __restrict__ a,
                                                                    const float* __restrict__ b, int64_t n, float* __restrict__ out) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     const float g = __ldg(grad);
     const float nf = (float)(unsigned)n;
@@ -153,6 +158,7 @@ __device__ __forceinline__ uint2 cached_pair(const uint2* p) {
 
 __global__ void __launch_bounds__(kThreads) leaf_stats_kernel(const long long* __restrict__ indices, const float* __restrict__ weights,
                                                               int64_t n, int64_t n_leaves, uint2* __restrict__ stats) {
+    await_previous_kernel();
     // four samples per thread and round, their loads issued together: the kernel is bound by the latency of the
     // random reads of `stats`, not by bandwidth
     constexpr int kPer = 4;
@@ -187,6 +193,7 @@ __global__ void __launch_bounds__(kThreads) leaf_stats_kernel(const long long* _
 
 __global__ void __launch_bounds__(kThreads) leaf_update_kernel(float* __restrict__ leaf_weights, float* __restrict__ scores,
                                                                const uint2* __restrict__ stats, int64_t n_leaves, float decay) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x; l < n_leaves; l += stride) {
         const uint2 st = __ldg(stats + l);
@@ -205,6 +212,7 @@ __global__ void __launch_bounds__(kThreads) leaf_update_kernel(float* __restrict
 __global__ void __launch_bounds__(kThreads) compose_background_kernel(const float* __restrict__ image, const float* __restrict__ alpha,
                                                                       const float* __restrict__ background, int channels, int64_t n_px,
                                                                       float* __restrict__ out) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x; p < n_px; p += stride) {
         const float t = __fsub_rn(1.0f, __ldg(alpha + p));
@@ -220,6 +228,7 @@ __global__ void __launch_bounds__(kThreads) compose_background_backward_kernel(c
                                                                                const float* __restrict__ background, int channels,
                                                                                int64_t n_px, float* __restrict__ grad_alpha,
                                                                                float* __restrict__ grad_background) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x; p < n_px; p += stride) {
         const float t = 1.0f - __ldg(alpha + p);
@@ -240,6 +249,7 @@ __global__ void __launch_bounds__(kThreads) multisample_accumulate_kernel(float*
                                                                           float* __restrict__ acc_alpha, const float* __restrict__ image,
                                                                           const float* __restrict__ depth, const float* __restrict__ alpha,
                                                                           int channels, int64_t n_px, bool first, bool unpremultiply) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x; p < n_px; p += stride) {
         const float a = __ldg(alpha + p);
@@ -260,6 +270,7 @@ __global__ void __launch_bounds__(kThreads) multisample_resolve_kernel(float* __
                                                                        float* __restrict__ acc_alpha, float* __restrict__ alpha_sum,
                                                                        const float* __restrict__ background, int channels, int64_t n_px,
                                                                        float factor, bool remultiply) {
+    await_previous_kernel();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x; p < n_px; p += stride) {
         const float a_sum = acc_alpha[p];
@@ -290,8 +301,8 @@ extern "C" int inpc_weight_decay_grads(const float* weights, float* grads, int64
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     const bool vec_ok = ((reinterpret_cast<uintptr_t>(weights) | reinterpret_cast<uintptr_t>(grads)) & 15u) == 0;
     const int grid = grid_for(n / 4 + 1);
-    if (add) weight_decay_kernel<true><<<grid, kThreads, 0, stream>>>(weights, grads, n, vec_ok);
-    else weight_decay_kernel<false><<<grid, kThreads, 0, stream>>>(weights, grads, n, vec_ok);
+    if (add) launch_chained(weight_decay_kernel<true>, grid, kThreads, 0, stream, weights, grads, n, vec_ok);
+    else launch_chained(weight_decay_kernel<false>, grid, kThreads, 0, stream, weights, grads, n, vec_ok);
     INPC_LAUNCH_CHECK("weight_decay_kernel");
     return INPC_OK;
 }
@@ -299,7 +310,7 @@ extern "C" int inpc_weight_decay_grads(const float* weights, float* grads, int64
 extern "C" int inpc_spherical_contraction(const float* positions, float* out, int64_t n, void* stream_) {
     if (n == 0) return INPC_OK;
     if (n < 0 || !positions || !out) { set_error("inpc_spherical_contraction: bad argument"); return INPC_E_INVALID; }
-    contraction_kernel<<<grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(positions, out, n);
+    launch_chained(contraction_kernel, grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_), positions, out, n);
     INPC_LAUNCH_CHECK("contraction_kernel");
     return INPC_OK;
 }
@@ -311,9 +322,9 @@ extern "C" int inpc_cauchy_loss(const float* input, const float* target, int64_t
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     int grid = grid_for(n);
     if (grid > kCauchyMaxBlocks) grid = kCauchyMaxBlocks;
-    cauchy_partial_kernel<<<grid, kThreads, 0, stream>>>(input, target, n, static_cast<float*>(partials));
+    launch_chained(cauchy_partial_kernel, grid, kThreads, 0, stream, input, target, n, static_cast<float*>(partials));
     INPC_LAUNCH_CHECK("cauchy_partial_kernel");
-    cauchy_final_kernel<<<1, 1024, 0, stream>>>(static_cast<const float*>(partials), grid, loss);
+    launch_chained(cauchy_final_kernel, 1, 1024, 0, stream, static_cast<const float*>(partials), grid, loss);
     INPC_LAUNCH_CHECK("cauchy_final_kernel");
     return INPC_OK;
 }
@@ -322,7 +333,7 @@ extern "C" int inpc_cauchy_loss_backward(const float* grad, const float* input, 
                                          float* grad_input, void* stream_) {
     if (n == 0) return INPC_OK;
     if (n < 0 || n >= ((int64_t)1 << 32) || !grad || !input || !target || !grad_input) { set_error("inpc_cauchy_loss_backward: bad argument"); return INPC_E_INVALID; }
-    cauchy_backward_kernel<<<grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(grad, input, target, n, grad_input);
+    launch_chained(cauchy_backward_kernel, grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_), grad, input, target, n, grad_input);
     INPC_LAUNCH_CHECK("cauchy_backward_kernel");
     return INPC_OK;
 }
@@ -341,7 +352,7 @@ extern "C" int inpc_leaf_stats_accumulate(const int64_t* indices, const float* w
         set_error("inpc_leaf_stats_accumulate: bad argument");
         return INPC_E_INVALID;
     }
-    leaf_stats_kernel<<<grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(reinterpret_cast<const long long*>(indices), weights, n, n_leaves,
+    launch_chained(leaf_stats_kernel, grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_), reinterpret_cast<const long long*>(indices), weights, n, n_leaves,
                                                                                      reinterpret_cast<uint2*>(stats));
     INPC_LAUNCH_CHECK("leaf_stats_kernel");
     return INPC_OK;
@@ -362,7 +373,7 @@ extern "C" int inpc_leaf_update(float* leaf_weights, float* leaf_subdivision_sco
         set_error("inpc_leaf_update: bad argument");
         return INPC_E_INVALID;
     }
-    leaf_update_kernel<<<grid_for(n_leaves), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(leaf_weights, leaf_subdivision_scores,
+    launch_chained(leaf_update_kernel, grid_for(n_leaves), kThreads, 0, static_cast<cudaStream_t>(stream_), leaf_weights, leaf_subdivision_scores,
                                                                                              reinterpret_cast<const uint2*>(stats), n_leaves, decay);
     INPC_LAUNCH_CHECK("leaf_update_kernel");
     return INPC_OK;
@@ -372,7 +383,7 @@ extern "C" int inpc_compose_background(const float* image, const float* alpha, c
                                        float* out, void* stream_) {
     if (n_pixels == 0 || channels == 0) return INPC_OK;
     if (n_pixels < 0 || channels < 0 || !image || !alpha || !background || !out) { set_error("inpc_compose_background: bad argument"); return INPC_E_INVALID; }
-    compose_background_kernel<<<grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(image, alpha, background, channels, n_pixels, out);
+    launch_chained(compose_background_kernel, grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_), image, alpha, background, channels, n_pixels, out);
     INPC_LAUNCH_CHECK("compose_background_kernel");
     return INPC_OK;
 }
@@ -381,7 +392,7 @@ extern "C" int inpc_compose_background_backward(const float* grad_out, const flo
                                                 int64_t n_pixels, float* grad_alpha, float* grad_background, void* stream_) {
     if (n_pixels == 0 || channels == 0 || (!grad_alpha && !grad_background)) return INPC_OK;
     if (n_pixels < 0 || channels < 0 || !grad_out || !alpha || (grad_alpha && !background)) { set_error("inpc_compose_background_backward: bad argument"); return INPC_E_INVALID; }
-    compose_background_backward_kernel<<<grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(grad_out, alpha, background, channels,
+    launch_chained(compose_background_backward_kernel, grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_), grad_out, alpha, background, channels,
                                                                                                              n_pixels, grad_alpha, grad_background);
     INPC_LAUNCH_CHECK("compose_background_backward_kernel");
     return INPC_OK;
@@ -391,7 +402,7 @@ extern "C" int inpc_multisample_accumulate(float* acc_image, float* acc_depth, f
                                            const float* alpha, int channels, int64_t n_pixels, int first, int unpremultiply, void* stream_) {
     if (n_pixels == 0) return INPC_OK;
     if (n_pixels < 0 || channels < 0 || !acc_image || !acc_depth || !acc_alpha || !image || !depth || !alpha) { set_error("inpc_multisample_accumulate: bad argument"); return INPC_E_INVALID; }
-    multisample_accumulate_kernel<<<grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(acc_image, acc_depth, acc_alpha, image, depth, alpha,
+    launch_chained(multisample_accumulate_kernel, grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_), acc_image, acc_depth, acc_alpha, image, depth, alpha,
                                                                                                         channels, n_pixels, first != 0, unpremultiply != 0);
     INPC_LAUNCH_CHECK("multisample_accumulate_kernel");
     return INPC_OK;
@@ -403,7 +414,7 @@ extern "C" int inpc_multisample_resolve(float* acc_image, float* acc_depth, floa
     if (n_pixels < 0 || channels < 0 || n_multisamples < 1 || !acc_image || !acc_depth || !acc_alpha || !alpha_sum) { set_error("inpc_multisample_resolve: bad argument"); return INPC_E_INVALID; }
     // the factor is the double-precision 1/n rounded to float once, as a python float times an fp32 tensor is
     const float factor = (float)(1.0 / (double)n_multisamples);
-    multisample_resolve_kernel<<<grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(acc_image, acc_depth, acc_alpha, alpha_sum, background,
+    launch_chained(multisample_resolve_kernel, grid_for(n_pixels), kThreads, 0, static_cast<cudaStream_t>(stream_), acc_image, acc_depth, acc_alpha, alpha_sum, background,
                                                                                                      channels, n_pixels, factor, remultiply != 0);
     INPC_LAUNCH_CHECK("multisample_resolve_kernel");
     return INPC_OK;

@@ -30,6 +30,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kThreads) leaf_select_count_kernel(const float* __restrict__ values, const int32_t* __restrict__ levels,
                                                                      int64_t n, float threshold, int max_level,
                                                                      unsigned* __restrict__ block_sums) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kThreads / 32 + 1];
     const int64_t first = (int64_t)blockIdx.x * kChunk + (int64_t)threadIdx.x * kPerThread;
     unsigned c = 0;
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(kThreads) leaf_select_count_kernel(const float
 // Exclusive scan of the block sums in place by one block; the grand total goes to *total_out.
 __global__ void __launch_bounds__(kScanThreads) leaf_scan_sums_kernel(unsigned* __restrict__ sums, int64_t n_blocks,
                                                                       unsigned long long* __restrict__ total_out) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kScanThreads / 32 + 1];
     const int64_t per = ceil_div<int64_t>(n_blocks, kScanThreads);
     const int64_t lo = (int64_t)threadIdx.x * per, hi = min(n_blocks, lo + per);
@@ -85,6 +87,7 @@ template <int KIND>
 __global__ void __launch_bounds__(kThreads) leaf_fill_kernel(LeafArrays in, int64_t n, float threshold, int max_level, float initial_size,
                                                              const unsigned* __restrict__ block_offsets, int64_t n_selected,
                                                              LeafOutputs out) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kThreads / 32 + 1];
     const int64_t first = (int64_t)blockIdx.x * kChunk + (int64_t)threadIdx.x * kPerThread;
     bool sel[kPerThread];
@@ -161,12 +164,12 @@ extern "C" int inpc_leaf_select_count(int kind, const float* values, const int32
     unsigned* sums = static_cast<unsigned*>(workspace);
     const int64_t blocks = ceil_div<int64_t>(n, kChunk);
     if (kind == SELECT_PRUNE)
-        leaf_select_count_kernel<SELECT_PRUNE><<<(unsigned)blocks, kThreads, 0, stream>>>(values, levels, n, threshold, max_level, sums);
+        launch_chained(leaf_select_count_kernel<SELECT_PRUNE>, (unsigned)blocks, kThreads, 0, stream, values, levels, n, threshold, max_level, sums);
     else
-        leaf_select_count_kernel<SELECT_SUBDIVIDE><<<(unsigned)blocks, kThreads, 0, stream>>>(values, levels, n, threshold, max_level, sums);
+        launch_chained(leaf_select_count_kernel<SELECT_SUBDIVIDE>, (unsigned)blocks, kThreads, 0, stream, values, levels, n, threshold, max_level, sums);
     INPC_LAUNCH_CHECK("leaf_select_count_kernel");
     unsigned long long* total = total_slot(workspace, n);
-    leaf_scan_sums_kernel<<<1, kScanThreads, 0, stream>>>(sums, blocks, total);
+    launch_chained(leaf_scan_sums_kernel, 1, kScanThreads, 0, stream, sums, blocks, total);
     INPC_LAUNCH_CHECK("leaf_scan_sums_kernel");
     unsigned long long host = 0;
     INPC_CUDA_TRY(cudaMemcpyAsync(&host, total, sizeof(host), cudaMemcpyDeviceToHost, stream));
@@ -184,7 +187,7 @@ extern "C" int inpc_leaf_prune_fill(const float* centers, const int32_t* levels,
         return INPC_E_INVALID;
     }
     const int64_t blocks = ceil_div<int64_t>(n, kChunk);
-    leaf_fill_kernel<SELECT_PRUNE><<<(unsigned)blocks, kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(
+    launch_chained(leaf_fill_kernel<SELECT_PRUNE>, (unsigned)blocks, kThreads, 0, static_cast<cudaStream_t>(stream_),
         LeafArrays{centers, levels, weights, scores}, n, threshold, 0, 0.0f, static_cast<const unsigned*>(workspace), 0,
         LeafOutputs{out_centers, out_levels, out_weights, out_scores});
     INPC_LAUNCH_CHECK("leaf_fill_kernel");
@@ -201,7 +204,7 @@ extern "C" int inpc_leaf_subdivide_fill(const float* centers, const int32_t* lev
         return INPC_E_INVALID;
     }
     const int64_t blocks = ceil_div<int64_t>(n, kChunk);
-    leaf_fill_kernel<SELECT_SUBDIVIDE><<<(unsigned)blocks, kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(
+    launch_chained(leaf_fill_kernel<SELECT_SUBDIVIDE>, (unsigned)blocks, kThreads, 0, static_cast<cudaStream_t>(stream_),
         LeafArrays{centers, levels, weights, scores}, n, threshold, max_level, initial_size, static_cast<const unsigned*>(workspace), n_selected,
         LeafOutputs{out_centers, out_levels, out_weights, out_scores});
     INPC_LAUNCH_CHECK("leaf_fill_kernel");

@@ -50,6 +50,7 @@ constexpr int kHistItemsPerBlock = kHistThreads * 4 * 8;   // 8 uint4 loads per 
 __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
     const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, PassTable pt, unsigned* hist, unsigned* blocks_done,
     unsigned* __restrict__ base) {
+    await_previous_kernel();
     const int64_t n = n_dev ? (int64_t)*n_dev : n_arg;
     if ((int64_t)blockIdx.x * kHistItemsPerBlock >= n) return;
     __shared__ unsigned s_hist[kMaxPasses][kRadix];
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n_arg, const unsigned long long* __restrict__ n_dev,
     int shift, int bits_arg, const unsigned* __restrict__ digit_base, volatile unsigned* tile_state, unsigned* ticket,
     volatile unsigned* status, int spin_limit, unsigned mute_tile) {
+    await_previous_kernel();
     using Smem = PassSmem<BITS, ITEMS>;
     constexpr int kBins = Smem::kBins;
     constexpr unsigned kTile = kThreads * ITEMS;
@@ -349,7 +351,7 @@ int launch_onesweep_instance(const PassArgs& a, cudaStream_t stream) {
     const int rc = opt_in_dynamic_smem(radix_onesweep_pass_kernel<BITS, ITEMS>, kSmemBytes, attr_set);
     if (rc != INPC_OK) return rc;
     const int64_t resident = (int64_t)sm_count() * 2;
-    radix_onesweep_pass_kernel<BITS, ITEMS><<<(unsigned)(a.tiles < resident ? a.tiles : resident), kThreads, kSmemBytes, stream>>>(
+    launch_chained(radix_onesweep_pass_kernel<BITS, ITEMS>, (unsigned)(a.tiles < resident ? a.tiles : resident), kThreads, kSmemBytes, stream,
         a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base, a.state, a.ticket, a.status, a.spin_limit, a.mute_tile);
     INPC_LAUNCH_CHECK("radix_onesweep_pass_kernel");
     return INPC_OK;
@@ -439,7 +441,7 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
     if (!zeroed) INPC_CUDA_TRY(cudaMemsetAsync(workspace, 0, w.zero_bytes + state_words(tiles, end_bit) * sizeof(unsigned), stream));
 
     const int64_t hist_blocks = ceil_div<int64_t>(n, kHistItemsPerBlock), hist_cap = (int64_t)sm_count() * 4;
-    radix_histogram_kernel<<<(unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap), kHistThreads, 0, stream>>>(keys, n, n_dev, pt, w.hist, w.ticket + kMaxPasses, w.base);
+    launch_chained(radix_histogram_kernel, (unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap), kHistThreads, 0, stream, keys, n, n_dev, pt, w.hist, w.ticket + kMaxPasses, w.base);
     INPC_LAUNCH_CHECK("radix_histogram_kernel");
 
     PassArgs a;

@@ -191,6 +191,7 @@ struct ClearList {
     }
 };
 __global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearList list) {
+    await_previous_kernel();
     const size_t tid = (size_t)blockIdx.x * 256 + threadIdx.x, stride = (size_t)gridDim.x * 256;
     for (int r = 0; r < list.count; ++r) {
         char* p = static_cast<char*>(list.ptr[r]);
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(kPreThreads, 4) visibility_count_kernel(
     const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_chunks, unsigned* __restrict__ block_visible,
     unsigned* group_visible, unsigned long long* instances, unsigned* range, unsigned* done, unsigned fixed_lo, unsigned fixed_hi,
     unsigned* __restrict__ depth_min, unsigned* __restrict__ depth_max, unsigned long long* __restrict__ counters) {
+    await_previous_kernel();
     constexpr int kPerThread = 4;
     constexpr unsigned kStep = 32 * kPerThread;        // points of a warp and step
     static_assert(kPreThreads == 2 * kStep, "a chunk is two steps");
@@ -421,6 +423,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     const unsigned* __restrict__ depth_max, PointRec* __restrict__ rec, uint2* __restrict__ bounds, uint32_t* __restrict__ quad,
     float4* __restrict__ conic, uint4* __restrict__ foot, uint32_t* __restrict__ depth_keys,
     uint32_t* __restrict__ point_ids, int pack_count, int rec_stride, volatile unsigned* status) {
+    await_previous_kernel();
     constexpr int kHalves = VARIANT == VAR_RAW37 ? 37 : 36;
     constexpr int kSlabBytes = VARIANT == VAR_ROWS ? 16 : kPreThreads * kHalves * 2;   // multiple of 16 for both layouts
     __shared__ __align__(16) unsigned char s_feat[kSlabBytes];
@@ -543,6 +546,7 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
                                                                           const uint2* __restrict__ bounds, int64_t n_visible_arg,
                                                                           const unsigned long long* __restrict__ n_visible_dev,
                                                                           unsigned* block_sums, unsigned n_groups, unsigned* done) {
+    await_previous_kernel();
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     // a block of kInstThreads / 4 threads covers kInstThreads points, four consecutive ones per thread
     // (one 16-byte load when the keys carry the count), and takes several such groups one after the other
@@ -616,6 +620,7 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
                                                                       const unsigned* __restrict__ block_base, int gw,
                                                                       uint32_t* __restrict__ inst_keys,
                                                                       uint32_t* __restrict__ inst_ids) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kInstThreads / 32 + 1];
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     if ((int64_t)blockIdx.x * kInstThreads >= n_visible) return;
@@ -672,6 +677,7 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
 __global__ void __launch_bounds__(256) tile_ranges_kernel(const uint32_t* __restrict__ keys, int64_t n_instances_arg,
                                                           const unsigned long long* __restrict__ n_instances_dev,
                                                           uint2* __restrict__ ranges) {
+    await_previous_kernel();
     constexpr int kPer = 8;   // two 16-byte loads per thread (the key array is 256-byte aligned)
     const int64_t n_instances = n_instances_dev ? (int64_t)*n_instances_dev : n_instances_arg;
     // the grid fits the chip: sized for the bound on the instance count it was three quarters empty blocks
@@ -741,6 +747,7 @@ __device__ __forceinline__ unsigned segment_length(unsigned len, unsigned batch)
 __global__ void __launch_bounds__(kScanThreads) count_segments_kernel(const uint2* __restrict__ ranges, int n_tiles, int batch,
                                                                       uint32_t* __restrict__ tile_first,
                                                                       uint32_t* __restrict__ n_segments) {
+    await_previous_kernel();
     // four consecutive tiles per thread: short serial chains, two 16-byte loads
     constexpr int kItems = 4;
     __shared__ unsigned s_scan[kScanThreads / 32 + 1];
@@ -774,6 +781,7 @@ __global__ void __launch_bounds__(kScanThreads) count_segments_kernel(const uint
 // One thread per tile writes the tile's segment records.
 __global__ void __launch_bounds__(256) emit_segments_kernel(const uint2* __restrict__ ranges, int n_tiles, int batch,
                                                             const uint32_t* __restrict__ tile_first, Segment* __restrict__ segs) {
+    await_previous_kernel();
     const int t = blockIdx.x * 256 + threadIdx.x;
     if (t >= n_tiles) return;
     const uint2 r = ranges[t];
@@ -871,6 +879,7 @@ template <int T, int IPT>
 __global__ void __launch_bounds__(T * T) blend_bilinear_transmittance_kernel(
     const Segment* __restrict__ segs, const uint32_t* __restrict__ n_segments, const uint32_t* __restrict__ inst_ids,
     const PointRec* __restrict__ rec, float* __restrict__ seg_T, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     constexpr int B = P * IPT;
     constexpr int WORDS = B / 32;
@@ -924,6 +933,7 @@ __global__ void __launch_bounds__(T * T) blend_bilinear_transmittance_kernel(
 template <int T>
 __global__ void __launch_bounds__(T * T) blend_prefix_kernel(const Segment* __restrict__ segs, const uint32_t* __restrict__ tile_first,
                                                              float* __restrict__ seg_T) {
+    await_previous_kernel();
     constexpr int P = T * T;
     const unsigned first = tile_first[blockIdx.x];
     const unsigned n_seg = segs[first].info >> 16;
@@ -952,6 +962,7 @@ __global__ void __launch_bounds__(T * T) blend_bilinear_forward_kernel(
     const PointRec* __restrict__ rec, float* __restrict__ seg_T, float4* __restrict__ seg_C, float* __restrict__ seg_Z,
     float* __restrict__ image, float* __restrict__ depth_image, float* __restrict__ alpha_image,
     float* __restrict__ blending_weights, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     constexpr int B = P * IPT;
     constexpr int WORDS = B / 32;
@@ -1077,6 +1088,7 @@ __global__ void __launch_bounds__(T * T) blend_combine_kernel(const Segment* __r
                                                               const float* __restrict__ seg_T, float* __restrict__ image,
                                                               float* __restrict__ depth_image, float* __restrict__ alpha_image,
                                                               int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     const unsigned first = tile_first[blockIdx.x];
     const unsigned n_seg = segs[first].info >> 16;
@@ -1135,6 +1147,7 @@ __global__ void __launch_bounds__(T * T) blend_bilinear_backward_kernel(
     const float* __restrict__ grad_image, const float* __restrict__ grad_alpha, const float* __restrict__ image,
     const float* __restrict__ alpha_image, float4* __restrict__ grad_feat_view, float* __restrict__ grad_opacity,
     int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     constexpr int B = P * IPT;
     constexpr int WORDS = B / 32;
@@ -1384,6 +1397,7 @@ __device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ran
 __global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, unsigned long long n_instances_arg,
                                                                         const unsigned long long* __restrict__ n_instances_dev, uint2* block_sums, unsigned* done,
                                                                         uint32_t* __restrict__ counts) {
+    await_previous_kernel();
     __shared__ unsigned s_seg[kItemThreads / 32], s_tiles[kItemThreads / 32];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
@@ -1442,6 +1456,7 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
                                                                       const unsigned long long* __restrict__ n_instances_dev,
                                                                       const uint2* __restrict__ block_base, WarpItem* __restrict__ items0,
                                                                       WarpItem* __restrict__ items1) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kItemThreads / 32 + 1];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
@@ -1616,6 +1631,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
     float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1,
     uint32_t* __restrict__ n_kept, int width, int height, int gw, int gh) {
+    await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     constexpr bool kBlend = PASS != PASS_PRODUCT;               // colours and weights; PRODUCT only multiplies
@@ -1908,6 +1924,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
 // the transmittance at its start = (state behind segment 0) * product of the segments 1 .. s-1.
 __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel(const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts,
                                                                                  float* __restrict__ seg_T) {
+    await_previous_kernel();
     const unsigned lane = lane_id();
     const unsigned n_parts = __ldg(counts) * 2u;
     for (unsigned w = blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5); w < n_parts; w += gridDim.x * kWarpBlendWarps) {
@@ -1943,6 +1960,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
     const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts, float4* __restrict__ seg_C, const float* __restrict__ seg_Z,
     const float* __restrict__ seg_E,
     float* __restrict__ image, float* __restrict__ depth_image, float* __restrict__ alpha_image, int width, int height, int gw, int gh) {
+    await_previous_kernel();
     const unsigned lane = lane_id();
     const unsigned n_parts = __ldg(counts) * 2u;
     // a warp takes one group of four channels of a tile half
@@ -2040,6 +2058,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
     const float* __restrict__ seg_T, const float4* __restrict__ seg_C, const float* __restrict__ grad_image,
     const float* __restrict__ grad_alpha, const float* __restrict__ image, const float* __restrict__ alpha_image,
     float4* __restrict__ slot_grad, unsigned* __restrict__ slot_mask, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     constexpr int kGatherDepth = kGatherDepthBackward;
@@ -2270,6 +2289,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
     const float* __restrict__ seg_T, const float4* __restrict__ seg_C, const float* __restrict__ grad_image,
     const float* __restrict__ grad_alpha, const float* __restrict__ image, const float* __restrict__ alpha_image,
     float4* __restrict__ grad_rows, float* __restrict__ grad_opacity, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     constexpr int kGatherDepth = kGatherDepthBackward;
@@ -2461,6 +2481,7 @@ __global__ void __launch_bounds__(T * T) blend_rows_forward_kernel(
     const PointRec* __restrict__ rec, const float4* __restrict__ features, float* __restrict__ seg_T,
     float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     constexpr int WORDS = P / 32;
     if (blockIdx.x >= *n_segments) return;
@@ -2580,6 +2601,7 @@ __global__ void __launch_bounds__(T * T) blend_rows_combine_kernel(const Segment
                                                                    const float* __restrict__ seg_T, float* __restrict__ image,
                                                                    float* __restrict__ depth_image, float* __restrict__ alpha_image,
                                                                    int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     const unsigned first = tile_first[blockIdx.x];
     const unsigned n_seg = segs[first].info >> 16;
@@ -2641,6 +2663,7 @@ __global__ void __launch_bounds__(T * T) blend_rows_backward_kernel(
     const float4* __restrict__ seg_C, const float* __restrict__ grad_image, const float* __restrict__ grad_alpha,
     const float* __restrict__ image, const float* __restrict__ alpha_image, float4* __restrict__ grad_features,
     float* __restrict__ grad_opacity, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int P = T * T;
     constexpr int WORDS = P / 32;
     if (blockIdx.x >= *n_segments) return;
@@ -2821,6 +2844,7 @@ __global__ void __launch_bounds__(T * T) blend_gaussian_transmittance_kernel(
     const Segment* __restrict__ segs, const uint32_t* __restrict__ n_segments, const uint32_t* __restrict__ inst_ids,
     const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T, int width, int height, int gw,
     float threshold, float neg_log_threshold) {
+    await_previous_kernel();
     constexpr int B = T * T;
     constexpr int WORDS = B / 32;
     if (blockIdx.x >= *n_segments) return;
@@ -2880,6 +2904,7 @@ __global__ void __launch_bounds__(T * T) blend_gaussian_forward_kernel(
     float* __restrict__ seg_Z, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, int width, int height, int gw,
     float threshold, float neg_log_threshold) {
+    await_previous_kernel();
     constexpr int B = T * T;
     constexpr int WORDS = B / 32;
     if (blockIdx.x >= *n_segments) return;
@@ -2992,6 +3017,7 @@ __global__ void __launch_bounds__(T * T) blend_gaussian_backward_kernel(
     const float4* __restrict__ seg_C, const float* __restrict__ grad_image, const float* __restrict__ grad_alpha,
     const float* __restrict__ image, const float* __restrict__ alpha_image, float4* __restrict__ grad_feat_view,
     float* __restrict__ grad_opacity, int width, int height, int gw) {
+    await_previous_kernel();
     constexpr int B = T * T;
     constexpr int WORDS = B / 32;
     if (blockIdx.x >= *n_segments) return;
@@ -3171,6 +3197,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_f
     float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
     int width, int height, int gw, float threshold, float reach) {
+    await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     constexpr bool kBlend = PASS != PASS_PRODUCT;
@@ -3395,6 +3422,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_b
     const float* __restrict__ grad_image, const float* __restrict__ grad_alpha, const float* __restrict__ image,
     const float* __restrict__ alpha_image, float4* __restrict__ grad_feat_view, float* __restrict__ grad_opacity, int width, int height, int gw,
     float reach) {
+    await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char blend_smem[];
@@ -3551,6 +3579,7 @@ __global__ void __launch_bounds__(kPreThreads, 8) preprocess_backward_kernel(
     const float* __restrict__ positions, const float* __restrict__ cam, const uint2* __restrict__ bounds,
     const float4* __restrict__ grad_feat_view, GradientSlots slots, float* __restrict__ grad_opacities,
     __half* __restrict__ grad_features, int64_t n, bool bulk_ok) {
+    await_previous_kernel();
     __shared__ __align__(16) __half s_out[kPreThreads * 36];
     const int64_t block_first = (int64_t)blockIdx.x * kPreThreads;
     const int in_block = (int)min((int64_t)kPreThreads, n - block_first);
@@ -3847,7 +3876,7 @@ int launch_clear(const ClearList& list, cudaStream_t stream) {
     size_t total = 0;
     for (int k = 0; k < list.count; ++k) total += list.bytes[k];
     const size_t blocks = ceil_div<size_t>(total, 256 * 16 * 4), cap = (size_t)sm_count() * 8;
-    clear_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks < cap ? blocks : cap), 256, 0, stream>>>(list);
+    launch_chained(clear_kernel, (unsigned)(blocks < 1 ? 1 : blocks < cap ? blocks : cap), 256, 0, stream, list);
     INPC_LAUNCH_CHECK("clear_kernel");
     return INPC_OK;
 }
@@ -3948,10 +3977,10 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             const unsigned count_grid = (unsigned)(count_blocks < count_cap ? count_blocks : count_cap);
             unsigned long long* instances = reinterpret_cast<unsigned long long*>(pb.state + 8);
             if (deferred)
-                visibility_count_kernel<MODE, VARIANT, false><<<count_grid, kPreThreads, 0, stream>>>(
+                launch_chained(visibility_count_kernel<MODE, VARIANT, false>, count_grid, kPreThreads, 0, stream,
                     ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, instances, nullptr, pb.state + 2, lo_bits, hi_bits, pb.depth_min, pb.depth_max, pb.counters);
             else
-                visibility_count_kernel<MODE, VARIANT, true><<<count_grid, kPreThreads, 0, stream>>>(
+                launch_chained(visibility_count_kernel<MODE, VARIANT, true>, count_grid, kPreThreads, 0, stream,
                     ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, instances, pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min, pb.depth_max, pb.counters);
             INPC_LAUNCH_CHECK("visibility_count_kernel");
             if (!deferred) {
@@ -3959,7 +3988,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                 INPC_CUDA_TRY(cudaEventRecord(ready, stream));
             }
             // the projection pass needs nothing from the host: it runs while the host waits for the counters
-            preprocess_kernel<MODE, VARIANT><<<(unsigned)nb, kPreThreads, 0, stream>>>(
+            launch_chained(preprocess_kernel<MODE, VARIANT>, (unsigned)nb, kPreThreads, 0, stream,
                 ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max,
                 pb.rec, pb.bounds, pb.quad, pb.conic, pb.foot, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
             INPC_LAUNCH_CHECK("preprocess_kernel");
@@ -4012,16 +4041,16 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles rides in the top key bits when the depth offsets left them free
             if (MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift)
-                instance_count_kernel<true><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
+                launch_chained(instance_count_kernel<true>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             else
-                instance_count_kernel<false><<<count_blocks, kInstThreads / 4, 0, stream>>>(pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
+                launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (warp_blend && MODE == INPC_MODE_GAUSSIAN)
-                emit_instances_kernel<EMIT_CELLS><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, pb.foot, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                launch_chained(emit_instances_kernel<EMIT_CELLS>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, nullptr, pb.foot, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             else if (warp_blend)
-                emit_instances_kernel<EMIT_QUAD><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, pb.quad, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                launch_chained(emit_instances_kernel<EMIT_QUAD>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.quad, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             else
-                emit_instances_kernel<EMIT_BOUNDS><<<(unsigned)ibk, kInstThreads, 0, stream>>>(sorted_ids, pb.bounds, nullptr, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+                launch_chained(emit_instances_kernel<EMIT_BOUNDS>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, nullptr, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             INPC_LAUNCH_CHECK("emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
@@ -4030,22 +4059,22 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                       : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
         if (rc != INPC_OK) return rc;
         const int64_t range_blocks = ceil_div<int64_t>(n_instances, 256 * 8), range_cap = (int64_t)sm_count() * 8;
-        tile_ranges_kernel<<<(unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream>>>(ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
+        launch_chained(tile_ranges_kernel, (unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream, ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
         INPC_LAUNCH_CHECK("tile_ranges_kernel");
     }
     if (warp_blend) {
         StageScope scope(STAGE_SORT_TILE, stream);
         const int item_blocks = ceil_div(n_tiles, kItemTilesPerBlock);
         uint2* item_sums = reinterpret_cast<uint2*>(ib.tile_rank);
-        warp_items_count_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
+        launch_chained(warp_items_count_kernel, item_blocks, kItemThreads, 0, stream, ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
         INPC_LAUNCH_CHECK("warp_items_count_kernel");
-        warp_items_fill_kernel<<<item_blocks, kItemThreads, 0, stream>>>(ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
+        launch_chained(warp_items_fill_kernel, item_blocks, kItemThreads, 0, stream, ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
         INPC_LAUNCH_CHECK("warp_items_fill_kernel");
     } else {
         StageScope scope(STAGE_SORT_TILE, stream);
-        count_segments_kernel<<<1, kScanThreads, 0, stream>>>(ib.ranges, n_tiles, blend_batch(rp.tile), ib.tile_first, ib.n_segments);
+        launch_chained(count_segments_kernel, 1, kScanThreads, 0, stream, ib.ranges, n_tiles, blend_batch(rp.tile), ib.tile_first, ib.n_segments);
         INPC_LAUNCH_CHECK("count_segments_kernel");
-        emit_segments_kernel<<<ceil_div(n_tiles, 256), 256, 0, stream>>>(ib.ranges, n_tiles, blend_batch(rp.tile), ib.tile_first, ib.segs);
+        launch_chained(emit_segments_kernel, ceil_div(n_tiles, 256), 256, 0, stream, ib.ranges, n_tiles, blend_batch(rp.tile), ib.tile_first, ib.segs);
         INPC_LAUNCH_CHECK("emit_segments_kernel");
     }
     st->point_blob = pblob;
@@ -4112,7 +4141,7 @@ int launch_warp_forward_pass(unsigned grid, const WarpItem* items, const uint32_
     constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
     const int rc = opt_in_dynamic_smem(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
+    launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, grid, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, a.gh);
     INPC_LAUNCH_CHECK("blend_bilinear_warp_forward_kernel");
@@ -4139,11 +4168,11 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     if (rc_pass != INPC_OK) return rc_pass;
     rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    warp_blend_prefix_kernel<<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_T);
+    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
     rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    warp_blend_combine_kernel<KIND, C4><<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E,
+    launch_chained(warp_blend_combine_kernel<KIND, C4>, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E,
                                                                       image, depth, alpha, W, H, rp.gw, rp.gh);
     INPC_LAUNCH_CHECK("warp_blend_combine_kernel");
     return INPC_OK;
@@ -4158,7 +4187,7 @@ int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, c
     static bool attr_set[kMaxDevices] = {false};
     const int rc_attr = opt_in_dynamic_smem(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, attr_set);
     if (rc_attr != INPC_OK) return rc_attr;
-    blend_bilinear_warp_backward_kernel<<<grid, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream>>>(
+    launch_chained(blend_bilinear_warp_backward_kernel, grid, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
         ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, rp.v.width, rp.v.height, rp.gw);
     INPC_LAUNCH_CHECK("blend_bilinear_warp_backward_kernel");
@@ -4172,14 +4201,14 @@ int launch_bilinear_forward(const RasterParams& rp, const PointBlob& pb, const I
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const int W = rp.v.width, H = rp.v.height;
     const unsigned grid = (unsigned)ib.max_segments;
-    blend_bilinear_transmittance_kernel<T, IPT><<<grid, T * T, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, W, H, rp.gw);
+    launch_chained(blend_bilinear_transmittance_kernel<T, IPT>, grid, T * T, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_bilinear_transmittance_kernel");
-    blend_prefix_kernel<T><<<n_tiles, T * T, 0, stream>>>(ib.segs, ib.tile_first, ib.seg_T);
+    launch_chained(blend_prefix_kernel<T>, n_tiles, T * T, 0, stream, ib.segs, ib.tile_first, ib.seg_T);
     INPC_LAUNCH_CHECK("blend_prefix_kernel");
-    blend_bilinear_forward_kernel<T, IPT, KIND><<<grid, T * T, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, ib.seg_C, ib.seg_Z,
+    launch_chained(blend_bilinear_forward_kernel<T, IPT, KIND>, grid, T * T, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, ib.seg_C, ib.seg_Z,
                                                                            image, depth, alpha, blending_weights, W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_bilinear_forward_kernel");
-    blend_combine_kernel<T, KIND><<<n_tiles, T * T, 0, stream>>>(ib.segs, ib.tile_first, ib.seg_C, ib.seg_Z, ib.seg_T, image, depth, alpha,
+    launch_chained(blend_combine_kernel<T, KIND>, n_tiles, T * T, 0, stream, ib.segs, ib.tile_first, ib.seg_C, ib.seg_Z, ib.seg_T, image, depth, alpha,
                                                                 W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_combine_kernel");
     return INPC_OK;
@@ -4196,7 +4225,7 @@ int launch_bilinear_backward(const RasterParams& rp, const PointBlob& pb, const 
         const int rc_attr = opt_in_dynamic_smem(blend_bilinear_backward_kernel<T, IPT>, smem, attr_set);
         if (rc_attr != INPC_OK) return rc_attr;
     }
-    blend_bilinear_backward_kernel<T, IPT><<<(unsigned)ib.max_segments, T * T, smem, stream>>>(
+    launch_chained(blend_bilinear_backward_kernel<T, IPT>, (unsigned)ib.max_segments, T * T, smem, stream,
         ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities,
         rp.v.width, rp.v.height, rp.gw);
     INPC_LAUNCH_CHECK("blend_bilinear_backward_kernel");
@@ -4210,7 +4239,7 @@ int launch_gaussian_warp_forward_pass(unsigned grid, const WarpItem* items, cons
     constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
     const int rc = opt_in_dynamic_smem(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    blend_gaussian_warp_forward_kernel<PASS, KIND><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
+    launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, threshold, reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_forward_kernel");
@@ -4231,11 +4260,11 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     if (rc != INPC_OK) return rc;
     rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    warp_blend_prefix_kernel<<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_T);
+    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
     rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    warp_blend_combine_kernel<KIND, 1><<<grid, threads, 0, stream>>>(ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
+    launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
                                                                      rp.gw, rp.gh);
     INPC_LAUNCH_CHECK("warp_blend_combine_kernel");
     return INPC_OK;
@@ -4250,7 +4279,7 @@ int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, c
     static bool attr_set[kMaxDevices] = {false};
     const int rc_attr = opt_in_dynamic_smem(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, attr_set);
     if (rc_attr != INPC_OK) return rc_attr;
-    blend_gaussian_warp_backward_kernel<<<grid, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream>>>(
+    launch_chained(blend_gaussian_warp_backward_kernel, grid, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
         grad_image, grad_alpha, image, alpha, gfv, grad_opacities, rp.v.width, rp.v.height, rp.gw, rp.reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_backward_kernel");
@@ -4264,15 +4293,15 @@ int launch_gaussian_forward(const RasterParams& rp, const PointBlob& pb, const I
     const int W = rp.v.width, H = rp.v.height;
     const unsigned grid = (unsigned)ib.max_segments;
     const float neg_log_threshold = -logf(threshold);
-    blend_gaussian_transmittance_kernel<T, KIND == BLEND_INFER><<<grid, T * T, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, W, H,
+    launch_chained(blend_gaussian_transmittance_kernel<T, KIND == BLEND_INFER>, grid, T * T, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, W, H,
                                                                                           rp.gw, threshold, neg_log_threshold);
     INPC_LAUNCH_CHECK("blend_gaussian_transmittance_kernel");
-    blend_prefix_kernel<T><<<n_tiles, T * T, 0, stream>>>(ib.segs, ib.tile_first, ib.seg_T);
+    launch_chained(blend_prefix_kernel<T>, n_tiles, T * T, 0, stream, ib.segs, ib.tile_first, ib.seg_T);
     INPC_LAUNCH_CHECK("blend_prefix_kernel");
-    blend_gaussian_forward_kernel<T, KIND><<<grid, T * T, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, ib.seg_Z, image,
+    launch_chained(blend_gaussian_forward_kernel<T, KIND>, grid, T * T, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, ib.seg_Z, image,
                                                                       depth, alpha, blending_weights, W, H, rp.gw, threshold, neg_log_threshold);
     INPC_LAUNCH_CHECK("blend_gaussian_forward_kernel");
-    blend_combine_kernel<T, KIND><<<n_tiles, T * T, 0, stream>>>(ib.segs, ib.tile_first, ib.seg_C, ib.seg_Z, ib.seg_T, image, depth, alpha, W, H, rp.gw);
+    launch_chained(blend_combine_kernel<T, KIND>, n_tiles, T * T, 0, stream, ib.segs, ib.tile_first, ib.seg_C, ib.seg_Z, ib.seg_T, image, depth, alpha, W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_combine_kernel");
     return INPC_OK;
 }
@@ -4306,14 +4335,14 @@ int launch_rows_forward(const RasterParams& rp, const PointBlob& pb, const Insta
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const int W = rp.v.width, H = rp.v.height;
     const unsigned grid = (unsigned)ib.max_segments;
-    blend_bilinear_transmittance_kernel<T, 1><<<grid, T * T, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, W, H, rp.gw);
+    launch_chained(blend_bilinear_transmittance_kernel<T, 1>, grid, T * T, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, ib.seg_T, W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_bilinear_transmittance_kernel");
-    blend_prefix_kernel<T><<<n_tiles, T * T, 0, stream>>>(ib.segs, ib.tile_first, ib.seg_T);
+    launch_chained(blend_prefix_kernel<T>, n_tiles, T * T, 0, stream, ib.segs, ib.tile_first, ib.seg_T);
     INPC_LAUNCH_CHECK("blend_prefix_kernel");
-    blend_rows_forward_kernel<T, C4, KIND><<<grid, T * T, smem, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, reinterpret_cast<const float4*>(features),
+    launch_chained(blend_rows_forward_kernel<T, C4, KIND>, grid, T * T, smem, stream, ib.segs, ib.n_segments, ids, pb.rec, reinterpret_cast<const float4*>(features),
                                                                          ib.seg_T, ib.seg_C, ib.seg_Z, image, depth, alpha, blending_weights, W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_rows_forward_kernel");
-    blend_rows_combine_kernel<T, C4, KIND><<<n_tiles, T * T, 0, stream>>>(ib.segs, ib.tile_first, ib.seg_C, ib.seg_Z, ib.seg_T, image, depth, alpha,
+    launch_chained(blend_rows_combine_kernel<T, C4, KIND>, n_tiles, T * T, 0, stream, ib.segs, ib.tile_first, ib.seg_C, ib.seg_Z, ib.seg_T, image, depth, alpha,
                                                                          W, H, rp.gw);
     INPC_LAUNCH_CHECK("blend_rows_combine_kernel");
     return INPC_OK;
@@ -4330,7 +4359,7 @@ int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
     const int rc_attr = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
     if (rc_attr != INPC_OK) return rc_attr;
-    blend_rows_warp_backward_kernel<C4><<<grid, kWarpBlendWarps * 32, smem, stream>>>(
+    launch_chained(blend_rows_warp_backward_kernel<C4>, grid, kWarpBlendWarps * 32, smem, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
         reinterpret_cast<const float4*>(features), ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha,
         reinterpret_cast<float4*>(grad_features), grad_opacities, rp.v.width, rp.v.height, rp.gw);
@@ -4348,7 +4377,7 @@ int launch_rows_backward(const RasterParams& rp, const PointBlob& pb, const Inst
         const int rc_attr = opt_in_dynamic_smem(blend_rows_backward_kernel<T, C4>, smem, attr_set);
         if (rc_attr != INPC_OK) return rc_attr;
     }
-    blend_rows_backward_kernel<T, C4><<<(unsigned)ib.max_segments, T * T, smem, stream>>>(
+    launch_chained(blend_rows_backward_kernel<T, C4>, (unsigned)ib.max_segments, T * T, smem, stream,
         ib.segs, ib.n_segments, ids, pb.rec, reinterpret_cast<const float4*>(features), ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha,
         reinterpret_cast<float4*>(grad_features), grad_opacities, rp.v.width, rp.v.height, rp.gw);
     INPC_LAUNCH_CHECK("blend_rows_backward_kernel");
@@ -4488,7 +4517,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
                 rc = launch_gaussian_warp_backward(rp, pb, ib, tile_buffer_of(state, n_tiles), grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
                 if (rc != INPC_OK) return rc;
             } else {
-                blend_gaussian_backward_kernel<16><<<(unsigned)ib.max_segments, 256, 0, stream>>>(ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, W, H, rp.gw);
+                launch_chained(blend_gaussian_backward_kernel<16>, (unsigned)ib.max_segments, 256, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, W, H, rp.gw);
                 INPC_LAUNCH_CHECK("blend_gaussian_backward_kernel");
             }
         }
@@ -4497,10 +4526,10 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     const GradientSlots gs{slot_grad, slot_mask};
     const bool bulk_ok = (reinterpret_cast<uintptr_t>(grad_features) & 15u) == 0;
     if (slots)
-        preprocess_backward_kernel<true><<<(unsigned)ceil_div<int64_t>(n, kPreThreads), kPreThreads, 0, stream>>>(
+        launch_chained(preprocess_backward_kernel<true>, (unsigned)ceil_div<int64_t>(n, kPreThreads), kPreThreads, 0, stream,
             positions, view->cam_position, pb.bounds, gfv, gs, grad_opacities, static_cast<__half*>(grad_features), n, bulk_ok);
     else
-        preprocess_backward_kernel<false><<<(unsigned)ceil_div<int64_t>(n, kPreThreads), kPreThreads, 0, stream>>>(
+        launch_chained(preprocess_backward_kernel<false>, (unsigned)ceil_div<int64_t>(n, kPreThreads), kPreThreads, 0, stream,
             positions, view->cam_position, pb.bounds, gfv, gs, grad_opacities, static_cast<__half*>(grad_features), n, bulk_ok);
     INPC_LAUNCH_CHECK("preprocess_backward_kernel");
     return end_index_checks(stream);
@@ -4710,12 +4739,14 @@ extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
 
 namespace inpc_debug {
 __global__ void add_base_kernel(const uint32_t* __restrict__ src, int64_t n, uint32_t base, uint32_t mask, uint32_t* __restrict__ dst) {
+    await_previous_kernel();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = (src[i] & mask) + base;
 }
 
 __global__ void unpack_points_kernel(const PointRec* __restrict__ rec, int rec_stride, const uint2* __restrict__ bounds, int64_t n, int which,
                                      void* __restrict__ dst) {
+    await_previous_kernel();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint2 b = bounds[i];
@@ -4748,7 +4779,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
         case 0: INPC_CUDA_TRY(cudaMemcpyAsync(dst, pb.ids[d], 4 * (size_t)state->n_visible, cudaMemcpyDeviceToDevice, stream)); break;
         case 1:   // the sort works on offsets from the smallest depth key: add the base back
             if (state->n_visible > 0) {
-                inpc_debug::add_base_kernel<<<(unsigned)ceil_div<int64_t>(state->n_visible, 256), 256, 0, stream>>>(
+                launch_chained(inpc_debug::add_base_kernel, (unsigned)ceil_div<int64_t>(state->n_visible, 256), 256, 0, stream,
                     pb.keys[d], state->n_visible, state->depth_key_base,
                     state->depth_key_bits <= 30 ? 0x3FFFFFFFu : 0xFFFFFFFFu, static_cast<uint32_t*>(dst));
                 INPC_LAUNCH_CHECK("add_base_kernel");
@@ -4758,7 +4789,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
         case 3: INPC_CUDA_TRY(cudaMemcpyAsync(dst, ib.ranges, 8 * (size_t)n_tiles, cudaMemcpyDeviceToDevice, stream)); break;
         case 4: case 5: case 6: case 7: case 8:
             if (state->n_points > 0) {
-                inpc_debug::unpack_points_kernel<<<(unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream>>>(pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, state->n_points, which, dst);
+                launch_chained(inpc_debug::unpack_points_kernel, (unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream, pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, state->n_points, which, dst);
                 INPC_LAUNCH_CHECK("unpack_points_kernel");
             }
             break;

@@ -73,6 +73,7 @@ __device__ __forceinline__ float4 leaf_record(float cx, float cy, float cz, int 
 // of the counting call.  (Reading the caller's four words per slot instead: 30 us more for 4 x 2^23 slots of 2^18 leaves.)
 __global__ void __launch_bounds__(kThreads) leaf_records_kernel(int64_t n_cells, const float* __restrict__ centers, const int* __restrict__ levels,
                                                                 float initial_size, float4* __restrict__ leaf_pack) {
+    await_previous_kernel();
     const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (l < n_cells) leaf_pack[l] = leaf_record(__ldg(centers + 3 * l), __ldg(centers + 3 * l + 1), __ldg(centers + 3 * l + 2), __ldg(levels + l), initial_size);
 }
@@ -84,6 +85,7 @@ __global__ void __launch_bounds__(kThreads) viewpoint_weights_kernel(ViewParams 
                                                                      const float* __restrict__ weights,
                                                                      float initial_size, float* __restrict__ out,
                                                                      float4* __restrict__ leaf_pack, unsigned* max_bits) {
+    await_previous_kernel();
     const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const unsigned active = __ballot_sync(0xffffffffu, l < n_cells);
     if (l >= n_cells) return;
@@ -109,6 +111,7 @@ struct ViewSet {
 __global__ void __launch_bounds__(kThreads) max_viewpoint_weights_kernel(const __grid_constant__ ViewSet views, int64_t n_cells, const float* __restrict__ centers,
                                                                          const int* __restrict__ levels, const float* __restrict__ weights,
                                                                          float initial_size, bool first, float* __restrict__ out) {
+    await_previous_kernel();
     const int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (l >= n_cells) return;
     const float cx = __ldg(centers + 3 * l), cy = __ldg(centers + 3 * l + 1), cz = __ldg(centers + 3 * l + 2);
@@ -140,6 +143,7 @@ __device__ __forceinline__ unsigned long long to_fixed(float w, float w_max) {
 
 // largest weight via atomicMax on the bit pattern (valid for non-negative floats; order-free)
 __global__ void __launch_bounds__(kCdfThreads) cdf_max_kernel(const float* __restrict__ w, int64_t n, unsigned* __restrict__ max_bits) {
+    await_previous_kernel();
     const int64_t base = (int64_t)blockIdx.x * kCdfChunk + (int64_t)threadIdx.x * kCdfItems;
     float m = 0.0f;
 #pragma unroll
@@ -186,6 +190,7 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_chunk_sums_kernel(const float
                                                                      const unsigned* __restrict__ max_bits, unsigned* done,
                                                                      unsigned long long* chunk_sums, unsigned long long* __restrict__ total_out,
                                                                      float* __restrict__ sum_out) {
+    await_previous_kernel();
     __shared__ unsigned long long s[kCdfThreads / 32 + 1];
     const float w_max = __uint_as_float(__ldg(max_bits));
     const int64_t base = (int64_t)blockIdx.x * kCdfChunk + (int64_t)threadIdx.x * kCdfItems;
@@ -217,6 +222,7 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_finalize_kernel(const float* 
                                                                    const unsigned long long* __restrict__ chunk_base,
                                                                    const unsigned long long* __restrict__ total_ptr,
                                                                    float* __restrict__ cdf) {
+    await_previous_kernel();
     __shared__ unsigned long long s[kCdfThreads / 32 + 1];
     const float w_max = __uint_as_float(__ldg(max_bits));
     const double total = (double)__ldg(total_ptr);
@@ -293,6 +299,7 @@ __device__ __forceinline__ unsigned lower_bound_clamped(const float* __restrict_
 // CDF steps, nine in ten with as many buckets as leaves, in one sector where separate guide and CDF arrays took three.
 constexpr int kGuidePerBlock = kThreads - 1;   // the last thread of a block only finds the end of the last bucket
 __global__ void __launch_bounds__(kThreads) guide_table_kernel(const float* __restrict__ cdf, unsigned n_cells, int k, uint4* __restrict__ guide) {
+    await_previous_kernel();
     __shared__ unsigned s_first[kThreads];
     const unsigned b = blockIdx.x * kGuidePerBlock + threadIdx.x, n_buckets = 1u << k;
     unsigned first = 0, count = b <= n_buckets ? n_cells : 0u;
@@ -352,6 +359,7 @@ __global__ void __launch_bounds__(kThreads, 6) training_samples_kernel(
     const uint4* __restrict__ guide, int guide_bits, const float* __restrict__ sum_ptr, unsigned n_cells,
     const float4* __restrict__ leaf_pack, int64_t n_samples, float* __restrict__ positions, long long* __restrict__ indices,
     volatile unsigned* status) {
+    await_previous_kernel();
     __shared__ __align__(16) float s_pos[3 * kThreads];
     const int64_t block_first = (int64_t)blockIdx.x * kThreads;
     const int64_t s = block_first + threadIdx.x;
@@ -392,6 +400,7 @@ __global__ void __launch_bounds__(kThreads) samples_kernel(const __grid_constant
                                                            int guide_bits, unsigned n_cells,
                                                            const float4* __restrict__ leaf_pack, int64_t n_samples,
                                                            float* __restrict__ positions) {
+    await_previous_kernel();
     __shared__ __align__(16) float s_pos[3 * kThreads];
     const int64_t block_first = (int64_t)blockIdx.x * kThreads;
     const Draw d = philox_draw(keys, (unsigned)(block_first + threadIdx.x), 0u);
@@ -403,6 +412,7 @@ __global__ void __launch_bounds__(kThreads) samples_kernel(const __grid_constant
 __global__ void __launch_bounds__(kThreads) draw_leaves_kernel(const float* __restrict__ cdf, unsigned n_cells,
                                                                const float* __restrict__ u, int64_t n,
                                                                long long* __restrict__ out) {
+    await_previous_kernel();
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (i >= n) return;
     out[i] = (long long)lower_bound_clamped(cdf, __ldg(u + i), n_cells);
@@ -414,6 +424,7 @@ __global__ void __launch_bounds__(kThreads) draw_leaves_kernel(const float* __re
 __global__ void __launch_bounds__(kThreads) count_chunk_sums_kernel(const float* __restrict__ weights, const float* __restrict__ sum_ptr, unsigned n_samples,
                                                                     unsigned* __restrict__ counts, int64_t n, unsigned* done, unsigned* chunk_sums,
                                                                     unsigned long long* __restrict__ total_out) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kThreads / 32 + 1];
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     unsigned c = 0;
@@ -455,6 +466,7 @@ __global__ void __launch_bounds__(kThreads) count_chunk_sums_kernel(const float*
 __global__ void __launch_bounds__(kThreads) count_offsets_kernel(const unsigned* __restrict__ counts, int64_t n,
                                                                  const unsigned* __restrict__ chunk_base,
                                                                  unsigned* __restrict__ offsets) {
+    await_previous_kernel();
     __shared__ unsigned s_scan[kThreads / 32 + 1];
     const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const unsigned c = i < n ? counts[i] : 0u;
@@ -531,6 +543,7 @@ __global__ void __launch_bounds__(kThreads) expected_samples_kernel(const __grid
                                                                     const unsigned* __restrict__ offsets, unsigned n_cells,
                                                                     const float4* __restrict__ leaf_pack, unsigned n_created,
                                                                     unsigned n_copies, float* __restrict__ positions) {
+    await_previous_kernel();
     __shared__ LeafRun run;
     __shared__ __align__(16) float s_pos[3 * kThreads];
     const unsigned r0 = blockIdx.x * (unsigned)kRunSlots;
@@ -557,6 +570,7 @@ __global__ void __launch_bounds__(kThreads) leaf_histogram_kernel(const __grid_c
                                                                   const float* __restrict__ cdf, const uint4* __restrict__ guide,
                                                                   int guide_bits, unsigned n_cells, int64_t n_samples,
                                                                   unsigned* __restrict__ counts) {
+    await_previous_kernel();
     // the table gathers of a thread's draws are in flight together
     const int64_t first = (int64_t)blockIdx.x * (kThreads * kDrawsPerThread) + threadIdx.x;
     unsigned leaf[kDrawsPerThread];
@@ -626,6 +640,7 @@ __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned
                                                                   unsigned n_cells, const float* __restrict__ centers,
                                                                   const int* __restrict__ levels, float initial_size, unsigned n_total,
                                                                   float* __restrict__ positions) {
+    await_previous_kernel();
     __shared__ LeafRun run;
     __shared__ __align__(16) float s_pos[3 * kThreads];
     __shared__ double s_tables[sizeof(HaltonTables) / 8];
@@ -702,6 +717,7 @@ __device__ __forceinline__ void block_box(float* box, float (*s_box)[6]) {
 }
 
 __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, float* __restrict__ partial) {
+    await_previous_kernel();
     __shared__ float s_box[kThreads / 32][6];
     float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
     auto add = [&](float x, float y, float z) {
@@ -731,6 +747,7 @@ struct MortonBox {
 };
 __global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, MortonBox mb,
                                                                 unsigned* __restrict__ codes, unsigned* __restrict__ order) {
+    await_previous_kernel();
     if (mb.box_parts > 0) {
         __shared__ float s_box[kThreads / 32][6];
         float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -772,6 +789,7 @@ __global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __r
 // point per thread with three 4-byte stores 201, the same with the stores staged through shared memory 211).
 __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float* __restrict__ positions, const unsigned* __restrict__ order,
                                                                     int64_t n, bool vec_ok, float* __restrict__ out) {
+    await_previous_kernel();
     const int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
     if (i >= n) return;
     if (vec_ok && i + 4 <= n) {
@@ -843,16 +861,16 @@ int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out,
     const int64_t chunks = ceil_div<int64_t>(n_cells, kCdfChunk);
     if (!max_known) {
         INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
-        cdf_max_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits);
+        launch_chained(cdf_max_kernel, (unsigned)chunks, kCdfThreads, 0, stream, weights, n_cells, w.max_bits);
         INPC_LAUNCH_CHECK("cdf_max_kernel");
     }
-    cdf_chunk_sums_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits, w.max_bits + 1, w.chunk_sums64, w.total64, sum_out);
+    launch_chained(cdf_chunk_sums_kernel, (unsigned)chunks, kCdfThreads, 0, stream, weights, n_cells, w.max_bits, w.max_bits + 1, w.chunk_sums64, w.total64, sum_out);
     INPC_LAUNCH_CHECK("cdf_chunk_sums_kernel");
     if (cdf) {
-        cdf_finalize_kernel<<<(unsigned)chunks, kCdfThreads, 0, stream>>>(weights, n_cells, w.max_bits, w.chunk_sums64, w.total64, cdf);
+        launch_chained(cdf_finalize_kernel, (unsigned)chunks, kCdfThreads, 0, stream, weights, n_cells, w.max_bits, w.chunk_sums64, w.total64, cdf);
         INPC_LAUNCH_CHECK("cdf_finalize_kernel");
         if (cdf == w.cdf) {
-            guide_table_kernel<<<(unsigned)ceil_div<int64_t>((int64_t)1 << w.guide_bits, kGuidePerBlock), kThreads, 0, stream>>>(
+            launch_chained(guide_table_kernel, (unsigned)ceil_div<int64_t>((int64_t)1 << w.guide_bits, kGuidePerBlock), kThreads, 0, stream,
                 cdf, (unsigned)n_cells, w.guide_bits, w.guide);
             INPC_LAUNCH_CHECK("guide_table_kernel");
         }
@@ -864,7 +882,7 @@ int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out,
 int view_weights(const ViewParams& v, int64_t n_cells, const float* centers, const int32_t* levels, const float* weights, float initial_size,
                  const SamplerWs& w, float4* leaf_pack, cudaStream_t stream) {
     INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
-    viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(v, n_cells, centers, levels, weights, initial_size, w.vw,
+    launch_chained(viewpoint_weights_kernel, (unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream, v, n_cells, centers, levels, weights, initial_size, w.vw,
                                                                                                    leaf_pack, w.max_bits);
     INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
     return INPC_OK;
@@ -927,7 +945,7 @@ extern "C" int inpc_compute_viewpoint_weights(const inpc_view* view, int64_t n_c
     int rc = check_cells(view, n_cells, centers, levels, weights);
     if (rc != INPC_OK) return rc;
     if (!out) { set_error("inpc_compute_viewpoint_weights: null output"); return INPC_E_INVALID; }
-    viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(
+    launch_chained(viewpoint_weights_kernel, (unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream,
         to_params(view), n_cells, centers, levels, weights, initial_size, out, nullptr, nullptr);
     INPC_LAUNCH_CHECK("viewpoint_weights_kernel");
     return INPC_OK;
@@ -946,7 +964,7 @@ extern "C" int inpc_max_viewpoint_weights(const inpc_view* views, int n_views, i
         ViewSet set;
         set.count = n_views - j < kViewsPerPass ? n_views - j : kViewsPerPass;
         for (int k = 0; k < set.count; ++k) set.v[k] = to_params(views + j + k);
-        max_viewpoint_weights_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(set, n_cells, centers, levels, weights,
+        launch_chained(max_viewpoint_weights_kernel, (unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream, set, n_cells, centers, levels, weights,
                                                                                                            initial_size, j == 0, out);
         INPC_LAUNCH_CHECK("max_viewpoint_weights_kernel");
     }
@@ -963,7 +981,7 @@ extern "C" int inpc_build_cdf(const float* weights, int64_t n_cells, float* cdf,
 extern "C" int inpc_draw_leaves(const float* cdf, int64_t n_cells, const float* u, int64_t n, int64_t* out, void* stream_) {
     if (n == 0) return INPC_OK;
     if (n_cells <= 0 || n_cells >= ((int64_t)1 << 31) || !cdf || !u || !out || n < 0) { set_error("inpc_draw_leaves: bad argument"); return INPC_E_INVALID; }
-    draw_leaves_kernel<<<(unsigned)ceil_div<int64_t>(n, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream_)>>>(
+    launch_chained(draw_leaves_kernel, (unsigned)ceil_div<int64_t>(n, kThreads), kThreads, 0, static_cast<cudaStream_t>(stream_),
         cdf, (unsigned)n_cells, u, n, reinterpret_cast<long long*>(out));
     INPC_LAUNCH_CHECK("draw_leaves_kernel");
     return INPC_OK;
@@ -988,7 +1006,7 @@ extern "C" int inpc_generate_training_samples(inpc_sampler* s, const inpc_view* 
     if (rc != INPC_OK) return rc;
     unsigned* status = acquire_status("inpc_generate_training_samples", &s->training_ticket);
     if (!status) return INPC_E_CUDA;
-    training_samples_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream>>>(
+    launch_chained(training_samples_kernel, (unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream,
         v, philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, w.sum, (unsigned)n_cells, w.leaf_pack, n_samples, positions,
         reinterpret_cast<long long*>(indices), status);
     INPC_LAUNCH_CHECK("training_samples_kernel");
@@ -1017,7 +1035,7 @@ extern "C" int inpc_generate_samples(inpc_sampler* s, const inpc_view* view, int
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
     if (!(host[0] > 0.0f)) return INPC_OK;   // src/sampling_api.cu:154: empty result
     if (n_samples > 0) {
-        samples_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream>>>(
+        launch_chained(samples_kernel, (unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream,
             philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, w.leaf_pack, n_samples, positions);
         INPC_LAUNCH_CHECK("samples_kernel");
     }
@@ -1043,9 +1061,9 @@ extern "C" int inpc_generate_expected_samples_count(inpc_sampler* s, const inpc_
     if (rc != INPC_OK) return rc;
     rc = build_cdf(w.vw, n_cells, nullptr, w.sum, w, true, stream);
     if (rc != INPC_OK) return rc;
-    count_chunk_sums_kernel<<<blocks, kThreads, 0, stream>>>(w.vw, w.sum, (unsigned)n_samples, w.counts, n_cells, w.max_bits + 2, w.chunk_sums, w.total);
+    launch_chained(count_chunk_sums_kernel, blocks, kThreads, 0, stream, w.vw, w.sum, (unsigned)n_samples, w.counts, n_cells, w.max_bits + 2, w.chunk_sums, w.total);
     INPC_LAUNCH_CHECK("count_chunk_sums_kernel");
-    count_offsets_kernel<<<blocks, kThreads, 0, stream>>>(w.counts, n_cells, w.chunk_sums, w.offsets);
+    launch_chained(count_offsets_kernel, blocks, kThreads, 0, stream, w.counts, n_cells, w.chunk_sums, w.offsets);
     INPC_LAUNCH_CHECK("count_offsets_kernel");
     unsigned long long* host = reinterpret_cast<unsigned long long*>(pinned_float());
     if (!host) return cuda_fail(cudaGetLastError(), "cudaHostAlloc");
@@ -1067,10 +1085,10 @@ extern "C" int inpc_generate_expected_samples_fill(inpc_sampler* s, int64_t n_ce
         return INPC_E_INVALID;
     }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
-    leaf_records_kernel<<<(unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream>>>(n_cells, centers, levels, initial_size, w.leaf_pack);
+    launch_chained(leaf_records_kernel, (unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream, n_cells, centers, levels, initial_size, w.leaf_pack);
     INPC_LAUNCH_CHECK("leaf_records_kernel");
     const dim3 grid((unsigned)ceil_div<int64_t>(n_created, kRunSlots), (unsigned)(n_multi < 65535 ? n_multi : 65535));
-    expected_samples_kernel<<<grid, kThreads, 0, stream>>>(philox_keys(s->seed, s->counter), w.offsets, (unsigned)n_cells, w.leaf_pack, (unsigned)n_created,
+    launch_chained(expected_samples_kernel, grid, kThreads, 0, stream, philox_keys(s->seed, s->counter), w.offsets, (unsigned)n_cells, w.leaf_pack, (unsigned)n_created,
                                                            (unsigned)n_multi, positions);
     INPC_LAUNCH_CHECK("expected_samples_kernel");
     s->counter += 1;
@@ -1082,9 +1100,9 @@ namespace {
 int scan_counts(const SamplerWs& w, int64_t n_cells, cudaStream_t stream) {
     const unsigned blocks = (unsigned)ceil_div<int64_t>(n_cells, kThreads);
     INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
-    count_chunk_sums_kernel<<<blocks, kThreads, 0, stream>>>(nullptr, nullptr, 0u, w.counts, n_cells, w.max_bits + 2, w.chunk_sums, w.total);
+    launch_chained(count_chunk_sums_kernel, blocks, kThreads, 0, stream, nullptr, nullptr, 0u, w.counts, n_cells, w.max_bits + 2, w.chunk_sums, w.total);
     INPC_LAUNCH_CHECK("count_chunk_sums_kernel");
-    count_offsets_kernel<<<blocks, kThreads, 0, stream>>>(w.counts, n_cells, w.chunk_sums, w.offsets);
+    launch_chained(count_offsets_kernel, blocks, kThreads, 0, stream, w.counts, n_cells, w.chunk_sums, w.offsets);
     INPC_LAUNCH_CHECK("count_offsets_kernel");
     return INPC_OK;
 }
@@ -1107,7 +1125,7 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
     if (!(host[0] > 0.0f)) { set_error("inpc_draw_leaf_counts: the weights sum to zero"); return INPC_E_INVALID; }
     if (n_samples > 0) {
-        leaf_histogram_kernel<<<(unsigned)ceil_div<int64_t>(n_samples, kThreads * kDrawsPerThread), kThreads, 0, stream>>>(
+        launch_chained(leaf_histogram_kernel, (unsigned)ceil_div<int64_t>(n_samples, kThreads * kDrawsPerThread), kThreads, 0, stream,
             philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, n_samples, counts);
         INPC_LAUNCH_CHECK("leaf_histogram_kernel");
     }
@@ -1127,7 +1145,7 @@ extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, cons
     INPC_CUDA_TRY(cudaMemcpyAsync(w.counts, counts, sizeof(uint32_t) * (size_t)n_cells, cudaMemcpyDeviceToDevice, stream));
     const int rc = scan_counts(w, n_cells, stream);
     if (rc != INPC_OK) return rc;
-    halton_samples_kernel<<<(unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream>>>(w.counts, w.offsets, (unsigned)n_cells, centers, levels,
+    launch_chained(halton_samples_kernel, (unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream, w.counts, w.offsets, (unsigned)n_cells, centers, levels,
                                                                                                  initial_size, (unsigned)n_total, positions);
     INPC_LAUNCH_CHECK("halton_samples_kernel");
     return INPC_OK;
@@ -1159,12 +1177,12 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
     } else {
         const int64_t blocks = ceil_div<int64_t>(n, 4 * kThreads), cap = 4 * sm_count() < kMaxBoxBlocks ? 4 * sm_count() : kMaxBoxBlocks;
         mb.box_parts = (int)(blocks < cap ? blocks : cap);
-        bounding_box_kernel<<<mb.box_parts, kThreads, 0, stream>>>(positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, parts);
+        launch_chained(bounding_box_kernel, mb.box_parts, kThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, parts);
         INPC_LAUNCH_CHECK("bounding_box_kernel");
     }
     const bool vec_ok = (reinterpret_cast<uintptr_t>(positions) & 15u) == 0;
     const int64_t code_blocks = ceil_div<int64_t>(n, 4 * kThreads), code_cap = (int64_t)sm_count() * 8;
-    morton_codes_kernel<<<(unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kThreads, 0, stream>>>(positions, n, vec_ok, mb, codes[0], order[0]);
+    launch_chained(morton_codes_kernel, (unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kThreads, 0, stream, positions, n, vec_ok, mb, codes[0], order[0]);
     INPC_LAUNCH_CHECK("morton_codes_kernel");
     int in_alt = 0;
     {
@@ -1175,7 +1193,7 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
     if (!status) return INPC_E_CUDA;
     const int rc = sort_pairs(codes[0], codes[1], order[0], order[1], n, n, 30, sort_ws, false, status, &in_alt, stream, true);
     if (rc != INPC_OK) return rc;
-    gather_positions_kernel<<<(unsigned)ceil_div<int64_t>(n, 4 * kThreads), kThreads, 0, stream>>>(positions, order[in_alt], n, (reinterpret_cast<uintptr_t>(out) & 15u) == 0, out);
+    launch_chained(gather_positions_kernel, (unsigned)ceil_div<int64_t>(n, 4 * kThreads), kThreads, 0, stream, positions, order[in_alt], n, (reinterpret_cast<uintptr_t>(out) & 15u) == 0, out);
     INPC_LAUNCH_CHECK("gather_positions_kernel");
     return INPC_OK;
 }
