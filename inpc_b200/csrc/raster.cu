@@ -1833,7 +1833,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
                         const float4 a = sm.ring_a[stage][j[u]];
                         if (C4 == 1) f[u] = sm.ring_f[stage][j[u]];
                         wg[u] = __saturatef(1.0f - fabsf(a.x - pcx)) * __saturatef(1.0f - fabsf(a.y - pcy));
-                        al[u] = a.z * wg[u];
+                        al[u] = __fmul_rn(a.z, wg[u]);   // rounded, as the backward pass has it: 1 - alpha must not be formed from the exact product
                         zd[u] = a.w;
                         ok[u] = ok[u] && wg[u] > 0.0f;
                     }
@@ -2406,7 +2406,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
                     const float4 f = row[c];
                     fg += f.x * g[c].x + f.y * g[c].y + f.z * g[c].z + f.w * g[c].w;
                 }
-                const float al = a.z * wg;
+                const float al = __fmul_rn(a.z, wg);   // rounded, as in the forward pass
                 const float bw = Tr * al;
                 G_run += bw * fg;
                 const float oma = 1.0f - al;
