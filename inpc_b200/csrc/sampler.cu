@@ -7,6 +7,7 @@
 // slots with an atomic ticket and is not (sampling/src/sampling_kernels.cu:104-125).
 // Citations are paths below INPCCudaBackend/INPCCudaBackend/sampling/ of the reference.
 #include "common.cuh"
+#include <type_traits>
 
 namespace inpc {
 
@@ -298,7 +299,14 @@ __device__ __forceinline__ unsigned lower_bound_clamped(const float* __restrict_
 // sectors it gathers from L2 (all tables are larger than L1): the record settles the draws whose bucket holds at most two
 // CDF steps, nine in ten with as many buckets as leaves, in one sector where separate guide and CDF arrays took three.
 constexpr int kGuidePerBlock = kThreads - 1;   // the last thread of a block only finds the end of the last bucket
-__global__ void __launch_bounds__(kThreads) guide_table_kernel(const float* __restrict__ cdf, unsigned n_cells, int k, uint4* __restrict__ guide) {
+// With `leaf_pack` a record is 32 bytes, one sector: behind the four words lies the geometry of its first leaf, which is the leaf of
+// most draws (a leaf of some weight covers whole buckets), and a draw that ends there makes one gather instead of two.
+struct __align__(32) GuideRecord {
+    uint4 steps;
+    float4 leaf;
+};
+__global__ void __launch_bounds__(kThreads) guide_table_kernel(const float* __restrict__ cdf, unsigned n_cells, int k, uint4* __restrict__ guide,
+                                                               const float4* __restrict__ leaf_pack) {
     await_previous_kernel();
     __shared__ unsigned s_first[kThreads];
     const unsigned b = blockIdx.x * kGuidePerBlock + threadIdx.x, n_buckets = 1u << k;
@@ -314,13 +322,23 @@ __global__ void __launch_bounds__(kThreads) guide_table_kernel(const float* __re
     __syncthreads();
     if (threadIdx.x == kGuidePerBlock || b >= n_buckets) return;
     const float c0 = first < n_cells ? __ldg(cdf + first) : 2.0f, c1 = first + 1u < n_cells ? __ldg(cdf + first + 1u) : 2.0f;
-    guide[b] = make_uint4(first, __float_as_uint(c0), __float_as_uint(c1), s_first[threadIdx.x + 1]);
+    const uint4 steps = make_uint4(first, __float_as_uint(c0), __float_as_uint(c1), s_first[threadIdx.x + 1]);
+    if (leaf_pack) reinterpret_cast<GuideRecord*>(guide)[b] = GuideRecord{steps, __ldg(leaf_pack + min(first, n_cells - 1u))};
+    else guide[b] = steps;
 }
 
-// r: the raw 32 random bits the uniform is made of (u = (r >> 9) * 2^-23)
-__device__ __forceinline__ unsigned guided_lower_bound(const float* __restrict__ cdf, const uint4* __restrict__ guide, int k,
-                                                       unsigned r, float u, unsigned n) {
-    const uint4 g = __ldg(guide + ((r >> 9) >> (23 - k)));
+// The record of a uniform's bucket; r: the raw 32 random bits the uniform is made of (u = (r >> 9) * 2^-23)
+__device__ __forceinline__ uint4 guide_record(const uint4* __restrict__ guide, int k, unsigned r) { return __ldg(guide + ((r >> 9) >> (23 - k))); }
+// ... with its first leaf, in one 32-byte load
+__device__ __forceinline__ GuideRecord packed_guide_record(const uint4* __restrict__ guide, int k, unsigned r) {
+    const GuideRecord* p = reinterpret_cast<const GuideRecord*>(guide) + ((r >> 9) >> (23 - k));
+    GuideRecord g;
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(g.steps.x), "=r"(g.steps.y), "=r"(g.steps.z), "=r"(g.steps.w), "=f"(g.leaf.x), "=f"(g.leaf.y), "=f"(g.leaf.z), "=f"(g.leaf.w)
+                 : "l"(p));
+    return g;
+}
+__device__ __forceinline__ unsigned settle_lower_bound(const float* __restrict__ cdf, const uint4& g, float u, unsigned n) {
     unsigned first = g.x;
     if (__uint_as_float(g.y) < u) {
         first += 1u;
@@ -335,6 +353,10 @@ __device__ __forceinline__ unsigned guided_lower_bound(const float* __restrict__
         }
     }
     return min(first, n - 1);
+}
+__device__ __forceinline__ unsigned guided_lower_bound(const float* __restrict__ cdf, const uint4* __restrict__ guide, int k,
+                                                       unsigned r, float u, unsigned n) {
+    return settle_lower_bound(cdf, guide_record(guide, k, r), u, n);
 }
 
 // Positions of the kThreads consecutive samples of a block, first sample `first`, leave as 16-byte vectors through shared
@@ -352,46 +374,102 @@ __device__ __forceinline__ void store_positions(float* s_pos, float x, float y, 
 }
 
 // ---- training samples: same acceptance test as src/sampling_kernels.cu:98-113 -------------------
-// Bound by the latency of its two dependent gathers and the integer work of Philox: six blocks per multiprocessor (40 registers)
-// hide more of it than the four that 60 registers allow.
-__global__ void __launch_bounds__(kThreads, 6) training_samples_kernel(
+// A block makes PER * kThreads consecutive samples.  The first attempts of a thread's PER slots go together, their gathers in
+// flight at the same time; slots whose point lies outside the view go to a list in shared memory, which all threads of the block then
+// work off, attempt by attempt.  What a slot draws at an attempt depends on nothing else, so the samples are those of a loop per slot.
+// Bound by instruction issue (240 instructions per sample, a third of them Philox; 54 % of the issue slots) and by waiting for the
+// gather.  2^23 samples of 2^18 leaves: one slot per thread looping until it succeeds (a warp then makes as many attempts as its
+// unluckiest slot) 109 us; two slots per thread and the list 101, with the leaf's geometry in the guide record 97 (five blocks per
+// multiprocessor; with six 101, four 107; four slots per thread 111).
+template <int PER>
+__global__ void __launch_bounds__(kThreads, PER == 1 ? 6 : 5) training_samples_kernel(
     ViewParams v, const __grid_constant__ PhiloxKeys keys, const float* __restrict__ cdf,
     const uint4* __restrict__ guide, int guide_bits, const float* __restrict__ sum_ptr, unsigned n_cells,
     const float4* __restrict__ leaf_pack, int64_t n_samples, float* __restrict__ positions, long long* __restrict__ indices,
     volatile unsigned* status) {
     await_previous_kernel();
-    __shared__ __align__(16) float s_pos[3 * kThreads];
-    const int64_t block_first = (int64_t)blockIdx.x * kThreads;
-    const int64_t s = block_first + threadIdx.x;
-    const bool mine = s < n_samples;
-    float x = 0.0f, y = 0.0f, z = 0.0f;
-    if (!(__ldg(sum_ptr) > 0.0f)) {
-        // src/sampling.cu:107-111: zero positions, indices of -1
-        if (mine) indices[s] = -1;
-    } else if (mine) {
-        const Rows m = load_rows(v.w2c);
-        unsigned leaf = 0;
-        bool ok = false;
-        for (unsigned a = 0; a < (unsigned)kMaxAttempts && !ok; ++a) {
-            const Draw d = philox_draw(keys, (unsigned)s, a);
-            leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
-            const float4 lp = __ldg(leaf_pack + leaf);
-            x = fmaf(d.jx - 0.5f, lp.w, lp.x);
-            y = fmaf(d.jy - 0.5f, lp.w, lp.y);
-            z = fmaf(d.jz - 0.5f, lp.w, lp.z);
-            const float vz = affine(m.r2, x, y, z);
-            if (vz < v.near_plane || vz > v.far_plane) continue;
-            const float inv_z = 1.0f / (vz + kEps);
-            const float sx = fmaf(affine(m.r0, x, y, z) * inv_z, v.fx, v.cx);
-            if (sx < 0.0f || sx >= (float)v.width) continue;
-            const float sy = fmaf(affine(m.r1, x, y, z) * inv_z, v.fy, v.cy);
-            if (sy < 0.0f || sy >= (float)v.height) continue;
-            ok = true;
+    constexpr unsigned kBlock = PER * kThreads;
+    __shared__ __align__(16) float s_pos[3 * kBlock];
+    __shared__ unsigned s_leaf[kBlock];
+    __shared__ unsigned short s_retry[2][kBlock];   // slots of the block that make another attempt: of this round, of the next
+    __shared__ unsigned s_count[2];
+    const unsigned tid = threadIdx.x;
+    const int64_t block_first = (int64_t)blockIdx.x * kBlock;
+    const unsigned in_block = (unsigned)min((int64_t)kBlock, n_samples - block_first);
+    const bool any = __ldg(sum_ptr) > 0.0f;
+    if (tid < 2u) s_count[tid] = 0u;
+    __syncthreads();
+    const Rows m = load_rows(v.w2c);
+    // the point of slot `local` in the leaf a draw has found; false if it lies outside the view
+    auto place = [&](unsigned local, const Draw& d, const GuideRecord& g) -> bool {
+        const unsigned leaf = settle_lower_bound(cdf, g.steps, d.u, n_cells);
+        float4 lp = g.leaf;
+        if (leaf != min(g.steps.x, n_cells - 1u)) lp = __ldg(leaf_pack + leaf);
+        const float x = fmaf(d.jx - 0.5f, lp.w, lp.x);
+        const float y = fmaf(d.jy - 0.5f, lp.w, lp.y);
+        const float z = fmaf(d.jz - 0.5f, lp.w, lp.z);
+        s_pos[3 * local] = x; s_pos[3 * local + 1] = y; s_pos[3 * local + 2] = z;
+        s_leaf[local] = leaf;
+        const float vz = affine(m.r2, x, y, z);
+        if (vz < v.near_plane || vz > v.far_plane) return false;
+        const float inv_z = 1.0f / (vz + kEps);
+        const float sx = fmaf(affine(m.r0, x, y, z) * inv_z, v.fx, v.cx);
+        if (sx < 0.0f || sx >= (float)v.width) return false;
+        const float sy = fmaf(affine(m.r1, x, y, z) * inv_z, v.fy, v.cy);
+        return !(sy < 0.0f || sy >= (float)v.height);
+    };
+    auto retry = [&](unsigned list, unsigned local) { s_retry[list][atomicAdd(&s_count[list], 1u)] = (unsigned short)local; };
+    if (any) {
+        Draw d[PER];
+        GuideRecord g[PER];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            d[k] = philox_draw(keys, (unsigned)(block_first + k * kThreads + tid), 0u);
+            g[k] = packed_guide_record(guide, guide_bits, d[k].raw_u);
         }
-        if (!ok) status[STATUS_SAMPLER_EXHAUSTED] = 1u;
-        indices[s] = (long long)leaf;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const unsigned local = k * kThreads + tid;
+            if (local < in_block && !place(local, d[k], g[k])) retry(0u, local);
+        }
+        unsigned cur = 0u;
+        for (unsigned a = 1; a < (unsigned)kMaxAttempts; ++a, cur ^= 1u) {
+            __syncthreads();
+            const unsigned n = s_count[cur];
+            if (n == 0u) break;
+            for (unsigned i = tid; i < n; i += kThreads) {
+                const unsigned local = s_retry[cur][i];
+                const Draw e = philox_draw(keys, (unsigned)(block_first + local), a);
+                const bool ok = place(local, e, packed_guide_record(guide, guide_bits, e.raw_u));
+                if (!ok) {
+                    if (a + 1u < (unsigned)kMaxAttempts) retry(cur ^ 1u, local);
+                    else status[STATUS_SAMPLER_EXHAUSTED] = 1u;   // the last attempt's point stays
+                }
+            }
+            __syncthreads();
+            if (tid == 0u) s_count[cur] = 0u;
+        }
+    } else {
+        // src/sampling.cu:107-111: zero positions, indices of -1
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const unsigned local = k * kThreads + tid;
+            s_pos[3 * local] = s_pos[3 * local + 1] = s_pos[3 * local + 2] = 0.0f;
+        }
     }
-    store_positions(s_pos, x, y, z, block_first, n_samples, positions);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const unsigned local = k * kThreads + tid;
+        if (local < in_block) indices[block_first + local] = any ? (long long)s_leaf[local] : -1;
+    }
+    const unsigned floats = 3u * in_block;
+    float* dst = positions + 3 * block_first;
+    if (in_block == kBlock && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        for (unsigned k = tid; k < 3u * kBlock / 4u; k += kThreads) reinterpret_cast<float4*>(dst)[k] = reinterpret_cast<const float4*>(s_pos)[k];
+    } else {
+        for (unsigned k = tid; k < floats; k += kThreads) dst[k] = s_pos[k];
+    }
 }
 
 // ---- unconditional samples: src/sampling_kernels.cu:128-150 with the Philox stream ----------------
@@ -404,8 +482,10 @@ __global__ void __launch_bounds__(kThreads) samples_kernel(const __grid_constant
     __shared__ __align__(16) float s_pos[3 * kThreads];
     const int64_t block_first = (int64_t)blockIdx.x * kThreads;
     const Draw d = philox_draw(keys, (unsigned)(block_first + threadIdx.x), 0u);
-    const unsigned leaf = guided_lower_bound(cdf, guide, guide_bits, d.raw_u, d.u, n_cells);
-    const float4 lp = __ldg(leaf_pack + leaf);
+    const GuideRecord g = packed_guide_record(guide, guide_bits, d.raw_u);
+    const unsigned leaf = settle_lower_bound(cdf, g.steps, d.u, n_cells);
+    float4 lp = g.leaf;
+    if (leaf != min(g.steps.x, n_cells - 1u)) lp = __ldg(leaf_pack + leaf);
     store_positions(s_pos, fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), block_first, n_samples, positions);
 }
 
@@ -823,7 +903,7 @@ struct SamplerWs {
     unsigned* offsets;  // inclusive offsets (n_cells)
     unsigned* chunk_sums;
     unsigned long long* total;
-    uint4* guide;       // 2^guide_bits bucket records
+    uint4* guide;       // 2^guide_bits bucket records, of 16 or (GuideRecord) 32 bytes
     int guide_bits;
     float4* leaf_pack;  // (n_cells) centre + edge length
     size_t bytes;
@@ -850,14 +930,16 @@ SamplerWs carve_sampler_ws(void* p, int64_t n_cells) {
     w.chunk_sums = c.take<unsigned>(ceil_div<int64_t>(n, kThreads));
     w.total = c.take<unsigned long long>(2);
     w.guide_bits = guide_bits_for(n);
-    w.guide = c.take<uint4>((size_t)1 << w.guide_bits);
+    // one record more than there are buckets: its 32-byte loads need an alignment the caller's workspace need not have
+    const uintptr_t guide = reinterpret_cast<uintptr_t>(c.take<GuideRecord>(((size_t)1 << w.guide_bits) + 1));
+    w.guide = reinterpret_cast<uint4*>((guide + sizeof(GuideRecord) - 1) / sizeof(GuideRecord) * sizeof(GuideRecord));
     w.leaf_pack = c.take<float4>(n);
     w.bytes = c.used();
     return w;
 }
 
 // weight sum only (expected-sample mode) or sum + CDF.  `max_known`: the largest weight is in w.max_bits already.
-int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out, const SamplerWs& w, bool max_known, cudaStream_t stream) {
+int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out, const SamplerWs& w, bool max_known, cudaStream_t stream, const float4* leaf_pack = nullptr) {
     const int64_t chunks = ceil_div<int64_t>(n_cells, kCdfChunk);
     if (!max_known) {
         INPC_CUDA_TRY(cudaMemsetAsync(w.max_bits, 0, 4 * sizeof(unsigned), stream));
@@ -871,7 +953,7 @@ int build_cdf(const float* weights, int64_t n_cells, float* cdf, float* sum_out,
         INPC_LAUNCH_CHECK("cdf_finalize_kernel");
         if (cdf == w.cdf) {
             launch_chained(guide_table_kernel, (unsigned)ceil_div<int64_t>((int64_t)1 << w.guide_bits, kGuidePerBlock), kThreads, 0, stream,
-                cdf, (unsigned)n_cells, w.guide_bits, w.guide);
+                cdf, (unsigned)n_cells, w.guide_bits, w.guide, leaf_pack);
             INPC_LAUNCH_CHECK("guide_table_kernel");
         }
     }
@@ -1002,13 +1084,18 @@ extern "C" int inpc_generate_training_samples(inpc_sampler* s, const inpc_view* 
     StageScope scope(STAGE_SAMPLE, stream);
     rc = view_weights(v, n_cells, centers, levels, weights, initial_size, w, w.leaf_pack, stream);
     if (rc != INPC_OK) return rc;
-    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, true, stream);
+    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, true, stream, w.leaf_pack);
     if (rc != INPC_OK) return rc;
     unsigned* status = acquire_status("inpc_generate_training_samples", &s->training_ticket);
     if (!status) return INPC_E_CUDA;
-    launch_chained(training_samples_kernel, (unsigned)ceil_div<int64_t>(n_samples, kThreads), kThreads, 0, stream,
-        v, philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, w.sum, (unsigned)n_cells, w.leaf_pack, n_samples, positions,
-        reinterpret_cast<long long*>(indices), status);
+    constexpr int kPer = 2;   // small calls need the blocks
+    auto launch = [&](auto per) {
+        launch_chained(training_samples_kernel<decltype(per)::value>, (unsigned)ceil_div<int64_t>(n_samples, kThreads * decltype(per)::value), kThreads, 0, stream,
+            v, philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, w.sum, (unsigned)n_cells, w.leaf_pack, n_samples, positions,
+            reinterpret_cast<long long*>(indices), status);
+    };
+    if (n_samples >= (int64_t)kThreads * kPer * sm_count() * 4) launch(std::integral_constant<int, kPer>());
+    else launch(std::integral_constant<int, 1>());
     INPC_LAUNCH_CHECK("training_samples_kernel");
     s->counter += 1;
     return INPC_OK;
@@ -1027,7 +1114,7 @@ extern "C" int inpc_generate_samples(inpc_sampler* s, const inpc_view* view, int
     const ViewParams v = to_params(view);
     rc = view_weights(v, n_cells, centers, levels, weights, initial_size, w, w.leaf_pack, stream);
     if (rc != INPC_OK) return rc;
-    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, true, stream);
+    rc = build_cdf(w.vw, n_cells, w.cdf, w.sum, w, true, stream, w.leaf_pack);
     if (rc != INPC_OK) return rc;
     float* host = pinned_float();
     if (!host) return cuda_fail(cudaGetLastError(), "cudaHostAlloc");
