@@ -394,6 +394,15 @@ __device__ __forceinline__ uint32_t pack_quad(const Projection& pr, int tile_row
     const unsigned ry1 = (unsigned)(__float2int_rd(pr.sy - 0.5f) - ((int)pr.y0 - tile_rows_before) * 8 + 1);
     return (qx1 & 0x7FFFu) | ((pr.x1 - pr.x0 - 1u) << 15) | ((pr.y0 & 0x7FFu) << 16) | ((ry1 & 0xFu) << 27) | ((pr.y1 - pr.y0 - 1u) << 31);
 }
+constexpr uint32_t kNoQuad = 0xFFFFFFFFu;  // of a culled point (its column would lie beyond kMaxCodedSide)
+
+// Tile bounds of a splat in the form of the `bounds` array: the first tile is floor(origin / 8), never below 0.
+__device__ __forceinline__ uint2 quad_bounds(uint32_t q) {
+    if (q == kNoQuad) return make_uint2(0u, 0u);
+    const int qx = (int)(q & 0x7FFFu) - 1;
+    const unsigned x0 = qx < 0 ? 0u : (unsigned)qx >> 3, y0 = (q >> 16) & 0x7FFu;
+    return make_uint2(x0 | ((x0 + 1u + ((q >> 15) & 1u)) << 16), y0 | ((y0 + 1u + (q >> 31)) << 16));
+}
 
 // What the instance emission needs of a gaussian splat on 8x8 tiles: its tile bounds, and how far its ellipse stays away from
 // their sides in cells of 2x2 pixels, four bits each (left, right, top, bottom; rounded down, so the cells between are a superset).
@@ -476,14 +485,19 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     if (bulk) slab_ready = mbarrier_wait_bounded(&s_bar, 0u);
     if (!slab_ready && status) status[STATUS_BULK_COPY_TIMEOUT] = 1u;
     __syncthreads();
-    if (i >= n && iv < ps.start[ps.count]) bounds[iv] = make_uint2(0u, 0u);   // padding behind a set
+    // what the instance passes need of a point: its packed footprint where splats are bilinear on 8x8 tiles, else its tile bounds
+    // (both until now: 8 of 148 bytes per point)
+    auto write_bounds = [&](bool visible) {
+        if (MODE == INPC_MODE_BILINEAR && quad) quad[iv] = visible ? pack_quad(pr, set * rp.gh) : kNoQuad;
+        else bounds[iv] = visible ? make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16)) : make_uint2(0u, 0u);
+    };
+    if (i >= n && iv < ps.start[ps.count]) write_bounds(false);   // padding behind a set
     if (i < n && slab_ready) {
         if (pr.visible && VARIANT == VAR_ROWS) {
             // feature rows are gathered by the blend itself: the record carries the geometry only.  The warp blend reads such
             // records 16 bytes apart (rec_stride 1): half-written 32-byte sectors cost as much DRAM traffic as whole ones
             reinterpret_cast<float4*>(rec)[(size_t)iv * rec_stride] = make_float4(pr.sx, pr.sy, __ldg(opacities + i), pr.depth);
-            bounds[iv] = make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16));
-            if (quad) quad[iv] = pack_quad(pr, set * rp.gh);
+            write_bounds(true);
         } else if (pr.visible) {
             const __half* h = reinterpret_cast<const __half*>(s_feat) + threadIdx.x * kHalves;
             float b[9];
@@ -502,14 +516,13 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
             float4* dst = reinterpret_cast<float4*>(rec + iv);
             dst[0] = make_float4(r.sx, r.sy, r.opacity, r.depth);
             dst[1] = make_float4(r.f[0], r.f[1], r.f[2], r.f[3]);
-            bounds[iv] = make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16));
-            if (quad) quad[iv] = pack_quad(pr, set * rp.gh);
+            write_bounds(true);
             if (MODE == INPC_MODE_GAUSSIAN) {
                 conic[iv] = make_float4(pr.cx, pr.cy, pr.cz, 0.0f);
                 if (foot) foot[iv] = pack_footprint(pr, rp.reach);
             }
         } else {
-            bounds[iv] = make_uint2(0u, 0u);
+            write_bounds(false);
         }
     }
     unsigned total;
@@ -543,7 +556,7 @@ constexpr int kInstThreads = 1024;   // block sums over 1024 points keep the one
 template <bool PACKED>
 __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const uint32_t* __restrict__ sorted_keys,
                                                                           const uint32_t* __restrict__ sorted_ids,
-                                                                          const uint2* __restrict__ bounds, int64_t n_visible_arg,
+                                                                          const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
                                                                           const unsigned long long* __restrict__ n_visible_dev,
                                                                           unsigned* block_sums, unsigned n_groups, unsigned* done) {
     await_previous_kernel();
@@ -562,7 +575,13 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int64_t s = first + q;
-                if (s < n_visible) c += PACKED ? (__ldg(sorted_keys + s) >> kCountShift) + 1u : tiles_of(__ldg(bounds + checked_point(__ldg(sorted_ids + s))));
+                if (s >= n_visible) continue;
+                if (PACKED) {
+                    c += (__ldg(sorted_keys + s) >> kCountShift) + 1u;
+                } else {
+                    const uint32_t id = checked_point(__ldg(sorted_ids + s));
+                    c += tiles_of(quad ? quad_bounds(__ldg(quad + id)) : __ldg(bounds + id));
+                }
             }
         }
         c = __reduce_add_sync(0xffffffffu, c);
@@ -3648,7 +3667,7 @@ __global__ void __launch_bounds__(kPreThreads, 8) preprocess_backward_kernel(
 // ------------------------------------------------------------------------------------------------
 struct PointBlob {
     PointRec* rec;
-    uint2* bounds;
+    uint2* bounds;                        // tile bounds per point; not written where they follow from `quad`
     uint32_t* quad;                       // bilinear, warp blend: packed footprint origin per point (see pack_quad)
     float4* conic;
     uint4* foot;                          // gaussian, warp blend: tile bounds and ellipse per point (see pack_footprint)
@@ -4041,9 +4060,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles rides in the top key bits when the depth offsets left them free
             if (MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift)
-                launch_chained(instance_count_kernel<true>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
+                launch_chained(instance_count_kernel<true>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             else
-                launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
+                launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (warp_blend && MODE == INPC_MODE_GAUSSIAN)
                 launch_chained(emit_instances_kernel<EMIT_CELLS>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, nullptr, pb.foot, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
@@ -4744,12 +4763,12 @@ __global__ void add_base_kernel(const uint32_t* __restrict__ src, int64_t n, uin
     if (i < n) dst[i] = (src[i] & mask) + base;
 }
 
-__global__ void unpack_points_kernel(const PointRec* __restrict__ rec, int rec_stride, const uint2* __restrict__ bounds, int64_t n, int which,
+__global__ void unpack_points_kernel(const PointRec* __restrict__ rec, int rec_stride, const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, int64_t n, int which,
                                      void* __restrict__ dst) {
     await_previous_kernel();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint2 b = bounds[i];
+    const uint2 b = quad ? quad_bounds(quad[i]) : bounds[i];
     const bool vis = tiles_of(b) != 0u;
     const float4* r = reinterpret_cast<const float4*>(rec) + i * rec_stride;
     if (which == 4) static_cast<unsigned*>(dst)[i] = tiles_of(b);
@@ -4789,7 +4808,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
         case 3: INPC_CUDA_TRY(cudaMemcpyAsync(dst, ib.ranges, 8 * (size_t)n_tiles, cudaMemcpyDeviceToDevice, stream)); break;
         case 4: case 5: case 6: case 7: case 8:
             if (state->n_points > 0) {
-                launch_chained(inpc_debug::unpack_points_kernel, (unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream, pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, state->n_points, which, dst);
+                launch_chained(inpc_debug::unpack_points_kernel, (unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream, pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, pb.quad, state->n_points, which, dst);
                 INPC_LAUNCH_CHECK("unpack_points_kernel");
             }
             break;
