@@ -553,6 +553,8 @@ __device__ __forceinline__ unsigned tiles_of(const uint2 b) {
 // Instances per depth-sorted point, reduced per block (src/bilinear/kernels.cu:186-196 + the
 // cub::DeviceScan::ExclusiveSum of src/bilinear/forward.cu:109-115, first half).
 constexpr int kInstThreads = 1024;   // block sums over 1024 points keep the one-block scan short
+// Packed: a warp sums one block's worth of points, all its loads in flight together, no barrier before the last block's scan (a barrier
+// per group of a block and one load per thread: 2^23 / 2^25 points 16 / 61 -> 11 / 39 us).
 template <bool PACKED>
 __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const uint32_t* __restrict__ sorted_keys,
                                                                           const uint32_t* __restrict__ sorted_ids,
@@ -561,37 +563,47 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
                                                                           unsigned* block_sums, unsigned n_groups, unsigned* done) {
     await_previous_kernel();
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
-    // a block of kInstThreads / 4 threads covers kInstThreads points, four consecutive ones per thread
-    // (one 16-byte load when the keys carry the count), and takes several such groups one after the other
-    __shared__ unsigned s_w[2][kInstThreads / 4 / 32];
-    int flip = 0;
-    for (unsigned group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1) {
-        const int64_t first = (int64_t)group * kInstThreads + 4 * (int64_t)threadIdx.x;
-        unsigned c = 0;
-        if (PACKED && first + 4 <= n_visible) {
-            const uint4 k = __ldg(reinterpret_cast<const uint4*>(sorted_keys + first));   // the key buffers are 16-byte aligned
-            c = (k.x >> kCountShift) + (k.y >> kCountShift) + (k.z >> kCountShift) + (k.w >> kCountShift) + 4u;
-        } else {
+    constexpr unsigned kWarps = kInstThreads / 4 / 32;
+    if (PACKED) {
+        constexpr int kLoads = kInstThreads / 128;   // 16-byte loads per lane and group
+        for (unsigned group = blockIdx.x * kWarps + (threadIdx.x >> 5); group < n_groups; group += gridDim.x * kWarps) {
+            const int64_t first = (int64_t)group * kInstThreads + 4 * (int64_t)lane_id();
+            unsigned c = 0;
+            if ((int64_t)(group + 1) * kInstThreads <= n_visible) {
+                uint4 k[kLoads];
+#pragma unroll
+                for (int q = 0; q < kLoads; ++q) k[q] = __ldg(reinterpret_cast<const uint4*>(sorted_keys + first + 128 * q));   // the key buffers are 16-byte aligned
+#pragma unroll
+                for (int q = 0; q < kLoads; ++q) c += (k[q].x >> kCountShift) + (k[q].y >> kCountShift) + (k[q].z >> kCountShift) + (k[q].w >> kCountShift) + 4u;
+            } else {
+                for (int64_t s = (int64_t)group * kInstThreads + lane_id(); s < n_visible; s += 32) c += (__ldg(sorted_keys + s) >> kCountShift) + 1u;
+            }
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (lane_id() == 0) block_sums[group] = c;
+        }
+    } else {
+        // two dependent gathers per point: a block per group, so that more of them are in flight (a warp per group: 16 -> 27 us for 2 * 10^6 points)
+        __shared__ unsigned s_w[2][kWarps];
+        int flip = 0;
+        for (unsigned group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1) {
+            const int64_t first = (int64_t)group * kInstThreads + 4 * (int64_t)threadIdx.x;
+            unsigned c = 0;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int64_t s = first + q;
                 if (s >= n_visible) continue;
-                if (PACKED) {
-                    c += (__ldg(sorted_keys + s) >> kCountShift) + 1u;
-                } else {
-                    const uint32_t id = checked_point(__ldg(sorted_ids + s));
-                    c += tiles_of(quad ? quad_bounds(__ldg(quad + id)) : __ldg(bounds + id));
-                }
+                const uint32_t id = checked_point(__ldg(sorted_ids + s));
+                c += tiles_of(quad ? quad_bounds(__ldg(quad + id)) : __ldg(bounds + id));
             }
-        }
-        c = __reduce_add_sync(0xffffffffu, c);
-        if (lane_id() == 0) s_w[flip][threadIdx.x >> 5] = c;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned t = 0;
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (lane_id() == 0) s_w[flip][threadIdx.x >> 5] = c;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                unsigned t = 0;
 #pragma unroll
-            for (int w = 0; w < kInstThreads / 4 / 32; ++w) t += s_w[flip][w];
-            block_sums[group] = t;
+                for (unsigned w = 0; w < kWarps; ++w) t += s_w[flip][w];
+                block_sums[group] = t;
+            }
         }
     }
     __shared__ unsigned s_scan[kInstThreads / 4 / 32 + 1];
@@ -627,10 +639,12 @@ __device__ __forceinline__ unsigned cell_code(int left, int right, int top, int 
 // order (src/bilinear/kernels.cu:198-220).  EMIT_QUAD (bilinear, 8x8 tiles): bounds and footprint origin come
 // from the packed word the projection pass left per point (see pack_quad), a 4-byte gather.  EMIT_CELLS (gaussian, 8x8 tiles):
 // the key also says which cells of the tile the ellipse can reach (see cell_code).
-// Bound by the throughput of the random 4-byte gathers, one 32-byte sector each, not by their latency.  What is read or written
-// once bypasses the caches' replacement, so that more of the gathered array stays in L2: 2^23 / 2^24 / 2^25 points
-// 104 / 221 / 488 -> 97 / 205 / 469 us.  (Four consecutive points per thread with their gathers in flight together and the
-// instances staged in shared memory: 116 / 396 / 952 us, the gathers of fewer, busier warps miss L2 more often.)
+// Bound by the random 4-byte gathers, one 32-byte sector each, and by instruction issue.  What is read or written once bypasses
+// the caches' replacement, so that more of the gathered array stays in L2.  A bilinear splat has one, two or four instances: the sums over a warp
+// come from three ballots, those over a block from one barrier and a warp reduction, and the keys are put together without a loop: 2^23 / 2^24 /
+// 2^25 points 97 / 204 / 451 -> 85 / 178 / 455 us (a scan of three barriers and loops over the tiles, 189 instructions per warp; the last
+// is bound by DRAM, the gathered array being larger than L2).  (Four consecutive points per thread with their gathers in
+// flight together and the instances staged in shared memory: 116 / 396 / 952 us.)
 enum { EMIT_BOUNDS = 0, EMIT_QUAD = 1, EMIT_CELLS = 2 };
 template <int KEYS>
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
@@ -640,47 +654,69 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
                                                                       uint32_t* __restrict__ inst_keys,
                                                                       uint32_t* __restrict__ inst_ids) {
     await_previous_kernel();
-    __shared__ unsigned s_scan[kInstThreads / 32 + 1];
+    __shared__ unsigned s_total[kInstThreads / 32];
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     if ((int64_t)blockIdx.x * kInstThreads >= n_visible) return;
     const int64_t s = (int64_t)blockIdx.x * kInstThreads + threadIdx.x;
-    uint32_t id = 0;
-    unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0, inset = 0;
-    int qx = 0, qy = 0;
-    if (s < n_visible) {
-        id = checked_point(__ldcs(sorted_ids + s));
-        if (KEYS == EMIT_QUAD) {
-            // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0
-            const uint32_t q = __ldg(quad + id);
-            qx = (int)(q & 0x7FFFu) - 1;
-            x0 = qx < 0 ? 0u : (unsigned)qx >> 3;
-            y0 = (q >> 16) & 0x7FFu;
-            qy = (int)y0 * 8 + (int)((q >> 27) & 0xFu) - 1;   // row of the upper pixel in the stacked grid (or one above its image)
-            x1 = x0 + 1u + ((q >> 15) & 1u);
-            y1 = y0 + 1u + (q >> 31);
-        } else {
-            uint2 b;
-            if (KEYS == EMIT_CELLS) {
-                const uint4 f = __ldg(foot + id);
-                b = make_uint2(f.x, f.y);
-                inset = f.z;
-            } else {
-                b = __ldg(bounds + id);
-            }
-            x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const bool there = s < n_visible;
+    const uint32_t id = there ? checked_point(__ldcs(sorted_ids + s)) : 0u;
+    // instances of the warps of this block before this one; one barrier
+    auto before_warp = [&](unsigned total) -> unsigned {
+        if (lane == 0) s_total[warp] = total;
+        __syncthreads();
+        return __ldg(block_base + blockIdx.x) + __reduce_add_sync(0xffffffffu, lane < warp ? s_total[lane] : 0u);
+    };
+    if (KEYS == EMIT_QUAD) {
+        const uint32_t q = there ? __ldg(quad + id) : 0u;
+        const bool two_columns = there && ((q >> 15) & 1u), two_rows = there && (q >> 31);
+        // one, two or four instances per point: the sum over the lanes before this one from three ballots
+        const unsigned bt = __ballot_sync(0xffffffffu, there), bc = __ballot_sync(0xffffffffu, two_columns), br = __ballot_sync(0xffffffffu, two_rows);
+        const unsigned lt_mask = (1u << lane) - 1u;
+        unsigned off = before_warp(__popc(bt) + __popc(bc) + __popc(br) + __popc(bc & br)) + __popc(bt & lt_mask) + __popc(bc & lt_mask) + __popc(br & lt_mask) +
+                       __popc(bc & br & lt_mask);
+        if (!there) return;
+        // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0.  In a second column or
+        // row of tiles the footprint starts one pixel before the tile: its code there is zero
+        const int qx = (int)(q & 0x7FFFu) - 1;
+        const unsigned x0 = qx < 0 ? 0u : (unsigned)qx >> 3, y0 = (q >> 16) & 0x7FFu;
+        const uint32_t column = (unsigned)(qx - (int)x0 * 8 + 1) << kTileKeyBits, row = min((q >> 27) & 0xFu, 8u) << (kTileKeyBits + 4);
+        const uint32_t tile = y0 * (unsigned)gw + x0;
+        __stcs(inst_keys + off, tile | column | row);
+        __stcs(inst_ids + off, id);
+        if (two_columns) {
+            __stcs(inst_keys + off + 1u, (tile + 1u) | row);
+            __stcs(inst_ids + off + 1u, id);
         }
+        if (two_rows) {
+            off += two_columns ? 2u : 1u;
+            __stcs(inst_keys + off, (tile + (unsigned)gw) | column);
+            __stcs(inst_ids + off, id);
+            if (two_columns) {
+                __stcs(inst_keys + off + 1u, tile + (unsigned)gw + 1u);
+                __stcs(inst_ids + off + 1u, id);
+            }
+        }
+        return;
+    }
+    unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0, inset = 0;
+    if (there) {
+        uint2 b;
+        if (KEYS == EMIT_CELLS) {
+            const uint4 f = __ldg(foot + id);
+            b = make_uint2(f.x, f.y);
+            inset = f.z;
+        } else {
+            b = __ldg(bounds + id);
+        }
+        x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
     }
     const unsigned c = (x1 - x0) * (y1 - y0);
-    unsigned total;
-    unsigned off = block_base[blockIdx.x] + block_exclusive_scan(c, s_scan, &total);
+    const unsigned inc = warp_inclusive_scan(c);
+    unsigned off = before_warp(__shfl_sync(0xffffffffu, inc, 31)) + inc - c;
     for (unsigned ty = y0; ty < y1; ++ty)
         for (unsigned tx = x0; tx < x1; ++tx) {
             uint32_t key = ty * (unsigned)gw + tx;
-            if (KEYS == EMIT_QUAD) {
-                const unsigned cx = (unsigned)min(max(qx - (int)tx * 8 + 1, 0), 8);
-                const unsigned cy = (unsigned)min(max(qy - (int)ty * 8 + 1, 0), 8);
-                key |= (cx << kTileKeyBits) | (cy << (kTileKeyBits + 4));
-            }
             if (KEYS == EMIT_CELLS) {
                 const int left = (int)(inset & 15u) - 4 * (int)(tx - x0), right = 4 * (int)(x1 - tx) - 1 - (int)((inset >> 4) & 15u);
                 const int top = (int)((inset >> 8) & 15u) - 4 * (int)(ty - y0), bottom = 4 * (int)(y1 - ty) - 1 - (int)(inset >> 12);
@@ -4054,8 +4090,8 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     if (rc != INPC_OK) return rc;
     const uint32_t* sorted_ids = pb.ids[in_alt];
     if (n_visible > 0 && n_instances > 0) {
-        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_cap = (int64_t)sm_count() * 8;
-        const unsigned count_blocks = (unsigned)(ibk < count_cap ? ibk : count_cap);
+        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_need = MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift ? ceil_div<int64_t>(ibk, kInstThreads / 4 / 32) : ibk, count_cap = (int64_t)sm_count() * 8;
+        const unsigned count_blocks = (unsigned)(count_need < count_cap ? count_need : count_cap);
         {
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles rides in the top key bits when the depth offsets left them free
