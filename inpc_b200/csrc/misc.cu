@@ -51,17 +51,31 @@ __global__ void __launch_bounds__(kThreads) weight_decay_kernel(const float* __r
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     const int64_t tid = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int64_t n4 = vec_ok ? n / 4 : 0;
-    for (int64_t v = tid; v < n4; v += stride) {
-        const float f = decay_factor((unsigned)(4 * v));
-        const float4 wv = __ldg(reinterpret_cast<const float4*>(w) + v);
-        float4 gv;
-        if (ADD) {
-            gv = reinterpret_cast<float4*>(g)[v];
-            gv.x += f * wv.x; gv.y += f * wv.y; gv.z += f * wv.z; gv.w += f * wv.w;
-        } else {
-            gv = make_float4(f * wv.x, f * wv.y, f * wv.z, f * wv.w);
+    // 12 bytes per parameter, read and written once: four vectors per thread in flight and no room taken in the caches bring it to the rate of a
+    // plain copy (210.9 * 10^6 parameters: one vector 410 us, two 396, four 392)
+    constexpr int kPer = 4;
+    for (int64_t v0 = tid; v0 < n4; v0 += stride * kPer) {
+        float4 wv[kPer], gv[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int64_t v = v0 + k * stride;
+            if (v < n4) {
+                wv[k] = __ldcs(reinterpret_cast<const float4*>(w) + v);
+                if (ADD) gv[k] = __ldcs(reinterpret_cast<const float4*>(g) + v);
+            }
         }
-        reinterpret_cast<float4*>(g)[v] = gv;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int64_t v = v0 + k * stride;
+            if (v >= n4) continue;
+            const float f = decay_factor((unsigned)(4 * v));
+            if (ADD) {
+                gv[k].x += f * wv[k].x; gv[k].y += f * wv[k].y; gv[k].z += f * wv[k].z; gv[k].w += f * wv[k].w;
+            } else {
+                gv[k] = make_float4(f * wv[k].x, f * wv[k].y, f * wv[k].z, f * wv[k].w);
+            }
+            __stcs(reinterpret_cast<float4*>(g) + v, gv[k]);
+        }
     }
     for (int64_t i = 4 * n4 + tid; i < n; i += stride) {
         const float f = decay_factor((unsigned)i);
