@@ -598,46 +598,65 @@ __device__ __forceinline__ void find_leaf_run(LeafRun& run, const unsigned* __re
     __syncthreads();
 }
 
-__device__ __forceinline__ unsigned leaf_of_slot(const LeafRun& run, const unsigned* __restrict__ offsets, unsigned r) {
+// The leaf (index within the run) of slot r, r ascending over the lanes of a warp and from row to row; `k`: where the last row ended, all lanes
+// the same.  Most rows lie in one leaf, which one comparison shows; the others search from there.
+__device__ __forceinline__ unsigned leaf_of_row(const LeafRun& run, const unsigned* __restrict__ offsets, unsigned r, unsigned& k) {
     const unsigned m = run.count;
-    unsigned first = 0, count = m;
-    if (m <= kRunLeaves) {
+    const bool local = m <= kRunLeaves;
+    auto end_of = [&](unsigned l) { return local ? run.offsets[l] : __ldg(offsets + run.first + l); };
+    unsigned l = k;
+    if (__any_sync(0xffffffffu, l + 1u < m && end_of(l) <= r)) {
+        unsigned count = m - l;
         while (count > 0) {
             const unsigned step = count >> 1;
-            if (run.offsets[first + step] <= r) { first += step + 1; count -= step + 1; }
+            if (end_of(l + step) <= r) { l += step + 1; count -= step + 1; }
             else count = step;
         }
-    } else {
-        while (count > 0) {
-            const unsigned step = count >> 1;
-            if (__ldg(offsets + run.first + first + step) <= r) { first += step + 1; count -= step + 1; }
-            else count = step;
-        }
+        l = min(l, m - 1u);
     }
-    return run.first + min(first, m - 1u);
+    k = __shfl_sync(0xffffffffu, l, 31);
+    return l;
+}
+
+// The positions of a warp's row of `here` consecutive slots leave as 16-byte vectors where they are aligned, in whole 128-byte lines otherwise.
+__device__ __forceinline__ void store_row(float* s_row, float x, float y, float z, unsigned here, float* __restrict__ dst) {
+    const unsigned lane = lane_id();
+    __syncwarp();   // the row before has been read
+    s_row[3 * lane] = x; s_row[3 * lane + 1] = y; s_row[3 * lane + 2] = z;
+    __syncwarp();
+    if (here == 32u && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        if (lane < 24u) reinterpret_cast<float4*>(dst)[lane] = reinterpret_cast<const float4*>(s_row)[lane];
+    } else {
+#pragma unroll
+        for (unsigned k = 0; k < 3; ++k)
+            if (32u * k + lane < 3u * here) dst[32u * k + lane] = s_row[32u * k + lane];
+    }
 }
 
 // slot i jitters inside leaf upper_bound(offsets, i % n_created): the load-balanced form of the reference's per-leaf fill
-// loop + gather.  blockIdx.y counts the copies i / n_created, whose slots a run never leaves.
+// loop + gather.  blockIdx.y counts the copies i / n_created, whose slots a run never leaves; a warp takes kRunPerThread rows of 32 consecutive
+// slots, finds their leaves once for all copies (before: a search in every slot and copy, the run found once per copy, and a barrier per store: 4 x 2^23 slots 242 -> 156 us).
 __global__ void __launch_bounds__(kThreads) expected_samples_kernel(const __grid_constant__ PhiloxKeys keys,
                                                                     const unsigned* __restrict__ offsets, unsigned n_cells,
                                                                     const float4* __restrict__ leaf_pack, unsigned n_created,
                                                                     unsigned n_copies, float* __restrict__ positions) {
     await_previous_kernel();
     __shared__ LeafRun run;
-    __shared__ __align__(16) float s_pos[3 * kThreads];
+    __shared__ __align__(16) float s_pos[kThreads / 32][96];
     const unsigned r0 = blockIdx.x * (unsigned)kRunSlots;
     const unsigned in_block = min((unsigned)kRunSlots, n_created - r0);
     find_leaf_run(run, offsets, n_cells, r0, r0 + in_block - 1u);
-    for (unsigned copy = blockIdx.y; copy < n_copies; copy += gridDim.y) {
-        const int64_t copy_first = (int64_t)copy * n_created, copy_end = copy_first + n_created;
-        for (unsigned k0 = 0; k0 < in_block; k0 += kThreads) {
-            const unsigned r = min(r0 + k0 + threadIdx.x, n_created - 1u);
-            const float4 lp = __ldg(leaf_pack + leaf_of_slot(run, offsets, r));
+    const unsigned warp = threadIdx.x >> 5, lane = lane_id();
+    unsigned k = 0;
+    for (unsigned row = 0; row < (unsigned)kRunPerThread; ++row) {
+        const unsigned first = (warp * kRunPerThread + row) * 32u;
+        if (first >= in_block) break;
+        const unsigned here = min(32u, in_block - first), r = r0 + first + min(lane, here - 1u);
+        const float4 lp = __ldg(leaf_pack + run.first + leaf_of_row(run, offsets, r, k));
+        for (unsigned copy = blockIdx.y; copy < n_copies; copy += gridDim.y) {
+            const int64_t copy_first = (int64_t)copy * n_created;
             const Draw d = philox_draw(keys, (unsigned)(copy_first + r), 0u);
-            store_positions(s_pos, fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), copy_first + r0 + k0,
-                            copy_end, positions);
-            __syncthreads();
+            store_row(s_pos[warp], fmaf(d.jx - 0.5f, lp.w, lp.x), fmaf(d.jy - 0.5f, lp.w, lp.y), fmaf(d.jz - 0.5f, lp.w, lp.z), here, positions + 3 * (copy_first + r0 + first));
         }
     }
 }
@@ -646,11 +665,24 @@ __global__ void __launch_bounds__(kThreads) expected_samples_kernel(const __grid
 // counts[leaf] = number of the n multinomial draws that fell into the leaf (torch.multinomial +
 // bincount in the reference; here the library's own Philox stream, one draw per slot)
 constexpr int kDrawsPerThread = 4;
+// One counter takes an addition every 2.7 ns, and the heaviest of 2.3 * 10^5 leaves of a trained field is drawn every two hundredth time: with
+// one array of counts that leaf alone set the time: 2^25 draws 355 us, with 4 / 8 / 16 arrays 294 / 270 / 264.  The blocks share kCountParts, added up afterwards.
+constexpr unsigned kCountParts = 8;
+constexpr int64_t kManyDraws = 1 << 20;
+__global__ void __launch_bounds__(kThreads) add_count_parts_kernel(const unsigned* __restrict__ parts, int64_t n, unsigned n_parts, unsigned* __restrict__ counts) {
+    await_previous_kernel();
+    const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    if (i >= n) return;
+    unsigned sum = 0;
+    for (unsigned k = 0; k < n_parts; ++k) sum += __ldg(parts + k * n + i);
+    counts[i] = sum;
+}
 __global__ void __launch_bounds__(kThreads) leaf_histogram_kernel(const __grid_constant__ PhiloxKeys keys,
                                                                   const float* __restrict__ cdf, const uint4* __restrict__ guide,
                                                                   int guide_bits, unsigned n_cells, int64_t n_samples,
-                                                                  unsigned* __restrict__ counts) {
+                                                                  unsigned* __restrict__ counts, unsigned n_parts) {
     await_previous_kernel();
+    counts += (size_t)(blockIdx.x % n_parts) * n_cells;
     // the table gathers of a thread's draws are in flight together
     const int64_t first = (int64_t)blockIdx.x * (kThreads * kDrawsPerThread) + threadIdx.x;
     unsigned leaf[kDrawsPerThread];
@@ -674,7 +706,7 @@ template <unsigned B, int HEAD, int DIGITS>
 struct HaltonTable {
     static constexpr unsigned kBase = B;
     static constexpr int kHead = HEAD;         // digits summed up in advance
-    static constexpr unsigned kHeads = B == 3u ? 81u : 125u;   // B^HEAD
+    static constexpr unsigned kHeads = B == 3u ? 729u : 625u;   // B^HEAD
     double head[kHeads];
     double term[DIGITS][B];                    // digit value * f
     constexpr HaltonTable() : head(), term() {
@@ -692,10 +724,9 @@ struct HaltonTable {
     }
 };
 struct HaltonTables {
-    HaltonTable<3u, 4, 21> b3;
-    HaltonTable<5u, 3, 14> b5;
+    HaltonTable<3u, 6, 21> b3;
+    HaltonTable<5u, 4, 14> b5;
 };
-static_assert(sizeof(HaltonTables) % 8 == 0, "copied as doubles");
 __device__ const HaltonTables g_halton{};
 
 __device__ __forceinline__ float halton_base2(unsigned index) {
@@ -716,36 +747,63 @@ __device__ __forceinline__ float halton_element(const Table& t, unsigned index) 
 // Sample i lies in leaf upper_bound(offsets, i) and is that leaf's h-th sample, h = i - first sample
 // of the leaf: Halton point h+1 in bases (2, 3, 5) scaled into the cell; a leaf with a single sample
 // puts it at its centre (ProbabilityField.py:131-140).
+// Bound by instruction issue.  Of a run's leaves the corner and the edge lie in shared memory, a warp finds the leaves of 32 consecutive samples
+// at a time, and heads of 729 and 625 values, read through L1, settle most digits: 2^25 samples of 2.3 * 10^5 leaves 234 -> 197 us (before: a
+// search, six gathers and a division per sample, heads of 81 and 125 values in shared memory; with those and the rest as here 212, with the long heads in shared
+// memory 201, with persistent blocks 229 to 254).
+constexpr unsigned kRunRecords = 256;   // leaves of a run whose records are staged; a run over more makes them per sample
+struct HaltonLeaf {
+    float x, y, z, cell;   // lower corner and edge, or the centre where there is a single sample
+};
+__device__ __forceinline__ HaltonLeaf halton_leaf(const float* __restrict__ centers, const int* __restrict__ levels, float initial_size, unsigned leaf, unsigned count) {
+    HaltonLeaf l;
+    l.x = __ldg(centers + 3 * (int64_t)leaf); l.y = __ldg(centers + 3 * (int64_t)leaf + 1); l.z = __ldg(centers + 3 * (int64_t)leaf + 2);
+    l.cell = 0.0f;
+    if (count != 1u) {
+        // cell edge = initial_size / 2^level, exact in fp32 for the levels an octree has; every further
+        // operation rounds on its own like the torch expression  centre - cell/2 + halton * cell
+        l.cell = __fdiv_rn(initial_size, (float)(1u << __ldg(levels + leaf)));
+        const float half = __fmul_rn(l.cell, 0.5f);
+        l.x = __fsub_rn(l.x, half); l.y = __fsub_rn(l.y, half); l.z = __fsub_rn(l.z, half);
+    }
+    return l;
+}
 __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned* __restrict__ counts, const unsigned* __restrict__ offsets,
                                                                   unsigned n_cells, const float* __restrict__ centers,
                                                                   const int* __restrict__ levels, float initial_size, unsigned n_total,
                                                                   float* __restrict__ positions) {
     await_previous_kernel();
     __shared__ LeafRun run;
-    __shared__ __align__(16) float s_pos[3 * kThreads];
-    __shared__ double s_tables[sizeof(HaltonTables) / 8];
-    const HaltonTables& tables = *reinterpret_cast<const HaltonTables*>(s_tables);
-    for (unsigned k = threadIdx.x; k < sizeof(HaltonTables) / 8; k += kThreads) s_tables[k] = reinterpret_cast<const double*>(&g_halton)[k];
+    __shared__ unsigned s_start;   // first sample of the run's first leaf
+    __shared__ HaltonLeaf s_leaf[kRunRecords];
+    __shared__ __align__(16) float s_pos[kThreads / 32][96];
+    const HaltonTables& tables = g_halton;
+    const unsigned warp = threadIdx.x >> 5, lane = lane_id();
     const unsigned r0 = blockIdx.x * (unsigned)kRunSlots;
     const unsigned in_block = min((unsigned)kRunSlots, n_total - r0);
     find_leaf_run(run, offsets, n_cells, r0, r0 + in_block - 1u);
-    for (unsigned k0 = 0; k0 < in_block; k0 += kThreads) {
-        const unsigned i = min(r0 + k0 + threadIdx.x, n_total - 1u);
-        const unsigned leaf = leaf_of_slot(run, offsets, i);
-        const unsigned c = __ldg(counts + leaf);
-        const unsigned h = i - (__ldg(offsets + leaf) - c);
-        float x = __ldg(centers + 3 * (int64_t)leaf), y = __ldg(centers + 3 * (int64_t)leaf + 1), z = __ldg(centers + 3 * (int64_t)leaf + 2);
+    const unsigned m = run.count, leaf0 = run.first;
+    const bool staged = m <= kRunRecords;
+    if (threadIdx.x == 0) s_start = __ldg(offsets + leaf0) - __ldg(counts + leaf0);
+    if (staged)
+        for (unsigned k = threadIdx.x; k < m; k += kThreads) s_leaf[k] = halton_leaf(centers, levels, initial_size, leaf0 + k, __ldg(counts + leaf0 + k));
+    __syncthreads();
+    unsigned k = 0;
+    for (unsigned row = 0; row < (unsigned)kRunPerThread; ++row) {
+        const unsigned first = (warp * kRunPerThread + row) * 32u;
+        if (first >= in_block) break;
+        const unsigned here = min(32u, in_block - first), i = r0 + first + min(lane, here - 1u);
+        const unsigned l = leaf_of_row(run, offsets, i, k);
+        const unsigned c = __ldg(counts + leaf0 + l);
+        const unsigned h = i - (l == 0u ? s_start : m <= kRunLeaves ? run.offsets[l - 1u] : __ldg(offsets + leaf0 + l - 1u));
+        const HaltonLeaf at = staged ? s_leaf[l] : halton_leaf(centers, levels, initial_size, leaf0 + l, c);
+        float x = at.x, y = at.y, z = at.z;
         if (c != 1u) {
-            // cell edge = initial_size / 2^level, exact in fp32 for the levels an octree has; every further
-            // operation rounds on its own like the torch expression  centre - cell/2 + halton * cell
-            const float cell = __fdiv_rn(initial_size, (float)(1u << __ldg(levels + leaf)));
-            const float half = __fmul_rn(cell, 0.5f);
-            x = __fadd_rn(__fsub_rn(x, half), __fmul_rn(halton_base2(h + 1u), cell));
-            y = __fadd_rn(__fsub_rn(y, half), __fmul_rn(halton_element(tables.b3, h + 1u), cell));
-            z = __fadd_rn(__fsub_rn(z, half), __fmul_rn(halton_element(tables.b5, h + 1u), cell));
+            x = __fadd_rn(x, __fmul_rn(halton_base2(h + 1u), at.cell));
+            y = __fadd_rn(y, __fmul_rn(halton_element(tables.b3, h + 1u), at.cell));
+            z = __fadd_rn(z, __fmul_rn(halton_element(tables.b5, h + 1u), at.cell));
         }
-        store_positions(s_pos, x, y, z, (int64_t)r0 + k0, n_total, positions);
-        __syncthreads();
+        store_row(s_pos[warp], x, y, z, here, positions + 3 * (int64_t)(r0 + first));
     }
 }
 
@@ -900,6 +958,7 @@ struct SamplerWs {
     unsigned* max_bits;                 // [0] bit pattern of the largest weight, [1] finished blocks of the CDF's sums, [2] of the counts': zero before
     float* sum;         // 1 float (+ padding)
     unsigned* counts;   // expected-sample counts (n_cells)
+    unsigned* count_parts;   // kCountParts arrays of draw counts
     unsigned* offsets;  // inclusive offsets (n_cells)
     unsigned* chunk_sums;
     unsigned long long* total;
@@ -926,6 +985,7 @@ SamplerWs carve_sampler_ws(void* p, int64_t n_cells) {
     w.max_bits = c.take<unsigned>(4);
     w.sum = c.take<float>(4);
     w.counts = c.take<unsigned>(n);
+    w.count_parts = c.take<unsigned>((size_t)n * kCountParts);
     w.offsets = c.take<unsigned>(n);
     w.chunk_sums = c.take<unsigned>(ceil_div<int64_t>(n, kThreads));
     w.total = c.take<unsigned long long>(2);
@@ -1174,7 +1234,9 @@ extern "C" int inpc_generate_expected_samples_fill(inpc_sampler* s, int64_t n_ce
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     launch_chained(leaf_records_kernel, (unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream, n_cells, centers, levels, initial_size, w.leaf_pack);
     INPC_LAUNCH_CHECK("leaf_records_kernel");
-    const dim3 grid((unsigned)ceil_div<int64_t>(n_created, kRunSlots), (unsigned)(n_multi < 65535 ? n_multi : 65535));
+    // all copies in one block where there are blocks enough without
+    const int64_t runs = ceil_div<int64_t>(n_created, kRunSlots), copies = runs >= (int64_t)sm_count() * 8 ? 1 : n_multi < 65535 ? n_multi : 65535;
+    const dim3 grid((unsigned)runs, (unsigned)copies);
     launch_chained(expected_samples_kernel, grid, kThreads, 0, stream, philox_keys(s->seed, s->counter), w.offsets, (unsigned)n_cells, w.leaf_pack, (unsigned)n_created,
                                                            (unsigned)n_multi, positions);
     INPC_LAUNCH_CHECK("expected_samples_kernel");
@@ -1205,7 +1267,10 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     int rc = build_cdf(weights, n_cells, w.cdf, w.sum, w, false, stream);
     if (rc != INPC_OK) return rc;
-    INPC_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * (size_t)n_cells, stream));
+    // few draws per leaf and block do not wait for one another
+    const unsigned n_parts = n_samples >= kManyDraws ? kCountParts : 1u;
+    unsigned* parts = n_parts > 1u ? w.count_parts : counts;
+    INPC_CUDA_TRY(cudaMemsetAsync(parts, 0, sizeof(uint32_t) * (size_t)n_cells * n_parts, stream));
     float* host = pinned_float();
     if (!host) return cuda_fail(cudaGetLastError(), "cudaHostAlloc");
     INPC_CUDA_TRY(cudaMemcpyAsync(host, w.sum, sizeof(float), cudaMemcpyDeviceToHost, stream));
@@ -1213,8 +1278,12 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
     if (!(host[0] > 0.0f)) { set_error("inpc_draw_leaf_counts: the weights sum to zero"); return INPC_E_INVALID; }
     if (n_samples > 0) {
         launch_chained(leaf_histogram_kernel, (unsigned)ceil_div<int64_t>(n_samples, kThreads * kDrawsPerThread), kThreads, 0, stream,
-            philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, n_samples, counts);
+            philox_keys(s->seed, s->counter), w.cdf, w.guide, w.guide_bits, (unsigned)n_cells, n_samples, parts, n_parts);
         INPC_LAUNCH_CHECK("leaf_histogram_kernel");
+        if (n_parts > 1u) {
+            launch_chained(add_count_parts_kernel, (unsigned)ceil_div<int64_t>(n_cells, kThreads), kThreads, 0, stream, parts, n_cells, n_parts, counts);
+            INPC_LAUNCH_CHECK("add_count_parts_kernel");
+        }
     }
     s->counter += 1;
     return INPC_OK;
