@@ -1,0 +1,62 @@
+"""GPU tests of the sampler at the sizes where its kernels take another form: slots draw from streams of their own, so what a slot
+gets must not depend on how many slots, copies or arrays of counts a call has."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _scene():
+    import synthetic_workloads as syn
+    tree = syn.adaptive_octree(20000, seed=7, min_level=3, max_level=7)
+    return tree.to(DEV), syn.orbit_view(0.8, -0.3, 2.2, 200, 150, 170.0).to(DEV)      # part of the tree is outside
+
+
+def _training(n):
+    from inpc_b200 import ProbabilityFieldSampler
+    t, v = _scene()
+    return ProbabilityFieldSampler(11).generate_training_samples(t.centers, t.levels, t.weights, v, n, t.initial_size)
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 511, 513, 400_001])
+def test_training_samples_of_a_slot_do_not_depend_on_the_call(n):
+    # one slot per thread below some 300,000 samples, two above; the blocks' last slots and retries at every remainder
+    few, many = _training(n), _training(700_003)
+    assert torch.equal(few[0], many[0][:n]) and torch.equal(few[1], many[1][:n])
+
+
+@pytest.mark.parametrize("n", [1500, 40_000, 2_600_000])
+def test_copies_of_expected_samples_share_their_leaves(n):
+    from inpc_b200 import ProbabilityFieldSampler
+    t, v = _scene()
+    args = (t.centers, t.levels, t.weights, v, n)
+    one = ProbabilityFieldSampler(5).generate_expected_samples(*args, 1, t.initial_size)
+    three = ProbabilityFieldSampler(5).generate_expected_samples(*args, 3, t.initial_size)
+    m = one.shape[0]
+    assert three.shape[0] == 3 * m and torch.equal(three[:m], one)      # the first copy has the slots 0 .. m - 1
+    # every slot's copies lie in the same cell: no further apart than its edge on any axis (2^-3 of the cube at most)
+    assert float((three.view(3, m, 3) - one).abs().max()) <= t.initial_size * 2.0 ** -3
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 4099])
+def test_leaf_counts_in_one_and_in_several_arrays(n):
+    from inpc_b200 import ProbabilityFieldSampler
+    w = torch.rand(3001, generator=torch.Generator().manual_seed(3)).to(DEV) ** 8
+    below, counts = (ProbabilityFieldSampler(5).draw_leaf_counts(w, k).long() for k in ((1 << 20) - 1, n))
+    more = counts - below                                                # the slots both have draw the same
+    assert int(counts.sum()) == n and int(more.min()) >= 0 and int(more.sum()) == n - (1 << 20) + 1
+
+
+@pytest.mark.parametrize("n", [3, 4, 1023, 4 * 256 * 3 + 1])
+def test_weight_decay_at_the_edges_of_its_vectors(n):
+    from inpc_b200 import add_normalized_weight_decay_grads
+    g = torch.Generator().manual_seed(n)
+    n += 6144                                                            # below that index the factor is zero
+    p = torch.nn.Parameter(torch.randn(n, generator=g).to(DEV))
+    p.grad = torch.randn(n, generator=g).to(DEV)
+    want = p.grad.double()
+    want[6144:] += p.detach()[6144:].double() * (0.2 / (22528 - 6144))
+    add_normalized_weight_decay_grads(p)
+    # one fused product and sum: half a unit in the last place of a value below 8
+    assert float((p.grad.double() - want).abs().max()) <= 2.0 ** -22
