@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, PER == 1 ? 6 : 5) training_samples_k
     constexpr unsigned kBlock = PER * kThreads;
     __shared__ __align__(16) float s_pos[3 * kBlock];
     __shared__ unsigned s_leaf[kBlock];
-    __shared__ unsigned short s_retry[2][kBlock];   // slots of the block that make another attempt: of this round, of the next
+    __shared__ unsigned short s_retry[2][kBlock];   // slots of the block that make another attempt: now, and after that
     __shared__ unsigned s_count[2];
     const unsigned tid = threadIdx.x;
     const int64_t block_first = (int64_t)blockIdx.x * kBlock;
