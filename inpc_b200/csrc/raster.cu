@@ -1347,7 +1347,10 @@ constexpr size_t backward_smem_bytes() {
 // up the slots of instance j in a fixed order.  Against forming weight and alpha per instance and sorting the fragments by pixel in
 // shared memory (masks by atomics, a scan, a slot per fragment): forward passes of 16-channel rows 614 -> 496 us (2^23
 // samples at 1237x822), first pass of a 2^25-point cloud at 1920x1080 411 -> 343, all passes of the 4-channel
-// training step 342 -> 332.  The backward pass of four channels still sorts its fragments (walking: 243 -> 262 us).
+// training step 342 -> 332.  In the backward passes lane j also forms weight, alpha and <g, f> of its instance in the (up to) four pixels beforehand, so that
+// a step of the walk is left with the transmittance and a running sum (see FragmentSlots): against sorting the fragments by pixel (four
+// channels) and forming everything in the walk (rows), 10^6 samples at 801x533 50 -> 44 us, 2^24 points at 3840x2160 466 -> 453, 2^23 samples of 16 channels
+// at 1237x822 373 -> 332; of four channels 236 -> 233, which its longest list takes whatever a step costs less.
 //
 // (3) Segments.  Front-to-back compositing is associative: (C, T) o (C', T') = (C + T C', T T').  A
 // tile's list is cut into a first segment and later ones (see segment_lengths), and every (tile half, segment) is one
@@ -1566,7 +1569,6 @@ __device__ __forceinline__ void async_copy_wait() { asm volatile("cp.async.wait_
 constexpr int kGatherDepthFilter = 2;     // stages of the ring, a power of two: first segments and products,
 constexpr int kGatherDepthRest = 2;       // later segments,
 constexpr int kGatherDepthBackward = 2;   // backward pass
-constexpr int kBatchFragments = 128;      // 32 instances x 4 fragments
 constexpr int kIdsAhead = 3;      // later segments: batches whose point ids are loaded ahead of their gather
 
 // Where the features of a splat come from: the second half of its record (four view-space channels), or, for feature rows,
@@ -1604,6 +1606,21 @@ __device__ __forceinline__ unsigned footprint_pixels(float x, float y, int px0, 
     const int qx = __float2int_rd(x - 0.5f) - px0, qy = __float2int_rd(y - 0.5f) - py0;   // left column, upper row
     if ((unsigned)(qx + 1) > 8u || (unsigned)(qy + 1) > 4u) return 0u;
     const unsigned two_by_two = qx < 0 ? 0x202u : qx == 7 ? 0x101u : 0x303u;              // clipped to the eight columns
+    return (unsigned)(((unsigned long long)two_by_two << (8 * qy + qx + 9)) >> 9);        // rows outside the half fall off either end
+}
+
+// The same for the backward passes: `weights` receives the bilinear weights in the four pixels, by the parity of a pixel's column
+// and row (the halves start at even ones), and pixels with a weight of zero are not named.
+__device__ __forceinline__ unsigned footprint_weights(float x, float y, int px0, int py0, float4& weights) {
+    const int qx = __float2int_rd(x - 0.5f) - px0, qy = __float2int_rd(y - 0.5f) - py0;   // left column, upper row
+    const float wx0 = __saturatef(1.0f - fabsf(x - ((float)(px0 + qx) + 0.5f))), wx1 = __saturatef(1.0f - fabsf(x - ((float)(px0 + qx + 1) + 0.5f)));
+    const float wy0 = __saturatef(1.0f - fabsf(y - ((float)(py0 + qy) + 0.5f))), wy1 = __saturatef(1.0f - fabsf(y - ((float)(py0 + qy + 1) + 0.5f)));
+    const bool odd_x = qx & 1, odd_y = qy & 1;
+    const float even_column = odd_x ? wx1 : wx0, odd_column = odd_x ? wx0 : wx1, even_row = odd_y ? wy1 : wy0, odd_row = odd_y ? wy0 : wy1;
+    weights = make_float4(even_column * even_row, odd_column * even_row, even_column * odd_row, odd_column * odd_row);
+    if ((unsigned)(qx + 1) > 8u || (unsigned)(qy + 1) > 4u) return 0u;
+    const unsigned columns = (qx >= 0 && wx0 > 0.0f ? 0x101u : 0u) | (qx < 7 && wx1 > 0.0f ? 0x202u : 0u);
+    const unsigned two_by_two = columns & ((wy0 > 0.0f ? 0x003u : 0u) | (wy1 > 0.0f ? 0x300u : 0u));
     return (unsigned)(((unsigned long long)two_by_two << (8 * qy + qx + 9)) >> 9);        // rows outside the half fall off either end
 }
 
@@ -2095,18 +2112,124 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kerne
     }
 }
 
+// What the passes backward through a list share.  Per staged instance and pixel of its footprint (by the parity of the pixel's column
+// and row, see footprint_weights) lane j leaves {alpha, G} with G = <g, f>, the upstream gradient of the pixel times the features of
+// the instance; the lanes of the pixels run down their lists and leave {T, S}: the transmittance the fragment met and
+// S = K - <g, what lies behind it>, K = grad_alpha * (1 - alpha of the pixel).  With these dL/dalpha = T G + S / (1 - alpha), formed per instance again.
+struct __align__(16) FragmentSlots {
+    float4 in[32][2];     // {alpha, G} of the parities 0 and 1 | 2 and 3
+    float4 out[32][2];    // {T, S}; T = 0: the pixel had stopped, or does not belong to the footprint
+};
+
+// Stores without a branch around it.  (What it writes is read behind a __syncwarp only, across which volatile assembly does not move.)
+__device__ __forceinline__ void store_shared_if(bool p, float2* dst, float2 v) {
+    asm volatile("{\n.reg .pred q;\nsetp.ne.u32 q, %0, 0;\n@q st.shared.v2.f32 [%1], {%2, %3};\n}" ::"r"((unsigned)p), "r"(shared_address(dst)), "f"(v.x), "f"(v.y));
+}
+
+// Every lane runs down the instances `todo` of its pixel, front to back, a few at a time: what they load does not wait for one another,
+// the chain from one transmittance to the next is one multiply, and the steps are written without branches.
+//
+// What lies behind a fragment is the final sum less the running one, but nothing lies behind the fragment at which a pixel stops: there
+// the difference of the two, zero but for their roundings, would be multiplied by 1 / (1 - alpha), up to 10^8.  (At any other fragment
+// T' = T (1 - alpha) >= 10^-4 bounds the factor by 10^4 T.)
+__device__ __forceinline__ void walk_backward(unsigned todo, FragmentSlots& slots, unsigned parity, float G_final, float K, float& Tr, float& G_run, bool& done) {
+    const float2* in = reinterpret_cast<const float2*>(slots.in) + parity;
+    float2* out = reinterpret_cast<float2*>(slots.out) + parity;
+    constexpr int kChunk = 4;
+    while (todo) {
+        int j[kChunk];
+        float al[kChunk], G[kChunk], met[kChunk];
+        bool ok[kChunk], live[kChunk];
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+            ok[u] = todo != 0u;
+            j[u] = ok[u] ? __ffs(todo) - 1 : 0;
+            todo &= todo - 1u;
+            const float2 e = in[4 * j[u]];
+            al[u] = e.x;
+            G[u] = e.y;
+        }
+        float next = Tr;
+        bool open = true;   // no fragment so far has stopped the pixel (it is not called with pixels that had stopped before)
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+            met[u] = next;
+            live[u] = open && ok[u];
+            const float behind = next * (1.0f - al[u]);
+            next = live[u] ? behind : next;
+            open = open && !(next < kTransmittanceEps);
+        }
+        Tr = next;
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+            G_run = live[u] ? G_run + met[u] * al[u] * G[u] : G_run;
+            const float rest = met[u] * (1.0f - al[u]) < kTransmittanceEps ? 0.0f : G_run - G_final;
+            store_shared_if(live[u], out + 4 * j[u], make_float2(met[u], rest + K));
+        }
+        if (!open) { done = true; todo = 0u; }
+    }
+}
+
+// The same for four channels, whose running colours are kept one by one: at the last fragment of a list their sum is the final colour to the bit, and what
+// lies behind it exactly zero.  (With the running sum <g, C> alone the opacity gradient is 1.35 to 1.5 times as far from 64 bits.)
+__device__ __forceinline__ void walk_backward(unsigned todo, FragmentSlots& slots, const float4* features, unsigned parity, const float4& g, const float4& C_final, float K,
+                                              float& Tr, float4& C_run, bool& done) {
+    const float2* in = reinterpret_cast<const float2*>(slots.in) + parity;
+    float2* out = reinterpret_cast<float2*>(slots.out) + parity;
+    constexpr int kChunk = 4;
+    while (todo) {
+        int j[kChunk];
+        float al[kChunk], met[kChunk];
+        float4 f[kChunk];
+        bool live[kChunk];
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+            live[u] = todo != 0u;
+            j[u] = live[u] ? __ffs(todo) - 1 : 0;
+            todo &= todo - 1u;
+            al[u] = in[4 * j[u]].x;
+            f[u] = features[j[u]];
+        }
+        bool open = true;
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+            met[u] = Tr;
+            live[u] = open && live[u];
+            Tr = live[u] ? Tr * (1.0f - al[u]) : Tr;
+            open = open && !(Tr < kTransmittanceEps);
+        }
+#pragma unroll
+        for (int u = 0; u < kChunk; ++u) {
+            const float bw = met[u] * al[u];
+            C_run.x = live[u] ? C_run.x + bw * f[u].x : C_run.x;
+            C_run.y = live[u] ? C_run.y + bw * f[u].y : C_run.y;
+            C_run.z = live[u] ? C_run.z + bw * f[u].z : C_run.z;
+            C_run.w = live[u] ? C_run.w + bw * f[u].w : C_run.w;
+            const float S = (C_run.x - C_final.x) * g.x + (C_run.y - C_final.y) * g.y + (C_run.z - C_final.z) * g.z + (C_run.w - C_final.w) * g.w;
+            store_shared_if(live[u], out + 4 * j[u], make_float2(met[u], S + K));
+        }
+        if (!open) { done = true; todo = 0u; }
+    }
+}
+
+// Pixels of a footprint (index row * 8 + column in the half) by parity; one that lies outside the half has an index (modulo 32) whose bit is not
+// among the pixels footprint_weights names.
+__device__ __forceinline__ void footprint_indices(float x, float y, int px0, int py0, unsigned (&pix)[4]) {
+    const int qx = __float2int_rd(x - 0.5f) - px0, qy = __float2int_rd(y - 0.5f) - py0;
+    const int even_column = qx + (qx & 1), odd_column = qx | 1, even_row = qy + (qy & 1), odd_row = qy | 1;
+    pix[0] = (unsigned)(even_row * 8 + even_column) & 31u;
+    pix[1] = (unsigned)(even_row * 8 + odd_column) & 31u;
+    pix[2] = (unsigned)(odd_row * 8 + even_column) & 31u;
+    pix[3] = (unsigned)(odd_row * 8 + odd_column) & 31u;
+}
+
 // Shared memory of one warp of the backward pass.
 struct __align__(16) WarpBackwardSmem {
     float4 ring_a[kGatherDepthBackward][32];   // records of the batches in flight (see the forward pass): position, alpha ...
     float4 ring_f[kGatherDepthBackward][32];   // ... and features
     float4 pixel_grad[32];                  // image gradient of the half's pixels
-    float4 frag_diff[kBatchFragments];      // per fragment: colour accumulated up to and including it, minus the final colour
-    float2 frag[kBatchFragments];           // fragments in per-pixel order: alpha, lane of the staged instance
-    float frag_seen[kBatchFragments];       // transmittance the fragment met (negative: it was dropped)
-    float pixel_k[32];                      // grad_alpha * (1 - alpha) of the half's pixels
+    FragmentSlots slots;
     uint32_t ring_id[kGatherDepthBackward][32];   // point ids of the batches in flight (0xFFFFFFFF: no instance)
-    unsigned mask[32];
-    unsigned off[32];
 };
 constexpr size_t kWarpBackwardSmemBytes = kWarpBlendWarps * sizeof(WarpBackwardSmem);
 
@@ -2123,10 +2246,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
     constexpr int kGatherDepth = kGatherDepthBackward;
     extern __shared__ __align__(16) unsigned char blend_smem[];
     const unsigned lane = lane_id();
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned parity = (lane & 1u) | ((lane >> 2) & 2u);   // of this lane's pixel: a footprint has each of the four once
     WarpBackwardSmem& sm = reinterpret_cast<WarpBackwardSmem*>(blend_smem)[threadIdx.x >> 5];
-    sm.mask[lane] = 0u;
-    __syncwarp();
     const unsigned n_first = __ldg(counts) * 2u;
     const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
     const unsigned n_rest = n_items - n_first;
@@ -2156,7 +2277,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
         const int px0 = tx * 8, py0 = ty * 8 + 4 * half;
         const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
 
-        float4 g = make_float4(0.f, 0.f, 0.f, 0.f), Cfin = g, Crun = g;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f), C_final = g, C_run = g;
         float K = 0.0f, Tr = 1.0f;
         bool done = !(px < width && py < height);
         if (!done) {
@@ -2165,15 +2286,15 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
             g = make_float4(__ldg(grad_image + pi), __ldg(grad_image + n_px + pi), __ldg(grad_image + 2 * n_px + pi),
                             __ldg(grad_image + 3 * n_px + pi));
             // what this segment and the ones behind it add to the pixel: the running colour starts at zero
-            Cfin = n_seg > 1u ? seg_C[sidx * 32 + lane]
-                              : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
+            C_final = n_seg > 1u ? seg_C[sidx * 32 + lane]
+                                 : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
             if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
         sm.pixel_grad[lane] = g;
-        sm.pixel_k[lane] = K;
+        __syncwarp();
         unsigned done_w = __ballot_sync(kFull, done);
 
         // ids kIdsAhead batches ahead of their gather, records kGatherDepth - 1 batches ahead of their use
@@ -2207,98 +2328,49 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
             const uint32_t id_cur = sm.ring_id[stage][lane];
             const bool staged = id_cur != kNoInstance;
             if (__ballot_sync(kFull, staged) == 0u) break;
-            const float4 a_cur = sm.ring_a[stage][lane];
             // ---- lane j: the fragments of staged instance j
-            const int qx = __float2int_rd(a_cur.x - 0.5f) - px0;
-            const int qy = __float2int_rd(a_cur.y - 0.5f) - py0;
-            float al[4], wg[4];
-            int pix[4];
+            const float4 own = sm.ring_a[stage][lane], fo = sm.ring_f[stage][lane];
+            float4 wg = make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned pixels = 0u, pix[4];
+            if (staged) pixels = footprint_weights(own.x, own.y, px0, py0, wg) & ~done_w;
+            footprint_indices(own.x, own.y, px0, py0, pix);
+            {
+                float G[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int cx = qx + (c & 1), cy = qy + (c >> 1);
-                const float pcx = (float)(px0 + cx) + 0.5f, pcy = (float)(py0 + cy) + 0.5f;
-                const float dx = fabsf(a_cur.x - pcx), dy = fabsf(a_cur.y - pcy);
-                wg[c] = __saturatef(1.0f - dx) * __saturatef(1.0f - dy);
-                al[c] = a_cur.z * wg[c];
-                const int p = cy * 8 + cx;
-                const bool ok = staged && cx >= 0 && cx < 8 && cy >= 0 && cy < 4 && dx < 1.0f && dy < 1.0f &&
-                                !((done_w >> (p & 31)) & 1u);
-                pix[c] = ok ? p : -1;
-                if (ok) atomicOr(sm.mask + p, 1u << lane);
-            }
-            __syncwarp();
-            const unsigned my_mask = sm.mask[lane];
-            const unsigned cnt = __popc(my_mask);
-            const unsigned off = warp_inclusive_scan(cnt) - cnt;
-            sm.off[lane] = off;
-            __syncwarp();
-            int slot[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                slot[c] = 0;
-                if (pix[c] >= 0) {
-                    slot[c] = (int)(sm.off[pix[c]] + __popc(sm.mask[pix[c]] & lt_mask));
-                    sm.frag[slot[c]] = make_float2(al[c], __uint_as_float(lane));
+                for (int c = 0; c < 4; ++c) {
+                    const float4 pg = sm.pixel_grad[pix[c]];
+                    G[c] = fo.x * pg.x + fo.y * pg.y + fo.z * pg.z + fo.w * pg.w;
                 }
+                sm.slots.in[lane][0] = make_float4(rounded_alpha(own.z, wg.x), G[0], rounded_alpha(own.z, wg.y), G[1]);
+                sm.slots.in[lane][1] = make_float4(rounded_alpha(own.z, wg.z), G[2], rounded_alpha(own.z, wg.w), G[3]);
+                sm.slots.out[lane][0] = sm.slots.out[lane][1] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
+            const unsigned todo = warp_transpose_bits(pixels, lane);
+            __syncwarp();   // (every lane sees the records the others have copied, too)
+            // ---- every lane runs down the instances of its own pixel, front to back
+            walk_backward(todo, sm.slots, sm.ring_f[stage], parity, g, C_final, K, Tr, C_run, done);
             __syncwarp();
-            if (my_mask) sm.mask[lane] = 0u;
-            // The serial part, per pixel: only what one fragment hands to the next (transmittance, running colour) is
-            // computed here, where the lanes with short lists idle; each fragment's state is left in shared memory
-            // and the gradient arithmetic follows below, per instance, with every staged lane busy.  Branch-free
-            // steps in chunks whose loads are issued together (see the forward pass).
-            constexpr int kChunk = 4;
-            for (unsigned k0 = off; k0 < off + cnt; k0 += kChunk) {
-                float a[kChunk];
-                float4 f[kChunk];
-#pragma unroll
-                for (int u = 0; u < kChunk; ++u) {
-                    const unsigned k = min(k0 + u, off + cnt - 1u);
-                    const float2 e = sm.frag[k];
-                    a[u] = e.x;
-                    f[u] = sm.ring_f[stage][__float_as_uint(e.y)];
-                }
-#pragma unroll
-                for (int u = 0; u < kChunk; ++u) {
-                    const bool in_list = k0 + u < off + cnt;
-                    const bool live = !done && in_list;
-                    const float bw = Tr * a[u];
-                    const float4 cr = make_float4(Crun.x + bw * f[u].x, Crun.y + bw * f[u].y, Crun.z + bw * f[u].z, Crun.w + bw * f[u].w);
-                    if (in_list) {
-                        sm.frag_seen[k0 + u] = live ? Tr : -1.0f;
-                        sm.frag_diff[k0 + u] = make_float4(cr.x - Cfin.x, cr.y - Cfin.y, cr.z - Cfin.z, cr.w - Cfin.w);
-                    }
-                    Crun = live ? cr : Crun;
-                    Tr = live ? Tr * (1.0f - a[u]) : Tr;
-                    done = done || Tr < kTransmittanceEps;
-                }
-            }
-            __syncwarp();
-            // gradients of every staged instance: its (up to) four fragments in fixed corner order
-            if (staged) {
-                const float4 fo = sm.ring_f[stage][lane];
+            // ---- lane j: the sums of instance j over its (up to) four pixels, in a fixed order
+            if (pixels) {
+                const float4 in01 = sm.slots.in[lane][0], in23 = sm.slots.in[lane][1], out01 = sm.slots.out[lane][0], out23 = sm.slots.out[lane][1];
+                const float al[4] = {in01.x, in01.z, in23.x, in23.z}, G[4] = {in01.y, in01.w, in23.y, in23.w};
+                const float met[4] = {out01.x, out01.z, out23.x, out23.z}, S[4] = {out01.y, out01.w, out23.y, out23.w};
+                const float w[4] = {wg.x, wg.y, wg.z, wg.w};
                 float4 sf = make_float4(0.f, 0.f, 0.f, 0.f);
                 float so = 0.0f;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    float o = 0.0f;
-                    if (pix[c] >= 0) {
-                        const float seen = sm.frag_seen[slot[c]];
-                        if (seen >= 0.0f) {
-                            const float4 d = sm.frag_diff[slot[c]];
+                    if (met[c] != 0.0f) {
+                        const float rcp = 1.0f / fmaxf(1.0f - al[c], kOneMinusAlphaEps);
+                        const float bw = met[c] * al[c];
+                        so += (met[c] * G[c] + S[c] * rcp) * w[c];
+                        if (bw > 0.0f) {   // (zero times an upstream gradient that has overflowed would be no number)
                             const float4 pg = sm.pixel_grad[pix[c]];
-                            const float rcp = 1.0f / fmaxf(1.0f - al[c], kOneMinusAlphaEps);
-                            const float bw = seen * al[c];
-                            const float from_features = (seen * fo.x + d.x * rcp) * pg.x + (seen * fo.y + d.y * rcp) * pg.y +
-                                                        (seen * fo.z + d.z * rcp) * pg.z + (seen * fo.w + d.w * rcp) * pg.w;
-                            o = (from_features + sm.pixel_k[pix[c]] * rcp) * wg[c];
-                            if (bw > 0.0f) v = make_float4(bw * pg.x, bw * pg.y, bw * pg.z, bw * pg.w);
+                            sf.x += bw * pg.x; sf.y += bw * pg.y; sf.z += bw * pg.z; sf.w += bw * pg.w;
                         }
                     }
-                    if (c == 0) { sf = v; so = o; }
-                    else { sf.x += v.x; sf.y += v.y; sf.z += v.z; sf.w += v.w; so += o; }
                 }
+                const int qx = __float2int_rd(own.x - 0.5f) - px0, qy = __float2int_rd(own.y - 0.5f) - py0;
                 // A splat's 2x2 pixels lie in at most two tile columns and two (tile row, half) groups, and which of
                 // them this item is follows from where the footprint starts: it holds the left column unless the
                 // footprint starts left of it, and the upper row unless it starts above it.  So every (point, slot)
@@ -2323,10 +2395,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
     }
 }
 
-// Backward pass over feature rows, the walk and the lists of the kernel above.  Per fragment only scalars are kept: with
-// G = <g, .> over the channels, dL/dalpha = Tr * G(f) + (G(C_run) - G(C_final)) / (1 - alpha) + K / (1 - alpha), and
-// G(C_run) is a running scalar.  The pixel lanes leave a fragment's blending weight and dL/dalpha in shared memory; the
-// gradient of a point's row, sum over its pixels of weight * g, is then formed per instance with every staged lane busy.
+// Backward pass over feature rows, the lists and the walk of the kernel above with a scalar in the place of the running colour: with
+// G = <g, .> over the channels, dL/dalpha = T G(f) + (G(C_run) - G(C_final) + K) / (1 - alpha).  G(f) is formed per instance and pixel,
+// and so is the gradient of a point's row, sum over its pixels of weight * g, with every staged lane busy.
 // A splat whose 2x2 pixels all lie in this 8x4 half has no other writer in the launch and stores its row; the others
 // (about a third) add theirs with one vector atomic per four channels.
 template <int C4>
@@ -2334,7 +2405,7 @@ struct __align__(16) RowsBackwardSmem {
     float4 ring_a[kGatherDepthBackward][32];
     float4 ring_f[kGatherDepthBackward][32 * feature_stride(C4)];
     float4 pixel_grad[32 * feature_stride(C4)];   // image gradient of the half's pixels
-    float4 out[32][2];                            // per staged instance and parity of the pixel: blending weight, opacity gradient
+    FragmentSlots slots;
     uint32_t ring_id[kGatherDepthBackward][32];
 };
 template <int C4>
@@ -2384,7 +2455,6 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
         const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
         const int px0 = tx * 8, py0 = ty * 8 + 4 * half;
         const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
-        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
 
         float4 g[C4];
         float G_final = 0.0f, G_run = 0.0f, K = 0.0f, Tr = 1.0f;
@@ -2414,6 +2484,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
         __syncwarp();   // the previous item's readers of pixel_grad are through
 #pragma unroll
         for (int c = 0; c < C4; ++c) sm.pixel_grad[lane * kStride + c] = g[c];
+        __syncwarp();
         unsigned done_w = __ballot_sync(kFull, done);
 
         uint32_t idf[kIdsAhead];
@@ -2445,50 +2516,50 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
             const uint32_t id_cur = sm.ring_id[stage][lane];
             const bool staged = id_cur != kNoInstance;
             if (__ballot_sync(kFull, staged) == 0u) break;
-            // ---- lane j: the pixels of staged instance j that have not stopped
-            const float4 own = sm.ring_a[stage][lane];
-            const unsigned pixels = staged ? footprint_pixels(own.x, own.y, px0, py0) & ~done_w : 0u;
-            sm.out[lane][0] = sm.out[lane][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-            unsigned todo = warp_transpose_bits(pixels, lane);
             __syncwarp();   // every lane sees what the others have copied
-            // ---- every lane runs down the instances of its own pixel, front to back
-            while (todo) {
-                const int j = __ffs(todo) - 1;
-                todo &= todo - 1u;
-                const float4 a = sm.ring_a[stage][j];
-                const float wg = __saturatef(1.0f - fabsf(a.x - pcx)) * __saturatef(1.0f - fabsf(a.y - pcy));
-                if (!(wg > 0.0f)) continue;
-                const float4* row = sm.ring_f[stage] + j * kStride;
-                float fg = 0.0f;
+            // ---- lane j: the fragments of staged instance j in the pixels that have not stopped
+            const float4 own = sm.ring_a[stage][lane];
+            float4 wg = make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned pixels = 0u, pix[4];
+            if (staged) pixels = footprint_weights(own.x, own.y, px0, py0, wg) & ~done_w;
+            footprint_indices(own.x, own.y, px0, py0, pix);
+            {
+                float G[4] = {0.f, 0.f, 0.f, 0.f};
+                const float4* row = sm.ring_f[stage] + lane * kStride;
 #pragma unroll
                 for (int c = 0; c < C4; ++c) {
                     const float4 f = row[c];
-                    fg += f.x * g[c].x + f.y * g[c].y + f.z * g[c].z + f.w * g[c].w;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 v = sm.pixel_grad[pix[q] * kStride + c];
+                        G[q] += f.x * v.x + f.y * v.y + f.z * v.z + f.w * v.w;
+                    }
                 }
-                const float al = rounded_alpha(a.z, wg);
-                const float bw = Tr * al;
-                G_run += bw * fg;
-                const float oma = 1.0f - al;
-                const float rcp = 1.0f / fmaxf(oma, kOneMinusAlphaEps);
-                // (no feature gradient from a weight that is not positive: a negative opacity, or not a number)
-                reinterpret_cast<float2*>(sm.out[j])[parity] = make_float2(bw > 0.0f ? bw : 0.0f, (Tr * fg + (G_run - G_final) * rcp + K * rcp) * wg);
-                Tr *= oma;
-                done = Tr < kTransmittanceEps;
-                if (done) todo = 0u;
+                sm.slots.in[lane][0] = make_float4(rounded_alpha(own.z, wg.x), G[0], rounded_alpha(own.z, wg.y), G[1]);
+                sm.slots.in[lane][1] = make_float4(rounded_alpha(own.z, wg.z), G[2], rounded_alpha(own.z, wg.w), G[3]);
+                sm.slots.out[lane][0] = sm.slots.out[lane][1] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
+            const unsigned todo = warp_transpose_bits(pixels, lane);
             __syncwarp();
-            // ---- lane j: the sums of instance j over its (up to) four pixels, in fixed corner order
+            // ---- every lane runs down the instances of its own pixel, front to back
+            walk_backward(todo, sm.slots, parity, G_final, K, Tr, G_run, done);
+            __syncwarp();
+            // ---- lane j: the sums of instance j over its (up to) four pixels, in a fixed order
             if (pixels) {
                 const int qx = __float2int_rd(own.x - 0.5f) - px0, qy = __float2int_rd(own.y - 0.5f) - py0;
-                const unsigned first_parity = ((unsigned)qx & 1u) | (((unsigned)qy & 1u) << 1);
+                const float4 in01 = sm.slots.in[lane][0], in23 = sm.slots.in[lane][1], out01 = sm.slots.out[lane][0], out23 = sm.slots.out[lane][1];
+                const float al[4] = {in01.x, in01.z, in23.x, in23.z}, G[4] = {in01.y, in01.w, in23.y, in23.w};
+                const float met[4] = {out01.x, out01.z, out23.x, out23.z}, S[4] = {out01.y, out01.w, out23.y, out23.w};
+                const float w[4] = {wg.x, wg.y, wg.z, wg.w};
                 float bw[4], so = 0.0f;
                 bool any = false;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float2 o = reinterpret_cast<const float2*>(sm.out[lane])[first_parity ^ (unsigned)c];
-                    bw[c] = o.x;
-                    so += o.y;
-                    any = any || o.x != 0.0f;
+                for (int q = 0; q < 4; ++q) {
+                    // (no feature gradient from a weight that is not positive: a negative opacity, or not a number)
+                    const float b = met[q] * al[q];
+                    bw[q] = b > 0.0f ? b : 0.0f;
+                    any = any || bw[q] != 0.0f;
+                    if (met[q] != 0.0f) so += (met[q] * G[q] + S[q] * (1.0f / fmaxf(1.0f - al[q], kOneMinusAlphaEps))) * w[q];
                 }
                 const bool alone = qx >= 0 && qx < 7 && qy >= 0 && qy < 3;   // all four pixels in this half
                 if (any) {
@@ -2499,7 +2570,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             if (bw[q] != 0.0f) {
-                                const float4 v = sm.pixel_grad[((qy + (q >> 1)) * 8 + qx + (q & 1)) * kStride + c];
+                                const float4 v = sm.pixel_grad[pix[q] * kStride + c];
                                 sum.x += bw[q] * v.x; sum.y += bw[q] * v.y; sum.z += bw[q] * v.z; sum.w += bw[q] * v.w;
                             }
                         }
