@@ -125,6 +125,12 @@ int sort_pass_count(int end_bit);   // passes sort_pairs makes; the result is in
 size_t sort_zero_bytes(int64_t n, int64_t n_likely, int end_bit);
 int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
                int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, bool position_values = false);
+// Sorts the positions 0 .. n - 1 of the keys other than kNoKey and leaves how many there are in *count (device memory): the first pass
+// leaves the others out, so that whoever writes the keys need not compact them.  The workspace is sized for (n, n); the result is in the
+// alternate buffers iff sort_pass_count(end_bit) is odd.  No key that takes part may equal kNoKey, also in bits above end_bit.
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
+                     bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for (n_max, n_likely).  The result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,

@@ -256,18 +256,18 @@ constexpr unsigned kCountShift = 30;   // bilinear: (tiles touched - 1) in key b
 // Pass 1 of the deterministic compaction: per chunk of kPreThreads points, how many points survive culling, and how many
 // (point, tile) instances there are in all.  The last block scans the counts of the groups of 4 chunks (group_visible and
 // *instances start at zero) and leaves the totals in counters[0] (visible) and counters[1] (instances), the range of depth bit
-// patterns the keys are offsets into in counters[2..3] and *depth_min, *depth_max: measured (RANGE: the words of `range` start
-// at zero and collect the largest pattern and the largest complement), or fixed_lo .. fixed_hi.
+// patterns the keys are offsets into in counters[2..3] and *depth_min, *depth_max (the words of `range` start
+// at zero and collect the largest pattern and the largest complement).  Only where the host needs the counts: see the projection pass.
 //
 // Bound by the instructions of the projection (96 per point; 33 % of DRAM).  Every lane takes 4 consecutive points (three 16-byte
 // loads when the array is aligned), a warp a chunk in two steps, the positions of the next step travelling while this one's are
 // projected; nothing waits for other warps before the last block's scan.  2^23 / 2^25 points 36 / 129 us
 // (one block per group with its fence and atomic 62 / 226; persistent blocks with a barrier per group 44 / 154, with the
 // positions loaded ahead 39 / 144).
-template <int MODE, int VARIANT, bool RANGE>
+template <int MODE, int VARIANT>
 __global__ void __launch_bounds__(kPreThreads, 4) visibility_count_kernel(
     const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_chunks, unsigned* __restrict__ block_visible,
-    unsigned* group_visible, unsigned long long* instances, unsigned* range, unsigned* done, unsigned fixed_lo, unsigned fixed_hi,
+    unsigned* group_visible, unsigned long long* instances, unsigned* range, unsigned* done,
     unsigned* __restrict__ depth_min, unsigned* __restrict__ depth_max, unsigned long long* __restrict__ counters) {
     await_previous_kernel();
     constexpr int kPerThread = 4;
@@ -320,11 +320,9 @@ __global__ void __launch_bounds__(kPreThreads, 4) visibility_count_kernel(
                     if (pr.visible) {
                         v += 1u;
                         inst += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
-                        if (RANGE) {
-                            const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
-                            lo = min(lo, bits);
-                            hi = max(hi, bits);
-                        }
+                        const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
+                        lo = min(lo, bits);
+                        hi = max(hi, bits);
                     }
                 }
             }
@@ -338,17 +336,14 @@ __global__ void __launch_bounds__(kPreThreads, 4) visibility_count_kernel(
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
     if (lane_id() == 0 && inst) atomicAdd(instances, inst);
-    // (callers that know a bound on the depths beforehand do not ask for the range)
-    if (RANGE) {
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane_id() == 0 && lo <= hi) { atomicMax(range, ~lo); atomicMax(range + 1, hi); }
-    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane_id() == 0 && lo <= hi) { atomicMax(range, ~lo); atomicMax(range + 1, hi); }
     if (!last_block(done, gridDim.x)) return;
     __shared__ unsigned s_scan[kPreThreads / 32 + 1];
     const unsigned visible = scan_words<kPreThreads>(group_visible, (n_chunks + 3u) / 4u, s_scan);
     if (threadIdx.x == 0) {
-        const unsigned first_key = RANGE ? ~__ldcg(range) : fixed_lo, last_key = RANGE ? __ldcg(range + 1) : fixed_hi;
+        const unsigned first_key = ~__ldcg(range), last_key = __ldcg(range + 1);
         counters[0] = visible;
         counters[1] = __ldcg(instances);
         counters[2] = *depth_min = first_key;
@@ -429,11 +424,13 @@ __device__ __forceinline__ uint4 pack_footprint(const Projection& pr, float reac
 // bounds, and append (depth key, point id) at the slot given by the block offset plus the rank of
 // the point among the block's survivors — index order, hence reproducible.
 // src/bilinear/kernels.cu:11-84, :106-184; src/gaussian/kernels.cu:11-111, :113-217, :219-324.
-template <int MODE, int VARIANT>
+// COMPACT: see above; otherwise every point's key is written where the point lies, that of a culled one is kNoKey, and the depth sort leaves it out
+// (the base of the keys is known to the host then, and neither the counts nor the depth range nor the point ids are used).
+template <int MODE, int VARIANT, bool COMPACT>
 __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     PointSets ps, RasterParams rp, const unsigned* __restrict__ block_visible, const unsigned* __restrict__ group_offset,
     const unsigned* __restrict__ depth_min,
-    const unsigned* __restrict__ depth_max, PointRec* __restrict__ rec, uint2* __restrict__ bounds, uint32_t* __restrict__ quad,
+    const unsigned* __restrict__ depth_max, unsigned key_base, PointRec* __restrict__ rec, uint2* __restrict__ bounds, uint32_t* __restrict__ quad,
     float4* __restrict__ conic, uint4* __restrict__ foot, uint32_t* __restrict__ depth_keys,
     uint32_t* __restrict__ point_ids, int pack_count, int rec_stride, volatile unsigned* status) {
     await_previous_kernel();
@@ -528,23 +525,27 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
             write_bounds(false);
         }
     }
+    // sort key: offset of the depth's bit pattern from the smallest there can be (fewer radix passes).
+    // A bilinear splat touches 1, 2 or 4 tiles; when the offsets leave the two top bits free that
+    // count rides there (the sort ignores bits above its range and carries them along), which
+    // saves the instance pass a gather.
+    // pack_count: 1 yes, 0 no (the host knows a bound on the offsets), -1 decide from the measured depth range
+    auto depth_key = [&](unsigned lo) -> unsigned {
+        const unsigned key = __float_as_uint(pr.depth) - lo;
+        const bool pack = pack_count >= 0 ? pack_count != 0 : __ldg(depth_max) - lo < (1u << kCountShift);
+        return MODE == INPC_MODE_BILINEAR && pack ? key | (((pr.x1 - pr.x0) * (pr.y1 - pr.y0) - 1u) << kCountShift) : key;
+    };
+    if (!COMPACT) {
+        if (iv < ps.start[ps.count]) depth_keys[iv] = pr.visible ? depth_key(key_base) : kNoKey;
+        return;
+    }
     unsigned total;
     const unsigned rank = block_exclusive_scan(pr.visible ? 1u : 0u, s_scan, &total);
     if (pr.visible) {
         // slot = survivors of all groups before + of the earlier chunks of this group + rank in this chunk
         unsigned slot = __ldg(group_offset + (blockIdx.x >> 2)) + rank;
         for (unsigned c = blockIdx.x & ~3u; c < blockIdx.x; ++c) slot += __ldg(block_visible + c);
-        // sort key: offset of the depth's bit pattern from the smallest visible one (fewer radix passes).
-        // A bilinear splat touches 1, 2 or 4 tiles; when the offsets leave the two top bits free that
-        // count rides there (the sort ignores bits above its range and carries them along), which
-        // saves the instance pass a gather.
-        const unsigned lo = __ldg(depth_min);
-        unsigned key = __float_as_uint(pr.depth) - lo;
-        // pack_count: 1 yes, 0 no (the host knows a bound on the offsets), -1 decide from the measured depth range
-        const bool pack = pack_count >= 0 ? pack_count != 0 : __ldg(depth_max) - lo < (1u << kCountShift);
-        if (MODE == INPC_MODE_BILINEAR && pack)
-            key |= ((pr.x1 - pr.x0) * (pr.y1 - pr.y0) - 1u) << kCountShift;
-        depth_keys[slot] = key;
+        depth_keys[slot] = depth_key(__ldg(depth_min));
         point_ids[slot] = (uint32_t)iv;
     }
 }
@@ -563,7 +564,7 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
                                                                           const uint32_t* __restrict__ sorted_ids,
                                                                           const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
                                                                           const unsigned long long* __restrict__ n_visible_dev,
-                                                                          unsigned* block_sums, unsigned n_groups, unsigned* done) {
+                                                                          unsigned* block_sums, unsigned n_groups, unsigned* done, unsigned long long* n_instances) {
     await_previous_kernel();
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     constexpr unsigned kWarps = kInstThreads / 4 / 32;
@@ -610,7 +611,9 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
         }
     }
     __shared__ unsigned s_scan[kInstThreads / 4 / 32 + 1];
-    if (last_block(done, gridDim.x)) scan_words<kInstThreads / 4>(block_sums, n_groups, s_scan);   // sums -> first instance of every block
+    if (!last_block(done, gridDim.x)) return;
+    const unsigned total = scan_words<kInstThreads / 4>(block_sums, n_groups, s_scan);   // sums -> first instance of every block
+    if (threadIdx.x == 0 && n_instances) *n_instances = total;
 }
 
 // Instance key: the tile index in the low 24 bits, the only bits the tile sort looks at (it carries the
@@ -4085,6 +4088,8 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             if (!(rp.v.near_plane > 0.0f)) { lo_bits = 0u; hi_bits = 0xFFFFFFFFu; }
             key_bits = rp.v.near_plane > 0.0f ? bit_length(hi_bits - lo_bits) : 32;
             if (key_bits == 0) key_bits = 1;
+            // with offsets of up to 2^30 - 1, a splat of four tiles at the far plane would have the key of a culled point
+            if (key_bits == (int)kCountShift && hi_bits - lo_bits == (1u << kCountShift) - 1u) ++key_bits;
             key_base = lo_bits;
             pack_count = key_bits <= (int)kCountShift ? 1 : 0;
             n_visible = n;                // capacities from here on
@@ -4100,27 +4105,26 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         {
             StageScope scope(STAGE_PREPROCESS, stream);
             // (non-deferred: the number of key bits is not known yet, the sort clears its own state)
-            clear.add(pb.group_visible, sizeof(unsigned) * (size_t)ceil_div<int64_t>(nb, 4));
+            if (!deferred) clear.add(pb.group_visible, sizeof(unsigned) * (size_t)ceil_div<int64_t>(nb, 4));
             clear.add(pb.state, (size_t)(static_cast<char*>(pb.sort_ws) - reinterpret_cast<char*>(pb.state)) + (deferred ? sort_zero_bytes(n, n, key_bits) : 0));
             rc = launch_clear(clear, stream);
             if (rc != INPC_OK) return rc;
-            const int64_t count_blocks = ceil_div<int64_t>(nb, kPreThreads / 32), count_cap = (int64_t)sm_count() * 4;
-            const unsigned count_grid = (unsigned)(count_blocks < count_cap ? count_blocks : count_cap);
-            unsigned long long* instances = reinterpret_cast<unsigned long long*>(pb.state + 8);
-            if (deferred)
-                launch_chained(visibility_count_kernel<MODE, VARIANT, false>, count_grid, kPreThreads, 0, stream,
-                    ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, instances, nullptr, pb.state + 2, lo_bits, hi_bits, pb.depth_min, pb.depth_max, pb.counters);
-            else
-                launch_chained(visibility_count_kernel<MODE, VARIANT, true>, count_grid, kPreThreads, 0, stream,
-                    ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, instances, pb.state, pb.state + 2, lo_bits, hi_bits, pb.depth_min, pb.depth_max, pb.counters);
-            INPC_LAUNCH_CHECK("visibility_count_kernel");
             if (!deferred) {
+                const int64_t count_blocks = ceil_div<int64_t>(nb, kPreThreads / 32), count_cap = (int64_t)sm_count() * 4;
+                const unsigned count_grid = (unsigned)(count_blocks < count_cap ? count_blocks : count_cap);
+                launch_chained(visibility_count_kernel<MODE, VARIANT>, count_grid, kPreThreads, 0, stream,
+                    ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, reinterpret_cast<unsigned long long*>(pb.state + 8), pb.state, pb.state + 2, pb.depth_min, pb.depth_max, pb.counters);
+                INPC_LAUNCH_CHECK("visibility_count_kernel");
                 INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
                 INPC_CUDA_TRY(cudaEventRecord(ready, stream));
             }
             // the projection pass needs nothing from the host: it runs while the host waits for the counters
-            launch_chained(preprocess_kernel<MODE, VARIANT>, (unsigned)nb, kPreThreads, 0, stream,
-                ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max,
+            auto* project = preprocess_kernel<MODE, VARIANT, true>;
+            if constexpr (MODE == INPC_MODE_BILINEAR) {
+                if (deferred) project = preprocess_kernel<MODE, VARIANT, false>;
+            }
+            launch_chained(project, (unsigned)nb, kPreThreads, 0, stream,
+                ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max, key_base,
                 pb.rec, pb.bounds, pb.quad, pb.conic, pb.foot, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
             INPC_LAUNCH_CHECK("preprocess_kernel");
         }
@@ -4160,7 +4164,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     int in_alt = 0;
     {
         StageScope scope(STAGE_SORT_DEPTH, stream);
-        rc = deferred ? sort_pairs_device_count(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n_visible, n_visible_dev, key_bits, pb.sort_ws, true, status, &in_alt, stream)
+        rc = deferred ? sort_marked_keys(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, pb.sort_ws, true, status, &in_alt, stream)
                       : sort_pairs(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n, key_bits, pb.sort_ws, false, status, &in_alt, stream);
     }
     if (rc != INPC_OK) return rc;
@@ -4172,9 +4176,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles rides in the top key bits when the depth offsets left them free
             if (MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift)
-                launch_chained(instance_count_kernel<true>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
+                launch_chained(instance_count_kernel<true>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr);
             else
-                launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3);
+                launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (warp_blend && MODE == INPC_MODE_GAUSSIAN)
                 launch_chained(emit_instances_kernel<EMIT_CELLS>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, nullptr, pb.foot, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
@@ -4854,12 +4858,12 @@ extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
     if (!(state->deferred_counts & 1) || state->n_points == 0) return INPC_OK;
     if (!state->point_blob) { set_error("inpc_raster_resolve: state without a point blob"); return INPC_E_INVALID; }
     const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode, state->tile_size);
-    unsigned long long host[4];
+    unsigned long long host[2];
     INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, sizeof(host), cudaMemcpyDeviceToHost, stream));
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
     state->n_visible = (int64_t)host[0];
     state->n_instances = (int64_t)host[1];
-    state->depth_key_base = state->n_visible > 0 ? (uint32_t)host[2] : 0u;
+    if (state->n_visible == 0) state->depth_key_base = 0u;
     if (state->n_visible > state->n_points || state->n_instances > 4 * state->n_visible) {
         set_error("inconsistent counts from the visibility pass: %lld visible of %lld points, %lld instances", (long long)state->n_visible,
                   (long long)state->n_points, (long long)state->n_instances);
