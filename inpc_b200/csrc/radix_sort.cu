@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
     const int64_t n = n_dev ? (int64_t)*n_dev : n_arg;
     if ((int64_t)blockIdx.x * kHistItemsPerBlock >= n) return;
     __shared__ unsigned s_hist[kMaxPasses][kRadix];
-    __shared__ unsigned s_scan[kHistThreads / 32 + 1];
+    __shared__ unsigned s_scan[kMaxPasses][kHistThreads / 32];
     for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads) (&s_hist[0][0])[i] = 0;
     __syncthreads();
 
@@ -84,12 +84,26 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
     }
     const int64_t all = ceil_div<int64_t>(n, kHistItemsPerBlock);
     if (!last_block(blocks_done, (unsigned)min(all, (int64_t)gridDim.x))) return;
-    for (int p = 0; p < pt.n_passes; ++p) {
-        unsigned total;
-        const unsigned ex = block_exclusive_scan(__ldcg(hist + p * kRadix + threadIdx.x), s_scan, &total);
-        base[p * kRadix + threadIdx.x] = ex;
-        if (MARKED && p == 0 && threadIdx.x == 0) *count_out = total;
+    // all passes side by side: one round trip to memory, two barriers
+    unsigned inc[kMaxPasses], own[kMaxPasses];
+#pragma unroll
+    for (int p = 0; p < kMaxPasses; ++p) own[p] = p < pt.n_passes ? __ldcg(hist + p * kRadix + threadIdx.x) : 0u;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int p = 0; p < kMaxPasses; ++p) {
+        inc[p] = warp_inclusive_scan(own[p]);
+        if (lane == 31) s_scan[p][warp] = inc[p];
     }
+    __syncthreads();
+    if (warp < (unsigned)kMaxPasses) {
+        const unsigned sum = lane < kHistThreads / 32 ? s_scan[warp][lane] : 0u, before = warp_inclusive_scan(sum) - sum;
+        if (lane < kHistThreads / 32) s_scan[warp][lane] = before;
+        if (MARKED && warp == 0 && lane == kHistThreads / 32 - 1) *count_out = before + sum;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < kMaxPasses; ++p)
+        if (p < pt.n_passes) base[p * kRadix + threadIdx.x] = s_scan[p][warp] + inc[p] - own[p];
 }
 
 // ---- one pass ---------------------------------------------------------------------------------
