@@ -1437,9 +1437,20 @@ __device__ __forceinline__ unsigned warp_segments(unsigned len, const SegmentLen
     return len <= sl.first ? 1u : 1u + ceil_div(len - sl.first, sl.later);
 }
 
-// Work lists of the warp blend.  Step 1 (one block per 1024 tiles): segments and non-empty tiles of the block's tiles.
-// Its last block scans those block sums; counts[0] = non-empty tiles, counts[1] = segments behind a tile's first.  Step 2 (same blocks as step 1): every tile's position from its block's base and a scan inside the
+// Work lists of the warp blend.  The first segments lie in the order of three classes of length, so that the longest are taken first and a
+// pass does not end with one that was found late (with the tiles in order within a class, since neighbours share records in L1): 2^24 points
+// of which nine tenths crowd one corner of a 3840x2160 image, first pass and backward 397 + 455 -> 345 + 442 us, 2^22 gaussian splats at 1237x822 backward
+// 309 -> 289, 2 * 10^6 with sizes at 1297x840 171 -> 167, 2^25 points at 1920x1080 the same.  Not for feature rows: their backward pass, whose points' rows several
+// tiles add to, took 331 -> 344 with 2^23 samples of 16 channels.
+// Step 1 (one block per 1024 tiles): segments and non-empty tiles of each class of the block's tiles.
+// Its last block scans those block sums; counts[0] = non-empty tiles, counts[1] = segments behind a tile's first, counts[kLongTiles] and counts[kLongTiles + 1] =
+// tiles of the first class and of the first two.  Step 2 (same blocks as step 1): every tile's position from its block's base and a scan inside the
 // block, and its items.  (One block scanning all tiles took 177 us for the 129,600 tiles of a 3840x2160 image.)
+constexpr int kLongTiles = 8;
+__device__ __forceinline__ unsigned length_class(unsigned len, const SegmentLengths& sl, bool by_length) {
+    return !by_length ? 2u : len >= sl.first ? 0u : len >= sl.first / 4u ? 1u : 2u;
+}
+
 constexpr int kItemThreads = 256;
 constexpr int kItemTilesPerThread = 4;
 constexpr int kItemTilesPerBlock = kItemThreads * kItemTilesPerThread;
@@ -1459,45 +1470,65 @@ __device__ __forceinline__ void load_tile_segments(const uint2* __restrict__ ran
     }
 }
 
-__global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, unsigned long long n_instances_arg,
-                                                                        const unsigned long long* __restrict__ n_instances_dev, uint2* block_sums, unsigned* done,
+// {segments, non-empty tiles of class 0, 1, 2} of a thread's tiles
+__device__ __forceinline__ uint4 count_tile_segments(const unsigned (&ns)[kItemTilesPerThread], const uint2 (&rg)[kItemTilesPerThread], const SegmentLengths& sl,
+                                                     bool by_length) {
+    uint4 c = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int k = 0; k < kItemTilesPerThread; ++k) {
+        if (ns[k] == 0u) continue;
+        const unsigned cls = length_class(rg[k].y - rg[k].x, sl, by_length);
+        c.x += ns[k];
+        c.y += cls == 0u ? 1u : 0u;
+        c.z += cls == 1u ? 1u : 0u;
+        c.w += cls == 2u ? 1u : 0u;
+    }
+    return c;
+}
+
+__global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, bool by_length, unsigned long long n_instances_arg,
+                                                                        const unsigned long long* __restrict__ n_instances_dev, uint4* block_sums, unsigned* done,
                                                                         uint32_t* __restrict__ counts) {
     await_previous_kernel();
-    __shared__ unsigned s_seg[kItemThreads / 32], s_tiles[kItemThreads / 32];
+    __shared__ uint4 s_sums[kItemThreads / 32];
     unsigned ns[kItemTilesPerThread];
     uint2 rg[kItemTilesPerThread];
     const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles, limits);
     load_tile_segments(ranges, n_tiles, blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread, sl, ns, rg);
-    unsigned seg = 0, tiles = 0;
-#pragma unroll
-    for (int k = 0; k < kItemTilesPerThread; ++k) { seg += ns[k]; tiles += ns[k] ? 1u : 0u; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        seg += __shfl_down_sync(0xffffffffu, seg, o);
-        tiles += __shfl_down_sync(0xffffffffu, tiles, o);
-    }
-    if (lane_id() == 0) { s_seg[threadIdx.x >> 5] = seg; s_tiles[threadIdx.x >> 5] = tiles; }
+    uint4 c = count_tile_segments(ns, rg, sl, by_length);
+    c.x = __reduce_add_sync(0xffffffffu, c.x);
+    c.y = __reduce_add_sync(0xffffffffu, c.y);
+    c.z = __reduce_add_sync(0xffffffffu, c.z);
+    c.w = __reduce_add_sync(0xffffffffu, c.w);
+    if (lane_id() == 0) s_sums[threadIdx.x >> 5] = c;
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned a = 0, c = 0;
+        uint4 t = s_sums[0];
 #pragma unroll
-        for (int w = 0; w < kItemThreads / 32; ++w) { a += s_seg[w]; c += s_tiles[w]; }
-        block_sums[blockIdx.x] = make_uint2(a, c);
+        for (int w = 1; w < kItemThreads / 32; ++w) { t.x += s_sums[w].x; t.y += s_sums[w].y; t.z += s_sums[w].z; t.w += s_sums[w].w; }
+        block_sums[blockIdx.x] = t;
     }
     if (!last_block(done, gridDim.x)) return;
     __shared__ unsigned s_scan[kItemThreads / 32 + 1];
-    unsigned run_seg = 0, run_tiles = 0;
+    uint4 run = make_uint4(0u, 0u, 0u, 0u);
     for (unsigned base = 0; base < gridDim.x; base += kItemThreads) {
         const unsigned j = base + threadIdx.x;
-        const uint2 v = j < gridDim.x ? __ldcg(block_sums + j) : make_uint2(0u, 0u);
-        unsigned total_seg, total_tiles;
-        const unsigned ex_seg = run_seg + block_exclusive_scan(v.x, s_scan, &total_seg);
-        const unsigned ex_tiles = run_tiles + block_exclusive_scan(v.y, s_scan, &total_tiles);
-        if (j < gridDim.x) block_sums[j] = make_uint2(ex_seg, ex_tiles);
-        run_seg += total_seg;
-        run_tiles += total_tiles;
+        const uint4 v = j < gridDim.x ? __ldcg(block_sums + j) : make_uint4(0u, 0u, 0u, 0u);
+        uint4 total, ex;
+        ex.x = run.x + block_exclusive_scan(v.x, s_scan, &total.x);
+        ex.y = run.y + block_exclusive_scan(v.y, s_scan, &total.y);
+        ex.z = run.z + block_exclusive_scan(v.z, s_scan, &total.z);
+        ex.w = run.w + block_exclusive_scan(v.w, s_scan, &total.w);
+        if (j < gridDim.x) block_sums[j] = ex;
+        run.x += total.x; run.y += total.y; run.z += total.z; run.w += total.w;
     }
-    if (threadIdx.x == 0) { counts[0] = run_tiles; counts[1] = run_seg - run_tiles; }
+    if (threadIdx.x == 0) {
+        const unsigned tiles = run.y + run.z + run.w;
+        counts[0] = tiles;
+        counts[1] = run.x - tiles;
+        counts[kLongTiles] = run.y;
+        counts[kLongTiles + 1] = run.y + run.z;
+    }
 }
 
 // Everything a warp needs to know about a (tile, segment), in one 32-byte record: the blend kernels read it with
@@ -1516,10 +1547,10 @@ __device__ __forceinline__ WarpItem load_item(const WarpItem* p) {
     return w;
 }
 
-// Step 2: items0 = segment 0 of the non-empty tiles, items1 = every later segment, tile by tile.
-__global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, unsigned long long n_instances_arg,
+// Step 2: items0 = segment 0 of the non-empty tiles by class, items1 = every later segment, tile by tile.
+__global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, bool by_length, unsigned long long n_instances_arg,
                                                                       const unsigned long long* __restrict__ n_instances_dev,
-                                                                      const uint2* __restrict__ block_base, WarpItem* __restrict__ items0,
+                                                                      const uint4* __restrict__ block_base, const uint32_t* __restrict__ counts, WarpItem* __restrict__ items0,
                                                                       WarpItem* __restrict__ items1) {
     await_previous_kernel();
     __shared__ unsigned s_scan[kItemThreads / 32 + 1];
@@ -1528,22 +1559,27 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
     const int t0 = blockIdx.x * kItemTilesPerBlock + threadIdx.x * kItemTilesPerThread;
     const SegmentLengths sl = segment_lengths(n_instances_dev ? *n_instances_dev : n_instances_arg, n_tiles, limits);
     load_tile_segments(ranges, n_tiles, t0, sl, ns, rg);
-    unsigned seg = 0, tiles = 0;
-#pragma unroll
-    for (int k = 0; k < kItemTilesPerThread; ++k) { seg += ns[k]; tiles += ns[k] ? 1u : 0u; }
-    const uint2 base = __ldg(block_base + blockIdx.x);
+    const uint4 c = count_tile_segments(ns, rg, sl, by_length), base = __ldg(block_base + blockIdx.x);
+    // a block has at most 1024 tiles: the counts of two classes share a word
     unsigned total;
-    unsigned first = base.x + block_exclusive_scan(seg, s_scan, &total);     // segments of the tiles before this one
-    unsigned rank = base.y + block_exclusive_scan(tiles, s_scan, &total);    // non-empty tiles before this one
+    const unsigned seg_before = block_exclusive_scan(c.x, s_scan, &total);
+    const unsigned first_two = block_exclusive_scan(c.y | (c.z << 16), s_scan, &total);
+    const unsigned third = block_exclusive_scan(c.w, s_scan, &total);
+    unsigned before[3] = {base.y + (first_two & 0xFFFFu), base.z + (first_two >> 16), base.w + third};   // non-empty tiles of a class before this one
+    const unsigned class_base[3] = {0u, __ldg(counts + kLongTiles), __ldg(counts + kLongTiles + 1)};
+    unsigned first = base.x + seg_before;                      // segments of the tiles before this one
+    unsigned rank = before[0] + before[1] + before[2];         // non-empty tiles before this one
 #pragma unroll
     for (int k = 0; k < kItemTilesPerThread; ++k) {
         if (ns[k] == 0u) continue;
         const uint2 r = rg[k];
+        const unsigned cls = length_class(r.y - r.x, sl, by_length);
+        const unsigned place = cls == 0u ? class_base[0] + before[0]++ : cls == 1u ? class_base[1] + before[1]++ : class_base[2] + before[2]++;
         for (unsigned sg = 0; sg < ns[k]; ++sg) {
             const unsigned begin = sg == 0 ? r.x : r.x + sl.first + (sg - 1u) * sl.later;
             const unsigned end = min(r.y, begin + (sg == 0 ? sl.first : sl.later));
             // later segments: position = segments before this tile minus tiles before it
-            WarpItem* dst = sg == 0 ? items0 + rank : items1 + (first - rank + sg - 1u);
+            WarpItem* dst = sg == 0 ? items0 + place : items1 + (first - rank + sg - 1u);
             reinterpret_cast<uint4*>(dst)[0] = make_uint4((uint32_t)(t0 + k), sg, begin, end);
             reinterpret_cast<uint4*>(dst)[1] = make_uint4(first, ns[k], 0u, 0u);
         }
@@ -1551,6 +1587,32 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
         rank += 1u;
     }
 }
+
+// The items of a pass as a warp takes them, through a ticket counter: consecutive items cost about the same (neighbouring
+// tiles, or consecutive segments of one tile), so a warp that reserved items ahead would sit on work that idle warps
+// could take (measured: holding two tickets ahead to prefetch the records made every pass 10-70 % slower).
+// ... unless there are very many of them: a single counter hands out one ticket every 2.7 ns at best (measured:
+// 259,200 items of a 3840x2160 image took 700 us whatever the occupancy), so with many small items a warp takes
+// several consecutive ones per visit, behind the first n_single, which are long.
+struct ItemQueue {
+    unsigned n_items, n_single, per_visit;
+    unsigned next = 0, end = 0;
+    __device__ __forceinline__ ItemQueue(unsigned n_items_, unsigned n_single_, unsigned n_warps)
+        : n_items(n_items_), n_single(min(n_single_, n_items_)), per_visit(max(1u, min(8u, (n_items_ - min(n_single_, n_items_)) / (n_warps * 8u)))) {}
+    __device__ __forceinline__ bool take(unsigned* ticket, unsigned lane, unsigned* item) {
+        if (next == end) {
+            unsigned visit = 0;
+            if (lane == 0) visit = atomicAdd(ticket, 1u);
+            visit = __shfl_sync(0xffffffffu, visit, 0);
+            const bool single = visit < n_single;
+            next = single ? visit : n_single + (visit - n_single) * per_visit;
+            if (next >= n_items) return false;
+            end = single ? next + 1u : min(next + per_visit, n_items);
+        }
+        *item = next++;
+        return true;
+    }
+};
 
 // Asynchronous copies (global -> shared, 16 bytes, not through registers) and their completion groups.
 __device__ __forceinline__ void async_copy_16(void* smem_dst, const void* gmem_src) {
@@ -1734,24 +1796,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4
     if (PASS == PASS_PRODUCT) { sm.sum[0][lane] = 0u; sm.sum[1][lane] = 0u; }   // every batch leaves the sums at zero again
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
-    // Items are handed out one at a time through a ticket counter: consecutive items cost about the same (neighbouring
-    // tiles, or consecutive segments of one tile), so a warp that reserved items ahead would sit on work that idle warps
-    // could take (measured: holding two tickets ahead to prefetch the records made every pass 10-70 % slower).
-    // ... unless there are very many of them: a single counter hands out one ticket every 2.7 ns at best (measured:
-    // 259,200 items of a 3840x2160 image took 700 us whatever the occupancy), so with many small items a warp takes
-    // several consecutive ones per visit.
-    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));
-    unsigned next_item = 0, visit_end = 0;
-    for (;;) {
-        if (next_item == visit_end) {
-            unsigned first_item = 0;
-            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
-            first_item = __shfl_sync(kFull, first_item, 0);
-            if (first_item >= n_items) break;
-            next_item = first_item;
-            visit_end = min(first_item + per_visit, n_items);
-        }
-        const unsigned item = next_item++;
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps);
+    unsigned item;
+    while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(items + (item >> 1));
         const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg, first = it.first;
         const int half = (int)(item & 1u);
@@ -2255,20 +2302,10 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_b
     const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
     const unsigned n_rest = n_items - n_first;
 
-    // items one at a time through a ticket counter, the later segments first (they belong to the longest lists)
-    // (several consecutive ones per visit when there are very many, see the forward pass)
-    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));
-    unsigned next_item = 0, visit_end = 0;
-    for (;;) {
-        if (next_item == visit_end) {
-            unsigned first_item = 0;
-            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
-            first_item = __shfl_sync(kFull, first_item, 0);
-            if (first_item >= n_items) break;
-            next_item = first_item;
-            visit_end = min(first_item + per_visit, n_items);
-        }
-        const unsigned item = next_item++;
+    // the later segments first (they belong to the longest lists)
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps);
+    unsigned item;
+    while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
         const int half = (int)((item < n_rest ? item : item - n_rest) & 1u);
         const unsigned n_list = __ldg(n_kept + (size_t)(it.first + it.seg) * 2u + half);
@@ -2436,18 +2473,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
     const unsigned n_rest = n_items - n_first;
     const int64_t n_px = (int64_t)width * height;
 
-    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));
-    unsigned next_item = 0, visit_end = 0;
-    for (;;) {
-        if (next_item == visit_end) {
-            unsigned first_item = 0;
-            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
-            first_item = __shfl_sync(kFull, first_item, 0);
-            if (first_item >= n_items) break;
-            next_item = first_item;
-            visit_end = min(first_item + per_visit, n_items);
-        }
-        const unsigned item = next_item++;
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps);
+    unsigned item;
+    while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
         const int half = (int)((item < n_rest ? item : item - n_rest) & 1u);
         const unsigned n_list = __ldg(n_kept + (size_t)(it.first + it.seg) * 2u + half);
@@ -3349,18 +3377,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_f
     }
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
-    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));   // see the bilinear kernel
-    unsigned next_item = 0, visit_end = 0;
-    for (;;) {
-        if (next_item == visit_end) {
-            unsigned first_item = 0;
-            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
-            first_item = __shfl_sync(kFull, first_item, 0);
-            if (first_item >= n_items) break;
-            next_item = first_item;
-            visit_end = min(first_item + per_visit, n_items);
-        }
-        const unsigned item = next_item++;
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps);
+    unsigned item;
+    while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(items + (item >> 1));
         const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg, first = it.first;
         const int half = (int)(item & 1u);
@@ -3564,18 +3583,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_b
     const unsigned n_first = __ldg(counts) * 2u;
     const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
     const unsigned n_rest = n_items - n_first;
-    const unsigned per_visit = max(1u, min(8u, n_items / (gridDim.x * kWarpBlendWarps * 8u)));
-    unsigned next_item = 0, visit_end = 0;
-    for (;;) {
-        if (next_item == visit_end) {
-            unsigned first_item = 0;
-            if (lane == 0) first_item = atomicAdd(ticket, per_visit);
-            first_item = __shfl_sync(kFull, first_item, 0);
-            if (first_item >= n_items) break;
-            next_item = first_item;
-            visit_end = min(first_item + per_visit, n_items);
-        }
-        const unsigned item = next_item++;
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps);
+    unsigned item;
+    while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
         const int half = (int)((item < n_rest ? item : item - n_rest) & 1u);
         const unsigned n_list = __ldg(n_kept + (size_t)(it.first + it.seg) * 2u + half);
@@ -3842,7 +3852,7 @@ struct InstanceBlob {
     float* seg_Z;
     float* seg_E;         // warp blend, inference: transmittance at the end of every segment
     int64_t max_segments;
-    uint32_t* tile_rank;  // warp blend: per block of 1024 tiles, the segments and the non-empty tiles before it
+    uint32_t* tile_rank;  // warp blend: per block of 1024 tiles, the segments and the non-empty tiles of each class before it
     WarpItem* items0;     // warp blend: segment 0 of the non-empty tiles
     WarpItem* items1;     // warp blend: every segment behind a tile's first
     uint32_t* n_kept;     // warp blend: per item, length of the compacted list the forward pass blended
@@ -3912,7 +3922,7 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, bool deferred, in
     b.seg_C = c.take<float4>(px * (size_t)c4);
     b.seg_Z = c.take<float>(with_depth ? px : 0);
     b.seg_E = c.take<float>(with_depth && warp_blend ? px : 0);
-    b.tile_rank = c.take<uint32_t>(warp_blend ? (size_t)n_tiles + 8 : 0);   // warp blend: (segments, tiles) per block of 1024 tiles
+    b.tile_rank = c.take<uint32_t>(warp_blend ? (size_t)n_tiles + 8 : 0);   // four words per block of 1024 tiles
     b.items0 = c.take<WarpItem>(warp_blend ? (size_t)n_tiles : 0);
     b.items1 = c.take<WarpItem>(warp_blend ? (size_t)b.max_segments : 0);
     b.n_kept = c.take<uint32_t>(warp_blend ? (size_t)b.max_segments * kWarpBlendParts : 0);
@@ -4200,10 +4210,10 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     if (warp_blend) {
         StageScope scope(STAGE_SORT_TILE, stream);
         const int item_blocks = ceil_div(n_tiles, kItemTilesPerBlock);
-        uint2* item_sums = reinterpret_cast<uint2*>(ib.tile_rank);
-        launch_chained(warp_items_count_kernel, item_blocks, kItemThreads, 0, stream, ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
+        uint4* item_sums = reinterpret_cast<uint4*>(ib.tile_rank);
+        launch_chained(warp_items_count_kernel, item_blocks, kItemThreads, 0, stream, ib.ranges, n_tiles, segment_limits(MODE, !with_depth), VARIANT != VAR_ROWS, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments + 6, ib.n_segments);
         INPC_LAUNCH_CHECK("warp_items_count_kernel");
-        launch_chained(warp_items_fill_kernel, item_blocks, kItemThreads, 0, stream, ib.ranges, n_tiles, segment_limits(MODE, !with_depth), (unsigned long long)n_instances, n_instances_dev, item_sums, ib.items0, ib.items1);
+        launch_chained(warp_items_fill_kernel, item_blocks, kItemThreads, 0, stream, ib.ranges, n_tiles, segment_limits(MODE, !with_depth), VARIANT != VAR_ROWS, (unsigned long long)n_instances, n_instances_dev, item_sums, ib.n_segments, ib.items0, ib.items1);
         INPC_LAUNCH_CHECK("warp_items_fill_kernel");
     } else {
         StageScope scope(STAGE_SORT_TILE, stream);
