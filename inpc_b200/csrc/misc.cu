@@ -176,38 +176,73 @@ __device__ __forceinline__ uint2 cached_pair(const uint2* p) {
     return v;
 }
 
+// Both halves only grow, so a value that does not beat what a plain (possibly stale) read returns cannot beat the current one either: most
+// samples of a leaf that has already seen a few skip both atomics.
+__device__ __forceinline__ void grow_pair(uint2* p, unsigned largest, unsigned flipped, const uint2& read) {
+    if (largest > read.x) atomicMax(&p->x, largest);
+    if (flipped > read.y) atomicMax(&p->y, flipped);
+}
+
+// Bound by the latency of the random reads of `stats`, not by bandwidth (four samples per thread and round, their loads issued together), and,
+// as long as few have landed, by the atomics of the leaves that many samples fall into: all those in flight go to the same word.  So
+// a block's first round is added up in shared memory, in a table without chains: a slot belongs to whichever of its leaves was
+// written last, the samples of the others go to memory by themselves.  2^20 / 2^22 / 2^23 samples 22.8 / 37.5 / 51.3 ->
+// 12.0 / 29.5 / 47.7 us (every round through a table of 1024 slots 13.4 / 39.9 / 70.5, the first one only 11.8 / 33.5 / 58.2).
+constexpr int kStatsPer = 4, kStatsRound = kThreads * kStatsPer;
 __global__ void __launch_bounds__(kThreads) leaf_stats_kernel(const long long* __restrict__ indices, const float* __restrict__ weights,
                                                               int64_t n, int64_t n_leaves, uint2* __restrict__ stats) {
     await_previous_kernel();
-    // four samples per thread and round, their loads issued together: the kernel is bound by the latency of the
-    // random reads of `stats`, not by bandwidth
-    constexpr int kPer = 4;
-    const int64_t stride = (int64_t)gridDim.x * kThreads;
-    for (int64_t i0 = (int64_t)blockIdx.x * kThreads + threadIdx.x; i0 < n; i0 += stride * kPer) {
-        long long leaf[kPer];
-        unsigned bits[kPer];
-        uint2 cur[kPer];
+    __shared__ long long s_leaf[kThreads];   // (small: the reads of the later rounds live on what L1 holds)
+    __shared__ unsigned s_largest[kThreads], s_flipped[kThreads];
+    static_assert(kThreads == 1 << 8, "slots are the top eight bits of a product");
+    long long leaf[kStatsPer];
+    unsigned bits[kStatsPer];
+    auto load_round = [&](int64_t first) {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const int64_t i = i0 + k * stride;
+        for (int k = 0; k < kStatsPer; ++k) {
+            const int64_t i = first + k * kThreads + threadIdx.x;
             leaf[k] = i < n ? __ldg(indices + i) : -1;
             bits[k] = i < n ? __float_as_uint(fmaxf(__ldg(weights + i), 0.0f)) : 0u;
         }
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            if (leaf[k] < 0 || leaf[k] >= n_leaves) leaf[k] = -1;
-            cur[k] = leaf[k] >= 0 ? cached_pair(stats + leaf[k]) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
-        }
-        // Both halves only grow, so a value that does not beat what a plain (possibly stale) read
-        // returns cannot beat the current one either: most samples of a leaf that has already seen a
-        // few skip both atomics.
+        for (int k = 0; k < kStatsPer; ++k)
+            if (leaf[k] >= n_leaves) leaf[k] = -1;
+    };
+    int64_t first = (int64_t)blockIdx.x * kStatsRound;
+    load_round(first);
+    unsigned slot[kStatsPer];
+    s_largest[threadIdx.x] = s_flipped[threadIdx.x] = 0u;
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            if (leaf[k] < 0) continue;
-            const unsigned flipped = kMinFlip - bits[k];
-            if (bits[k] > cur[k].x) atomicMax(&stats[leaf[k]].x, bits[k]);
-            if (flipped > cur[k].y) atomicMax(&stats[leaf[k]].y, flipped);
+    for (int k = 0; k < kStatsPer; ++k) {
+        slot[k] = ((unsigned)leaf[k] * 0x9E3779B1u) >> 24;
+        if (leaf[k] >= 0) s_leaf[slot[k]] = leaf[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kStatsPer; ++k) {
+        if (leaf[k] < 0) continue;
+        const unsigned flipped = kMinFlip - bits[k];
+        if (s_leaf[slot[k]] == leaf[k]) {
+            atomicMax(&s_largest[slot[k]], bits[k]);
+            atomicMax(&s_flipped[slot[k]], flipped);
+        } else {
+            grow_pair(stats + leaf[k], bits[k], flipped, __ldcg(stats + leaf[k]));
         }
+    }
+    __syncthreads();
+    if (s_flipped[threadIdx.x]) {   // not zero where the slot was used
+        // (past L1, so that the later rounds do not find what was there before the first)
+        uint2* const p = stats + s_leaf[threadIdx.x];
+        grow_pair(p, s_largest[threadIdx.x], s_flipped[threadIdx.x], __ldcg(p));
+    }
+    for (first += (int64_t)gridDim.x * kStatsRound; first < n; first += (int64_t)gridDim.x * kStatsRound) {
+        load_round(first);
+        uint2 cur[kStatsPer];
+#pragma unroll
+        for (int k = 0; k < kStatsPer; ++k) cur[k] = leaf[k] >= 0 ? cached_pair(stats + leaf[k]) : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+#pragma unroll
+        for (int k = 0; k < kStatsPer; ++k)
+            if (leaf[k] >= 0) grow_pair(stats + leaf[k], bits[k], kMinFlip - bits[k], cur[k]);
     }
 }
 
@@ -374,7 +409,7 @@ extern "C" int inpc_leaf_stats_accumulate(const int64_t* indices, const float* w
         set_error("inpc_leaf_stats_accumulate: bad argument");
         return INPC_E_INVALID;
     }
-    launch_chained(leaf_stats_kernel, grid_for(n), kThreads, 0, static_cast<cudaStream_t>(stream_), reinterpret_cast<const long long*>(indices), weights, n, n_leaves,
+    launch_chained(leaf_stats_kernel, grid_for(ceil_div<int64_t>(n, kStatsPer)), kThreads, 0, static_cast<cudaStream_t>(stream_), reinterpret_cast<const long long*>(indices), weights, n, n_leaves,
                                                                                      reinterpret_cast<uint2*>(stats));
     INPC_LAUNCH_CHECK("leaf_stats_kernel");
     return INPC_OK;
