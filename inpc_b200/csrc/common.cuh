@@ -124,7 +124,25 @@ int sort_pass_count(int end_bit);   // passes sort_pairs makes; the result is in
 // sort_zero_bytes(n, n_likely, end_bit) bytes of the workspace.
 size_t sort_zero_bytes(int64_t n, int64_t n_likely, int end_bit);
 int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
-               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, bool position_values = false);
+               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, bool position_values = false,
+               bool counted = false);
+// Digits of a sort, and where the histograms of its passes are collected and their exclusive scans (the digit bases) go.
+constexpr int kRadixBits = 9;            // widest digit of a pass: 27 key bits sort in 3 passes, 32 in 4 x 8
+constexpr int kRadix = 1 << kRadixBits;  // capacity of every per-digit array
+constexpr int kMaxPasses = 4;
+struct PassTable {
+    int n_passes;
+    int shift[kMaxPasses];
+    int bits[kMaxPasses];
+};
+struct KeyHistogram {
+    PassTable pt;
+    unsigned *hist, *base;     // [kMaxPasses][kRadix]
+    unsigned* blocks_done;
+};
+// A kernel that makes the keys of a sort can count their digits too (count_key, finish_histogram below) and spare the sort its pass over the
+// keys: the histogram it fills, inside the workspace whose first sort_zero_bytes bytes have been cleared.  The sort is then called with `counted`.
+KeyHistogram key_histogram(void* workspace, int64_t n, int64_t n_likely, int end_bit);
 // Sorts the positions 0 .. n - 1 of the keys other than kNoKey and leaves how many there are in *count (device memory): the first pass
 // leaves the others out, so that whoever writes the keys need not compact them.  The workspace is sized for (n, n); the result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd.  No key that takes part may equal kNoKey, also in bits above end_bit.
@@ -135,7 +153,7 @@ int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint3
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
                             const unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
-                            cudaStream_t stream);
+                            cudaStream_t stream, bool counted = false);
 
 // More than 48 KB of dynamic shared memory is an opt-in per kernel AND per device: `done` is the
 // caller's per-kernel table of devices already set up.
@@ -255,6 +273,56 @@ __device__ __forceinline__ bool last_block(unsigned* done, unsigned n_blocks) {
     }
     __syncthreads();
     return s_last;
+}
+
+// ---- digit histograms of the keys of a sort (see KeyHistogram) ------------------------------------------------
+using BlockHistogram = unsigned[kMaxPasses][kRadix];   // in shared memory
+
+__device__ __forceinline__ void clear_histogram(BlockHistogram& h) {
+    for (unsigned i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) (&h[0][0])[i] = 0u;
+}
+
+__device__ __forceinline__ void count_key(BlockHistogram& h, const PassTable& pt, uint32_t key) {
+#pragma unroll
+    for (int p = 0; p < kMaxPasses; ++p)
+        if (p < pt.n_passes) atomicAdd(&h[p][(key >> pt.shift[p]) & ((1u << pt.bits[p]) - 1u)], 1u);
+}
+
+// Every block of the launch, behind its last count: adds the block's counts to the launch's; the block that finishes last turns those into
+// digit bases (exclusive scans, all passes side by side: one round trip to memory and two barriers), which is a launch less.  *total, if
+// asked for, receives the number of keys.  Blocks of kRadix or 2 kRadix threads.
+__device__ __forceinline__ void finish_histogram(BlockHistogram& h, const KeyHistogram& out, unsigned n_blocks, unsigned long long* total) {
+    __shared__ unsigned s_sum[kMaxPasses][kRadix / 32];
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) {
+        const unsigned c = (&h[0][0])[i];
+        if (c) atomicAdd(out.hist + i, c);
+    }
+    if (!last_block(out.blocks_done, n_blocks)) return;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const bool scans = threadIdx.x < kRadix;
+    unsigned inc[kMaxPasses], own[kMaxPasses];
+    if (scans) {
+#pragma unroll
+        for (int p = 0; p < kMaxPasses; ++p) own[p] = p < out.pt.n_passes ? __ldcg(out.hist + p * kRadix + threadIdx.x) : 0u;
+#pragma unroll
+        for (int p = 0; p < kMaxPasses; ++p) {
+            inc[p] = warp_inclusive_scan(own[p]);
+            if (lane == 31) s_sum[p][warp] = inc[p];
+        }
+    }
+    __syncthreads();
+    if (warp < (unsigned)kMaxPasses) {
+        const unsigned sum = lane < kRadix / 32 ? s_sum[warp][lane] : 0u, before = warp_inclusive_scan(sum) - sum;
+        if (lane < kRadix / 32) s_sum[warp][lane] = before;
+        if (total && warp == 0 && lane == kRadix / 32 - 1) *total = before + sum;
+    }
+    __syncthreads();
+    if (scans) {
+#pragma unroll
+        for (int p = 0; p < kMaxPasses; ++p)
+            if (p < out.pt.n_passes) out.base[p * kRadix + threadIdx.x] = s_sum[p][warp] + inc[p] - own[p];
+    }
 }
 
 // Block-wide exclusive scan of one unsigned per thread; `smem` needs (blockDim.x/32 + 1) words.

@@ -16,9 +16,6 @@ namespace inpc {
 
 namespace {
 
-constexpr int kRadixBits = 9;            // widest digit of a pass: 27 key bits sort in 3 passes, 32 in 4 x 8
-constexpr int kRadix = 1 << kRadixBits;  // capacity of every per-digit array
-constexpr int kMaxPasses = 4;
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kLargeItems = 16;          // pairs per thread and tile, see tile_items
@@ -31,12 +28,6 @@ constexpr unsigned kFlagPrefix = 2u << 30;
 constexpr unsigned kFlagMask = 3u << 30;
 constexpr unsigned kValueMask = ~kFlagMask;
 constexpr int kSpinLimit = 1 << 22;
-
-struct PassTable {
-    int n_passes;
-    int shift[kMaxPasses];
-    int bits[kMaxPasses];
-};
 
 // ---- histogram of every pass in one read ---------------------------------------------------
 constexpr int kHistThreads = 512;
@@ -51,21 +42,16 @@ constexpr int kHistItemsPerBlock = kHistThreads * 4 * 8;   // 8 uint4 loads per 
 // MARKED: keys of kNoKey are left out, and *count_out receives the number of the others.
 template <bool MARKED>
 __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
-    const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, PassTable pt, unsigned* hist, unsigned* blocks_done,
-    unsigned* __restrict__ base, unsigned long long* __restrict__ count_out) {
+    const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, KeyHistogram out, unsigned long long* __restrict__ count_out) {
     await_previous_kernel();
     const int64_t n = n_dev ? (int64_t)*n_dev : n_arg;
     if ((int64_t)blockIdx.x * kHistItemsPerBlock >= n) return;
-    __shared__ unsigned s_hist[kMaxPasses][kRadix];
-    __shared__ unsigned s_scan[kMaxPasses][kHistThreads / 32];
-    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads) (&s_hist[0][0])[i] = 0;
+    __shared__ BlockHistogram s_hist;
+    clear_histogram(s_hist);
     __syncthreads();
 
     auto count = [&](uint32_t k) {
-        if (MARKED && k == kNoKey) return;
-#pragma unroll
-        for (int p = 0; p < kMaxPasses; ++p)
-            if (p < pt.n_passes) atomicAdd(&s_hist[p][(k >> pt.shift[p]) & ((1u << pt.bits[p]) - 1u)], 1u);
+        if (!MARKED || k != kNoKey) count_key(s_hist, out.pt, k);
     };
     for (int64_t block_base = (int64_t)blockIdx.x * kHistItemsPerBlock; block_base < n; block_base += (int64_t)gridDim.x * kHistItemsPerBlock) {
         const int64_t block_end = min(n, block_base + (int64_t)kHistItemsPerBlock);
@@ -78,33 +64,8 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
         }
         for (int64_t i = block_base + (int64_t)n_vec * 4 + threadIdx.x; i < block_end; i += kHistThreads) count(keys[i]);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads) {
-        const unsigned c = (&s_hist[0][0])[i];
-        if (c) atomicAdd(hist + i, c);
-    }
     const int64_t all = ceil_div<int64_t>(n, kHistItemsPerBlock);
-    if (!last_block(blocks_done, (unsigned)min(all, (int64_t)gridDim.x))) return;
-    // all passes side by side: one round trip to memory, two barriers
-    unsigned inc[kMaxPasses], own[kMaxPasses];
-#pragma unroll
-    for (int p = 0; p < kMaxPasses; ++p) own[p] = p < pt.n_passes ? __ldcg(hist + p * kRadix + threadIdx.x) : 0u;
-    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int p = 0; p < kMaxPasses; ++p) {
-        inc[p] = warp_inclusive_scan(own[p]);
-        if (lane == 31) s_scan[p][warp] = inc[p];
-    }
-    __syncthreads();
-    if (warp < (unsigned)kMaxPasses) {
-        const unsigned sum = lane < kHistThreads / 32 ? s_scan[warp][lane] : 0u, before = warp_inclusive_scan(sum) - sum;
-        if (lane < kHistThreads / 32) s_scan[warp][lane] = before;
-        if (MARKED && warp == 0 && lane == kHistThreads / 32 - 1) *count_out = before + sum;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kMaxPasses; ++p)
-        if (p < pt.n_passes) base[p * kRadix + threadIdx.x] = s_scan[p][warp] + inc[p] - own[p];
+    finish_histogram(s_hist, out, (unsigned)min(all, (int64_t)gridDim.x), MARKED ? count_out : nullptr);
 }
 
 // ---- one pass ---------------------------------------------------------------------------------
@@ -415,6 +376,28 @@ static size_t state_words(int64_t tiles, int end_bit) {
     return words;
 }
 
+static PassTable pass_table(int end_bit) {
+    PassTable pt;
+    pt.n_passes = ceil_div(end_bit, kRadixBits);
+    int bit = 0;
+    for (int p = 0; p < kMaxPasses; ++p) { pt.shift[p] = 0; pt.bits[p] = 0; }
+    for (int p = 0; p < pt.n_passes; ++p) {
+        // spread the bits evenly over the passes (e.g. 12 bits -> 6 + 6): fewer digits per pass
+        // means longer, better-coalesced output runs
+        const int b = (end_bit - bit + (pt.n_passes - p) - 1) / (pt.n_passes - p);
+        pt.shift[p] = bit;
+        pt.bits[p] = b;
+        bit += b;
+    }
+    return pt;
+}
+
+static KeyHistogram histogram_of(const SortWorkspace& w, int end_bit) { return {pass_table(end_bit), w.hist, w.base, w.ticket + kMaxPasses}; }
+
+KeyHistogram key_histogram(void* workspace, int64_t n, int64_t n_likely, int end_bit) {
+    return histogram_of(carve_sort_workspace(workspace, n, tile_items(n_likely)), end_bit);
+}
+
 // Histograms, tickets and the look-back state lie at the front of the workspace.
 size_t sort_zero_bytes(int64_t n, int64_t n_likely, int end_bit) {
     if (n <= 0 || end_bit <= 0) return 0;
@@ -453,34 +436,22 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 // `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
                            int items, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
-                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, unsigned long long* marked_count = nullptr) {
+                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, unsigned long long* marked_count = nullptr, bool counted = false) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
 
-    PassTable pt;
-    pt.n_passes = ceil_div(end_bit, kRadixBits);
-    int bit = 0;
-    for (int p = 0; p < kMaxPasses; ++p) { pt.shift[p] = 0; pt.bits[p] = 0; }
-    for (int p = 0; p < pt.n_passes; ++p) {
-        // spread the bits evenly over the passes (e.g. 12 bits -> 6 + 6): fewer digits per pass
-        // means longer, better-coalesced output runs
-        const int b = (end_bit - bit + (pt.n_passes - p) - 1) / (pt.n_passes - p);
-        pt.shift[p] = bit;
-        pt.bits[p] = b;
-        bit += b;
-    }
-
+    const PassTable pt = pass_table(end_bit);
     SortWorkspace w = carve_sort_workspace(workspace, n, items);
     const int64_t tiles = ceil_div<int64_t>(n, (int64_t)kThreads * items);
     // a workspace that is reused keeps the previous call's contents, so everything this call reads is cleared first
     if (!zeroed) INPC_CUDA_TRY(cudaMemsetAsync(workspace, 0, w.zero_bytes + state_words(tiles, end_bit) * sizeof(unsigned), stream));
 
-    const int64_t hist_blocks = ceil_div<int64_t>(n, kHistItemsPerBlock), hist_cap = (int64_t)sm_count() * 4;
-    const unsigned hist_grid = (unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap);
-    unsigned* hist_done = w.ticket + kMaxPasses;
-    if (marked_count) launch_chained(radix_histogram_kernel<true>, hist_grid, kHistThreads, 0, stream, keys, n, n_dev, pt, w.hist, hist_done, w.base, marked_count);
-    else launch_chained(radix_histogram_kernel<false>, hist_grid, kHistThreads, 0, stream, keys, n, n_dev, pt, w.hist, hist_done, w.base, nullptr);
-    INPC_LAUNCH_CHECK("radix_histogram_kernel");
+    if (!counted) {
+        const int64_t hist_blocks = ceil_div<int64_t>(n, kHistItemsPerBlock), hist_cap = (int64_t)sm_count() * 4;
+        const unsigned hist_grid = (unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap);
+        launch_chained(marked_count ? radix_histogram_kernel<true> : radix_histogram_kernel<false>, hist_grid, kHistThreads, 0, stream, keys, n, n_dev, histogram_of(w, end_bit), marked_count);
+        INPC_LAUNCH_CHECK("radix_histogram_kernel");
+    }
 
     PassArgs a;
     a.tiles = tiles; a.n = n; a.n_dev = n_dev; a.status = status;
@@ -509,14 +480,14 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
 // `position_values`: the values to be sorted are 0 .. n - 1 and need not lie in `values` (with fewer than two pairs, where nothing
 // is done, they do).
 int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int64_t n_likely,
-               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, bool position_values) {
+               int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, bool position_values, bool counted) {
     if (result_in_alt) *result_in_alt = 0;
     bool nothing = false;
     const int rc = check_sort_args("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, &nothing);
     if (rc != INPC_OK || nothing) return rc;
     if (!workspace) { set_error("sort_pairs: null workspace"); return INPC_E_INVALID; }
     return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n_likely), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
-                           0xFFFFFFFFu, nullptr, position_values);
+                           0xFFFFFFFFu, nullptr, position_values, nullptr, counted);
 }
 
 int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
@@ -535,7 +506,7 @@ int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint3
 // the number of passes is odd.  No host synchronisation anywhere.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
                             const unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
-                            cudaStream_t stream) {
+                            cudaStream_t stream, bool counted) {
     if (result_in_alt) *result_in_alt = 0;
     if (n_max <= 0 || end_bit == 0) return INPC_OK;
     bool nothing = false;
@@ -543,7 +514,7 @@ int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values
     if (rc != INPC_OK) return rc;
     if (!workspace || !n_dev) { set_error("sort_pairs: null workspace or count"); return INPC_E_INVALID; }
     return sort_pairs_with("sort_pairs", keys, keys_alt, values, values_alt, n_max, end_bit, tile_items(n_likely), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
-                           0xFFFFFFFFu, n_dev);
+                           0xFFFFFFFFu, n_dev, false, nullptr, counted);
 }
 
 }  // namespace inpc

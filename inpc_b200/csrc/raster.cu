@@ -642,19 +642,69 @@ __device__ __forceinline__ unsigned cell_code(int left, int right, int top, int 
 }
 
 // One (tile key, point id) pair per touched tile, row-major over the point's bounds, points in depth
-// order (src/bilinear/kernels.cu:198-220).  EMIT_QUAD (bilinear, 8x8 tiles): bounds and footprint origin come
-// from the packed word the projection pass left per point (see pack_quad), a 4-byte gather.  EMIT_CELLS (gaussian, 8x8 tiles):
-// the key also says which cells of the tile the ellipse can reach (see cell_code).
-// Bound by the random 4-byte gathers, one 32-byte sector each, and by instruction issue.  What is read or written once bypasses
-// the caches' replacement, so that more of the gathered array stays in L2.  A bilinear splat has one, two or four instances: the sums over a warp
-// come from three ballots, those over a block from one barrier and a warp reduction, and the keys are put together without a loop: 2^23 / 2^24 /
-// 2^25 points 97 / 204 / 451 -> 85 / 178 / 455 us (a scan of three barriers and loops over the tiles, 189 instructions per warp; the last
-// is bound by DRAM, the gathered array being larger than L2).  (Four consecutive points per thread with their gathers in
-// flight together and the instances staged in shared memory: 116 / 396 / 952 us.)
-enum { EMIT_BOUNDS = 0, EMIT_QUAD = 1, EMIT_CELLS = 2 };
-template <int KEYS>
+// order (src/bilinear/kernels.cu:198-220).
+//
+// Bilinear splats on 8x8 tiles: bounds and footprint origin come from the packed word the projection pass left per point (see pack_quad), a 4-byte
+// gather.  Bound by these random gathers, one 32-byte sector each, and by instruction issue.  What is read or written once bypasses
+// the caches' replacement, so that more of the gathered array stays in L2.  A splat has one, two or four instances: the sums over a warp
+// come from three ballots, those over a block from one barrier and a warp reduction, and the keys are put together without a loop.  A block takes
+// groups of 1024 points one after the other and counts the digits of the keys it writes, which spares the tile sort its pass over them: emission and
+// histogram of 2^20 / 2^23 / 2^24 / 2^25 points 21 / 104 / 207 / 496 -> 16 / 95 / 192 / 412 us (half of the last by fewer blocks).
+// (Four consecutive points per thread with their gathers in flight together and the instances staged in shared memory: the emission alone 116 us for
+// 2^23 points, 396 for 2^24, 952 for 2^25.)
+__global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
+                                                                     const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
+                                                                     KeyHistogram digits, uint32_t* __restrict__ inst_keys, uint32_t* __restrict__ inst_ids) {
+    await_previous_kernel();
+    __shared__ unsigned s_total[2][kInstThreads / 32];   // of two groups in turn, so that one barrier does
+    __shared__ BlockHistogram s_digits;
+    const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
+    const int64_t n_groups = ceil_div<int64_t>(n_visible, kInstThreads);
+    if ((int64_t)blockIdx.x >= n_groups) return;
+    clear_histogram(s_digits);
+    __syncthreads();
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5, lt_mask = (1u << lane) - 1u;
+    auto emit = [&](unsigned at, uint32_t key, uint32_t id) {
+        __stcs(inst_keys + at, key);
+        __stcs(inst_ids + at, id);
+        count_key(s_digits, digits.pt, key);
+    };
+    unsigned flip = 0;
+    for (int64_t group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1u) {
+        const int64_t s = group * kInstThreads + threadIdx.x;
+        const bool there = s < n_visible;
+        const uint32_t id = there ? checked_point(__ldcs(sorted_ids + s)) : 0u;
+        const uint32_t q = there ? __ldg(quad + id) : 0u;
+        const bool two_columns = there && ((q >> 15) & 1u), two_rows = there && (q >> 31);
+        // one, two or four instances per point: the sum over the lanes before this one from three ballots
+        const unsigned bt = __ballot_sync(0xffffffffu, there), bc = __ballot_sync(0xffffffffu, two_columns), br = __ballot_sync(0xffffffffu, two_rows);
+        if (lane == 0) s_total[flip][warp] = __popc(bt) + __popc(bc) + __popc(br) + __popc(bc & br);
+        __syncthreads();
+        unsigned off = __ldg(block_base + group) + __reduce_add_sync(0xffffffffu, lane < warp ? s_total[flip][lane] : 0u) + __popc(bt & lt_mask) + __popc(bc & lt_mask) +
+                       __popc(br & lt_mask) + __popc(bc & br & lt_mask);
+        if (!there) continue;
+        // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0.  In a second column or
+        // row of tiles the footprint starts one pixel before the tile: its code there is zero
+        const int qx = (int)(q & 0x7FFFu) - 1;
+        const unsigned x0 = qx < 0 ? 0u : (unsigned)qx >> 3, y0 = (q >> 16) & 0x7FFu;
+        const uint32_t column = (unsigned)(qx - (int)x0 * 8 + 1) << kTileKeyBits, row = min((q >> 27) & 0xFu, 8u) << (kTileKeyBits + 4);
+        const uint32_t tile = y0 * (unsigned)gw + x0;
+        emit(off, tile | column | row, id);
+        if (two_columns) emit(off + 1u, (tile + 1u) | row, id);
+        if (two_rows) {
+            off += two_columns ? 2u : 1u;
+            emit(off, (tile + (unsigned)gw) | column, id);
+            if (two_columns) emit(off + 1u, tile + (unsigned)gw + 1u, id);
+        }
+    }
+    finish_histogram(s_digits, digits, (unsigned)min(n_groups, (int64_t)gridDim.x), nullptr);
+}
+
+// Other splats.  CELLS (gaussian, 8x8 tiles): the key also says which cells of the tile the ellipse can reach (see cell_code).  The keys are counted by the
+// sort: a gaussian splat has many instances, whose atomics would go one after the other (2^22 of them, emission and histogram 61 + 13 -> 90 us).
+template <bool CELLS>
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
-                                                                      const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad,
+                                                                      const uint2* __restrict__ bounds,
                                                                       const uint4* __restrict__ foot, int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
                                                                       const unsigned* __restrict__ block_base, int gw,
                                                                       uint32_t* __restrict__ inst_keys,
@@ -673,42 +723,10 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
         __syncthreads();
         return __ldg(block_base + blockIdx.x) + __reduce_add_sync(0xffffffffu, lane < warp ? s_total[lane] : 0u);
     };
-    if (KEYS == EMIT_QUAD) {
-        const uint32_t q = there ? __ldg(quad + id) : 0u;
-        const bool two_columns = there && ((q >> 15) & 1u), two_rows = there && (q >> 31);
-        // one, two or four instances per point: the sum over the lanes before this one from three ballots
-        const unsigned bt = __ballot_sync(0xffffffffu, there), bc = __ballot_sync(0xffffffffu, two_columns), br = __ballot_sync(0xffffffffu, two_rows);
-        const unsigned lt_mask = (1u << lane) - 1u;
-        unsigned off = before_warp(__popc(bt) + __popc(bc) + __popc(br) + __popc(bc & br)) + __popc(bt & lt_mask) + __popc(bc & lt_mask) + __popc(br & lt_mask) +
-                       __popc(bc & br & lt_mask);
-        if (!there) return;
-        // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0.  In a second column or
-        // row of tiles the footprint starts one pixel before the tile: its code there is zero
-        const int qx = (int)(q & 0x7FFFu) - 1;
-        const unsigned x0 = qx < 0 ? 0u : (unsigned)qx >> 3, y0 = (q >> 16) & 0x7FFu;
-        const uint32_t column = (unsigned)(qx - (int)x0 * 8 + 1) << kTileKeyBits, row = min((q >> 27) & 0xFu, 8u) << (kTileKeyBits + 4);
-        const uint32_t tile = y0 * (unsigned)gw + x0;
-        __stcs(inst_keys + off, tile | column | row);
-        __stcs(inst_ids + off, id);
-        if (two_columns) {
-            __stcs(inst_keys + off + 1u, (tile + 1u) | row);
-            __stcs(inst_ids + off + 1u, id);
-        }
-        if (two_rows) {
-            off += two_columns ? 2u : 1u;
-            __stcs(inst_keys + off, (tile + (unsigned)gw) | column);
-            __stcs(inst_ids + off, id);
-            if (two_columns) {
-                __stcs(inst_keys + off + 1u, tile + (unsigned)gw + 1u);
-                __stcs(inst_ids + off + 1u, id);
-            }
-        }
-        return;
-    }
     unsigned x0 = 0, x1 = 0, y0 = 0, y1 = 0, inset = 0;
     if (there) {
         uint2 b;
-        if (KEYS == EMIT_CELLS) {
+        if (CELLS) {
             const uint4 f = __ldg(foot + id);
             b = make_uint2(f.x, f.y);
             inset = f.z;
@@ -723,7 +741,7 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
     for (unsigned ty = y0; ty < y1; ++ty)
         for (unsigned tx = x0; tx < x1; ++tx) {
             uint32_t key = ty * (unsigned)gw + tx;
-            if (KEYS == EMIT_CELLS) {
+            if (CELLS) {
                 const int left = (int)(inset & 15u) - 4 * (int)(tx - x0), right = 4 * (int)(x1 - tx) - 1 - (int)((inset >> 4) & 15u);
                 const int top = (int)((inset >> 8) & 15u) - 4 * (int)(ty - y0), bottom = 4 * (int)(y1 - ty) - 1 - (int)(inset >> 12);
                 key |= cell_code(left, right, top, bottom) << kTileKeyBits;
@@ -4171,6 +4189,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         if (rc != INPC_OK) return rc;
     }
 
+    const bool counted = MODE == INPC_MODE_BILINEAR && warp_blend;   // the emission counts the digits of the keys
     int in_alt = 0;
     {
         StageScope scope(STAGE_SORT_DEPTH, stream);
@@ -4190,18 +4209,21 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             else
                 launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr);
             INPC_LAUNCH_CHECK("instance_count_kernel");
-            if (warp_blend && MODE == INPC_MODE_GAUSSIAN)
-                launch_chained(emit_instances_kernel<EMIT_CELLS>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, nullptr, pb.foot, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
-            else if (warp_blend)
-                launch_chained(emit_instances_kernel<EMIT_QUAD>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.quad, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
-            else
-                launch_chained(emit_instances_kernel<EMIT_BOUNDS>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, nullptr, nullptr, n_visible, n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+            if (counted) {
+                const int64_t emit_cap = (int64_t)sm_count() * 2;   // two blocks of 1024 threads fill a multiprocessor
+                const KeyHistogram digits = key_histogram(ib.sort_ws, n_instances, likely_instances(n_instances, deferred), tile_bits);
+                launch_chained(emit_quads_kernel, (unsigned)(ibk < emit_cap ? ibk : emit_cap), kInstThreads, 0, stream, sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums,
+                    rp.gw, digits, ib.keys[0], ib.ids[0]);
+            } else {
+                launch_chained(warp_blend ? emit_instances_kernel<true> : emit_instances_kernel<false>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.foot, n_visible,
+                    n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
+            }
             INPC_LAUNCH_CHECK("emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
-        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream)
-                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), tile_bits, ib.sort_ws, true, status, &t_alt, stream);
+        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream, counted)
+                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), tile_bits, ib.sort_ws, true, status, &t_alt, stream, false, counted);
         if (rc != INPC_OK) return rc;
         const int64_t range_blocks = ceil_div<int64_t>(n_instances, 256 * 8), range_cap = (int64_t)sm_count() * 8;
         launch_chained(tile_ranges_kernel, (unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream, ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);

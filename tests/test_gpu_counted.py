@@ -1,0 +1,35 @@
+"""GPU tests of kernels that count the digits of the keys they make for the sort behind them, at the edges of their blocks, bit for bit against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# groups of 1024 points, blocks that take several of them; images of one tile (nothing to sort by), of 2^7 tiles and one more, of more than 2^14; 2^18 tiles for three passes
+@pytest.mark.parametrize("tile, width, height", [(8, 8, 8), (8, 16, 8), (8, 128, 64), (8, 136, 64), (8, 1032, 1024), (8, 4096, 4104), (16, 40, 24), (16, 2064, 2048)])
+@pytest.mark.parametrize("n", [1, 1023, 1025, 400_001])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_lists_of_points_counted_while_their_instances_are_emitted(tile, width, height, n, mode):
+    from helpers import oracle_camera
+    from inpc_b200 import rasterization as R
+    from inpc_b200.views import look_at_view
+    if n > 2000 and width * height > 1 << 21:
+        pytest.skip("the oracle takes long")
+    g = torch.Generator().manual_seed(n + width)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, float(width), float(width))
+    z = torch.rand(n, generator=g)
+    px, py = torch.rand(n, generator=g) * (width + 8) - 4, torch.rand(n, generator=g) * (height + 8) - 4
+    pos = torch.stack([(px - width / 2) / width * (3 - z), -(py - height / 2) / width * (3 - z), z], dim=1).contiguous()
+    feats, opac = torch.zeros((n, 36), dtype=torch.float16), torch.full((n, 1), 0.01)
+    v = view.to(DEV)
+    settings = R.INPCRasterizer.extract_settings(v, mode)
+    _, _, _, state, blobs, _ = R.forward_with_state(pos.to(DEV), feats.to(DEV), opac.to(DEV), settings, tile)
+    st = O.preprocess_and_order(mode, O.TRAIN, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy(), tile=tile)
+    dbg = R.debug_arrays(state, settings, blobs.point, blobs.instance)
+    assert int(state.n_visible) == len(st.sorted_points) and int(state.n_instances) == len(st.inst_point)
+    assert np.array_equal(dbg["inst_point"].cpu().numpy().view(np.uint32), st.inst_point)
+    assert np.array_equal(dbg["ranges"].cpu().numpy().view(np.uint32), st.ranges)
