@@ -438,8 +438,10 @@ int inpc_multisample_resolve(float* acc_image, float* acc_depth, float* acc_alph
  *                          Stands in for NeRFICG's CudaUtils.MortonEncoding.morton_encode + argsort
  *                          (ProbabilityField.py:141-143), which is not part of the reference tree:
  *                          the code width and the box are this library's choice.
+ *   inpc_halton_morton_order  the two in one call, in the cloud's own bounding cube: `positions` receives
+ *                          the samples leaf by leaf, `out` the same in Morton order.
  * `workspace`: inpc_sampler_workspace_bytes(n_cells) for the first two, inpc_morton_workspace_bytes(n)
- * for the third. */
+ * for the third, both for the last. */
 int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const float* weights, int64_t n_samples,
                           uint32_t* counts, void* workspace, void* stream);
 int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels,
@@ -447,6 +449,9 @@ int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, const float* ce
 size_t inpc_morton_workspace_bytes(int64_t n);
 int inpc_morton_order(const float* positions, int64_t n, const float* box_lo, float box_extent, float* out,
                       void* workspace, void* stream);
+int inpc_halton_morton_order(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels,
+                             float initial_size, int64_t n_total, float* positions, float* out,
+                             void* sampler_workspace, void* morton_workspace, void* stream);
 
 #ifdef __cplusplus
 }

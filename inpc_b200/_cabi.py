@@ -88,6 +88,7 @@ PROTOTYPES = {
     "inpc_draw_leaf_counts": (_I, [_P, _L, _P, _L, _P, _P, _P]),
     "inpc_halton_samples": (_I, [_P, _L, _P, _P, _F, _L, _P, _P, _P]),
     "inpc_morton_workspace_bytes": (_Z, [_L]),
+    "inpc_halton_morton_order": (_I, [_P, _L, _P, _P, _F, _L, _P, _P, _P, _P, _P]),
     "inpc_morton_order": (_I, [_P, _L, C.POINTER(C.c_float), _F, _P, _P, _P]),
     "inpc_compose_background": (_I, [_P, _P, _P, _I, _L, _P, _P]),
     "inpc_compose_background_backward": (_I, [_P, _P, _P, _I, _L, _P, _P, _P]),

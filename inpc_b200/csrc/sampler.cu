@@ -766,6 +766,59 @@ __device__ __forceinline__ float halton_element(const Table& t, unsigned index) 
     return __double2float_rn(result);
 }
 
+// Minimum and maximum that are NaN when an operand is, as a tensor's amin and amax are.
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// Corners of the cloud's bounding box, one partial result {min x, y, z, max x, y, z} per block: one pass over the positions,
+// four of them per thread and round in three 16-byte loads where the array allows.
+constexpr int kMaxBoxBlocks = 1024;   // room for the partial boxes; four blocks per multiprocessor are launched
+template <int WARPS>
+__device__ __forceinline__ void block_box(float* box, float (&s_box)[WARPS][6]) {
+    // box[0..2] minima, box[3..5] maxima of a thread -> of the block, in every thread
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float t = __shfl_xor_sync(0xffffffffu, box[c], o);
+            box[c] = c < 3 ? min_nan(box[c], t) : max_nan(box[c], t);
+        }
+    if (lane_id() == 0) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) s_box[threadIdx.x >> 5][c] = box[c];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        box[c] = s_box[0][c];
+#pragma unroll
+        for (int w = 1; w < WARPS; ++w) box[c] = c < 3 ? min_nan(box[c], s_box[w][c]) : max_nan(box[c], s_box[w][c]);
+    }
+}
+
+// A bounding box collected by many blocks: words that start at zero and only grow, the maxima as keys that order
+// like the values, the minima as the complements of such keys; all ones where a coordinate is no number.  Several copies, so that the blocks do not queue
+// for six words.
+constexpr int kBoxCopies = 64;
+__device__ __forceinline__ unsigned box_word(float v, bool minimum) {
+    const unsigned bits = __float_as_uint(v), key = bits & 0x80000000u ? ~bits : bits | 0x80000000u;
+    return v != v ? 0xFFFFFFFFu : minimum ? ~key : key;
+}
+__device__ __forceinline__ float box_value(unsigned word, bool minimum) {
+    if (word == 0u) return minimum ? INFINITY : -INFINITY;   // of no position
+    if (word == 0xFFFFFFFFu) return __uint_as_float(0x7FFFFFFFu);
+    const unsigned key = minimum ? ~word : word;
+    return __uint_as_float(key & 0x80000000u ? key & 0x7FFFFFFFu : ~key);
+}
+
 // Sample i lies in leaf upper_bound(offsets, i) and is that leaf's h-th sample, h = i - first sample
 // of the leaf: Halton point h+1 in bases (2, 3, 5) scaled into the cell; a leaf with a single sample
 // puts it at its centre (ProbabilityField.py:131-140).
@@ -829,6 +882,54 @@ __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned
     }
 }
 
+// Of the indices 1 .. c the one whose radical inverse is largest: digit by digit from the least significant, which weighs most, the largest there is an index for.
+template <unsigned BASE>
+__device__ __forceinline__ unsigned largest_halton_index(unsigned c) {
+    unsigned h = 0u;
+    for (unsigned long long m = 1u; m <= c - h; m *= BASE) h += (unsigned)m * min(BASE - 1u, (unsigned)((c - h) / (unsigned)m));
+    return h;
+}
+// ... and smallest: the largest power of the base.
+template <unsigned BASE>
+__device__ __forceinline__ unsigned smallest_halton_index(unsigned c) {
+    unsigned long long m = 1u;
+    while (m * BASE <= c) m *= BASE;
+    return (unsigned)m;
+}
+
+// Bounding box of the cloud that halton_samples_kernel makes, from the leaves: along an axis the extreme samples of a leaf are those of its extreme Halton elements
+// (placing one rounds, but monotonically).  Spares the Morton order a pass over the positions: 2^25 samples of 2.3 * 10^5 leaves 78 us -> 11 (in the placement itself,
+// six comparisons per sample, 39).
+__global__ void __launch_bounds__(kThreads) halton_box_kernel(const unsigned* __restrict__ counts, unsigned n_cells, const float* __restrict__ centers, const int* __restrict__ levels,
+                                                              float initial_size, unsigned* box_words) {
+    await_previous_kernel();
+    __shared__ float s_box[kThreads / 32][6];
+    float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    auto add = [&](int axis, float v) {
+        box[axis] = min_nan(box[axis], v);
+        box[3 + axis] = max_nan(box[3 + axis], v);
+    };
+    for (unsigned leaf = blockIdx.x * kThreads + threadIdx.x; leaf < n_cells; leaf += gridDim.x * kThreads) {
+        const unsigned c = __ldg(counts + leaf);
+        if (c == 0u) continue;
+        const HaltonLeaf at = halton_leaf(centers, levels, initial_size, leaf, c);
+        if (c == 1u) {
+            add(0, at.x); add(1, at.y); add(2, at.z);
+            continue;
+        }
+        add(0, __fadd_rn(at.x, __fmul_rn(halton_base2(smallest_halton_index<2u>(c)), at.cell)));
+        add(0, __fadd_rn(at.x, __fmul_rn(halton_base2(largest_halton_index<2u>(c)), at.cell)));
+        add(1, __fadd_rn(at.y, __fmul_rn(halton_element(g_halton.b3, smallest_halton_index<3u>(c)), at.cell)));
+        add(1, __fadd_rn(at.y, __fmul_rn(halton_element(g_halton.b3, largest_halton_index<3u>(c)), at.cell)));
+        add(2, __fadd_rn(at.z, __fmul_rn(halton_element(g_halton.b5, smallest_halton_index<5u>(c)), at.cell)));
+        add(2, __fadd_rn(at.z, __fmul_rn(halton_element(g_halton.b5, largest_halton_index<5u>(c)), at.cell)));
+    }
+    block_box(box, s_box);
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+        if (threadIdx.x == c) atomicMax(box_words + (blockIdx.x % kBoxCopies) * 6 + c, box_word(box[c], c < 3));
+}
+
 // 30-bit Morton code (10 bits per axis, x lowest) of a position inside the box [lo, lo + extent]^3
 __device__ __forceinline__ unsigned spread_bits_10(unsigned v) {
     v &= 0x3FFu;
@@ -837,43 +938,6 @@ __device__ __forceinline__ unsigned spread_bits_10(unsigned v) {
     v = (v | (v << 4)) & 0x030C30C3u;
     v = (v | (v << 2)) & 0x09249249u;
     return v;
-}
-
-// Minimum and maximum that are NaN when an operand is, as a tensor's amin and amax are.
-__device__ __forceinline__ float min_nan(float a, float b) {
-    float r;
-    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float max_nan(float a, float b) {
-    float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-    return r;
-}
-
-// Corners of the cloud's bounding box, one partial result {min x, y, z, max x, y, z} per block: one pass over the positions,
-// four of them per thread and round in three 16-byte loads where the array allows.
-constexpr int kMaxBoxBlocks = 1024;   // room for the partial boxes; four blocks per multiprocessor are launched
-__device__ __forceinline__ void block_box(float* box, float (*s_box)[6]) {
-    // box[0..2] minima, box[3..5] maxima of a thread -> of the block, in every thread of warp 0
-#pragma unroll
-    for (int c = 0; c < 6; ++c)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float t = __shfl_xor_sync(0xffffffffu, box[c], o);
-            box[c] = c < 3 ? min_nan(box[c], t) : max_nan(box[c], t);
-        }
-    if (lane_id() == 0) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) s_box[threadIdx.x >> 5][c] = box[c];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-        box[c] = s_box[0][c];
-#pragma unroll
-        for (int w = 1; w < kThreads / 32; ++w) box[c] = c < 3 ? min_nan(box[c], s_box[w][c]) : max_nan(box[c], s_box[w][c]);
-    }
 }
 
 __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, float* __restrict__ partial) {
@@ -902,19 +966,25 @@ __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __r
 struct MortonBox {
     float lo[3];
     float inv_extent;
-    const float* parts;
+    const float* parts;       // partial boxes as values ...
+    const unsigned* words;    // ... or as words, see box_word
     int box_parts;
 };
-__global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, MortonBox mb,
+// Also counts the digits of the codes for their sort, which spares it a pass over them: 2^25 codes and their histogram 90 + 53 -> 132 us.
+constexpr int kCodeThreads = kRadix;
+__global__ void __launch_bounds__(kCodeThreads) morton_codes_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, MortonBox mb, KeyHistogram digits,
                                                                 unsigned* __restrict__ codes, unsigned* __restrict__ order) {
     await_previous_kernel();
+    __shared__ BlockHistogram s_digits;
+    clear_histogram(s_digits);
+    __syncthreads();
     if (mb.box_parts > 0) {
-        __shared__ float s_box[kThreads / 32][6];
+        __shared__ float s_box[kCodeThreads / 32][6];
         float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        for (int k = threadIdx.x; k < mb.box_parts; k += kThreads)
+        for (int k = threadIdx.x; k < mb.box_parts; k += kCodeThreads)
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                const float t = __ldg(mb.parts + 6 * k + c);
+                const float t = mb.words ? box_value(__ldg(mb.words + 6 * k + c), c < 3) : __ldg(mb.parts + 6 * k + c);
                 box[c] = c < 3 ? min_nan(box[c], t) : max_nan(box[c], t);
             }
         block_box(box, s_box);
@@ -928,12 +998,14 @@ __global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __r
         const float qz = (pz - mb.lo[2]) * mb.inv_extent * 1024.0f;
         const unsigned x = (unsigned)fminf(fmaxf(qx, 0.0f), 1023.0f), y = (unsigned)fminf(fmaxf(qy, 0.0f), 1023.0f),
                        z = (unsigned)fminf(fmaxf(qz, 0.0f), 1023.0f);
-        return spread_bits_10(x) | (spread_bits_10(y) << 1) | (spread_bits_10(z) << 2);
+        const unsigned key = spread_bits_10(x) | (spread_bits_10(y) << 1) | (spread_bits_10(z) << 2);
+        count_key(s_digits, digits.pt, key);
+        return key;
     };
     // four points per thread: three 16-byte loads where the positions are aligned, one 16-byte store.  Bound by DRAM: 2^25 points
     // 91 us (one point per thread, and the point numbers written for the sort, which now makes them itself: 131)
-    const int64_t stride = (int64_t)gridDim.x * kThreads * 4;
-    for (int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4; i < n; i += stride) {
+    const int64_t stride = (int64_t)gridDim.x * kCodeThreads * 4;
+    for (int64_t i = ((int64_t)blockIdx.x * kCodeThreads + threadIdx.x) * 4; i < n; i += stride) {
         if (vec_ok && i + 4 <= n) {
             const float4* src = reinterpret_cast<const float4*>(positions + 3 * i);
             const float4 a = __ldg(src), b = __ldg(src + 1), c = __ldg(src + 2);
@@ -943,6 +1015,7 @@ __global__ void __launch_bounds__(kThreads) morton_codes_kernel(const float* __r
         }
     }
     if (n == 1 && blockIdx.x == 0 && threadIdx.x == 0) order[0] = 0u;   // a single pair is not sorted
+    finish_histogram(s_digits, digits, gridDim.x, nullptr);
 }
 
 // Four points per thread, their gathers in flight together and three 16-byte stores (2^25 points 167 us; one
@@ -1323,28 +1396,78 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
     return INPC_OK;
 }
 
-extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size,
-                                   int64_t n_total, float* positions, void* workspace, void* stream_) {
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    if (n_total == 0) return INPC_OK;
+// `box_words` (optional): 6 kBoxCopies words that start at zero, see box_word.
+static int launch_halton(const char* who, const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size, int64_t n_total,
+                         float* positions, void* workspace, unsigned* box_words, cudaStream_t stream) {
     if (n_cells <= 0 || n_cells >= ((int64_t)1 << 31) || n_total < 0 || n_total >= ((int64_t)1 << 32) || !counts || !centers || !levels || !positions || !workspace) {
-        set_error("inpc_halton_samples: bad argument");
+        set_error("%s: bad argument", who);
         return INPC_E_INVALID;
     }
     SamplerWs w = carve_sampler_ws(workspace, n_cells);
     INPC_CUDA_TRY(cudaMemcpyAsync(w.counts, counts, sizeof(uint32_t) * (size_t)n_cells, cudaMemcpyDeviceToDevice, stream));
     const int rc = scan_counts(w, n_cells, stream);
     if (rc != INPC_OK) return rc;
-    launch_chained(halton_samples_kernel, (unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream, w.counts, w.offsets, (unsigned)n_cells, centers, levels,
-                                                                                                 initial_size, (unsigned)n_total, positions);
+    if (box_words) {
+        const int64_t box_blocks = ceil_div<int64_t>(n_cells, kThreads), box_cap = (int64_t)sm_count() * 8;
+        launch_chained(halton_box_kernel, (unsigned)(box_blocks < box_cap ? box_blocks : box_cap), kThreads, 0, stream, w.counts, (unsigned)n_cells, centers, levels, initial_size, box_words);
+        INPC_LAUNCH_CHECK("halton_box_kernel");
+    }
+    launch_chained(halton_samples_kernel, (unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream, w.counts, w.offsets,
+                   (unsigned)n_cells, centers, levels, initial_size, (unsigned)n_total, positions);
     INPC_LAUNCH_CHECK("halton_samples_kernel");
     return INPC_OK;
+}
+
+extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size,
+                                   int64_t n_total, float* positions, void* workspace, void* stream) {
+    if (n_total == 0) return INPC_OK;
+    return launch_halton("inpc_halton_samples", counts, n_cells, centers, levels, initial_size, n_total, positions, workspace, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t inpc_morton_workspace_bytes(int64_t n) {
     const size_t arr = align_up(sizeof(uint32_t) * (size_t)(n > 0 ? n : 1));
     return 4 * arr + align_up(6 * sizeof(float) * kMaxBoxBlocks) + sort_workspace_bytes(n, n) + 256;
 }
+
+namespace {
+struct MortonWs {
+    uint32_t *codes[2], *order[2];
+    float* parts;             // partial boxes
+    void* sort_ws;
+};
+MortonWs carve_morton_ws(void* workspace, int64_t n) {
+    Carver c(workspace);
+    MortonWs w;
+    for (int k = 0; k < 2; ++k) w.codes[k] = c.take<uint32_t>(n);
+    for (int k = 0; k < 2; ++k) w.order[k] = c.take<uint32_t>(n);
+    w.parts = c.take<float>(6 * kMaxBoxBlocks);
+    c.off = align_up(c.off);
+    w.sort_ws = c.base + c.off;
+    return w;
+}
+
+// Codes inside the box `mb` (or the one its parts make up), their sort, and the positions in that order.
+int order_along_curve(const char* who, const float* positions, int64_t n, const MortonBox& mb, const MortonWs& w, float* out, cudaStream_t stream) {
+    constexpr int kCodeBits = 30;
+    INPC_CUDA_TRY(cudaMemsetAsync(w.sort_ws, 0, sort_zero_bytes(n, n, kCodeBits), stream));
+    const int64_t code_blocks = ceil_div<int64_t>(n, 4 * kCodeThreads), code_cap = (int64_t)sm_count() * 4;
+    launch_chained(morton_codes_kernel, (unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kCodeThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0,
+                   mb, key_histogram(w.sort_ws, n, n, kCodeBits), w.codes[0], w.order[0]);
+    INPC_LAUNCH_CHECK("morton_codes_kernel");
+    int in_alt = 0;
+    {
+        const int rc_prev = check_previous_calls();
+        if (rc_prev != INPC_OK) return rc_prev;
+    }
+    unsigned* status = acquire_status(who);
+    if (!status) return INPC_E_CUDA;
+    const int rc = sort_pairs(w.codes[0], w.codes[1], w.order[0], w.order[1], n, n, kCodeBits, w.sort_ws, true, status, &in_alt, stream, true, true);
+    if (rc != INPC_OK) return rc;
+    launch_chained(gather_positions_kernel, (unsigned)ceil_div<int64_t>(n, 4 * kThreads), kThreads, 0, stream, positions, w.order[in_alt], n, (reinterpret_cast<uintptr_t>(out) & 15u) == 0, out);
+    INPC_LAUNCH_CHECK("gather_positions_kernel");
+    return INPC_OK;
+}
+}  // namespace
 
 extern "C" int inpc_morton_order(const float* positions, int64_t n, const float* box_lo, float box_extent, float* out, void* workspace,
                                  void* stream_) {
@@ -1354,36 +1477,33 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
         set_error("inpc_morton_order: bad argument");
         return INPC_E_INVALID;
     }
-    Carver c(workspace);
-    uint32_t* codes[2] = {c.take<uint32_t>(n), c.take<uint32_t>(n)};
-    uint32_t* order[2] = {c.take<uint32_t>(n), c.take<uint32_t>(n)};
-    float* parts = c.take<float>(6 * kMaxBoxBlocks);
-    c.off = align_up(c.off);
-    void* sort_ws = c.base + c.off;
-    MortonBox mb{{0.0f, 0.0f, 0.0f}, 1.0f, parts, 0};
+    const MortonWs w = carve_morton_ws(workspace, n);
+    MortonBox mb{{0.0f, 0.0f, 0.0f}, 1.0f, w.parts, nullptr, 0};
     if (box_lo) {
         for (int k = 0; k < 3; ++k) mb.lo[k] = box_lo[k];
         mb.inv_extent = 1.0f / box_extent;
     } else {
         const int64_t blocks = ceil_div<int64_t>(n, 4 * kThreads), cap = 4 * sm_count() < kMaxBoxBlocks ? 4 * sm_count() : kMaxBoxBlocks;
         mb.box_parts = (int)(blocks < cap ? blocks : cap);
-        launch_chained(bounding_box_kernel, mb.box_parts, kThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, parts);
+        launch_chained(bounding_box_kernel, mb.box_parts, kThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, w.parts);
         INPC_LAUNCH_CHECK("bounding_box_kernel");
     }
-    const bool vec_ok = (reinterpret_cast<uintptr_t>(positions) & 15u) == 0;
-    const int64_t code_blocks = ceil_div<int64_t>(n, 4 * kThreads), code_cap = (int64_t)sm_count() * 8;
-    launch_chained(morton_codes_kernel, (unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kThreads, 0, stream, positions, n, vec_ok, mb, codes[0], order[0]);
-    INPC_LAUNCH_CHECK("morton_codes_kernel");
-    int in_alt = 0;
-    {
-        const int rc_prev = check_previous_calls();
-        if (rc_prev != INPC_OK) return rc_prev;
+    return order_along_curve("inpc_morton_order", positions, n, mb, w, out, stream);
+}
+
+extern "C" int inpc_halton_morton_order(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size, int64_t n_total,
+                                        float* positions, float* out, void* sampler_workspace, void* morton_workspace, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (n_total == 0) return INPC_OK;
+    if (n_total < 0 || n_total >= ((int64_t)1 << 30) || !out || !morton_workspace || out == positions) {
+        set_error("inpc_halton_morton_order: bad argument");
+        return INPC_E_INVALID;
     }
-    unsigned* status = acquire_status("inpc_morton_order");
-    if (!status) return INPC_E_CUDA;
-    const int rc = sort_pairs(codes[0], codes[1], order[0], order[1], n, n, 30, sort_ws, false, status, &in_alt, stream, true);
+    const MortonWs w = carve_morton_ws(morton_workspace, n_total);
+    static_assert(kBoxCopies <= kMaxBoxBlocks, "the words of the box lie where the partial boxes would");
+    unsigned* words = reinterpret_cast<unsigned*>(w.parts);
+    INPC_CUDA_TRY(cudaMemsetAsync(words, 0, sizeof(unsigned) * 6 * kBoxCopies, stream));
+    const int rc = launch_halton("inpc_halton_morton_order", counts, n_cells, centers, levels, initial_size, n_total, positions, sampler_workspace, words, stream);
     if (rc != INPC_OK) return rc;
-    launch_chained(gather_positions_kernel, (unsigned)ceil_div<int64_t>(n, 4 * kThreads), kThreads, 0, stream, positions, order[in_alt], n, (reinterpret_cast<uintptr_t>(out) & 15u) == 0, out);
-    INPC_LAUNCH_CHECK("gather_positions_kernel");
-    return INPC_OK;
+    return order_along_curve("inpc_halton_morton_order", positions, n_total, MortonBox{{0.0f, 0.0f, 0.0f}, 1.0f, nullptr, words, kBoxCopies}, w, out, stream);
 }

@@ -241,8 +241,18 @@ def extract_global(sampler: "ProbabilityFieldSampler", centers: torch.Tensor, le
     else:
         global_weights = weights * torch.exp2(-levels * 0.5)             # ProbabilityField.get_current_weights(None)
     counts = sampler.draw_leaf_counts(global_weights, n_samples)
-    positions = _halton_samples(counts, centers, levels, initial_size, int(n_samples))   # every draw lands in a leaf
-    return morton_order(positions) if use_morton_order else positions
+    total = int(n_samples)   # every draw lands in a leaf
+    if not use_morton_order or total == 0:
+        return _halton_samples(counts, centers, levels, initial_size, total)
+    lib, dev = _cabi.lib(), centers.device
+    with _on(dev):
+        # the placement collects the cloud's bounding box on the way, which spares the Morton order a pass over the positions
+        positions, out = (torch.empty((total, 3), dtype=torch.float32, device=dev) for _ in range(2))
+        ws, ws_morton = (torch.empty(int(size), dtype=torch.uint8, device=dev)
+                         for size in (lib.inpc_sampler_workspace_bytes(n), lib.inpc_morton_workspace_bytes(total)))
+        _cabi.check(lib.inpc_halton_morton_order(_ptr(counts), n, _ptr(centers), _ptr(levels), float(initial_size), total,
+                                                 _ptr(positions), _ptr(out), _ptr(ws), _ptr(ws_morton), _stream()))
+    return out
 
 
 def build_cdf(weights: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:

@@ -1,4 +1,5 @@
-"""GPU tests of kernels that count the digits of the keys they make for the sort behind them, at the edges of their blocks, bit for bit against the oracle."""
+"""GPU tests of kernels that count the digits of the keys they make for the sort behind them, and of the cloud whose bounding box is collected while it is
+placed: at the edges of their blocks, bit for bit against the forms that do neither."""
 import numpy as np
 import pytest
 import torch
@@ -33,3 +34,24 @@ def test_lists_of_points_counted_while_their_instances_are_emitted(tile, width, 
     assert int(state.n_visible) == len(st.sorted_points) and int(state.n_instances) == len(st.inst_point)
     assert np.array_equal(dbg["inst_point"].cpu().numpy().view(np.uint32), st.inst_point)
     assert np.array_equal(dbg["ranges"].cpu().numpy().view(np.uint32), st.ranges)
+
+
+@pytest.mark.parametrize("total", [1, 2, 31, 2047, 4097, 300_001])
+@pytest.mark.parametrize("odd", [None, "negative", "zero", "nan", "infinite"])
+def test_cloud_placed_with_its_box_is_the_cloud_ordered_afterwards(total, odd):
+    from inpc_b200 import sampling as S
+    g = torch.Generator().manual_seed(total)
+    leaves = 700
+    centers = torch.rand((leaves, 3), generator=g) * 2 - 1
+    levels = torch.randint(2, 9, (leaves,), generator=g, dtype=torch.int32)
+    weights = torch.rand(leaves, generator=g)
+    if odd == "negative":
+        centers = centers - 5.0
+    elif odd == "zero":
+        centers[:, 1] = -0.0
+    elif odd is not None:
+        centers[leaves // 2, 2] = float("nan") if odd == "nan" else float("inf")
+    c, l, w = centers.to(DEV), levels.to(DEV), weights.to(DEV)
+    cloud = S.extract_global(S.ProbabilityFieldSampler(3), c, l, w, [], total, 2.0)
+    plain = S.extract_global(S.ProbabilityFieldSampler(3), c, l, w, [], total, 2.0, use_morton_order=False)
+    assert torch.equal(cloud.view(torch.int32), S.morton_order(plain).view(torch.int32))
