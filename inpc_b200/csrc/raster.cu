@@ -4078,7 +4078,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         if (rc_check != INPC_OK) return rc_check;
     }
 
-    // Bilinear splats touch at most 2x2 tiles, so the warp-blend path sizes everything behind the visibility pass
+    // Bilinear splats touch at most 2x2 tiles, so the warp-blend path sizes everything behind the projection
     // for 4 n instances and lets the kernels read the two counts from device memory: no host synchronisation at
     // all (the reference reads both counts back with blocking copies, src/bilinear/forward.cu:86-89).  The other
     // paths (gaussian splats have no such bound, feature rows keep their scratch small) read the counts back once.
