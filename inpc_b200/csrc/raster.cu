@@ -2580,6 +2580,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_r
                     const float4 f = row[c];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
+                        // 32 channels: not for pixels outside the half or stopped (2^24 points at 3840x2160 1441 -> 1408 us; of 16 channels 824 -> 840)
+                        if (C4 == 8 && !((pixels >> pix[q]) & 1u)) continue;
                         const float4 v = sm.pixel_grad[pix[q] * kStride + c];
                         G[q] += f.x * v.x + f.y * v.y + f.z * v.z + f.w * v.w;
                     }
