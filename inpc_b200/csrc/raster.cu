@@ -1439,6 +1439,10 @@ __device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_i
 __device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f, (float)(len + 8u) * 1.1920928955078125e-07f); }
 
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
+// Resident blocks per multiprocessor of the passes: their launch bounds, and their persistent grids.
+__host__ __device__ constexpr int forward_blocks(int pass, int c4) { return pass == PASS_PRODUCT ? 4 : c4 == 8 ? 2 : 3; }
+__host__ __device__ constexpr int rows_backward_blocks(int c4) { return c4 == 8 ? 2 : 3; }
+constexpr int kBackwardBlocks = 3, kGaussForwardBlocks = 3, kGaussBackwardBlocks = 2;
 constexpr float kLogScale = 67108864.0f;   // 2^26, see the product of pass PRODUCT
 constexpr float kLogNaN = 1048576.0f;      // far above what 32 factors add up to
 
@@ -1784,7 +1788,7 @@ constexpr size_t warp_forward_smem_bytes() {
 
 // ROWS: features are rows of 4 C4 channels in `rows` (a (4 C4, H, W) image); otherwise C4 is 1 and they are in the record.
 template <int PASS, int KIND, int C4, bool ROWS>
-__global__ void __launch_bounds__(kWarpBlendWarps * 32, PASS == PASS_PRODUCT ? 4 : C4 == 8 ? 2 : 3) blend_bilinear_warp_forward_kernel(
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)) blend_bilinear_warp_forward_kernel(
     const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, const uint32_t* __restrict__ inst_keys,
     const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ rows, float* __restrict__ seg_T, float4* __restrict__ seg_C,
     float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
@@ -2301,7 +2305,7 @@ struct __align__(16) WarpBackwardSmem {
 };
 constexpr size_t kWarpBackwardSmemBytes = kWarpBlendWarps * sizeof(WarpBackwardSmem);
 
-__global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_bilinear_warp_backward_kernel(
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_bilinear_warp_backward_kernel(
     const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
     unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0,
     const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept, const PointRec* __restrict__ rec,
@@ -2470,7 +2474,7 @@ template <int C4>
 constexpr size_t rows_warp_backward_smem_bytes() { return kWarpBlendWarps * sizeof(RowsBackwardSmem<C4>); }
 
 template <int C4>
-__global__ void __launch_bounds__(kWarpBlendWarps * 32, C4 == 8 ? 2 : 3) blend_rows_warp_backward_kernel(
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)) blend_rows_warp_backward_kernel(
     const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
     unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0,
     const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept, const PointRec* __restrict__ rec, const float4* __restrict__ rows,
@@ -3372,7 +3376,7 @@ constexpr size_t gauss_forward_smem_bytes() {
 }
 
 template <int PASS, int KIND>
-__global__ void __launch_bounds__(kWarpBlendWarps * 32, 3) blend_gaussian_warp_forward_kernel(
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) blend_gaussian_warp_forward_kernel(
     const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, const uint32_t* __restrict__ inst_keys,
     const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T,
     float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
@@ -3587,7 +3591,7 @@ struct __align__(16) GaussBackwardSmem {
 };
 constexpr size_t kGaussBackwardSmemBytes = kWarpBlendWarps * sizeof(GaussBackwardSmem);
 
-__global__ void __launch_bounds__(kWarpBlendWarps * 32, 2) blend_gaussian_warp_backward_kernel(
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussBackwardBlocks) blend_gaussian_warp_backward_kernel(
     const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
     unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0, const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept,
     const PointRec* __restrict__ rec, const float4* __restrict__ conic, const float* __restrict__ seg_T, const float4* __restrict__ seg_C,
@@ -4285,11 +4289,10 @@ template <> struct BlendConfig<16> { static constexpr int kIpt = 1; };
 
 int blend_batch(int tile) { return tile * tile * BlendConfig<16>::kIpt; }
 
-// Persistent grid of the warp blend: enough blocks to fill the GPU (the item counts live on the device).
-int warp_blend_grid(unsigned* grid) {
-    *grid = (unsigned)max(1, sm_count() * 4);
-    return INPC_OK;
-}
+// Blocks of a persistent pass (the item counts live on the device): those that fit the chip, as the launch bounds of its kernel have it.  With four per multiprocessor for all passes the last
+// quarter of the blocks of most found nothing left, and a warp's share of the items (see ItemQueue) was counted too small: step of 2^24 points crowding a corner of 3840x2160
+// 2633 -> 2540 us (first pass 347 -> 297, backward 441 -> 392), of 2^23 samples at 1237x822 1623 -> 1608.
+unsigned warp_blend_grid(int blocks_per_sm) { return (unsigned)(sm_count() * blocks_per_sm); }
 
 struct ForwardPassArgs {
     const uint32_t *keys, *ids;
@@ -4304,13 +4307,13 @@ struct ForwardPassArgs {
 
 // One pass of the warp blend's forward: its shared memory (the per-warp rings) is above the 48 KB a kernel gets unasked.
 template <int PASS, int KIND, int C4, bool ROWS>
-int launch_warp_forward_pass(unsigned grid, const WarpItem* items, const uint32_t* counts, unsigned* ticket, const ForwardPassArgs& a,
+int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const ForwardPassArgs& a,
                              cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
     const int rc = opt_in_dynamic_smem(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, grid, kWarpBlendWarps * 32, smem, stream,
+    launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, warp_blend_grid(forward_blocks(PASS, C4)), kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, a.gh);
     INPC_LAUNCH_CHECK("blend_bilinear_warp_forward_kernel");
@@ -4321,9 +4324,7 @@ int launch_warp_forward_pass(unsigned grid, const WarpItem* items, const uint32_
 template <int KIND, int C4 = 1, bool ROWS = false>
 int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float4* rows, float* image,
                                  float* depth, float* alpha, float* blending_weights, cudaStream_t stream) {
-    unsigned grid = 1;
-    const int rc = warp_blend_grid(&grid);
-    if (rc != INPC_OK) return rc;
+    const unsigned grid = warp_blend_grid(4);   // of the two small kernels between the passes
     const int W = rp.v.width, H = rp.v.height;
     // the ping-pong buffers the tile sort left unused receive the compacted lists (part 0: ids, part 1: keys)
     const uint32_t* keys = ib.keys[t_alt];
@@ -4333,13 +4334,13 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{keys, ids, pb.rec, rows, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             kept0, kept1, ib.n_kept, W, H, rp.gw, rp.gh};
-    int rc_pass = launch_warp_forward_pass<PASS_FIRST, KIND, C4, ROWS>(grid, ib.items0, ib.n_segments, ib.n_segments + 2, a, stream);
+    int rc_pass = launch_warp_forward_pass<PASS_FIRST, KIND, C4, ROWS>(ib.items0, ib.n_segments, ib.n_segments + 2, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
+    rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
-    rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
+    rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     launch_chained(warp_blend_combine_kernel<KIND, C4>, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E,
                                                                       image, depth, alpha, W, H, rp.gw, rp.gh);
@@ -4350,9 +4351,7 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
-    unsigned grid = 1;
-    const int rc = warp_blend_grid(&grid);
-    if (rc != INPC_OK) return rc;
+    const unsigned grid = warp_blend_grid(kBackwardBlocks);
     static bool attr_set[kMaxDevices] = {false};
     const int rc_attr = opt_in_dynamic_smem(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, attr_set);
     if (rc_attr != INPC_OK) return rc_attr;
@@ -4402,13 +4401,13 @@ int launch_bilinear_backward(const RasterParams& rp, const PointBlob& pb, const 
 }
 
 template <int PASS, int KIND>
-int launch_gaussian_warp_forward_pass(unsigned grid, const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic,
+int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic,
                                       const ForwardPassArgs& a, float threshold, float reach, cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
     const int rc = opt_in_dynamic_smem(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid, kWarpBlendWarps * 32, smem, stream,
+    launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, warp_blend_grid(kGaussForwardBlocks), kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, threshold, reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_forward_kernel");
@@ -4418,20 +4417,19 @@ int launch_gaussian_warp_forward_pass(unsigned grid, const WarpItem* items, cons
 template <int KIND>
 int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image, float* depth,
                                  float* alpha, float* blending_weights, float threshold, cudaStream_t stream) {
-    unsigned grid = 1;
-    int rc = warp_blend_grid(&grid);
-    if (rc != INPC_OK) return rc;
+    const unsigned grid = warp_blend_grid(4);   // of the two small kernels between the passes
+    int rc;
     const int W = rp.v.width, H = rp.v.height;
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{ib.keys[t_alt], ib.ids[t_alt], pb.rec, nullptr, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, W, H, rp.gw, rp.gh};
-    rc = launch_gaussian_warp_forward_pass<PASS_FIRST, KIND>(grid, ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, threshold, rp.reach, stream);
+    rc = launch_gaussian_warp_forward_pass<PASS_FIRST, KIND>(ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
+    rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
     launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
-    rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(grid, ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
+    rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
     launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
                                                                      rp.gw, rp.gh);
@@ -4442,9 +4440,7 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* gfv, float* grad_opacities,
                                   cudaStream_t stream) {
-    unsigned grid = 1;
-    const int rc = warp_blend_grid(&grid);
-    if (rc != INPC_OK) return rc;
+    const unsigned grid = warp_blend_grid(kGaussBackwardBlocks);
     static bool attr_set[kMaxDevices] = {false};
     const int rc_attr = opt_in_dynamic_smem(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, attr_set);
     if (rc_attr != INPC_OK) return rc_attr;
@@ -4521,9 +4517,7 @@ template <int C4>
 int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* features,
                               const float* grad_image, const float* grad_alpha, const float* image, const float* alpha,
                               float* grad_features, float* grad_opacities, cudaStream_t stream) {
-    unsigned grid = 1;
-    const int rc = warp_blend_grid(&grid);
-    if (rc != INPC_OK) return rc;
+    const unsigned grid = warp_blend_grid(rows_backward_blocks(C4));
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
     const int rc_attr = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
