@@ -1616,11 +1616,17 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
 // ... unless there are very many of them: a single counter hands out one ticket every 2.7 ns at best (measured:
 // 259,200 items of a 3840x2160 image took 700 us whatever the occupancy), so with many small items a warp takes
 // several consecutive ones per visit, behind the first n_single, which are long.
+// How many visits a warp is left with is measured, with 8 / 4 / 2 of them (8 / 16 / 32 items per visit at most):
+// bilinear, 3840x2160, points crowding one part of the image: first pass 295 / 255 / 259 us, backward 391 / 373 / 415;
+// the same at 2560x1440, first pass 91 / 75 / 89, backward 98 / 100 / 127.  Gaussian splats, 1920x1080: first pass
+// 238 / 248 / 271, so these keep 8.  Rows: step 1827 / 1829 / 1834, no gain, 8 as before.
+constexpr unsigned kVisits = 8, kVisitsShort = 4;
 struct ItemQueue {
     unsigned n_items, n_single, per_visit;
     unsigned next = 0, end = 0;
-    __device__ __forceinline__ ItemQueue(unsigned n_items_, unsigned n_single_, unsigned n_warps)
-        : n_items(n_items_), n_single(min(n_single_, n_items_)), per_visit(max(1u, min(8u, (n_items_ - min(n_single_, n_items_)) / (n_warps * 8u)))) {}
+    // `visits` of a warp at least, as far as there are items; 64 / visits items per visit at most
+    __device__ __forceinline__ ItemQueue(unsigned n_items_, unsigned n_single_, unsigned n_warps, unsigned visits)
+        : n_items(n_items_), n_single(min(n_single_, n_items_)), per_visit(max(1u, min(64u / visits, (n_items_ - min(n_single_, n_items_)) / (n_warps * visits)))) {}
     __device__ __forceinline__ bool take(unsigned* ticket, unsigned lane, unsigned* item) {
         if (next == end) {
             unsigned visit = 0;
@@ -1818,7 +1824,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
     if (PASS == PASS_PRODUCT) { sm.sum[0][lane] = 0u; sm.sum[1][lane] = 0u; }   // every batch leaves the sums at zero again
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
-    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps);
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps, ROWS ? kVisits : kVisitsShort);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(items + (item >> 1));
@@ -2325,7 +2331,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
     const unsigned n_rest = n_items - n_first;
 
     // the later segments first (they belong to the longest lists)
-    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps);
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps, kVisitsShort);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
@@ -2495,7 +2501,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
     const unsigned n_rest = n_items - n_first;
     const int64_t n_px = (int64_t)width * height;
 
-    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps);
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps, kVisits);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
@@ -3401,7 +3407,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
     }
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
-    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps);
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps, kVisits);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(items + (item >> 1));
@@ -3607,7 +3613,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussBackwardBlocks) bl
     const unsigned n_first = __ldg(counts) * 2u;
     const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
     const unsigned n_rest = n_items - n_first;
-    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps);
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps, kVisits);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
