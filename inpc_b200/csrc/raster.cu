@@ -1616,17 +1616,21 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
 // ... unless there are very many of them: a single counter hands out one ticket every 2.7 ns at best (measured:
 // 259,200 items of a 3840x2160 image took 700 us whatever the occupancy), so with many small items a warp takes
 // several consecutive ones per visit, behind the first n_single, which are long.
-// How many visits a warp is left with is measured, with 8 / 4 / 2 of them (8 / 16 / 32 items per visit at most):
+// How many items a visit takes is measured, with 8 / 4 / 2 visits per resident warp (8 / 16 / 32 items per visit at most):
 // bilinear, 3840x2160, points crowding one part of the image: first pass 295 / 255 / 259 us, backward 391 / 373 / 415;
 // the same at 2560x1440, first pass 91 / 75 / 89, backward 98 / 100 / 127.  Gaussian splats, 1920x1080: first pass
-// 238 / 248 / 271, so these keep 8.  Rows: step 1827 / 1829 / 1834, no gain, 8 as before.
-constexpr unsigned kVisits = 8, kVisitsShort = 4;
+// 238 / 248 / 271, rows: step 1827 / 1829 / 1834, so these keep 8 items at most, and 8 visits for each of 32 warps of a multiprocessor, resident or not:
+// with 8 for each resident one (24, 16, 8) the items come in larger shares and a pass ends later, step of rows of 32 / 16 channels, 2^24 points crowding
+// one part of 3840x2160, 4050 -> 4210 / 3028 -> 3113 us (first pass 675 -> 808 / 570 -> 587, backward 1400 -> 1447 / 813 -> 873), 2^23 gaussian splats evenly over
+// 3840x2160 3522 -> 3572.  Of later segments, which are long or find every pixel stopped, larger shares do no harm: 8 visits for each of 24 warps (2^20 opaque
+// gaussian splats of 8 pixels at 1920x1080, products and later segments 49 + 51 -> 27 + 29).
+constexpr unsigned kMostItems = 8, kMostItemsBilinear = 16;
 struct ItemQueue {
     unsigned n_items, n_single, per_visit;
     unsigned next = 0, end = 0;
-    // `visits` of a warp at least, as far as there are items; 64 / visits items per visit at most
-    __device__ __forceinline__ ItemQueue(unsigned n_items_, unsigned n_single_, unsigned n_warps, unsigned visits)
-        : n_items(n_items_), n_single(min(n_single_, n_items_)), per_visit(max(1u, min(64u / visits, (n_items_ - min(n_single_, n_items_)) / (n_warps * visits)))) {}
+    // `n_visits` at least, as far as there are items; `most` items per visit at most
+    __device__ __forceinline__ ItemQueue(unsigned n_items_, unsigned n_single_, unsigned n_visits, unsigned most)
+        : n_items(n_items_), n_single(min(n_single_, n_items_)), per_visit(max(1u, min(most, (n_items_ - n_single) / n_visits))) {}
     __device__ __forceinline__ bool take(unsigned* ticket, unsigned lane, unsigned* item) {
         if (next == end) {
             unsigned visit = 0;
@@ -1795,7 +1799,7 @@ constexpr size_t warp_forward_smem_bytes() {
 // ROWS: features are rows of 4 C4 channels in `rows` (a (4 C4, H, W) image); otherwise C4 is 1 and they are in the record.
 template <int PASS, int KIND, int C4, bool ROWS>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)) blend_bilinear_warp_forward_kernel(
-    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, const uint32_t* __restrict__ inst_keys,
+    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ inst_keys,
     const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ rows, float* __restrict__ seg_T, float4* __restrict__ seg_C,
     float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1,
@@ -1824,7 +1828,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
     if (PASS == PASS_PRODUCT) { sm.sum[0][lane] = 0u; sm.sum[1][lane] = 0u; }   // every batch leaves the sums at zero again
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
-    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps, ROWS ? kVisits : kVisitsShort);
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, n_visits, ROWS ? kMostItems : kMostItemsBilinear);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(items + (item >> 1));
@@ -2313,7 +2317,7 @@ constexpr size_t kWarpBackwardSmemBytes = kWarpBlendWarps * sizeof(WarpBackwardS
 
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_bilinear_warp_backward_kernel(
     const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
-    unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0,
+    unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ kept0,
     const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept, const PointRec* __restrict__ rec,
     const float* __restrict__ seg_T, const float4* __restrict__ seg_C, const float* __restrict__ grad_image,
     const float* __restrict__ grad_alpha, const float* __restrict__ image, const float* __restrict__ alpha_image,
@@ -2331,7 +2335,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
     const unsigned n_rest = n_items - n_first;
 
     // the later segments first (they belong to the longest lists)
-    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps, kVisitsShort);
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, n_visits, kMostItemsBilinear);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
@@ -2482,7 +2486,7 @@ constexpr size_t rows_warp_backward_smem_bytes() { return kWarpBlendWarps * size
 template <int C4>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)) blend_rows_warp_backward_kernel(
     const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
-    unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0,
+    unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ kept0,
     const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept, const PointRec* __restrict__ rec, const float4* __restrict__ rows,
     const float* __restrict__ seg_T, const float4* __restrict__ seg_C, const float* __restrict__ grad_image,
     const float* __restrict__ grad_alpha, const float* __restrict__ image, const float* __restrict__ alpha_image,
@@ -2501,7 +2505,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
     const unsigned n_rest = n_items - n_first;
     const int64_t n_px = (int64_t)width * height;
 
-    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps, kVisits);
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, n_visits, kMostItems);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
@@ -3383,7 +3387,7 @@ constexpr size_t gauss_forward_smem_bytes() {
 
 template <int PASS, int KIND>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) blend_gaussian_warp_forward_kernel(
-    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, const uint32_t* __restrict__ inst_keys,
+    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ inst_keys,
     const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T,
     float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
     float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
@@ -3407,7 +3411,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
     }
     __syncthreads();
     const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
-    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, gridDim.x * kWarpBlendWarps, kVisits);
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, n_visits, kMostItems);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(items + (item >> 1));
@@ -3599,7 +3603,7 @@ constexpr size_t kGaussBackwardSmemBytes = kWarpBlendWarps * sizeof(GaussBackwar
 
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussBackwardBlocks) blend_gaussian_warp_backward_kernel(
     const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
-    unsigned* __restrict__ ticket, const uint32_t* __restrict__ kept0, const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept,
+    unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ kept0, const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept,
     const PointRec* __restrict__ rec, const float4* __restrict__ conic, const float* __restrict__ seg_T, const float4* __restrict__ seg_C,
     const float* __restrict__ grad_image, const float* __restrict__ grad_alpha, const float* __restrict__ image,
     const float* __restrict__ alpha_image, float4* __restrict__ grad_feat_view, float* __restrict__ grad_opacity, int width, int height, int gw,
@@ -3613,7 +3617,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussBackwardBlocks) bl
     const unsigned n_first = __ldg(counts) * 2u;
     const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
     const unsigned n_rest = n_items - n_first;
-    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, gridDim.x * kWarpBlendWarps, kVisits);
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, n_visits, kMostItems);
     unsigned item;
     while (queue.take(ticket, lane, &item)) {
         const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
@@ -4298,7 +4302,15 @@ int blend_batch(int tile) { return tile * tile * BlendConfig<16>::kIpt; }
 // Blocks of a persistent pass (the item counts live on the device): those that fit the chip, as the launch bounds of its kernel have it.  With four per multiprocessor for all passes the last
 // quarter of the blocks of most found nothing left, and a warp's share of the items (see ItemQueue) was counted too small: step of 2^24 points crowding a corner of 3840x2160
 // 2633 -> 2540 us (first pass 347 -> 297, backward 441 -> 392), of 2^23 samples at 1237x822 1623 -> 1608.
-unsigned warp_blend_grid(int blocks_per_sm) { return (unsigned)(sm_count() * blocks_per_sm); }
+// `visits`: see ItemQueue; `pass`: of the forward passes (PASS_FIRST also for a backward pass).
+struct BlendGrid {
+    unsigned blocks, visits;
+};
+BlendGrid warp_blend_grid(int blocks_per_sm, bool bilinear, int pass) {
+    const unsigned blocks = (unsigned)(sm_count() * blocks_per_sm);
+    return {blocks, bilinear ? blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u};
+}
+unsigned small_grid() { return (unsigned)(sm_count() * 4); }   // of the two small kernels between the passes
 
 struct ForwardPassArgs {
     const uint32_t *keys, *ids;
@@ -4317,10 +4329,11 @@ int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsi
                              cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
+    const BlendGrid grid = warp_blend_grid(forward_blocks(PASS, C4), !ROWS, PASS);
     const int rc = opt_in_dynamic_smem(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, warp_blend_grid(forward_blocks(PASS, C4)), kWarpBlendWarps * 32, smem, stream,
-        items, counts, ticket, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
+    launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
+        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, a.gh);
     INPC_LAUNCH_CHECK("blend_bilinear_warp_forward_kernel");
     return INPC_OK;
@@ -4330,7 +4343,7 @@ int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsi
 template <int KIND, int C4 = 1, bool ROWS = false>
 int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float4* rows, float* image,
                                  float* depth, float* alpha, float* blending_weights, cudaStream_t stream) {
-    const unsigned grid = warp_blend_grid(4);   // of the two small kernels between the passes
+    const unsigned grid = small_grid();
     const int W = rp.v.width, H = rp.v.height;
     // the ping-pong buffers the tile sort left unused receive the compacted lists (part 0: ids, part 1: keys)
     const uint32_t* keys = ib.keys[t_alt];
@@ -4357,12 +4370,12 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
-    const unsigned grid = warp_blend_grid(kBackwardBlocks);
     static bool attr_set[kMaxDevices] = {false};
-    const int rc_attr = opt_in_dynamic_smem(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, attr_set);
-    if (rc_attr != INPC_OK) return rc_attr;
-    launch_chained(blend_bilinear_warp_backward_kernel, grid, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream,
-        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
+    const BlendGrid grid = warp_blend_grid(kBackwardBlocks, true, PASS_FIRST);
+    const int rc = opt_in_dynamic_smem(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, attr_set);
+    if (rc != INPC_OK) return rc;
+    launch_chained(blend_bilinear_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream,
+        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
         ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, rp.v.width, rp.v.height, rp.gw);
     INPC_LAUNCH_CHECK("blend_bilinear_warp_backward_kernel");
     return INPC_OK;
@@ -4411,10 +4424,11 @@ int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* cou
                                       const ForwardPassArgs& a, float threshold, float reach, cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
+    const BlendGrid grid = warp_blend_grid(kGaussForwardBlocks, false, PASS);
     const int rc = opt_in_dynamic_smem(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, attr_set);
     if (rc != INPC_OK) return rc;
-    launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, warp_blend_grid(kGaussForwardBlocks), kWarpBlendWarps * 32, smem, stream,
-        items, counts, ticket, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
+    launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
+        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, threshold, reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_forward_kernel");
     return INPC_OK;
@@ -4423,7 +4437,7 @@ int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* cou
 template <int KIND>
 int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image, float* depth,
                                  float* alpha, float* blending_weights, float threshold, cudaStream_t stream) {
-    const unsigned grid = warp_blend_grid(4);   // of the two small kernels between the passes
+    const unsigned grid = small_grid();
     int rc;
     const int W = rp.v.width, H = rp.v.height;
     const unsigned threads = kWarpBlendWarps * 32;
@@ -4446,12 +4460,12 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* gfv, float* grad_opacities,
                                   cudaStream_t stream) {
-    const unsigned grid = warp_blend_grid(kGaussBackwardBlocks);
     static bool attr_set[kMaxDevices] = {false};
-    const int rc_attr = opt_in_dynamic_smem(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, attr_set);
-    if (rc_attr != INPC_OK) return rc_attr;
-    launch_chained(blend_gaussian_warp_backward_kernel, grid, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream,
-        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
+    const BlendGrid grid = warp_blend_grid(kGaussBackwardBlocks, false, PASS_FIRST);
+    const int rc = opt_in_dynamic_smem(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, attr_set);
+    if (rc != INPC_OK) return rc;
+    launch_chained(blend_gaussian_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream,
+        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
         grad_image, grad_alpha, image, alpha, gfv, grad_opacities, rp.v.width, rp.v.height, rp.gw, rp.reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_backward_kernel");
     return INPC_OK;
@@ -4523,13 +4537,13 @@ template <int C4>
 int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* features,
                               const float* grad_image, const float* grad_alpha, const float* image, const float* alpha,
                               float* grad_features, float* grad_opacities, cudaStream_t stream) {
-    const unsigned grid = warp_blend_grid(rows_backward_blocks(C4));
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
-    const int rc_attr = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
-    if (rc_attr != INPC_OK) return rc_attr;
-    launch_chained(blend_rows_warp_backward_kernel<C4>, grid, kWarpBlendWarps * 32, smem, stream,
-        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
+    const BlendGrid grid = warp_blend_grid(rows_backward_blocks(C4), false, PASS_FIRST);
+    const int rc = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
+    if (rc != INPC_OK) return rc;
+    launch_chained(blend_rows_warp_backward_kernel<C4>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
+        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
         reinterpret_cast<const float4*>(features), ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha,
         reinterpret_cast<float4*>(grad_features), grad_opacities, rp.v.width, rp.v.height, rp.gw);
     INPC_LAUNCH_CHECK("blend_rows_warp_backward_kernel");
