@@ -174,6 +174,23 @@ int opt_in_dynamic_smem(Kernel kernel, size_t bytes, bool (&done)[kMaxDevices]) 
     return INPC_OK;
 }
 
+// Blocks of `threads` threads and `bytes` of dynamic shared memory that fit a multiprocessor together, by what the runtime knows of the
+// kernel's registers and shared memory (asked for once per kernel and device, with the opt-in above): the grid of a persistent kernel.
+template <typename Kernel>
+int resident_blocks(Kernel kernel, int threads, size_t bytes, int (&known)[kMaxDevices], int* blocks) {
+    static std::mutex table_mutex;
+    std::lock_guard<std::mutex> lock(table_mutex);
+    int dev = 0;
+    INPC_CUDA_TRY(cudaGetDevice(&dev));
+    const bool tracked = dev >= 0 && dev < kMaxDevices;
+    if (tracked && known[dev] > 0) { *blocks = known[dev]; return INPC_OK; }
+    INPC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    INPC_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, kernel, threads, bytes));
+    if (*blocks < 1) *blocks = 1;
+    if (tracked) known[dev] = *blocks;
+    return INPC_OK;
+}
+
 // ---- device helpers ------------------------------------------------------------------------
 #ifdef __CUDACC__
 // ---- launches that overlap the end of the kernel before them ------------------------------------------

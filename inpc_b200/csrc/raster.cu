@@ -1439,9 +1439,9 @@ __device__ __forceinline__ SegmentLengths segment_lengths(unsigned long long n_i
 __device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f, (float)(len + 8u) * 1.1920928955078125e-07f); }
 
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
-// Resident blocks per multiprocessor of the passes: their launch bounds, and their persistent grids.
+// Launch bounds of the passes: blocks per multiprocessor that the registers must leave room for.
 __host__ __device__ constexpr int forward_blocks(int pass, int c4) { return pass == PASS_PRODUCT ? 4 : c4 == 8 ? 2 : 3; }
-__host__ __device__ constexpr int rows_backward_blocks(int c4) { return c4 == 8 ? 2 : 3; }
+__host__ __device__ constexpr int rows_backward_blocks(int c4) { return c4 == 8 ? 1 : c4 == 4 ? 2 : 3; }   // 16 and 32 channels: as many as have shared memory
 constexpr int kBackwardBlocks = 3, kGaussForwardBlocks = 3, kGaussBackwardBlocks = 2;
 constexpr float kLogScale = 67108864.0f;   // 2^26, see the product of pass PRODUCT
 constexpr float kLogNaN = 1048576.0f;      // far above what 32 factors add up to
@@ -4299,16 +4299,21 @@ template <> struct BlendConfig<16> { static constexpr int kIpt = 1; };
 
 int blend_batch(int tile) { return tile * tile * BlendConfig<16>::kIpt; }
 
-// Blocks of a persistent pass (the item counts live on the device): those that fit the chip, as the launch bounds of its kernel have it.  With four per multiprocessor for all passes the last
-// quarter of the blocks of most found nothing left, and a warp's share of the items (see ItemQueue) was counted too small: step of 2^24 points crowding a corner of 3840x2160
-// 2633 -> 2540 us (first pass 347 -> 297, backward 441 -> 392), of 2^23 samples at 1237x822 1623 -> 1608.
+// Grid of a persistent pass (the item counts live on the device): the blocks that are resident, which registers limit for some kernels and shared memory for
+// others.  With four per multiprocessor for all passes, blocks that found nothing left came last, and a warp's share of the items (see ItemQueue) was
+// counted too small: step of 2^24 points crowding a corner of 3840x2160 2633 -> 2540 us (first pass 347 -> 297, backward 441 -> 392), of 2^23 samples
+// at 1237x822 1623 -> 1608.
 // `visits`: see ItemQueue; `pass`: of the forward passes (PASS_FIRST also for a backward pass).
 struct BlendGrid {
-    unsigned blocks, visits;
+    unsigned blocks = 1, visits = 1;
 };
-BlendGrid warp_blend_grid(int blocks_per_sm, bool bilinear, int pass) {
-    const unsigned blocks = (unsigned)(sm_count() * blocks_per_sm);
-    return {blocks, bilinear ? blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u};
+template <typename Kernel>
+int warp_blend_grid(Kernel kernel, size_t smem, bool bilinear, int pass, int (&known)[kMaxDevices], BlendGrid* grid) {
+    int blocks = 1;
+    const int rc = resident_blocks(kernel, kWarpBlendWarps * 32, smem, known, &blocks);
+    grid->blocks = (unsigned)(sm_count() * blocks);
+    grid->visits = bilinear ? grid->blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u;
+    return rc;
 }
 unsigned small_grid() { return (unsigned)(sm_count() * 4); }   // of the two small kernels between the passes
 
@@ -4327,10 +4332,10 @@ struct ForwardPassArgs {
 template <int PASS, int KIND, int C4, bool ROWS>
 int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const ForwardPassArgs& a,
                              cudaStream_t stream) {
-    static bool attr_set[kMaxDevices] = {false};
+    static int known[kMaxDevices] = {0};
     constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
-    const BlendGrid grid = warp_blend_grid(forward_blocks(PASS, C4), !ROWS, PASS);
-    const int rc = opt_in_dynamic_smem(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, attr_set);
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, !ROWS, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
@@ -4370,9 +4375,9 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
-    static bool attr_set[kMaxDevices] = {false};
-    const BlendGrid grid = warp_blend_grid(kBackwardBlocks, true, PASS_FIRST);
-    const int rc = opt_in_dynamic_smem(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, attr_set);
+    static int known[kMaxDevices] = {0};
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, true, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_bilinear_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
@@ -4422,10 +4427,10 @@ int launch_bilinear_backward(const RasterParams& rp, const PointBlob& pb, const 
 template <int PASS, int KIND>
 int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic,
                                       const ForwardPassArgs& a, float threshold, float reach, cudaStream_t stream) {
-    static bool attr_set[kMaxDevices] = {false};
+    static int known[kMaxDevices] = {0};
     constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
-    const BlendGrid grid = warp_blend_grid(kGaussForwardBlocks, false, PASS);
-    const int rc = opt_in_dynamic_smem(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, attr_set);
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, false, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
@@ -4460,9 +4465,9 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* gfv, float* grad_opacities,
                                   cudaStream_t stream) {
-    static bool attr_set[kMaxDevices] = {false};
-    const BlendGrid grid = warp_blend_grid(kGaussBackwardBlocks, false, PASS_FIRST);
-    const int rc = opt_in_dynamic_smem(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, attr_set);
+    static int known[kMaxDevices] = {0};
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, false, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
@@ -4537,10 +4542,10 @@ template <int C4>
 int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* features,
                               const float* grad_image, const float* grad_alpha, const float* image, const float* alpha,
                               float* grad_features, float* grad_opacities, cudaStream_t stream) {
-    static bool attr_set[kMaxDevices] = {false};
+    static int known[kMaxDevices] = {0};
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
-    const BlendGrid grid = warp_blend_grid(rows_backward_blocks(C4), false, PASS_FIRST);
-    const int rc = opt_in_dynamic_smem(blend_rows_warp_backward_kernel<C4>, smem, attr_set);
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_rows_warp_backward_kernel<C4>, smem, false, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_rows_warp_backward_kernel<C4>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,

@@ -37,3 +37,44 @@ def test_tiles_of_every_class_of_length(width, height, mode):
     for a, b in zip(*out):
         # products of up to 3000 factors in another grouping: 3000 * 2^-24, times the size of the sums they stand in
         assert float((a - b).norm()) <= 1e-4 * float(b.norm())
+
+
+# The blocks of a pass that stay for the whole of it are those that fit the chip, by the registers and shared memory of the kernel: of 2048 threads, 65536 registers (a
+# warp takes them in units of 256) and 228 KB of shared memory (units of 128 bytes, 1 KB of every block for the system) per multiprocessor
+def test_blend_passes_launch_the_blocks_that_are_resident(tmp_path):
+    import json
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    from torch.profiler import ProfilerActivity, profile
+    n, side = 3000, 64
+    g = torch.Generator().manual_seed(0)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), side, side, float(side), float(side)).to(DEV)
+    pos, opac = (torch.rand((n, 3), generator=g) - 0.5).to(DEV), (torch.rand((n, 1), generator=g) * 0.3).to(DEV)
+    rast = inpc_b200.INPCRasterizer()
+
+    def passes():
+        for mode in (0, 1):
+            f, o = torch.zeros((n, 36), dtype=torch.float16, device=DEV).requires_grad_(True), opac.clone().requires_grad_(True)
+            image, alpha, _ = rast(view, mode, pos, f, o)
+            (image.sum() + alpha.sum()).backward()
+            rast.render_preextracted(view, mode, pos, f.detach(), opac)
+        for channels in (4, 8, 16, 32):
+            f, o = torch.zeros((n, channels), device=DEV).requires_grad_(True), opac.clone().requires_grad_(True)
+            image, alpha, _ = rast.forward_rows(view, pos, f, o)
+            (image.sum() + alpha.sum()).backward()
+
+    passes()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        passes()
+        torch.cuda.synchronize()
+    p.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    seen = {e["name"].split("(")[-2 if "anonymous" in e["name"] else 0] + str(e["args"].get("shared memory")): e["args"] for e in events
+            if "blend" in e.get("name", "") and ("warp_forward" in e["name"] or "warp_backward" in e["name"]) and "grid" in e.get("args", {})}
+    if not seen:
+        pytest.skip("no activity records of kernels here")
+    multiprocessors = torch.cuda.get_device_properties(0).multi_processor_count
+    for name, a in seen.items():
+        threads, registers, shared = a["block"][0], a["registers per thread"], a["shared memory"]
+        fit = min(2048 // threads, 65536 // (-(-registers * 32 // 256) * 256 * threads // 32), 228 * 1024 // (-(-(shared + 1024) // 128) * 128))
+        assert a["grid"][0] == multiprocessors * fit, (name, a["grid"][0] / multiprocessors, fit)
