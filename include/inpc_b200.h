@@ -200,9 +200,10 @@ int inpc_render_rows(int tile_size, const inpc_view* view, int64_t n, const floa
                      float* alpha, inpc_alloc_fn alloc_point, inpc_alloc_fn alloc_instance, void* alloc_user,
                      void* stream);
 
-/* Fills in state->n_visible, n_instances and depth_key_base of a forward that deferred them: one small
- * device-to-host copy on `stream` and a synchronisation of that stream.  A no-op for states whose counts were
- * read back by the forward itself.  The values the reference returns from its blocking copies at
+/* Fills in state->n_visible and n_instances of a forward that deferred them (depth_key_base, known to the forward, becomes 0 if
+ * nothing is visible): one small device-to-host copy on `stream` and a synchronisation of that stream.  A no-op for states whose
+ * counts were read back by the forward itself.  INPC_E_DEVICE if the counts on the device contradict one another.
+ * The values the reference returns from its blocking copies at
  * rasterization/src/bilinear/forward.cu:86-89. */
 int inpc_raster_resolve(inpc_raster_state* state, void* stream);
 

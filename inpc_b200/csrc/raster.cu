@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
     __shared__ unsigned s_scan[kInstThreads / 4 / 32 + 1];
     if (!last_block(done, gridDim.x)) return;
     const unsigned total = scan_words<kInstThreads / 4>(block_sums, n_groups, s_scan);   // sums -> first instance of every block
-    if (threadIdx.x == 0 && n_instances) *n_instances = total;
+    if (threadIdx.x == 0 && n_instances) n_instances[0] = n_instances[1] = total;   // the second: see emit_quads_kernel
 }
 
 // Instance key: the tile index in the low 24 bits, the only bits the tile sort looks at (it carries the
@@ -648,13 +648,15 @@ __device__ __forceinline__ unsigned cell_code(int left, int right, int top, int 
 // gather.  Bound by these random gathers, one 32-byte sector each, and by instruction issue.  What is read or written once bypasses
 // the caches' replacement, so that more of the gathered array stays in L2.  A splat has one, two or four instances: the sums over a warp
 // come from three ballots, those over a block from one barrier and a warp reduction, and the keys are put together without a loop.  A block takes
-// groups of 1024 points one after the other and counts the digits of the keys it writes, which spares the tile sort its pass over them: emission and
+// groups of 1024 points one after the other and counts the digits of the keys it writes (and so the keys: *n_emitted, which inpc_raster_resolve compares with the
+// count made from the sorted keys; not where there is one tile, or nothing is visible), which spares the tile sort its pass over them: emission and
 // histogram of 2^20 / 2^23 / 2^24 / 2^25 points 21 / 104 / 207 / 496 -> 16 / 95 / 192 / 412 us (half of the last by fewer blocks).
 // (Four consecutive points per thread with their gathers in flight together and the instances staged in shared memory: the emission alone 116 us for
 // 2^23 points, 396 for 2^24, 952 for 2^25.)
 __global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
                                                                      const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
-                                                                     KeyHistogram digits, uint32_t* __restrict__ inst_keys, uint32_t* __restrict__ inst_ids) {
+                                                                     KeyHistogram digits, unsigned long long* __restrict__ n_emitted, uint32_t* __restrict__ inst_keys,
+                                                                     uint32_t* __restrict__ inst_ids) {
     await_previous_kernel();
     __shared__ unsigned s_total[2][kInstThreads / 32];   // of two groups in turn, so that one barrier does
     __shared__ BlockHistogram s_digits;
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint3
             if (two_columns) emit(off + 1u, tile + (unsigned)gw + 1u, id);
         }
     }
-    finish_histogram(s_digits, digits, (unsigned)min(n_groups, (int64_t)gridDim.x), nullptr);
+    finish_histogram(s_digits, digits, (unsigned)min(n_groups, (int64_t)gridDim.x), n_emitted);
 }
 
 // Other splats.  CELLS (gaussian, 8x8 tiles): the key also says which cells of the tile the ellipse can reach (see cell_code).  The keys are counted by the
@@ -3831,7 +3833,7 @@ struct PointBlob {
     uint4* foot;                          // gaussian, warp blend: tile bounds and ellipse per point (see pack_footprint)
     unsigned* block_visible;              // survivors per chunk of kPreThreads points
     unsigned* group_visible;              // per group of 4 chunks; scanned in place
-    unsigned long long* counters;   // visible, instances, smallest / largest depth bit pattern
+    unsigned long long* counters;   // visible, instances, smallest / largest depth bit pattern; deferred: visible, instances, instances emitted
     unsigned* depth_min;
     unsigned* depth_max;
     uint32_t* keys[2];
@@ -4229,7 +4231,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                 const int64_t emit_cap = (int64_t)sm_count() * 2;   // two blocks of 1024 threads fill a multiprocessor
                 const KeyHistogram digits = key_histogram(ib.sort_ws, n_instances, likely_instances(n_instances, deferred), tile_bits);
                 launch_chained(emit_quads_kernel, (unsigned)(ibk < emit_cap ? ibk : emit_cap), kInstThreads, 0, stream, sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums,
-                    rp.gw, digits, ib.keys[0], ib.ids[0]);
+                    rp.gw, digits, deferred && tile_bits > 0 ? pb.counters + 2 : nullptr, ib.keys[0], ib.ids[0]);
             } else {
                 launch_chained(warp_blend ? emit_instances_kernel<true> : emit_instances_kernel<false>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.foot, n_visible,
                     n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
@@ -4911,15 +4913,16 @@ extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
     if (!(state->deferred_counts & 1) || state->n_points == 0) return INPC_OK;
     if (!state->point_blob) { set_error("inpc_raster_resolve: state without a point blob"); return INPC_E_INVALID; }
     const PointBlob pb = carve_point_blob(state->point_blob, state->n_points, state->mode, state->tile_size);
-    unsigned long long host[2];
+    unsigned long long host[3];
     INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, sizeof(host), cudaMemcpyDeviceToHost, stream));
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
     state->n_visible = (int64_t)host[0];
     state->n_instances = (int64_t)host[1];
     if (state->n_visible == 0) state->depth_key_base = 0u;
-    if (state->n_visible > state->n_points || state->n_instances > 4 * state->n_visible) {
-        set_error("inconsistent counts from the visibility pass: %lld visible of %lld points, %lld instances", (long long)state->n_visible,
-                  (long long)state->n_points, (long long)state->n_instances);
+    // three counts made independently: by the depth sort's histogram, from the sorted keys, and of the instances written
+    if (state->n_visible < 0 || state->n_visible > state->n_points || state->n_instances < state->n_visible || state->n_instances > 4 * state->n_visible || host[2] != host[1]) {
+        set_error("inconsistent counts: %lld of %lld points in the depth sort, %lld instances by its keys, %lld emitted", (long long)state->n_visible,
+                  (long long)state->n_points, (long long)state->n_instances, (long long)host[2]);
         return INPC_E_DEVICE;
     }
     return INPC_OK;

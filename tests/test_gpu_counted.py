@@ -55,3 +55,31 @@ def test_cloud_placed_with_its_box_is_the_cloud_ordered_afterwards(total, odd):
     cloud = S.extract_global(S.ProbabilityFieldSampler(3), c, l, w, [], total, 2.0)
     plain = S.extract_global(S.ProbabilityFieldSampler(3), c, l, w, [], total, 2.0, use_morton_order=False)
     assert torch.equal(cloud.view(torch.int32), S.morton_order(plain).view(torch.int32))
+
+
+# The counts a forward leaves on the device are three, made independently (points in the depth sort, instances by its keys, instances
+# emitted): one that contradicts the others is an error.  Images of many tiles, and of one, whose instances the emission does not count.
+@pytest.mark.parametrize("width, height", [(40, 24), (8, 8)])
+@pytest.mark.parametrize("word, change", [(0, 10_000), (0, -(1 << 40)), (1, -1), (1, 1 << 20), (2, -1), (2, 1)])
+def test_counts_that_contradict_one_another(width, height, word, change):
+    from inpc_b200 import _cabi
+    from inpc_b200 import rasterization as R
+    from inpc_b200.views import look_at_view
+    n = 5000
+    g = torch.Generator().manual_seed(word)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, 40.0, 40.0).to(DEV)
+    pos, opac = (torch.rand((n, 3), generator=g) * 2 - 1).to(DEV), torch.full((n, 1), 0.01, device=DEV)
+    settings = R.INPCRasterizer.extract_settings(view, 0)
+    _, _, _, state, blobs, _ = R.forward_with_state(pos, torch.zeros((n, 36), dtype=torch.float16, device=DEV), opac, settings, 8)
+    want = (state.n_visible, state.n_instances)
+    words = blobs.point[:blobs.point.numel() // 8 * 8].view(torch.int64)
+    at = torch.nonzero((words[:-2] == want[0]) & (words[1:-1] == want[1]) & (words[2:] == want[1])).reshape(-1)
+    assert at.numel() == 1 and 0 < want[0] < n
+    R.resolve_counts(state)
+    assert (state.n_visible, state.n_instances) == want
+    words[at[0] + word] += change
+    with pytest.raises(_cabi.InpcError, match="inconsistent counts"):
+        R.resolve_counts(state)
+    words[at[0] + word] -= change
+    R.resolve_counts(state)
+    assert (state.n_visible, state.n_instances) == want
