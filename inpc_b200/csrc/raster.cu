@@ -4236,7 +4236,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                 launch_chained(warp_blend ? emit_instances_kernel<true> : emit_instances_kernel<false>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.foot, n_visible,
                     n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             }
-            INPC_LAUNCH_CHECK("emit_instances_kernel");
+            INPC_LAUNCH_CHECK(counted ? "emit_quads_kernel" : "emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
