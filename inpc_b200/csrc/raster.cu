@@ -2434,7 +2434,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
                 float so = 0.0f;
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    if (met[c] != 0.0f) {
+                    if (met[c] != 0.0f) {   // (a transmittance that is no number gives a gradient that is none, as in src/bilinear/kernels.cu:361-415)
                         const float rcp = 1.0f / fmaxf(1.0f - al[c], kOneMinusAlphaEps);
                         const float bw = met[c] * al[c];
                         so += (met[c] * G[c] + S[c] * rcp) * w[c];

@@ -147,6 +147,41 @@ def test_odd_opacities_in_lists_of_several_segments(n, odd, rows):
     assert bool(np.isnan(st.alpha).any()) == (odd == "nan")
 
 
+# A pixel whose colour is no number gives none to the opacities of all points it meets, before and behind the one at fault, and no feature gradient to
+# those behind; the others are as they were.
+@pytest.mark.parametrize("n", [1, 5, 40, 700, 4097])
+@pytest.mark.parametrize("rows, tile", [(0, 8), (0, 16), (4, 8), (16, 8), (8, 16)])
+def test_gradients_behind_an_opacity_that_is_no_number(n, rows, tile):
+    import inpc_b200
+    from helpers import assert_close, oracle_camera
+    view, pos, opac = _one_tile_scene(n, n)
+    opac = opac.clone()
+    opac[torch.argsort(3.0 - pos[:, 2])[n * 3 // 4]] = float("nan")
+    g = torch.Generator().manual_seed(n + 1)
+    gi, ga = torch.randn((rows or 4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
+    cam, v, rast = oracle_camera(view), view.to(DEV), inpc_b200.INPCRasterizer(tile_size=tile)
+    o = opac.to(DEV).requires_grad_(True)
+    if rows:
+        feats = torch.randn((n, rows), generator=g) * 0.5
+        f = feats.to(DEV).requires_grad_(True)
+        image, alpha, _ = rast.forward_rows(v, pos.to(DEV), f, o)
+        gf, go = O.rasterize_rows_backward(O.rasterize_rows_forward(cam, pos.numpy(), feats.numpy(), opac.numpy()), gi.numpy(), ga.numpy())
+    else:
+        feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
+        f = feats.to(DEV).requires_grad_(True)
+        image, alpha, _ = rast(v, 0, pos.to(DEV), f, o)
+        gf, go, _ = O.rasterize_backward(O.rasterize_forward(O.BILINEAR, cam, pos.numpy(), feats.numpy(), opac.numpy()), gi.numpy(), ga.numpy())
+    torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
+    assert np.isnan(go).any() and (n < 40 or not np.isnan(go).all())
+    for got, want, tol, what in ((f.grad, gf, dict(rtol=2e-4, atol=1e-9) if rows else dict(rtol=2e-3, atol=1.2e-7), "features"),
+                                 (o.grad, go, dict(rtol=1e-3, atol=2e-8), "opacities")):
+        got, want = got.float().cpu().numpy(), np.asarray(want, np.float32)
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want), err_msg=what)
+        ok = ~np.isnan(want)
+        eps = n / 16 * 2.0 ** -25      # see the test of the segment edges
+        assert_close(got[ok], want[ok], rtol=tol["rtol"] + eps, atol=tol["atol"] + 1e-3 * eps, what=what)
+
+
 # Where a pixel stops, its colour minus the running colour is zero to the bit, which 1 / (1 - alpha) would else multiply by up to 10^8:
 # also where the opaque splat lies in a later segment.
 @pytest.mark.parametrize("mode", [0, 1])
