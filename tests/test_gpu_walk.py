@@ -9,9 +9,15 @@ DEV = "cuda:0"
 SIDE = 24
 
 
+U = 2.0 ** -24      # largest relative error of a rounding to 32 bits
+
+
 def _exact(x, y, opacity, features, grad_image, grad_alpha):
-    """Gradients of opacities and features of splats at (x, y) (front to back) in 64 bits."""
+    """Gradients of opacities and features of splats at (x, y) (front to back) in 64 bits, and how far 32-bit arithmetic may be off, per
+    splat: every operation rounds by U of its result, and what a fragment meets or leaves behind carries the errors of the fragments before it."""
     go, gf = np.zeros(len(x)), np.zeros(features.shape)
+    go_bound, gf_bound = np.zeros(len(x)), np.zeros(features.shape)
+    channels = features.shape[1]
     for row in range(SIDE):
         for column in range(SIDE):
             w = np.clip(1 - np.abs(x - (column + 0.5)), 0, 1) * np.clip(1 - np.abs(y - (row + 0.5)), 0, 1)
@@ -22,14 +28,32 @@ def _exact(x, y, opacity, features, grad_image, grad_alpha):
             met = np.cumprod(np.concatenate([[1.0], 1 - al]))
             stop = np.nonzero(met[1:] < 1e-4)[0]
             m = int(stop[0]) + 1 if len(stop) else len(k)
-            k, al, T = k[:m], al[:m], met[:m]
+            k, al, T, end = k[:m], al[:m], met[:m], met[m]
             g = grad_image[:, row, column]
             G, bw = features[k] @ g, T * al
             behind = (bw * G).sum() - np.cumsum(bw * G)
-            K = 0.0 if len(stop) else grad_alpha[0, row, column] * met[m]
+            upstream = 0.0 if len(stop) else grad_alpha[0, row, column]
+            K = upstream * end
             go[k] += (T * G + (K - behind) / np.maximum(1 - al, 1e-8)) * w[k]
             gf[k] += bw[:, None] * g[None]
-    return go, gf
+            # alpha is off by 4 U of itself (weight: two differences, two products), a transmittance by that over one minus alpha, and by two
+            # roundings, of every fragment before
+            off_T = np.concatenate([[0.0], np.cumsum((4 * al / (1 - al) + 2) * U)])
+            G_abs = np.abs(features[k]) @ np.abs(g)
+            sum_abs = (bw * G_abs).sum()
+            off_behind = (bw * G_abs * (off_T[:m] + (channels + 6) * U)).sum() + 2 * (m + channels) * U * sum_abs   # two running sums of m terms
+            off_K = np.abs(upstream) * (end * off_T[m] + 2 * U)
+            go_bound[k] += w[k] * (T * G_abs * (off_T[:m] + (channels + 6) * U) +
+                                   (off_behind + off_K + np.abs(K - behind) * (6 + 4 * al / (1 - al)) * U) / (1 - al))
+            gf_bound[k] += bw[:, None] * np.abs(g)[None] * (off_T[:m, None] + 8 * U)
+    return go, gf, go_bound, gf_bound
+
+
+def _sh_basis(position, eye):
+    x, y, z = ((position - eye) / np.linalg.norm(position - eye, axis=1, keepdims=True)).T
+    return np.stack([np.full_like(x, 0.28209479177387814), -0.48860251190291987 * y, 0.48860251190291987 * z, -0.48860251190291987 * x, 1.0925484305920792 * x * y,
+                     -1.0925484305920792 * y * z, 0.94617469575755997 * z * z - 0.31539156525251999, -1.0925484305920792 * x * z,
+                     0.54627421529603959 * (x * x - y * y)], axis=1)
 
 
 @pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 8, 9, 31, 32, 33, 65])
@@ -61,10 +85,12 @@ def test_lists_of_one_footprint(n, opaque, site):
         gi_c = gi if rows != 16 else gi.repeat(4, 1, 1)
         torch.autograd.backward([image, alpha], [gi_c.to(DEV), ga.to(DEV)])
         seen = (f.detach() if rows else dbg["feat_view"]).double().cpu().numpy()
-        go, gf = _exact(x, y, opacity.double().numpy()[:, 0], seen, gi_c.double().numpy(), ga.double().numpy())
-        # sums of up to n terms of order one, rounded by 2^-24 each; what lies behind a fragment is divided by its 1 - alpha, at least
-        # 10^-3, times a transmittance of at least 10^-4 where the list does not end: sqrt(n) 2^-24 / (1 - alpha) of the largest gradient
-        bound = (8 + np.sqrt(n)) * 2.0 ** -24 * (1e3 if opaque else 1.0) * max(1.0, np.abs(gi_c.numpy()).max()) * (1 + rows)
-        np.testing.assert_allclose(o.grad.double().cpu().numpy()[:, 0], go, rtol=1e-4, atol=bound)
-        if rows:
-            np.testing.assert_allclose(f.grad.double().cpu().numpy(), gf, rtol=1e-5, atol=(8 + np.sqrt(n)) * 2.0 ** -24)
+        go, gf, go_bound, gf_bound = _exact(x, y, opacity.double().numpy()[:, 0], seen, gi_c.double().numpy(), ga.double().numpy())
+        off = np.abs(o.grad.double().cpu().numpy()[:, 0] - go)
+        assert (off <= go_bound).all(), (rows, (off / go_bound).max())
+        if not rows:   # through the basis, and to halves: 2^-11 of the value, or half a step of the smallest ones
+            basis = _sh_basis(pos.double().cpu().numpy(), np.array([0.0, 0.0, 3.0]))
+            gf, gf_bound = ((basis[:, :, None] * v[:, None, :]).reshape(n, 36) for v in (gf, gf_bound))
+            gf_bound = np.abs(gf_bound) + np.abs(gf) * 2.0 ** -11 + 2.0 ** -25 + 32 * U * np.abs(gf).max(axis=1, keepdims=True)
+        off = np.abs(f.grad.double().cpu().numpy() - gf)
+        assert (off <= gf_bound + 1e-30).all(), (rows, (off / (gf_bound + 1e-30)).max())
