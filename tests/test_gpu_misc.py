@@ -99,6 +99,30 @@ def test_probability_field_update_matches_reference_formula():
         stats.accumulate(idx.int().to(DEV), w.to(DEV))
 
 
+# The first samples of a block go through a table in shared memory, those of the rounds behind it, from 1.2 million samples on, do not
+@pytest.mark.parametrize("n", [1, 1023, 1025, 1_212_416, 1_212_417, 5_000_003])
+@pytest.mark.parametrize("n_leaves", [1, 3, 777, 300_007])
+def test_leaf_statistics_over_all_rounds(n, n_leaves):
+    from inpc_b200 import probability_field as PF
+    g = torch.Generator().manual_seed(n + n_leaves)
+    idx = (torch.rand(n, generator=g) ** 3 * n_leaves).to(torch.int64).clamp_(max=n_leaves - 1)     # many samples in the first leaves
+    w = torch.rand(n, generator=g) + 0.5
+    w[torch.rand(n, generator=g) < 0.1] = 0.0
+    none = torch.rand(n, generator=g) < 0.1
+    nowhere = torch.tensor([-1, -(1 << 63), n_leaves, n_leaves + (1 << 32), 1 << 32])[torch.randint(0, 5, (n,), generator=g)]
+    if n > 1000:
+        idx = torch.where(none, nowhere, idx)       # (an index modulo 2^32 names no leaf)
+        w[n // 2], w[n - 1] = float("inf"), float("nan")
+    valid = (idx >= 0) & (idx < n_leaves)
+    mx, mn = torch.zeros(n_leaves), torch.zeros(n_leaves)
+    clean = w.nan_to_num(nan=0.0, posinf=float("inf")).clamp(min=0.0)
+    mx.scatter_reduce_(0, idx[valid], clean[valid], reduce="amax", include_self=False)
+    mn.scatter_reduce_(0, idx[valid], clean[valid], reduce="amin", include_self=False)
+    stats = PF.LeafStatistics(n_leaves, DEV)
+    stats.accumulate(idx.to(DEV), w.to(DEV))
+    assert torch.equal(stats.max_sampled.cpu(), mx) and torch.equal(stats.min_sampled.cpu(), mn)
+
+
 # weights and gradients of up to 100 MiB keep their room in L2, of more take none
 @pytest.mark.parametrize("add", [False, True])
 @pytest.mark.parametrize("n", [(100 << 17) - 3, 100 << 17, (100 << 17) + 1, (100 << 17) + 5])
