@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
 
         // 1. stable rank within the warp's segment, per digit
         // Two 16-bit positions in a word: 64 registers do not hold keys, values and positions otherwise, and what they spilled
-        // (13 of them) went through the unit the pass is bound by.  10.6 M pairs of 14 bits 130.5 -> 126.5 us, 2^25 of 30 bits 594 -> 573.
+        // (13 of them; one is left in the passes of 7 and 8 bits over large tiles) went through the unit the pass is bound by.  10.6 M pairs of 14 bits 130.5 -> 126.5 us, 2^25 of 30 bits 594 -> 573.
         unsigned pos2[ITEMS / 2];
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {

@@ -5,14 +5,15 @@
 //   per point   : PointRec 32 B {screen x, screen y, opacity, depth | 4 view-space feature channels}
 //                 (one 32-byte sector per gather in the blend), tile bounds 8 B or, bilinear on 8x8 tiles, a packed
 //                 footprint of 4 B that they follow from, conic 16 B (gaussian)
-//   per visible : depth key + point id, ping-pong pair for the depth sort
+//                 depth key + point id, ping-pong pair for the depth sort: of the visible points side by side or, bilinear on 8x8
+//                 tiles, of every point where it lies, culled ones marked
 //   per instance: tile key + point id, ping-pong pair for the tile sort
 //   per tile    : [first, last+1) instance range
 //
 // The arithmetic follows the reference kernels expression by expression (cited per function, paths
 // below INPCCudaBackend/INPCCudaBackend/rasterization/ of the reference); the organisation of the
-// work does not: compaction is a deterministic two-pass scan instead of atomics, the sorts are the
-// library's own onesweep, and the bilinear blend walks per-pixel bit masks of the staged batch
+// work does not: culled points are left out by the first pass of the depth sort (bilinear on 8x8 tiles) or by a deterministic
+// two-pass scan instead of atomics, the sorts are the library's own onesweep, and the bilinear blend walks per-pixel bit masks of the staged batch
 // instead of testing every staged point against every pixel.
 #include "common.cuh"
 
@@ -420,12 +421,12 @@ __device__ __forceinline__ uint4 pack_footprint(const Projection& pr, float reac
     return make_uint4(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16), inset, 0u);
 }
 
-// Pass 2: project again (same arithmetic, same outcome), evaluate SH, write the point record and
-// bounds, and append (depth key, point id) at the slot given by the block offset plus the rank of
-// the point among the block's survivors — index order, hence reproducible.
+// Project (pass 2 of the compaction projects again: same arithmetic, same outcome), evaluate SH, write the point record and bounds, and the depth key.
 // src/bilinear/kernels.cu:11-84, :106-184; src/gaussian/kernels.cu:11-111, :113-217, :219-324.
-// COMPACT: see above; otherwise every point's key is written where the point lies, that of a culled one is kNoKey, and the depth sort leaves it out
-// (the base of the keys is known to the host then, and neither the counts nor the depth range nor the point ids are used).
+// COMPACT: key and point id of a visible point are appended at the slot given by the block offset plus the rank of the point
+// among the block's survivors: index order, hence reproducible.  Otherwise (bilinear on 8x8 tiles, counts left on the device) there was no pass 1: every point's key is
+// written where the point lies, that of a culled one is kNoKey, and the depth sort leaves it out (the base of the keys is known to the host then, and
+// neither the counts nor the depth range nor the point ids are used).
 template <int MODE, int VARIANT, bool COMPACT>
 __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     PointSets ps, RasterParams rp, const unsigned* __restrict__ block_visible, const unsigned* __restrict__ group_offset,
@@ -1626,6 +1627,10 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
 // one part of 3840x2160, 4050 -> 4210 / 3028 -> 3113 us (first pass 675 -> 808 / 570 -> 587, backward 1400 -> 1447 / 813 -> 873), 2^23 gaussian splats evenly over
 // 3840x2160 3522 -> 3572.  Of later segments, which are long or find every pixel stopped, larger shares do no harm: 8 visits for each of 24 warps (2^20 opaque
 // gaussian splats of 8 pixels at 1920x1080, products and later segments 49 + 51 -> 27 + 29).
+// The long ones go out one by one however many there are.  Evenly filled images of 3840x2160, where nearly all are long, one by one / the first four
+// of every warp one by one, the others 8 or 16 per visit / before there were classes, 6 per visit: training step of 2^25 bilinear splats 9955 / 10620 /
+// 10425 us (first pass 2733 / 2590 / 2488, backward 3658 / 4450 / 4100), 2^26 almost opaque ones 19300 / 21870 / 21460, 2^25 gaussian splats 13630 / 15940 /
+// 15960; inference, 2^22 splats of 3 pixels, faint 4648 / 4778 / 4760, opaque, where most of a list is behind stopped pixels, 2800 / 2856 / 2840.
 constexpr unsigned kMostItems = 8, kMostItemsBilinear = 16;
 struct ItemQueue {
     unsigned n_items, n_single, per_visit;
@@ -3940,7 +3945,8 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, bool deferred, in
     Carver c(p);
     const bool warp_blend = uses_warp_blend(tile);
     // [0] segments (block blend) or non-empty tiles (warp blend), [1] later segments (warp blend), [2..5] work tickets of
-    // the warp blend passes FIRST, PRODUCT, REST and of its backward pass.  Counters, tile ranges and the sort's state lie side
+    // the warp blend passes FIRST, PRODUCT, REST and of its backward pass, [6] blocks of warp_items_count_kernel that are done, [8..9] tiles of
+    // the longest class and of the two longer ones (kLongTiles).  Counters, tile ranges and the sort's state lie side
     // by side: they are cleared together.
     b.n_segments = c.take<uint32_t>(64);
     b.ranges = c.take<uint2>(n_tiles);

@@ -1002,8 +1002,8 @@ __global__ void __launch_bounds__(kCodeThreads) morton_codes_kernel(const float*
         count_key(s_digits, digits.pt, key);
         return key;
     };
-    // four points per thread: three 16-byte loads where the positions are aligned, one 16-byte store.  Bound by DRAM: 2^25 points
-    // 91 us (one point per thread, and the point numbers written for the sort, which now makes them itself: 131)
+    // four points per thread: three 16-byte loads where the positions are aligned, one 16-byte store (without counting, 2^25 points 91 us, bound by DRAM;
+    // one point per thread, and the point numbers written for the sort, which now makes them itself: 131; with the four shared-memory atomics per code 132)
     const int64_t stride = (int64_t)gridDim.x * kCodeThreads * 4;
     for (int64_t i = ((int64_t)blockIdx.x * kCodeThreads + threadIdx.x) * 4; i < n; i += stride) {
         if (vec_ok && i + 4 <= n) {

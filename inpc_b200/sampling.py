@@ -246,7 +246,7 @@ def extract_global(sampler: "ProbabilityFieldSampler", centers: torch.Tensor, le
         return _halton_samples(counts, centers, levels, initial_size, total)
     lib, dev = _cabi.lib(), centers.device
     with _on(dev):
-        # the placement collects the cloud's bounding box on the way, which spares the Morton order a pass over the positions
+        # the box of the cloud follows from the leaves, which spares the Morton order a pass over the positions
         positions, out = (torch.empty((total, 3), dtype=torch.float32, device=dev) for _ in range(2))
         ws, ws_morton = (torch.empty(int(size), dtype=torch.uint8, device=dev)
                          for size in (lib.inpc_sampler_workspace_bytes(n), lib.inpc_morton_workspace_bytes(total)))
