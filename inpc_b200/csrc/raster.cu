@@ -4308,7 +4308,8 @@ template <> struct BlendConfig<16> { static constexpr int kIpt = 1; };
 int blend_batch(int tile) { return tile * tile * BlendConfig<16>::kIpt; }
 
 // Grid of a persistent pass (the item counts live on the device): the blocks that are resident, which registers limit for some kernels and shared memory for
-// others.  With four per multiprocessor for all passes, blocks that found nothing left came last, and a warp's share of the items (see ItemQueue) was
+// others, and not more than the launch bounds ask for (in passes of gaussian splats over later segments, of 63 registers, four would fit: the products of a training
+// step of 2^22 samples take 206 to 217 us with three and 204 to 213 with four, but a frame of 2 * 10^6 splats, where they are short, 581 and 585).  With four per multiprocessor for all passes, blocks that found nothing left came last, and a warp's share of the items (see ItemQueue) was
 // counted too small: step of 2^24 points crowding a corner of 3840x2160 2633 -> 2540 us (first pass 347 -> 297, backward 441 -> 392), of 2^23 samples
 // at 1237x822 1623 -> 1608.
 // `visits`: see ItemQueue; `pass`: of the forward passes (PASS_FIRST also for a backward pass).
@@ -4316,10 +4317,10 @@ struct BlendGrid {
     unsigned blocks = 1, visits = 1;
 };
 template <typename Kernel>
-int warp_blend_grid(Kernel kernel, size_t smem, bool bilinear, int pass, int (&known)[kMaxDevices], BlendGrid* grid) {
+int warp_blend_grid(Kernel kernel, size_t smem, int most, bool bilinear, int pass, int (&known)[kMaxDevices], BlendGrid* grid) {
     int blocks = 1;
     const int rc = resident_blocks(kernel, kWarpBlendWarps * 32, smem, known, &blocks);
-    grid->blocks = (unsigned)(sm_count() * blocks);
+    grid->blocks = (unsigned)(sm_count() * min(blocks, most));
     grid->visits = bilinear ? grid->blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u;
     return rc;
 }
@@ -4343,7 +4344,7 @@ int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsi
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, !ROWS, PASS, known, &grid);
+    const int rc = warp_blend_grid(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, forward_blocks(PASS, C4), !ROWS, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
@@ -4385,7 +4386,7 @@ int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, c
                                   unsigned* slot_mask, cudaStream_t stream) {
     static int known[kMaxDevices] = {0};
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, true, PASS_FIRST, known, &grid);
+    const int rc = warp_blend_grid(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, kBackwardBlocks, true, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_bilinear_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
@@ -4438,7 +4439,7 @@ int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* cou
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, false, PASS, known, &grid);
+    const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, kGaussForwardBlocks, false, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
@@ -4475,7 +4476,7 @@ int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, c
                                   cudaStream_t stream) {
     static int known[kMaxDevices] = {0};
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, false, PASS_FIRST, known, &grid);
+    const int rc = warp_blend_grid(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, kGaussBackwardBlocks, false, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
@@ -4553,7 +4554,7 @@ int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_rows_warp_backward_kernel<C4>, smem, false, PASS_FIRST, known, &grid);
+    const int rc = warp_blend_grid(blend_rows_warp_backward_kernel<C4>, smem, rows_backward_blocks(C4), false, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_rows_warp_backward_kernel<C4>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,

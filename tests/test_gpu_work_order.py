@@ -39,7 +39,8 @@ def test_tiles_of_every_class_of_length(width, height, mode):
         assert float((a - b).norm()) <= 1e-4 * float(b.norm())
 
 
-# The blocks of a pass that stay for the whole of it are those that fit the chip, by the registers and shared memory of the kernel: of 2048 threads, 65536 registers (a
+# The blocks of a pass that stay for the whole of it are those that fit the chip (of gaussian forward passes three per multiprocessor at most), by the registers
+# and shared memory of the kernel: of 2048 threads, 65536 registers (a
 # warp takes them in units of 256) and 228 KB of shared memory (units of 128 bytes, 1 KB of every block for the system) per multiprocessor
 def test_blend_passes_launch_the_blocks_that_are_resident(tmp_path):
     import json
@@ -69,7 +70,7 @@ def test_blend_passes_launch_the_blocks_that_are_resident(tmp_path):
         torch.cuda.synchronize()
     p.export_chrome_trace(str(tmp_path / "trace.json"))
     events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
-    seen = {e["name"].split("(")[-2 if "anonymous" in e["name"] else 0] + str(e["args"].get("shared memory")): e["args"] for e in events
+    seen = {e["name"].split("blend_", 1)[1].split("(")[0] + " " + str(e["args"].get("shared memory")): e["args"] for e in events
             if "blend" in e.get("name", "") and ("warp_forward" in e["name"] or "warp_backward" in e["name"]) and "grid" in e.get("args", {})}
     if not seen:
         pytest.skip("no activity records of kernels here")
@@ -77,4 +78,6 @@ def test_blend_passes_launch_the_blocks_that_are_resident(tmp_path):
     for name, a in seen.items():
         threads, registers, shared = a["block"][0], a["registers per thread"], a["shared memory"]
         fit = min(2048 // threads, 65536 // (-(-registers * 32 // 256) * 256 * threads // 32), 228 * 1024 // (-(-(shared + 1024) // 128) * 128))
+        if "gaussian_warp_forward" in name:
+            fit = min(fit, 3)
         assert a["grid"][0] == multiprocessors * fit, (name, a["grid"][0] / multiprocessors, fit)
