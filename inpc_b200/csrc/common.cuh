@@ -149,6 +149,20 @@ KeyHistogram key_histogram(void* workspace, int64_t n, int64_t n_likely, int end
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
 int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
                      bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream);
+// The same, and every point carries a code with it: the first pass makes it from the point's footprint word (see Footprint in raster.cu), and code and position go
+// through the other passes in one 64-bit word with the key bits that are still to be sorted by (the first pass's own are no longer needed), so that whoever
+// reads the sorted positions need not gather the words.  Sorted positions and codes land in the values and in the keys of the result buffers (the
+// keys themselves are gone).  A code is the word itself where bit 31 is clear, else `escape` + log2(tiles): the word is to be looked up then.
+struct CarriedCodes {
+    const uint32_t* quad = nullptr;   // per point; anything where the key is kNoKey
+    int bits = 0;                     // of a code; 0: not carried
+    uint32_t escape = 0;              // above every word with bit 31 clear
+};
+// The codes for n points with keys of end_bit bits and words below `words`; none (bits == 0) where key bits behind the first pass, code and position do
+// not fit 64 bits.
+CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t words);
+int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes& codes,
+                                void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for (n_max, n_likely).  The result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,

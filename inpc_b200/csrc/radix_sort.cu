@@ -100,17 +100,38 @@ struct PassSmem {
     unsigned tile_id;
 };
 
+// What a pass reads and writes.
+//   PASS_PAIRS    keys and values, as they are.
+//   PASS_MARKED   (a first pass) keys of kNoKey take no part, and the values are the positions.
+//   PASS_PACK     (a first pass) the same, and the position is written as a 64-bit word with the key bits above this pass's digit on top, then the code
+//                 of the point's footprint word: its upper half goes where the keys go and its lower half where the values go, so
+//                 that the passes behind it sort by bits of the upper half and need not know.
+//   PASS_UNPACK   (the last pass behind it) the values written are the positions, the keys the codes.
+enum { PASS_PAIRS = 0, PASS_MARKED = 1, PASS_PACK = 2, PASS_UNPACK = 3 };
+
+// Widths of the fields of such a word; `codes` for PASS_PACK only.
+struct PackedFields {
+    int key_bits, position_bits;
+    CarriedCodes codes;
+};
+
+// log2 of the tiles a splat touches, of a footprint word with bit 31 set.
+__device__ __forceinline__ unsigned tiles_log2_of_escaped(uint32_t q) { return ((q & 0xFu) == 9u ? 1u : 0u) + ((q >> 16 & 0xFu) == 9u ? 1u : 0u); }
+
 // BITS > 0 fixes the digit width at compile time; BITS == 0 takes it from `bits_arg`.
-// MARKED (a first pass): keys of kNoKey take no part, and the values are the positions.  Points that are culled get such a key where they lie, which
+// PASS_MARKED: keys of kNoKey take no part, and the values are the positions.  Points that are culled get such a key where they lie, which
 // spares the projection a pass that counts the visible ones beforehand, a scan and the point ids: training step of 2^23 samples at 1237x822
 // 1684 -> 1639 us, of 2^24 points at 3840x2160 2795 -> 2703, 2^25 points of a cloud at 1920x1080 3158 -> 3008.
-template <int BITS, int ITEMS, bool MARKED>
+template <int BITS, int ITEMS, int FORM>
 __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n_arg, const unsigned long long* __restrict__ n_dev,
     int shift, int bits_arg, const unsigned* __restrict__ digit_base, volatile unsigned* tile_state, unsigned* ticket,
-    volatile unsigned* status, int spin_limit, unsigned mute_tile) {
+    volatile unsigned* status, int spin_limit, unsigned mute_tile, const PackedFields fields) {
     await_previous_kernel();
+    constexpr bool MARKED = FORM == PASS_MARKED || FORM == PASS_PACK;
+    constexpr int kLocalBits = ITEMS == kLargeItems ? 13 : 11;   // of a position in the tile
+    static_assert(kThreads * ITEMS == 1 << kLocalBits, "positions of a tile");
     using Smem = PassSmem<BITS, ITEMS>;
     constexpr int kBins = Smem::kBins;
     constexpr unsigned kTile = kThreads * ITEMS;
@@ -188,7 +209,14 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
         {
             const unsigned first = tile * kTile + local;
             const uint32_t* vp = vals_in + first;
-            if (MARKED || !vals_in) {   // the values are the positions
+            if (FORM == PASS_PACK) {
+                // the words of marked points are not used
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) val[i] = full || first + i * 32u < n ? __ldg(fields.codes.quad + first + i * 32u) : 0u;
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i)
+                    if (val[i] >> 31) val[i] = fields.codes.escape + tiles_log2_of_escaped(val[i]);
+            } else if (MARKED || !vals_in) {   // the values are the positions
 #pragma unroll
                 for (int i = 0; i < ITEMS; ++i) val[i] = first + i * 32u;
             } else if (full) {
@@ -263,7 +291,15 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
         __syncthreads();   // the counters are dead from here on: their storage holds the staged pairs
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i)
-            if (!MARKED || key[i] != kNoKey) s.pairs[i & 1 ? pos2[i / 2] >> 16 : pos2[i / 2] & 0xFFFFu] = make_uint2(key[i], val[i]);
+            if (!MARKED || key[i] != kNoKey) {
+                uint2 staged = make_uint2(key[i], val[i]);
+                if (FORM == PASS_PACK) {   // key, code and position in the tile: with the pass's digit the word has no room for the whole position
+                    const unsigned long long word = ((unsigned long long)(key[i] & (0xFFFFFFFFu >> (32 - fields.key_bits))) << (fields.codes.bits + kLocalBits)) |
+                                                    ((unsigned long long)val[i] << kLocalBits) | (local + i * 32u);
+                    staged = make_uint2((unsigned)(word >> 32), (unsigned)word);
+                }
+                s.pairs[i & 1 ? pos2[i / 2] >> 16 : pos2[i / 2] & 0xFFFFu] = staged;
+            }
         __syncthreads();
 
         // 4. write-out.  Padding ranks behind every real pair of the last tile, i.e. at slots >= valid.  dst < n always holds
@@ -273,8 +309,22 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
         for (int i = 0; i < ITEMS; ++i) {
             const unsigned q = tid + i * kThreads;
             if (MARKED ? q < block_total : full || q < valid) {
-                const uint2 kv = s.pairs[q];
-                const unsigned dst = s.global_off[(kv.x >> shift) & digit_mask] + q;
+                uint2 kv = s.pairs[q];
+                unsigned digit = (kv.x >> shift) & digit_mask;
+                if (FORM == PASS_PACK) {   // shift is 0: the digit lies at the lower end of the key
+                    const unsigned long long word = ((unsigned long long)kv.x << 32) | kv.y;
+                    digit = (unsigned)(word >> (fields.codes.bits + kLocalBits)) & digit_mask;
+                    const int rest = fields.key_bits - (BITS > 0 ? BITS : bits_arg);
+                    const unsigned long long out = ((word >> (fields.codes.bits + kLocalBits + (BITS > 0 ? BITS : bits_arg))) << (64 - rest)) |
+                                                   (((word >> kLocalBits) & ((1ull << fields.codes.bits) - 1ull)) << fields.position_bits) |
+                                                   (tile * kTile + (kv.y & (kTile - 1u)));
+                    kv = make_uint2((unsigned)(out >> 32), (unsigned)out);
+                }
+                if (FORM == PASS_UNPACK) {
+                    const unsigned long long word = ((unsigned long long)kv.x << 32) | kv.y;
+                    kv = make_uint2((unsigned)(word >> fields.position_bits) & ((1u << fields.codes.bits) - 1u), kv.y & ((1u << fields.position_bits) - 1u));
+                }
+                const unsigned dst = s.global_off[digit] + q;
                 if (dst < n) {
                     keys_out[dst] = kv.x;
                     vals_out[dst] = kv.y;
@@ -330,37 +380,43 @@ struct PassArgs {
     int shift, bits;
     const unsigned* base;
     unsigned *state, *ticket, *status;
-    bool marked;           // leaves out keys of kNoKey (first pass)
+    int form;              // PASS_...
+    PackedFields fields;   // of PASS_PACK and PASS_UNPACK
     int spin_limit;        // polls a tile spends on one unpublished predecessor before it gives up
     unsigned mute_tile;    // tile that never publishes (tests only); 0xFFFFFFFF = none
 };
 
-template <int BITS, int ITEMS, bool MARKED>
+template <int BITS, int ITEMS, int FORM>
 int launch_onesweep_instance(const PassArgs& a, cudaStream_t stream) {
     static bool attr_set[kMaxDevices] = {false};
     constexpr size_t kSmemBytes = sizeof(PassSmem<BITS, ITEMS>);
-    const int rc = opt_in_dynamic_smem(radix_onesweep_pass_kernel<BITS, ITEMS, MARKED>, kSmemBytes, attr_set);
+    const int rc = opt_in_dynamic_smem(radix_onesweep_pass_kernel<BITS, ITEMS, FORM>, kSmemBytes, attr_set);
     if (rc != INPC_OK) return rc;
     const int64_t resident = (int64_t)sm_count() * 2;
-    launch_chained(radix_onesweep_pass_kernel<BITS, ITEMS, MARKED>, (unsigned)(a.tiles < resident ? a.tiles : resident), kThreads, kSmemBytes, stream,
-        a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base, a.state, a.ticket, a.status, a.spin_limit, a.mute_tile);
+    launch_chained(radix_onesweep_pass_kernel<BITS, ITEMS, FORM>, (unsigned)(a.tiles < resident ? a.tiles : resident), kThreads, kSmemBytes, stream,
+        a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base, a.state, a.ticket, a.status, a.spin_limit, a.mute_tile, a.fields);
     INPC_LAUNCH_CHECK("radix_onesweep_pass_kernel");
     return INPC_OK;
 }
 
-template <int ITEMS, bool MARKED>
-int launch_onesweep_pass(const PassArgs& a, cudaStream_t stream) {
+template <int ITEMS, int FORM>
+int launch_onesweep_form(const PassArgs& a, cudaStream_t stream) {
     switch (a.bits) {
-        case 7: return launch_onesweep_instance<7, ITEMS, MARKED>(a, stream);
-        case 8: return launch_onesweep_instance<8, ITEMS, MARKED>(a, stream);
-        case 9: return launch_onesweep_instance<9, ITEMS, MARKED>(a, stream);
-        default: return launch_onesweep_instance<0, ITEMS, MARKED>(a, stream);
+        case 7: return launch_onesweep_instance<7, ITEMS, FORM>(a, stream);
+        case 8: return launch_onesweep_instance<8, ITEMS, FORM>(a, stream);
+        case 9: return launch_onesweep_instance<9, ITEMS, FORM>(a, stream);
+        default: return launch_onesweep_instance<0, ITEMS, FORM>(a, stream);
     }
 }
 
 template <int ITEMS>
 int launch_onesweep_pass(const PassArgs& a, cudaStream_t stream) {
-    return a.marked ? launch_onesweep_pass<ITEMS, true>(a, stream) : launch_onesweep_pass<ITEMS, false>(a, stream);
+    switch (a.form) {
+        case PASS_MARKED: return launch_onesweep_form<ITEMS, PASS_MARKED>(a, stream);
+        case PASS_PACK: return launch_onesweep_form<ITEMS, PASS_PACK>(a, stream);
+        case PASS_UNPACK: return launch_onesweep_form<ITEMS, PASS_UNPACK>(a, stream);
+        default: return launch_onesweep_form<ITEMS, PASS_PAIRS>(a, stream);
+    }
 }
 
 }  // namespace
@@ -436,7 +492,7 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 // `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
                            int items, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
-                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, unsigned long long* marked_count = nullptr, bool counted = false) {
+                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, unsigned long long* marked_count = nullptr, bool counted = false, const CarriedCodes* codes = nullptr) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
 
@@ -458,17 +514,16 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
     a.spin_limit = spin_limit; a.mute_tile = mute_tile;
     a.kin = keys; a.kout = keys_alt; a.vin = position_values || marked_count ? nullptr : values; a.vout = values_alt;
     a.state = w.state;
-    a.marked = marked_count != nullptr;
+    a.fields = {end_bit, bit_length((uint32_t)(n - 1)), codes ? *codes : CarriedCodes{}};
     for (int p = 0; p < pt.n_passes; ++p) {
         a.shift = pt.shift[p]; a.bits = pt.bits[p];
+        a.form = p == 0 && marked_count ? (codes ? PASS_PACK : PASS_MARKED) : codes && p == pt.n_passes - 1 ? PASS_UNPACK : PASS_PAIRS;
+        if (codes && p > 0) a.shift += 32 - end_bit;   // the key's upper bits lie at the upper end of the first word
         a.base = w.base + p * kRadix;
         a.ticket = w.ticket + p;
         const int rc = items == kLargeItems ? launch_onesweep_pass<kLargeItems>(a, stream) : launch_onesweep_pass<kSmallItems>(a, stream);
         if (rc != INPC_OK) return rc;
-        if (a.marked) {   // the passes behind the first find only the keys that take part
-            a.marked = false;
-            a.n_dev = marked_count;
-        }
+        if (p == 0 && marked_count) a.n_dev = marked_count;   // the passes behind the first find only the keys that take part
         a.state += (size_t)tiles * pass_bins(a.bits);
         const uint32_t* t = a.kin; a.kin = a.kout; a.kout = const_cast<uint32_t*>(t);
         a.vin = a.vout; a.vout = a.vout == values ? values_alt : values;
@@ -499,6 +554,30 @@ int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint3
     if (n < 1 || nothing || !workspace || !count) { set_error("sort_marked_keys: needs keys, key bits, a workspace and a place for the count"); return INPC_E_INVALID; }
     return sort_pairs_with("sort_marked_keys", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
                            0xFFFFFFFFu, nullptr, true, count);
+}
+
+CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t words) {
+    CarriedCodes c;
+    if (n < 1 || end_bit < 1 || end_bit > 32 || words < 1 || words > (int64_t)1 << 30) return c;
+    const PassTable pt = pass_table(end_bit);
+    const int bits = bit_length((uint32_t)(words + 2));
+    // behind the first pass: the key bits that are left, code, position; staged in the first one: key, code, position in the tile
+    if (pt.n_passes < 2 || end_bit - pt.bits[0] + bits + bit_length((uint32_t)(n - 1)) > 64 || end_bit + bits + bit_length(kLargeTile - 1) > 64) return c;
+    c.quad = quad;
+    c.bits = bits;
+    c.escape = (uint32_t)words;
+    return c;
+}
+
+int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes& codes,
+                                void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream) {
+    if (result_in_alt) *result_in_alt = 0;
+    bool nothing = false;
+    const int rc = check_sort_args("sort_marked_keys", keys, keys_alt, values, values_alt, n < 2 ? 2 : n, end_bit, &nothing);
+    if (rc != INPC_OK) return rc;
+    if (nothing || !workspace || !count || !codes.quad || codes.bits < 1 || sort_pass_count(end_bit) < 2) { set_error("sort_marked_keys: needs keys and codes that fit, a workspace and a place for the count"); return INPC_E_INVALID; }
+    return sort_pairs_with("sort_marked_keys", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
+                           0xFFFFFFFFu, nullptr, true, count, false, &codes);
 }
 
 // The same sort with the number of pairs in device memory (*n_dev <= n_max): grids and the look-back state are

@@ -380,28 +380,47 @@ __device__ __forceinline__ float sh_eval_channel(const float* b, const __half* h
            b[6] * __half2float(h[24 + c]) - b[7] * __half2float(h[28 + c]) + b[8] * __half2float(h[32 + c]);
 }
 
-// What the instance emission of the warp blend needs of a bilinear splat, in one word.  Columns: pixel column of the
-// left pixel of its 2x2 footprint plus one (15 bits; a visible splat's footprint starts at pixel -1 at the earliest),
-// whether it touches two tile columns (1 bit).  Rows: the first tile row it touches in the stacked grid (11 bits), the
-// row of its upper pixel relative to that tile plus one (4 bits, 0..8), whether it touches two tile rows (1 bit).
-// Rows are kept relative to the tile because the first row of an image other than the first is not row 0 of the
-// grid.  4 bytes per point keep the array (33 MB for 2^23 points) resident in L2 while the emission gathers from
-// it in depth order.
+// What the instance emission of the warp blend needs of a bilinear splat, in one word: 4 bytes per point keep the array (33 MB for 2^23 points) resident
+// in L2 where the emission gathers from it in depth order, and in most calls the depth sort has room to carry the word along (CarriedCodes).
+//   bit 31 clear: first tile it touches in the (stacked) grid * 64 + row * 8 + column of the upper left pixel of its 2x2 footprint in that tile; it touches a
+//                 second tile column or row if and only if that is the last pixel column or row of the tile.
+//   bit 31 set:   the splats of which this is not so -- the footprint begins in front of the image, or ends at its border, or the splat lies exactly between two
+//                 pixels at a tile's edge: first tile column in bits 4..15, row in bits 20..30, and in front of them the column and row of that pixel in
+//                 the tile plus one (0..8), 9 for 8 and a second tile.  (8 it is whenever there is a second tile: with sx - 0.5 rounded below the last
+//                 pixel of a tile, sx + 0.5 rounds to the tile's end at most.)
 constexpr int kMaxCodedSide = 32760;       // widest image of this path, in pixels
 constexpr int kMaxCodedTileRows = 2047;    // most tile rows of the (stacked) grid
-__device__ __forceinline__ uint32_t pack_quad(const Projection& pr, int tile_rows_before) {
-    const unsigned qx1 = (unsigned)(__float2int_rd(pr.sx - 0.5f) + 1);
-    const unsigned ry1 = (unsigned)(__float2int_rd(pr.sy - 0.5f) - ((int)pr.y0 - tile_rows_before) * 8 + 1);
-    return (qx1 & 0x7FFFu) | ((pr.x1 - pr.x0 - 1u) << 15) | ((pr.y0 & 0x7FFu) << 16) | ((ry1 & 0xFu) << 27) | ((pr.y1 - pr.y0 - 1u) << 31);
+constexpr uint32_t kNoQuad = 0xFFFFFFFFu;  // of a culled point
+struct Footprint {
+    unsigned tile;          // first tile
+    unsigned column, row;   // of the upper left pixel in that tile, plus one: 0 .. 8
+    bool two_columns, two_rows;
+};
+__device__ __forceinline__ uint32_t pack_quad(const Projection& pr, int tile_rows_before, int gw) {
+    // rows are relative to the tile: the first row of an image other than the first is not row 0 of the grid
+    const unsigned column = (unsigned)(__float2int_rd(pr.sx - 0.5f) - (int)pr.x0 * 8 + 1);
+    const unsigned row = (unsigned)(__float2int_rd(pr.sy - 0.5f) - ((int)pr.y0 - tile_rows_before) * 8 + 1);
+    const unsigned two_columns = pr.x1 - pr.x0 - 1u, two_rows = pr.y1 - pr.y0 - 1u;
+    if (column - 1u < 8u && row - 1u < 8u && two_columns == (column == 8u ? 1u : 0u) && two_rows == (row == 8u ? 1u : 0u))
+        return (pr.y0 * (unsigned)gw + pr.x0) << 6 | (row - 1u) << 3 | (column - 1u);
+    return 0x80000000u | pr.y0 << 20 | (min(row, 8u) + two_rows) << 16 | pr.x0 << 4 | (min(column, 8u) + two_columns);
 }
-constexpr uint32_t kNoQuad = 0xFFFFFFFFu;  // of a culled point (its column would lie beyond kMaxCodedSide)
+__device__ __forceinline__ Footprint footprint_of_quad(uint32_t q, int gw) {
+    if (!(q >> 31)) {
+        const unsigned column = (q & 7u) + 1u, row = (q >> 3 & 7u) + 1u;
+        return {q >> 6, column, row, column == 8u, row == 8u};
+    }
+    const unsigned column = q & 0xFu, row = q >> 16 & 0xFu;
+    return {(q >> 20 & 0x7FFu) * (unsigned)gw + (q >> 4 & 0xFFFu), min(column, 8u), min(row, 8u), column == 9u, row == 9u};
+}
+__device__ __forceinline__ unsigned tiles_of_footprint(bool two_columns, bool two_rows) { return (two_columns ? 2u : 1u) << (two_rows ? 1 : 0); }
 
-// Tile bounds of a splat in the form of the `bounds` array: the first tile is floor(origin / 8), never below 0.
-__device__ __forceinline__ uint2 quad_bounds(uint32_t q) {
+// Tile bounds of a splat in the form of the `bounds` array.
+__device__ __forceinline__ uint2 quad_bounds(uint32_t q, int gw) {
     if (q == kNoQuad) return make_uint2(0u, 0u);
-    const int qx = (int)(q & 0x7FFFu) - 1;
-    const unsigned x0 = qx < 0 ? 0u : (unsigned)qx >> 3, y0 = (q >> 16) & 0x7FFu;
-    return make_uint2(x0 | ((x0 + 1u + ((q >> 15) & 1u)) << 16), y0 | ((y0 + 1u + (q >> 31)) << 16));
+    const Footprint f = footprint_of_quad(q, gw);
+    const unsigned y0 = f.tile / (unsigned)gw, x0 = f.tile - y0 * (unsigned)gw;
+    return make_uint2(x0 | ((x0 + 1u + f.two_columns) << 16), y0 | ((y0 + 1u + f.two_rows) << 16));
 }
 
 // What the instance emission needs of a gaussian splat on 8x8 tiles: its tile bounds, and how far its ellipse stays away from
@@ -489,7 +508,7 @@ __global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
     __syncthreads();
     // what the instance passes need of a point: its packed footprint where splats are bilinear on 8x8 tiles, else its tile bounds
     auto write_bounds = [&](bool visible) {
-        if (MODE == INPC_MODE_BILINEAR && quad) quad[iv] = visible ? pack_quad(pr, set * rp.gh) : kNoQuad;
+        if (MODE == INPC_MODE_BILINEAR && quad) quad[iv] = visible ? pack_quad(pr, set * rp.gh, rp.gw) : kNoQuad;
         else bounds[iv] = visible ? make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16)) : make_uint2(0u, 0u);
     };
     if (i >= n && iv < ps.start[ps.count]) write_bounds(false);   // padding behind a set
@@ -558,18 +577,27 @@ __device__ __forceinline__ unsigned tiles_of(const uint2 b) {
 // Instances per depth-sorted point, reduced per block (src/bilinear/kernels.cu:186-196 + the
 // cub::DeviceScan::ExclusiveSum of src/bilinear/forward.cu:109-115, first half).
 constexpr int kInstThreads = 1024;   // block sums over 1024 points keep the one-block scan short
-// Packed: a warp sums one block's worth of points, all its loads in flight together, no barrier before the last block's scan (a barrier
-// per group of a block and one load per thread: 2^23 / 2^25 points 16 / 61 -> 11 / 39 us).
-template <bool PACKED>
+__device__ __forceinline__ unsigned tiles_of_code(uint32_t code, uint32_t escape) {
+    return code >= escape ? 1u << (code - escape) : tiles_of_footprint((code & 7u) == 7u, (code >> 3 & 7u) == 7u);
+}
+
+// COUNTS_IN_KEYS, COUNTS_IN_CODES (see CarriedCodes): a warp sums one block's worth of points, all its loads in flight together, no barrier before the last
+// block's scan (a barrier per group of a block and one load per thread: 2^23 / 2^25 points 16 / 61 -> 11 / 39 us).
+enum { COUNTS_GATHERED = 0, COUNTS_IN_KEYS = 1, COUNTS_IN_CODES = 2 };
+template <int SOURCE>
 __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const uint32_t* __restrict__ sorted_keys,
                                                                           const uint32_t* __restrict__ sorted_ids,
                                                                           const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
                                                                           const unsigned long long* __restrict__ n_visible_dev,
-                                                                          unsigned* block_sums, unsigned n_groups, unsigned* done, unsigned long long* n_instances) {
+                                                                          unsigned* block_sums, unsigned n_groups, unsigned* done, unsigned long long* n_instances, uint32_t escape) {
     await_previous_kernel();
     const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
     constexpr unsigned kWarps = kInstThreads / 4 / 32;
-    if (PACKED) {
+    if (SOURCE != COUNTS_GATHERED) {
+        auto count_of = [&](uint32_t word) -> unsigned {
+            if (SOURCE == COUNTS_IN_KEYS) return (word >> kCountShift) + 1u;
+            return tiles_of_code(word, escape);
+        };
         constexpr int kLoads = kInstThreads / 128;   // 16-byte loads per lane and group
         for (unsigned group = blockIdx.x * kWarps + (threadIdx.x >> 5); group < n_groups; group += gridDim.x * kWarps) {
             const int64_t first = (int64_t)group * kInstThreads + 4 * (int64_t)lane_id();
@@ -579,9 +607,9 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
 #pragma unroll
                 for (int q = 0; q < kLoads; ++q) k[q] = __ldg(reinterpret_cast<const uint4*>(sorted_keys + first + 128 * q));   // the key buffers are 16-byte aligned
 #pragma unroll
-                for (int q = 0; q < kLoads; ++q) c += (k[q].x >> kCountShift) + (k[q].y >> kCountShift) + (k[q].z >> kCountShift) + (k[q].w >> kCountShift) + 4u;
+                for (int q = 0; q < kLoads; ++q) c += count_of(k[q].x) + count_of(k[q].y) + count_of(k[q].z) + count_of(k[q].w);
             } else {
-                for (int64_t s = (int64_t)group * kInstThreads + lane_id(); s < n_visible; s += 32) c += (__ldg(sorted_keys + s) >> kCountShift) + 1u;
+                for (int64_t s = (int64_t)group * kInstThreads + lane_id(); s < n_visible; s += 32) c += count_of(__ldg(sorted_keys + s));
             }
             c = __reduce_add_sync(0xffffffffu, c);
             if (lane_id() == 0) block_sums[group] = c;
@@ -598,7 +626,12 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
                 const int64_t s = first + q;
                 if (s >= n_visible) continue;
                 const uint32_t id = checked_point(__ldg(sorted_ids + s));
-                c += tiles_of(quad ? quad_bounds(__ldg(quad + id)) : __ldg(bounds + id));
+                if (quad) {
+                    const Footprint f = footprint_of_quad(__ldg(quad + id), 0);
+                    c += tiles_of_footprint(f.two_columns, f.two_rows);
+                } else {
+                    c += tiles_of(__ldg(bounds + id));
+                }
             }
             c = __reduce_add_sync(0xffffffffu, c);
             if (lane_id() == 0) s_w[flip][threadIdx.x >> 5] = c;
@@ -678,7 +711,8 @@ __global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint3
         const bool there = s < n_visible;
         const uint32_t id = there ? checked_point(__ldcs(sorted_ids + s)) : 0u;
         const uint32_t q = there ? __ldg(quad + id) : 0u;
-        const bool two_columns = there && ((q >> 15) & 1u), two_rows = there && (q >> 31);
+        const Footprint f = footprint_of_quad(q, gw);
+        const bool two_columns = there && f.two_columns, two_rows = there && f.two_rows;
         // one, two or four instances per point: the sum over the lanes before this one from three ballots
         const unsigned bt = __ballot_sync(0xffffffffu, there), bc = __ballot_sync(0xffffffffu, two_columns), br = __ballot_sync(0xffffffffu, two_rows);
         if (lane == 0) s_total[flip][warp] = __popc(bt) + __popc(bc) + __popc(br) + __popc(bc & br);
@@ -686,12 +720,8 @@ __global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint3
         unsigned off = __ldg(block_base + group) + __reduce_add_sync(0xffffffffu, lane < warp ? s_total[flip][lane] : 0u) + __popc(bt & lt_mask) + __popc(bc & lt_mask) +
                        __popc(br & lt_mask) + __popc(bc & br & lt_mask);
         if (!there) continue;
-        // the tile bounds follow from the footprint origin: first tile = floor(origin / 8), never below 0.  In a second column or
-        // row of tiles the footprint starts one pixel before the tile: its code there is zero
-        const int qx = (int)(q & 0x7FFFu) - 1;
-        const unsigned x0 = qx < 0 ? 0u : (unsigned)qx >> 3, y0 = (q >> 16) & 0x7FFu;
-        const uint32_t column = (unsigned)(qx - (int)x0 * 8 + 1) << kTileKeyBits, row = min((q >> 27) & 0xFu, 8u) << (kTileKeyBits + 4);
-        const uint32_t tile = y0 * (unsigned)gw + x0;
+        // in a second column or row of tiles the footprint starts one pixel before the tile: its code there is zero
+        const uint32_t column = f.column << kTileKeyBits, row = f.row << (kTileKeyBits + 4), tile = f.tile;
         emit(off, tile | column | row, id);
         if (two_columns) emit(off + 1u, (tile + 1u) | row, id);
         if (two_rows) {
@@ -701,6 +731,93 @@ __global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint3
         }
     }
     finish_histogram(s_digits, digits, (unsigned)min(n_groups, (int64_t)gridDim.x), n_emitted);
+}
+
+// Bilinear splats whose codes the depth sort has carried along: no gather, but where a code does not say it all (one splat in 500 at 1237x822).  A thread takes four
+// consecutive points, the loads of the next group under way while this one's instances are written; a warp stages its instances in shared memory and writes them side
+// by side.  Bound by instruction issue: 2^20 / 2^23 / 2^25 points 11.5 / 47 / 166 us (16 / 95 / 412 with the kernel above; 43 million instances in 166 us are 3.7 TB/s read and
+// written).  What the sort pays for it: 0.2 us of 66 for 2^23 points, 13 of 220 for 2^25, where the words it reads come from DRAM.
+// Two points per thread 54 / 216 us for 2^23 / 2^25; 256 staged pairs per warp and four blocks 58 / 201; no loads ahead 52 / 188; codes of a grid that is one pixel
+// larger, which name the splats at the border too but take a division, 59 / 207.  With the gathers of the kernel above this form is the slower one: 2^24 points 193 -> 408 us,
+// fewer and busier warps miss L2 more often.
+constexpr int kCodedThreads = 512, kCodedPoints = 4, kCodedBlocks = 3;
+struct EmitCodedSmem {
+    uint2 pairs[kCodedThreads / 32][32 * kCodedPoints * 4];   // the most a warp's points can make
+};
+__global__ void __launch_bounds__(kCodedThreads, kCodedBlocks) emit_coded_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ sorted_codes, const CarriedCodes codes,
+                                                                      const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
+                                                                      KeyHistogram digits, unsigned long long* __restrict__ n_emitted, uint32_t* __restrict__ inst_keys,
+                                                                      uint32_t* __restrict__ inst_ids) {
+    await_previous_kernel();
+    constexpr unsigned kGroup = kCodedThreads * kCodedPoints, kWarps = kCodedThreads / 32, kSums = kInstThreads / (32 * kCodedPoints);   // kSums: warps per sum
+    static_assert(kGroup % kInstThreads == 0 && kCodedPoints == 4, "groups begin where sums do; 16-byte loads");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    EmitCodedSmem& s_stage = *reinterpret_cast<EmitCodedSmem*>(smem_raw);
+    __shared__ unsigned s_total[2][kWarps];   // of two groups in turn, so that one barrier does
+    __shared__ BlockHistogram s_digits;
+    const unsigned n_visible = (unsigned)*n_visible_dev, n_groups = (n_visible + kGroup - 1u) / kGroup;
+    if (blockIdx.x >= n_groups) return;
+    clear_histogram(s_digits);
+    __syncthreads();
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    uint2* const stage = s_stage.pairs[warp];
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    uint32_t next_id[kCodedPoints], next_code[kCodedPoints];
+    auto load = [&](unsigned group) {
+        const unsigned first = group * kGroup + threadIdx.x * kCodedPoints;
+        if (group < n_groups && first + kCodedPoints <= n_visible) {
+            const uint4 a = __ldcs(reinterpret_cast<const uint4*>(sorted_ids + first)), b = __ldcs(reinterpret_cast<const uint4*>(sorted_codes + first));
+            next_id[0] = a.x; next_id[1] = a.y; next_id[2] = a.z; next_id[3] = a.w;
+            next_code[0] = b.x; next_code[1] = b.y; next_code[2] = b.z; next_code[3] = b.w;
+        } else {
+#pragma unroll
+            for (int k = 0; k < kCodedPoints; ++k) {
+                const bool there = group < n_groups && first + k < n_visible;
+                next_id[k] = there ? __ldg(sorted_ids + first + k) : 0u;
+                next_code[k] = there ? __ldg(sorted_codes + first + k) : kNone;
+            }
+        }
+    };
+    load(blockIdx.x);
+    unsigned flip = 0;
+    for (unsigned group = blockIdx.x; group < n_groups; group += gridDim.x, flip ^= 1u) {
+        uint32_t id[kCodedPoints], code[kCodedPoints];
+#pragma unroll
+        for (int k = 0; k < kCodedPoints; ++k) { id[k] = next_id[k]; code[k] = next_code[k]; }
+        load(group + gridDim.x);
+        unsigned own = 0u;
+#pragma unroll
+        for (int k = 0; k < kCodedPoints; ++k) own += code[k] == kNone ? 0u : tiles_of_code(code[k], codes.escape);
+        const unsigned inc = warp_inclusive_scan(own), warp_total = __shfl_sync(0xffffffffu, inc, 31);
+        if (lane == 0) s_total[flip][warp] = warp_total;
+        unsigned at = inc - own;
+#pragma unroll
+        for (int k = 0; k < kCodedPoints; ++k) {
+            if (code[k] == kNone) continue;
+            const Footprint f = footprint_of_quad(code[k] >= codes.escape ? __ldg(codes.quad + checked_point(id[k])) : code[k], gw);
+            // in a second column or row of tiles the footprint starts one pixel before the tile: its code there is zero
+            const uint32_t column = f.column << kTileKeyBits, row = f.row << (kTileKeyBits + 4);
+            stage[at++] = make_uint2(f.tile | column | row, id[k]);
+            if (f.two_columns) stage[at++] = make_uint2((f.tile + 1u) | row, id[k]);
+            if (f.two_rows) {
+                stage[at++] = make_uint2((f.tile + (unsigned)gw) | column, id[k]);
+                if (f.two_columns) stage[at++] = make_uint2(f.tile + (unsigned)gw + 1u, id[k]);
+            }
+        }
+        __syncthreads();
+        // behind the sums of kInstThreads points each, those of the warps between them and this one
+        const unsigned sum_first = warp / kSums * kSums;
+        const unsigned base = __ldg(block_base + (group * kGroup + warp * 32u * kCodedPoints) / kInstThreads) +
+                              __reduce_add_sync(0xffffffffu, lane >= sum_first && lane < warp ? s_total[flip][lane] : 0u);
+        for (unsigned i = lane; i < warp_total; i += 32u) {
+            const uint2 pair = stage[i];
+            __stcs(inst_keys + base + i, pair.x);
+            __stcs(inst_ids + base + i, pair.y);
+            count_key(s_digits, digits.pt, pair.x);
+        }
+        __syncwarp();
+    }
+    finish_histogram(s_digits, digits, min(n_groups, gridDim.x), n_emitted);
 }
 
 // Other splats.  CELLS (gaussian, 8x8 tiles): the key also says which cells of the tile the ellipse can reach (see cell_code).  The keys are counted by the
@@ -4215,34 +4332,46 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
 
     const bool counted = MODE == INPC_MODE_BILINEAR && warp_blend;   // the emission counts the digits of the keys
     int in_alt = 0;
+    CarriedCodes codes;   // the depth sort carries the footprints along where they fit
+    if (deferred) codes = carried_codes(pb.quad, n, key_bits, (int64_t)n_tiles * 64);
+    const bool carried = codes.bits > 0;
     {
         StageScope scope(STAGE_SORT_DEPTH, stream);
-        rc = deferred ? sort_marked_keys(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, pb.sort_ws, true, status, &in_alt, stream)
+        rc = carried  ? sort_marked_keys_with_codes(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, codes, pb.sort_ws, true, status, &in_alt, stream)
+             : deferred ? sort_marked_keys(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, pb.sort_ws, true, status, &in_alt, stream)
                       : sort_pairs(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n, key_bits, pb.sort_ws, false, status, &in_alt, stream);
     }
     if (rc != INPC_OK) return rc;
     const uint32_t* sorted_ids = pb.ids[in_alt];
     if (n_visible > 0 && n_instances > 0) {
-        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_need = MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift ? ceil_div<int64_t>(ibk, kInstThreads / 4 / 32) : ibk, count_cap = (int64_t)sm_count() * 8;
+        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_need = MODE == INPC_MODE_BILINEAR && (carried || key_bits <= (int)kCountShift) ? ceil_div<int64_t>(ibk, kInstThreads / 4 / 32) : ibk, count_cap = (int64_t)sm_count() * 8;
         const unsigned count_blocks = (unsigned)(count_need < count_cap ? count_need : count_cap);
         {
             StageScope scope(STAGE_INSTANCES, stream);
-            // the count of touched tiles rides in the top key bits when the depth offsets left them free
-            if (MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift)
-                launch_chained(instance_count_kernel<true>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr);
-            else
-                launch_chained(instance_count_kernel<false>, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr);
+            // the count of touched tiles follows from the codes, or rides in the top key bits when the depth offsets left them free
+            auto* count = carried ? instance_count_kernel<COUNTS_IN_CODES> : MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift ? instance_count_kernel<COUNTS_IN_KEYS> : instance_count_kernel<COUNTS_GATHERED>;
+            launch_chained(count, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr, codes.escape);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (counted) {
-                const int64_t emit_cap = (int64_t)sm_count() * 2;   // two blocks of 1024 threads fill a multiprocessor
                 const KeyHistogram digits = key_histogram(ib.sort_ws, n_instances, likely_instances(n_instances, deferred), tile_bits);
-                launch_chained(emit_quads_kernel, (unsigned)(ibk < emit_cap ? ibk : emit_cap), kInstThreads, 0, stream, sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums,
-                    rp.gw, digits, deferred && tile_bits > 0 ? pb.counters + 2 : nullptr, ib.keys[0], ib.ids[0]);
+                unsigned long long* n_emitted = deferred && tile_bits > 0 ? pb.counters + 2 : nullptr;
+                if (carried) {
+                    static bool attr_set[kMaxDevices] = {false};
+                    rc = opt_in_dynamic_smem(emit_coded_kernel, sizeof(EmitCodedSmem), attr_set);
+                    if (rc != INPC_OK) return rc;
+                    const int64_t need = ceil_div<int64_t>(n_visible, kCodedThreads * kCodedPoints), cap = (int64_t)sm_count() * kCodedBlocks;
+                    launch_chained(emit_coded_kernel, (unsigned)(need < cap ? need : cap), kCodedThreads, sizeof(EmitCodedSmem), stream, sorted_ids, pb.keys[in_alt], codes, n_visible_dev,
+                        pb.inst_block_sums, rp.gw, digits, n_emitted, ib.keys[0], ib.ids[0]);
+                } else {
+                    const int64_t cap = (int64_t)sm_count() * 2;   // two blocks of 1024 threads fill a multiprocessor
+                    launch_chained(emit_quads_kernel, (unsigned)(ibk < cap ? ibk : cap), kInstThreads, 0, stream, sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums,
+                        rp.gw, digits, n_emitted, ib.keys[0], ib.ids[0]);
+                }
             } else {
                 launch_chained(warp_blend ? emit_instances_kernel<true> : emit_instances_kernel<false>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.foot, n_visible,
                     n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             }
-            INPC_LAUNCH_CHECK(counted ? "emit_quads_kernel" : "emit_instances_kernel");
+            INPC_LAUNCH_CHECK(carried ? "emit_coded_kernel" : counted ? "emit_quads_kernel" : "emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
@@ -4936,18 +5065,18 @@ extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
 }
 
 namespace inpc_debug {
-__global__ void add_base_kernel(const uint32_t* __restrict__ src, int64_t n, uint32_t base, uint32_t mask, uint32_t* __restrict__ dst) {
+__global__ void sorted_depths_kernel(const uint32_t* __restrict__ ids, const PointRec* __restrict__ rec, int rec_stride, int64_t n, uint32_t* __restrict__ dst) {
     await_previous_kernel();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = (src[i] & mask) + base;
+    if (i < n) dst[i] = __float_as_uint(reinterpret_cast<const float4*>(rec)[(int64_t)ids[i] * rec_stride].w);
 }
 
 __global__ void unpack_points_kernel(const PointRec* __restrict__ rec, int rec_stride, const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, int64_t n, int which,
-                                     void* __restrict__ dst) {
+                                     int gw, void* __restrict__ dst) {
     await_previous_kernel();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint2 b = quad ? quad_bounds(quad[i]) : bounds[i];
+    const uint2 b = quad ? quad_bounds(quad[i], gw) : bounds[i];
     const bool vis = tiles_of(b) != 0u;
     const float4* r = reinterpret_cast<const float4*>(rec) + i * rec_stride;
     if (which == 4) static_cast<unsigned*>(dst)[i] = tiles_of(b);
@@ -4975,19 +5104,18 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
     const int ti = tile_buffer_of(state, n_tiles);
     switch (which) {
         case 0: INPC_CUDA_TRY(cudaMemcpyAsync(dst, pb.ids[d], 4 * (size_t)state->n_visible, cudaMemcpyDeviceToDevice, stream)); break;
-        case 1:   // the sort works on offsets from the smallest depth key: add the base back
+        case 1:   // not every sort keeps its keys: the depths of the points in their order
             if (state->n_visible > 0) {
-                launch_chained(inpc_debug::add_base_kernel, (unsigned)ceil_div<int64_t>(state->n_visible, 256), 256, 0, stream,
-                    pb.keys[d], state->n_visible, state->depth_key_base,
-                    state->depth_key_bits <= 30 ? 0x3FFFFFFFu : 0xFFFFFFFFu, static_cast<uint32_t*>(dst));
-                INPC_LAUNCH_CHECK("add_base_kernel");
+                launch_chained(inpc_debug::sorted_depths_kernel, (unsigned)ceil_div<int64_t>(state->n_visible, 256), 256, 0, stream,
+                    pb.ids[d], pb.rec, (state->deferred_counts & 2) ? 1 : 2, state->n_visible, static_cast<uint32_t*>(dst));
+                INPC_LAUNCH_CHECK("sorted_depths_kernel");
             }
             break;
         case 2: INPC_CUDA_TRY(cudaMemcpyAsync(dst, ib.ids[ti], 4 * (size_t)state->n_instances, cudaMemcpyDeviceToDevice, stream)); break;
         case 3: INPC_CUDA_TRY(cudaMemcpyAsync(dst, ib.ranges, 8 * (size_t)n_tiles, cudaMemcpyDeviceToDevice, stream)); break;
         case 4: case 5: case 6: case 7: case 8:
             if (state->n_points > 0) {
-                launch_chained(inpc_debug::unpack_points_kernel, (unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream, pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, pb.quad, state->n_points, which, dst);
+                launch_chained(inpc_debug::unpack_points_kernel, (unsigned)ceil_div<int64_t>(state->n_points, 256), 256, 0, stream, pb.rec, (state->deferred_counts & 2) ? 1 : 2, pb.bounds, pb.quad, state->n_points, which, gw, dst);
                 INPC_LAUNCH_CHECK("unpack_points_kernel");
             }
             break;

@@ -60,3 +60,41 @@ def test_key_ranges_next_to_the_mark_of_a_culled_point(near, far):
     n = 5000
     view, pos, opac = _scene(n, torch.arange(n) % 3 != 0, 7, near, far)
     assert _check(view, pos, opac) > n // 2
+
+
+# Splats that lie exactly between two pixels, also at the edges of tiles (no second tile is touched) and at the border of the image, in front of it and behind it,
+# beside others: their footprints do not follow from the codes that the depth sort carries along.  One tile; a few; so many that the codes do not fit beside
+# 32-bit keys (near plane at zero), where the words are gathered instead, as where keys are sorted in one pass (planes close together); both sizes of the sort's tiles.
+@pytest.mark.parametrize("width, height", [(8, 8), (64, 24), (1024, 1040)])
+@pytest.mark.parametrize("near, far", [(0.01, 100.0), (0.0, 100.0), (1.0, 1.0 + 2.0 ** -16)])
+@pytest.mark.parametrize("n", [3000, (1 << 18) + 77])
+def test_footprints_that_end_exactly_at_a_tile(width, height, near, far, n):
+    from inpc_b200.views import look_at_view
+    g = torch.Generator().manual_seed(n + width)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, float(width), float(width), near_plane=near, far_plane=far)
+    depth = torch.tensor([1.0, 2.0, 4.0])[torch.randint(0, 3, (n,), generator=g)]
+    px, py = ((torch.randint(-2, 2 * s + 3, (n,), generator=g)) * 0.5 for s in (width, height))
+    other = torch.rand(n, generator=g) < 0.5
+    px, py = torch.where(other, px + torch.rand(n, generator=g) - 0.5, px), torch.where(other, py + torch.rand(n, generator=g) - 0.5, py)
+    pos = torch.stack([(px - width / 2) / width * depth, -(py - height / 2) / width * depth, 3.0 - depth], dim=1).contiguous()
+    assert _check(view, pos, torch.full((n, 1), 0.01)) > n // (5 if far < 2.0 else 2)
+
+
+def test_codes_of_stacked_images():
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    g = torch.Generator().manual_seed(5)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 72, 40, 64.0, 64.0).to(DEV)
+    sets = []
+    for n in (5000, 1, 4097):
+        px, py = torch.randint(-2, 147, (n,), generator=g) * 0.5, torch.randint(-2, 83, (n,), generator=g) * 0.5
+        depth = torch.tensor([1.0, 2.0, 4.0])[torch.randint(0, 3, (n,), generator=g)]
+        pos = torch.stack([(px - 36) / 64 * depth, -(py - 20) / 64 * depth, 3.0 - depth], dim=1).contiguous().to(DEV)
+        sets.append((pos, (torch.randn((n, 37), generator=g) - 2.0).to(torch.float16).to(DEV)))
+    images, depths, alphas = inpc_b200.INPCRasterizer(tile_size=8).render_multi(view, sets)
+    for k, (pos, raw) in enumerate(sets):
+        for tile in (8, 16):   # 16x16 tiles know no codes; sums in another order
+            image, depth, alpha = inpc_b200.INPCRasterizer(tile_size=tile).render(view, 0, pos, raw, 1.0, 3.0)
+            for a, b in ((images[k], image), (depths[k], depth), (alphas[k], alpha)):
+                assert torch.equal(a, b) if tile == 8 else torch.allclose(a, b, rtol=1e-5, atol=1e-5)
+        assert k == 1 or float(alpha.max()) > 0.1
