@@ -36,7 +36,7 @@ void count_launch();
 // around the launches of one pipeline stage on the stream they are issued to.
 enum Stage : int {
     STAGE_SAMPLE = 0,        // leaf weights, CDF, draws
-    STAGE_PREPROCESS = 1,    // visibility count, scan, project + SH
+    STAGE_PREPROCESS = 1,    // project + SH
     STAGE_SORT_DEPTH = 2,
     STAGE_INSTANCES = 3,     // per-point tile counts, scan, emission
     STAGE_SORT_TILE = 4,     // tile sort + ranges
@@ -143,12 +143,12 @@ struct KeyHistogram {
 // A kernel that makes the keys of a sort can count their digits too (count_key, finish_histogram below) and spare the sort its pass over the
 // keys: the histogram it fills, inside the workspace whose first sort_zero_bytes bytes have been cleared.  The sort is then called with `counted`.
 KeyHistogram key_histogram(void* workspace, int64_t n, int64_t n_likely, int end_bit);
-// Sorts the positions 0 .. n - 1 of the keys other than kNoKey and leaves how many there are in *count (device memory): the first pass
-// leaves the others out, so that whoever writes the keys need not compact them.  The workspace is sized for (n, n); the result is in the
+// Sorts the positions 0 .. n - 1 of the keys other than kNoKey: the first pass leaves the others out, so that whoever writes the keys need not compact them.  The
+// keys have been counted (key_histogram(workspace, n, n, end_bit)), how many there are is in *count (device memory).  The workspace is sized for (n, n); the result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd.  No key that takes part may equal kNoKey, also in bits above end_bit.
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
-int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
-                     bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream);
+int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, void* workspace,
+                     unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The same, and every point carries a code with it: the first pass makes it from the point's footprint word (see Footprint in raster.cu), and code and position go
 // through the other passes in one 64-bit word with the key bits that are still to be sorted by (the first pass's own are no longer needed), so that whoever
 // reads the sorted positions need not gather the words.  Sorted positions and codes land in the values and in the keys of the result buffers (the
@@ -161,8 +161,8 @@ struct CarriedCodes {
 // The codes for n points with keys of end_bit bits and words below `words`; none (bits == 0) where key bits behind the first pass, code and position do
 // not fit 64 bits.
 CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t words);
-int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes& codes,
-                                void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream);
+int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, const CarriedCodes& codes,
+                                void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for (n_max, n_likely).  The result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
@@ -321,9 +321,10 @@ __device__ __forceinline__ void count_key(BlockHistogram& h, const PassTable& pt
 
 // Every block of the launch, behind its last count: adds the block's counts to the launch's; the block that finishes last turns those into
 // digit bases (exclusive scans, all passes side by side: one round trip to memory and two barriers), which is a launch less.  *total, if
-// asked for, receives the number of keys.  Blocks of kRadix or 2 kRadix threads.
+// asked for, receives the number of keys.  Blocks of at least kRadix / 2 threads.
 __device__ __forceinline__ void finish_histogram(BlockHistogram& h, const KeyHistogram& out, unsigned n_blocks, unsigned long long* total) {
-    __shared__ unsigned s_sum[kMaxPasses][kRadix / 32];
+    constexpr unsigned kScanThreads = kRadix / 2, kScanWarps = kScanThreads / 32;   // two digits each
+    __shared__ unsigned s_sum[kMaxPasses][kScanWarps];
     __syncthreads();
     for (unsigned i = threadIdx.x; i < kMaxPasses * kRadix; i += blockDim.x) {
         const unsigned c = (&h[0][0])[i];
@@ -331,28 +332,32 @@ __device__ __forceinline__ void finish_histogram(BlockHistogram& h, const KeyHis
     }
     if (!last_block(out.blocks_done, n_blocks)) return;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
-    const bool scans = threadIdx.x < kRadix;
-    unsigned inc[kMaxPasses], own[kMaxPasses];
+    const bool scans = threadIdx.x < kScanThreads;
+    uint2 own[kMaxPasses];
+    unsigned inc[kMaxPasses];
     if (scans) {
 #pragma unroll
-        for (int p = 0; p < kMaxPasses; ++p) own[p] = p < out.pt.n_passes ? __ldcg(out.hist + p * kRadix + threadIdx.x) : 0u;
+        for (int p = 0; p < kMaxPasses; ++p) own[p] = p < out.pt.n_passes ? __ldcg(reinterpret_cast<const uint2*>(out.hist + p * kRadix) + threadIdx.x) : make_uint2(0u, 0u);
 #pragma unroll
         for (int p = 0; p < kMaxPasses; ++p) {
-            inc[p] = warp_inclusive_scan(own[p]);
+            inc[p] = warp_inclusive_scan(own[p].x + own[p].y);
             if (lane == 31) s_sum[p][warp] = inc[p];
         }
     }
     __syncthreads();
     if (warp < (unsigned)kMaxPasses) {
-        const unsigned sum = lane < kRadix / 32 ? s_sum[warp][lane] : 0u, before = warp_inclusive_scan(sum) - sum;
-        if (lane < kRadix / 32) s_sum[warp][lane] = before;
-        if (total && warp == 0 && lane == kRadix / 32 - 1) *total = before + sum;
+        const unsigned sum = lane < kScanWarps ? s_sum[warp][lane] : 0u, before = warp_inclusive_scan(sum) - sum;
+        if (lane < kScanWarps) s_sum[warp][lane] = before;
+        if (total && warp == 0 && lane == kScanWarps - 1) *total = before + sum;
     }
     __syncthreads();
     if (scans) {
 #pragma unroll
         for (int p = 0; p < kMaxPasses; ++p)
-            if (p < out.pt.n_passes) out.base[p * kRadix + threadIdx.x] = s_sum[p][warp] + inc[p] - own[p];
+            if (p < out.pt.n_passes) {
+                const unsigned second = s_sum[p][warp] + inc[p] - own[p].y;
+                reinterpret_cast<uint2*>(out.base + p * kRadix)[threadIdx.x] = make_uint2(second - own[p].x, second);
+            }
     }
 }
 

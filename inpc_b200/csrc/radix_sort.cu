@@ -39,10 +39,8 @@ constexpr int kHistItemsPerBlock = kHistThreads * 4 * 8;   // 8 uint4 loads per 
 // measured the same on B200 -- whole sort of 2^23 pairs, 32 / 27 / 24 key bits: 316 / 271 / 241 us against
 // 314 / 267 / 239 us with the plain 16-byte loads below; 2^25 pairs, 25 bits: 794 against 799 us.
 // The block that finishes last turns the counts of every pass into digit bases (exclusive scans): no launch of its own.
-// MARKED: keys of kNoKey are left out, and *count_out receives the number of the others.
-template <bool MARKED>
 __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
-    const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, KeyHistogram out, unsigned long long* __restrict__ count_out) {
+    const uint32_t* __restrict__ keys, int64_t n_arg, const unsigned long long* __restrict__ n_dev, KeyHistogram out) {
     await_previous_kernel();
     const int64_t n = n_dev ? (int64_t)*n_dev : n_arg;
     if ((int64_t)blockIdx.x * kHistItemsPerBlock >= n) return;
@@ -50,9 +48,7 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
     clear_histogram(s_hist);
     __syncthreads();
 
-    auto count = [&](uint32_t k) {
-        if (!MARKED || k != kNoKey) count_key(s_hist, out.pt, k);
-    };
+    auto count = [&](uint32_t k) { count_key(s_hist, out.pt, k); };
     for (int64_t block_base = (int64_t)blockIdx.x * kHistItemsPerBlock; block_base < n; block_base += (int64_t)gridDim.x * kHistItemsPerBlock) {
         const int64_t block_end = min(n, block_base + (int64_t)kHistItemsPerBlock);
         // keys is 16-byte aligned (carved at 256 bytes) and block_base is a multiple of 4
@@ -65,7 +61,7 @@ __global__ void __launch_bounds__(kHistThreads) radix_histogram_kernel(
         for (int64_t i = block_base + (int64_t)n_vec * 4 + threadIdx.x; i < block_end; i += kHistThreads) count(keys[i]);
     }
     const int64_t all = ceil_div<int64_t>(n, kHistItemsPerBlock);
-    finish_histogram(s_hist, out, (unsigned)min(all, (int64_t)gridDim.x), MARKED ? count_out : nullptr);
+    finish_histogram(s_hist, out, (unsigned)min(all, (int64_t)gridDim.x), nullptr);
 }
 
 // ---- one pass ---------------------------------------------------------------------------------
@@ -492,7 +488,7 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 // `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
                            int items, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
-                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, unsigned long long* marked_count = nullptr, bool counted = false, const CarriedCodes* codes = nullptr) {
+                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, const unsigned long long* marked_count = nullptr, bool counted = false, const CarriedCodes* codes = nullptr) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
 
@@ -505,7 +501,7 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
     if (!counted) {
         const int64_t hist_blocks = ceil_div<int64_t>(n, kHistItemsPerBlock), hist_cap = (int64_t)sm_count() * 4;
         const unsigned hist_grid = (unsigned)(hist_blocks < hist_cap ? hist_blocks : hist_cap);
-        launch_chained(marked_count ? radix_histogram_kernel<true> : radix_histogram_kernel<false>, hist_grid, kHistThreads, 0, stream, keys, n, n_dev, histogram_of(w, end_bit), marked_count);
+        launch_chained(radix_histogram_kernel, hist_grid, kHistThreads, 0, stream, keys, n, n_dev, histogram_of(w, end_bit));
         INPC_LAUNCH_CHECK("radix_histogram_kernel");
     }
 
@@ -545,17 +541,6 @@ int sort_pairs(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* v
                            0xFFFFFFFFu, nullptr, position_values, nullptr, counted);
 }
 
-int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
-                     bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream) {
-    if (result_in_alt) *result_in_alt = 0;
-    bool nothing = false;
-    const int rc = check_sort_args("sort_marked_keys", keys, keys_alt, values, values_alt, n < 2 ? 2 : n, end_bit, &nothing);
-    if (rc != INPC_OK) return rc;
-    if (n < 1 || nothing || !workspace || !count) { set_error("sort_marked_keys: needs keys, key bits, a workspace and a place for the count"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_marked_keys", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
-                           0xFFFFFFFFu, nullptr, true, count);
-}
-
 CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t words) {
     CarriedCodes c;
     if (n < 1 || end_bit < 1 || end_bit > 32 || words < 1 || words > (int64_t)1 << 30) return c;
@@ -569,15 +554,29 @@ CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t
     return c;
 }
 
-int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes& codes,
-                                void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream) {
+// (one pair is sorted like more: how many take part is not known here)
+static int sort_marked(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, const CarriedCodes* codes,
+                       void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream) {
     if (result_in_alt) *result_in_alt = 0;
     bool nothing = false;
     const int rc = check_sort_args("sort_marked_keys", keys, keys_alt, values, values_alt, n < 2 ? 2 : n, end_bit, &nothing);
     if (rc != INPC_OK) return rc;
-    if (nothing || !workspace || !count || !codes.quad || codes.bits < 1 || sort_pass_count(end_bit) < 2) { set_error("sort_marked_keys: needs keys and codes that fit, a workspace and a place for the count"); return INPC_E_INVALID; }
-    return sort_pairs_with("sort_marked_keys", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, zeroed, status, result_in_alt, stream, kSpinLimit,
-                           0xFFFFFFFFu, nullptr, true, count, false, &codes);
+    if (n < 1 || nothing || !workspace || !count || (codes && (!codes->quad || codes->bits < 1 || sort_pass_count(end_bit) < 2))) {
+        set_error("sort_marked_keys: needs keys, key bits, a workspace, the count and codes that fit");
+        return INPC_E_INVALID;
+    }
+    return sort_pairs_with("sort_marked_keys", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, true, status, result_in_alt, stream, kSpinLimit,
+                           0xFFFFFFFFu, nullptr, true, count, true, codes);
+}
+
+int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, void* workspace,
+                     unsigned* status, int* result_in_alt, cudaStream_t stream) {
+    return sort_marked(keys, keys_alt, values, values_alt, n, count, end_bit, nullptr, workspace, status, result_in_alt, stream);
+}
+
+int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, const CarriedCodes& codes,
+                                void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream) {
+    return sort_marked(keys, keys_alt, values, values_alt, n, count, end_bit, &codes, workspace, status, result_in_alt, stream);
 }
 
 // The same sort with the number of pairs in device memory (*n_dev <= n_max): grids and the look-back state are

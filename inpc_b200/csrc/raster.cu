@@ -5,15 +5,13 @@
 //   per point   : PointRec 32 B {screen x, screen y, opacity, depth | 4 view-space feature channels}
 //                 (one 32-byte sector per gather in the blend), tile bounds 8 B or, bilinear on 8x8 tiles, a packed
 //                 footprint of 4 B that they follow from, conic 16 B (gaussian)
-//                 depth key + point id, ping-pong pair for the depth sort: of the visible points side by side or, bilinear on 8x8
-//                 tiles, of every point where it lies, culled ones marked
+//                 depth key + point id, ping-pong pair for the depth sort: the key of every point where it lies, culled ones marked
 //   per instance: tile key + point id, ping-pong pair for the tile sort
 //   per tile    : [first, last+1) instance range
 //
 // The arithmetic follows the reference kernels expression by expression (cited per function, paths
 // below INPCCudaBackend/INPCCudaBackend/rasterization/ of the reference); the organisation of the
-// work does not: culled points are left out by the first pass of the depth sort (bilinear on 8x8 tiles) or by a deterministic
-// two-pass scan instead of atomics, the sorts are the library's own onesweep, and the bilinear blend walks per-pixel bit masks of the staged batch
+// work does not: culled points are left out by the first pass of the depth sort instead of compacted by atomics, the sorts are the library's own onesweep, and the bilinear blend walks per-pixel bit masks of the staged batch
 // instead of testing every staged point against every pixel.
 #include "common.cuh"
 
@@ -98,10 +96,10 @@ struct W2C {
     float r0[4], r1[4], r2[4];
 };
 
-__device__ __forceinline__ W2C load_w2c(const float* __restrict__ w2c) {
+__device__ __forceinline__ W2C load_w2c(const float* w2c) {
     W2C m;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { m.r0[k] = __ldg(w2c + k); m.r1[k] = __ldg(w2c + 4 + k); m.r2[k] = __ldg(w2c + 8 + k); }
+    for (int k = 0; k < 4; ++k) { m.r0[k] = w2c[k]; m.r1[k] = w2c[4 + k]; m.r2[k] = w2c[8 + k]; }
     return m;
 }
 
@@ -252,105 +250,8 @@ __device__ __forceinline__ unsigned scan_words(unsigned* data, int64_t n, unsign
 }
 
 constexpr int kPreThreads = 256;
+constexpr int projection_blocks(int mode) { return mode == INPC_MODE_GAUSSIAN ? 5 : 6; }   // per multiprocessor, see preprocess_kernel
 constexpr unsigned kCountShift = 30;   // bilinear: (tiles touched - 1) in key bits 30..31 when the depth offsets fit below
-
-// Pass 1 of the deterministic compaction: per chunk of kPreThreads points, how many points survive culling, and how many
-// (point, tile) instances there are in all.  The last block scans the counts of the groups of 4 chunks (group_visible and
-// *instances start at zero) and leaves the totals in counters[0] (visible) and counters[1] (instances), the range of depth bit
-// patterns the keys are offsets into in counters[2..3] and *depth_min, *depth_max (the words of `range` start
-// at zero and collect the largest pattern and the largest complement).  Only where the host needs the counts: see the projection pass.
-//
-// Bound by the instructions of the projection (96 per point; 33 % of DRAM).  Every lane takes 4 consecutive points (three 16-byte
-// loads when the array is aligned), a warp a chunk in two steps, the positions of the next step travelling while this one's are
-// projected; nothing waits for other warps before the last block's scan.  2^23 / 2^25 points 36 / 129 us
-// (one block per group with its fence and atomic 62 / 226; persistent blocks with a barrier per group 44 / 154, with the
-// positions loaded ahead 39 / 144).
-template <int MODE, int VARIANT>
-__global__ void __launch_bounds__(kPreThreads, 4) visibility_count_kernel(
-    const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_chunks, unsigned* __restrict__ block_visible,
-    unsigned* group_visible, unsigned long long* instances, unsigned* range, unsigned* done,
-    unsigned* __restrict__ depth_min, unsigned* __restrict__ depth_max, unsigned long long* __restrict__ counters) {
-    await_previous_kernel();
-    constexpr int kPerThread = 4;
-    constexpr unsigned kStep = 32 * kPerThread;        // points of a warp and step
-    static_assert(kPreThreads == 2 * kStep, "a chunk is two steps");
-    const W2C m = load_w2c(rp.v.w2c);
-    unsigned lo = 0xFFFFFFFFu, hi = 0u;
-    unsigned long long inst = 0;
-    // the positions of this lane's points of a step, zeros behind the end of their set; returns how many points there are
-    auto load_step = [&](unsigned step, float (&p)[3 * kPerThread], int& set, int64_t& first) -> int {
-        // indices are local to the step's set
-        set = set_of_block(ps, (int64_t)step * kStep);
-        const float* __restrict__ positions = ps.positions[set];
-        const int64_t n = ps.size[set];
-        first = (int64_t)step * kStep + lane_id() * kPerThread - ps.start[set];
-        if (first + kPerThread <= n && (reinterpret_cast<uintptr_t>(positions) & 15u) == 0) {
-            const float4* src = reinterpret_cast<const float4*>(positions + 3 * first);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float4 v = __ldg(src + k);
-                p[4 * k] = v.x; p[4 * k + 1] = v.y; p[4 * k + 2] = v.z; p[4 * k + 3] = v.w;
-            }
-            return kPerThread;
-        }
-#pragma unroll
-        for (int k = 0; k < 3 * kPerThread; ++k) p[k] = first * 3 + k < 3 * n ? __ldg(positions + 3 * first + k) : 0.0f;
-        return (int)max((int64_t)0, min((int64_t)kPerThread, n - first));
-    };
-    const unsigned n_warps = gridDim.x * (kPreThreads / 32);
-    unsigned chunk = blockIdx.x * (kPreThreads / 32) + (threadIdx.x >> 5);
-    float next[3 * kPerThread];
-    int next_set = 0, next_here = 0;
-    int64_t next_first = 0;
-    if (chunk < n_chunks) next_here = load_step(2u * chunk, next, next_set, next_first);
-    for (; chunk < n_chunks; chunk += n_warps) {
-        unsigned v = 0;
-#pragma unroll 1
-        for (unsigned half = 0; half < 2u; ++half) {
-            float p[3 * kPerThread];
-#pragma unroll
-            for (int k = 0; k < 3 * kPerThread; ++k) p[k] = next[k];
-            const int set = next_set, here = next_here;
-            const int64_t first = next_first;
-            const unsigned following = half == 0u ? chunk : chunk + n_warps;
-            if (following < n_chunks) next_here = load_step(2u * following + (half ^ 1u), next, next_set, next_first);
-#pragma unroll
-            for (int k = 0; k < kPerThread; ++k) {
-                if (k < here) {
-                    const Projection pr = project_point<MODE, VARIANT>(p[3 * k], p[3 * k + 1], p[3 * k + 2], m, rp, first + k, set);
-                    if (pr.visible) {
-                        v += 1u;
-                        inst += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
-                        const unsigned bits = __float_as_uint(pr.depth);   // visible depths are positive: bit patterns order like the values
-                        lo = min(lo, bits);
-                        hi = max(hi, bits);
-                    }
-                }
-            }
-        }
-        v = __reduce_add_sync(0xffffffffu, v);
-        if (lane_id() == 0) {
-            block_visible[chunk] = v;
-            if (v) atomicAdd(group_visible + (chunk >> 2), v);   // the scan runs over groups, four times fewer entries
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, o);
-    if (lane_id() == 0 && inst) atomicAdd(instances, inst);
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if (lane_id() == 0 && lo <= hi) { atomicMax(range, ~lo); atomicMax(range + 1, hi); }
-    if (!last_block(done, gridDim.x)) return;
-    __shared__ unsigned s_scan[kPreThreads / 32 + 1];
-    const unsigned visible = scan_words<kPreThreads>(group_visible, (n_chunks + 3u) / 4u, s_scan);
-    if (threadIdx.x == 0) {
-        const unsigned first_key = ~__ldcg(range), last_key = __ldcg(range + 1);
-        counters[0] = visible;
-        counters[1] = __ldcg(instances);
-        counters[2] = *depth_min = first_key;
-        counters[3] = *depth_max = last_key;
-    }
-}
 
 constexpr int kScanThreads = 1024;
 
@@ -374,10 +275,40 @@ __device__ __forceinline__ void sh_basis(const float px, const float py, const f
     b[8] = 0.54627421529603959f * xx - 0.54627421529603959f * yy;
 }
 
-__device__ __forceinline__ float sh_eval_channel(const float* b, const __half* h, int c) {
-    return b[0] * __half2float(h[c]) - b[1] * __half2float(h[4 + c]) + b[2] * __half2float(h[8 + c]) -
-           b[3] * __half2float(h[12 + c]) + b[4] * __half2float(h[16 + c]) - b[5] * __half2float(h[20 + c]) +
-           b[6] * __half2float(h[24 + c]) - b[7] * __half2float(h[28 + c]) + b[8] * __half2float(h[32 + c]);
+// One point's 36 coefficients from the shared slab, four channels of a coefficient at a time.  ODD (rows of 37 halves, the first of which is the raw opacity): the
+// coefficients begin at a multiple of four bytes in every second row only, so whole words are read and shifted by half a word in the others.  (Rows of 36: nine 8-byte
+// loads that meet every bank once, where 36 loads of a half took four times the wavefronts.)
+template <bool ODD>
+__device__ __forceinline__ void sh_eval(const float* b, const unsigned char* slab, unsigned row, float* f, float* raw_opacity) {
+    unsigned carry = 0u;
+    const unsigned char* p = slab + row * (ODD ? 74u : 72u);
+    const bool half_word = ODD && (row & 1u) == 0u;   // the coefficients begin in the middle of a word
+    if (ODD) {
+        const unsigned first = *reinterpret_cast<const unsigned*>(p - (half_word ? 0u : 2u));
+        *raw_opacity = __half2float(__ushort_as_half((unsigned short)(half_word ? first : first >> 16)));
+        carry = first;
+        p += half_word ? 4u : 2u;
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        uint2 w;
+        if (ODD) {
+            const unsigned* q = reinterpret_cast<const unsigned*>(p) + 2 * k;
+            const unsigned w0 = q[0], w1 = q[1];
+            w = half_word ? make_uint2(__funnelshift_r(carry, w0, 16), __funnelshift_r(w0, w1, 16)) : make_uint2(w0, w1);
+            carry = w1;
+        } else {
+            w = reinterpret_cast<const uint2*>(p)[k];
+        }
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+        const float h[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (k == 0) f[c] = b[0] * h[c];
+            else if (k & 1) f[c] = f[c] - b[k] * h[c];
+            else f[c] = f[c] + b[k] * h[c];
+        }
+    }
 }
 
 // What the instance emission of the warp blend needs of a bilinear splat, in one word: 4 bytes per point keep the array (33 MB for 2^23 points) resident
@@ -440,134 +371,127 @@ __device__ __forceinline__ uint4 pack_footprint(const Projection& pr, float reac
     return make_uint4(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16), inset, 0u);
 }
 
-// Project (pass 2 of the compaction projects again: same arithmetic, same outcome), evaluate SH, write the point record and bounds, and the depth key.
+// Project, evaluate SH, write the point record, what the instance passes need of the splat, and the depth key, all of it where the point lies: the key of a culled
+// point is kNoKey, and the depth sort leaves it out, so that nothing is compacted.
 // src/bilinear/kernels.cu:11-84, :106-184; src/gaussian/kernels.cu:11-111, :113-217, :219-324.
-// COMPACT: key and point id of a visible point are appended at the slot given by the block offset plus the rank of the point
-// among the block's survivors: index order, hence reproducible.  Otherwise (bilinear on 8x8 tiles, counts left on the device) there was no pass 1: every point's key is
-// written where the point lies, that of a culled one is kNoKey, and the depth sort leaves it out (the base of the keys is known to the host then, and
-// neither the counts nor the depth range nor the point ids are used).
-template <int MODE, int VARIANT, bool COMPACT>
-__global__ void __launch_bounds__(kPreThreads) preprocess_kernel(
-    PointSets ps, RasterParams rp, const unsigned* __restrict__ block_visible, const unsigned* __restrict__ group_offset,
-    const unsigned* __restrict__ depth_min,
-    const unsigned* __restrict__ depth_max, unsigned key_base, PointRec* __restrict__ rec, uint2* __restrict__ bounds, uint32_t* __restrict__ quad,
-    float4* __restrict__ conic, uint4* __restrict__ foot, uint32_t* __restrict__ depth_keys,
-    uint32_t* __restrict__ point_ids, int pack_count, int rec_stride, volatile unsigned* status) {
+//
+// Persistent blocks take chunks of kPreThreads points; they count the digits of the keys for the depth sort (and so the visible points: *n_visible), and, where the host
+// wants to know, the (point, tile) instances (*n_instances, which starts at zero).  The pass is bound by DRAM (128 bytes per point) as long as enough copies are in
+// flight: six blocks of 40 registers (five of 48 where ellipses are formed), the matrix in shared memory, or they spill.  Against one block per chunk, a histogram of the keys of its
+// own and, where the host sizes the instance arrays, a pass that projected and counted first: 2^23 bilinear 156 + 19 -> 167 us, 2^25 of a cloud 598 + 51 -> 630, 2^22 gaussian
+// 119 + 36 + 13 -> 115, 2^23 feature rows 97 + 40 + 17 -> 91.  Four blocks of 63 registers with positions loaded and the next slab asked for ahead: 168 / 635 / 130; five blocks of the same with 80 bytes
+// spilled 200 / 760; eight of 32 registers, 44 bytes spilled, 178 / 653.
+template <int MODE, int VARIANT>
+__global__ void __launch_bounds__(kPreThreads, projection_blocks(MODE)) preprocess_kernel(
+    const __grid_constant__ PointSets ps, const __grid_constant__ RasterParams rp, unsigned n_chunks, unsigned key_base, PointRec* __restrict__ rec, uint2* __restrict__ bounds,
+    uint32_t* __restrict__ quad, float4* __restrict__ conic, uint4* __restrict__ foot, uint32_t* __restrict__ depth_keys, int pack_count, int rec_stride,
+    KeyHistogram digits, unsigned long long* n_visible, unsigned long long* n_instances, volatile unsigned* status) {
     await_previous_kernel();
     constexpr int kHalves = VARIANT == VAR_RAW37 ? 37 : 36;
     constexpr int kSlabBytes = VARIANT == VAR_ROWS ? 16 : kPreThreads * kHalves * 2;   // multiple of 16 for both layouts
     __shared__ __align__(16) unsigned char s_feat[kSlabBytes];
-    __shared__ unsigned s_scan[kPreThreads / 32 + 1];
-
-    // this block's set: the input arrays are indexed by the point's position in its set (i), everything this pass
-    // writes by its position in the virtual index space of the call (iv); the two coincide for a single set
-    const int64_t block_first_v = (int64_t)blockIdx.x * kPreThreads;
-    const int set = set_of_block(ps, block_first_v);
-    const float* __restrict__ positions = ps.positions[set];
-    const __half* __restrict__ features = static_cast<const __half*>(ps.features[set]);
-    const float* __restrict__ opacities = ps.opacities[set];
-    const int64_t n = ps.size[set];
-    const bool bulk_ok = (reinterpret_cast<uintptr_t>(features) & 15u) == 0;
-    const int64_t block_first = block_first_v - ps.start[set];
-    const int in_block = (int)max((int64_t)0, min((int64_t)kPreThreads, n - block_first));
+    __shared__ BlockHistogram s_digits;
     __shared__ __align__(8) unsigned long long s_bar;
-    // The block's feature slab is contiguous in global memory.  When base and size allow (multiples of
-    // 16 bytes) one bulk asynchronous copy brings it in while the threads project their points;
-    // otherwise (odd tail block, unaligned caller view) 16-byte loads through registers do.
-    const bool bulk = VARIANT != VAR_ROWS && bulk_ok && in_block > 0 && ((in_block * kHalves * 2) & 15) == 0;
-    if (bulk) {
-        if (threadIdx.x == 0) mbarrier_init(&s_bar, 1);
-        __syncthreads();
-        if (threadIdx.x == 0)
-            bulk_load_to_shared(s_feat, reinterpret_cast<const unsigned char*>(features) + block_first * (kHalves * 2),
-                                (unsigned)(in_block * kHalves * 2), &s_bar);
-    } else if (VARIANT != VAR_ROWS) {
-        // coalesced 16-byte staging of the block's contiguous feature slab
-        const unsigned char* src = reinterpret_cast<const unsigned char*>(features) + block_first * (kHalves * 2);
-        const int bytes = in_block * kHalves * 2;
-        const int n16 = bytes / 16;
-        const uint4* src16 = reinterpret_cast<const uint4*>(src);
-        uint4* dst16 = reinterpret_cast<uint4*>(s_feat);
-        for (int k = threadIdx.x; k < n16; k += kPreThreads) dst16[k] = __ldg(src16 + k);
-        for (int k = n16 * 16 + 2 * threadIdx.x; k < bytes; k += 2 * kPreThreads)
-            *reinterpret_cast<unsigned short*>(s_feat + k) = __ldg(reinterpret_cast<const unsigned short*>(src + k));
-    }
-    const W2C m = load_w2c(rp.v.w2c);
-    const int64_t i = block_first + threadIdx.x;
-    const int64_t iv = block_first_v + threadIdx.x;
-    Projection pr;
-    pr.visible = false;
-    float px = 0, py = 0, pz = 0;
-    if (i < n) {
-        px = __ldg(positions + 3 * i); py = __ldg(positions + 3 * i + 1); pz = __ldg(positions + 3 * i + 2);
-        pr = project_point<MODE, VARIANT>(px, py, pz, m, rp, i, set);
-    }
-    bool slab_ready = true;
-    if (bulk) slab_ready = mbarrier_wait_bounded(&s_bar, 0u);
-    if (!slab_ready && status) status[STATUS_BULK_COPY_TIMEOUT] = 1u;
+    __shared__ float s_w2c[12];
+    clear_histogram(s_digits);
+    if (threadIdx.x < 12u) s_w2c[threadIdx.x] = __ldg(rp.v.w2c + threadIdx.x);
+    if (VARIANT != VAR_ROWS && threadIdx.x == 0) mbarrier_init(&s_bar, 1);
     __syncthreads();
-    // what the instance passes need of a point: its packed footprint where splats are bilinear on 8x8 tiles, else its tile bounds
-    auto write_bounds = [&](bool visible) {
-        if (MODE == INPC_MODE_BILINEAR && quad) quad[iv] = visible ? pack_quad(pr, set * rp.gh, rp.gw) : kNoQuad;
-        else bounds[iv] = visible ? make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16)) : make_uint2(0u, 0u);
-    };
-    if (i >= n && iv < ps.start[ps.count]) write_bounds(false);   // padding behind a set
-    if (i < n && slab_ready) {
-        if (pr.visible && VARIANT == VAR_ROWS) {
-            // feature rows are gathered by the blend itself: the record carries the geometry only.  The warp blend reads such
-            // records 16 bytes apart (rec_stride 1): half-written 32-byte sectors cost as much DRAM traffic as whole ones
-            reinterpret_cast<float4*>(rec)[(size_t)iv * rec_stride] = make_float4(pr.sx, pr.sy, __ldg(opacities + i), pr.depth);
-            write_bounds(true);
-        } else if (pr.visible) {
-            const __half* h = reinterpret_cast<const __half*>(s_feat) + threadIdx.x * kHalves;
-            float b[9];
-            sh_basis(px, py, pz, rp.v.cam, b);
-            PointRec r;
-            r.sx = pr.sx; r.sy = pr.sy; r.depth = pr.depth;
-            if (VARIANT == VAR_RAW37) {
-                // opacity = 1 - exp(-exp(raw)) with the fast exponential: src/bilinear/kernels.cu:144
-                r.opacity = 1.0f - __expf(-__expf(__half2float(h[0])));
-                h += 1;
+    unsigned phase = 0u;
+    unsigned long long instances = 0ull;
+    bool slab_ready = true;
+    for (unsigned chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
+        // this chunk's set: the input arrays are indexed by the point's position in its set (i), everything this pass
+        // writes by its position in the virtual index space of the call (iv); the two coincide for a single set
+        const int64_t block_first_v = (int64_t)chunk * kPreThreads;
+        const int set = set_of_block(ps, block_first_v);
+        const float* __restrict__ positions = ps.positions[set];
+        const __half* __restrict__ features = static_cast<const __half*>(ps.features[set]);
+        const int64_t n = ps.size[set];
+        const int64_t block_first = block_first_v - ps.start[set];
+        const int in_block = (int)max((int64_t)0, min((int64_t)kPreThreads, n - block_first));
+        // The chunk's feature slab is contiguous in global memory.  When base and size allow (multiples of
+        // 16 bytes) one bulk asynchronous copy brings it in while the threads project their points;
+        // otherwise loads through registers do, of 16 bytes (odd last chunk) or 2 (caller view that is not aligned).
+        const bool aligned = (reinterpret_cast<uintptr_t>(features) & 15u) == 0;
+        const bool bulk = VARIANT != VAR_ROWS && slab_ready && aligned && in_block > 0 && ((in_block * kHalves * 2) & 15) == 0;
+        if (bulk) {
+            if (threadIdx.x == 0)
+                bulk_load_to_shared(s_feat, reinterpret_cast<const unsigned char*>(features) + block_first * (kHalves * 2), (unsigned)(in_block * kHalves * 2), &s_bar);
+        } else if (VARIANT != VAR_ROWS) {
+            const unsigned char* src = reinterpret_cast<const unsigned char*>(features) + block_first * (kHalves * 2);
+            const int bytes = in_block * kHalves * 2;
+            const int n16 = aligned ? bytes / 16 : 0;
+            const uint4* src16 = reinterpret_cast<const uint4*>(src);
+            uint4* dst16 = reinterpret_cast<uint4*>(s_feat);
+            for (int k = threadIdx.x; k < n16; k += kPreThreads) dst16[k] = __ldg(src16 + k);
+            for (int k = n16 * 16 + 2 * threadIdx.x; k < bytes; k += 2 * kPreThreads)
+                *reinterpret_cast<unsigned short*>(s_feat + k) = __ldg(reinterpret_cast<const unsigned short*>(src + k));
+            fence_shared_for_bulk();   // a bulk copy may overwrite the slab in the next round
+        }
+        const int64_t i = block_first + threadIdx.x;
+        const int64_t iv = block_first_v + threadIdx.x;
+        Projection pr;
+        pr.visible = false;
+        float px = 0, py = 0, pz = 0;
+        if (i < n) {
+            px = __ldg(positions + 3 * i); py = __ldg(positions + 3 * i + 1); pz = __ldg(positions + 3 * i + 2);
+            pr = project_point<MODE, VARIANT>(px, py, pz, load_w2c(s_w2c), rp, i, set);
+        }
+        if (bulk) {
+            slab_ready = mbarrier_wait_bounded(&s_bar, phase);
+            phase ^= 1u;
+            if (!slab_ready && status) status[STATUS_BULK_COPY_TIMEOUT] = 1u;
+        } else if (VARIANT != VAR_ROWS) {
+            __syncthreads();
+        }
+        if (!slab_ready) pr.visible = false;   // the results are invalid, and reported so, but everything behind this pass finds keys and words that it can read
+        if (pr.visible) {
+            float4* const dst = reinterpret_cast<float4*>(rec) + (VARIANT == VAR_ROWS ? (size_t)iv * rec_stride : 2 * (size_t)iv);
+            if (VARIANT == VAR_ROWS) {
+                // feature rows are gathered by the blend itself: the record carries the geometry only.  The warp blend reads such
+                // records 16 bytes apart (rec_stride 1): half-written 32-byte sectors cost as much DRAM traffic as whole ones
+                dst[0] = make_float4(pr.sx, pr.sy, __ldg(ps.opacities[set] + i), pr.depth);
             } else {
-                r.opacity = __ldg(opacities + i);
+                float b[9];
+                sh_basis(px, py, pz, rp.v.cam, b);
+                float opacity, f[4];
+                sh_eval<VARIANT == VAR_RAW37>(b, s_feat, threadIdx.x, f, &opacity);
+                // opacity = 1 - exp(-exp(raw)) with the fast exponential: src/bilinear/kernels.cu:144
+                if (VARIANT == VAR_RAW37) opacity = 1.0f - __expf(-__expf(opacity));
+                else opacity = __ldg(ps.opacities[set] + i);
+                dst[0] = make_float4(pr.sx, pr.sy, opacity, pr.depth);
+                dst[1] = make_float4(f[0], f[1], f[2], f[3]);
             }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) r.f[c] = sh_eval_channel(b, h, c);
-            float4* dst = reinterpret_cast<float4*>(rec + iv);
-            dst[0] = make_float4(r.sx, r.sy, r.opacity, r.depth);
-            dst[1] = make_float4(r.f[0], r.f[1], r.f[2], r.f[3]);
-            write_bounds(true);
             if (MODE == INPC_MODE_GAUSSIAN) {
                 conic[iv] = make_float4(pr.cx, pr.cy, pr.cz, 0.0f);
                 if (foot) foot[iv] = pack_footprint(pr, rp.reach);
             }
-        } else {
-            write_bounds(false);
+            if (n_instances) instances += (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
         }
+        if (iv < ps.start[ps.count]) {   // (also the padding behind a set)
+            // what the instance passes need of a point: its packed footprint where splats are bilinear on 8x8 tiles, else its tile bounds
+            if (MODE == INPC_MODE_BILINEAR && quad) quad[iv] = pr.visible ? pack_quad(pr, set * rp.gh, rp.gw) : kNoQuad;
+            else bounds[iv] = pr.visible ? make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16)) : make_uint2(0u, 0u);
+            // sort key: offset of the depth's bit pattern from the smallest there can be (fewer radix passes).
+            // A bilinear splat touches 1, 2 or 4 tiles; when the offsets leave the two top bits free that count rides there (the
+            // sort ignores bits above its range and carries them along), which saves the instance pass a gather.
+            uint32_t key = kNoKey;
+            if (pr.visible) {
+                key = __float_as_uint(pr.depth) - key_base;
+                count_key(s_digits, digits.pt, key);
+                if (MODE == INPC_MODE_BILINEAR && pack_count) key |= ((pr.x1 - pr.x0) * (pr.y1 - pr.y0) - 1u) << kCountShift;
+            }
+            depth_keys[iv] = key;
+        }
+        if (VARIANT != VAR_ROWS) slab_ready = !__syncthreads_or(!slab_ready);   // everybody has read the slab
     }
-    // sort key: offset of the depth's bit pattern from the smallest there can be (fewer radix passes).
-    // A bilinear splat touches 1, 2 or 4 tiles; when the offsets leave the two top bits free that
-    // count rides there (the sort ignores bits above its range and carries them along), which
-    // saves the instance pass a gather.
-    // pack_count: 1 yes, 0 no (the host knows a bound on the offsets), -1 decide from the measured depth range
-    auto depth_key = [&](unsigned lo) -> unsigned {
-        const unsigned key = __float_as_uint(pr.depth) - lo;
-        const bool pack = pack_count >= 0 ? pack_count != 0 : __ldg(depth_max) - lo < (1u << kCountShift);
-        return MODE == INPC_MODE_BILINEAR && pack ? key | (((pr.x1 - pr.x0) * (pr.y1 - pr.y0) - 1u) << kCountShift) : key;
-    };
-    if (!COMPACT) {
-        if (iv < ps.start[ps.count]) depth_keys[iv] = pr.visible ? depth_key(key_base) : kNoKey;
-        return;
+    if (n_instances) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) instances += __shfl_down_sync(0xffffffffu, instances, o);
+        if (lane_id() == 0 && instances) atomicAdd(n_instances, instances);
     }
-    unsigned total;
-    const unsigned rank = block_exclusive_scan(pr.visible ? 1u : 0u, s_scan, &total);
-    if (pr.visible) {
-        // slot = survivors of all groups before + of the earlier chunks of this group + rank in this chunk
-        unsigned slot = __ldg(group_offset + (blockIdx.x >> 2)) + rank;
-        for (unsigned c = blockIdx.x & ~3u; c < blockIdx.x; ++c) slot += __ldg(block_visible + c);
-        depth_keys[slot] = depth_key(__ldg(depth_min));
-        point_ids[slot] = (uint32_t)iv;
-    }
+    finish_histogram(s_digits, digits, gridDim.x, n_visible);
 }
 
 __device__ __forceinline__ unsigned tiles_of(const uint2 b) {
@@ -745,7 +669,7 @@ struct EmitCodedSmem {
     uint2 pairs[kCodedThreads / 32][32 * kCodedPoints * 4];   // the most a warp's points can make
 };
 __global__ void __launch_bounds__(kCodedThreads, kCodedBlocks) emit_coded_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ sorted_codes, const CarriedCodes codes,
-                                                                      const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
+                                                                      int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
                                                                       KeyHistogram digits, unsigned long long* __restrict__ n_emitted, uint32_t* __restrict__ inst_keys,
                                                                       uint32_t* __restrict__ inst_ids) {
     await_previous_kernel();
@@ -755,7 +679,7 @@ __global__ void __launch_bounds__(kCodedThreads, kCodedBlocks) emit_coded_kernel
     EmitCodedSmem& s_stage = *reinterpret_cast<EmitCodedSmem*>(smem_raw);
     __shared__ unsigned s_total[2][kWarps];   // of two groups in turn, so that one barrier does
     __shared__ BlockHistogram s_digits;
-    const unsigned n_visible = (unsigned)*n_visible_dev, n_groups = (n_visible + kGroup - 1u) / kGroup;
+    const unsigned n_visible = n_visible_dev ? (unsigned)*n_visible_dev : (unsigned)n_visible_arg, n_groups = (n_visible + kGroup - 1u) / kGroup;   // < 2^30
     if (blockIdx.x >= n_groups) return;
     clear_histogram(s_digits);
     __syncthreads();
@@ -3953,15 +3877,11 @@ struct PointBlob {
     uint32_t* quad;                       // bilinear, warp blend: packed footprint origin per point (see pack_quad), else none
     float4* conic;
     uint4* foot;                          // gaussian, warp blend: tile bounds and ellipse per point (see pack_footprint)
-    unsigned* block_visible;              // survivors per chunk of kPreThreads points
-    unsigned* group_visible;              // per group of 4 chunks; scanned in place
-    unsigned long long* counters;   // visible, instances, smallest / largest depth bit pattern; deferred: visible, instances, instances emitted
-    unsigned* depth_min;
-    unsigned* depth_max;
     uint32_t* keys[2];
     uint32_t* ids[2];
     unsigned* inst_block_sums;
-    unsigned* state;                      // words that start at zero: [0..1] depth range, [2..4] finished blocks of the counting passes, [8..9] instances
+    unsigned* state;                      // words that start at zero: [0] finished blocks of the instance count, then
+    unsigned long long* counters;         // visible, instances; deferred: instances emitted
     void* sort_ws;                        // directly behind `state`: cleared together
     size_t total;
 };
@@ -3975,22 +3895,17 @@ bool uses_warp_blend(int tile) { return tile == 8; }
 PointBlob carve_point_blob(void* p, int64_t n, int mode, int tile) {
     PointBlob b;
     Carver c(p);
-    const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
     b.rec = c.take<PointRec>(n);
     const bool quads = mode == INPC_MODE_BILINEAR && uses_warp_blend(tile);
     b.bounds = quads ? nullptr : c.take<uint2>(n);
     b.quad = quads ? c.take<uint32_t>(n) : nullptr;
     b.conic = mode == INPC_MODE_GAUSSIAN ? c.take<float4>(n) : nullptr;
     b.foot = mode == INPC_MODE_GAUSSIAN && uses_warp_blend(tile) ? c.take<uint4>(n) : nullptr;
-    b.block_visible = c.take<unsigned>(nb);
-    b.group_visible = c.take<unsigned>(ceil_div<int64_t>(nb, 4));
-    b.counters = c.take<unsigned long long>(4);
-    b.depth_min = c.take<unsigned>(1);
-    b.depth_max = c.take<unsigned>(1);
     for (int k = 0; k < 2; ++k) b.keys[k] = c.take<uint32_t>(n);
     for (int k = 0; k < 2; ++k) b.ids[k] = c.take<uint32_t>(n);
     b.inst_block_sums = c.take<unsigned>(ceil_div<int64_t>(n > 0 ? n : 1, kInstThreads));
     b.state = c.take<unsigned>(64);
+    b.counters = reinterpret_cast<unsigned long long*>(b.state + 16);
     c.off = align_up(c.off);
     b.sort_ws = c.base + c.off;
     c.off += sort_workspace_bytes(n, n);
@@ -4091,7 +4006,6 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, bool deferred, in
 
 // The state handed back to the caller only stores blob bases and counts; which ping-pong buffer holds
 // a sorted result follows from the number of radix passes, which follows from the counts.
-int depth_result_buffer(int64_t n_visible, int depth_key_bits) { return n_visible > 1 ? (sort_pass_count(depth_key_bits) & 1) : 0; }
 int tile_result_buffer(int64_t n_instances, int n_tiles) {
     const int end_bit = bit_length((uint32_t)(n_tiles - 1));
     return n_instances > 1 ? (sort_pass_count(end_bit) & 1) : 0;
@@ -4104,10 +4018,7 @@ int tile_buffer_of(const inpc_raster_state* st, int n_tiles) {
     if (st->deferred_counts & 1) return sort_pass_count(bit_length((uint32_t)(n_tiles - 1))) & 1;
     return tile_result_buffer(st->n_instances, n_tiles);
 }
-int depth_buffer_of(const inpc_raster_state* st) {
-    if (st->deferred_counts & 1) return sort_pass_count(st->depth_key_bits) & 1;
-    return depth_result_buffer(st->n_visible, st->depth_key_bits);
-}
+int depth_buffer_of(const inpc_raster_state* st) { return sort_pass_count(st->depth_key_bits) & 1; }
 
 cudaEvent_t counters_event() {
     static thread_local cudaEvent_t events[kMaxDevices] = {nullptr};
@@ -4209,7 +4120,6 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     unsigned* status = acquire_status(entry);
     if (!status) return INPC_E_CUDA;
     const bool warp_blend = uses_warp_blend(rp.tile);
-    const int64_t nb = ceil_div<int64_t>(n > 0 ? n : 1, kPreThreads);
     const PointBlob sizing = carve_point_blob(nullptr, n, MODE, rp.tile);
     void* pblob = alloc_point(user, sizing.total);
     if (!pblob) { set_error("point allocator returned NULL for %zu bytes", sizing.total); return INPC_E_ALLOC; }
@@ -4225,9 +4135,21 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     // paths (gaussian splats have no such bound, feature rows keep their scratch small) read the counts back once.
     const bool deferred = defers_counts(MODE, rp.tile, VARIANT == VAR_ROWS, n, stream);
     int64_t n_visible = 0, n_instances = 0;
-    uint32_t key_base = 0;
-    int key_bits = 0;
+    // depth keys are offsets from the near plane's bit pattern, bounded by the far plane's: nothing is measured
+    const float near_depth = rp.v.near_plane > 0.0f ? rp.v.near_plane : 0.0f, far_depth = rp.v.far_plane > near_depth ? rp.v.far_plane : near_depth;
+    uint32_t key_base, last_key;
+    memcpy(&key_base, &near_depth, 4);
+    memcpy(&last_key, &far_depth, 4);
+    if (!(rp.v.near_plane > 0.0f)) { key_base = 0u; last_key = 0xFFFFFFFFu; }
+    int key_bits = bit_length(last_key - key_base);
+    if (key_bits == 0) key_bits = 1;
+    // with offsets of up to 2^30 - 1, a splat of four tiles at the far plane would have the key of a culled point
+    if (key_bits == (int)kCountShift && last_key - key_base == (1u << kCountShift) - 1u) ++key_bits;
+    const bool counts_in_keys = MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift;
     const int tile_bits = bit_length((uint32_t)(n_tiles - 1));
+    CarriedCodes codes;   // the depth sort carries the footprints along where they fit
+    if (MODE == INPC_MODE_BILINEAR && warp_blend) codes = carried_codes(pb.quad, n, key_bits, (int64_t)n_tiles * 64);
+    const bool carried = codes.bits > 0;
     void* iblob = nullptr;
     InstanceBlob ib;
     auto make_instance_blob = [&]() -> int {
@@ -4241,26 +4163,13 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         list.add(ib.n_segments, (size_t)(static_cast<char*>(ib.sort_ws) - reinterpret_cast<char*>(ib.n_segments)) +
                                     sort_zero_bytes(n_instances, likely_instances(n_instances, deferred), tile_bits));
     };
-    int rc;
+    int rc, in_alt = 0;
     const unsigned long long* n_visible_dev = deferred ? pb.counters : nullptr;
     const unsigned long long* n_instances_dev = deferred ? pb.counters + 1 : nullptr;
     if (n > 0) {
         unsigned long long* host = nullptr;
         cudaEvent_t ready = nullptr;
-        int pack_count = -1;
-        uint32_t lo_bits = 0u, hi_bits = 0u;
         if (deferred) {
-            // depth keys are offsets from the near plane's bit pattern, bounded by the far plane's: nothing is measured
-            const float lo = rp.v.near_plane > 0.0f ? rp.v.near_plane : 0.0f, hi = rp.v.far_plane > lo ? rp.v.far_plane : lo;
-            memcpy(&lo_bits, &lo, 4);
-            memcpy(&hi_bits, &hi, 4);
-            if (!(rp.v.near_plane > 0.0f)) { lo_bits = 0u; hi_bits = 0xFFFFFFFFu; }
-            key_bits = rp.v.near_plane > 0.0f ? bit_length(hi_bits - lo_bits) : 32;
-            if (key_bits == 0) key_bits = 1;
-            // with offsets of up to 2^30 - 1, a splat of four tiles at the far plane would have the key of a culled point
-            if (key_bits == (int)kCountShift && hi_bits - lo_bits == (1u << kCountShift) - 1u) ++key_bits;
-            key_base = lo_bits;
-            pack_count = key_bits <= (int)kCountShift ? 1 : 0;
             n_visible = n;                // capacities from here on
             n_instances = 4 * n;
             rc = make_instance_blob();
@@ -4273,29 +4182,26 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         }
         {
             StageScope scope(STAGE_PREPROCESS, stream);
-            // (non-deferred: the number of key bits is not known yet, the sort clears its own state)
-            if (!deferred) clear.add(pb.group_visible, sizeof(unsigned) * (size_t)ceil_div<int64_t>(nb, 4));
-            clear.add(pb.state, (size_t)(static_cast<char*>(pb.sort_ws) - reinterpret_cast<char*>(pb.state)) + (deferred ? sort_zero_bytes(n, n, key_bits) : 0));
+            clear.add(pb.state, (size_t)(static_cast<char*>(pb.sort_ws) - reinterpret_cast<char*>(pb.state)) + sort_zero_bytes(n, n, key_bits));
             rc = launch_clear(clear, stream);
             if (rc != INPC_OK) return rc;
+            const int64_t chunks = ceil_div<int64_t>(n, kPreThreads), resident = (int64_t)sm_count() * projection_blocks(MODE);
+            auto* project = preprocess_kernel<MODE, VARIANT>;
+            launch_chained(project, (unsigned)(chunks < resident ? chunks : resident), kPreThreads, 0, stream,
+                ps, rp, (unsigned)chunks, key_base, pb.rec, pb.bounds, pb.quad, pb.conic, pb.foot, pb.keys[0], counts_in_keys ? 1 : 0, VARIANT == VAR_ROWS && warp_blend ? 1 : 2,
+                key_histogram(pb.sort_ws, n, n, key_bits), pb.counters, deferred ? nullptr : pb.counters + 1, status);
+            INPC_LAUNCH_CHECK("preprocess_kernel");
             if (!deferred) {
-                const int64_t count_blocks = ceil_div<int64_t>(nb, kPreThreads / 32), count_cap = (int64_t)sm_count() * 4;
-                const unsigned count_grid = (unsigned)(count_blocks < count_cap ? count_blocks : count_cap);
-                launch_chained(visibility_count_kernel<MODE, VARIANT>, count_grid, kPreThreads, 0, stream,
-                    ps, rp, (unsigned)nb, pb.block_visible, pb.group_visible, reinterpret_cast<unsigned long long*>(pb.state + 8), pb.state, pb.state + 2, pb.depth_min, pb.depth_max, pb.counters);
-                INPC_LAUNCH_CHECK("visibility_count_kernel");
-                INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
+                INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, stream));
                 INPC_CUDA_TRY(cudaEventRecord(ready, stream));
             }
-            // the projection pass needs nothing from the host: it runs while the host waits for the counters
-            auto* project = preprocess_kernel<MODE, VARIANT, true>;
-            if constexpr (MODE == INPC_MODE_BILINEAR) {
-                if (deferred) project = preprocess_kernel<MODE, VARIANT, false>;
-            }
-            launch_chained(project, (unsigned)nb, kPreThreads, 0, stream,
-                ps, rp, pb.block_visible, pb.group_visible, pb.depth_min, pb.depth_max, key_base,
-                pb.rec, pb.bounds, pb.quad, pb.conic, pb.foot, pb.keys[0], pb.ids[0], pack_count, VARIANT == VAR_ROWS && warp_blend ? 1 : 2, status);
-            INPC_LAUNCH_CHECK("preprocess_kernel");
+        }
+        {
+            // needs nothing from the host: it runs while the host waits for the counters
+            StageScope scope(STAGE_SORT_DEPTH, stream);
+            rc = carried ? sort_marked_keys_with_codes(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, codes, pb.sort_ws, status, &in_alt, stream)
+                         : sort_marked_keys(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, pb.sort_ws, status, &in_alt, stream);
+            if (rc != INPC_OK) return rc;
         }
         if (!deferred) {
             INPC_CUDA_TRY(cudaEventSynchronize(ready));
@@ -4304,13 +4210,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             // counts that cannot be: more survivors than points, or (bilinear: at most 2x2 tiles per splat)
             // more instances than four per survivor, or instances without survivors
             if (n_visible > n || (n_visible == 0 && n_instances != 0) || (MODE == INPC_MODE_BILINEAR && n_instances > 4 * n_visible)) {
-                set_error("inconsistent counts from the visibility pass: %lld visible of %lld points, %lld instances", (long long)n_visible,
+                set_error("inconsistent counts from the projection pass: %lld visible of %lld points, %lld instances", (long long)n_visible,
                           (long long)n, (long long)n_instances);
                 return INPC_E_DEVICE;
-            }
-            if (n_visible > 0) {
-                key_base = (uint32_t)host[2];
-                key_bits = bit_length((uint32_t)host[3] - key_base);
             }
         }
     }
@@ -4330,27 +4232,16 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         if (rc != INPC_OK) return rc;
     }
 
-    const bool counted = MODE == INPC_MODE_BILINEAR && warp_blend;   // the emission counts the digits of the keys
-    int in_alt = 0;
-    CarriedCodes codes;   // the depth sort carries the footprints along where they fit
-    if (deferred) codes = carried_codes(pb.quad, n, key_bits, (int64_t)n_tiles * 64);
-    const bool carried = codes.bits > 0;
-    {
-        StageScope scope(STAGE_SORT_DEPTH, stream);
-        rc = carried  ? sort_marked_keys_with_codes(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, codes, pb.sort_ws, true, status, &in_alt, stream)
-             : deferred ? sort_marked_keys(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n, pb.counters, key_bits, pb.sort_ws, true, status, &in_alt, stream)
-                      : sort_pairs(pb.keys[0], pb.keys[1], pb.ids[0], pb.ids[1], n_visible, n, key_bits, pb.sort_ws, false, status, &in_alt, stream);
-    }
-    if (rc != INPC_OK) return rc;
+    const bool counted = MODE == INPC_MODE_BILINEAR && warp_blend;   // the emission counts the digits of its keys
     const uint32_t* sorted_ids = pb.ids[in_alt];
     if (n_visible > 0 && n_instances > 0) {
-        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_need = MODE == INPC_MODE_BILINEAR && (carried || key_bits <= (int)kCountShift) ? ceil_div<int64_t>(ibk, kInstThreads / 4 / 32) : ibk, count_cap = (int64_t)sm_count() * 8;
+        const int64_t ibk = ceil_div<int64_t>(n_visible, kInstThreads), count_need = carried || counts_in_keys ? ceil_div<int64_t>(ibk, kInstThreads / 4 / 32) : ibk, count_cap = (int64_t)sm_count() * 8;
         const unsigned count_blocks = (unsigned)(count_need < count_cap ? count_need : count_cap);
         {
             StageScope scope(STAGE_INSTANCES, stream);
             // the count of touched tiles follows from the codes, or rides in the top key bits when the depth offsets left them free
-            auto* count = carried ? instance_count_kernel<COUNTS_IN_CODES> : MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift ? instance_count_kernel<COUNTS_IN_KEYS> : instance_count_kernel<COUNTS_GATHERED>;
-            launch_chained(count, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state + 3, deferred ? pb.counters + 1 : nullptr, codes.escape);
+            auto* count = carried ? instance_count_kernel<COUNTS_IN_CODES> : counts_in_keys ? instance_count_kernel<COUNTS_IN_KEYS> : instance_count_kernel<COUNTS_GATHERED>;
+            launch_chained(count, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state, deferred ? pb.counters + 1 : nullptr, codes.escape);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (counted) {
                 const KeyHistogram digits = key_histogram(ib.sort_ws, n_instances, likely_instances(n_instances, deferred), tile_bits);
@@ -4360,7 +4251,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                     rc = opt_in_dynamic_smem(emit_coded_kernel, sizeof(EmitCodedSmem), attr_set);
                     if (rc != INPC_OK) return rc;
                     const int64_t need = ceil_div<int64_t>(n_visible, kCodedThreads * kCodedPoints), cap = (int64_t)sm_count() * kCodedBlocks;
-                    launch_chained(emit_coded_kernel, (unsigned)(need < cap ? need : cap), kCodedThreads, sizeof(EmitCodedSmem), stream, sorted_ids, pb.keys[in_alt], codes, n_visible_dev,
+                    launch_chained(emit_coded_kernel, (unsigned)(need < cap ? need : cap), kCodedThreads, sizeof(EmitCodedSmem), stream, sorted_ids, pb.keys[in_alt], codes, n_visible, n_visible_dev,
                         pb.inst_block_sums, rp.gw, digits, n_emitted, ib.keys[0], ib.ids[0]);
                 } else {
                     const int64_t cap = (int64_t)sm_count() * 2;   // two blocks of 1024 threads fill a multiprocessor
