@@ -83,3 +83,22 @@ def test_counts_that_contradict_one_another(width, height, word, change):
     words[at[0] + word] -= change
     R.resolve_counts(state)
     assert (state.n_visible, state.n_instances) == want
+
+
+# Runs of the tile keys that end at, before and behind the first key of a thread (every 16th) and of a warp (every 512th), behind the last whole group of either, and empty tiles
+@pytest.mark.parametrize("lengths", [(1,), (16,), (16, 16, 480), (15, 1, 16, 17, 463, 1, 511, 0, 0, 513), (512, 512, 511), (0, 1024, 1, 0), (1000, 0, 40, 7, 17, 16), (0, 2048, 2048, 15)])
+@pytest.mark.parametrize("tile", [8, 16])
+def test_ranges_of_runs_that_end_beside_a_threads_keys(lengths, tile):
+    from inpc_b200 import rasterization as R
+    from inpc_b200.views import look_at_view
+    width = tile * len(lengths)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, tile, float(width), float(width)).to(DEV)
+    n = sum(lengths)
+    px = torch.repeat_interleave(torch.arange(len(lengths)) * tile + tile / 2, torch.tensor(lengths))
+    z = torch.rand(n, generator=torch.Generator().manual_seed(n))
+    pos = torch.stack([(px - width / 2) / width * (3 - z), torch.zeros(n), z], dim=1)[torch.randperm(n, generator=torch.Generator().manual_seed(1))].contiguous()
+    settings = R.INPCRasterizer.extract_settings(view, 0)
+    _, _, _, state, blobs, _ = R.forward_with_state(pos.to(DEV), torch.zeros((n, 36), dtype=torch.float16, device=DEV), torch.full((n, 1), 0.01, device=DEV), settings, tile)
+    ranges = R.debug_arrays(state, settings, blobs.point, blobs.instance)["ranges"].cpu()
+    ends = np.cumsum(lengths)
+    assert ranges.tolist() == [[int(e) - k, int(e)] if k else [0, 0] for e, k in zip(ends, lengths)]
