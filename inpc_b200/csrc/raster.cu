@@ -1623,7 +1623,7 @@ __device__ __forceinline__ WarpItem load_item(const WarpItem* p) {
     return w;
 }
 
-// Step 2: items0 = segment 0 of the non-empty tiles by class, items1 = every later segment, tile by tile.
+// Step 2: items0 = segment 0 of the non-empty tiles by class, and from its end backwards the empty tiles (their number alone); items1 = every later segment, tile by tile.
 __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uint2* __restrict__ ranges, int n_tiles, const SegmentLimits limits, bool by_length, unsigned long long n_instances_arg,
                                                                       const unsigned long long* __restrict__ n_instances_dev,
                                                                       const uint4* __restrict__ block_base, const uint32_t* __restrict__ counts, WarpItem* __restrict__ items0,
@@ -1647,7 +1647,10 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
     unsigned rank = before[0] + before[1] + before[2];         // non-empty tiles before this one
 #pragma unroll
     for (int k = 0; k < kItemTilesPerThread; ++k) {
-        if (ns[k] == 0u) continue;
+        if (ns[k] == 0u) {
+            if (t0 + k < n_tiles) items0[n_tiles - 1 - (t0 + k - (int)rank)].tile = (uint32_t)(t0 + k);
+            continue;
+        }
         const uint2 r = rg[k];
         const unsigned cls = length_class(r.y - r.x, sl, by_length);
         const unsigned place = cls == 0u ? class_base[0] + before[0]++ : cls == 1u ? class_base[1] + before[1]++ : class_base[2] + before[2]++;
@@ -2138,11 +2141,12 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
 
 // Per tile half with several segments, between the PRODUCT and REST passes: seg_T of segment s >= 1 becomes
 // the transmittance at its start = (state behind segment 0) * product of the segments 1 .. s-1.
-__global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel(const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts,
+// `n_tiles_at`: where in `counts` the number of tiles to look at is, see tiles_with_segments.
+__global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel(const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts, int n_tiles_at,
                                                                                  float* __restrict__ seg_T) {
     await_previous_kernel();
     const unsigned lane = lane_id();
-    const unsigned n_parts = __ldg(counts) * 2u;
+    const unsigned n_parts = __ldg(counts + n_tiles_at) * 2u;
     for (unsigned w = blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5); w < n_parts; w += gridDim.x * kWarpBlendWarps) {
         const WarpItem it = load_item(items0 + (w >> 1));
         const unsigned half = w & 1u;
@@ -2164,7 +2168,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel
     }
 }
 
-// Per tile half with several segments, after the REST pass: image = sum of the segment colours in order.
+// Last kernel of the forward passes.  Empty tiles, up to n_tiles (feature rows: none, their images are cleared beforehand): zeros; the passes write every pixel of the others.
+// Per tile half with several segments: image = sum of the segment colours in order.
 // For training the sum of a segment's colour and those behind it replaces the segment's own: what the backward pass takes the
 // segment's running colour from.  Where a pixel stops in a segment nothing is behind it, and the two agree to the bit at the last
 // fragment, as in an undivided list; the image less the colours before the segment would leave their rounding there, which an
@@ -2173,12 +2178,26 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel
 // of the first segment that fell below the threshold.
 template <int KIND, int C4>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_combine_kernel(
-    const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts, float4* __restrict__ seg_C, const float* __restrict__ seg_Z,
+    const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts, int n_tiles_at, float4* __restrict__ seg_C, const float* __restrict__ seg_Z,
     const float* __restrict__ seg_E,
-    float* __restrict__ image, float* __restrict__ depth_image, float* __restrict__ alpha_image, int width, int height, int gw, int gh) {
+    float* __restrict__ image, float* __restrict__ depth_image, float* __restrict__ alpha_image, int width, int height, int gw, int gh, int n_tiles) {
     await_previous_kernel();
     const unsigned lane = lane_id();
-    const unsigned n_parts = __ldg(counts) * 2u;
+    const unsigned n_parts = __ldg(counts + n_tiles_at) * 2u;
+    // four empty tiles at a time, a row of eight pixels of each: they mostly lie side by side
+    for (int t = (int)(__ldg(counts) + 4u * (blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5))); t < n_tiles; t += (int)(gridDim.x * kWarpBlendWarps * 4u)) {
+        if (t + (int)(lane >> 3) >= n_tiles) continue;
+        const int tile = (int)__ldg(&items0[t + (lane >> 3)].tile), tx = tile % gw, ty_all = tile / gw, set = ty_all / gh;
+        const int px = tx * 8 + (int)(lane & 7u), py = (ty_all - set * gh) * 8, rows = px < width ? min(8, height - py) : 0;
+        const int64_t n_px = (int64_t)width * height, pi = (int64_t)py * width + px;
+#pragma unroll 1
+        for (int c = 0; c < 4 * C4 + (KIND == BLEND_INFER ? 2 : 1); ++c) {
+            float* plane = (c < 4 * C4 ? image + ((int64_t)set * 4 * C4 + c) * n_px : (c == 4 * C4 ? alpha_image : depth_image) + (int64_t)set * n_px) + pi;
+#pragma unroll
+            for (int y = 0; y < 8; ++y)
+                if (y < rows) plane[(int64_t)y * width] = 0.0f;
+        }
+    }
     // a warp takes one group of four channels of a tile half
     for (unsigned wc = blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5); wc < n_parts * C4; wc += gridDim.x * kWarpBlendWarps) {
         const unsigned w = wc / C4, ch = wc % C4;
@@ -4354,6 +4373,9 @@ int warp_blend_grid(Kernel kernel, size_t smem, int most, bool bilinear, int pas
     grid->visits = bilinear ? grid->blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u;
     return rc;
 }
+// Tiles of several segments are longer than a first segment, i.e. in the first class where the tiles lie by length: the two small kernels look at no others then
+// (129,600 tiles, few of which have more than one segment: 22 + 12 -> 4 + 5 us).
+constexpr int tiles_with_segments(bool by_length) { return by_length ? kLongTiles : 0; }
 unsigned small_grid() { return (unsigned)(sm_count() * 4); }   // of the two small kernels between the passes
 
 struct ForwardPassArgs {
@@ -4401,12 +4423,12 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     if (rc_pass != INPC_OK) return rc_pass;
     rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_T);
+    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(!ROWS), ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
     rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    launch_chained(warp_blend_combine_kernel<KIND, C4>, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E,
-                                                                      image, depth, alpha, W, H, rp.gw, rp.gh);
+    launch_chained(warp_blend_combine_kernel<KIND, C4>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(!ROWS), ib.seg_C, ib.seg_Z, ib.seg_E,
+                                                                      image, depth, alpha, W, H, rp.gw, rp.gh, ROWS ? 0 : rp.gw * rp.gh * rp.n_sets);
     INPC_LAUNCH_CHECK("warp_blend_combine_kernel");
     return INPC_OK;
 }
@@ -4491,12 +4513,12 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     if (rc != INPC_OK) return rc;
     rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_T);
+    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(true), ib.seg_T);
     INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
     rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
-                                                                     rp.gw, rp.gh);
+    launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(true), ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
+                                                                     rp.gw, rp.gh, rp.gw * rp.gh * rp.n_sets);
     INPC_LAUNCH_CHECK("warp_blend_combine_kernel");
     return INPC_OK;
 }
@@ -4622,17 +4644,21 @@ int dispatch_rows(int channels, F&& f) {
     return INPC_E_INVALID;
 }
 
-// The outputs of a call that start at zero.  The warp blend has no work items for tiles without instances, so their pixels
-// are cleared; the block blend writes every tile.  `depth` and `weights` may be null.
-ClearList outputs_to_clear(const RasterParams& rp, int channels, float* image, float* depth, float* alpha, float* weights, int64_t n) {
+// The outputs of a call that start at zero.  Images do so for feature rows on 8x8 tiles alone: of 16 planes the empty tiles take longer to blank (28 us of a
+// 1237x822 image, warp_blend_combine_kernel) than everything to clear (10); with four channels and the alpha 3840x2160 pixels take 25 us to clear, the empty tiles 8.
+ClearList weights_to_clear(float* weights, int64_t n) {
     ClearList list;
+    list.add(weights, sizeof(float) * (size_t)n);
+    return list;
+}
+ClearList rows_to_clear(const RasterParams& rp, int channels, float* image, float* depth, float* alpha, float* weights, int64_t n) {
+    ClearList list = weights_to_clear(weights, n);
     if (uses_warp_blend(rp.tile)) {
-        const size_t n_px = (size_t)rp.v.width * rp.v.height * rp.n_sets;
+        const size_t n_px = (size_t)rp.v.width * rp.v.height;
         list.add(image, sizeof(float) * channels * n_px);
         list.add(depth, sizeof(float) * n_px);
         list.add(alpha, sizeof(float) * n_px);
     }
-    list.add(weights, sizeof(float) * (size_t)n);
     return list;
 }
 
@@ -4645,7 +4671,7 @@ int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* p
     InstanceBlob ib;
     int rc = run_front<INPC_MODE_BILINEAR, VAR_ROWS>(rp, n, positions, nullptr, opacities, alloc_point, alloc_instance, alloc_user, state,
                                                      KIND == BLEND_INFER, &pb, &ib, stream, KIND == BLEND_INFER ? "inpc_render_rows" : "inpc_rasterize_rows_forward",
-                                                     outputs_to_clear(rp, channels, image, depth, alpha, blending_weights, n), channels / 4);
+                                                     rows_to_clear(rp, channels, image, depth, alpha, blending_weights, n), channels / 4);
     if (rc != INPC_OK) return rc;
     const int t_alt = tile_buffer_of(state, rp.gw * rp.gh);
     {
@@ -4678,13 +4704,12 @@ extern "C" int inpc_rasterize_forward(int mode, int tile_size, const inpc_view* 
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, 0.0f, 3.0f, nullptr);
-    const ClearList clear = outputs_to_clear(rp, 4, image, nullptr, alpha, blending_weights, n);
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
-        rc = run_front<INPC_MODE_BILINEAR, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward", clear);
+        rc = run_front<INPC_MODE_BILINEAR, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward", weights_to_clear(blending_weights, n));
     else
-        rc = run_front<INPC_MODE_GAUSSIAN, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward", clear);
+        rc = run_front<INPC_MODE_GAUSSIAN, VAR_TRAIN>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, state, false, &pb, &ib, stream, "inpc_rasterize_forward", weights_to_clear(blending_weights, n));
     if (rc != INPC_OK) return rc;
     rc = launch_blend_forward<BLEND_TRAIN>(mode, rp, pb, ib, state, image, nullptr, alpha, blending_weights, kTrainGaussThreshold, stream);
     return rc != INPC_OK ? rc : end_index_checks(stream);
@@ -4774,14 +4799,13 @@ extern "C" int inpc_render(int mode, int tile_size, const inpc_view* view, int64
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, sigma_world, sigma_cutoff, nullptr);
-    const ClearList clear = outputs_to_clear(rp, 4, image, depth, alpha, nullptr, n);
     inpc_raster_state st;
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
-        rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render", clear);
+        rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render", ClearList());
     else
-        rc = run_front<INPC_MODE_GAUSSIAN, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render", clear);
+        rc = run_front<INPC_MODE_GAUSSIAN, VAR_RAW37>(rp, n, positions, features_raw, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render", ClearList());
     if (rc != INPC_OK) return rc;
     // runtime cut-off exp(-cutoff^2/2): src/gaussian/inference.cu:171
     const float threshold = expf(-0.5f * sigma_cutoff * sigma_cutoff);
@@ -4802,14 +4826,13 @@ extern "C" int inpc_render_preextracted(int mode, int tile_size, const inpc_view
         return INPC_E_INVALID;
     }
     const RasterParams rp = make_params(view, tile_size, sigma_world, sigma_cutoff, scales);
-    const ClearList clear = outputs_to_clear(rp, 4, image, depth, alpha, nullptr, n);
     inpc_raster_state st;
     PointBlob pb;
     InstanceBlob ib;
     if (mode == INPC_MODE_BILINEAR)
-        rc = run_front<INPC_MODE_BILINEAR, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted", clear);
+        rc = run_front<INPC_MODE_BILINEAR, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted", ClearList());
     else
-        rc = run_front<INPC_MODE_GAUSSIAN, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted", clear);
+        rc = run_front<INPC_MODE_GAUSSIAN, VAR_PREEXTRACTED>(rp, n, positions, features, opacities, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib, stream, "inpc_render_preextracted", ClearList());
     if (rc != INPC_OK) return rc;
     const float threshold = expf(-0.5f * sigma_cutoff * sigma_cutoff);
     rc = launch_blend_forward<BLEND_INFER>(mode, rp, pb, ib, &st, image, depth, alpha, nullptr, threshold, stream);
@@ -4853,7 +4876,7 @@ extern "C" int inpc_render_multi(int tile_size, const inpc_view* view, int n_set
     PointBlob pb;
     InstanceBlob ib;
     rc = run_front<INPC_MODE_BILINEAR, VAR_RAW37>(rp, n_virtual, nullptr, nullptr, nullptr, alloc_point, alloc_instance, alloc_user, &st, true, &pb, &ib,
-                                                  stream, "inpc_render_multi", outputs_to_clear(rp, 4, images, depths, alphas, nullptr, n_virtual), 1, &ps);
+                                                  stream, "inpc_render_multi", ClearList(), 1, &ps);
     if (rc != INPC_OK) return rc;
     rc = launch_blend_forward<BLEND_INFER>(INPC_MODE_BILINEAR, rp, pb, ib, &st, images, depths, alphas, nullptr, 0.0f, stream);
     return rc != INPC_OK ? rc : end_index_checks(stream);

@@ -81,3 +81,52 @@ def test_blend_passes_launch_the_blocks_that_are_resident(tmp_path):
         if "gaussian_warp_forward" in name:
             fit = min(fit, 3)
         assert a["grid"][0] == multiprocessors * fit, (name, a["grid"][0] / multiprocessors, fit)
+
+
+# Images are not cleared beforehand: tiles without instances are blanked at the end.  Into memory full of NaN; odd sizes; nothing, one point, all points culled, a few tiles with lists
+# of one and of several segments among many empty ones
+@pytest.mark.parametrize("width, height", [(8, 8), (101, 53), (1237, 40)])
+@pytest.mark.parametrize("n", [0, 1, 40, 9000])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_empty_tiles_are_blank_in_memory_that_is_not(width, height, n, mode):
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    g = torch.Generator().manual_seed(n + width)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, float(width), float(width)).to(DEV)
+    spot = torch.rand(n, generator=g) < 0.7                       # most points in one place, the others in a strip of the image
+    px = torch.where(spot, width * 0.3 + torch.rand(n, generator=g) * 4, torch.rand(n, generator=g) * width * 0.4)
+    py = torch.where(spot, height * 0.5 + torch.rand(n, generator=g) * 2, torch.rand(n, generator=g) * height)
+    pos = torch.stack([(px - width / 2) / width * 3, -(py - height / 2) / width * 3, torch.zeros(n)], dim=1).contiguous().to(DEV)
+    behind = pos + torch.tensor([0.0, 0.0, 9.0], device=DEV)
+    feats, raw = ((torch.randn((n, k), generator=g) * 0.1 + 1.0).to(torch.float16).to(DEV) for k in (36, 37))
+    opac, rows = torch.full((n, 1), 0.01, device=DEV), torch.ones((n, 8), device=DEV)
+    rast = inpc_b200.INPCRasterizer()
+
+    def calls(p):
+        yield rast(view, mode, p, feats, opac)[:2]
+        yield rast.render_preextracted(view, mode, p, feats, opac)
+        yield rast.render(view, mode, p, raw, 1.0, 3.0)
+        if mode == 0:
+            yield rast.forward_rows(view, p, rows, opac)[:2]
+            yield rast.render_multi(view, [(p, raw), (behind, raw), (p, raw)])
+
+    def dirty():
+        for k in (1, 4, 8, 3, 12):
+            for _ in range(4):
+                torch.full((k, height, width), float("nan"), device=DEV)
+
+    for p in (pos, behind):
+        torch.cuda.empty_cache()
+        dirty()
+        for out in calls(p):
+            alpha = out[-1].reshape(-1, height, width)
+            for t in out:
+                assert bool(torch.isfinite(t).all())
+                planes = t.reshape(alpha.shape[0], -1, height, width)
+                assert bool((planes.transpose(0, 1)[:, alpha == 0.0] == 0.0).all())
+            assert bool((alpha[:, :, int(width * 0.45) + 8:] == 0.0).all())
+            if p is behind or n == 0:
+                assert bool((alpha == 0.0).all())
+            elif n > 30:
+                assert bool((alpha[0] > 0.0).any())
+            dirty()
