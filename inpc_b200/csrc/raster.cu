@@ -251,7 +251,9 @@ __device__ __forceinline__ unsigned scan_words(unsigned* data, int64_t n, unsign
 
 constexpr int kPreThreads = 256;
 constexpr int projection_blocks(int mode) { return mode == INPC_MODE_GAUSSIAN ? 5 : 6; }   // per multiprocessor, see preprocess_kernel
-constexpr unsigned kCountShift = 30;   // bilinear: (tiles touched - 1) in key bits 30..31 when the depth offsets fit below
+// The number of tiles a splat touches rides in the key bits above the depth offsets where these leave room (the sort ignores bits above its range and carries
+// them along), which saves the instance count a gather: bilinear 1, 2 or 4, less one, in bits 30..31; gaussian 1..30 in bits 27..31, 0 for more, which are looked up.
+constexpr unsigned kCountShift = 30, kGaussCountShift = 27, kMostKeyTiles = 30;
 
 constexpr int kScanThreads = 1024;
 
@@ -473,14 +475,13 @@ __global__ void __launch_bounds__(kPreThreads, projection_blocks(MODE)) preproce
             // what the instance passes need of a point: its packed footprint where splats are bilinear on 8x8 tiles, else its tile bounds
             if (MODE == INPC_MODE_BILINEAR && quad) quad[iv] = pr.visible ? pack_quad(pr, set * rp.gh, rp.gw) : kNoQuad;
             else bounds[iv] = pr.visible ? make_uint2(pr.x0 | (pr.x1 << 16), pr.y0 | (pr.y1 << 16)) : make_uint2(0u, 0u);
-            // sort key: offset of the depth's bit pattern from the smallest there can be (fewer radix passes).
-            // A bilinear splat touches 1, 2 or 4 tiles; when the offsets leave the two top bits free that count rides there (the
-            // sort ignores bits above its range and carries them along), which saves the instance pass a gather.
+            // sort key: offset of the depth's bit pattern from the smallest there can be (fewer radix passes), and the number of tiles
             uint32_t key = kNoKey;
             if (pr.visible) {
                 key = __float_as_uint(pr.depth) - key_base;
                 count_key(s_digits, digits.pt, key);
-                if (MODE == INPC_MODE_BILINEAR && pack_count) key |= ((pr.x1 - pr.x0) * (pr.y1 - pr.y0) - 1u) << kCountShift;
+                const unsigned tiles = (pr.x1 - pr.x0) * (pr.y1 - pr.y0);
+                if (pack_count) key |= MODE == INPC_MODE_BILINEAR ? (tiles - 1u) << kCountShift : (tiles <= kMostKeyTiles ? tiles : 0u) << kGaussCountShift;
             }
             depth_keys[iv] = key;
         }
@@ -507,7 +508,7 @@ __device__ __forceinline__ unsigned tiles_of_code(uint32_t code, uint32_t escape
 
 // COUNTS_IN_KEYS, COUNTS_IN_CODES (see CarriedCodes): a warp sums one block's worth of points, all its loads in flight together, no barrier before the last
 // block's scan (a barrier per group of a block and one load per thread: 2^23 / 2^25 points 16 / 61 -> 11 / 39 us).
-enum { COUNTS_GATHERED = 0, COUNTS_IN_KEYS = 1, COUNTS_IN_CODES = 2 };
+enum { COUNTS_GATHERED = 0, COUNTS_IN_KEYS = 1, COUNTS_IN_CODES = 2, COUNTS_IN_GAUSS_KEYS = 3 };
 template <int SOURCE>
 __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const uint32_t* __restrict__ sorted_keys,
                                                                           const uint32_t* __restrict__ sorted_ids,
@@ -520,6 +521,7 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
     if (SOURCE != COUNTS_GATHERED) {
         auto count_of = [&](uint32_t word) -> unsigned {
             if (SOURCE == COUNTS_IN_KEYS) return (word >> kCountShift) + 1u;
+            if (SOURCE == COUNTS_IN_GAUSS_KEYS) return word >> kGaussCountShift;
             return tiles_of_code(word, escape);
         };
         constexpr int kLoads = kInstThreads / 128;   // 16-byte loads per lane and group
@@ -531,9 +533,23 @@ __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const 
 #pragma unroll
                 for (int q = 0; q < kLoads; ++q) k[q] = __ldg(reinterpret_cast<const uint4*>(sorted_keys + first + 128 * q));   // the key buffers are 16-byte aligned
 #pragma unroll
-                for (int q = 0; q < kLoads; ++q) c += count_of(k[q].x) + count_of(k[q].y) + count_of(k[q].z) + count_of(k[q].w);
+                for (int q = 0; q < kLoads; ++q) {
+                    const unsigned t[4] = {count_of(k[q].x), count_of(k[q].y), count_of(k[q].z), count_of(k[q].w)};
+                    if (SOURCE == COUNTS_IN_GAUSS_KEYS && (t[0] == 0u || t[1] == 0u || t[2] == 0u || t[3] == 0u)) {
+                        // more tiles than the field holds
+                        const uint4 id = __ldg(reinterpret_cast<const uint4*>(sorted_ids + first + 128 * q));
+                        const uint2 none = make_uint2(0u, 0u);
+                        const uint2 b0 = t[0] ? none : __ldg(bounds + checked_point(id.x)), b1 = t[1] ? none : __ldg(bounds + checked_point(id.y));
+                        const uint2 b2 = t[2] ? none : __ldg(bounds + checked_point(id.z)), b3 = t[3] ? none : __ldg(bounds + checked_point(id.w));
+                        c += tiles_of(b0) + tiles_of(b1) + tiles_of(b2) + tiles_of(b3);
+                    }
+                    c += t[0] + t[1] + t[2] + t[3];
+                }
             } else {
-                for (int64_t s = (int64_t)group * kInstThreads + lane_id(); s < n_visible; s += 32) c += count_of(__ldg(sorted_keys + s));
+                for (int64_t s = (int64_t)group * kInstThreads + lane_id(); s < n_visible; s += 32) {
+                    const unsigned t = count_of(__ldg(sorted_keys + s));
+                    c += SOURCE == COUNTS_IN_GAUSS_KEYS && t == 0u ? tiles_of(__ldg(bounds + checked_point(__ldg(sorted_ids + s)))) : t;
+                }
             }
             c = __reduce_add_sync(0xffffffffu, c);
             if (lane_id() == 0) block_sums[group] = c;
@@ -747,6 +763,17 @@ __global__ void __launch_bounds__(kCodedThreads, kCodedBlocks) emit_coded_kernel
 // Other splats.  CELLS (gaussian, 8x8 tiles): the key also says which cells of the tile the ellipse can reach (see cell_code).  The keys are counted by the
 // sort: a gaussian splat has many instances, whose atomics would go one after the other (2^22 of them, emission and histogram 61 + 13 -> 90 us).
 template <bool CELLS>
+__device__ __forceinline__ uint32_t instance_key(unsigned tx, unsigned ty, unsigned x0, unsigned x1, unsigned y0, unsigned y1, unsigned inset, int gw) {
+    const uint32_t tile = ty * (unsigned)gw + tx;
+    if (!CELLS) return tile;
+    const int left = (int)(inset & 15u) - 4 * (int)(tx - x0), right = 4 * (int)(x1 - tx) - 1 - (int)((inset >> 4) & 15u);
+    const int top = (int)((inset >> 8) & 15u) - 4 * (int)(ty - y0), bottom = 4 * (int)(y1 - ty) - 1 - (int)(inset >> 12);
+    return tile | cell_code(left, right, top, bottom) << kTileKeyBits;
+}
+// Up to how many instances of a warp's points every lane writes those of its own; of more the lanes take equal shares and write side by side.  2^22 splats of 1.4
+// tiles on average 62 us with own ones, 69 shared (68 staged in shared memory); 2 * 10^6 splats of about a pixel and more 59 and 45 (47).
+constexpr unsigned kFewInstances = 64;
+template <bool CELLS>
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
                                                                       const uint2* __restrict__ bounds,
                                                                       const uint4* __restrict__ foot, int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
@@ -779,21 +806,37 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
         }
         x0 = b.x & 0xffffu; x1 = b.x >> 16; y0 = b.y & 0xffffu; y1 = b.y >> 16;
     }
-    const unsigned c = (x1 - x0) * (y1 - y0);
-    const unsigned inc = warp_inclusive_scan(c);
-    unsigned off = before_warp(__shfl_sync(0xffffffffu, inc, 31)) + inc - c;
-    for (unsigned ty = y0; ty < y1; ++ty)
-        for (unsigned tx = x0; tx < x1; ++tx) {
-            uint32_t key = ty * (unsigned)gw + tx;
-            if (CELLS) {
-                const int left = (int)(inset & 15u) - 4 * (int)(tx - x0), right = 4 * (int)(x1 - tx) - 1 - (int)((inset >> 4) & 15u);
-                const int top = (int)((inset >> 8) & 15u) - 4 * (int)(ty - y0), bottom = 4 * (int)(y1 - ty) - 1 - (int)(inset >> 12);
-                key |= cell_code(left, right, top, bottom) << kTileKeyBits;
+    const unsigned c = (x1 - x0) * (y1 - y0), inc = warp_inclusive_scan(c), before = inc - c, total = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned base = before_warp(total);
+    if (total <= kFewInstances) {
+        unsigned at = base + before;
+        for (unsigned ty = y0; ty < y1; ++ty)
+            for (unsigned tx = x0; tx < x1; ++tx) {
+                __stcs(inst_keys + at, instance_key<CELLS>(tx, ty, x0, x1, y0, y1, inset, gw));
+                __stcs(inst_ids + at, id);
+                ++at;
             }
-            __stcs(inst_keys + off, key);
-            __stcs(inst_ids + off, id);
-            ++off;
+        return;
+    }
+    // the lanes share them: lane l takes every 32nd and finds the point it belongs to among the sums
+    const unsigned columns = x0 | (x1 << 16), rows = y0 | (y1 << 16);
+    for (unsigned first = 0; first < total; first += 32u) {
+        const unsigned i = first + lane;
+        unsigned point = 0u;   // the last lane whose instances begin at i at the latest (lanes without a point lie behind all others)
+#pragma unroll
+        for (unsigned step = 16u; step > 0u; step >>= 1) {
+            const unsigned begins = __shfl_sync(0xffffffffu, before, point + step);
+            point += begins <= i ? step : 0u;
         }
+        const unsigned at = i - __shfl_sync(0xffffffffu, before, point), cols = __shfl_sync(0xffffffffu, columns, point), rws = __shfl_sync(0xffffffffu, rows, point);
+        const uint32_t who = __shfl_sync(0xffffffffu, id, point);
+        const unsigned in = CELLS ? __shfl_sync(0xffffffffu, inset, point) : 0u;
+        if (i >= total) continue;
+        const unsigned px0 = cols & 0xffffu, px1 = cols >> 16, py0 = rws & 0xffffu, py1 = rws >> 16, width = px1 - px0;
+        const unsigned dy = at / width, dx = at - dy * width;
+        __stcs(inst_keys + base + i, instance_key<CELLS>(px0 + dx, py0 + dy, px0, px1, py0, py1, in, gw));
+        __stcs(inst_ids + base + i, who);
+    }
 }
 
 // Run boundaries of the sorted tile keys -> [first, last+1) per tile (src/bilinear/kernels.cu:222-239).  A thread compares the first of its 16 or
@@ -4174,7 +4217,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     if (key_bits == 0) key_bits = 1;
     // with offsets of up to 2^30 - 1, a splat of four tiles at the far plane would have the key of a culled point
     if (key_bits == (int)kCountShift && last_key - key_base == (1u << kCountShift) - 1u) ++key_bits;
-    const bool counts_in_keys = MODE == INPC_MODE_BILINEAR && key_bits <= (int)kCountShift;
+    const bool counts_in_keys = key_bits <= (int)(MODE == INPC_MODE_BILINEAR ? kCountShift : kGaussCountShift);
     const int tile_bits = bit_length((uint32_t)(n_tiles - 1));
     CarriedCodes codes;   // the depth sort carries the footprints along where they fit
     if (MODE == INPC_MODE_BILINEAR && warp_blend) codes = carried_codes(pb.quad, n, key_bits, (int64_t)n_tiles * 64);
@@ -4268,8 +4311,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
         const unsigned count_blocks = (unsigned)(count_need < count_cap ? count_need : count_cap);
         {
             StageScope scope(STAGE_INSTANCES, stream);
-            // the count of touched tiles follows from the codes, or rides in the top key bits when the depth offsets left them free
-            auto* count = carried ? instance_count_kernel<COUNTS_IN_CODES> : counts_in_keys ? instance_count_kernel<COUNTS_IN_KEYS> : instance_count_kernel<COUNTS_GATHERED>;
+            // the count of touched tiles follows from the codes, or rides in the top key bits where the depth offsets leave them free
+            auto* count = carried ? instance_count_kernel<COUNTS_IN_CODES> : !counts_in_keys ? instance_count_kernel<COUNTS_GATHERED>
+                          : MODE == INPC_MODE_BILINEAR ? instance_count_kernel<COUNTS_IN_KEYS> : instance_count_kernel<COUNTS_IN_GAUSS_KEYS>;
             launch_chained(count, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state, deferred ? pb.counters + 1 : nullptr, codes.escape);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (counted) {
