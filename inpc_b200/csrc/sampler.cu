@@ -819,6 +819,35 @@ __device__ __forceinline__ float box_value(unsigned word, bool minimum) {
     return __uint_as_float(key & 0x80000000u ? key & 0x7FFFFFFFu : ~key);
 }
 
+// 30-bit Morton code (10 bits per axis, x lowest) of a position inside the box [lo, lo + extent]^3: the bits of an axis two apart, by table (through L1, where neighbouring
+// samples meet few entries; eight operations per axis otherwise)
+struct SpreadTable {
+    unsigned spread[1024];
+    constexpr SpreadTable() : spread() {
+        for (unsigned v = 0; v < 1024u; ++v)
+            for (unsigned bit = 0; bit < 10u; ++bit) spread[v] |= (v >> bit & 1u) << (3u * bit);
+    }
+};
+__device__ const SpreadTable g_spread{};
+// The cube the codes refer to: lower corner and reciprocal edge.
+struct MortonCube {
+    float lo[3];
+    float inv_extent;
+};
+__device__ __forceinline__ unsigned morton_code(const MortonCube& cube, float px, float py, float pz) {
+    // trunc(1024 t) of t in [0, 1], 1023 at most, without a conversion (a quarter of the rate of an addition and less): a sum rounded down, whose unit is one.  No number counts as 0
+    auto cell = [&](float p, float lo) -> unsigned {
+        return __ldg(g_spread.spread + (min(__float_as_uint(__fmaf_rz(__saturatef(__fmul_rn(p - lo, cube.inv_extent)), 1024.0f, 8388608.0f)), 0x4B0003FFu) & 0x3FFu));
+    };
+    return cell(px, cube.lo[0]) | (cell(py, cube.lo[1]) << 1) | (cell(pz, cube.lo[2]) << 2);
+}
+// A bounding box {min x, y, z, max x, y, z} -> its cube, the edge widened by a millionth so that the largest coordinate stays inside.  Same roundings as float32
+// corners and a double product.  An axis with a NaN in it has no corner and takes no part in the codes, and the edge is then 1.
+__device__ __forceinline__ MortonCube cube_of_box(const float* box) {
+    const float extent = max_nan(max_nan(__fsub_rn(box[3], box[0]), __fsub_rn(box[4], box[1])), __fsub_rn(box[5], box[2]));
+    return {{box[0], box[1], box[2]}, extent > 0.0f ? __fdiv_rn(1.0f, __double2float_rn(__dmul_rn((double)extent, 1.0 + 1e-6))) : 1.0f};
+}
+
 // Sample i lies in leaf upper_bound(offsets, i) and is that leaf's h-th sample, h = i - first sample
 // of the leaf: Halton point h+1 in bases (2, 3, 5) scaled into the cell; a leaf with a single sample
 // puts it at its centre (ProbabilityField.py:131-140).
@@ -826,6 +855,8 @@ __device__ __forceinline__ float box_value(unsigned word, bool minimum) {
 // at a time, and heads of 729 and 625 values, read through L1, settle most digits: 2^25 samples of 2.3 * 10^5 leaves 234 -> 197 us (before: a
 // search, six gathers and a division per sample, heads of 81 and 125 values in shared memory; with those and the rest as here 212, with the long heads in shared
 // memory 201, with persistent blocks 229 to 254).
+// CODES: also the Morton codes, whose cube is known from the leaves (halton_box_kernel), so that nothing reads the positions for them: 2^25 samples 191 -> 243 us, and 53 for the
+// histogram of the codes, where a kernel that read the positions and counted took 134 (with conversions and spread by shifts 267).
 constexpr unsigned kRunRecords = 256;   // leaves of a run whose records are staged; a run over more makes them per sample
 struct HaltonLeaf {
     float x, y, z, cell;   // lower corner and edge, or the centre where there is a single sample
@@ -843,10 +874,11 @@ __device__ __forceinline__ HaltonLeaf halton_leaf(const float* __restrict__ cent
     }
     return l;
 }
+template <bool CODES>
 __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned* __restrict__ counts, const unsigned* __restrict__ offsets,
                                                                   unsigned n_cells, const float* __restrict__ centers,
                                                                   const int* __restrict__ levels, float initial_size, unsigned n_total,
-                                                                  float* __restrict__ positions) {
+                                                                  float* __restrict__ positions, const MortonCube* __restrict__ cube_at, unsigned* __restrict__ codes) {
     await_previous_kernel();
     __shared__ LeafRun run;
     __shared__ unsigned s_start;   // first sample of the run's first leaf
@@ -863,6 +895,11 @@ __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned
     if (staged)
         for (unsigned k = threadIdx.x; k < m; k += kThreads) s_leaf[k] = halton_leaf(centers, levels, initial_size, leaf0 + k, __ldg(counts + leaf0 + k));
     __syncthreads();
+    MortonCube cube;
+    if (CODES) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(cube_at));
+        cube = {{q.x, q.y, q.z}, q.w};
+    }
     unsigned k = 0;
     for (unsigned row = 0; row < (unsigned)kRunPerThread; ++row) {
         const unsigned first = (warp * kRunPerThread + row) * 32u;
@@ -878,6 +915,7 @@ __global__ void __launch_bounds__(kThreads) halton_samples_kernel(const unsigned
             y = __fadd_rn(y, __fmul_rn(halton_element(tables.b3, h + 1u), at.cell));
             z = __fadd_rn(z, __fmul_rn(halton_element(tables.b5, h + 1u), at.cell));
         }
+        if (CODES && lane < here) codes[i] = morton_code(cube, x, y, z);
         store_row(s_pos[warp], x, y, z, here, positions + 3 * (int64_t)(r0 + first));
     }
 }
@@ -899,9 +937,9 @@ __device__ __forceinline__ unsigned smallest_halton_index(unsigned c) {
 
 // Bounding box of the cloud that halton_samples_kernel makes, from the leaves: along an axis the extreme samples of a leaf are those of its extreme Halton elements
 // (placing one rounds, but monotonically).  Spares the Morton order a pass over the positions: 2^25 samples of 2.3 * 10^5 leaves 78 us -> 11 (in the placement itself,
-// six comparisons per sample, 39).
+// six comparisons per sample, 39).  The block that finishes last leaves the cube of the codes.  box_words: kBoxCopies boxes, and a word for the finished blocks.
 __global__ void __launch_bounds__(kThreads) halton_box_kernel(const unsigned* __restrict__ counts, unsigned n_cells, const float* __restrict__ centers, const int* __restrict__ levels,
-                                                              float initial_size, unsigned* box_words) {
+                                                              float initial_size, unsigned* box_words, MortonCube* __restrict__ cube) {
     await_previous_kernel();
     __shared__ float s_box[kThreads / 32][6];
     float box[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -928,16 +966,12 @@ __global__ void __launch_bounds__(kThreads) halton_box_kernel(const unsigned* __
 #pragma unroll
     for (int c = 0; c < 6; ++c)
         if (threadIdx.x == c) atomicMax(box_words + (blockIdx.x % kBoxCopies) * 6 + c, box_word(box[c], c < 3));
-}
-
-// 30-bit Morton code (10 bits per axis, x lowest) of a position inside the box [lo, lo + extent]^3
-__device__ __forceinline__ unsigned spread_bits_10(unsigned v) {
-    v &= 0x3FFu;
-    v = (v | (v << 16)) & 0x030000FFu;
-    v = (v | (v << 8)) & 0x0300F00Fu;
-    v = (v | (v << 4)) & 0x030C30C3u;
-    v = (v | (v << 2)) & 0x09249249u;
-    return v;
+    if (!last_block(box_words + 6 * kBoxCopies, gridDim.x)) return;
+    static_assert(kBoxCopies <= kThreads, "a thread per copy");
+#pragma unroll
+    for (int c = 0; c < 6; ++c) box[c] = box_value(threadIdx.x < kBoxCopies ? __ldcg(box_words + 6 * threadIdx.x + c) : 0u, c < 3);
+    block_box(box, s_box);
+    if (threadIdx.x == 0) *cube = cube_of_box(box);
 }
 
 __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, float* __restrict__ partial) {
@@ -960,20 +994,16 @@ __global__ void __launch_bounds__(kThreads) bounding_box_kernel(const float* __r
     if (threadIdx.x < 6) partial[6 * blockIdx.x + threadIdx.x] = threadIdx.x == 0 ? box[0] : threadIdx.x == 1 ? box[1] : threadIdx.x == 2 ? box[2] : threadIdx.x == 3 ? box[3] : threadIdx.x == 4 ? box[4] : box[5];
 }
 
-// The cube the codes refer to: the caller's, or (box_parts > 0) the cloud's own from the partial boxes, its edge widened by
-// a millionth so that the largest coordinate stays inside.  Same roundings as float32 corners and a double product.  An axis with
-// a NaN in it has no corner and takes no part in the codes, and the edge is then 1.
+// The cube of a cloud that lies there already: the caller's, or (box_parts > 0) from the partial boxes.
 struct MortonBox {
-    float lo[3];
-    float inv_extent;
-    const float* parts;       // partial boxes as values ...
-    const unsigned* words;    // ... or as words, see box_word
+    MortonCube cube;
+    const float* parts;
     int box_parts;
 };
 // Also counts the digits of the codes for their sort, which spares it a pass over them: 2^25 codes and their histogram 90 + 53 -> 132 us.
 constexpr int kCodeThreads = kRadix;
 __global__ void __launch_bounds__(kCodeThreads) morton_codes_kernel(const float* __restrict__ positions, int64_t n, bool vec_ok, MortonBox mb, KeyHistogram digits,
-                                                                unsigned* __restrict__ codes, unsigned* __restrict__ order) {
+                                                                unsigned* __restrict__ codes) {
     await_previous_kernel();
     __shared__ BlockHistogram s_digits;
     clear_histogram(s_digits);
@@ -984,21 +1014,14 @@ __global__ void __launch_bounds__(kCodeThreads) morton_codes_kernel(const float*
         for (int k = threadIdx.x; k < mb.box_parts; k += kCodeThreads)
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                const float t = mb.words ? box_value(__ldg(mb.words + 6 * k + c), c < 3) : __ldg(mb.parts + 6 * k + c);
+                const float t = __ldg(mb.parts + 6 * k + c);
                 box[c] = c < 3 ? min_nan(box[c], t) : max_nan(box[c], t);
             }
         block_box(box, s_box);
-        const float extent = max_nan(max_nan(__fsub_rn(box[3], box[0]), __fsub_rn(box[4], box[1])), __fsub_rn(box[5], box[2]));
-        mb.inv_extent = extent > 0.0f ? __fdiv_rn(1.0f, __double2float_rn(__dmul_rn((double)extent, 1.0 + 1e-6))) : 1.0f;
-        mb.lo[0] = box[0]; mb.lo[1] = box[1]; mb.lo[2] = box[2];
+        mb.cube = cube_of_box(box);
     }
     auto code = [&](float px, float py, float pz) -> unsigned {
-        const float qx = (px - mb.lo[0]) * mb.inv_extent * 1024.0f;
-        const float qy = (py - mb.lo[1]) * mb.inv_extent * 1024.0f;
-        const float qz = (pz - mb.lo[2]) * mb.inv_extent * 1024.0f;
-        const unsigned x = (unsigned)fminf(fmaxf(qx, 0.0f), 1023.0f), y = (unsigned)fminf(fmaxf(qy, 0.0f), 1023.0f),
-                       z = (unsigned)fminf(fmaxf(qz, 0.0f), 1023.0f);
-        const unsigned key = spread_bits_10(x) | (spread_bits_10(y) << 1) | (spread_bits_10(z) << 2);
+        const unsigned key = morton_code(mb.cube, px, py, pz);
         count_key(s_digits, digits.pt, key);
         return key;
     };
@@ -1014,14 +1037,13 @@ __global__ void __launch_bounds__(kCodeThreads) morton_codes_kernel(const float*
             for (int64_t k = i; k < n && k < i + 4; ++k) codes[k] = code(__ldg(positions + 3 * k), __ldg(positions + 3 * k + 1), __ldg(positions + 3 * k + 2));
         }
     }
-    if (n == 1 && blockIdx.x == 0 && threadIdx.x == 0) order[0] = 0u;   // a single pair is not sorted
     finish_histogram(s_digits, digits, gridDim.x, nullptr);
 }
 
-// Four points per thread, their gathers in flight together and three 16-byte stores (2^25 points 167 us; one
+// Four points per thread, their gathers in flight together, two loads of 8 bytes each, and three 16-byte stores (2^25 points 142 us; three loads of 4 bytes 166; one
 // point per thread with three 4-byte stores 201, the same with the stores staged through shared memory 211).
 __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float* __restrict__ positions, const unsigned* __restrict__ order,
-                                                                    int64_t n, bool vec_ok, float* __restrict__ out) {
+                                                                    int64_t n, bool pairs_ok, bool vec_ok, float* __restrict__ out) {
     await_previous_kernel();
     const int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
     if (i >= n) return;
@@ -1030,9 +1052,21 @@ __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float*
         const unsigned j[4] = {o.x, o.y, o.z, o.w};
         float v[12];
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+        for (int k = 0; k < 4; ++k) {
+            if (!pairs_ok) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[3 * k + c] = __ldg(positions + 3 * (int64_t)j[k] + c);
+                for (int c = 0; c < 3; ++c) v[3 * k + c] = __ldg(positions + 3 * (int64_t)j[k] + c);
+                continue;
+            }
+            // around the 12 bytes (behind the last point there may be nothing)
+            const float2* src = reinterpret_cast<const float2*>(positions) + ((3 * (int64_t)j[k]) >> 1);
+            const float2 a = __ldg(src);
+            float2 b = make_float2(0.0f, 0.0f);
+            if (j[k] + 1u < n || (j[k] & 1u)) b = __ldg(src + 1);
+            else b.x = __ldg(reinterpret_cast<const float*>(src + 1));
+            const bool odd = j[k] & 1u;
+            v[3 * k] = odd ? a.y : a.x; v[3 * k + 1] = odd ? b.x : a.y; v[3 * k + 2] = odd ? b.y : b.x;
+        }
         float4* dst = reinterpret_cast<float4*>(out + 3 * i);
 #pragma unroll
         for (int k = 0; k < 3; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
@@ -1398,7 +1432,7 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
 
 // `box_words` (optional): 6 kBoxCopies words that start at zero, see box_word.
 static int launch_halton(const char* who, const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size, int64_t n_total,
-                         float* positions, void* workspace, unsigned* box_words, cudaStream_t stream) {
+                         float* positions, void* workspace, unsigned* box_words, MortonCube* cube, unsigned* codes, cudaStream_t stream) {
     if (n_cells <= 0 || n_cells >= ((int64_t)1 << 31) || n_total < 0 || n_total >= ((int64_t)1 << 32) || !counts || !centers || !levels || !positions || !workspace) {
         set_error("%s: bad argument", who);
         return INPC_E_INVALID;
@@ -1409,11 +1443,11 @@ static int launch_halton(const char* who, const uint32_t* counts, int64_t n_cell
     if (rc != INPC_OK) return rc;
     if (box_words) {
         const int64_t box_blocks = ceil_div<int64_t>(n_cells, kThreads), box_cap = (int64_t)sm_count() * 8;
-        launch_chained(halton_box_kernel, (unsigned)(box_blocks < box_cap ? box_blocks : box_cap), kThreads, 0, stream, w.counts, (unsigned)n_cells, centers, levels, initial_size, box_words);
+        launch_chained(halton_box_kernel, (unsigned)(box_blocks < box_cap ? box_blocks : box_cap), kThreads, 0, stream, w.counts, (unsigned)n_cells, centers, levels, initial_size, box_words, cube);
         INPC_LAUNCH_CHECK("halton_box_kernel");
     }
-    launch_chained(halton_samples_kernel, (unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream, w.counts, w.offsets,
-                   (unsigned)n_cells, centers, levels, initial_size, (unsigned)n_total, positions);
+    launch_chained(codes ? halton_samples_kernel<true> : halton_samples_kernel<false>, (unsigned)ceil_div<int64_t>(n_total, kRunSlots), kThreads, 0, stream, w.counts, w.offsets,
+                   (unsigned)n_cells, centers, levels, initial_size, (unsigned)n_total, positions, cube, codes);
     INPC_LAUNCH_CHECK("halton_samples_kernel");
     return INPC_OK;
 }
@@ -1421,7 +1455,7 @@ static int launch_halton(const char* who, const uint32_t* counts, int64_t n_cell
 extern "C" int inpc_halton_samples(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size,
                                    int64_t n_total, float* positions, void* workspace, void* stream) {
     if (n_total == 0) return INPC_OK;
-    return launch_halton("inpc_halton_samples", counts, n_cells, centers, levels, initial_size, n_total, positions, workspace, nullptr, static_cast<cudaStream_t>(stream));
+    return launch_halton("inpc_halton_samples", counts, n_cells, centers, levels, initial_size, n_total, positions, workspace, nullptr, nullptr, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t inpc_morton_workspace_bytes(int64_t n) {
@@ -1446,14 +1480,10 @@ MortonWs carve_morton_ws(void* workspace, int64_t n) {
     return w;
 }
 
-// Codes inside the box `mb` (or the one its parts make up), their sort, and the positions in that order.
-int order_along_curve(const char* who, const float* positions, int64_t n, const MortonBox& mb, const MortonWs& w, float* out, cudaStream_t stream) {
-    constexpr int kCodeBits = 30;
-    INPC_CUDA_TRY(cudaMemsetAsync(w.sort_ws, 0, sort_zero_bytes(n, n, kCodeBits), stream));
-    const int64_t code_blocks = ceil_div<int64_t>(n, 4 * kCodeThreads), code_cap = (int64_t)sm_count() * 4;
-    launch_chained(morton_codes_kernel, (unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kCodeThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0,
-                   mb, key_histogram(w.sort_ws, n, n, kCodeBits), w.codes[0], w.order[0]);
-    INPC_LAUNCH_CHECK("morton_codes_kernel");
+constexpr int kCodeBits = 30;
+
+// The codes' sort and the positions in that order.  `counted`: see sort_pairs; the front of the sort's workspace has been cleared.
+int order_along_curve(const char* who, const float* positions, int64_t n, const MortonWs& w, bool counted, float* out, cudaStream_t stream) {
     int in_alt = 0;
     {
         const int rc_prev = check_previous_calls();
@@ -1461,9 +1491,11 @@ int order_along_curve(const char* who, const float* positions, int64_t n, const 
     }
     unsigned* status = acquire_status(who);
     if (!status) return INPC_E_CUDA;
-    const int rc = sort_pairs(w.codes[0], w.codes[1], w.order[0], w.order[1], n, n, kCodeBits, w.sort_ws, true, status, &in_alt, stream, true, true);
+    if (n == 1) INPC_CUDA_TRY(cudaMemsetAsync(w.order[0], 0, sizeof(uint32_t), stream));   // a single pair is not sorted
+    const int rc = sort_pairs(w.codes[0], w.codes[1], w.order[0], w.order[1], n, n, kCodeBits, w.sort_ws, true, status, &in_alt, stream, true, counted);
     if (rc != INPC_OK) return rc;
-    launch_chained(gather_positions_kernel, (unsigned)ceil_div<int64_t>(n, 4 * kThreads), kThreads, 0, stream, positions, w.order[in_alt], n, (reinterpret_cast<uintptr_t>(out) & 15u) == 0, out);
+    launch_chained(gather_positions_kernel, (unsigned)ceil_div<int64_t>(n, 4 * kThreads), kThreads, 0, stream, positions, w.order[in_alt], n,
+                   (reinterpret_cast<uintptr_t>(positions) & 7u) == 0, (reinterpret_cast<uintptr_t>(out) & 15u) == 0, out);
     INPC_LAUNCH_CHECK("gather_positions_kernel");
     return INPC_OK;
 }
@@ -1478,17 +1510,22 @@ extern "C" int inpc_morton_order(const float* positions, int64_t n, const float*
         return INPC_E_INVALID;
     }
     const MortonWs w = carve_morton_ws(workspace, n);
-    MortonBox mb{{0.0f, 0.0f, 0.0f}, 1.0f, w.parts, nullptr, 0};
+    MortonBox mb{{{0.0f, 0.0f, 0.0f}, 1.0f}, w.parts, 0};
     if (box_lo) {
-        for (int k = 0; k < 3; ++k) mb.lo[k] = box_lo[k];
-        mb.inv_extent = 1.0f / box_extent;
+        for (int k = 0; k < 3; ++k) mb.cube.lo[k] = box_lo[k];
+        mb.cube.inv_extent = 1.0f / box_extent;
     } else {
         const int64_t blocks = ceil_div<int64_t>(n, 4 * kThreads), cap = 4 * sm_count() < kMaxBoxBlocks ? 4 * sm_count() : kMaxBoxBlocks;
         mb.box_parts = (int)(blocks < cap ? blocks : cap);
         launch_chained(bounding_box_kernel, mb.box_parts, kThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0, w.parts);
         INPC_LAUNCH_CHECK("bounding_box_kernel");
     }
-    return order_along_curve("inpc_morton_order", positions, n, mb, w, out, stream);
+    INPC_CUDA_TRY(cudaMemsetAsync(w.sort_ws, 0, sort_zero_bytes(n, n, kCodeBits), stream));
+    const int64_t code_blocks = ceil_div<int64_t>(n, 4 * kCodeThreads), code_cap = (int64_t)sm_count() * 4;
+    launch_chained(morton_codes_kernel, (unsigned)(code_blocks < code_cap ? code_blocks : code_cap), kCodeThreads, 0, stream, positions, n, (reinterpret_cast<uintptr_t>(positions) & 15u) == 0,
+                   mb, key_histogram(w.sort_ws, n, n, kCodeBits), w.codes[0]);
+    INPC_LAUNCH_CHECK("morton_codes_kernel");
+    return order_along_curve("inpc_morton_order", positions, n, w, true, out, stream);
 }
 
 extern "C" int inpc_halton_morton_order(const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size, int64_t n_total,
@@ -1500,10 +1537,12 @@ extern "C" int inpc_halton_morton_order(const uint32_t* counts, int64_t n_cells,
         return INPC_E_INVALID;
     }
     const MortonWs w = carve_morton_ws(morton_workspace, n_total);
-    static_assert(kBoxCopies <= kMaxBoxBlocks, "the words of the box lie where the partial boxes would");
+    static_assert(kBoxCopies + 2 <= kMaxBoxBlocks, "words and cube lie where partial boxes would");
     unsigned* words = reinterpret_cast<unsigned*>(w.parts);
-    INPC_CUDA_TRY(cudaMemsetAsync(words, 0, sizeof(unsigned) * 6 * kBoxCopies, stream));
-    const int rc = launch_halton("inpc_halton_morton_order", counts, n_cells, centers, levels, initial_size, n_total, positions, sampler_workspace, words, stream);
+    MortonCube* cube = reinterpret_cast<MortonCube*>(words + 6 * kBoxCopies + 4);   // 16-byte aligned
+    INPC_CUDA_TRY(cudaMemsetAsync(words, 0, sizeof(unsigned) * (6 * kBoxCopies + 1), stream));
+    INPC_CUDA_TRY(cudaMemsetAsync(w.sort_ws, 0, sort_zero_bytes(n_total, n_total, kCodeBits), stream));
+    const int rc = launch_halton("inpc_halton_morton_order", counts, n_cells, centers, levels, initial_size, n_total, positions, sampler_workspace, words, cube, w.codes[0], stream);
     if (rc != INPC_OK) return rc;
-    return order_along_curve("inpc_halton_morton_order", positions, n_total, MortonBox{{0.0f, 0.0f, 0.0f}, 1.0f, nullptr, words, kBoxCopies}, w, out, stream);
+    return order_along_curve("inpc_halton_morton_order", positions, n_total, w, false, out, stream);
 }
