@@ -1475,9 +1475,8 @@ constexpr size_t backward_smem_bytes() {
 // item, so a tile with 100x the average load does not set the critical path.  Pass FIRST blends
 // segment 0 of every tile exactly; the pixels that dense clusters hit stop there.  Pass PRODUCT
 // computes, for the later segments, the per-pixel product of (1 - alpha) over the segment, starting
-// from (and filtering by) the state segment 0 left, so the work it repeats is small; a per-tile
-// prefix turns the products into the transmittance at segment start; pass REST blends the later
-// segments from that state; a per-tile combine adds the segment colours in order (and leaves the
+// from (and filtering by) the state segment 0 left, so the work it repeats is small; pass REST blends the later
+// segments from the transmittance at their start, the product of those in front; a per-tile combine adds the segment colours in order (and leaves the
 // colour prefix for the backward pass, whose items are then independent).
 //
 // An item covers the upper or lower 8x4 half of a tile, one pixel per lane; both halves stream the same
@@ -1882,6 +1881,21 @@ struct CandidateStream {
     }
 };
 
+// Transmittance of a lane's pixel at the start of a later segment of its tile half: the state behind segment 0 times the products of the segments between.  Every item forms it for
+// itself; the loads do not wait for one another.  (A kernel of its own between the passes took 4 to 8 us and a launch: 10^6 samples 380 -> 375 us, 2^25 points 2636 -> 2630.)
+__device__ __forceinline__ float segment_start(const float* __restrict__ seg_T, unsigned first, unsigned half, unsigned seg, unsigned lane) {
+    const float* base = seg_T + ((size_t)first * 2u + half) * 32 + lane;   // segment g of this half: base[g * 64]
+    float run = base[0];
+    for (unsigned g0 = 1; g0 < seg; g0 += 8) {
+        float product[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) product[k] = g0 + k < seg ? base[(size_t)(g0 + k) * 64] : 1.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) run *= product[k];
+    }
+    return run;
+}
+
 // Shared memory of one warp of the forward passes.
 template <bool BLEND, bool WEIGHTS, int DEPTH, int C4>
 struct __align__(16) WarpForwardSmem {
@@ -1964,7 +1978,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
             done = done || T0 < kTransmittanceEps;
             log_stop = done ? 0.0 : log2((double)T0 / (double)kTransmittanceEps) + (double)stop_margin(rg.y - rg.x);
         } else if (PASS == PASS_REST) {
-            Tr = seg_T[sidx * 32 + lane];
+            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
             done = done || Tr < kTransmittanceEps;
         }
         unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
@@ -2177,35 +2191,6 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
                 seg_E[si] = Tr;
             } else if (seg + 1u == n_seg && inside) {
                 alpha_s[pi] = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
-            }
-        }
-    }
-}
-
-// Per tile half with several segments, between the PRODUCT and REST passes: seg_T of segment s >= 1 becomes
-// the transmittance at its start = (state behind segment 0) * product of the segments 1 .. s-1.
-// `n_tiles_at`: where in `counts` the number of tiles to look at is, see tiles_with_segments.
-__global__ void __launch_bounds__(kWarpBlendWarps * 32) warp_blend_prefix_kernel(const WarpItem* __restrict__ items0, const uint32_t* __restrict__ counts, int n_tiles_at,
-                                                                                 float* __restrict__ seg_T) {
-    await_previous_kernel();
-    const unsigned lane = lane_id();
-    const unsigned n_parts = __ldg(counts + n_tiles_at) * 2u;
-    for (unsigned w = blockIdx.x * kWarpBlendWarps + (threadIdx.x >> 5); w < n_parts; w += gridDim.x * kWarpBlendWarps) {
-        const WarpItem it = load_item(items0 + (w >> 1));
-        const unsigned half = w & 1u;
-        const unsigned n_seg = it.n_seg;
-        if (n_seg == 1u) continue;
-        const unsigned first = it.first;
-        float* base = seg_T + ((size_t)first * 2u + half) * 32 + lane;   // segment g of this half: base[g * 64]
-        float run = base[0];
-        for (unsigned g0 = 1; g0 < n_seg; g0 += 8) {
-            float product[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) product[k] = g0 + k + 1u < n_seg ? base[(size_t)(g0 + k) * 64] : 1.0f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (g0 + k < n_seg) base[(size_t)(g0 + k) * 64] = run;
-                run *= product[k];
             }
         }
     }
@@ -2481,7 +2466,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
             C_final = n_seg > 1u ? seg_C[sidx * 32 + lane]
                                  : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
+            if (seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, seg, lane);
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -2661,7 +2646,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
                 G_final += v.x * g[c].x + v.y * g[c].y + v.z * g[c].z + v.w * g[c].w;
             }
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
+            if (seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, seg, lane);
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -3556,7 +3541,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
             done = done || T0 < kTransmittanceEps;
             if (!done) stop = kTransmittanceEps / T0 * (1.0f - stop_margin(rg.y - rg.x));
         } else if (PASS == PASS_REST) {
-            Tr = seg_T[sidx * 32 + lane];
+            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
             done = done || Tr < kTransmittanceEps;
         }
         unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
@@ -3764,7 +3749,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussBackwardBlocks) bl
             Cfin = n_seg > 1u ? seg_C[sidx * 32 + lane]
                               : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
+            if (seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, seg, lane);
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -4417,10 +4402,10 @@ int warp_blend_grid(Kernel kernel, size_t smem, int most, bool bilinear, int pas
     grid->visits = bilinear ? grid->blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u;
     return rc;
 }
-// Tiles of several segments are longer than a first segment, i.e. in the first class where the tiles lie by length: the two small kernels look at no others then
-// (129,600 tiles, few of which have more than one segment: 22 + 12 -> 4 + 5 us).
+// Where in the counts the number of tiles is among which those of several segments lie: they are longer than a first segment, i.e. in the first class where the tiles lie by
+// length, and the combine kernel looks at no others then (129,600 tiles, few of which have more than one segment: 12 -> 5 us, before it blanked empty tiles).
 constexpr int tiles_with_segments(bool by_length) { return by_length ? kLongTiles : 0; }
-unsigned small_grid() { return (unsigned)(sm_count() * 4); }   // of the two small kernels between the passes
+unsigned small_grid() { return (unsigned)(sm_count() * 4); }   // of the combine kernel
 
 struct ForwardPassArgs {
     const uint32_t *keys, *ids;
@@ -4467,8 +4452,6 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     if (rc_pass != INPC_OK) return rc_pass;
     rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(!ROWS), ib.seg_T);
-    INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
     rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     launch_chained(warp_blend_combine_kernel<KIND, C4>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(!ROWS), ib.seg_C, ib.seg_Z, ib.seg_E,
@@ -4557,8 +4540,6 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     if (rc != INPC_OK) return rc;
     rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    launch_chained(warp_blend_prefix_kernel, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(true), ib.seg_T);
-    INPC_LAUNCH_CHECK("warp_blend_prefix_kernel");
     rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
     launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(true), ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
