@@ -2205,6 +2205,263 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
     }
 }
 
+// ---- first and later segments of a training pass: two warps per item ---------------------------------------------
+// What bounds these passes is the chain of instructions of one batch after the other of the longest lists.  Half of it does not depend on the pixels' state: finding the
+// candidates, their records, the pixels they reach and the transposition of those masks.  One warp of a pair does that for the next batch while the other runs down the pixels'
+// lists of this one; they meet at one barrier per batch.
+// Batch b lies in stage b % 3 of the ring (b is walked, b + 1 made ready, b + 2 under way); its words, and whether there is such a batch, in place b % 2, where the state of the pixels before
+// it lies too.  Both warps leave the loop at the same barrier: what they decide by is written before it and not again before the next but one.
+// Step of 2^23 samples at 1237x822, first / later segments 96 / 112 -> 84 / 106 us, 16 channels 156 / 231 -> 156 / 189, 10^6 samples 24 / 34 -> 21 / 34.  Half as many items are under way, so
+// where there are many short ones (more than kManyTiles tiles) or the passes wait for memory (inference) one warp per item is the faster form: 2^24 points crowding a corner of
+// 3840x2160, first segments 255 against 290 us, 2^25 points of a cloud 347 + 109 against 367 + 118.  Four blocks per multiprocessor of 64 registers (of wide rows three): with three
+// 333 us in place of 290, with five (48 registers) 333; four stages the same.
+constexpr int kPairs = kWarpBlendWarps / 2;
+template <int C4>
+struct __align__(16) PairForwardSmem {
+    float4 ring_a[3][32];                        // records of the batches in flight: position, alpha, depth ...
+    float4 ring_f[3][32 * feature_stride(C4)];   // ... and features
+    float4 weight[32];                           // per staged instance: what its pixels add to its blending weight, by parity
+    uint32_t ring_id[3][32];                     // point ids of the batches in flight (0xFFFFFFFF: no instance)
+    unsigned words[2][32];                       // per pixel, the instances of a batch that reach it
+    unsigned stopped[2];                         // pixels that have stopped before a batch
+    unsigned end[2];                             // there is no such batch
+    unsigned item;                               // 0xFFFFFFFF: no more
+    uint32_t queue[kQueueCap];
+};
+template <int C4>
+constexpr size_t pair_forward_smem_bytes() { return 2 * 256 * sizeof(unsigned) + kPairs * sizeof(PairForwardSmem<C4>); }
+__host__ __device__ constexpr int pair_forward_blocks(int c4) { return c4 == 1 ? 4 : c4 == 8 ? 2 : 3; }
+
+__device__ __forceinline__ void pair_barrier(unsigned pair) {
+    __syncwarp();
+    asm volatile("bar.sync %0, 64;" ::"r"(1u + pair) : "memory");
+}
+
+// ROWS: features are rows of 4 C4 channels in `rows` (a (4 C4, H, W) image); otherwise C4 is 1 and they are in the record.
+template <int PASS, int C4, bool ROWS>
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, pair_forward_blocks(C4)) blend_bilinear_pair_forward_kernel(
+    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ inst_keys,
+    const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ rows, float* __restrict__ seg_T, float4* __restrict__ seg_C,
+    float* __restrict__ image, float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1,
+    uint32_t* __restrict__ n_kept, int width, int height, int gw) {
+    await_previous_kernel();
+    static_assert(PASS != PASS_PRODUCT && (ROWS || C4 == 1), "blends; a record holds four channels");
+    constexpr unsigned kFull = 0xffffffffu, kNoInstance = 0xffffffffu, kNoItem = 0xffffffffu;
+    constexpr int kStride = feature_stride(C4);
+    using Smem = PairForwardSmem<C4>;
+    extern __shared__ __align__(16) unsigned char blend_smem[];
+    unsigned* s_reach = reinterpret_cast<unsigned*>(blend_smem);     // [half][key code] -> pixels of the half reached
+    const unsigned lane = lane_id(), pair = threadIdx.x >> 6;
+    const bool prepares = ((threadIdx.x >> 5) & 1u) == 0u;
+    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 2 * 256 * sizeof(unsigned))[pair];
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned parity = (lane & 1u) | ((lane >> 2) & 2u);        // of this lane's pixel: a footprint has each of the four once
+    {
+        const unsigned long long m = key_pixels(threadIdx.x);
+        s_reach[threadIdx.x] = (unsigned)m;
+        s_reach[256 + threadIdx.x] = (unsigned)(m >> 32);
+    }
+    if (!prepares) sm.weight[lane] = make_float4(0.f, 0.f, 0.f, 0.f);   // every batch leaves them at zero again
+    __syncthreads();
+    const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, n_visits, ROWS ? kMostItems : kMostItemsBilinear);
+    for (;;) {
+        if (prepares) {
+            unsigned taken;
+            if (!queue.take(ticket, lane, &taken)) taken = kNoItem;
+            if (lane == 0) sm.item = taken;
+        }
+        pair_barrier(pair);
+        const unsigned item = sm.item;
+        if (item == kNoItem) break;
+        const WarpItem it = load_item(items + (item >> 1));
+        const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg, first = it.first;
+        const int half = (int)(item & 1u);
+        const size_t sidx = (size_t)(first + seg) * 2u + half;      // this item's slot in the per-segment arrays
+        const uint2 rg = make_uint2(it.begin, it.end);
+        const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
+        const int px0 = tx * 8, py0 = ty * 8 + 4 * half;            // first pixel of this half
+        const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+        const bool inside = px < width && py < height;
+
+        if (prepares) {
+            // ---- where the instances come from.  FIRST filters the item's keys; REST blends the list PRODUCT
+            // compacted for this item (a superset of what is still alive at the true transmittance, see above), its ids
+            // loaded kIdsAhead batches ahead of their gather.
+            uint32_t* kept = half ? kept1 : kept0;
+            const unsigned* reach = s_reach + 256 * half;
+            CandidateStream in;
+            uint32_t idf[kIdsAhead];
+            if (PASS == PASS_REST) {
+                in.head = 0u;
+                in.tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
+#pragma unroll
+                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < in.tail ? kept[rg.x + 32u * k + lane] : 0u;
+            } else {
+                in.start(inst_keys, inst_ids, rg.x, rg.y, lane);
+            }
+            pair_barrier(pair);
+            unsigned done_w = sm.stopped[0], n_out = 0;
+            if (done_w != kFull) {   // else: nothing in this list can have an effect
+                auto fill = [&]() {
+                    if (PASS != PASS_REST) in.fill(reach, done_w, sm.queue, lane, lt_mask);
+                    __syncwarp();
+                };
+                // the next (up to) 32 candidates become a batch: their records start to travel into `stage` of the ring
+                auto gather = [&](unsigned stage) {
+                    const unsigned n = min(32u, in.tail - in.head);
+                    uint32_t id = kNoInstance;
+                    if (lane < n) {
+                        id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(in.head + lane) & (kQueueCap - 1)]);
+                        const float4* p = reinterpret_cast<const float4*>(rec) + (size_t)id * (ROWS ? 1 : 2);
+                        async_copy_16(&sm.ring_a[stage][lane], p);
+                        if (!ROWS) async_copy_16(&sm.ring_f[stage][lane], p + 1);
+                    }
+                    if (ROWS) gather_rows<C4>(sm.ring_f[stage], rows, id, lane);
+                    sm.ring_id[stage][lane] = id;
+                    async_copy_commit();   // one group per batch, empty or not: the waits below count groups
+                    if (PASS == PASS_REST) {
+#pragma unroll
+                        for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
+                        const unsigned nxt = in.head + 32u * kIdsAhead + lane;
+                        idf[kIdsAhead - 1] = nxt < in.tail ? kept[rg.x + nxt] : 0u;
+                    }
+                    in.head += n;
+                };
+                fill();
+                gather(0u);
+                fill();
+                gather(1u);
+                unsigned stage = 0u;   // of batch b
+                for (unsigned b = 0;; ++b) {
+                    fill();
+                    async_copy_wait<1>();   // all but the newest group: batch b has arrived
+                    const uint32_t id_cur = sm.ring_id[stage][lane];
+                    const bool staged = id_cur != kNoInstance;
+                    const bool end = __ballot_sync(kFull, staged) == 0u;   // batches are filled in order: nothing is left
+                    if (!end) {
+                        // ---- lane j: the pixels of staged instance j that have not stopped
+                        const float4 own = sm.ring_a[stage][lane];
+                        const unsigned pixels = staged ? footprint_pixels(own.x, own.y, px0, py0) & ~done_w : 0u;
+                        // what reaches a pixel that has not stopped goes into the list of this item, as in blend_bilinear_warp_forward_kernel
+                        const unsigned alive = __ballot_sync(kFull, pixels != 0u);
+                        if (pixels) kept[rg.x + n_out + __popc(alive & lt_mask)] = id_cur;
+                        n_out += __popc(alive);
+                        sm.words[b & 1u][lane] = warp_transpose_bits(pixels, lane);
+                    }
+                    if (lane == 0) sm.end[b & 1u] = end ? 1u : 0u;
+                    pair_barrier(pair);
+                    if (end) break;
+                    done_w = sm.stopped[b & 1u];
+                    if (done_w == kFull) break;   // every pixel has stopped: the rest of the list has no effect
+                    stage = stage == 2u ? 0u : stage + 1u;
+                    gather(stage == 2u ? 0u : stage + 1u);   // batch b + 2, where batch b - 1 lay
+                }
+                async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
+                __syncwarp();
+            }
+            if (lane == 0) n_kept[sidx] = n_out;
+            continue;
+        }
+
+        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
+        float Tr = 1.0f;
+        float4 C[C4];
+#pragma unroll
+        for (int c = 0; c < C4; ++c) C[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool done = !inside;
+        if (PASS == PASS_REST) {
+            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
+            done = done || Tr < kTransmittanceEps;
+        }
+        unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
+        if (lane == 0) sm.stopped[0] = done_w;
+        pair_barrier(pair);
+        if (done_w != kFull) {
+            unsigned stage = 0u;
+            for (unsigned b = 0;; ++b, stage = stage == 2u ? 0u : stage + 1u) {
+                pair_barrier(pair);
+                if (sm.end[b & 1u] || done_w == kFull) break;
+                // ---- every lane runs down the instances of its own pixel, front to back
+                unsigned todo = done ? 0u : sm.words[b & 1u][lane];   // (made before the pixels that stopped in the batch in front of it were known)
+                while (todo) {
+                    // a few at a time, without branches: see blend_bilinear_warp_forward_kernel
+                    constexpr int kChunk = C4 == 1 ? 3 : 2;
+                    int j[kChunk];
+                    float wg[kChunk], al[kChunk];
+                    float4 f[kChunk];
+                    bool ok[kChunk];
+#pragma unroll
+                    for (int u = 0; u < kChunk; ++u) {
+                        ok[u] = todo != 0u;
+                        j[u] = ok[u] ? __ffs(todo) - 1 : j[0];
+                        todo &= todo - 1u;
+                        const float4 a = sm.ring_a[stage][j[u]];
+                        if (C4 == 1) f[u] = sm.ring_f[stage][j[u]];
+                        wg[u] = __saturatef(1.0f - fabsf(a.x - pcx)) * __saturatef(1.0f - fabsf(a.y - pcy));
+                        al[u] = rounded_alpha(a.z, wg[u]);
+                        ok[u] = ok[u] && wg[u] > 0.0f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kChunk; ++u) {
+                        const bool live = ok[u] && !done;
+                        const float bw = Tr * al[u];
+                        if (live && bw > 0.0f) reinterpret_cast<float*>(sm.weight + j[u])[parity] = bw * wg[u];
+                        if (C4 == 1) {
+                            C[0].x = live ? C[0].x + bw * f[u].x : C[0].x;
+                            C[0].y = live ? C[0].y + bw * f[u].y : C[0].y;
+                            C[0].z = live ? C[0].z + bw * f[u].z : C[0].z;
+                            C[0].w = live ? C[0].w + bw * f[u].w : C[0].w;
+                        } else if (live) {
+                            // wide rows are read where they are used: a chunk of them would not fit the registers
+                            const float4* row = sm.ring_f[stage] + j[u] * kStride;
+#pragma unroll
+                            for (int c = 0; c < C4; ++c) {
+                                const float4 v = row[c];
+                                C[c].x += bw * v.x; C[c].y += bw * v.y; C[c].z += bw * v.z; C[c].w += bw * v.w;
+                            }
+                        }
+                        Tr = live ? Tr * (1.0f - al[u]) : Tr;
+                        done = done || Tr < kTransmittanceEps;
+                    }
+                    if (done) todo = 0u;
+                }
+                __syncwarp();
+                // blending weight of every staged instance: its (up to) four pixels in a fixed order
+                const float4 v = sm.weight[lane];
+                const float sum = ((v.x + v.y) + v.z) + v.w;
+                if (sum > 0.0f) {
+                    sm.weight[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    atomicAdd(blending_weights + sm.ring_id[stage][lane], sum);
+                }
+                done_w = __ballot_sync(kFull, done);
+                if (lane == 0) sm.stopped[(b + 1u) & 1u] = done_w;
+            }
+        }
+        const int64_t n_px = (int64_t)width * height, pi = (int64_t)py * width + px;
+        const float alpha = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
+        if (n_seg == 1u) {
+            if (inside) {
+#pragma unroll
+                for (int c = 0; c < C4; ++c) {
+                    float* plane = image + (int64_t)(4 * c) * n_px + pi;
+                    plane[0] = C[c].x;
+                    plane[n_px] = C[c].y;
+                    plane[2 * n_px] = C[c].z;
+                    plane[3 * n_px] = C[c].w;
+                }
+                alpha_image[pi] = alpha;
+            }
+        } else {
+            // partial colour of this segment; the per-tile combine adds the segments up in order
+#pragma unroll
+            for (int c = 0; c < C4; ++c) seg_C[(sidx * C4 + c) * 32 + lane] = C[c];
+            if (PASS == PASS_FIRST) seg_T[sidx * 32 + lane] = Tr;   // the exact state behind segment 0
+            if (seg + 1u == n_seg && inside) alpha_image[pi] = alpha;
+        }
+    }
+}
+
 // Last kernel of the forward passes.  Empty tiles, up to n_tiles (feature rows: none, their images are cleared beforehand): zeros; the passes write every pixel of the others.
 // Per tile half with several segments: image = sum of the segment colours in order.
 // For training the sum of a segment's colour and those behind it replaces the segment's own: what the backward pass takes the
@@ -4462,6 +4719,27 @@ int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsi
     return INPC_OK;
 }
 
+// The same with two warps per item.
+template <int PASS, int C4, bool ROWS>
+int launch_pair_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const ForwardPassArgs& a, cudaStream_t stream) {
+    static int known[kMaxDevices] = {0};
+    constexpr size_t smem = pair_forward_smem_bytes<C4>();
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_bilinear_pair_forward_kernel<PASS, C4, ROWS>, smem, pair_forward_blocks(C4), !ROWS, PASS, known, &grid);
+    if (rc != INPC_OK) return rc;
+    launch_chained(blend_bilinear_pair_forward_kernel<PASS, C4, ROWS>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
+        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.image, a.alpha, a.blending_weights, a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw);
+    INPC_LAUNCH_CHECK("blend_bilinear_pair_forward_kernel");
+    return INPC_OK;
+}
+template <int PASS, int KIND, int C4, bool ROWS>
+int launch_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const ForwardPassArgs& a, bool pairs, cudaStream_t stream) {
+    if constexpr (KIND == BLEND_TRAIN) {
+        if (pairs) return launch_pair_forward_pass<PASS, C4, ROWS>(items, counts, ticket, a, stream);
+    }
+    return launch_warp_forward_pass<PASS, KIND, C4, ROWS>(items, counts, ticket, a, stream);
+}
+
 // C4, `rows`: feature rows of 4 C4 channels (ROWS), or one group of four channels in the records.
 template <int KIND, int C4 = 1, bool ROWS = false>
 int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float4* rows, float* image,
@@ -4476,11 +4754,12 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{keys, ids, pb.rec, rows, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             kept0, kept1, ib.n_kept, W, H, rp.gw, rp.gh};
-    int rc_pass = launch_warp_forward_pass<PASS_FIRST, KIND, C4, ROWS>(ib.items0, ib.n_segments, ib.n_segments + 2, a, stream);
+    const bool pairs = rp.gw * rp.gh <= kManyTiles;   // see blend_bilinear_pair_forward_kernel
+    int rc_pass = launch_forward_pass<PASS_FIRST, KIND, C4, ROWS>(ib.items0, ib.n_segments, ib.n_segments + 2, a, pairs, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
     if (rc_pass != INPC_OK) return rc_pass;
-    rc_pass = launch_warp_forward_pass<PASS_REST, KIND, C4, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 4, a, stream);
+    rc_pass = launch_forward_pass<PASS_REST, KIND, C4, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 4, a, pairs, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     launch_chained(warp_blend_combine_kernel<KIND, C4>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(!ROWS), ib.seg_C, ib.seg_Z, ib.seg_E,
                                                                       image, depth, alpha, W, H, rp.gw, rp.gh, ROWS ? 0 : rp.gw * rp.gh * rp.n_sets);

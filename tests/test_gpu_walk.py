@@ -94,3 +94,39 @@ def test_lists_of_one_footprint(n, opaque, site):
             gf_bound = np.abs(gf_bound) + np.abs(gf) * 2.0 ** -11 + 2.0 ** -25 + 32 * U * np.abs(gf).max(axis=1, keepdims=True)
         off = np.abs(f.grad.double().cpu().numpy() - gf)
         assert (off <= gf_bound + 1e-30).all(), (rows, (off / (gf_bound + 1e-30)).max())
+
+
+# Two warps per list (images of up to 2^15 tiles) against one: the same points in the upper left corner of an image that has more tiles.  Lists of every length beside a batch of 32, of
+# faint splats, of which nothing stops, and of opaque ones, where the pixels stop in the middle of a batch, at its end, and one after the other
+@pytest.mark.parametrize("opacity", [0.004, 0.3, 0.97, None])
+@pytest.mark.parametrize("channels", [None, 4, 8, 16, 32])
+def test_lists_walked_by_two_warps_and_by_one(channels, opacity):
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    width, height = 128, 16
+    lengths = torch.tensor([1, 2, 31, 32, 33, 63, 64, 65, 66, 95, 96, 97, 98, 127, 128, 129, 160, 161, 192, 200, 223, 224, 225, 240, 250, 254, 255, 256, 0, 3, 48, 80])
+    g = torch.Generator().manual_seed(channels or 0)
+    n = int(lengths.sum())
+    tile = torch.repeat_interleave(torch.arange(lengths.numel()), lengths)
+    px, py = (tile % 16) * 8 + torch.rand(n, generator=g) * 6 + 1, (tile // 16) * 8 + torch.rand(n, generator=g) * 6 + 1
+    z = torch.rand(n, generator=g)
+    pos = torch.stack([(px - 64) / 64 * (3 - z), -(py - 8) / 64 * (3 - z), z], dim=1)[torch.randperm(n, generator=g)].contiguous().to(DEV)
+    opac = (torch.rand((n, 1), generator=g) if opacity is None else torch.full((n, 1), opacity)).to(DEV)
+    feats = torch.randn((n, channels or 36), generator=g).to(DEV)
+    feats = feats if channels else (feats * 0.5).half()
+    gi, ga = torch.randn((channels or 4, height, width), generator=g).to(DEV), torch.randn((1, height, width), generator=g).to(DEV)
+    out = []
+    for w, h in ((width, height), (4096, 520)):
+        view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), w, h, 64.0, 64.0, center_x=64.0, center_y=8.0).to(DEV)
+        f, o = feats.clone().requires_grad_(True), opac.clone().requires_grad_(True)
+        rast = inpc_b200.INPCRasterizer()
+        image, alpha, weights = rast.forward_rows(view, pos, f, o) if channels else rast(view, 0, pos, f, o)
+        torch.autograd.backward([image[:, :height, :width], alpha[:, :height, :width]], [gi, ga])
+        out.append((image[:, :height, :width].detach(), alpha[:, :height, :width].detach(), weights, f.grad, o.grad))
+    assert int((out[0][1] > 0).sum()) > 500
+    for k, (a, b) in enumerate(zip(*out)):
+        # images and alphas to the bit, and the gradients of four channels, which have one writer each; the others are sums of up to four atomic additions in any order
+        if k < 2 or (k > 2 and channels is None):
+            assert torch.equal(a, b), k
+        else:
+            assert float((a - b).abs().max()) <= 8 * 2.0 ** -24 * float(torch.maximum(a.abs(), b.abs()).max()), k
