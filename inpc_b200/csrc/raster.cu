@@ -3969,6 +3969,221 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
     }
 }
 
+// First and later segments of a training pass by two warps per item, as in blend_bilinear_pair_forward_kernel.
+struct __align__(16) GaussPairSmem {
+    float4 ring_a[3][32], ring_c[3][32], ring_f[3][32];   // records and conics of the batches in flight
+    float out[32][33];                                    // [staged instance][pixel]: what the fragment adds to the blending weight
+    uint32_t ring_id[3][32];
+    unsigned words[2][32];
+    unsigned stopped[2], end[2], item;
+    uint32_t queue[kQueueCap];
+};
+constexpr size_t kGaussPairSmemBytes = 2 * 256 * sizeof(unsigned) + kPairs * sizeof(GaussPairSmem);
+constexpr int kGaussPairBlocks = 3;
+template <int PASS>
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussPairBlocks) blend_gaussian_pair_forward_kernel(
+    const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ inst_keys,
+    const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T, float4* __restrict__ seg_C,
+    float* __restrict__ image, float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1,
+    uint32_t* __restrict__ n_kept, int width, int height, int gw, float reach) {
+    await_previous_kernel();
+    static_assert(PASS != PASS_PRODUCT, "blends");
+    constexpr unsigned kFull = 0xffffffffu, kNoInstance = 0xffffffffu, kNoItem = 0xffffffffu;
+    using Smem = GaussPairSmem;
+    extern __shared__ __align__(16) unsigned char blend_smem[];
+    unsigned* s_reach = reinterpret_cast<unsigned*>(blend_smem);     // [half][key code] -> pixels of the half reached
+    const unsigned lane = lane_id(), pair = threadIdx.x >> 6;
+    const bool prepares = ((threadIdx.x >> 5) & 1u) == 0u;
+    Smem& sm = reinterpret_cast<Smem*>(blend_smem + 2 * 256 * sizeof(unsigned))[pair];
+    const unsigned lt_mask = (1u << lane) - 1u;
+    {
+        const unsigned long long m = cell_pixels(threadIdx.x);
+        s_reach[threadIdx.x] = (unsigned)m;
+        s_reach[256 + threadIdx.x] = (unsigned)(m >> 32);
+    }
+    __syncthreads();
+    const unsigned n_items = __ldg(counts + (PASS == PASS_FIRST ? 0 : 1)) * 2u;
+    ItemQueue queue(n_items, PASS == PASS_FIRST ? __ldg(counts + kLongTiles + 1) * 2u : 0u, n_visits, kMostItems);
+    for (;;) {
+        if (prepares) {
+            unsigned taken;
+            if (!queue.take(ticket, lane, &taken)) taken = kNoItem;
+            if (lane == 0) sm.item = taken;
+        }
+        pair_barrier(pair);
+        const unsigned item = sm.item;
+        if (item == kNoItem) break;
+        const WarpItem it = load_item(items + (item >> 1));
+        const unsigned tile = it.tile, seg = it.seg, n_seg = it.n_seg, first = it.first;
+        const int half = (int)(item & 1u);
+        const size_t sidx = (size_t)(first + seg) * 2u + half;      // this item's slot in the per-segment arrays
+        const uint2 rg = make_uint2(it.begin, it.end);
+        const int tx = (int)(tile % (unsigned)gw), ty = (int)(tile / (unsigned)gw);
+        const int px0 = tx * 8, py0 = ty * 8 + 4 * half;            // first pixel of this half
+        const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+        const bool inside = px < width && py < height;
+
+        if (prepares) {
+            // ---- where the instances come from.  FIRST filters the item's keys; REST blends the list PRODUCT
+            // compacted for this item (a superset of what is still alive at the true transmittance, see above), its ids
+            // loaded kIdsAhead batches ahead of their gather.
+            uint32_t* kept = half ? kept1 : kept0;
+            const unsigned* reach_of_key = s_reach + 256 * half;
+            CandidateStream in;
+            uint32_t idf[kIdsAhead];
+            if (PASS == PASS_REST) {
+                in.head = 0u;
+                in.tail = n_kept[sidx];     // length of PRODUCT's list; the list itself starts at kept[rg.x]
+#pragma unroll
+                for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < in.tail ? kept[rg.x + 32u * k + lane] : 0u;
+            } else {
+                in.start(inst_keys, inst_ids, rg.x, rg.y, lane);
+            }
+            pair_barrier(pair);
+            unsigned done_w = sm.stopped[0], n_out = 0;
+            if (done_w != kFull) {   // else: nothing in this list can have an effect
+                auto fill = [&]() {
+                    if (PASS != PASS_REST) in.fill(reach_of_key, done_w, sm.queue, lane, lt_mask);
+                    __syncwarp();
+                };
+                // the next (up to) 32 candidates become a batch: their records start to travel into `stage` of the ring
+                auto gather = [&](unsigned stage) {
+                    const unsigned n = min(32u, in.tail - in.head);
+                    uint32_t id = kNoInstance;
+                    if (lane < n) {
+                        id = checked_point(PASS == PASS_REST ? idf[0] : sm.queue[(in.head + lane) & (kQueueCap - 1)]);
+                        const float4* p = reinterpret_cast<const float4*>(rec + id);
+                        async_copy_16(&sm.ring_a[stage][lane], p);
+                        async_copy_16(&sm.ring_c[stage][lane], conic + id);
+                        async_copy_16(&sm.ring_f[stage][lane], p + 1);
+                    }
+                    sm.ring_id[stage][lane] = id;
+                    async_copy_commit();   // one group per batch, empty or not: the waits below count groups
+                    if (PASS == PASS_REST) {
+#pragma unroll
+                        for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
+                        const unsigned nxt = in.head + 32u * kIdsAhead + lane;
+                        idf[kIdsAhead - 1] = nxt < in.tail ? kept[rg.x + nxt] : 0u;
+                    }
+                    in.head += n;
+                };
+                fill();
+                gather(0u);
+                fill();
+                gather(1u);
+                unsigned stage = 0u;   // of batch b
+                for (unsigned b = 0;; ++b) {
+                    fill();
+                    async_copy_wait<1>();   // all but the newest group: batch b has arrived
+                    const uint32_t id_cur = sm.ring_id[stage][lane];
+                    const bool staged = id_cur != kNoInstance;
+                    const bool end = __ballot_sync(kFull, staged) == 0u;   // batches are filled in order: nothing is left
+                    if (!end) {
+                        // ---- lane j: the pixels of staged instance j that have not stopped
+                        const unsigned pixels = staged ? ellipse_pixels(sm.ring_a[stage][lane], sm.ring_c[stage][lane], reach, px0, py0) & ~done_w : 0u;
+                        // what reaches a pixel that has not stopped goes into the list of this item, as in blend_bilinear_warp_forward_kernel
+                        const unsigned alive = __ballot_sync(kFull, pixels != 0u);
+                        if (pixels) kept[rg.x + n_out + __popc(alive & lt_mask)] = id_cur;
+                        n_out += __popc(alive);
+                        sm.words[b & 1u][lane] = warp_transpose_bits(pixels, lane);
+                    }
+                    if (lane == 0) sm.end[b & 1u] = end ? 1u : 0u;
+                    pair_barrier(pair);
+                    if (end) break;
+                    done_w = sm.stopped[b & 1u];
+                    if (done_w == kFull) break;   // every pixel has stopped: the rest of the list has no effect
+                    stage = stage == 2u ? 0u : stage + 1u;
+                    gather(stage == 2u ? 0u : stage + 1u);   // batch b + 2, where batch b - 1 lay
+                }
+                async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
+                __syncwarp();
+            }
+            if (lane == 0) n_kept[sidx] = n_out;
+            continue;
+        }
+
+        const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
+        float Tr = 1.0f;
+        float4 C = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool done = !inside;
+        if (PASS == PASS_REST) {
+            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
+            done = done || Tr < kTransmittanceEps;
+        }
+        unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
+        if (lane == 0) sm.stopped[0] = done_w;
+        pair_barrier(pair);
+        if (done_w != kFull) {
+            unsigned stage = 0u;
+            for (unsigned b = 0;; ++b, stage = stage == 2u ? 0u : stage + 1u) {
+                pair_barrier(pair);
+                if (sm.end[b & 1u] || done_w == kFull) break;
+                // ---- every lane runs down the instances of its own pixel, front to back
+                unsigned todo = done ? 0u : sm.words[b & 1u][lane];   // (made before the pixels that stopped in the batch in front of it were known)
+                unsigned taken = 0u;   // instances whose blending weight this pixel adds to
+                while (todo) {
+                    constexpr int kPair = 2;
+                    int j[kPair];
+                    float al[kPair], G[kPair];
+                    bool ok[kPair];
+#pragma unroll
+                    for (int u = 0; u < kPair; ++u) {
+                        ok[u] = todo != 0u;
+                        j[u] = ok[u] ? __ffs(todo) - 1 : j[0];
+                        todo &= todo - 1u;
+                        const float4 a = sm.ring_a[stage][j[u]], c = sm.ring_c[stage][j[u]];
+                        const float dx = a.x - pcx, dy = a.y - pcy;
+                        const float e = -0.5f * (c.x * dx * dx + c.z * dy * dy) - c.y * dx * dy;
+                        G[u] = expf(e);
+                        ok[u] = ok[u] && !(e > 0.0f) && !(G[u] < kTrainGaussThreshold);
+                        al[u] = rounded_alpha(a.z, G[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kPair; ++u) {
+                        if (!ok[u] || done) continue;
+                        const float bw = Tr * al[u];
+                        if (bw > 0.0f) {
+                            sm.out[j[u]][lane] = G[u] * bw;
+                            taken |= 1u << j[u];
+                        }
+                        const float4 f = sm.ring_f[stage][j[u]];
+                        C.x += bw * f.x; C.y += bw * f.y; C.z += bw * f.z; C.w += bw * f.w;
+                        Tr *= 1.0f - al[u];
+                        if (Tr < kTransmittanceEps) done = true;
+                    }
+                    if (done) todo = 0u;
+                }
+                __syncwarp();
+                unsigned from = warp_transpose_bits(taken, lane);
+                float sum = 0.0f;
+                while (from) {
+                    sum += sm.out[lane][__ffs(from) - 1];
+                    from &= from - 1u;
+                }
+                if (sum > 0.0f) atomicAdd(blending_weights + sm.ring_id[stage][lane], sum);
+                done_w = __ballot_sync(kFull, done);
+                if (lane == 0) sm.stopped[(b + 1u) & 1u] = done_w;
+            }
+        }
+        const int64_t n_px = (int64_t)width * height, pi = (int64_t)py * width + px;
+        const float alpha = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
+        if (n_seg == 1u) {
+            if (inside) {
+                image[pi] = C.x;
+                image[n_px + pi] = C.y;
+                image[2 * n_px + pi] = C.z;
+                image[3 * n_px + pi] = C.w;
+                alpha_image[pi] = alpha;
+            }
+        } else {
+            // partial colour of this segment; the per-tile combine adds the segments up in order
+            seg_C[sidx * 32 + lane] = C;
+            if (PASS == PASS_FIRST) seg_T[sidx * 32 + lane] = Tr;   // the exact state behind segment 0
+            if (seg + 1u == n_seg && inside) alpha_image[pi] = alpha;
+        }
+    }
+}
+
 struct __align__(16) GaussBackwardSmem {
     float4 ring_a[2][32], ring_c[2][32], ring_f[2][32];
     float4 pixel_grad[32];      // image gradient of the half's pixels
@@ -4834,6 +5049,18 @@ int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* cou
     return INPC_OK;
 }
 
+template <int PASS>
+int launch_gaussian_pair_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic, const ForwardPassArgs& a, float reach, cudaStream_t stream) {
+    static int known[kMaxDevices] = {0};
+    BlendGrid grid;
+    const int rc = warp_blend_grid(blend_gaussian_pair_forward_kernel<PASS>, kGaussPairSmemBytes, kGaussPairBlocks, false, PASS, known, &grid);
+    if (rc != INPC_OK) return rc;
+    launch_chained(blend_gaussian_pair_forward_kernel<PASS>, grid.blocks, kWarpBlendWarps * 32, kGaussPairSmemBytes, stream,
+        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.image, a.alpha, a.blending_weights, a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, reach);
+    INPC_LAUNCH_CHECK("blend_gaussian_pair_forward_kernel");
+    return INPC_OK;
+}
+
 template <int KIND>
 int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image, float* depth,
                                  float* alpha, float* blending_weights, float threshold, cudaStream_t stream) {
@@ -4843,11 +5070,14 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{ib.keys[t_alt], ib.ids[t_alt], pb.rec, nullptr, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, W, H, rp.gw, rp.gh};
-    rc = launch_gaussian_warp_forward_pass<PASS_FIRST, KIND>(ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, threshold, rp.reach, stream);
+    const bool pairs = KIND == BLEND_TRAIN && rp.gw * rp.gh <= kManyTiles;
+    rc = pairs ? launch_gaussian_pair_forward_pass<PASS_FIRST>(ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, rp.reach, stream)
+               : launch_gaussian_warp_forward_pass<PASS_FIRST, KIND>(ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
     rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    rc = launch_gaussian_warp_forward_pass<PASS_REST, KIND>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
+    rc = pairs ? launch_gaussian_pair_forward_pass<PASS_REST>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, rp.reach, stream)
+               : launch_gaussian_warp_forward_pass<PASS_REST, KIND>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
     launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(true), ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
                                                                      rp.gw, rp.gh, rp.gw * rp.gh * rp.n_sets);
