@@ -3749,33 +3749,31 @@ __device__ __forceinline__ unsigned ellipse_pixels(const float4& a, const float4
     return m;
 }
 
-template <bool BLEND, bool WEIGHTS>
+// One warp per item: the products, and all passes of inference, which have less to do per fragment (2^22 splats: products 184 us, 199 with two warps; 2 * 10^6 splats of a frame, first
+// segments 151 and 194).
+template <bool BLEND>
 struct __align__(16) GaussForwardSmem {
     float4 ring_a[2][32], ring_c[2][32];              // records and conics of the batches in flight
     float4 ring_f[BLEND ? 2 : 1][BLEND ? 32 : 1];     // ... and features
-    float out[WEIGHTS ? 32 : 1][33];                  // [staged instance][pixel]: what the fragment adds to the blending weight
     uint32_t ring_id[2][32];
     uint32_t queue[kQueueCap];
 };
-template <int PASS, int KIND>
-constexpr size_t gauss_forward_smem_bytes() {
-    return 2 * 256 * sizeof(unsigned) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN>);
-}
+template <int PASS>
+constexpr size_t gauss_forward_smem_bytes() { return 2 * 256 * sizeof(unsigned) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT>); }
 
 template <int PASS, int KIND>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) blend_gaussian_warp_forward_kernel(
     const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ inst_keys,
     const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T,
     float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
-    float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
+    float* __restrict__ alpha_image, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
     int width, int height, int gw, float threshold, float reach) {
     await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     constexpr bool kBlend = PASS != PASS_PRODUCT;
-    constexpr bool kWeights = kBlend && KIND == BLEND_TRAIN;
-    constexpr bool kDepth = kBlend && KIND == BLEND_INFER;
-    using Smem = GaussForwardSmem<kBlend, kWeights>;
+    static_assert(!kBlend || KIND == BLEND_INFER, "training blends by two warps");
+    using Smem = GaussForwardSmem<kBlend>;
     extern __shared__ __align__(16) unsigned char blend_smem[];
     unsigned* s_reach = reinterpret_cast<unsigned*>(blend_smem);     // [half][key code] -> pixels of the half reached
     Smem& sm = reinterpret_cast<Smem*>(blend_smem + 2 * 256 * sizeof(unsigned))[threadIdx.x >> 5];
@@ -3870,7 +3868,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                 unsigned pixels = 0u;
                 if (staged) pixels = ellipse_pixels(sm.ring_a[stage][lane], sm.ring_c[stage][lane], reach, px0, py0) & ~done_w;
                 fill();   // (its __syncwarp also shows every lane the records the others have copied)
-                if (PASS == PASS_PRODUCT || kWeights) {
+                if (PASS == PASS_PRODUCT) {
                     // the list of this item: see the bilinear kernel
                     const unsigned b = __ballot_sync(kFull, pixels != 0u);
                     if (pixels) kept[rg.x + n_out + __popc(b & lt_mask)] = id_cur;
@@ -3878,7 +3876,6 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                 }
                 // ---- every lane runs down the instances of its own pixel, front to back
                 unsigned todo = warp_transpose_bits(pixels, lane);
-                unsigned taken = 0u;   // instances whose blending weight this pixel adds to
                 while (todo) {
                     // a few at a time: their exponentials do not wait for one another (products, three for two: 188 -> 183 us; the other passes the same or slower)
                     constexpr int kPair = PASS == PASS_PRODUCT ? 3 : 2;
@@ -3902,13 +3899,9 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                         if (!ok[u] || done) continue;
                         if (kBlend) {
                             const float bw = Tr * al[u];
-                            if (kWeights && bw > 0.0f) {
-                                sm.out[j[u]][lane] = G[u] * bw;
-                                taken |= 1u << j[u];
-                            }
                             const float4 f = sm.ring_f[stage][j[u]];
                             C.x += bw * f.x; C.y += bw * f.y; C.z += bw * f.z; C.w += bw * f.w;
-                            if (kDepth) Z += bw * sm.ring_a[stage][j[u]].w;
+                            Z += bw * sm.ring_a[stage][j[u]].w;
                         }
                         Tr *= 1.0f - al[u];
                         if (Tr < stop) done = true;
@@ -3916,15 +3909,6 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                     if (done) todo = 0u;
                 }
                 __syncwarp();
-                if (kWeights) {
-                    unsigned from = warp_transpose_bits(taken, lane);
-                    float sum = 0.0f;
-                    while (from) {
-                        sum += sm.out[lane][__ffs(from) - 1];
-                        from &= from - 1u;
-                    }
-                    if (sum > 0.0f) atomicAdd(blending_weights + id_cur, sum);
-                }
                 done_w = __ballot_sync(kFull, done);
                 __syncwarp();
                 if (done_w == kFull) break;   // every pixel has stopped: the rest of the list has no effect
@@ -3932,7 +3916,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
             async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
             __syncwarp();
         }
-        if ((PASS == PASS_PRODUCT || kWeights) && lane == 0) n_kept[sidx] = n_out;
+        if (PASS == PASS_PRODUCT && lane == 0) n_kept[sidx] = n_out;
 
         if (PASS == PASS_PRODUCT) {
             seg_T[sidx * 32 + lane] = Tr;   // this segment's product
@@ -3946,30 +3930,23 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                 image[n_px + pi] = C.y;
                 image[2 * n_px + pi] = C.z;
                 image[3 * n_px + pi] = C.w;
-                if (KIND == BLEND_INFER) {
-                    const float A = 1.0f - Tr;
-                    depth_image[pi] = A > 0.0f ? Z / A : 0.0f;
-                    alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : A;
-                } else {
-                    alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
-                }
+                const float A = 1.0f - Tr;
+                depth_image[pi] = A > 0.0f ? Z / A : 0.0f;
+                alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : A;
             }
         } else {
             // partial colour of this segment; the per-tile combine adds the segments up in order
             const size_t si = sidx * 32 + lane;
             seg_C[si] = C;
             if (PASS == PASS_FIRST) seg_T[si] = Tr;   // the exact state behind segment 0
-            if (KIND == BLEND_INFER) {
-                seg_Z[si] = Z;
-                seg_E[si] = Tr;
-            } else if (seg + 1u == n_seg && inside) {
-                alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
-            }
+            seg_Z[si] = Z;
+            seg_E[si] = Tr;
         }
     }
 }
 
-// First and later segments of a training pass by two warps per item, as in blend_bilinear_pair_forward_kernel.
+// First and later segments of a training pass by two warps per item, as in blend_bilinear_pair_forward_kernel: 2^22 splats at 1237x822 129 / 274 -> 98 / 200 us, the step at 3840x2160
+// (129,600 tiles) 1880 -> 1800.
 struct __align__(16) GaussPairSmem {
     float4 ring_a[3][32], ring_c[3][32], ring_f[3][32];   // records and conics of the batches in flight
     float out[32][33];                                    // [staged instance][pixel]: what the fragment adds to the blending weight
@@ -5038,12 +5015,12 @@ template <int PASS, int KIND>
 int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic,
                                       const ForwardPassArgs& a, float threshold, float reach, cudaStream_t stream) {
     static int known[kMaxDevices] = {0};
-    constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
+    constexpr size_t smem = gauss_forward_smem_bytes<PASS>();
     BlendGrid grid;
     const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, kGaussForwardBlocks, false, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
-        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
+        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, threshold, reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_forward_kernel");
     return INPC_OK;
@@ -5070,14 +5047,16 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{ib.keys[t_alt], ib.ids[t_alt], pb.rec, nullptr, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, W, H, rp.gw, rp.gh};
-    const bool pairs = KIND == BLEND_TRAIN && rp.gw * rp.gh <= kManyTiles;
-    rc = pairs ? launch_gaussian_pair_forward_pass<PASS_FIRST>(ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, rp.reach, stream)
-               : launch_gaussian_warp_forward_pass<PASS_FIRST, KIND>(ib.items0, ib.n_segments, ib.n_segments + 2, pb.conic, a, threshold, rp.reach, stream);
+    auto blend = [&](auto which, const WarpItem* items, int at) -> int {
+        constexpr int kPass = decltype(which)::value;
+        if constexpr (KIND == BLEND_TRAIN) return launch_gaussian_pair_forward_pass<kPass>(items, ib.n_segments, ib.n_segments + at, pb.conic, a, rp.reach, stream);
+        else return launch_gaussian_warp_forward_pass<kPass, KIND>(items, ib.n_segments, ib.n_segments + at, pb.conic, a, threshold, rp.reach, stream);
+    };
+    rc = blend(std::integral_constant<int, PASS_FIRST>{}, ib.items0, 2);
     if (rc != INPC_OK) return rc;
     rc = launch_gaussian_warp_forward_pass<PASS_PRODUCT, KIND>(ib.items1, ib.n_segments, ib.n_segments + 3, pb.conic, a, threshold, rp.reach, stream);
     if (rc != INPC_OK) return rc;
-    rc = pairs ? launch_gaussian_pair_forward_pass<PASS_REST>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, rp.reach, stream)
-               : launch_gaussian_warp_forward_pass<PASS_REST, KIND>(ib.items1, ib.n_segments, ib.n_segments + 4, pb.conic, a, threshold, rp.reach, stream);
+    rc = blend(std::integral_constant<int, PASS_REST>{}, ib.items1, 4);
     if (rc != INPC_OK) return rc;
     launch_chained(warp_blend_combine_kernel<KIND, 1>, grid, threads, 0, stream, ib.items0, ib.n_segments, tiles_with_segments(true), ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, W, H,
                                                                      rp.gw, rp.gh, rp.gw * rp.gh * rp.n_sets);
