@@ -2676,6 +2676,45 @@ __device__ __forceinline__ void footprint_indices(float x, float y, int px0, int
     pix[3] = (unsigned)(odd_row * 8 + odd_column) & 31u;
 }
 
+// Which of the four places for a point's gradients this half writes.  A splat's 2x2 pixels lie in at most two tile columns and two (tile row, half) groups, and which of
+// them this item is follows from where the footprint starts: it holds the left column unless the
+// footprint starts left of it, and the upper row unless it starts above it.  So every (point, slot)
+// has exactly one writer in the whole launch: the sums go there with plain stores, a bit marks the
+// slot as written, and the per-point pass adds the slots in fixed order -- no floating-point
+// atomics, the same gradient bits on every run.
+__device__ __forceinline__ unsigned footprint_slot(float x, float y, int px0, int py0) {
+    return (__float2int_rd(x - 0.5f) < px0 ? 1u : 0u) + (__float2int_rd(y - 0.5f) < py0 ? 2u : 0u);
+}
+
+// Lane j: the sums of instance j over its (up to) four pixels, in a fixed order.
+__device__ __forceinline__ void add_fragments(const FragmentSlots& slots, const float4* pixel_grad, const unsigned (&pix)[4], const float4& wg, unsigned slot, uint32_t id, unsigned lane,
+                                              float4* __restrict__ slot_grad, unsigned* __restrict__ slot_mask) {
+    const float4 in01 = slots.in[lane][0], in23 = slots.in[lane][1], out01 = slots.out[lane][0], out23 = slots.out[lane][1];
+    const float al[4] = {in01.x, in01.z, in23.x, in23.z}, G[4] = {in01.y, in01.w, in23.y, in23.w};
+    const float met[4] = {out01.x, out01.z, out23.x, out23.z}, S[4] = {out01.y, out01.w, out23.y, out23.w};
+    const float w[4] = {wg.x, wg.y, wg.z, wg.w};
+    float4 sf = make_float4(0.f, 0.f, 0.f, 0.f);
+    float so = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (met[c] != 0.0f) {   // (a transmittance that is no number gives a gradient that is none, as in src/bilinear/kernels.cu:361-415)
+            const float bw = met[c] * al[c];
+            so += (met[c] * G[c] + S[c] * one_minus_alpha_reciprocal(1.0f - al[c])) * w[c];   // (two warps per item: 214 us with a division, 207 so)
+            if (bw > 0.0f) {   // (zero times an upstream gradient that has overflowed would be no number)
+                const float4 pg = pixel_grad[pix[c]];
+                sf.x += bw * pg.x; sf.y += bw * pg.y; sf.z += bw * pg.z; sf.w += bw * pg.w;
+            }
+        }
+    }
+    if (sf.x != 0.0f || sf.y != 0.0f || sf.z != 0.0f || sf.w != 0.0f || so != 0.0f) {
+        // one aligned 32-byte record per slot: a whole memory sector, written without reading it first
+        float4* e = slot_grad + ((size_t)id * 4u + slot) * 2u;
+        e[0] = sf;
+        e[1] = make_float4(so, 0.0f, 0.0f, 0.0f);
+        atomicOr(slot_mask + id, 1u << slot);
+    }
+}
+
 // Shared memory of one warp of the backward pass.
 struct __align__(16) WarpBackwardSmem {
     float4 ring_a[kGatherDepthBackward][32];   // records of the batches in flight (see the forward pass): position, alpha ...
@@ -2793,42 +2832,8 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
             // ---- every lane runs down the instances of its own pixel, front to back
             walk_backward(todo, sm.slots, sm.ring_f[stage], parity, g, C_final, K, Tr, C_run, done);
             __syncwarp();
-            // ---- lane j: the sums of instance j over its (up to) four pixels, in a fixed order
-            if (pixels) {
-                const float4 in01 = sm.slots.in[lane][0], in23 = sm.slots.in[lane][1], out01 = sm.slots.out[lane][0], out23 = sm.slots.out[lane][1];
-                const float al[4] = {in01.x, in01.z, in23.x, in23.z}, G[4] = {in01.y, in01.w, in23.y, in23.w};
-                const float met[4] = {out01.x, out01.z, out23.x, out23.z}, S[4] = {out01.y, out01.w, out23.y, out23.w};
-                const float w[4] = {wg.x, wg.y, wg.z, wg.w};
-                float4 sf = make_float4(0.f, 0.f, 0.f, 0.f);
-                float so = 0.0f;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    if (met[c] != 0.0f) {   // (a transmittance that is no number gives a gradient that is none, as in src/bilinear/kernels.cu:361-415)
-                        const float rcp = 1.0f / fmaxf(1.0f - al[c], kOneMinusAlphaEps);
-                        const float bw = met[c] * al[c];
-                        so += (met[c] * G[c] + S[c] * rcp) * w[c];
-                        if (bw > 0.0f) {   // (zero times an upstream gradient that has overflowed would be no number)
-                            const float4 pg = sm.pixel_grad[pix[c]];
-                            sf.x += bw * pg.x; sf.y += bw * pg.y; sf.z += bw * pg.z; sf.w += bw * pg.w;
-                        }
-                    }
-                }
-                const int qx = __float2int_rd(own.x - 0.5f) - px0, qy = __float2int_rd(own.y - 0.5f) - py0;
-                // A splat's 2x2 pixels lie in at most two tile columns and two (tile row, half) groups, and which of
-                // them this item is follows from where the footprint starts: it holds the left column unless the
-                // footprint starts left of it, and the upper row unless it starts above it.  So every (point, slot)
-                // has exactly one writer in the whole launch: the sums go there with plain stores, a bit marks the
-                // slot as written, and the per-point pass adds the slots in fixed order -- no floating-point
-                // atomics, the same gradient bits on every run.
-                if (sf.x != 0.0f || sf.y != 0.0f || sf.z != 0.0f || sf.w != 0.0f || so != 0.0f) {
-                    const unsigned slot_of_point = (qx < 0 ? 1u : 0u) + (qy < 0 ? 2u : 0u);
-                    // one aligned 32-byte record per slot: a whole memory sector, written without reading it first
-                    float4* e = slot_grad + ((size_t)id_cur * 4u + slot_of_point) * 2u;
-                    e[0] = sf;
-                    e[1] = make_float4(so, 0.0f, 0.0f, 0.0f);
-                    atomicOr(slot_mask + id_cur, 1u << slot_of_point);
-                }
-            }
+            // ---- lane j: the sums of instance j
+            if (pixels) add_fragments(sm.slots, sm.pixel_grad, pix, wg, footprint_slot(own.x, own.y, px0, py0), id_cur, lane, slot_grad, slot_mask);
             done_w = __ballot_sync(kFull, done);
             __syncwarp();
             if (done_w == kFull) break;
@@ -2838,7 +2843,171 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
     }
 }
 
-// Backward pass over feature rows, the lists and the walk of the kernel above with a scalar in the place of the running colour: with
+// The same by two warps per item (see blend_bilinear_pair_forward_kernel): one makes the fragments of a batch ready and, a batch later, adds up what the walk has left per instance,
+// the other walks.  Slots and words of batch b lie in place b % 2: those of b - 1 are added up before those of b + 1 take their place.  2^23 samples at 1237x822 232 -> 207 us, 10^6 at
+// 801x533 46 -> 42.  Above kManyTiles tiles one warp per item is the faster form (2^24 points crowding a corner of 3840x2160 382 against 456 us), and for feature rows and Gaussian
+// splats at any number (2^23 samples of 16 channels 328 against 393, 2^22 splats 251 against 274, 288 with the sums where the ellipses are found), since their rings and sums
+// leave room for too few items.  Three blocks per multiprocessor of 80 registers; four of 64 224 us.
+struct __align__(16) PairBackwardSmem {
+    float4 ring_a[3][32];     // records of the batches in flight: position, alpha ...
+    float4 ring_f[3][32];     // ... and features
+    float4 pixel_grad[32];    // image gradient of the half's pixels
+    FragmentSlots slots[2];
+    uint32_t ring_id[3][32];
+    unsigned words[2][32];
+    unsigned stopped[2], end[2], item;
+};
+constexpr size_t kPairBackwardSmemBytes = kPairs * sizeof(PairBackwardSmem);
+constexpr int kPairBackwardBlocks = 3;
+
+__global__ void __launch_bounds__(kWarpBlendWarps * 32, kPairBackwardBlocks) blend_bilinear_pair_backward_kernel(
+    const WarpItem* __restrict__ items0, const WarpItem* __restrict__ items1, const uint32_t* __restrict__ counts,
+    unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ kept0,
+    const uint32_t* __restrict__ kept1, const uint32_t* __restrict__ n_kept, const PointRec* __restrict__ rec,
+    const float* __restrict__ seg_T, const float4* __restrict__ seg_C, const float* __restrict__ grad_image,
+    const float* __restrict__ grad_alpha, const float* __restrict__ image, const float* __restrict__ alpha_image,
+    float4* __restrict__ slot_grad, unsigned* __restrict__ slot_mask, int width, int height, int gw) {
+    await_previous_kernel();
+    constexpr unsigned kFull = 0xffffffffu, kNoInstance = 0xffffffffu, kNoItem = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char blend_smem[];
+    const unsigned lane = lane_id(), pair = threadIdx.x >> 6;
+    const bool prepares = ((threadIdx.x >> 5) & 1u) == 0u;
+    const unsigned parity = (lane & 1u) | ((lane >> 2) & 2u);   // of this lane's pixel: a footprint has each of the four once
+    PairBackwardSmem& sm = reinterpret_cast<PairBackwardSmem*>(blend_smem)[pair];
+    const unsigned n_first = __ldg(counts) * 2u;
+    const unsigned n_items = n_first + __ldg(counts + 1) * 2u;
+    const unsigned n_rest = n_items - n_first;
+
+    // the later segments first (they belong to the longest lists)
+    ItemQueue queue(n_items, n_rest + __ldg(counts + kLongTiles + 1) * 2u, n_visits, kMostItemsBilinear);
+    for (;;) {
+        if (prepares) {
+            unsigned taken;
+            if (!queue.take(ticket, lane, &taken)) taken = kNoItem;
+            if (lane == 0) sm.item = taken;
+        }
+        pair_barrier(pair);
+        const unsigned item = sm.item;
+        if (item == kNoItem) break;
+        const WarpItem it = load_item(item < n_rest ? items1 + (item >> 1) : items0 + ((item - n_rest) >> 1));
+        const int half = (int)((item < n_rest ? item : item - n_rest) & 1u);
+        const size_t sidx = (size_t)(it.first + it.seg) * 2u + half;
+        const unsigned n_list = __ldg(n_kept + sidx);
+        const int tx = (int)(it.tile % (unsigned)gw), ty = (int)(it.tile / (unsigned)gw);
+        const int px0 = tx * 8, py0 = ty * 8 + 4 * half;
+
+        if (prepares) {
+            const uint32_t* list = (half ? kept1 : kept0) + it.begin;
+            // ids kIdsAhead batches ahead of their gather, records two batches ahead of their use
+            uint32_t idf[kIdsAhead];
+#pragma unroll
+            for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < n_list ? __ldg(list + 32u * k + lane) : 0u;
+            pair_barrier(pair);
+            unsigned done_w = sm.stopped[0];
+            if (n_list == 0u || done_w == kFull) continue;
+            unsigned issued = 0;   // instances whose gather has started
+            auto gather = [&](unsigned stage) {
+                const unsigned n = min(32u, n_list - issued);
+                uint32_t id = kNoInstance;
+                if (lane < n) {
+                    id = checked_point(idf[0]);
+                    const float4* p = reinterpret_cast<const float4*>(rec + id);
+                    async_copy_16(&sm.ring_a[stage][lane], p);
+                    async_copy_16(&sm.ring_f[stage][lane], p + 1);
+                }
+                sm.ring_id[stage][lane] = id;
+                async_copy_commit();   // one group per batch, empty or not
+#pragma unroll
+                for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
+                const unsigned nxt = issued + 32u * kIdsAhead + lane;
+                idf[kIdsAhead - 1] = nxt < n_list ? __ldg(list + nxt) : 0u;
+                issued += n;
+            };
+            gather(0u);
+            gather(1u);
+            // lane j: instance j of the batch that is made ready, and of the one in front of it
+            uint32_t id = kNoInstance, id_before = kNoInstance;
+            unsigned pixels = 0u, pixels_before = 0u, pix[4], pix_before[4] = {0u, 0u, 0u, 0u};
+            float4 wg = make_float4(0.f, 0.f, 0.f, 0.f), wg_before = wg;
+            unsigned slot = 0u, slot_before = 0u;
+            unsigned stage = 0u;   // of batch b
+            for (unsigned b = 0;; ++b) {
+                async_copy_wait<1>();   // all but the newest group: batch b has arrived
+                id = sm.ring_id[stage][lane];
+                const bool staged = id != kNoInstance, end = __ballot_sync(kFull, staged) == 0u;
+                pixels = 0u;
+                if (!end) {
+                    // ---- lane j: the fragments of staged instance j
+                    const float4 own = sm.ring_a[stage][lane], fo = sm.ring_f[stage][lane];
+                    wg = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (staged) pixels = footprint_weights(own.x, own.y, px0, py0, wg) & ~done_w;
+                    footprint_indices(own.x, own.y, px0, py0, pix);
+                    slot = footprint_slot(own.x, own.y, px0, py0);
+                    float G[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 pg = sm.pixel_grad[pix[c]];
+                        G[c] = fo.x * pg.x + fo.y * pg.y + fo.z * pg.z + fo.w * pg.w;
+                    }
+                    FragmentSlots& slots = sm.slots[b & 1u];
+                    slots.in[lane][0] = make_float4(rounded_alpha(own.z, wg.x), G[0], rounded_alpha(own.z, wg.y), G[1]);
+                    slots.in[lane][1] = make_float4(rounded_alpha(own.z, wg.z), G[2], rounded_alpha(own.z, wg.w), G[3]);
+                    slots.out[lane][0] = slots.out[lane][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    sm.words[b & 1u][lane] = warp_transpose_bits(pixels, lane);
+                }
+                if (lane == 0) sm.end[b & 1u] = end ? 1u : 0u;
+                pair_barrier(pair);
+                // batch b - 1: the walk is through with it
+                if (pixels_before) add_fragments(sm.slots[(b + 1u) & 1u], sm.pixel_grad, pix_before, wg_before, slot_before, id_before, lane, slot_grad, slot_mask);
+                if (end) break;
+                done_w = sm.stopped[b & 1u];
+                if (done_w == kFull) break;
+                id_before = id; pixels_before = pixels; wg_before = wg; slot_before = slot;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) pix_before[c] = pix[c];
+                __syncwarp();   // batch b + 1 takes the place of b - 1
+                stage = stage == 2u ? 0u : stage + 1u;
+                gather(stage == 2u ? 0u : stage + 1u);   // batch b + 2
+            }
+            async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
+            __syncwarp();
+            continue;
+        }
+
+        const int px = px0 + (int)(lane & 7u), py = py0 + (int)(lane >> 3);
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f), C_final = g, C_run = g;
+        float K = 0.0f, Tr = 1.0f;
+        bool done = !(px < width && py < height);
+        if (!done && n_list > 0u) {
+            const int64_t n_px = (int64_t)width * height;
+            const int64_t pi = (int64_t)py * width + px;
+            g = make_float4(__ldg(grad_image + pi), __ldg(grad_image + n_px + pi), __ldg(grad_image + 2 * n_px + pi),
+                            __ldg(grad_image + 3 * n_px + pi));
+            // what this segment and the ones behind it add to the pixel: the running colour starts at zero
+            C_final = it.n_seg > 1u ? seg_C[sidx * 32 + lane]
+                                    : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
+            K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
+            if (it.seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, it.seg, lane);
+            done = Tr < kTransmittanceEps;
+        }
+        sm.pixel_grad[lane] = g;
+        unsigned done_w = __ballot_sync(kFull, done);
+        if (lane == 0) sm.stopped[0] = done_w;
+        pair_barrier(pair);
+        if (n_list == 0u || done_w == kFull) continue;
+        unsigned stage = 0u;
+        for (unsigned b = 0;; ++b, stage = stage == 2u ? 0u : stage + 1u) {
+            pair_barrier(pair);
+            if (sm.end[b & 1u] || done_w == kFull) break;
+            // ---- every lane runs down the instances of its own pixel, front to back
+            walk_backward(done ? 0u : sm.words[b & 1u][lane], sm.slots[b & 1u], sm.ring_f[stage], parity, g, C_final, K, Tr, C_run, done);
+            done_w = __ballot_sync(kFull, done);
+            if (lane == 0) sm.stopped[(b + 1u) & 1u] = done_w;
+        }
+    }
+}
+
+// Backward pass over feature rows, the lists and the walk of the kernels above with a scalar in the place of the running colour: with
 // G = <g, .> over the channels, dL/dalpha = T G(f) + (G(C_run) - G(C_final) + K) / (1 - alpha).  G(f) is formed per instance and pixel,
 // and so is the gradient of a point's row, sum over its pixels of weight * g, with every staged lane busy.
 // A splat whose 2x2 pixels all lie in this 8x4 half has no other writer in the launch and stores its row; the others
@@ -4962,14 +5131,20 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
 int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
-    static int known[kMaxDevices] = {0};
-    BlendGrid grid;
-    const int rc = warp_blend_grid(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, kBackwardBlocks, true, PASS_FIRST, known, &grid);
+    auto launch = [&](auto kernel, size_t smem, int most, int (&known)[kMaxDevices]) -> int {
+        BlendGrid grid;
+        const int rc = warp_blend_grid(kernel, smem, most, true, PASS_FIRST, known, &grid);
+        if (rc != INPC_OK) return rc;
+        launch_chained(kernel, grid.blocks, kWarpBlendWarps * 32, smem, stream,
+            ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
+            ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, rp.v.width, rp.v.height, rp.gw);
+        return INPC_OK;
+    };
+    static int known[kMaxDevices] = {0}, known_pairs[kMaxDevices] = {0};
+    const int rc = rp.gw * rp.gh <= kManyTiles ? launch(blend_bilinear_pair_backward_kernel, kPairBackwardSmemBytes, kPairBackwardBlocks, known_pairs)
+                                               : launch(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, kBackwardBlocks, known);
     if (rc != INPC_OK) return rc;
-    launch_chained(blend_bilinear_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kWarpBackwardSmemBytes, stream,
-        ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
-        ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, rp.v.width, rp.v.height, rp.gw);
-    INPC_LAUNCH_CHECK("blend_bilinear_warp_backward_kernel");
+    INPC_LAUNCH_CHECK("blend_bilinear backward");
     return INPC_OK;
 }
 
