@@ -1546,7 +1546,7 @@ __device__ __forceinline__ float stop_margin(unsigned len) { return fmaxf(1e-4f,
 enum { PASS_FIRST = 0, PASS_PRODUCT = 1, PASS_REST = 2 };
 // Launch bounds of the passes: blocks per multiprocessor that the registers must leave room for.
 __host__ __device__ constexpr int forward_blocks(int pass, int c4) { return pass == PASS_PRODUCT ? 4 : c4 == 8 ? 2 : 3; }
-__host__ __device__ constexpr int rows_backward_blocks(int c4) { return c4 == 8 ? 1 : c4 == 4 ? 2 : 3; }   // 16 and 32 channels: as many as have shared memory
+__host__ __device__ constexpr int rows_backward_blocks(int c4) { return c4 == 8 ? 1 : c4 == 4 ? 2 : 3; }   // 16 and 32 channels: one more takes L1 from the rows and registers from their sums (321 -> 360, 543 -> 586 us)
 constexpr int kBackwardBlocks = 3, kGaussForwardBlocks = 3, kGaussBackwardBlocks = 2;
 constexpr float kLogScale = 67108864.0f;   // 2^26, see the product of pass PRODUCT
 constexpr float kLogNaN = 1048576.0f;      // far above what 32 factors add up to
@@ -3012,13 +3012,14 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kPairBackwardBlocks) ble
 // and so is the gradient of a point's row, sum over its pixels of weight * g, with every staged lane busy.
 // A splat whose 2x2 pixels all lie in this 8x4 half has no other writer in the launch and stores its row; the others
 // (about a third) add theirs with one vector atomic per four channels.
+// Records and rows are read once, where a batch is made ready: the next batch travels into their place while this one is walked and added up, which leaves the L1 cache more for the rows that
+// neighbouring halves share (2^23 samples of 16 channels 330 -> 321 us against a ring of two batches, 4 channels 301 -> 296, 32 the same).
 template <int C4>
 struct __align__(16) RowsBackwardSmem {
-    float4 ring_a[kGatherDepthBackward][32];
-    float4 ring_f[kGatherDepthBackward][32 * feature_stride(C4)];
+    float4 ring_a[32];                            // records of the batch that is under way
+    float4 ring_f[32 * feature_stride(C4)];       // ... and their rows
     float4 pixel_grad[32 * feature_stride(C4)];   // image gradient of the half's pixels
     FragmentSlots slots;
-    uint32_t ring_id[kGatherDepthBackward][32];
 };
 template <int C4>
 constexpr size_t rows_warp_backward_smem_bytes() { return kWarpBlendWarps * sizeof(RowsBackwardSmem<C4>); }
@@ -3034,7 +3035,6 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
     await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
-    constexpr int kGatherDepth = kGatherDepthBackward;
     constexpr int kStride = feature_stride(C4);
     extern __shared__ __align__(16) unsigned char blend_smem[];
     const unsigned lane = lane_id();
@@ -3094,41 +3094,39 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
 #pragma unroll
         for (int k = 0; k < kIdsAhead; ++k) idf[k] = 32u * k + lane < n_list ? __ldg(list + 32u * k + lane) : 0u;
         unsigned issued = 0;
-        auto gather = [&](unsigned stage) {
+        uint32_t id_next = kNoInstance;   // of the batch that is under way
+        auto gather = [&]() {
             const unsigned n = min(32u, n_list - issued);
             uint32_t id = kNoInstance;
             if (lane < n) {
                 id = checked_point(idf[0]);
-                async_copy_16(&sm.ring_a[stage][lane], reinterpret_cast<const float4*>(rec) + id);
+                async_copy_16(&sm.ring_a[lane], reinterpret_cast<const float4*>(rec) + id);
             }
-            gather_rows<C4>(sm.ring_f[stage], rows, id, lane);
-            sm.ring_id[stage][lane] = id;
-            async_copy_commit();   // one group per batch, empty or not
+            gather_rows<C4>(sm.ring_f, rows, id, lane);
+            id_next = id;
+            async_copy_commit();
 #pragma unroll
             for (int k = 0; k + 1 < kIdsAhead; ++k) idf[k] = idf[k + 1];
             const unsigned nxt = issued + 32u * kIdsAhead + lane;
             idf[kIdsAhead - 1] = nxt < n_list ? __ldg(list + nxt) : 0u;
             issued += n;
         };
-#pragma unroll
-        for (int st = 0; st + 1 < kGatherDepth; ++st) gather((unsigned)st);
-        for (unsigned batch = 0;; ++batch) {
-            gather((batch + kGatherDepth - 1) & (kGatherDepth - 1));
-            async_copy_wait<kGatherDepth - 1>();
-            const unsigned stage = batch & (kGatherDepth - 1);
-            const uint32_t id_cur = sm.ring_id[stage][lane];
+        gather();
+        for (;;) {
+            async_copy_wait<0>();
+            const uint32_t id_cur = id_next;
             const bool staged = id_cur != kNoInstance;
             if (__ballot_sync(kFull, staged) == 0u) break;
             __syncwarp();   // every lane sees what the others have copied
             // ---- lane j: the fragments of staged instance j in the pixels that have not stopped
-            const float4 own = sm.ring_a[stage][lane];
+            const float4 own = sm.ring_a[lane];
             float4 wg = make_float4(0.f, 0.f, 0.f, 0.f);
             unsigned pixels = 0u, pix[4];
             if (staged) pixels = footprint_weights(own.x, own.y, px0, py0, wg) & ~done_w;
             footprint_indices(own.x, own.y, px0, py0, pix);
             {
                 float G[4] = {0.f, 0.f, 0.f, 0.f};
-                const float4* row = sm.ring_f[stage] + lane * kStride;
+                const float4* row = sm.ring_f + lane * kStride;
 #pragma unroll
                 for (int c = 0; c < C4; ++c) {
                     const float4 f = row[c];
@@ -3146,6 +3144,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
             }
             const unsigned todo = warp_transpose_bits(pixels, lane);
             __syncwarp();
+            gather();   // the next batch, where this one lay: nobody reads its records and rows any more
             // ---- every lane runs down the instances of its own pixel, front to back
             walk_backward(todo, sm.slots, parity, G_final, K, Tr, G_run, done);
             __syncwarp();
