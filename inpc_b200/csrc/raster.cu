@@ -684,12 +684,14 @@ __global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint3
 
 // Bilinear splats whose codes the depth sort has carried along: no gather, but where a code does not say it all (one splat in 500 at 1237x822).  A thread takes four
 // consecutive points, the loads of the next group under way while this one's instances are written; a warp stages its instances in shared memory and writes them side
-// by side.  Bound by instruction issue: 2^20 / 2^23 / 2^25 points 11.5 / 47 / 166 us (16 / 95 / 412 with the kernel above; 43 million instances in 166 us are 3.7 TB/s read and
+// by side.  Bound by instruction issue: 2^20 / 2^23 / 2^25 points 11.5 / 44 / 160 us (16 / 95 / 412 with the kernel above; 43 million instances in 160 us are 3.8 TB/s read and
 // written).  What the sort pays for it: 0.2 us of 66 for 2^23 points, 13 of 220 for 2^25, where the words it reads come from DRAM.
-// Two points per thread 54 / 216 us for 2^23 / 2^25; 256 staged pairs per warp and four blocks 58 / 201; no loads ahead 52 / 188; codes of a grid that is one pixel
+// With three blocks (47 / 166 us): two points per thread 54 / 216 us for 2^23 / 2^25; 256 staged pairs per warp and four blocks 58 / 201; no loads ahead 52 / 188; codes of a grid that is one pixel
 // larger, which name the splats at the border too but take a division, 59 / 207.  With the gathers of the kernel above this form is the slower one: 2^24 points 193 -> 408 us,
 // fewer and busier warps miss L2 more often.
-constexpr int kCodedThreads = 512, kCodedPoints = 4, kCodedBlocks = 3;
+// Two blocks per multiprocessor, which stage 128 of its 228 KB: three take 47 / 163 us alone and leave no room for blocks of other streams' kernels until they end (64 views of 2^23
+// samples, four in flight: 1.388 ms per view with three, 1.251 with two, 1.246 with one, which takes longer alone: a view at a time 1.475 / 1.472 / 1.488).
+constexpr int kCodedThreads = 512, kCodedPoints = 4, kCodedBlocks = 2;
 struct EmitCodedSmem {
     uint2 pairs[kCodedThreads / 32][32 * kCodedPoints * 4];   // the most a warp's points can make
 };
