@@ -256,6 +256,12 @@ int inpc_sort_pairs_static_status(void* stream, unsigned* words);
  * in the reference (cub's look-back spins without a limit). */
 int inpc_debug_sort_lookback_timeout(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt,
                                      int64_t n, int end_bit, void* workspace, long long* ticket, void* stream);
+/* The same for the sorts inside the rasterizer, whose number of pairs is in device memory: *count = n at the call, and zero
+ * behind it, so that nothing reads a list with holes.  `marked`: as the depth sort, which sorts positions (values is
+ * scratch).  This hook has no counterpart in the reference. */
+int inpc_debug_counted_sort_lookback_timeout(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt,
+                                             int64_t n, unsigned long long* count, int marked, int end_bit, void* workspace,
+                                             long long* ticket, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Probability-field sampler

@@ -60,6 +60,7 @@ PROTOTYPES = {
     "inpc_sort_pairs_static": (_I, [_P, _P, _P, _P, _L, _I, C.POINTER(C.c_int), _P]),
     "inpc_sort_pairs_static_status": (_I, [_P, C.POINTER(C.c_uint)]),
     "inpc_debug_sort_lookback_timeout": (_I, [_P, _P, _P, _P, _L, _I, _P, C.POINTER(C.c_longlong), _P]),
+    "inpc_debug_counted_sort_lookback_timeout": (_I, [_P, _P, _P, _P, _L, _P, _I, _I, _P, C.POINTER(C.c_longlong), _P]),
     "inpc_last_call_ticket": (C.c_longlong, []),
     "inpc_call_status": (_I, [C.c_longlong, C.POINTER(C.c_uint)]),
     "inpc_sampler_exhausted": (_I, [_P]),

@@ -118,7 +118,7 @@ inline ViewParams to_params(const inpc_view* v) {
 // ---- radix sort (radix_sort.cu) ------------------------------------------------------------
 // The workspace for n pairs (an upper bound) of which n_likely are expected: the expectation picks the tile size, no more.
 size_t sort_workspace_bytes(int64_t n, int64_t n_likely);
-int sort_pass_count(int end_bit);   // passes sort_pairs makes; the result is in the alternate buffers iff odd (and n > 1)
+int sort_pass_count(int end_bit);   // passes a sort makes; the result is in the alternate buffers iff odd (sort_pairs: and n > 1)
 // `status`: device address of the STATUS_WORDS words a tile that gives up its look-back reports to.
 // `n_likely`: the one the workspace was sized with (for at least n pairs).  `zeroed`: the caller has cleared the first
 // sort_zero_bytes(n, n_likely, end_bit) bytes of the workspace.
@@ -147,7 +147,7 @@ KeyHistogram key_histogram(void* workspace, int64_t n, int64_t n_likely, int end
 // keys have been counted (key_histogram(workspace, n, n, end_bit)), how many there are is in *count (device memory).  The workspace is sized for (n, n); the result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd.  No key that takes part may equal kNoKey, also in bits above end_bit.
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
-int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, void* workspace,
+int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
                      unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The same, and every point carries a code with it: the first pass makes it from the point's footprint word (see Footprint in raster.cu), and code and position go
 // through the other passes in one 64-bit word with the key bits that are still to be sorted by (the first pass's own are no longer needed), so that whoever
@@ -161,12 +161,14 @@ struct CarriedCodes {
 // The codes for n points with keys of end_bit bits and words below `words`; none (bits == 0) where key bits behind the first pass, code and position do
 // not fit 64 bits.
 CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t words);
-int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, const CarriedCodes& codes,
+int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes& codes,
                                 void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream);
 // The number of pairs is *n_dev (device memory, <= n_max); the workspace is sized for (n_max, n_likely).  The result is in the
 // alternate buffers iff sort_pass_count(end_bit) is odd, whatever the count turns out to be.
+// Of this sort and of the marked ones: a tile that gives up its look-back leaves zero in the count.  Whatever reads the sorted lists has to take their length from there,
+// in device memory: positions and keys that were not written are anything.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
-                            const unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
+                            unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
                             cudaStream_t stream, bool counted = false);
 
 // More than 48 KB of dynamic shared memory is an opt-in per kernel AND per device: `done` is the

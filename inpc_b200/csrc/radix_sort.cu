@@ -121,8 +121,8 @@ __device__ __forceinline__ unsigned tiles_log2_of_escaped(uint32_t q) { return (
 template <int BITS, int ITEMS, int FORM>
 __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-    uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n_arg, const unsigned long long* __restrict__ n_dev,
-    int shift, int bits_arg, const unsigned* __restrict__ digit_base, volatile unsigned* tile_state, unsigned* ticket,
+    uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n_arg, const unsigned long long* n_dev,
+    int shift, int bits_arg, const unsigned* __restrict__ digit_base, volatile unsigned* tile_state, unsigned* ticket, unsigned long long* withdraw,
     volatile unsigned* status, int spin_limit, unsigned mute_tile, const PackedFields fields) {
     await_previous_kernel();
     constexpr bool MARKED = FORM == PASS_MARKED || FORM == PASS_PACK;
@@ -274,7 +274,11 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
                     }
                     j -= kWindow;
                 }
-                if (gave_up) status[STATUS_LOOKBACK_TIMEOUT] = 1u;
+                if (gave_up) {
+                    status[STATUS_LOOKBACK_TIMEOUT] = 1u;
+                    // what is sorted now has holes that hold whatever lay there: whoever reads the count finds nothing to read
+                    if (withdraw) *withdraw = 0ull;
+                }
                 tile_state[tile * kBins + tid] = ((exclusive + total) & kValueMask) | kFlagPrefix;
             }
             s.global_off[tid] = __ldg(digit_base + tid) + exclusive - start;
@@ -376,6 +380,7 @@ struct PassArgs {
     int shift, bits;
     const unsigned* base;
     unsigned *state, *ticket, *status;
+    unsigned long long* withdraw;   // the count in device memory, or null: zero once a tile has given up
     int form;              // PASS_...
     PackedFields fields;   // of PASS_PACK and PASS_UNPACK
     int spin_limit;        // polls a tile spends on one unpublished predecessor before it gives up
@@ -390,7 +395,7 @@ int launch_onesweep_instance(const PassArgs& a, cudaStream_t stream) {
     if (rc != INPC_OK) return rc;
     const int64_t resident = (int64_t)sm_count() * 2;
     launch_chained(radix_onesweep_pass_kernel<BITS, ITEMS, FORM>, (unsigned)(a.tiles < resident ? a.tiles : resident), kThreads, kSmemBytes, stream,
-        a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base, a.state, a.ticket, a.status, a.spin_limit, a.mute_tile, a.fields);
+        a.kin, a.vin, a.kout, a.vout, a.n, a.n_dev, a.shift, a.bits, a.base, a.state, a.ticket, a.withdraw, a.status, a.spin_limit, a.mute_tile, a.fields);
     INPC_LAUNCH_CHECK("radix_onesweep_pass_kernel");
     return INPC_OK;
 }
@@ -488,7 +493,7 @@ static int check_sort_args(const char* who, const uint32_t* keys, const uint32_t
 // `items`: pairs per thread of a tile, the value the workspace was sized with.
 static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, int end_bit,
                            int items, void* workspace, bool zeroed, unsigned* status, int* result_in_alt, cudaStream_t stream, int spin_limit = kSpinLimit,
-                           unsigned mute_tile = 0xFFFFFFFFu, const unsigned long long* n_dev = nullptr, bool position_values = false, const unsigned long long* marked_count = nullptr, bool counted = false, const CarriedCodes* codes = nullptr) {
+                           unsigned mute_tile = 0xFFFFFFFFu, unsigned long long* n_dev = nullptr, bool position_values = false, unsigned long long* marked_count = nullptr, bool counted = false, const CarriedCodes* codes = nullptr) {
     if (result_in_alt) *result_in_alt = 0;
     if (!workspace || !status) { set_error("%s: null workspace", who); return INPC_E_INVALID; }
 
@@ -508,6 +513,7 @@ static int sort_pairs_with(const char* who, uint32_t* keys, uint32_t* keys_alt, 
     PassArgs a;
     a.tiles = tiles; a.n = n; a.n_dev = n_dev; a.status = status;
     a.spin_limit = spin_limit; a.mute_tile = mute_tile;
+    a.withdraw = marked_count ? marked_count : n_dev;
     a.kin = keys; a.kout = keys_alt; a.vin = position_values || marked_count ? nullptr : values; a.vout = values_alt;
     a.state = w.state;
     a.fields = {end_bit, bit_length((uint32_t)(n - 1)), codes ? *codes : CarriedCodes{}};
@@ -555,7 +561,7 @@ CarriedCodes carried_codes(const uint32_t* quad, int64_t n, int end_bit, int64_t
 }
 
 // (one pair is sorted like more: how many take part is not known here)
-static int sort_marked(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, const CarriedCodes* codes,
+static int sort_marked(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes* codes,
                        void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream) {
     if (result_in_alt) *result_in_alt = 0;
     bool nothing = false;
@@ -569,12 +575,12 @@ static int sort_marked(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uin
                            0xFFFFFFFFu, nullptr, true, count, true, codes);
 }
 
-int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, void* workspace,
+int sort_marked_keys(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, void* workspace,
                      unsigned* status, int* result_in_alt, cudaStream_t stream) {
     return sort_marked(keys, keys_alt, values, values_alt, n, count, end_bit, nullptr, workspace, status, result_in_alt, stream);
 }
 
-int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, const unsigned long long* count, int end_bit, const CarriedCodes& codes,
+int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count, int end_bit, const CarriedCodes& codes,
                                 void* workspace, unsigned* status, int* result_in_alt, cudaStream_t stream) {
     return sort_marked(keys, keys_alt, values, values_alt, n, count, end_bit, &codes, workspace, status, result_in_alt, stream);
 }
@@ -583,7 +589,7 @@ int sort_marked_keys_with_codes(uint32_t* keys, uint32_t* keys_alt, uint32_t* va
 // sized for n_max, the kernels read the count themselves, and the result is always in the alternate buffers iff
 // the number of passes is odd.  No host synchronisation anywhere.
 int sort_pairs_device_count(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n_max, int64_t n_likely,
-                            const unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
+                            unsigned long long* n_dev, int end_bit, void* workspace, bool zeroed, unsigned* status, int* result_in_alt,
                             cudaStream_t stream, bool counted) {
     if (result_in_alt) *result_in_alt = 0;
     if (n_max <= 0 || end_bit == 0) return INPC_OK;
@@ -695,6 +701,21 @@ extern "C" int inpc_debug_sort_lookback_timeout(uint32_t* keys, uint32_t* keys_a
     if (!status) return INPC_E_CUDA;
     return sort_pairs_with("inpc_debug_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, false, status, nullptr,
                            static_cast<cudaStream_t>(stream), 1 << 10, 0u);
+}
+
+// The same for the sorts whose count is in device memory: all n keys, of which *count say there are n; `marked` as in a depth sort (no key equals kNoKey, the values are the
+// positions).  The tiles that give up leave *count at zero, and the passes behind them, and whoever else reads the count, find nothing to do.
+extern "C" int inpc_debug_counted_sort_lookback_timeout(uint32_t* keys, uint32_t* keys_alt, uint32_t* values, uint32_t* values_alt, int64_t n, unsigned long long* count,
+                                                        int marked, int end_bit, void* workspace, long long* ticket, void* stream) {
+    using namespace inpc;
+    bool nothing = false;
+    int rc = check_sort_args("inpc_debug_counted_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, &nothing);
+    if (rc != INPC_OK) return rc;
+    if (nothing || !workspace || !count || !ticket) { set_error("inpc_debug_counted_sort_lookback_timeout: needs n > 1, end_bit > 0, a workspace, a count and a ticket pointer"); return INPC_E_INVALID; }
+    unsigned* status = acquire_status("inpc_debug_counted_sort_lookback_timeout", ticket);
+    if (!status) return INPC_E_CUDA;
+    return sort_pairs_with("inpc_debug_counted_sort_lookback_timeout", keys, keys_alt, values, values_alt, n, end_bit, tile_items(n), workspace, false, status, nullptr,
+                           static_cast<cudaStream_t>(stream), 1 << 10, 0u, marked ? nullptr : count, false, marked ? count : nullptr);
 }
 
 // Status words of the last inpc_sort_pairs_static call on the current device, copied out of the fixed array

@@ -521,11 +521,10 @@ enum { COUNTS_GATHERED = 0, COUNTS_IN_KEYS = 1, COUNTS_IN_CODES = 2, COUNTS_IN_G
 template <int SOURCE>
 __global__ void __launch_bounds__(kInstThreads / 4) instance_count_kernel(const uint32_t* __restrict__ sorted_keys,
                                                                           const uint32_t* __restrict__ sorted_ids,
-                                                                          const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
-                                                                          const unsigned long long* __restrict__ n_visible_dev,
+                                                                          const uint2* __restrict__ bounds, const uint32_t* __restrict__ quad, const unsigned long long* __restrict__ n_visible_dev,
                                                                           unsigned* block_sums, unsigned n_groups, unsigned* done, unsigned long long* n_instances, uint32_t escape) {
     await_previous_kernel();
-    const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
+    const int64_t n_visible = (int64_t)*n_visible_dev;
     constexpr unsigned kWarps = kInstThreads / 4 / 32;
     if (SOURCE != COUNTS_GATHERED) {
         auto count_of = [&](uint32_t word) -> unsigned {
@@ -636,14 +635,13 @@ __device__ __forceinline__ unsigned cell_code(int left, int right, int top, int 
 // histogram of 2^20 / 2^23 / 2^24 / 2^25 points 21 / 104 / 207 / 496 -> 16 / 95 / 192 / 412 us (half of the last by fewer blocks).
 // (Four consecutive points per thread with their gathers in flight together and the instances staged in shared memory: the emission alone 116 us for
 // 2^23 points, 396 for 2^24, 952 for 2^25.)
-__global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ quad, int64_t n_visible_arg,
-                                                                     const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
+__global__ void __launch_bounds__(kInstThreads, 2) emit_quads_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ quad, const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
                                                                      KeyHistogram digits, unsigned long long* __restrict__ n_emitted, uint32_t* __restrict__ inst_keys,
                                                                      uint32_t* __restrict__ inst_ids) {
     await_previous_kernel();
     __shared__ unsigned s_total[2][kInstThreads / 32];   // of two groups in turn, so that one barrier does
     __shared__ BlockHistogram s_digits;
-    const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
+    const int64_t n_visible = (int64_t)*n_visible_dev;
     const int64_t n_groups = ceil_div<int64_t>(n_visible, kInstThreads);
     if ((int64_t)blockIdx.x >= n_groups) return;
     clear_histogram(s_digits);
@@ -696,7 +694,7 @@ struct EmitCodedSmem {
     uint2 pairs[kCodedThreads / 32][32 * kCodedPoints * 4];   // the most a warp's points can make
 };
 __global__ void __launch_bounds__(kCodedThreads, kCodedBlocks) emit_coded_kernel(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ sorted_codes, const CarriedCodes codes,
-                                                                      int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
+                                                                      const unsigned long long* __restrict__ n_visible_dev, const unsigned* __restrict__ block_base, int gw,
                                                                       KeyHistogram digits, unsigned long long* __restrict__ n_emitted, uint32_t* __restrict__ inst_keys,
                                                                       uint32_t* __restrict__ inst_ids) {
     await_previous_kernel();
@@ -706,7 +704,7 @@ __global__ void __launch_bounds__(kCodedThreads, kCodedBlocks) emit_coded_kernel
     EmitCodedSmem& s_stage = *reinterpret_cast<EmitCodedSmem*>(smem_raw);
     __shared__ unsigned s_total[2][kWarps];   // of two groups in turn, so that one barrier does
     __shared__ BlockHistogram s_digits;
-    const unsigned n_visible = n_visible_dev ? (unsigned)*n_visible_dev : (unsigned)n_visible_arg, n_groups = (n_visible + kGroup - 1u) / kGroup;   // < 2^30
+    const unsigned n_visible = (unsigned)*n_visible_dev, n_groups = (n_visible + kGroup - 1u) / kGroup;   // < 2^30
     if (blockIdx.x >= n_groups) return;
     clear_histogram(s_digits);
     __syncthreads();
@@ -787,13 +785,13 @@ constexpr unsigned kFewInstances = 64;
 template <bool CELLS>
 __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint32_t* __restrict__ sorted_ids,
                                                                       const uint2* __restrict__ bounds,
-                                                                      const uint4* __restrict__ foot, int64_t n_visible_arg, const unsigned long long* __restrict__ n_visible_dev,
+                                                                      const uint4* __restrict__ foot, const unsigned long long* __restrict__ n_visible_dev,
                                                                       const unsigned* __restrict__ block_base, int gw,
                                                                       uint32_t* __restrict__ inst_keys,
                                                                       uint32_t* __restrict__ inst_ids) {
     await_previous_kernel();
     __shared__ unsigned s_total[kInstThreads / 32];
-    const int64_t n_visible = n_visible_dev ? (int64_t)*n_visible_dev : n_visible_arg;
+    const int64_t n_visible = (int64_t)*n_visible_dev;
     if ((int64_t)blockIdx.x * kInstThreads >= n_visible) return;
     const int64_t s = (int64_t)blockIdx.x * kInstThreads + threadIdx.x;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -856,11 +854,10 @@ __global__ void __launch_bounds__(kInstThreads) emit_instances_kernel(const uint
 // 4 / 12 / 21 / 36 us, 3 / 8 / 16 / 32, 8 / 8 / 16 / 24.
 constexpr unsigned kRangeKeysFew = 16, kRangeKeysMany = 64, kRangeMany = 1 << 23;
 __host__ __device__ constexpr unsigned range_keys(int64_t n_instances) { return n_instances < kRangeMany ? kRangeKeysFew : kRangeKeysMany; }
-__global__ void __launch_bounds__(256) tile_ranges_kernel(const uint32_t* __restrict__ keys, int64_t n_instances_arg,
-                                                          const unsigned long long* __restrict__ n_instances_dev,
+__global__ void __launch_bounds__(256) tile_ranges_kernel(const uint32_t* __restrict__ keys, const unsigned long long* __restrict__ n_instances_dev,
                                                           uint2* __restrict__ ranges) {
     await_previous_kernel();
-    const unsigned n = n_instances_dev ? (unsigned)*n_instances_dev : (unsigned)n_instances_arg;   // < 2^30
+    const unsigned n = (unsigned)*n_instances_dev;   // < 2^30
     const unsigned per = range_keys(n), n_steps = (n + per * 32u - 1u) / (per * 32u), lane = lane_id();   // of a warp
     // the grid fits the chip: sized for the bound on the instance count it was three quarters empty blocks
     for (unsigned step = blockIdx.x * 8u + (threadIdx.x >> 5); step < n_steps; step += gridDim.x * 8u) {
@@ -4709,21 +4706,13 @@ InstanceBlob carve_instance_blob(void* p, int64_t n_instances, bool deferred, in
 }
 
 // The state handed back to the caller only stores blob bases and counts; which ping-pong buffer holds
-// a sorted result follows from the number of radix passes, which follows from the counts.
-int tile_result_buffer(int64_t n_instances, int n_tiles) {
-    const int end_bit = bit_length((uint32_t)(n_tiles - 1));
-    return n_instances > 1 ? (sort_pass_count(end_bit) & 1) : 0;
-}
+// a sorted result follows from the number of radix passes, which follows from the bits of the keys.
+int tile_buffer_of(int n_tiles) { return sort_pass_count(bit_length((uint32_t)(n_tiles - 1))) & 1; }
+int depth_buffer_of(const inpc_raster_state* st) { return sort_pass_count(st->depth_key_bits) & 1; }
+// Instance capacity the blobs of `st` were carved for.
+int64_t instance_capacity(const inpc_raster_state* st) { return (st->deferred_counts & 1) ? 4 * st->n_points : st->n_instances; }
 
 // One event per host thread and device: an event belongs to the device that was current when it was made.
-// Instance capacity the blobs of `st` were carved for, and which ping-pong buffer holds the tile-sorted lists.
-int64_t instance_capacity(const inpc_raster_state* st) { return (st->deferred_counts & 1) ? 4 * st->n_points : st->n_instances; }
-int tile_buffer_of(const inpc_raster_state* st, int n_tiles) {
-    if (st->deferred_counts & 1) return sort_pass_count(bit_length((uint32_t)(n_tiles - 1))) & 1;
-    return tile_result_buffer(st->n_instances, n_tiles);
-}
-int depth_buffer_of(const inpc_raster_state* st) { return sort_pass_count(st->depth_key_bits) & 1; }
-
 cudaEvent_t counters_event() {
     static thread_local cudaEvent_t events[kMaxDevices] = {nullptr};
     int dev = 0;
@@ -4868,8 +4857,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                                     sort_zero_bytes(n_instances, likely_instances(n_instances, deferred), tile_bits));
     };
     int rc, in_alt = 0;
-    const unsigned long long* n_visible_dev = deferred ? pb.counters : nullptr;
-    const unsigned long long* n_instances_dev = deferred ? pb.counters + 1 : nullptr;
+    // read from here by everything behind the sorts, also where the host knows the counts: zero if a sort has failed
+    unsigned long long* n_visible_dev = n > 0 ? pb.counters : nullptr;
+    unsigned long long* n_instances_dev = n > 0 ? pb.counters + 1 : nullptr;
     if (n > 0) {
         unsigned long long* host = nullptr;
         cudaEvent_t ready = nullptr;
@@ -4946,7 +4936,7 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
             // the count of touched tiles follows from the codes, or rides in the top key bits where the depth offsets leave them free
             auto* count = carried ? instance_count_kernel<COUNTS_IN_CODES> : !counts_in_keys ? instance_count_kernel<COUNTS_GATHERED>
                           : MODE == INPC_MODE_BILINEAR ? instance_count_kernel<COUNTS_IN_KEYS> : instance_count_kernel<COUNTS_IN_GAUSS_KEYS>;
-            launch_chained(count, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state, deferred ? pb.counters + 1 : nullptr, codes.escape);
+            launch_chained(count, count_blocks, kInstThreads / 4, 0, stream, pb.keys[in_alt], sorted_ids, pb.bounds, pb.quad, n_visible_dev, pb.inst_block_sums, (unsigned)ibk, pb.state, n_instances_dev, codes.escape);
             INPC_LAUNCH_CHECK("instance_count_kernel");
             if (counted) {
                 const KeyHistogram digits = key_histogram(ib.sort_ws, n_instances, likely_instances(n_instances, deferred), tile_bits);
@@ -4956,26 +4946,25 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
                     rc = opt_in_dynamic_smem(emit_coded_kernel, sizeof(EmitCodedSmem), attr_set);
                     if (rc != INPC_OK) return rc;
                     const int64_t need = ceil_div<int64_t>(n_visible, kCodedThreads * kCodedPoints), cap = (int64_t)sm_count() * kCodedBlocks;
-                    launch_chained(emit_coded_kernel, (unsigned)(need < cap ? need : cap), kCodedThreads, sizeof(EmitCodedSmem), stream, sorted_ids, pb.keys[in_alt], codes, n_visible, n_visible_dev,
+                    launch_chained(emit_coded_kernel, (unsigned)(need < cap ? need : cap), kCodedThreads, sizeof(EmitCodedSmem), stream, sorted_ids, pb.keys[in_alt], codes, n_visible_dev,
                         pb.inst_block_sums, rp.gw, digits, n_emitted, ib.keys[0], ib.ids[0]);
                 } else {
                     const int64_t cap = (int64_t)sm_count() * 2;   // two blocks of 1024 threads fill a multiprocessor
-                    launch_chained(emit_quads_kernel, (unsigned)(ibk < cap ? ibk : cap), kInstThreads, 0, stream, sorted_ids, pb.quad, n_visible, n_visible_dev, pb.inst_block_sums,
+                    launch_chained(emit_quads_kernel, (unsigned)(ibk < cap ? ibk : cap), kInstThreads, 0, stream, sorted_ids, pb.quad, n_visible_dev, pb.inst_block_sums,
                         rp.gw, digits, n_emitted, ib.keys[0], ib.ids[0]);
                 }
             } else {
-                launch_chained(warp_blend ? emit_instances_kernel<true> : emit_instances_kernel<false>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.foot, n_visible,
+                launch_chained(warp_blend ? emit_instances_kernel<true> : emit_instances_kernel<false>, (unsigned)ibk, kInstThreads, 0, stream, sorted_ids, pb.bounds, pb.foot,
                     n_visible_dev, pb.inst_block_sums, rp.gw, ib.keys[0], ib.ids[0]);
             }
             INPC_LAUNCH_CHECK(carried ? "emit_coded_kernel" : counted ? "emit_quads_kernel" : "emit_instances_kernel");
         }
         StageScope scope(STAGE_SORT_TILE, stream);
         int t_alt = 0;
-        rc = deferred ? sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream, counted)
-                      : sort_pairs(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), tile_bits, ib.sort_ws, true, status, &t_alt, stream, false, counted);
+        rc = sort_pairs_device_count(ib.keys[0], ib.keys[1], ib.ids[0], ib.ids[1], n_instances, likely_instances(n_instances, deferred), n_instances_dev, tile_bits, ib.sort_ws, true, status, &t_alt, stream, counted);
         if (rc != INPC_OK) return rc;
         const int64_t range_blocks = ceil_div<int64_t>(n_instances, 256 * (int64_t)kRangeKeysFew), range_cap = (int64_t)sm_count() * 8;
-        launch_chained(tile_ranges_kernel, (unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream, ib.keys[t_alt], n_instances, n_instances_dev, ib.ranges);
+        launch_chained(tile_ranges_kernel, (unsigned)(range_blocks < range_cap ? range_blocks : range_cap), 256, 0, stream, ib.keys[t_alt], n_instances_dev, ib.ranges);
         INPC_LAUNCH_CHECK("tile_ranges_kernel");
     }
     if (warp_blend) {
@@ -5279,7 +5268,7 @@ int launch_blend_forward(int mode, const RasterParams& rp, const PointBlob& pb, 
                          float* image, float* depth, float* alpha, float* blending_weights, float threshold,
                          cudaStream_t stream) {
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
-    const int t_alt = tile_buffer_of(st, n_tiles);
+    const int t_alt = tile_buffer_of(n_tiles);
     const uint32_t* ids = ib.ids[t_alt];
     StageScope scope(STAGE_BLEND_FWD, stream);
     if (mode == INPC_MODE_BILINEAR) {
@@ -5390,7 +5379,7 @@ int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* p
                                                      KIND == BLEND_INFER, &pb, &ib, stream, KIND == BLEND_INFER ? "inpc_render_rows" : "inpc_rasterize_rows_forward",
                                                      rows_to_clear(rp, channels, image, depth, alpha, blending_weights, n), channels / 4);
     if (rc != INPC_OK) return rc;
-    const int t_alt = tile_buffer_of(state, rp.gw * rp.gh);
+    const int t_alt = tile_buffer_of(rp.gw * rp.gh);
     {
         StageScope scope(STAGE_BLEND_FWD, stream);
         rc = dispatch_rows(channels, [&](auto c4) {
@@ -5453,7 +5442,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode, state->tile_size);
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false);
-    const uint32_t* ids = ib.ids[tile_buffer_of(state, n_tiles)];
+    const uint32_t* ids = ib.ids[tile_buffer_of(n_tiles)];
     float4* gfv = reinterpret_cast<float4*>(grad_features_view);
     const int W = rp.v.width, H = rp.v.height;
     // the caller's scratch holds 33 floats per point: four 32-byte slot records and one mask word for the warp blend
@@ -5478,12 +5467,12 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     {
         StageScope scope(STAGE_BLEND_BWD, stream);
         if (state->mode == INPC_MODE_BILINEAR) {
-            rc = rp.tile == 8 ? launch_bilinear_warp_backward(rp, pb, ib, tile_buffer_of(state, n_tiles), grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, stream)
+            rc = rp.tile == 8 ? launch_bilinear_warp_backward(rp, pb, ib, tile_buffer_of(n_tiles), grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, stream)
                               : launch_bilinear_backward<16>(rp, pb, ib, ids, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
             if (rc != INPC_OK) return rc;
         } else {
             if (rp.tile == 8) {
-                rc = launch_gaussian_warp_backward(rp, pb, ib, tile_buffer_of(state, n_tiles), grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
+                rc = launch_gaussian_warp_backward(rp, pb, ib, tile_buffer_of(n_tiles), grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
                 if (rc != INPC_OK) return rc;
             } else {
                 launch_chained(blend_gaussian_backward_kernel<16>, (unsigned)ib.max_segments, 256, 0, stream, ib.segs, ib.n_segments, ids, pb.rec, pb.conic, ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, W, H, rp.gw);
@@ -5663,7 +5652,7 @@ extern "C" int inpc_rasterize_rows_backward(const inpc_raster_state* state, cons
     const int n_tiles = rp.gw * rp.gh * rp.n_sets;
     const PointBlob pb = carve_point_blob(state->point_blob, n, state->mode, state->tile_size);
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false, channels / 4);
-    const int t_alt = tile_buffer_of(state, n_tiles);
+    const int t_alt = tile_buffer_of(n_tiles);
     ClearList clear;
     clear.add(grad_features, sizeof(float) * (size_t)n * channels);
     clear.add(grad_opacities, sizeof(float) * (size_t)n);
@@ -5693,6 +5682,9 @@ extern "C" int inpc_raster_resolve(inpc_raster_state* state, void* stream_) {
     unsigned long long host[3];
     INPC_CUDA_TRY(cudaMemcpyAsync(host, pb.counters, sizeof(host), cudaMemcpyDeviceToHost, stream));
     INPC_CUDA_TRY(cudaStreamSynchronize(stream));
+    // a call whose sort has failed has counted nothing, and says so here
+    const int rc_prev = check_previous_calls();
+    if (rc_prev != INPC_OK) return rc_prev;
     state->n_visible = (int64_t)host[0];
     state->n_instances = (int64_t)host[1];
     if (state->n_visible == 0) state->depth_key_base = 0u;
@@ -5742,7 +5734,7 @@ extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc
     if (state->n_visible < 0 || state->n_instances < 0) { set_error("inpc_raster_debug_copy: the counts of this state are still on the device; call inpc_raster_resolve first"); return INPC_E_INVALID; }
     const InstanceBlob ib = carve_instance_blob(state->instance_blob, instance_capacity(state), state->deferred_counts & 1, n_tiles, state->tile_size, state->mode, false);
     const int d = depth_buffer_of(state);
-    const int ti = tile_buffer_of(state, n_tiles);
+    const int ti = tile_buffer_of(n_tiles);
     switch (which) {
         case 0: INPC_CUDA_TRY(cudaMemcpyAsync(dst, pb.ids[d], 4 * (size_t)state->n_visible, cudaMemcpyDeviceToDevice, stream)); break;
         case 1:   // not every sort keeps its keys: the depths of the points in their order

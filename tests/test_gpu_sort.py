@@ -124,3 +124,36 @@ def test_lookback_wait_runs_out_and_is_reported():
     # ... and the library works again afterwards
     _check(keys.to(torch.int64) & 0xFFFFFFFF, 16)
     assert L.inpc_call_status(L.inpc_last_call_ticket(), None) == 0
+
+
+# the sorts of the rasterizer: of instances, and of marked depth keys (in two passes and in one)
+@pytest.mark.parametrize("marked, end_bit", [(0, 16), (1, 16), (1, 9)])
+def test_a_sort_that_gives_up_leaves_nothing_to_read(marked, end_bit):
+    """A list that a failed sort has left holes in must not be read: what took its length from the count in device memory
+    finds zero, the passes behind the one that failed among them, which write nothing any more."""
+    from inpc_b200 import _cabi
+    L = _cabi.lib()
+    n, guard = 100_000, 4096
+    g = torch.Generator(device=DEV).manual_seed(end_bit)
+    bufs = [torch.full((n + 2 * guard,), -7, dtype=torch.int32, device=DEV) for _ in range(4)]
+    k, ka, v, va = [b[guard:guard + n] for b in bufs]
+    k.copy_(torch.randint(0, 1 << 31, (n,), generator=g, device=DEV, dtype=torch.int64).to(torch.int32))
+    v.copy_(torch.arange(n, device=DEV, dtype=torch.int32))
+    first = k.clone()
+    ws = torch.empty(int(L.inpc_sort_workspace_bytes(n)), dtype=torch.uint8, device=DEV)
+    count = torch.tensor([-1, n, -1], dtype=torch.int64, device=DEV)
+    ticket = C.c_longlong(0)
+    _cabi.check(L.inpc_debug_counted_sort_lookback_timeout(k.data_ptr(), ka.data_ptr(), v.data_ptr(), va.data_ptr(), n, count[1:].data_ptr(),
+                                                           marked, end_bit, ws.data_ptr(), C.byref(ticket), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert count.tolist() == [-1, 0, -1]
+    assert L.inpc_call_status(ticket.value, None) == -4 and b"predecessor tile" in L.inpc_last_error()
+    for b in bufs:
+        assert bool((b[:guard] == -7).all()) and bool((b[guard + n:] == -7).all())
+    assert torch.equal(k, first)      # of two passes the second found nothing
+    k2, v2 = first.clone(), torch.arange(n, device=DEV, dtype=torch.int32)
+    alt = C.c_int(0)
+    args = (k2.data_ptr(), torch.empty_like(k2).data_ptr(), v2.data_ptr(), torch.empty_like(v2).data_ptr(), n, 16, ws.data_ptr(), C.byref(alt),
+            torch.cuda.current_stream().cuda_stream)
+    assert L.inpc_sort_pairs(*args) == -4 and b"counted_sort" in L.inpc_last_error()      # reported once at the thread's next call
+    _cabi.check(L.inpc_sort_pairs(*args))
