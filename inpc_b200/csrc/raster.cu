@@ -4829,7 +4829,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     const bool deferred = defers_counts(MODE, rp.tile, VARIANT == VAR_ROWS, n, stream);
     int64_t n_visible = 0, n_instances = 0;
     // depth keys are offsets from the near plane's bit pattern, bounded by the far plane's: nothing is measured
-    const float near_depth = rp.v.near_plane > 0.0f ? rp.v.near_plane : 0.0f, far_depth = rp.v.far_plane > near_depth ? rp.v.far_plane : near_depth;
+    const float near_depth = rp.v.near_plane > 0.0f ? rp.v.near_plane : 0.0f;
+    const float far_depth = rp.v.far_plane != rp.v.far_plane ? INFINITY   // a far plane that is no number culls nothing
+                                                             : rp.v.far_plane > near_depth ? rp.v.far_plane : near_depth;
     uint32_t key_base, last_key;
     memcpy(&key_base, &near_depth, 4);
     memcpy(&last_key, &far_depth, 4);

@@ -62,6 +62,29 @@ def test_key_ranges_next_to_the_mark_of_a_culled_point(near, far):
     assert _check(view, pos, opac) > n // 2
 
 
+# No depth is behind a far plane that is no number: the keys have to hold all of them, as with a plane at infinity
+@pytest.mark.parametrize("near", [0.01, 0.0])
+def test_a_far_plane_that_is_no_number(near):
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    n = 4000
+    g = torch.Generator().manual_seed(11)
+    pos = torch.rand((n, 3), generator=g) * 2 - 1
+    pos = (torch.tensor([0.0, 0.0, 3.0]) + (pos - torch.tensor([0.0, 0.0, 3.0])) * torch.exp(torch.rand((n, 1), generator=g) * 40)).contiguous().to(DEV)
+    feats, rows = torch.randn((n, 36), generator=g).to(torch.float16).to(DEV), torch.randn((n, 8), generator=g).to(DEV)
+    opac = (torch.rand((n, 1), generator=g) * 0.2).to(DEV)
+    out = []
+    for far in (float("inf"), float("nan")):
+        view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 72, 40, 64.0, 64.0, near_plane=near, far_plane=far).to(DEV)
+        rast = {tile: inpc_b200.INPCRasterizer(tile_size=tile) for tile in (8, 16)}
+        out.append([rast[tile](view, mode, pos, feats, opac) for tile in (8, 16) for mode in (0, 1)] + [rast[tile].forward_rows(view, pos, rows, opac) for tile in (8, 16)])
+    assert float(out[0][0][1].max()) > 0.3
+    for a, b in zip(*out):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+        # sums of atomic additions in any order
+        assert float((a[2] - b[2]).abs().max()) <= 32 * 2.0 ** -24 * float(a[2].max())
+
+
 # Splats that lie exactly between two pixels, also at the edges of tiles (no second tile is touched) and at the border of the image, in front of it and behind it,
 # beside others: their footprints do not follow from the codes that the depth sort carries along.  One tile; a few; so many that the codes do not fit beside
 # 32-bit keys (near plane at zero), where the words are gathered instead, as where keys are sorted in one pass (planes close together); both sizes of the sort's tiles.
