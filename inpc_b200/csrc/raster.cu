@@ -1483,8 +1483,8 @@ constexpr size_t backward_smem_bytes() {
 // item, so a tile with 100x the average load does not set the critical path.  Pass FIRST blends
 // segment 0 of every tile exactly; the pixels that dense clusters hit stop there.  Pass PRODUCT
 // computes, for the later segments, the per-pixel product of (1 - alpha) over the segment, starting
-// from (and filtering by) the state segment 0 left, so the work it repeats is small; pass REST blends the later
-// segments from the transmittance at their start, the product of those in front; a per-tile combine adds the segment colours in order (and leaves the
+// from (and filtering by) the state segment 0 left, so the work it repeats is small, and turns the products into the
+// transmittance at the start of every segment; pass REST blends the later segments from there; a per-tile combine adds the segment colours in order (and leaves the
 // colour prefix for the backward pass, whose items are then independent).
 //
 // An item covers the upper or lower 8x4 half of a tile, one pixel per lane; both halves stream the same
@@ -1658,18 +1658,19 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_count_kernel(const ui
 }
 
 // Everything a warp needs to know about a (tile, segment), in one 32-byte record: the blend kernels read it with
-// two 16-byte loads, one item ahead of the one they work on, instead of chasing tile -> range -> first segment.
+// loads of 16 and 8 bytes, one item ahead of the one they work on, instead of chasing tile -> range -> first segment.
 struct __align__(16) WarpItem {
     uint32_t tile, seg;       // which tile, which of its segments
     uint32_t begin, end;      // instance range of the segment
     uint32_t first, n_seg;    // slot of the tile's segment 0 in the per-segment arrays; segments of the tile
-    uint32_t pad0, pad1;
+    uint32_t finished[2];     // of the tile's first later segment: how many of the later ones pass PRODUCT is through with, per half
 };
 
 __device__ __forceinline__ WarpItem load_item(const WarpItem* p) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p)), b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint2 b = __ldg(reinterpret_cast<const uint2*>(p) + 2);
     WarpItem w;
-    w.tile = a.x; w.seg = a.y; w.begin = a.z; w.end = a.w; w.first = b.x; w.n_seg = b.y; w.pad0 = 0; w.pad1 = 0;
+    w.tile = a.x; w.seg = a.y; w.begin = a.z; w.end = a.w; w.first = b.x; w.n_seg = b.y; w.finished[0] = 0; w.finished[1] = 0;
     return w;
 }
 
@@ -1889,19 +1890,33 @@ struct CandidateStream {
     }
 };
 
-// Transmittance of a lane's pixel at the start of a later segment of its tile half: the state behind segment 0 times the products of the segments between.  Every item forms it for
-// itself; the loads do not wait for one another.  (A kernel of its own between the passes took 4 to 8 us and a launch: 10^6 samples 380 -> 375 us, 2^25 points 2636 -> 2630.)
-__device__ __forceinline__ float segment_start(const float* __restrict__ seg_T, unsigned first, unsigned half, unsigned seg, unsigned lane) {
-    const float* base = seg_T + ((size_t)first * 2u + half) * 32 + lane;   // segment g of this half: base[g * 64]
-    float run = base[0];
-    for (unsigned g0 = 1; g0 < seg; g0 += 8) {
-        float product[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) product[k] = g0 + k < seg ? base[(size_t)(g0 + k) * 64] : 1.0f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) run *= product[k];
+// Pass PRODUCT, a warp that has left an item's products in seg_T (a pixel per lane): where it is the last of the tile half to do so, seg_T of every later segment becomes the transmittance at its
+// start = the state behind segment 0 times the products of the segments between.  `item`: of the list of later segments, where those of a tile lie in a row.
+// A kernel of its own between the passes took 4 to 8 us and a launch.  Where every item formed its start itself, in the later segments and again backward, lists of many segments were read in the
+// square of their number: training step of 2^24 almost opaque splats in one tile (4096 segments) 2690 us, 2550 so (backward 132 -> 35), of 2^26 rows of four channels 10760 -> 9040
+// (511 -> 54); of 2^24 faint ones 5405 -> 5255; 2^23 samples at 1237x822 1268 -> 1272, 10^6 at 801x533 300 both.
+__device__ __forceinline__ void finish_products(const WarpItem* items, unsigned item, unsigned half, unsigned seg, unsigned n_seg, float* seg_T, unsigned first, unsigned lane) {
+    if (n_seg > 2u) {
+        __threadfence();   // every lane's product, before it counts as finished
+        __syncwarp();
+        unsigned before = 0u;
+        if (lane == 0u) before = atomicAdd(const_cast<uint32_t*>(&items[item - (seg - 1u)].finished[half]), 1u);
+        if (__shfl_sync(0xffffffffu, before, 0) != n_seg - 2u) return;
+        __threadfence();
     }
-    return run;
+    float* base = seg_T + ((size_t)first * 2u + half) * 32 + lane;   // segment g of this half: base[g * 64]
+    constexpr int kAtOnce = 16;   // loads that do not wait for one another
+    float run = base[0];
+    for (unsigned g0 = 1; g0 < n_seg; g0 += kAtOnce) {
+        float product[kAtOnce];
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) product[k] = g0 + k + 1u < n_seg ? __ldcg(base + (size_t)(g0 + k) * 64) : 1.0f;   // (of other warps: not through L1)
+#pragma unroll
+        for (int k = 0; k < kAtOnce; ++k) {
+            if (g0 + k < n_seg) base[(size_t)(g0 + k) * 64] = run;
+            run *= product[k];
+        }
+    }
 }
 
 // Shared memory of one warp of the forward passes.
@@ -1986,7 +2001,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
             done = done || T0 < kTransmittanceEps;
             log_stop = done ? 0.0 : log2((double)T0 / (double)kTransmittanceEps) + (double)stop_margin(rg.y - rg.x);
         } else if (PASS == PASS_REST) {
-            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
+            Tr = seg_T[sidx * 32 + lane];
             done = done || Tr < kTransmittanceEps;
         }
         unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
@@ -2164,6 +2179,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
 
         if (PASS == PASS_PRODUCT) {
             seg_T[sidx * 32 + lane] = (float)exp2(-log_sum);   // this segment's product
+            finish_products(items, item >> 1, (unsigned)half, seg, n_seg, seg_T, first, lane);
             continue;
         }
         const int64_t n_px = (int64_t)width * height;
@@ -2370,7 +2386,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, pair_forward_blocks(C4))
         for (int c = 0; c < C4; ++c) C[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         bool done = !inside;
         if (PASS == PASS_REST) {
-            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
+            Tr = seg_T[sidx * 32 + lane];
             done = done || Tr < kTransmittanceEps;
         }
         unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
@@ -2770,7 +2786,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
             C_final = n_seg > 1u ? seg_C[sidx * 32 + lane]
                                  : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, seg, lane);
+            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -2986,7 +3002,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kPairBackwardBlocks) ble
             C_final = it.n_seg > 1u ? seg_C[sidx * 32 + lane]
                                     : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (it.seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, it.seg, lane);
+            if (it.seg > 0u) Tr = seg_T[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         sm.pixel_grad[lane] = g;
@@ -3080,7 +3096,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, rows_backward_blocks(C4)
                 G_final += v.x * g[c].x + v.y * g[c].y + v.z * g[c].z + v.w * g[c].w;
             }
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, seg, lane);
+            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through
@@ -3978,7 +3994,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
             done = done || T0 < kTransmittanceEps;
             if (!done) stop = kTransmittanceEps / T0 * (1.0f - stop_margin(rg.y - rg.x));
         } else if (PASS == PASS_REST) {
-            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
+            Tr = seg_T[sidx * 32 + lane];
             done = done || Tr < kTransmittanceEps;
         }
         unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
@@ -4087,6 +4103,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
 
         if (PASS == PASS_PRODUCT) {
             seg_T[sidx * 32 + lane] = Tr;   // this segment's product
+            finish_products(items, item >> 1, (unsigned)half, seg, n_seg, seg_T, first, lane);
             continue;
         }
         const int64_t n_px = (int64_t)width * height;
@@ -4251,7 +4268,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussPairBlocks) blend_
         float4 C = make_float4(0.f, 0.f, 0.f, 0.f);
         bool done = !inside;
         if (PASS == PASS_REST) {
-            Tr = segment_start(seg_T, first, (unsigned)half, seg, lane);
+            Tr = seg_T[sidx * 32 + lane];
             done = done || Tr < kTransmittanceEps;
         }
         unsigned done_w = __ballot_sync(kFull, done);   // bit l = pixel of lane l has stopped (warp-uniform)
@@ -4380,7 +4397,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussBackwardBlocks) bl
             Cfin = n_seg > 1u ? seg_C[sidx * 32 + lane]
                               : make_float4(__ldg(image + pi), __ldg(image + n_px + pi), __ldg(image + 2 * n_px + pi), __ldg(image + 3 * n_px + pi));
             K = __ldg(grad_alpha + pi) * (1.0f - __ldg(alpha_image + pi));
-            if (seg > 0u) Tr = segment_start(seg_T, it.first, (unsigned)half, seg, lane);
+            if (seg > 0u) Tr = seg_T[sidx * 32 + lane];
             done = Tr < kTransmittanceEps;
         }
         __syncwarp();   // the previous item's readers of pixel_grad are through

@@ -96,6 +96,57 @@ def test_lists_of_one_footprint(n, opaque, site):
         assert (off <= gf_bound + 1e-30).all(), (rows, (off / (gf_bound + 1e-30)).max())
 
 
+# Lists of many segments (of 256 instances each, so few are there): the transmittances at their starts are formed 16 at a time, by whichever segment is through last
+@pytest.mark.parametrize("segments", [2, 3, 4, 16, 17, 18, 19, 33, 50])
+@pytest.mark.parametrize("opaque", [False, True])
+def test_lists_of_many_segments(segments, opaque):
+    import inpc_b200
+    from inpc_b200 import rasterization as R
+    from inpc_b200.views import look_at_view
+    n = 256 * segments - 100
+    g = torch.Generator().manual_seed(segments * 2 + opaque)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), SIDE, SIDE, float(SIDE), float(SIDE)).to(DEV)
+    depth = 2.0 + torch.arange(n, dtype=torch.float32) / 1024
+    px, py = 9.0 + torch.rand(n, generator=g) * 6, 9.0 + torch.rand(n, generator=g) * 6   # inside the second tile in both directions
+    pos = torch.stack([(px - SIDE / 2) / SIDE * depth, -(py - SIDE / 2) / SIDE * depth, 3.0 - depth], dim=1).contiguous().to(DEV)
+    opacity = torch.rand((n, 1), generator=g) * (4.0 / n)          # in a pixel about a tenth of them: most of what is behind is seen
+    if opaque:
+        opacity[torch.arange(n) % 256 == 255] = 0.3                # a pixel stops in the middle of the list, at another place for each
+    gi, ga = torch.randn((4, SIDE, SIDE), generator=g), torch.randn((1, SIDE, SIDE), generator=g)
+    rast, settings = inpc_b200.INPCRasterizer(tile_size=8), R.INPCRasterizer.extract_settings(view, 0)
+    sh = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16).to(DEV)
+    _, _, _, state, blobs, _ = R.forward_with_state(pos, sh, opacity.to(DEV), settings, 8)
+    dbg = R.debug_arrays(state, settings, blobs.point, blobs.instance)
+    x, y = dbg["screen"].double().cpu().numpy().T
+    assert int(state.n_visible) == n == int(state.n_instances)
+    for rows in (0, 4, 16):
+        features = torch.randn((n, rows), generator=g).to(DEV) if rows else sh
+        f, o = features.requires_grad_(True), opacity.to(DEV).requires_grad_(True)
+        image, alpha, _ = rast.forward_rows(view, pos, f, o) if rows else rast(view, 0, pos, f, o)
+        gi_c = gi if rows != 16 else gi.repeat(4, 1, 1)
+        torch.autograd.backward([image, alpha], [gi_c.to(DEV), ga.to(DEV)])
+        seen = (f.detach() if rows else dbg["feat_view"]).double().cpu().numpy()
+        go, gf, go_bound, gf_bound = _exact(x, y, opacity.double().numpy()[:, 0], seen, gi_c.double().numpy(), ga.double().numpy())
+        off = np.abs(o.grad.double().cpu().numpy()[:, 0] - go)
+        assert (off <= go_bound).all(), (rows, (off / go_bound).max())
+        if rows:
+            off = np.abs(f.grad.double().cpu().numpy() - gf)
+            assert (off <= gf_bound + 1e-30).all(), (rows, (off / (gf_bound + 1e-30)).max())
+    # gaussian splats, and inference of both: nothing depends on the tile size but the order of the sums
+    feats, opac = sh.detach(), opacity.to(DEV)
+    for mode in (0, 1):
+        out = []
+        for tile in (8, 16):
+            f, o = feats.clone().requires_grad_(True), opac.clone().requires_grad_(True)
+            r = inpc_b200.INPCRasterizer(tile_size=tile)
+            image, alpha, weights = r(view, mode, pos, f, o)
+            torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
+            out.append((image.detach(), alpha.detach(), weights, o.grad, f.grad.float(), *r.render_preextracted(view, mode, pos, feats, opac)))
+        for a, b in zip(*out):
+            # products of up to n factors in another grouping, twice (their terms' transmittance and the stop)
+            assert float((a - b).norm()) <= max(1e-4, 2 * n * U) * float(b.norm())
+
+
 # Two warps per list (images of up to 2^15 tiles) against one: the same points in the upper left corner of an image that has more tiles.  Lists of every length beside a batch of 32, of
 # faint splats, of which nothing stops, and of opaque ones, where the pixels stop in the middle of a batch, at its end, and one after the other
 @pytest.mark.parametrize("opacity", [0.004, 0.3, 0.97, None])
