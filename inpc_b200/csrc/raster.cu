@@ -1515,6 +1515,28 @@ constexpr int kManyTiles = 1 << 15;   // from here on the first segments alone k
 struct SegmentLengths {
     unsigned first, later;   // instances in a tile's first segment, and in every later one
 };
+// Whether the training passes that have such a form (first and later segments, and backward of four channels) take an item by two warps, see blend_bilinear_pair_forward_kernel.  It makes the
+// longest lists faster, by a third, and leaves room for half to two thirds as many items: a gain where the passes are as long as their longest items, nothing where all lists are long, a loss where
+// all are short.  How the points are spread over the tiles is not known here, how many there are for each is.  Whole step, one warp / two, with samples of an octree (part of the image, lists of any
+// length) and points spread evenly over the image:
+//   points per tile            16          32          64         128         256         512
+//   560x420    octree      140 / 133   168 / 158   196 / 185   246 / 239   312 / 306   455 / 434
+//              even        112 / 119   126 / 132   148 / 155   206 / 210   306 / 318   485 / 503
+//   1237x822   octree      188 / 184   248 / 248   332 / 333   505 / 502   796 / 770  1280 / 1244
+//              even        181 / 214   230 / 265   324 / 358   521 / 550   933 / 943  1868 / 1862
+//   1920x1080  octree      249 / 254   342 / 351   524 / 532   837 / 828  1389 / 1369 2380 / 2346
+//              even        282 / 342   355 / 416   550 / 612   960 / 991  2122 / 2106 4100 / 4076
+//   3840x2160  octree      602 / 634  1016 / 1022 1777 / 1758 3132 / 3098 5332 / 5290
+//              even        844 / 1080 1203 / 1412 2192 / 2248 4704 / 4391 9896 / 9782
+//              a corner    614 / 732   854 / 992  1290 / 1442 2236 / 2341 4074 / 4086
+// so two warps up to kFewTiles tiles, where the items are few, and with 128 points per tile up to kManyTiles.  Rows, whose longer lists weigh more, forward only: 16 channels at 1920x1080, 16 / 64 points
+// per tile, even 500 / 534 and 906 / 912, octree 328 / 327 and 676 / 672.  Gaussian splats, forward only: at 1237x822 octree 224 / 209 and 506 / 493 with 8 / 64 per tile, even 196 / 218 and 442 / 433;
+// 1920x1080 octree 267 / 257 and 848 / 811, even 315 / 363 and 930 / 900; 3840x2160, 16 / 32, octree 932 / 908 and 1585 / 1491, even 1109 / 1286 and 1693 / 1735.
+constexpr int kFewTiles = 1 << 12, kFewTilesGaussian = 1 << 14;
+bool by_two_warps(int mode, bool rows, int64_t tiles, int64_t n_points) {
+    if (mode == INPC_MODE_GAUSSIAN) return tiles <= kFewTilesGaussian || n_points >= 64 * tiles;
+    return tiles <= kFewTiles || (tiles <= kManyTiles && n_points >= (rows ? 32 : 128) * tiles);
+}
 // The largest lengths, and how many later segments are aimed at.  A batch of gaussian splats takes a training pass two to three
 // times as long (more fragments, their sums), so its long items weigh more than the states of more segments; inference has little of
 // that work.  Blend passes of a training step at 1237x822, forward and backward, first + later segment 1024 + 4096 / 512 + 2048 /
@@ -2227,7 +2249,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
 // Batch b lies in stage b % 3 of the ring (b is walked, b + 1 made ready, b + 2 under way); its words, and whether there is such a batch, in place b % 2, where the state of the pixels before
 // it lies too.  Both warps leave the loop at the same barrier: what they decide by is written before it and not again before the next but one.
 // Step of 2^23 samples at 1237x822, first / later segments 96 / 112 -> 84 / 106 us, 16 channels 156 / 231 -> 156 / 189, 10^6 samples 24 / 34 -> 21 / 34.  Half as many items are under way, so
-// where there are many short ones (more than kManyTiles tiles) or the passes wait for memory (inference) one warp per item is the faster form: 2^24 points crowding a corner of
+// where there are many short ones (see by_two_warps) or the passes wait for memory (inference) one warp per item is the faster form: 2^24 points crowding a corner of
 // 3840x2160, first segments 255 against 290 us, 2^25 points of a cloud 347 + 109 against 367 + 118.  Four blocks per multiprocessor of 64 registers (of wide rows three): with three
 // 333 us in place of 290, with five (48 registers) 333; four stages the same.
 constexpr int kPairs = kWarpBlendWarps / 2;
@@ -2860,7 +2882,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kBackwardBlocks) blend_b
 
 // The same by two warps per item (see blend_bilinear_pair_forward_kernel): one makes the fragments of a batch ready and, a batch later, adds up what the walk has left per instance,
 // the other walks.  Slots and words of batch b lie in place b % 2: those of b - 1 are added up before those of b + 1 take their place.  2^23 samples at 1237x822 232 -> 207 us, 10^6 at
-// 801x533 46 -> 42.  Above kManyTiles tiles one warp per item is the faster form (2^24 points crowding a corner of 3840x2160 382 against 456 us), and for feature rows and Gaussian
+// 801x533 46 -> 42.  Where lists are short one warp per item is the faster form (see by_two_warps; 2^24 points crowding a corner of 3840x2160 382 against 456 us), and for feature rows and Gaussian
 // splats at any number (2^23 samples of 16 channels 328 against 393, 2^22 splats 251 against 274, 288 with the sums where the ellipses are found), since their rings and sums
 // leave room for too few items.  Three blocks per multiprocessor of 80 registers; four of 64 224 us.
 struct __align__(16) PairBackwardSmem {
@@ -3932,31 +3954,35 @@ __device__ __forceinline__ unsigned ellipse_pixels(const float4& a, const float4
     return m;
 }
 
-// One warp per item: the products, and all passes of inference, which have less to do per fragment (2^22 splats: products 184 us, 199 with two warps; 2 * 10^6 splats of a frame, first
-// segments 151 and 194).
-template <bool BLEND>
+// One warp per item: training passes over short lists (see by_two_warps), the products, and all passes of inference, which have less to do per fragment (2^22 splats: products 184 us, 199 with two
+// warps; 2 * 10^6 splats of a frame, first segments 151 and 194).
+template <bool BLEND, bool WEIGHTS>
 struct __align__(16) GaussForwardSmem {
     float4 ring_a[2][32], ring_c[2][32];              // records and conics of the batches in flight
     float4 ring_f[BLEND ? 2 : 1][BLEND ? 32 : 1];     // ... and features
+    float out[WEIGHTS ? 32 : 1][33];                  // [staged instance][pixel]: what the fragment adds to the blending weight
     uint32_t ring_id[2][32];
     uint32_t queue[kQueueCap];
 };
-template <int PASS>
-constexpr size_t gauss_forward_smem_bytes() { return 2 * 256 * sizeof(unsigned) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT>); }
+template <int PASS, int KIND>
+constexpr size_t gauss_forward_smem_bytes() {
+    return 2 * 256 * sizeof(unsigned) + kWarpBlendWarps * sizeof(GaussForwardSmem<PASS != PASS_PRODUCT, PASS != PASS_PRODUCT && KIND == BLEND_TRAIN>);
+}
 
 template <int PASS, int KIND>
 __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) blend_gaussian_warp_forward_kernel(
     const WarpItem* __restrict__ items, const uint32_t* __restrict__ counts, unsigned* __restrict__ ticket, unsigned n_visits, const uint32_t* __restrict__ inst_keys,
     const uint32_t* __restrict__ inst_ids, const PointRec* __restrict__ rec, const float4* __restrict__ conic, float* __restrict__ seg_T,
     float4* __restrict__ seg_C, float* __restrict__ seg_Z, float* __restrict__ seg_E, float* __restrict__ image, float* __restrict__ depth_image,
-    float* __restrict__ alpha_image, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
+    float* __restrict__ alpha_image, float* __restrict__ blending_weights, uint32_t* kept0, uint32_t* kept1, uint32_t* __restrict__ n_kept,
     int width, int height, int gw, float threshold, float reach) {
     await_previous_kernel();
     constexpr unsigned kFull = 0xffffffffu;
     constexpr unsigned kNoInstance = 0xffffffffu;
     constexpr bool kBlend = PASS != PASS_PRODUCT;
-    static_assert(!kBlend || KIND == BLEND_INFER, "training blends by two warps");
-    using Smem = GaussForwardSmem<kBlend>;
+    constexpr bool kWeights = kBlend && KIND == BLEND_TRAIN;
+    constexpr bool kDepth = kBlend && KIND == BLEND_INFER;
+    using Smem = GaussForwardSmem<kBlend, kWeights>;
     extern __shared__ __align__(16) unsigned char blend_smem[];
     unsigned* s_reach = reinterpret_cast<unsigned*>(blend_smem);     // [half][key code] -> pixels of the half reached
     Smem& sm = reinterpret_cast<Smem*>(blend_smem + 2 * 256 * sizeof(unsigned))[threadIdx.x >> 5];
@@ -4051,7 +4077,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                 unsigned pixels = 0u;
                 if (staged) pixels = ellipse_pixels(sm.ring_a[stage][lane], sm.ring_c[stage][lane], reach, px0, py0) & ~done_w;
                 fill();   // (its __syncwarp also shows every lane the records the others have copied)
-                if (PASS == PASS_PRODUCT) {
+                if (PASS == PASS_PRODUCT || kWeights) {
                     // the list of this item: see the bilinear kernel
                     const unsigned b = __ballot_sync(kFull, pixels != 0u);
                     if (pixels) kept[rg.x + n_out + __popc(b & lt_mask)] = id_cur;
@@ -4059,6 +4085,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                 }
                 // ---- every lane runs down the instances of its own pixel, front to back
                 unsigned todo = warp_transpose_bits(pixels, lane);
+                unsigned taken = 0u;   // instances whose blending weight this pixel adds to
                 while (todo) {
                     // a few at a time: their exponentials do not wait for one another (products, three for two: 188 -> 183 us; the other passes the same or slower)
                     constexpr int kPair = PASS == PASS_PRODUCT ? 3 : 2;
@@ -4082,9 +4109,13 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                         if (!ok[u] || done) continue;
                         if (kBlend) {
                             const float bw = Tr * al[u];
+                            if (kWeights && bw > 0.0f) {
+                                sm.out[j[u]][lane] = G[u] * bw;
+                                taken |= 1u << j[u];
+                            }
                             const float4 f = sm.ring_f[stage][j[u]];
                             C.x += bw * f.x; C.y += bw * f.y; C.z += bw * f.z; C.w += bw * f.w;
-                            Z += bw * sm.ring_a[stage][j[u]].w;
+                            if (kDepth) Z += bw * sm.ring_a[stage][j[u]].w;
                         }
                         Tr *= 1.0f - al[u];
                         if (Tr < stop) done = true;
@@ -4092,6 +4123,15 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                     if (done) todo = 0u;
                 }
                 __syncwarp();
+                if (kWeights) {
+                    unsigned from = warp_transpose_bits(taken, lane);
+                    float sum = 0.0f;
+                    while (from) {
+                        sum += sm.out[lane][__ffs(from) - 1];
+                        from &= from - 1u;
+                    }
+                    if (sum > 0.0f) atomicAdd(blending_weights + id_cur, sum);
+                }
                 done_w = __ballot_sync(kFull, done);
                 __syncwarp();
                 if (done_w == kFull) break;   // every pixel has stopped: the rest of the list has no effect
@@ -4099,7 +4139,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
             async_copy_wait<0>();   // whatever is still travelling lands before the next item reuses the ring
             __syncwarp();
         }
-        if (PASS == PASS_PRODUCT && lane == 0) n_kept[sidx] = n_out;
+        if ((PASS == PASS_PRODUCT || kWeights) && lane == 0) n_kept[sidx] = n_out;
 
         if (PASS == PASS_PRODUCT) {
             seg_T[sidx * 32 + lane] = Tr;   // this segment's product
@@ -4115,7 +4155,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
                 image[2 * n_px + pi] = C.z;
                 image[3 * n_px + pi] = C.w;
                 const float A = 1.0f - Tr;
-                depth_image[pi] = A > 0.0f ? Z / A : 0.0f;
+                if (kDepth) depth_image[pi] = A > 0.0f ? Z / A : 0.0f;
                 alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : A;
             }
         } else {
@@ -4123,8 +4163,12 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
             const size_t si = sidx * 32 + lane;
             seg_C[si] = C;
             if (PASS == PASS_FIRST) seg_T[si] = Tr;   // the exact state behind segment 0
-            seg_Z[si] = Z;
-            seg_E[si] = Tr;
+            if (kDepth) {
+                seg_Z[si] = Z;
+                seg_E[si] = Tr;
+            } else if (seg + 1u == n_seg && inside) {
+                alpha_image[pi] = Tr < kTransmittanceEps ? 1.0f : 1.0f - Tr;
+            }
         }
     }
 }
@@ -5112,7 +5156,7 @@ int launch_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned*
 
 // C4, `rows`: feature rows of 4 C4 channels (ROWS), or one group of four channels in the records.
 template <int KIND, int C4 = 1, bool ROWS = false>
-int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float4* rows, float* image,
+int launch_bilinear_warp_forward(const RasterParams& rp, int64_t n_points, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float4* rows, float* image,
                                  float* depth, float* alpha, float* blending_weights, cudaStream_t stream) {
     const unsigned grid = small_grid();
     const int W = rp.v.width, H = rp.v.height;
@@ -5124,7 +5168,7 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{keys, ids, pb.rec, rows, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             kept0, kept1, ib.n_kept, W, H, rp.gw, rp.gh};
-    const bool pairs = rp.gw * rp.gh <= kManyTiles;   // see blend_bilinear_pair_forward_kernel
+    const bool pairs = by_two_warps(INPC_MODE_BILINEAR, ROWS, (int64_t)rp.gw * rp.gh, n_points);
     int rc_pass = launch_forward_pass<PASS_FIRST, KIND, C4, ROWS>(ib.items0, ib.n_segments, ib.n_segments + 2, a, pairs, stream);
     if (rc_pass != INPC_OK) return rc_pass;
     rc_pass = launch_warp_forward_pass<PASS_PRODUCT, KIND, 1, ROWS>(ib.items1, ib.n_segments, ib.n_segments + 3, a, stream);
@@ -5137,7 +5181,7 @@ int launch_bilinear_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     return INPC_OK;
 }
 
-int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
+int launch_bilinear_warp_backward(const RasterParams& rp, int64_t n_points, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
     auto launch = [&](auto kernel, size_t smem, int most, int (&known)[kMaxDevices]) -> int {
@@ -5150,7 +5194,7 @@ int launch_bilinear_warp_backward(const RasterParams& rp, const PointBlob& pb, c
         return INPC_OK;
     };
     static int known[kMaxDevices] = {0}, known_pairs[kMaxDevices] = {0};
-    const int rc = rp.gw * rp.gh <= kManyTiles ? launch(blend_bilinear_pair_backward_kernel, kPairBackwardSmemBytes, kPairBackwardBlocks, known_pairs)
+    const int rc = by_two_warps(INPC_MODE_BILINEAR, false, (int64_t)rp.gw * rp.gh, n_points) ? launch(blend_bilinear_pair_backward_kernel, kPairBackwardSmemBytes, kPairBackwardBlocks, known_pairs)
                                                : launch(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, kBackwardBlocks, known);
     if (rc != INPC_OK) return rc;
     INPC_LAUNCH_CHECK("blend_bilinear backward");
@@ -5199,12 +5243,12 @@ template <int PASS, int KIND>
 int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic,
                                       const ForwardPassArgs& a, float threshold, float reach, cudaStream_t stream) {
     static int known[kMaxDevices] = {0};
-    constexpr size_t smem = gauss_forward_smem_bytes<PASS>();
+    constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
     BlendGrid grid;
     const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, kGaussForwardBlocks, false, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
-        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha,
+        items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
         a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, threshold, reach);
     INPC_LAUNCH_CHECK("blend_gaussian_warp_forward_kernel");
     return INPC_OK;
@@ -5223,7 +5267,7 @@ int launch_gaussian_pair_forward_pass(const WarpItem* items, const uint32_t* cou
 }
 
 template <int KIND>
-int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image, float* depth,
+int launch_gaussian_warp_forward(const RasterParams& rp, int64_t n_points, const PointBlob& pb, const InstanceBlob& ib, int t_alt, float* image, float* depth,
                                  float* alpha, float* blending_weights, float threshold, cudaStream_t stream) {
     const unsigned grid = small_grid();
     int rc;
@@ -5231,10 +5275,13 @@ int launch_gaussian_warp_forward(const RasterParams& rp, const PointBlob& pb, co
     const unsigned threads = kWarpBlendWarps * 32;
     const ForwardPassArgs a{ib.keys[t_alt], ib.ids[t_alt], pb.rec, nullptr, ib.seg_T, ib.seg_C, ib.seg_Z, ib.seg_E, image, depth, alpha, blending_weights,
                             ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, W, H, rp.gw, rp.gh};
+    const bool pairs = by_two_warps(INPC_MODE_GAUSSIAN, false, (int64_t)rp.gw * rp.gh, n_points);
     auto blend = [&](auto which, const WarpItem* items, int at) -> int {
         constexpr int kPass = decltype(which)::value;
-        if constexpr (KIND == BLEND_TRAIN) return launch_gaussian_pair_forward_pass<kPass>(items, ib.n_segments, ib.n_segments + at, pb.conic, a, rp.reach, stream);
-        else return launch_gaussian_warp_forward_pass<kPass, KIND>(items, ib.n_segments, ib.n_segments + at, pb.conic, a, threshold, rp.reach, stream);
+        if constexpr (KIND == BLEND_TRAIN) {
+            if (pairs) return launch_gaussian_pair_forward_pass<kPass>(items, ib.n_segments, ib.n_segments + at, pb.conic, a, rp.reach, stream);
+        }
+        return launch_gaussian_warp_forward_pass<kPass, KIND>(items, ib.n_segments, ib.n_segments + at, pb.conic, a, threshold, rp.reach, stream);
     };
     rc = blend(std::integral_constant<int, PASS_FIRST>{}, ib.items0, 2);
     if (rc != INPC_OK) return rc;
@@ -5291,10 +5338,10 @@ int launch_blend_forward(int mode, const RasterParams& rp, const PointBlob& pb, 
     const uint32_t* ids = ib.ids[t_alt];
     StageScope scope(STAGE_BLEND_FWD, stream);
     if (mode == INPC_MODE_BILINEAR) {
-        if (rp.tile == 8) return launch_bilinear_warp_forward<KIND>(rp, pb, ib, t_alt, nullptr, image, depth, alpha, blending_weights, stream);
+        if (rp.tile == 8) return launch_bilinear_warp_forward<KIND>(rp, st->n_points, pb, ib, t_alt, nullptr, image, depth, alpha, blending_weights, stream);
         return launch_bilinear_forward<16, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, stream);
     }
-    if (rp.tile == 8) return launch_gaussian_warp_forward<KIND>(rp, pb, ib, t_alt, image, depth, alpha, blending_weights, threshold, stream);
+    if (rp.tile == 8) return launch_gaussian_warp_forward<KIND>(rp, st->n_points, pb, ib, t_alt, image, depth, alpha, blending_weights, threshold, stream);
     return launch_gaussian_forward<16, KIND>(rp, pb, ib, ids, image, depth, alpha, blending_weights, threshold, stream);
 }
 
@@ -5404,7 +5451,7 @@ int rows_forward(int tile_size, const inpc_view* view, int64_t n, const float* p
         rc = dispatch_rows(channels, [&](auto c4) {
             constexpr int kC4 = decltype(c4)::value;
             if (tile_size == 8)
-                return launch_bilinear_warp_forward<KIND, kC4, true>(rp, pb, ib, t_alt, reinterpret_cast<const float4*>(features), image, depth, alpha, blending_weights, stream);
+                return launch_bilinear_warp_forward<KIND, kC4, true>(rp, n, pb, ib, t_alt, reinterpret_cast<const float4*>(features), image, depth, alpha, blending_weights, stream);
             return launch_rows_forward<16, kC4, KIND>(rp, pb, ib, ib.ids[t_alt], features, image, depth, alpha, blending_weights, stream);
         });
     }
@@ -5486,7 +5533,7 @@ extern "C" int inpc_rasterize_backward(const inpc_raster_state* state, const inp
     {
         StageScope scope(STAGE_BLEND_BWD, stream);
         if (state->mode == INPC_MODE_BILINEAR) {
-            rc = rp.tile == 8 ? launch_bilinear_warp_backward(rp, pb, ib, tile_buffer_of(n_tiles), grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, stream)
+            rc = rp.tile == 8 ? launch_bilinear_warp_backward(rp, n, pb, ib, tile_buffer_of(n_tiles), grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, stream)
                               : launch_bilinear_backward<16>(rp, pb, ib, ids, grad_image, grad_alpha, image, alpha, gfv, grad_opacities, stream);
             if (rc != INPC_OK) return rc;
         } else {

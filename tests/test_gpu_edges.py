@@ -54,11 +54,11 @@ def test_halton_samples_over_runs_of_empty_leaves(total, gap, largest):
     np.testing.assert_array_equal(out.cpu().numpy(), O.halton_samples(counts.numpy(), centers.numpy(), levels.numpy(), 2.0))
 
 
-def _one_tile_scene(n, seed):
-    """n faint points in front of a 24x16 image, three quarters of them over one 8x8 tile."""
+def _one_tile_scene(n, seed, width=24, height=16):
+    """n faint points in front of the 24x16 pixels in the upper left corner of an image, three quarters of them over one 8x8 tile."""
     from inpc_b200.views import look_at_view
     g = torch.Generator().manual_seed(seed)
-    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 24, 16, 24.0, 24.0)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, 24.0, 24.0, center_x=12.0, center_y=8.0)
     z = torch.rand(n, generator=g) * 2 - 1
     px = torch.where(torch.rand(n, generator=g) < 0.75, 8 + torch.rand(n, generator=g) * 8, torch.rand(n, generator=g) * 24)
     py = torch.rand(n, generator=g) * 8
@@ -72,14 +72,15 @@ def _one_tile_scene(n, seed):
 # a tile's list is cut into segments of at least 256 instances; their length doubles from 655,360 instances on
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 511, 513, 769, 4097, 655_000, 700_001])
 @pytest.mark.parametrize("rows", [0, 4, 16, 32])
-def test_blend_at_the_edges_of_its_segments(n, rows):
+@pytest.mark.parametrize("width, height", [(24, 16), (1040, 1024)])    # all tiles by two warps per list; more tiles than that, by one
+def test_blend_at_the_edges_of_its_segments(n, rows, width, height):
     import inpc_b200
     from helpers import assert_close, oracle_camera
     if n > 100_000 and rows not in (0, 16):
         pytest.skip("the long lists are walked in one layout of each kind")
-    view, pos, opac = _one_tile_scene(n, n)
+    view, pos, opac = _one_tile_scene(n, n, width, height)
     g = torch.Generator().manual_seed(n + 1)
-    gi, ga = torch.randn((rows or 4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
+    gi, ga = torch.randn((rows or 4, height, width), generator=g) * 1e-3, torch.randn((1, height, width), generator=g) * 1e-3
     cam, v, rast = oracle_camera(view), view.to(DEV), inpc_b200.INPCRasterizer()
     o = opac.to(DEV).requires_grad_(True)
     if rows:
@@ -115,10 +116,11 @@ def test_blend_at_the_edges_of_its_segments(n, rows):
 @pytest.mark.parametrize("n", [700, 4097])
 @pytest.mark.parametrize("odd", ["negative", "nan"])
 @pytest.mark.parametrize("rows", [0, 8])
-def test_odd_opacities_in_lists_of_several_segments(n, odd, rows):
+@pytest.mark.parametrize("width, height", [(24, 16), (1040, 1024)])    # all tiles by two warps per list; more tiles than that, by one
+def test_odd_opacities_in_lists_of_several_segments(n, odd, rows, width, height):
     import inpc_b200
     from helpers import assert_close, oracle_camera
-    view, pos, opac = _one_tile_scene(n, n)
+    view, pos, opac = _one_tile_scene(n, n, width, height)
     opac = opac.clone()
     if odd == "negative":
         opac[::9] *= -0.5
@@ -151,14 +153,15 @@ def test_odd_opacities_in_lists_of_several_segments(n, odd, rows):
 # those behind; the others are as they were.
 @pytest.mark.parametrize("n", [1, 5, 40, 700, 4097])
 @pytest.mark.parametrize("rows, tile", [(0, 8), (0, 16), (4, 8), (16, 8), (8, 16)])
-def test_gradients_behind_an_opacity_that_is_no_number(n, rows, tile):
+@pytest.mark.parametrize("width, height", [(24, 16), (1040, 1024)])    # all tiles by two warps per list; more tiles than that, by one
+def test_gradients_behind_an_opacity_that_is_no_number(n, rows, tile, width, height):
     import inpc_b200
     from helpers import assert_close, oracle_camera
-    view, pos, opac = _one_tile_scene(n, n)
+    view, pos, opac = _one_tile_scene(n, n, width, height)
     opac = opac.clone()
     opac[torch.argsort(3.0 - pos[:, 2])[n * 3 // 4]] = float("nan")
     g = torch.Generator().manual_seed(n + 1)
-    gi, ga = torch.randn((rows or 4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
+    gi, ga = torch.randn((rows or 4, height, width), generator=g) * 1e-3, torch.randn((1, height, width), generator=g) * 1e-3
     cam, v, rast = oracle_camera(view), view.to(DEV), inpc_b200.INPCRasterizer(tile_size=tile)
     o = opac.to(DEV).requires_grad_(True)
     if rows:
@@ -186,18 +189,19 @@ def test_gradients_behind_an_opacity_that_is_no_number(n, rows, tile):
 # also where the opaque splat lies in a later segment.
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("n_before", [100, 255, 256, 300, 511, 700, 1500])
-def test_opacity_gradient_of_an_opaque_splat_in_a_later_segment(mode, n_before):
+@pytest.mark.parametrize("width, height", [(17, 9), (1033, 1025)])      # two warps per list; one
+def test_opacity_gradient_of_an_opaque_splat_in_a_later_segment(mode, n_before, width, height):
     import inpc_b200
     from helpers import assert_close, oracle_camera
     from inpc_b200.views import look_at_view
     n, g = n_before + 20, torch.Generator().manual_seed(n_before)
-    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), 17, 9, 16.0, 16.0)      # the axis meets the centre of pixel (8, 4)
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, 16.0, 16.0, center_x=8.5, center_y=4.5)      # the axis meets the centre of pixel (8, 4)
     pos = torch.zeros((n, 3))
     pos[:, 2] = 1.0 - torch.arange(n) * 2.0 ** -11
     opac = torch.rand((n, 1), generator=g) * min(2e-3, 1.0 / n)
     opac[n_before] = 1.0
     feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
-    gi, ga = torch.randn((4, 9, 17), generator=g) * 1e-3, torch.randn((1, 9, 17), generator=g) * 1e-3
+    gi, ga = torch.randn((4, height, width), generator=g) * 1e-3, torch.randn((1, height, width), generator=g) * 1e-3
     o = opac.to(DEV).requires_grad_(True)
     image, alpha, _ = inpc_b200.INPCRasterizer()(view.to(DEV), mode, pos.to(DEV), feats.to(DEV), o)
     torch.autograd.backward([image, alpha], [gi.to(DEV), ga.to(DEV)])
@@ -212,12 +216,13 @@ def test_opacity_gradient_of_an_opaque_splat_in_a_later_segment(mode, n_before):
 # the one behind them in the same or in the next.
 @pytest.mark.parametrize("apart", [False, True])
 @pytest.mark.parametrize("rows", [0, 8])
-def test_pixels_just_above_the_stop_in_a_later_segment(apart, rows):
+@pytest.mark.parametrize("width, height", [(64, 64), (1040, 1024)])     # two warps per list; one
+def test_pixels_just_above_the_stop_in_a_later_segment(apart, rows, width, height):
     import inpc_b200
     from helpers import assert_close, oracle_camera
     from inpc_b200.views import look_at_view
     side, u, stop = 64, 2.0 ** -24, float(np.float32(1e-4))
-    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), side, side, float(side), float(side))
+    view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, float(side), float(side), center_x=side / 2, center_y=side / 2)
     cam = oracle_camera(view)
 
     def at(px, py, depth):
@@ -260,22 +265,24 @@ def test_pixels_just_above_the_stop_in_a_later_segment(apart, rows):
         half[n - m:, :4] = 2e4
         st = O.rasterize_forward(O.BILINEAR, cam, pos.numpy(), half, opac)
         image, alpha, bw = rast(v, 0, p, torch.from_numpy(half).to(DEV), o)
-    assert (st.image[:, ::2, ::2] > 0.2).all()                                       # a ten-thousandth of what the last splats hold
+    sites = np.s_[:, 0:side:2, 0:side:2]
+    assert (st.image[sites] > 0.2).all()                                             # a ten-thousandth of what the last splats hold
     # the transmittance is 1 - alpha with alpha of almost 1: a rounding of the opacity's product is 2^-24 / 3.4e-4
-    assert_close(image.cpu().numpy()[:, ::2, ::2], st.image[:, ::2, ::2], rtol=4e-4, what="image")
+    assert_close(image.cpu().numpy()[sites], st.image[sites], rtol=4e-4, what="image")
     assert_close(bw.cpu().numpy()[n - m:], st.blending_weights[n - m:], rtol=4e-4, what="blending weights")
-    assert float(alpha.min()) >= 0.0 and bool((alpha[0, ::2, ::2] == 1.0).all())
+    assert float(alpha.min()) >= 0.0 and bool((alpha[sites] == 1.0).all())
 
 
 # The same over all blends, against the same splats in a list of one segment: clear splats between them do not move a pixel's stop.  The
 # opacities are chosen from what an almost opaque splat alone leaves, so that a pixel's transmittance lies within 10^-4 of the stop on either side.
 @pytest.mark.parametrize("inference", [False, True])
 @pytest.mark.parametrize("mode,tile", [(0, 8), (0, 16), (1, 8), (1, 16)])
-def test_clear_splats_do_not_move_the_stop(mode, tile, inference):
+@pytest.mark.parametrize("width, height", [(64, 64), (1040, 1024)])     # two warps per list; one
+def test_clear_splats_do_not_move_the_stop(mode, tile, inference, width, height):
     import inpc_b200
     from inpc_b200.views import look_at_view
     side, clear, trials = 64, 300 if tile == 8 else 6000, 8          # a first segment has 256 or 4096 instances here
-    v = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), side, side, float(side), float(side)).to(DEV)
+    v = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, float(side), float(side), center_x=side / 2, center_y=side / 2).to(DEV)
     rast, g = inpc_b200.INPCRasterizer(tile_size=tile), torch.Generator().manual_seed(tile + mode)
 
     def at(px, py, depth):
@@ -287,7 +294,7 @@ def test_clear_splats_do_not_move_the_stop(mode, tile, inference):
         feats[n - lit:, :4] = 2e4
         opac = torch.cat(opacities).reshape(-1, 1).contiguous().to(DEV)
         out = rast.render_preextracted(v, mode, pos, feats.to(DEV), opac) if inference else rast(v, mode, pos, feats.to(DEV), opac)
-        return out[0][0, 1::4, 1::4].cpu().reshape(-1), out[2 if inference else 1][0, 1::4, 1::4].cpu().double().reshape(-1)
+        return out[0][0, 1:side:4, 1:side:4].cpu().reshape(-1), out[2 if inference else 1][0, 1:side:4, 1:side:4].cpu().double().reshape(-1)
     c, t = torch.arange(1, side, 4, dtype=torch.float32) + 0.5, torch.arange(tile / 2, side, tile)
     py, px = (x.reshape(-1) for x in torch.meshgrid(c, c, indexing="ij"))
     ty, tx = (x.reshape(-1).repeat(clear) for x in torch.meshgrid(t, t, indexing="ij"))
@@ -310,11 +317,15 @@ def test_clear_splats_do_not_move_the_stop(mode, tile, inference):
 # Lists of several segments of very faint splats: the segments' transmittances come from sums of logarithms, which may be no
 # further from double precision than the chain of fp32 products the oracle forms.
 @pytest.mark.parametrize("n,opacity", [(40_000, 2e-6), (200_000, 2e-6), (200_000, 2e-5)])
-def test_faint_splats_are_as_exact_as_a_chain_of_products(n, opacity):
+@pytest.mark.parametrize("width, height", [(96, 64), (1040, 1024)])     # two warps per list; one
+def test_faint_splats_are_as_exact_as_a_chain_of_products(n, opacity, width, height):
+    from dataclasses import replace
     import inpc_b200
     from helpers import oracle_camera, small_scene
+    from inpc_b200.views import View
     view, pos, feats, opac = small_scene(n=n, width=96, height=64, focal=82.0)
     opac = (opac * opacity).contiguous()
+    view = View(replace(view.camera, width=width, height=height), view.w2c, view.position)      # (the same pixels in its upper left corner)
     _, alpha, _ = inpc_b200.INPCRasterizer()(view.to(DEV), 0, pos.to(DEV), feats.to(DEV), opac.to(DEV))
     st = O.rasterize_forward(O.BILINEAR, oracle_camera(view), pos.numpy(), feats.numpy(), opac.numpy())
     # double precision: -log of the product over the 2x2 pixels of every visible point
@@ -328,7 +339,7 @@ def test_faint_splats_are_as_exact_as_a_chain_of_products(n, opacity):
             ok = (px >= 0) & (px < 96) & (py >= 0) & (py < 64)
             np.add.at(total, (py[ok], px[ok]), np.log1p(-op[ok] * w[ok]))
     exact = -np.expm1(total)
-    off = [np.sqrt(((a.reshape(64, 96).astype(np.float64) - exact) ** 2).mean()) for a in (alpha.cpu().numpy(), st.alpha)]
+    off = [np.sqrt(((a.reshape(height, width)[:64, :96].astype(np.float64) - exact) ** 2).mean()) for a in (alpha.cpu().numpy(), st.alpha)]
     assert off[0] <= 1.25 * off[1], off
 
 
@@ -371,13 +382,14 @@ def _clear_of_the_cutoff(st, pos, threshold, reach):
 
 
 @pytest.mark.parametrize("n", [1, 31, 33, 255, 257, 513, 20_001, 700_001])
-def test_gaussian_blend_at_the_edges_of_its_segments(n):
+@pytest.mark.parametrize("width, height", [(24, 16), (1040, 1024)])    # all tiles by two warps per list; more tiles than that, by one
+def test_gaussian_blend_at_the_edges_of_its_segments(n, width, height):
     import inpc_b200
     from helpers import assert_close, oracle_camera
-    view, pos, opac = _one_tile_scene(n, n)
+    view, pos, opac = _one_tile_scene(n, n, width, height)
     cam = oracle_camera(view)
     g = torch.Generator().manual_seed(n + 1)
-    gi, ga = torch.randn((4, 16, 24), generator=g) * 1e-3, torch.randn((1, 16, 24), generator=g) * 1e-3
+    gi, ga = torch.randn((4, height, width), generator=g) * 1e-3, torch.randn((1, height, width), generator=g) * 1e-3
     feats = (torch.randn((n, 36), generator=g) * 0.5).to(torch.float16)
     pos, dropped = _clear_of_the_cutoff(O.preprocess_and_order(O.GAUSSIAN, O.TRAIN, cam, pos.numpy(), feats.numpy(), opac.numpy()), pos,
                                         0.01110899653, 3)

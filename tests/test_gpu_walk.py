@@ -147,11 +147,11 @@ def test_lists_of_many_segments(segments, opaque):
             assert float((a - b).norm()) <= max(1e-4, 2 * n * U) * float(b.norm())
 
 
-# Two warps per list (images of up to 2^15 tiles) against one: the same points in the upper left corner of an image that has more tiles.  Lists of every length beside a batch of 32, of
+# Two warps per list (images of few tiles) against one: the same points in the upper left corner of an image that has more tiles than that.  Lists of every length beside a batch of 32, of
 # faint splats, of which nothing stops, and of opaque ones, where the pixels stop in the middle of a batch, at its end, and one after the other
 @pytest.mark.parametrize("opacity", [0.004, 0.3, 0.97, None])
-@pytest.mark.parametrize("channels", [None, 4, 8, 16, 32])
-def test_lists_walked_by_two_warps_and_by_one(channels, opacity):
+@pytest.mark.parametrize("channels, mode", [(None, 0), (4, 0), (8, 0), (16, 0), (32, 0), (None, 1)])
+def test_lists_walked_by_two_warps_and_by_one(channels, mode, opacity):
     import inpc_b200
     from inpc_b200.views import look_at_view
     width, height = 128, 16
@@ -171,13 +171,14 @@ def test_lists_walked_by_two_warps_and_by_one(channels, opacity):
         view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), w, h, 64.0, 64.0, center_x=64.0, center_y=8.0).to(DEV)
         f, o = feats.clone().requires_grad_(True), opac.clone().requires_grad_(True)
         rast = inpc_b200.INPCRasterizer()
-        image, alpha, weights = rast.forward_rows(view, pos, f, o) if channels else rast(view, 0, pos, f, o)
+        image, alpha, weights = rast.forward_rows(view, pos, f, o) if channels else rast(view, mode, pos, f, o)
         torch.autograd.backward([image[:, :height, :width], alpha[:, :height, :width]], [gi, ga])
         out.append((image[:, :height, :width].detach(), alpha[:, :height, :width].detach(), weights, f.grad, o.grad))
     assert int((out[0][1] > 0).sum()) > 500
     for k, (a, b) in enumerate(zip(*out)):
         # images and alphas to the bit, and the gradients of four channels, which have one writer each; the others are sums of up to four atomic additions in any order
-        if k < 2 or (k > 2 and channels is None):
+        if k < 2 or (k > 2 and channels is None and mode == 0):
             assert torch.equal(a, b), k
         else:
-            assert float((a - b).abs().max()) <= 8 * 2.0 ** -24 * float(torch.maximum(a.abs(), b.abs()).max()), k
+            step = 2.0 ** -11 if k == 3 and mode == 1 else 8 * 2.0 ** -24       # (feature gradients of gaussian splats: a step of a half)
+            assert float((a.float() - b.float()).abs().max()) <= step * float(torch.maximum(a.abs(), b.abs()).max()), k

@@ -83,6 +83,41 @@ def test_blend_passes_launch_the_blocks_that_are_resident(tmp_path):
         assert a["grid"][0] == multiprocessors * fit, (name, a["grid"][0] / multiprocessors, fit)
 
 
+# Which form a training step takes, on both sides of each line: images of 4096 tiles, 4160, 16384, 16640 and 33280, and the points per tile from which two warps take an item
+@pytest.mark.parametrize("mode, channels, least, lines", [(0, None, 128, [(512, 512, True), (520, 512, None), (4096, 520, False)]), (0, 8, 32, [(512, 512, True), (520, 512, None), (4096, 520, False)]),
+                                                          (1, None, 64, [(1024, 1024, True), (1040, 1024, None)])])
+def test_where_two_warps_take_an_item(mode, channels, least, lines):
+    import inpc_b200
+    from inpc_b200.views import look_at_view
+    from torch.profiler import ProfilerActivity, profile
+    rast = inpc_b200.INPCRasterizer()
+
+    def step(width, height, n):
+        view = look_at_view((0.0, 0.0, 3.0), (0.0, 0.0, 0.0), width, height, float(width), float(width)).to(DEV)
+        pos, opac = torch.full((n, 3), 9.0, device=DEV), torch.full((n, 1), 0.1, device=DEV).requires_grad_(True)      # (behind the camera: the rule asks how many there are)
+        f = torch.zeros((n, channels), device=DEV) if channels else torch.zeros((n, 36), dtype=torch.float16, device=DEV)
+        f.requires_grad_(True)
+        image, alpha, _ = rast.forward_rows(view, pos, f, opac) if channels else rast(view, mode, pos, f, opac)
+        (image.sum() + alpha.sum()).backward()
+
+    step(64, 64, 10)
+    for width, height, always in lines:
+        tiles = width * height // 64
+        for n in (least * tiles - 1, least * tiles):
+            with profile(activities=[ProfilerActivity.CUDA]) as p:
+                step(width, height, n)
+                torch.cuda.synchronize()
+            names = [e.key for e in p.key_averages()]
+            if not any("inpc" in k for k in names):
+                pytest.skip("no activity records of kernels here")
+            paired = always if always is not None else n >= least * tiles
+            forward = [k for k in names if "blend" in k and "forward" in k]
+            assert sum("_pair_forward" in k for k in forward) == (2 if paired else 0), (width, height, n, forward)
+            assert sum("_warp_forward" in k for k in forward) == (1 if paired else 3), (width, height, n, forward)
+            if mode == 0 and not channels:
+                assert any("blend_bilinear_pair_backward" in k for k in names) == paired
+
+
 # Images are not cleared beforehand: tiles without instances are blanked at the end.  Into memory full of NaN; odd sizes; nothing, one point, all points culled, a few tiles with lists
 # of one and of several segments among many empty ones
 @pytest.mark.parametrize("width, height", [(8, 8), (101, 53), (1237, 40)])
