@@ -1915,21 +1915,26 @@ struct CandidateStream {
 // Pass PRODUCT, a warp that has left an item's products in seg_T (a pixel per lane): where it is the last of the tile half to do so, seg_T of every later segment becomes the transmittance at its
 // start = the state behind segment 0 times the products of the segments between.  `item`: of the list of later segments, where those of a tile lie in a row.
 // A kernel of its own between the passes took 4 to 8 us and a launch.  Where every item formed its start itself, in the later segments and again backward, lists of many segments were read in the
-// square of their number: training step of 2^24 almost opaque splats in one tile (4096 segments) 2690 us, 2550 so (backward 132 -> 35), of 2^26 rows of four channels 10760 -> 9040
-// (511 -> 54); of 2^24 faint ones 5405 -> 5255; 2^23 samples at 1237x822 1268 -> 1272, 10^6 at 801x533 300 both.
-__device__ __forceinline__ void finish_products(const WarpItem* items, unsigned item, unsigned half, unsigned seg, unsigned n_seg, float* seg_T, unsigned first, unsigned lane) {
+// square of their number: training step of 2^24 almost opaque splats in one tile (4096 segments) 2660 us, 2520 so (backward 132 -> 35), of 2^26 rows of four channels 10760 -> 9040
+// (511 -> 54); of 2^24 faint ones 5360 -> 5230.  Products 1 to 3 us longer for it, with a fence on either side of a relaxed addition 2 to 4: 2^23 samples at 1237x822 122.6 -> 125.3 (127.0), of
+// which the backward pass gains 1.5; 10^6 at 801x533 32.8 -> 34.8.  More loads at once than 16 spill.
+__device__ __forceinline__ void finish_products(const WarpItem* items, unsigned item, unsigned half, unsigned seg, unsigned n_seg, float* seg_T, unsigned first, bool inside, unsigned lane) {
     if (n_seg > 2u) {
-        __threadfence();   // every lane's product, before it counts as finished
-        __syncwarp();
+        __syncwarp();   // every lane's product, before it counts as finished
         unsigned before = 0u;
-        if (lane == 0u) before = atomicAdd(const_cast<uint32_t*>(&items[item - (seg - 1u)].finished[half]), 1u);
+        if (lane == 0u) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(&items[item - (seg - 1u)].finished[half]) : "memory");
         if (__shfl_sync(0xffffffffu, before, 0) != n_seg - 2u) return;
-        __threadfence();
+        __syncwarp();   // what the first lane has acquired, the others see too
     }
     float* base = seg_T + ((size_t)first * 2u + half) * 32 + lane;   // segment g of this half: base[g * 64]
     constexpr int kAtOnce = 16;   // loads that do not wait for one another
     float run = base[0];
     for (unsigned g0 = 1; g0 < n_seg; g0 += kAtOnce) {
+        if (__all_sync(0xffffffffu, !inside || run < kTransmittanceEps)) {
+            // every pixel has stopped: nothing behind has an effect, and any state below the threshold says so
+            for (unsigned g = g0; g < n_seg; ++g) base[(size_t)g * 64] = run;
+            break;
+        }
         float product[kAtOnce];
 #pragma unroll
         for (int k = 0; k < kAtOnce; ++k) product[k] = g0 + k + 1u < n_seg ? __ldcg(base + (size_t)(g0 + k) * 64) : 1.0f;   // (of other warps: not through L1)
@@ -2201,7 +2206,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, forward_blocks(PASS, C4)
 
         if (PASS == PASS_PRODUCT) {
             seg_T[sidx * 32 + lane] = (float)exp2(-log_sum);   // this segment's product
-            finish_products(items, item >> 1, (unsigned)half, seg, n_seg, seg_T, first, lane);
+            finish_products(items, item >> 1, (unsigned)half, seg, n_seg, seg_T, first, inside, lane);
             continue;
         }
         const int64_t n_px = (int64_t)width * height;
@@ -4143,7 +4148,7 @@ __global__ void __launch_bounds__(kWarpBlendWarps * 32, kGaussForwardBlocks) ble
 
         if (PASS == PASS_PRODUCT) {
             seg_T[sidx * 32 + lane] = Tr;   // this segment's product
-            finish_products(items, item >> 1, (unsigned)half, seg, n_seg, seg_T, first, lane);
+            finish_products(items, item >> 1, (unsigned)half, seg, n_seg, seg_T, first, inside, lane);
             continue;
         }
         const int64_t n_px = (int64_t)width * height;
