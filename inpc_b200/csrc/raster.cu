@@ -5189,21 +5189,20 @@ int launch_bilinear_warp_forward(const RasterParams& rp, int64_t n_points, const
 int launch_bilinear_warp_backward(const RasterParams& rp, int64_t n_points, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
-    auto launch = [&](auto kernel, size_t smem, int most, int (&known)[kMaxDevices]) -> int {
+    auto launch = [&](auto kernel, const char* name, size_t smem, int most, int (&known)[kMaxDevices]) -> int {
         BlendGrid grid;
         const int rc = warp_blend_grid(kernel, smem, most, true, PASS_FIRST, known, &grid);
         if (rc != INPC_OK) return rc;
         launch_chained(kernel, grid.blocks, kWarpBlendWarps * 32, smem, stream,
             ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
             ib.seg_T, ib.seg_C, grad_image, grad_alpha, image, alpha, slot_grad, slot_mask, rp.v.width, rp.v.height, rp.gw);
+        INPC_LAUNCH_CHECK(name);
         return INPC_OK;
     };
     static int known[kMaxDevices] = {0}, known_pairs[kMaxDevices] = {0};
-    const int rc = by_two_warps(INPC_MODE_BILINEAR, false, (int64_t)rp.gw * rp.gh, n_points) ? launch(blend_bilinear_pair_backward_kernel, kPairBackwardSmemBytes, kPairBackwardBlocks, known_pairs)
-                                               : launch(blend_bilinear_warp_backward_kernel, kWarpBackwardSmemBytes, kBackwardBlocks, known);
-    if (rc != INPC_OK) return rc;
-    INPC_LAUNCH_CHECK("blend_bilinear backward");
-    return INPC_OK;
+    return by_two_warps(INPC_MODE_BILINEAR, false, (int64_t)rp.gw * rp.gh, n_points)
+               ? launch(blend_bilinear_pair_backward_kernel, "blend_bilinear_pair_backward_kernel", kPairBackwardSmemBytes, kPairBackwardBlocks, known_pairs)
+               : launch(blend_bilinear_warp_backward_kernel, "blend_bilinear_warp_backward_kernel", kWarpBackwardSmemBytes, kBackwardBlocks, known);
 }
 
 template <int T, int KIND>

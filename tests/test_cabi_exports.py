@@ -81,6 +81,13 @@ def test_host_side_validation_without_gpu():
         _cabi.check(-1)
 
 
+def test_failed_launches_are_reported_under_the_name_of_their_kernel():
+    sources = "".join(p.read_text() for p in sorted((ROOT / "inpc_b200" / "csrc").glob("*.cu")))
+    kernels = set(re.findall(r"\b(\w+_kernel)\s*\(", sources))
+    named = [name for check in re.findall(r"INPC_LAUNCH_CHECK\((.*)\);", sources) for name in re.findall(r'"([^"]*)"', check)]
+    assert len(named) > 40 and not [name for name in named if name not in kernels]
+
+
 def test_product_never_touches_the_oracle():
     """The package must not import, load or execute anything under oracle/ (no CPU fallback)."""
     for path in (ROOT / "inpc_b200").rglob("*"):
