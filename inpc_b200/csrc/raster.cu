@@ -1504,7 +1504,7 @@ constexpr int kQueueCap = 256;            // ring of candidate point ids per war
 // warps are busy (2800 of the 3552 that fit) for a third of a pass and more, and shorter segments add more work (more lists to filter, more states to carry) than they
 // save.  With fewer instances the passes are as long as their longest items, at 1.3 - 2.4 us per batch of 32, while most
 // warps have none: the segments then get shorter, so that the later ones of all tiles number about kSegmentTarget (two items
-// each, one and a half times the resident warps).  10^6 samples, 801x533: forward / backward 283 / 153 us with 1024 + 4096,
+// each, one and a half times the resident warps, twice to three times the pairs of warps where two take an item).  10^6 samples, 801x533: forward / backward 283 / 153 us with 1024 + 4096,
 // 120 / 56 with the lengths below (149 / 70 with half the target); 2 * 10^5 samples, 600x400: 190 / 86 -> 85 / 35; first segments
 // of a quarter or of all of a later one measured the same or worse.
 constexpr unsigned kSegmentMin = 256;
@@ -1758,6 +1758,9 @@ __global__ void __launch_bounds__(kItemThreads) warp_items_fill_kernel(const uin
 // of every warp one by one, the others 8 or 16 per visit / before there were classes, 6 per visit: training step of 2^25 bilinear splats 9955 / 10620 /
 // 10425 us (first pass 2733 / 2590 / 2488, backward 3658 / 4450 / 4100), 2^26 almost opaque ones 19300 / 21870 / 21460, 2^25 gaussian splats 13630 / 15940 /
 // 15960; inference, 2^22 splats of 3 pixels, faint 4648 / 4778 / 4760, opaque, where most of a list is behind stopped pixels, 2800 / 2856 / 2840.
+// Where two warps take an item the visits are those of a pair (counted as if each warp took items, shares were half as large): step of 512 points per tile, nine tenths in a corner, 1237x822
+// 1066 -> 1001 us, 1920x1080 1865 -> 1819; points spread evenly, 128 per tile, 998 -> 1015 with 6 visits of a pair backward (4: 1028); rows of 16 channels evenly 1428 -> 1325, 2^22 gaussian splats,
+// nine tenths in a corner, 1048 -> 1015, samples of an octree all the same.
 constexpr unsigned kMostItems = 8, kMostItemsBilinear = 16;
 struct ItemQueue {
     unsigned n_items, n_single, per_visit;
@@ -5094,16 +5097,18 @@ int blend_batch(int tile) { return tile * tile * BlendConfig<16>::kIpt; }
 // step of 2^22 samples take 206 to 217 us with three and 204 to 213 with four, but a frame of 2 * 10^6 splats, where they are short, 581 and 585).  With four per multiprocessor for all passes, blocks that found nothing left came last, and a warp's share of the items (see ItemQueue) was
 // counted too small: step of 2^24 points crowding a corner of 3840x2160 2633 -> 2540 us (first pass 347 -> 297, backward 441 -> 392), of 2^23 samples
 // at 1237x822 1623 -> 1608.
-// `visits`: see ItemQueue; `pass`: of the forward passes (PASS_FIRST also for a backward pass).
+// `takers`: warps of a block that take items, or pairs of warps; `visits_each`: of a resident one, 0 for the rule of gaussian splats and rows (see ItemQueue); `pass`: of the forward
+// passes (PASS_FIRST also for a backward pass).
+constexpr unsigned kVisits = 4, kVisitsPairBackward = 6;   // bilinear splats of four channels
 struct BlendGrid {
     unsigned blocks = 1, visits = 1;
 };
 template <typename Kernel>
-int warp_blend_grid(Kernel kernel, size_t smem, int most, bool bilinear, int pass, int (&known)[kMaxDevices], BlendGrid* grid) {
+int warp_blend_grid(Kernel kernel, size_t smem, int most, unsigned takers, unsigned visits_each, int pass, int (&known)[kMaxDevices], BlendGrid* grid) {
     int blocks = 1;
     const int rc = resident_blocks(kernel, kWarpBlendWarps * 32, smem, known, &blocks);
     grid->blocks = (unsigned)(sm_count() * min(blocks, most));
-    grid->visits = bilinear ? grid->blocks * kWarpBlendWarps * 4u : (unsigned)sm_count() * (pass == PASS_FIRST ? 32u : 24u) * 8u;
+    grid->visits = visits_each ? grid->blocks * takers * visits_each : (unsigned)sm_count() * (pass == PASS_FIRST ? 4u : 3u) * takers * 8u;
     return rc;
 }
 // Where in the counts the number of tiles is among which those of several segments lie: they are longer than a first segment, i.e. in the first class where the tiles lie by
@@ -5129,7 +5134,7 @@ int launch_warp_forward_pass(const WarpItem* items, const uint32_t* counts, unsi
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = warp_forward_smem_bytes<PASS, KIND, C4>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, forward_blocks(PASS, C4), !ROWS, PASS, known, &grid);
+    const int rc = warp_blend_grid(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, smem, forward_blocks(PASS, C4), kWarpBlendWarps, ROWS ? 0u : kVisits, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_bilinear_warp_forward_kernel<PASS, KIND, C4, ROWS>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
@@ -5144,7 +5149,7 @@ int launch_pair_forward_pass(const WarpItem* items, const uint32_t* counts, unsi
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = pair_forward_smem_bytes<C4>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_bilinear_pair_forward_kernel<PASS, C4, ROWS>, smem, pair_forward_blocks(C4), !ROWS, PASS, known, &grid);
+    const int rc = warp_blend_grid(blend_bilinear_pair_forward_kernel<PASS, C4, ROWS>, smem, pair_forward_blocks(C4), kPairs, ROWS ? 0u : kVisits, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_bilinear_pair_forward_kernel<PASS, C4, ROWS>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, a.rows, a.seg_T, a.seg_C, a.image, a.alpha, a.blending_weights, a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw);
@@ -5189,9 +5194,9 @@ int launch_bilinear_warp_forward(const RasterParams& rp, int64_t n_points, const
 int launch_bilinear_warp_backward(const RasterParams& rp, int64_t n_points, const PointBlob& pb, const InstanceBlob& ib, int t_alt, const float* grad_image,
                                   const float* grad_alpha, const float* image, const float* alpha, float4* slot_grad,
                                   unsigned* slot_mask, cudaStream_t stream) {
-    auto launch = [&](auto kernel, const char* name, size_t smem, int most, int (&known)[kMaxDevices]) -> int {
+    auto launch = [&](auto kernel, const char* name, size_t smem, int most, unsigned takers, unsigned visits_each, int (&known)[kMaxDevices]) -> int {
         BlendGrid grid;
-        const int rc = warp_blend_grid(kernel, smem, most, true, PASS_FIRST, known, &grid);
+        const int rc = warp_blend_grid(kernel, smem, most, takers, visits_each, PASS_FIRST, known, &grid);
         if (rc != INPC_OK) return rc;
         launch_chained(kernel, grid.blocks, kWarpBlendWarps * 32, smem, stream,
             ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
@@ -5201,8 +5206,8 @@ int launch_bilinear_warp_backward(const RasterParams& rp, int64_t n_points, cons
     };
     static int known[kMaxDevices] = {0}, known_pairs[kMaxDevices] = {0};
     return by_two_warps(INPC_MODE_BILINEAR, false, (int64_t)rp.gw * rp.gh, n_points)
-               ? launch(blend_bilinear_pair_backward_kernel, "blend_bilinear_pair_backward_kernel", kPairBackwardSmemBytes, kPairBackwardBlocks, known_pairs)
-               : launch(blend_bilinear_warp_backward_kernel, "blend_bilinear_warp_backward_kernel", kWarpBackwardSmemBytes, kBackwardBlocks, known);
+               ? launch(blend_bilinear_pair_backward_kernel, "blend_bilinear_pair_backward_kernel", kPairBackwardSmemBytes, kPairBackwardBlocks, kPairs, kVisitsPairBackward, known_pairs)
+               : launch(blend_bilinear_warp_backward_kernel, "blend_bilinear_warp_backward_kernel", kWarpBackwardSmemBytes, kBackwardBlocks, kWarpBlendWarps, kVisits, known);
 }
 
 template <int T, int KIND>
@@ -5249,7 +5254,7 @@ int launch_gaussian_warp_forward_pass(const WarpItem* items, const uint32_t* cou
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = gauss_forward_smem_bytes<PASS, KIND>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, kGaussForwardBlocks, false, PASS, known, &grid);
+    const int rc = warp_blend_grid(blend_gaussian_warp_forward_kernel<PASS, KIND>, smem, kGaussForwardBlocks, kWarpBlendWarps, 0u, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_forward_kernel<PASS, KIND>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.seg_Z, a.seg_E, a.image, a.depth, a.alpha, a.blending_weights,
@@ -5262,7 +5267,7 @@ template <int PASS>
 int launch_gaussian_pair_forward_pass(const WarpItem* items, const uint32_t* counts, unsigned* ticket, const float4* conic, const ForwardPassArgs& a, float reach, cudaStream_t stream) {
     static int known[kMaxDevices] = {0};
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_gaussian_pair_forward_kernel<PASS>, kGaussPairSmemBytes, kGaussPairBlocks, false, PASS, known, &grid);
+    const int rc = warp_blend_grid(blend_gaussian_pair_forward_kernel<PASS>, kGaussPairSmemBytes, kGaussPairBlocks, kPairs, 0u, PASS, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_pair_forward_kernel<PASS>, grid.blocks, kWarpBlendWarps * 32, kGaussPairSmemBytes, stream,
         items, counts, ticket, grid.visits, a.keys, a.ids, a.rec, conic, a.seg_T, a.seg_C, a.image, a.alpha, a.blending_weights, a.kept0, a.kept1, a.n_kept, a.W, a.H, a.gw, reach);
@@ -5304,7 +5309,7 @@ int launch_gaussian_warp_backward(const RasterParams& rp, const PointBlob& pb, c
                                   cudaStream_t stream) {
     static int known[kMaxDevices] = {0};
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, kGaussBackwardBlocks, false, PASS_FIRST, known, &grid);
+    const int rc = warp_blend_grid(blend_gaussian_warp_backward_kernel, kGaussBackwardSmemBytes, kGaussBackwardBlocks, kWarpBlendWarps, 0u, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_gaussian_warp_backward_kernel, grid.blocks, kWarpBlendWarps * 32, kGaussBackwardSmemBytes, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec, pb.conic, ib.seg_T, ib.seg_C,
@@ -5382,7 +5387,7 @@ int launch_rows_warp_backward(const RasterParams& rp, const PointBlob& pb, const
     static int known[kMaxDevices] = {0};
     constexpr size_t smem = rows_warp_backward_smem_bytes<C4>();
     BlendGrid grid;
-    const int rc = warp_blend_grid(blend_rows_warp_backward_kernel<C4>, smem, rows_backward_blocks(C4), false, PASS_FIRST, known, &grid);
+    const int rc = warp_blend_grid(blend_rows_warp_backward_kernel<C4>, smem, rows_backward_blocks(C4), kWarpBlendWarps, 0u, PASS_FIRST, known, &grid);
     if (rc != INPC_OK) return rc;
     launch_chained(blend_rows_warp_backward_kernel<C4>, grid.blocks, kWarpBlendWarps * 32, smem, stream,
         ib.items0, ib.items1, ib.n_segments, ib.n_segments + 5, grid.visits, ib.ids[1 - t_alt], ib.keys[1 - t_alt], ib.n_kept, pb.rec,
