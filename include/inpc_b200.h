@@ -217,6 +217,11 @@ int inpc_raster_resolve(inpc_raster_state* state, void* stream);
 int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc_view* view, int which, void* dst,
                            void* stream);
 
+/* Test hook for the approximate arithmetic of the blend, which has no counterpart in the reference.  which 0: out (n f32) = 1 / max(x, 1e-8)
+ * as the backward passes form it of in (n f32); 1: out (n u32) = the pixels of an 8x4 half (bit = row * 8 + column)
+ * that a gaussian splat is taken to reach, of in (n,8 f32): screen x, y, conic (3), reach, first column and row of the half. */
+int inpc_debug_arithmetic(int which, int64_t n, const float* in, void* out, void* stream);
+
 /* Stable least-significant-digit radix sort of (u32 key, u32 value) pairs on bits [0, end_bit),
  * the library's own onesweep.  keys_alt / values_alt are same-sized ping-pong buffers; `workspace`
  * needs inpc_sort_workspace_bytes(n), which never falls as n grows: one sized for the largest n serves

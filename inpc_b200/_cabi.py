@@ -54,6 +54,7 @@ PROTOTYPES = {
     "inpc_rasterize_rows_backward": (_I, [_SP, _VP, _P, _P, _P, _P, _P, _P, _P, _P]),
     "inpc_render_rows": (_I, [_I, _VP, _L, _P, _P, _I, _P, _P, _P, _P, ALLOC_FN, ALLOC_FN, _P, _P]),
     "inpc_raster_debug_copy": (_I, [_SP, _VP, _I, _P, _P]),
+    "inpc_debug_arithmetic": (_I, [_I, _L, _P, _P, _P]),
     "inpc_raster_resolve": (_I, [_SP, _P]),
     "inpc_sort_workspace_bytes": (_Z, [_L]),
     "inpc_sort_pairs": (_I, [_P, _P, _P, _P, _L, _I, _P, C.POINTER(C.c_int), _P]),

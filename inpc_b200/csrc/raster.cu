@@ -5797,7 +5797,28 @@ __global__ void unpack_points_kernel(const PointRec* __restrict__ rec, int rec_s
         o[2] = (unsigned short)(b.y & 0xffffu); o[3] = (unsigned short)(b.y >> 16);
     }
 }
+
+__global__ void arithmetic_kernel(int which, int64_t n, const float* __restrict__ in, void* __restrict__ out) {
+    await_previous_kernel();
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (which == 0) {
+        static_cast<float*>(out)[i] = one_minus_alpha_reciprocal(in[i]);
+    } else {
+        const float* v = in + 8 * i;
+        static_cast<unsigned*>(out)[i] = ellipse_pixels(make_float4(v[0], v[1], 0.0f, 0.0f), make_float4(v[2], v[3], v[4], 0.0f), v[5], (int)v[6], (int)v[7]);
+    }
+}
 }  // namespace inpc_debug
+
+extern "C" int inpc_debug_arithmetic(int which, int64_t n, const float* in, void* out, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (which < 0 || which > 1 || n < 0 || n >= ((int64_t)1 << 30) || (n > 0 && (!in || !out))) { set_error("inpc_debug_arithmetic: bad argument"); return INPC_E_INVALID; }
+    if (n == 0) return INPC_OK;
+    launch_chained(inpc_debug::arithmetic_kernel, (unsigned)ceil_div<int64_t>(n, 256), 256, 0, stream, which, n, in, out);
+    INPC_LAUNCH_CHECK("arithmetic_kernel");
+    return INPC_OK;
+}
 
 extern "C" int inpc_raster_debug_copy(const inpc_raster_state* state, const inpc_view* view, int which, void* dst,
                                       void* stream_) {
