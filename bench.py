@@ -42,9 +42,9 @@ N_LEAVES = 1 << 18
 N_APPEARANCE = 1 << 22
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per (point, tile) instance of the kernels of a
 # stage, from an ncu capture of the warp blend kernels on the small case of this workload (2^22 points,
-# 5,274,412 instances, 8x8 tiles: forward passes 445.6 MB, backward 343.1 MB); the traffic of these kernels grows in
+# 5,274,412 instances, 8x8 tiles: forward passes 446.1 MB, backward 341.3 MB); the traffic of these kernels grows in
 # proportion to the instances.
-TRAFFIC_BYTES_PER_INSTANCE = {"blend_fwd": 445.6e6 / 5274412, "blend_bwd": 343.1e6 / 5274412}
+TRAFFIC_BYTES_PER_INSTANCE = {"blend_fwd": 446.1e6 / 5274412, "blend_bwd": 341.3e6 / 5274412}
 
 
 def parse_args():

@@ -4897,7 +4897,9 @@ int run_front(const RasterParams& rp, int64_t n, const float* positions, const v
     // paths (gaussian splats have no such bound, feature rows keep their scratch small) read the counts back once.
     const bool deferred = defers_counts(MODE, rp.tile, VARIANT == VAR_ROWS, n, stream);
     int64_t n_visible = 0, n_instances = 0;
-    // depth keys are offsets from the near plane's bit pattern, bounded by the far plane's: nothing is measured
+    // depth keys are offsets from the near plane's bit pattern, bounded by the far plane's: nothing is measured.  (Where the range of the depths was measured first, in a pass that also counted and
+    // compacted, planes 0.01 and 100 / 0.01 and 1000 / 0 and 100: step of 2^22 gaussian splats 1482 / 1479 / 1479 us, 1235 / 1272 / 1272 so; of 2^23 rows of 16 channels 1553 / 1556 / 1557,
+    // 1399 / 1430 / 1522; of 2^22 bilinear splats on 16x16 tiles 1475 / 1480 / 1476, 1457 / 1472 / 1486.)
     const float near_depth = rp.v.near_plane > 0.0f ? rp.v.near_plane : 0.0f;
     const float far_depth = rp.v.far_plane != rp.v.far_plane ? INFINITY   // a far plane that is no number culls nothing
                                                              : rp.v.far_plane > near_depth ? rp.v.far_plane : near_depth;

@@ -1430,7 +1430,7 @@ extern "C" int inpc_draw_leaf_counts(inpc_sampler* s, int64_t n_cells, const flo
     return INPC_OK;
 }
 
-// `box_words` (optional): 6 kBoxCopies words that start at zero, see box_word.
+// `box_words` (optional): 6 kBoxCopies words, see box_word, and the count of finished blocks behind them; all start at zero.
 static int launch_halton(const char* who, const uint32_t* counts, int64_t n_cells, const float* centers, const int32_t* levels, float initial_size, int64_t n_total,
                          float* positions, void* workspace, unsigned* box_words, MortonCube* cube, unsigned* codes, cudaStream_t stream) {
     if (n_cells <= 0 || n_cells >= ((int64_t)1 << 31) || n_total < 0 || n_total >= ((int64_t)1 << 32) || !counts || !centers || !levels || !positions || !workspace) {
