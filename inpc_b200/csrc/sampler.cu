@@ -1047,9 +1047,10 @@ __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float*
     await_previous_kernel();
     const int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 4;
     if (i >= n) return;
+    const unsigned last = (unsigned)(n - 1);   // behind a sort that has given up (and reported it) the order has holes, which may hold anything
     if (vec_ok && i + 4 <= n) {
         const uint4 o = __ldg(reinterpret_cast<const uint4*>(order + i));
-        const unsigned j[4] = {o.x, o.y, o.z, o.w};
+        const unsigned j[4] = {min(o.x, last), min(o.y, last), min(o.z, last), min(o.w, last)};
         float v[12];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -1062,7 +1063,7 @@ __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float*
             const float2* src = reinterpret_cast<const float2*>(positions) + ((3 * (int64_t)j[k]) >> 1);
             const float2 a = __ldg(src);
             float2 b = make_float2(0.0f, 0.0f);
-            if (j[k] + 1u < n || (j[k] & 1u)) b = __ldg(src + 1);
+            if (j[k] < last || (j[k] & 1u)) b = __ldg(src + 1);
             else b.x = __ldg(reinterpret_cast<const float*>(src + 1));
             const bool odd = j[k] & 1u;
             v[3 * k] = odd ? a.y : a.x; v[3 * k + 1] = odd ? b.x : a.y; v[3 * k + 2] = odd ? b.y : b.x;
@@ -1073,7 +1074,7 @@ __global__ void __launch_bounds__(kThreads) gather_positions_kernel(const float*
         return;
     }
     for (int64_t k = i; k < n && k < i + 4; ++k) {
-        const int64_t j = __ldg(order + k);
+        const int64_t j = min(__ldg(order + k), last);
 #pragma unroll
         for (int c = 0; c < 3; ++c) out[3 * k + c] = __ldg(positions + 3 * j + c);
     }
