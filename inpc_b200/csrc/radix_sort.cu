@@ -114,6 +114,14 @@ struct PackedFields {
 // log2 of the tiles a splat touches, of a footprint word with bit 31 set.
 __device__ __forceinline__ unsigned tiles_log2_of_escaped(uint32_t q) { return ((q & 0xFu) == 9u ? 1u : 0u) + ((q >> 16 & 0xFu) == 9u ? 1u : 0u); }
 
+// A look-back that has given up: reported, and the count withdrawn.  What is sorted now has holes that hold whatever lay there: whoever reads the count finds nothing to read.
+// (Not inlined: the passes over large tiles, which use all the registers there are, then spill nothing; inlined up to 8 bytes.  2^25 pairs of 30 bits 570 -> 566 us, the depth and tile
+// sorts of 2^24 points at 3840x2160 672 -> 662.)
+__device__ __noinline__ void give_up(volatile unsigned* status, unsigned long long* withdraw) {
+    status[STATUS_LOOKBACK_TIMEOUT] = 1u;
+    if (withdraw) *withdraw = 0ull;
+}
+
 // BITS > 0 fixes the digit width at compile time; BITS == 0 takes it from `bits_arg`.
 // PASS_MARKED: keys of kNoKey take no part, and the values are the positions.  Points that are culled get such a key where they lie, which
 // spares the projection a pass that counts the visible ones beforehand, a scan and the point ids: training step of 2^23 samples at 1237x822
@@ -176,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
 
         // 1. stable rank within the warp's segment, per digit
         // Two 16-bit positions in a word: 64 registers do not hold keys, values and positions otherwise, and what they spilled
-        // (13 of them; one is left in the passes of 7 and 8 bits over large tiles) went through the unit the pass is bound by.  10.6 M pairs of 14 bits 130.5 -> 126.5 us, 2^25 of 30 bits 594 -> 573.
+        // (13 of them) went through the unit the pass is bound by.  10.6 M pairs of 14 bits 130.5 -> 126.5 us, 2^25 of 30 bits 594 -> 573.
         unsigned pos2[ITEMS / 2];
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) {
@@ -274,11 +282,7 @@ __global__ void __launch_bounds__(kThreads, 2) radix_onesweep_pass_kernel(
                     }
                     j -= kWindow;
                 }
-                if (gave_up) {
-                    status[STATUS_LOOKBACK_TIMEOUT] = 1u;
-                    // what is sorted now has holes that hold whatever lay there: whoever reads the count finds nothing to read
-                    if (withdraw) *withdraw = 0ull;
-                }
+                if (gave_up) give_up(status, withdraw);
                 tile_state[tile * kBins + tid] = ((exclusive + total) & kValueMask) | kFlagPrefix;
             }
             s.global_off[tid] = __ldg(digit_base + tid) + exclusive - start;
